@@ -143,6 +143,18 @@ int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v
                            const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
                            float* states, int32_t* counts, int32_t* status, void* stream);
 /*
+ * The forward and the Fenwick state of B equally long prompts in one call, T any length.
+ * Replaces: hattention_prefill (models/hattention/kernel.py:470-560) with its split into whole chunks and the
+ * remaining T mod 64 tokens, which here take one launch (fp32, the arithmetic of lampa_hgdn_step) instead of one per token.
+ *   Arguments as in lampa_hgdn_fwd (no cu_seqlens) and lampa_hgdn_final_state, except: counts int32 [L], one row;
+ *   the state is the one after all T tokens, no null tokens; the workspace is the one of the whole chunks
+ *   (lampa_gdn_workspace_bytes with T rounded down to a multiple of 64).  L has to hold the T tokens; when the tail
+ *   needs a level that is missing, LAMPA_ERR_LEVELS is set in the status word and the remaining tokens are left out.
+ */
+int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                       const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
+                       float* states, int32_t* counts, int32_t* status, void* stream);
+/*
  * One decode step of the hierarchical rule on a Fenwick state, in place.
  * Replaces: hattention_step -> step_state / step_output (models/hattention/kernel.py:570-633,
  * recurrent.py:134-166, HState.cascade_weak / insert / dot: recurrent.py:42-100), reached through
@@ -159,6 +171,13 @@ int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v
 int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
                     const void* g, const void* beta, const void* lam, float* states,
                     int32_t* counts, void* o, int32_t* status, void* stream);
+/*
+ * The same step in one launch: `arrivals` is a device int32 that belongs to this state, zero before the first step
+ * and zero again after every step (the CTA that arrives last advances `counts`).
+ */
+int lampa_hgdn_step_counted(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
+                            const void* g, const void* beta, const void* lam, float* states,
+                            int32_t* counts, int32_t* arrivals, void* o, int32_t* status, void* stream);
 /*
  * E2LSH projection and integer bucket ids.
  * Replaces: E2LSH.forward (models/model_utils/hash_utils.py:359-371; copies in

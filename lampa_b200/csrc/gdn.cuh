@@ -68,6 +68,7 @@ struct GdnArgs {
     float scale;
     int nseq;
     int fixed_T;        // tokens per sequence when there is no cu_seqlens (0 otherwise)
+    int fixed_stride;   // tokens from one sequence to the next in that case (fixed_T, or more when a prompt's tail is left to hgdn_tail)
     int fixed_cps;      // chunks per sequence in that case: positions follow by arithmetic, no plan loads
     int plan_inline;    // no cu_seqlens: the first preparation CTA writes the offset tables below (no separate launch)
     int nc_max, nb_max, nhigh_max;
@@ -92,7 +93,7 @@ __device__ __forceinline__ void stage_tick(const GdnArgs& a, int cta, int slot) 
 __device__ __forceinline__ void write_fixed_plan(const GdnArgs& a) {
     const int bps = (a.fixed_cps + BLOCK_CHUNKS - 1) / BLOCK_CHUNKS;
     for (int s = threadIdx.x; s <= a.nseq; s += blockDim.x) {
-        const_cast<int64_t*>(a.tok_off)[s] = (int64_t)s * a.fixed_T;
+        const_cast<int64_t*>(a.tok_off)[s] = (int64_t)s * a.fixed_stride;
         const_cast<int32_t*>(a.chunk_off)[s] = s * a.fixed_cps;
         const_cast<int32_t*>(a.block_off)[s] = s * bps;
     }
@@ -115,7 +116,7 @@ __device__ __forceinline__ bool locate_chunk(const GdnArgs& a, int c, ChunkLoc& 
         if (c >= a.nseq * a.fixed_cps) return false;
         loc.seq = c / a.fixed_cps;
         const int local = c - loc.seq * a.fixed_cps;
-        loc.t0 = (int64_t)loc.seq * a.fixed_T + (int64_t)local * CHUNK;
+        loc.t0 = (int64_t)loc.seq * a.fixed_stride + (int64_t)local * CHUNK;
         loc.len = min(CHUNK, a.fixed_T - local * CHUNK);
         return true;
     }
@@ -159,7 +160,14 @@ int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st);
 int launch_out_plain_umma(const GdnArgs& a, cudaStream_t st);  // K = V = 64
 int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st);   // K = V = 64, 2-byte q/k/v
 template <int KD, int VD> int launch_final_high(const GdnArgs& a, float* states, cudaStream_t st);
-template <int KD, int VD> int launch_final_low(const GdnArgs& a, float* states, int32_t* counts, cudaStream_t st);
+// The end of every sequence in fp32 (gdn_state.cu): token levels of the state, and the tokens behind the last whole chunk.
+struct TailArgs {
+    float* states; int32_t* counts;       // [N][H][K][V][L]; [N][L], or [L] when one_count (all sequences equally long)
+    int n0;                               // whole chunks of every sequence, or -1: from chunk_off, ragged chunks completed by null tokens
+    int tail;                             // tokens behind them (only with n0 >= 0)
+    int one_count;
+};
+template <int KD, int VD> int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st);
 
 // One decode step of the hierarchical rule on a Fenwick state (gdn_state.cu).
 struct StepArgs {
@@ -167,6 +175,8 @@ struct StepArgs {
     float* states; int32_t* counts; void* o;
     int qkv_dt, gb_dt, lam_dt;
     int B, H, L, use_l2norm;
+    int32_t* arrivals;                    // zero between steps: counts the CTAs that are done, or NULL (counts advanced by a second launch)
+    int poll_budget;
     int32_t* status;
 };
 template <int KD, int VD> int launch_hgdn_step(const StepArgs& s, cudaStream_t st);

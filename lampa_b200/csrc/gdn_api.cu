@@ -80,6 +80,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     a.H = d->H; a.L = hier ? d->L : 0; a.LC = l.LC;
     a.use_l2norm = d->use_l2norm; a.scale = d->scale;
     a.fixed_T = cu ? 0 : d->T;
+    a.fixed_stride = a.fixed_T;
     a.fixed_cps = cu ? 0 : (d->T + CHUNK - 1) / CHUNK;
     a.plan_inline = 0;
     a.total_tokens = (long long)d->B * d->T;
@@ -101,7 +102,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
 int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const void* v, const void* g,
         const void* beta, const void* lam, const float* h0, const int64_t* cu, void* o, float* ht,
         void* ws, size_t ws_bytes, int32_t* status, void* stream, const int64_t* out_perm = nullptr,
-        int64_t out_perm_rows = 0) {
+        int64_t out_perm_rows = 0, int fixed_stride = 0) {
     Layout l;
     int rc = make_layout(d, hier, l);
     if (rc != LAMPA_OK) return rc;
@@ -119,6 +120,7 @@ int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const 
     fill_args(d, hier, l, base, cu, status, a);
     a.q = q; a.k = k; a.v = v; a.g = g; a.beta = beta; a.lam = lam; a.h0 = h0; a.ht = ht; a.o = o;
     a.out_perm = out_perm; a.out_perm_rows = out_perm ? out_perm_rows : 0;
+    if (fixed_stride > 0) { a.fixed_stride = fixed_stride; a.total_tokens = (long long)d->B * fixed_stride; }
 
     PlanArgs p;
     p.cu = cu; p.nseq = l.nseq; p.B = d->B; p.T = d->T; p.L = d->L; p.hier = hier ? 1 : 0;
@@ -233,6 +235,25 @@ extern "C" int lampa_hgdn_fwd_scatter(const lampa_gdn_desc* d, const void* q, co
                out_perm, out_perm_rows);
 }
 
+namespace {
+
+template <int KD, int VD>
+int final_state(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
+    if (ta.n0 != 0) {                                   // the chunk levels first: the tail continues from them
+        const int rc = launch_final_high<KD, VD>(a, ta.states, st);
+        if (rc != LAMPA_OK) return rc;
+    }
+    return launch_hgdn_tail<KD, VD>(a, ta, st);
+}
+
+int final_state(const lampa_gdn_desc* d, const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
+    if (d->K == 64) return final_state<64, 64>(a, ta, st);
+    if (d->K == 32) return final_state<32, 32>(a, ta, st);
+    return final_state<16, 32>(a, ta, st);
+}
+
+}  // namespace
+
 extern "C" int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v, const void* g,
                                       const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
                                       float* states, int32_t* counts, int32_t* status, void* stream) {
@@ -244,25 +265,42 @@ extern "C" int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, co
     if (!k || !v || !g || !beta || !ws || !states || !counts) return LAMPA_ERR_ARG;
     if (d->nseq > 0 && !cu_seqlens) return LAMPA_ERR_ARG;
     if (ws_bytes < l.total || ((uintptr_t)ws & 1023)) return LAMPA_ERR_WORKSPACE;
-    cudaStream_t st = (cudaStream_t)stream;
     GdnArgs a;
     fill_args(d, true, l, (char*)ws, cu_seqlens, status, a);
     a.k = k; a.v = v; a.g = g; a.beta = beta;
-#define LAMPA_DISPATCH(KD, VD)                                           \
-    do {                                                                 \
-        rc = launch_final_low<KD, VD>(a, states, counts, st);            \
-        if (rc != LAMPA_OK) return rc;                                   \
-        return launch_final_high<KD, VD>(a, states, st);                 \
-    } while (0)
-    if (d->K == 64) LAMPA_DISPATCH(64, 64);
-    if (d->K == 32) LAMPA_DISPATCH(32, 32);
-    LAMPA_DISPATCH(16, 32);
-#undef LAMPA_DISPATCH
+    TailArgs ta;
+    ta.states = states; ta.counts = counts; ta.n0 = -1; ta.tail = 0; ta.one_count = 0;
+    return final_state(d, a, ta, (cudaStream_t)stream);
 }
 
-extern "C" int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
-                               const void* g, const void* beta, const void* lam, float* states,
-                               int32_t* counts, void* o, int32_t* status, void* stream) {
+extern "C" int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                                  const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
+                                  float* states, int32_t* counts, int32_t* status, void* stream) {
+    if (!d || d->nseq != 0) return LAMPA_ERR_ARG;
+    Layout l;
+    lampa_gdn_desc whole = *d;                           // the whole chunks of every row
+    whole.T = d->T - d->T % CHUNK;
+    int rc = make_layout(&whole, true, l);
+    if (rc != LAMPA_OK) return rc;
+    if ((int64_t)d->B * d->T == 0) return LAMPA_OK;
+    if (!q || !k || !v || !g || !beta || !lam || !o || !ws || !states || !counts) return LAMPA_ERR_ARG;
+    if (whole.T > 0 && d->L < ELL0) return LAMPA_ERR_LEVELS;
+    if (whole.T > 0) {
+        rc = run(&whole, true, q, k, v, g, beta, lam, nullptr, nullptr, o, nullptr, ws, ws_bytes, status, stream, nullptr, 0, d->T);
+        if (rc != LAMPA_OK) return rc;
+    }
+    GdnArgs a;
+    fill_args(&whole, true, l, (char*)ws, nullptr, status, a);
+    a.fixed_stride = d->T;
+    a.q = q; a.k = k; a.v = v; a.g = g; a.beta = beta; a.lam = lam; a.o = o;
+    TailArgs ta;
+    ta.states = states; ta.counts = counts; ta.n0 = whole.T / CHUNK; ta.tail = d->T - whole.T; ta.one_count = 1;
+    return final_state(d, a, ta, (cudaStream_t)stream);
+}
+
+static int hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                     const void* beta, const void* lam, float* states, int32_t* counts, int32_t* arrivals, void* o,
+                     int32_t* status, void* stream) {
     if (!d || d->B <= 0 || d->H <= 0 || d->T != 1) return LAMPA_ERR_ARG;
     if (!dims_supported(d->K, d->V)) return LAMPA_ERR_UNSUPPORTED;
     if (d->L < 1 || d->L > 40) return LAMPA_ERR_ARG;
@@ -274,9 +312,24 @@ extern "C" int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const voi
     s.states = states; s.counts = counts; s.o = o;
     s.qkv_dt = d->qkv_dtype; s.gb_dt = d->gb_dtype; s.lam_dt = d->lam_dtype;
     s.B = d->B; s.H = d->H; s.L = d->L; s.use_l2norm = d->use_l2norm;
+    s.arrivals = arrivals;
+    s.poll_budget = g_poll_budget;
     s.status = status;
     cudaStream_t st = (cudaStream_t)stream;
     if (d->K == 64) return launch_hgdn_step<64, 64>(s, st);
     if (d->K == 32) return launch_hgdn_step<32, 32>(s, st);
     return launch_hgdn_step<16, 32>(s, st);
+}
+
+extern "C" int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
+                               const void* g, const void* beta, const void* lam, float* states,
+                               int32_t* counts, void* o, int32_t* status, void* stream) {
+    return hgdn_step(d, q, k, v, g, beta, lam, states, counts, nullptr, o, status, stream);
+}
+
+extern "C" int lampa_hgdn_step_counted(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
+                                       const void* g, const void* beta, const void* lam, float* states,
+                                       int32_t* counts, int32_t* arrivals, void* o, int32_t* status, void* stream) {
+    if (!arrivals) return LAMPA_ERR_ARG;
+    return hgdn_step(d, q, k, v, g, beta, lam, states, counts, arrivals, o, status, stream);
 }

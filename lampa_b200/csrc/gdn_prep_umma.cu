@@ -596,7 +596,7 @@ static bool make_map(CUtensorMap* m, const void* base, int dt, uint64_t rows, ui
 
 int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     if (a.qkv_dt == LAMPA_F32) return LAMPA_ERR_UNSUPPORTED;
-    const uint64_t tokens = a.fixed_T > 0 ? (uint64_t)a.nseq * a.fixed_T : (uint64_t)a.total_tokens;
+    const uint64_t tokens = (uint64_t)a.total_tokens;
     // lambda by TMA when it is a 2-byte type, a token row is a multiple of 16 bytes and the tile is small
     const int lam_tile = hier ? CHUNK * a.H * a.L * 2 : 0;
     const int lam_tma = hier && a.lam_dt != LAMPA_F32 && (a.H * a.L) % 8 == 0 && a.H * a.L <= 256 && lam_tile <= LAM_TMA_MAX;

@@ -1,5 +1,5 @@
 // Fenwick-state side of the hierarchical gated-delta rule: the token levels of the final state
-// after a chunkwise forward, and the single-token decode step.
+// after a chunkwise forward, the ragged end of a prompt, and the single-token decode step.
 //
 // The state of one (batch row, head) is L matrices S_l [K][V] with counts[l] tokens each
 // (models/hattention/recurrent.py:9-131).  Inserting token t first cascades (level l is merged
@@ -18,121 +18,272 @@ __device__ __forceinline__ float round_like(float x, int dt) {
 }
 
 // -------------------------------------------------------------------------------------------------
-// Token levels 0..6 of the final state: the recurrence itself over the last chunk of each sequence,
-// from an empty state, as the reference's postprocess_prefill_hstate_ does
-// (models/hattention/kernel.py:377-466).  Inside one chunk the cascade is fixed: before token
-// t > 0, levels 0..tz(t) collapse into level tz(t) + 1 (tz = trailing zeros).  Thread (v, kq) owns
-// rows kq*K/4 .. of column v of all seven levels in registers.  Also writes counts [N][L].
-// A ragged last chunk is completed with null tokens (k = v = 0, beta = 0, g = 0).
+// End of a sequence, token by token in fp32: the token levels 0..6 after its last whole chunk (the
+// recurrence over that chunk from an empty state, as the reference's postprocess_prefill_hstate_
+// does, models/hattention/kernel.py:377-466), then, for a prefill, the T mod 64 tokens behind it with
+// all levels and their outputs (what the reference hands to its step function, kernel.py:470-560).
+// Inside one chunk the cascade is fixed: before token t > 0, levels 0..tz(t) collapse into level
+// tz(t) + 1 (tz = trailing zeros); before the first token behind n0 chunks, the token levels and the
+// trailing full chunk levels collapse into level 7 + tz(n0), after which the live chunk levels are
+// the set bits of n0 and do not change any more: they sit in HS register slots, in bit order.
+// Without a tail a ragged last chunk (cu_seqlens) is completed with null tokens (k = v = 0,
+// beta = 0, g = 0).  Also writes counts.
+//
+// State columns are independent, so a half-warp owns one: lane kl has rows kl, kl + 16, ... of every
+// level in registers, a level's k^T S is K / 16 FMAs and four shuffles, and the levels of a token
+// are independent chains that hide each other's latency.  What bounds it is that chain, ~0.2 us per
+// token; with one CTA per (sequence, head) and a launch per tail token (61 us for the token levels
+// and 27 us per tail token) a 3001-token prompt spent 1.7 of its 1.9 ms on the device here.
 // -------------------------------------------------------------------------------------------------
-template <int KD, int VD>
-__global__ void __launch_bounds__(VD * 4) hgdn_final_low_kernel(GdnArgs a, float* states, int32_t* counts) {
-    constexpr int KQ = KD / 4;
-    __shared__ float sK[CHUNK][KD + 1];
-    __shared__ float sV[CHUNK][VD];
-    __shared__ float sEg[CHUNK], sBeta[CHUNK];
+constexpr int TAIL_COLS = 8, TAIL_THREADS = 128;
+
+template <int N>
+__device__ __forceinline__ void half_warp_sum(float (&x)[N]) {
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], o);
+}
+
+template <int KD, int VD, int HS>
+__global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, TailArgs ta) {
+    constexpr int KI = KD / 16;
+    extern __shared__ __align__(16) float tail_smem[];
+    float* sK = tail_smem;                       // [64][KD], normalised
+    float* sQ = sK + CHUNK * KD;                 // [64][KD], normalised (tail only)
+    float* sV = sQ + CHUNK * KD;                 // [64][8]
+    float* sEg = sV + CHUNK * TAIL_COLS;         // [64]
+    float* sBeta = sEg + CHUNK;                  // [64]
+    float* sLam = sBeta + CHUNK;                 // [64][L] (tail only)
     const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
-    const int tid = threadIdx.x, nthr = VD * 4;
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
-    const int vv = tid >> 2, kq = tid & 3;
-    float* dst = states + ((size_t)seq * H + h) * KD * VD * L;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col = 2 * warp + (lane >> 4), kl = lane & 15;
+    const int v0 = blockIdx.z * TAIL_COLS, vv = v0 + col;
+    const int nch = ta.n0 >= 0 ? ta.n0 : a.chunk_off[seq + 1] - a.chunk_off[seq];
+    const int64_t tok0 = ta.n0 >= 0 ? (int64_t)seq * a.fixed_stride : a.tok_off[seq];
 
-    if (h == 0 && tid == 0) {
-        int64_t rem = (int64_t)nch * CHUNK - 1;
-        int32_t* cn = counts + (size_t)seq * L;
-        for (int l = L - 1; l >= 1; --l) {
-            const int64_t cap = l - 1 < 40 ? (int64_t)1 << (l - 1) : (int64_t)1 << 40;
-            if (nch > 0 && rem >= cap) { rem -= cap; cn[l] = (int32_t)cap; }
-            else cn[l] = 0;
-        }
-        cn[0] = nch > 0 ? 1 : 0;
-        if (nch > 0 && rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
-    }
-
-    float S[ELL0][KQ];
+    // rows [t0, t0 + len) of the inputs as the kernel uses them; rows up to 64 become null tokens
+    auto stage = [&](int64_t t0, int len, bool tail) {
+#pragma unroll 4
+        for (int r = warp; r < CHUNK; r += TAIL_THREADS / 32) {
+            float kx[(KD + 31) / 32], qx[(KD + 31) / 32];
+            float sk = 0.f, sq = 0.f;
 #pragma unroll
-    for (int l = 0; l < ELL0; ++l)
+            for (int j = 0; j < (KD + 31) / 32; ++j) {
+                const int c = lane + 32 * j;
+                const bool in = r < len && c < KD;
+                kx[j] = in ? load_as_float(a.k, ((size_t)(t0 + r) * H + h) * KD + c, a.qkv_dt) : 0.f;
+                qx[j] = in && tail ? load_as_float(a.q, ((size_t)(t0 + r) * H + h) * KD + c, a.qkv_dt) : 0.f;
+                sk += kx[j] * kx[j];
+                sq += qx[j] * qx[j];
+            }
 #pragma unroll
-        for (int i = 0; i < KQ; ++i) S[l][i] = 0.f;
-
-    if (nch > 0) {
-        const int64_t t0 = a.tok_off[seq] + (int64_t)(nch - 1) * CHUNK;
-        const int len = (int)min((int64_t)CHUNK, a.tok_off[seq + 1] - t0);
-        for (int idx = tid; idx < CHUNK * KD; idx += nthr) {
-            const int r = idx / KD, c = idx - r * KD;
-            sK[r][c] = r < len ? load_as_float(a.k, ((size_t)(t0 + r) * H + h) * KD + c, a.qkv_dt) : 0.f;
+            for (int o = 16; o > 0; o >>= 1) {
+                sk += __shfl_xor_sync(0xffffffffu, sk, o);
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            }
+            const float rk = rsqrtf(sk + 1e-6f), rq = rsqrtf(sq + 1e-6f);
+#pragma unroll
+            for (int j = 0; j < (KD + 31) / 32; ++j) {
+                const int c = lane + 32 * j;
+                if (c < KD) {
+                    sK[r * KD + c] = a.use_l2norm ? round_like(kx[j] * rk, a.qkv_dt) : kx[j];
+                    if (tail) sQ[r * KD + c] = a.use_l2norm ? qx[j] * rq : qx[j];
+                }
+            }
         }
-        for (int idx = tid; idx < CHUNK * VD; idx += nthr) {
-            const int r = idx / VD, c = idx - r * VD;
-            sV[r][c] = r < len ? load_as_float(a.v, ((size_t)(t0 + r) * H + h) * VD + c, a.qkv_dt) : 0.f;
+        for (int i = tid; i < CHUNK * TAIL_COLS; i += TAIL_THREADS) {
+            const int r = i / TAIL_COLS, c = i - r * TAIL_COLS;
+            sV[i] = r < len ? load_as_float(a.v, ((size_t)(t0 + r) * H + h) * VD + v0 + c, a.qkv_dt) : 0.f;
         }
         if (tid < CHUNK) {
-            const bool in = tid < len;
-            sEg[tid] = in ? __expf(load_as_float(a.g, (size_t)(t0 + tid) * H + h, a.gb_dt)) : 1.f;
-            sBeta[tid] = in ? load_as_float(a.beta, (size_t)(t0 + tid) * H + h, a.gb_dt) : 0.f;
+            sEg[tid] = tid < len ? __expf(load_as_float(a.g, (size_t)(t0 + tid) * H + h, a.gb_dt)) : 1.f;
+            sBeta[tid] = tid < len ? load_as_float(a.beta, (size_t)(t0 + tid) * H + h, a.gb_dt) : 0.f;
         }
+        if (tail)
+            for (int i = tid; i < len * L; i += TAIL_THREADS) {
+                const int r = i / L, l = i - r * L;
+                sLam[i] = load_as_float(a.lam, ((size_t)(t0 + r) * H + h) * L + l, a.lam_dt);
+            }
         __syncthreads();
-        if (a.use_l2norm) {
-            if (tid < CHUNK) {
-                float ss = 0.f;
-                for (int c = 0; c < KD; ++c) ss += sK[tid][c] * sK[tid][c];
-                const float rn = rsqrtf(ss + 1e-6f);
-                for (int c = 0; c < KD; ++c) sK[tid][c] = round_like(sK[tid][c] * rn, a.qkv_dt);
-            }
-            __syncthreads();
-        }
-        for (int t = 0; t < CHUNK; ++t) {
-            if (t > 0) {
-                const int tz = __ffs(t) - 1;
-#pragma unroll
-                for (int j = 0; j < ELL0 - 1; ++j)
-                    if (j <= tz) {
-#pragma unroll
-                        for (int i = 0; i < KQ; ++i) { S[j + 1][i] += S[j][i]; S[j][i] = 0.f; }
-                    }
-            }
-            const float eg = sEg[t], bt = sBeta[t];
-            float kr[KQ];
-#pragma unroll
-            for (int i = 0; i < KQ; ++i) kr[i] = sK[t][kq * KQ + i];
-#pragma unroll
-            for (int l = 1; l < ELL0; ++l) {
-                float dot = 0.f;
-#pragma unroll
-                for (int i = 0; i < KQ; ++i) dot += kr[i] * S[l][i];
-                dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-                dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-                const float c = bt * dot;
-#pragma unroll
-                for (int i = 0; i < KQ; ++i) S[l][i] = eg * (S[l][i] - kr[i] * c);
-            }
-            const float bv = bt * sV[t][vv];
-#pragma unroll
-            for (int i = 0; i < KQ; ++i) S[0][i] = kr[i] * bv;
-        }
-    }
+    };
+
+    float S[ELL0][KI];
 #pragma unroll
     for (int l = 0; l < ELL0; ++l)
-        if (l < L) {
 #pragma unroll
-            for (int i = 0; i < KQ; ++i) dst[((size_t)(kq * KQ + i) * VD + vv) * L + l] = S[l][i];
+        for (int i = 0; i < KI; ++i) S[l][i] = 0.f;
+    auto cascade_low = [&](int tz) {
+#pragma unroll
+        for (int j = 0; j < ELL0 - 1; ++j)
+            if (j <= tz) {
+#pragma unroll
+                for (int i = 0; i < KI; ++i) { S[j + 1][i] += S[j][i]; S[j][i] = 0.f; }
+            }
+    };
+
+    if (nch > 0) {
+        const int64_t t0 = tok0 + (int64_t)(nch - 1) * CHUNK;
+        stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, a.tok_off[seq + 1] - t0), false);
+        for (int t = 0; t < CHUNK; ++t) {
+            if (t > 0) cascade_low(__ffs(t) - 1);
+            const float eg = sEg[t], bt = sBeta[t];
+            float kr[KI], dot[ELL0 - 1];
+#pragma unroll
+            for (int i = 0; i < KI; ++i) kr[i] = sK[t * KD + kl + 16 * i];
+#pragma unroll
+            for (int l = 1; l < ELL0; ++l) {
+                dot[l - 1] = 0.f;
+#pragma unroll
+                for (int i = 0; i < KI; ++i) dot[l - 1] += kr[i] * S[l][i];
+            }
+            half_warp_sum(dot);
+#pragma unroll
+            for (int l = 1; l < ELL0; ++l) {
+                const float c = bt * dot[l - 1];
+#pragma unroll
+                for (int i = 0; i < KI; ++i) S[l][i] = eg * (S[l][i] - kr[i] * c);
+            }
+            const float bv = bt * sV[t * TAIL_COLS + col];
+#pragma unroll
+            for (int i = 0; i < KI; ++i) S[0][i] = kr[i] * bv;
         }
+    }
+
+    float* st = ta.states + ((((size_t)seq * H + h) * KD + kl) * VD + vv) * L;     // row kl; row kl + 16 i is i * row16 further
+    const size_t row16 = (size_t)16 * VD * L;
+    float X[HS][KI];
+    int lvl[HS];
+    int done = 0;                                // tail tokens taken in
+    if (ta.tail > 0) {
+        uint32_t rem = (uint32_t)nch;
+#pragma unroll
+        for (int s = 0; s < HS; ++s) {
+            lvl[s] = rem ? ELL0 + __ffs(rem) - 1 : -1;
+            rem &= rem - 1;
+        }
+        const bool room = nch == 0 || lvl[0] < L;          // the first cascade must not leave the last level
+        if (room) {
+#pragma unroll
+            for (int s = 0; s < HS; ++s)
+#pragma unroll
+                for (int i = 0; i < KI; ++i) X[s][i] = lvl[s] >= 0 && s > 0 ? st[i * row16 + lvl[s]] : 0.f;
+            if (nch > 0) {
+#pragma unroll
+                for (int i = 0; i < KI; ++i) {
+#pragma unroll
+                    for (int l = 0; l < ELL0; ++l) { X[0][i] += S[l][i]; S[l][i] = 0.f; }
+                    for (int l = ELL0; l < lvl[0]; ++l) X[0][i] += st[i * row16 + l];
+                }
+            }
+            __syncthreads();                               // the last chunk's rows have been read
+            const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
+            stage(t0, ta.tail, true);
+            for (int t = 0; t < ta.tail; ++t) {
+                if (t > 0) {
+                    const int tz = __ffs(t) - 1;
+                    if (tz + 1 >= L) break;
+                    cascade_low(tz);
+                }
+                const float eg = sEg[t], bt = sBeta[t];
+                float kr[KI], dot[ELL0 - 1 + HS], acc[KI];
+#pragma unroll
+                for (int i = 0; i < KI; ++i) { kr[i] = sK[t * KD + kl + 16 * i]; acc[i] = 0.f; }
+#pragma unroll
+                for (int l = 0; l < ELL0 - 1 + HS; ++l) {
+                    dot[l] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < KI; ++i) dot[l] += kr[i] * (l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i]);
+                }
+                half_warp_sum(dot);
+                const float* lam = sLam + t * L;
+#pragma unroll
+                for (int l = 1; l < ELL0; ++l) {
+                    const float c = bt * dot[l - 1], w = l < L ? lam[l] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < KI; ++i) { S[l][i] = eg * (S[l][i] - kr[i] * c); acc[i] += w * S[l][i]; }
+                }
+#pragma unroll
+                for (int s = 0; s < HS; ++s) {
+                    const float c = bt * dot[ELL0 - 1 + s], w = lvl[s] >= 0 ? lam[lvl[s]] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < KI; ++i) { X[s][i] = eg * (X[s][i] - kr[i] * c); acc[i] += w * X[s][i]; }
+                }
+                const float bv = bt * sV[t * TAIL_COLS + col];
+                float out[1] = {0.f};
+#pragma unroll
+                for (int i = 0; i < KI; ++i) {
+                    S[0][i] = kr[i] * bv;
+                    out[0] += sQ[t * KD + kl + 16 * i] * (acc[i] + lam[0] * S[0][i]);
+                }
+                half_warp_sum(out);
+                if (kl == 0) store_from_float(a.o, ((size_t)(t0 + t) * H + h) * VD + vv, out[0], a.qkv_dt);
+                done = t + 1;
+            }
+        }
+        if (done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
+    }
+
+#pragma unroll
+    for (int i = 0; i < KI; ++i) {
+#pragma unroll
+        for (int l = 0; l < ELL0; ++l)
+            if (l < L && (done > 0 || ta.tail == 0)) st[i * row16 + l] = S[l][i];
+        if (done > 0)
+            for (int l = ELL0; l < L; ++l) {
+                float x = 0.f;
+#pragma unroll
+                for (int s = 0; s < HS; ++s)
+                    if (lvl[s] == l) x = X[s][i];
+                st[i * row16 + l] = x;
+            }
+        else if (ta.tail > 0)                              // the tail was refused: the state after the whole chunks
+#pragma unroll
+            for (int l = 0; l < ELL0; ++l)
+                if (l < L) st[i * row16 + l] = S[l][i];
+    }
+    if (h == 0 && blockIdx.z == 0 && tid == 0 && (ta.n0 < 0 || !ta.one_count || seq == 0)) {
+        const int64_t n = (int64_t)nch * CHUNK + done;     // tokens held
+        int32_t* cn = ta.counts + (size_t)seq * L;
+        int64_t rem = n > 0 ? n - 1 : 0;
+        for (int l = L - 1; l >= 1; --l) {
+            const int64_t cap = l - 1 < 40 ? (int64_t)1 << (l - 1) : (int64_t)1 << 40;
+            const bool held = n > 0 && rem >= cap;
+            cn[l] = held ? (int32_t)cap : 0;
+            if (held) rem -= cap;
+        }
+        cn[0] = n > 0 ? 1 : 0;
+        if (rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
+    }
 }
 
 template <int KD, int VD>
-int launch_final_low(const GdnArgs& a, float* states, int32_t* counts, cudaStream_t st) {
-    ProfScope prof("hgdn_final_low", st);
-    hgdn_final_low_kernel<KD, VD><<<dim3(a.nseq, a.H), VD * 4, 0, st>>>(a, states, counts);
-    if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
-    return LAMPA_OK;
+int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
+    const int slots = ta.tail > 0 ? __builtin_popcount((unsigned)ta.n0) : 0;
+    const size_t smem = (size_t)(CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L : 0)) * 4;   // at most 47 KB
+    const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
+    ProfScope prof("hgdn_tail", st);
+    if (slots <= 4) hgdn_tail_kernel<KD, VD, 4><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
+    else if (slots <= 8) hgdn_tail_kernel<KD, VD, 8><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
+    else hgdn_tail_kernel<KD, VD, 24><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
 // -------------------------------------------------------------------------------------------------
 // Decode step (hattention_step -> step_state / step_output, models/hattention/kernel.py:570-633,
-// recurrent.py:134-166): cascade, transition, insert, then o = q^T sum_l lambda_l S_l.  One CTA per
-// (batch row, head), thread (v, kq) as above; the levels of one (k, v) element are contiguous in
-// memory, so the cascade is a prefix sum over a thread's own elements.  counts is shared by the
-// batch and is advanced by a second, single-thread kernel once every CTA has read it.
+// recurrent.py:134-166): cascade, transition, insert, then o = q^T sum_l lambda_l S_l.  The levels of
+// one (k, v) element are contiguous in memory, so the cascade is a prefix sum over a thread's own
+// elements.  counts is shared by the batch: the last CTA to arrive at `arrivals` advances it (every
+// CTA has read it by then), or a second, single-thread kernel when the caller has no such counter.
+//
+// What bounds it: streaming the state tensor once in and once out.  Half of the levels are live at a
+// time, but they alternate inside every 32-byte sector, so the whole tensor moves.  A thread that
+// walks the levels of its own element touches 4 bytes per sector and instruction: 148 us for 64 rows
+// x 8 heads of 64 x 64 x 17 levels (286 MB, 1.9 TB/s).  Here a CTA owns 8 state columns: their
+// K rows of 8 * L floats (544 bytes at L = 17) enter shared memory as bulk copies, are updated in
+// place and leave the same way.  Eight columns keep the slab at 35 KB, so that several CTAs per SM
+// overlap their copies with each other's arithmetic, and give even a single stream of 4 heads of 32
+// columns 16 CTAs.
 // -------------------------------------------------------------------------------------------------
 __device__ __forceinline__ int cascade_depth(const int32_t* counts, int L, int& merged, bool& overflow) {
     // levels 0 .. depth-1 move into level `depth`, which then holds `merged` tokens
@@ -155,20 +306,52 @@ __device__ __forceinline__ int cascade_depth(const int32_t* counts, int L, int& 
     return depth;
 }
 
+constexpr int STEP_COLS = 8, STEP_THREADS = 128, STEP_MAX_L = 40;
+
 template <int KD, int VD>
-__global__ void __launch_bounds__(VD * 4) hgdn_step_kernel(StepArgs s) {
-    constexpr int KQ = KD / 4;
-    __shared__ float sK[KD], sQ[KD], sLam[64];
-    const int b = blockIdx.x, h = blockIdx.y, H = s.H, L = s.L;
-    const int tid = threadIdx.x;
-    const int vv = tid >> 2, kq = tid & 3;
+__global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
+    constexpr int KI = KD / 16;                  // rows kq + 4 warp + 16 i of a thread; lane = (kq, column)
+    extern __shared__ __align__(16) float slab[];              // [KD][8][L]
+    __shared__ float sK[KD], sQ[KD], sLam[STEP_MAX_L], sQk;
+    __shared__ float part[2][4][STEP_MAX_L][STEP_COLS];        // k^T S and q^T S of every level: one partial per warp
+    __shared__ int32_t sCnt[STEP_MAX_L];
+    __shared__ __align__(8) uint64_t bar;
+    const int b = blockIdx.x / (VD / STEP_COLS), v0 = (blockIdx.x - b * (VD / STEP_COLS)) * STEP_COLS;
+    const int h = blockIdx.y, H = s.H, L = s.L;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col = lane & 7, kq = (lane >> 3) + 4 * warp;
     const size_t bh = (size_t)b * H + h;
-    if (tid < 32) {
+    float* gsrc = s.states + (bh * KD * VD + v0) * L;           // row k: KD rows of 8 L floats, VD L floats apart
+    const uint32_t row_bytes = STEP_COLS * L * 4;               // a multiple of 32
+    const bool bulk = ((uintptr_t)s.states & 15) == 0;
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        if (bulk) mbar_expect_tx(&bar, KD * row_bytes);
+    }
+    __syncthreads();
+    if (bulk) {
+        if (tid < KD) bulk_g2s(slab + (size_t)tid * STEP_COLS * L, gsrc + (size_t)tid * VD * L, row_bytes, &bar);
+    } else {
+        for (int i = tid; i < KD * STEP_COLS * L; i += STEP_THREADS) {
+            const int r = i / (STEP_COLS * L);
+            slab[i] = gsrc[(size_t)r * VD * L + (i - r * STEP_COLS * L)];
+        }
+    }
+    if (tid >= STEP_THREADS - L) {
+        const int l = tid - (STEP_THREADS - L);
+        sCnt[l] = s.counts[l];
+        sLam[l] = load_as_float(s.lam, bh * L + l, s.lam_dt);
+    }
+    const float eg = __expf(load_as_float(s.g, bh, s.gb_dt));
+    const float bt = load_as_float(s.beta, bh, s.gb_dt);
+    const float vt = load_as_float(s.v, bh * VD + v0 + col, s.qkv_dt);
+    if (warp == 0) {
         float kx[(KD + 31) / 32], qx[(KD + 31) / 32];
-        float sk = 0.f, sq = 0.f;
+        float sk = 0.f, sq = 0.f, qk = 0.f;
 #pragma unroll
         for (int j = 0; j < (KD + 31) / 32; ++j) {
-            const int c = tid + 32 * j;
+            const int c = lane + 32 * j;
             kx[j] = c < KD ? load_as_float(s.k, bh * KD + c, s.qkv_dt) : 0.f;
             qx[j] = c < KD ? load_as_float(s.q, bh * KD + c, s.qkv_dt) : 0.f;
             sk += kx[j] * kx[j];
@@ -179,88 +362,105 @@ __global__ void __launch_bounds__(VD * 4) hgdn_step_kernel(StepArgs s) {
             sk += __shfl_xor_sync(0xffffffffu, sk, o);
             sq += __shfl_xor_sync(0xffffffffu, sq, o);
         }
-        const float rk = s.use_l2norm ? rsqrtf(sk + 1e-6f) : 1.f;
-        const float rq = s.use_l2norm ? rsqrtf(sq + 1e-6f) : 1.f;
+        const float rk = rsqrtf(sk + 1e-6f), rq = rsqrtf(sq + 1e-6f);
 #pragma unroll
         for (int j = 0; j < (KD + 31) / 32; ++j) {
-            const int c = tid + 32 * j;
-            if (c < KD) {
-                sK[c] = s.use_l2norm ? round_like(kx[j] * rk, s.qkv_dt) : kx[j];
-                sQ[c] = qx[j] * rq;
-            }
+            const int c = lane + 32 * j;
+            if (s.use_l2norm) { kx[j] = round_like(kx[j] * rk, s.qkv_dt); qx[j] *= rq; }
+            if (c < KD) { sK[c] = kx[j]; sQ[c] = qx[j]; }
+            qk += kx[j] * qx[j];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) qk += __shfl_xor_sync(0xffffffffu, qk, o);
+        if (lane == 0) sQk = qk;
     }
-    if (tid < L && tid < 64) sLam[tid] = load_as_float(s.lam, bh * L + tid, s.lam_dt);
     __syncthreads();
-
     int merged;
     bool overflow;
-    const int depth = cascade_depth(s.counts, L, merged, overflow);
-    if (overflow) {
-        if (tid == 0 && b == 0 && h == 0) set_status(s.status, LAMPA_ERR_LEVELS, 31, depth);
+    const int depth = cascade_depth(sCnt, L, merged, overflow);
+    bool dead = false;
+    if (bulk) mbar_wait(&bar, 0u, dead, s.status, 32, s.poll_budget);
+    if (overflow || __syncthreads_or(dead)) {     // nothing changes; the copies land before the CTA gives its memory back
+        if (overflow && tid == 0 && bh == 0 && v0 == 0) set_status(s.status, LAMPA_ERR_LEVELS, 31, depth);
+        if (bulk) mbar_drain(&bar, 0u);
+        __syncthreads();
+        if (tid == 0 && s.arrivals) atomicInc(reinterpret_cast<unsigned*>(s.arrivals), gridDim.x * gridDim.y - 1);
         return;
     }
-    const float eg = __expf(load_as_float(s.g, bh, s.gb_dt));
-    const float bt = load_as_float(s.beta, bh, s.gb_dt);
-    const float vt = load_as_float(s.v, bh * VD + vv, s.qkv_dt);
+    const auto live = [&](int l) { return l == depth ? merged > 0 : (l > depth && sCnt[l] != 0); };
 
-    float kr[KQ], qr[KQ], acc[KQ];
-    float* P[KQ];
+    float kr[KI], qr[KI];
+    float* P[KI];
 #pragma unroll
-    for (int i = 0; i < KQ; ++i) {
-        kr[i] = sK[kq * KQ + i];
-        qr[i] = sQ[kq * KQ + i];
-        P[i] = s.states + ((bh * KD + kq * KQ + i) * VD + vv) * (size_t)L;
-        acc[i] = 0.f;
+    for (int i = 0; i < KI; ++i) {
+        kr[i] = sK[kq + 16 * i];
+        qr[i] = sQ[kq + 16 * i];
+        P[i] = slab + ((size_t)(kq + 16 * i) * STEP_COLS + col) * L;
     }
-    for (int j = 0; j <= depth; ++j)
-        if (j == depth ? merged > 0 : true) {
+    if (depth > 0) {                               // levels 0 .. depth - 1 join level `depth`
 #pragma unroll
-            for (int i = 0; i < KQ; ++i) acc[i] += P[i][j];
+        for (int i = 0; i < KI; ++i) {
+            float x = 0.f;
+            for (int j = 0; j <= depth; ++j) { x += P[i][j]; P[i][j] = 0.f; }
+            P[i][depth] = x;
         }
-    float out = 0.f;
-    for (int l = L - 1; l >= 1; --l) {
-        const int cnt = l < depth ? 0 : (l == depth ? merged : s.counts[l]);
-        if (cnt == 0) {
-            if (l < depth) {
+    }
+    for (int l = 1; l < L; ++l) {
+        if (!live(l)) continue;
+        float dk = 0.f, dq = 0.f;
 #pragma unroll
-                for (int i = 0; i < KQ; ++i) P[i][l] = 0.f;
+        for (int i = 0; i < KI; ++i) { const float x = P[i][l]; dk += kr[i] * x; dq += qr[i] * x; }
+        dk += __shfl_xor_sync(0xffffffffu, dk, 8);
+        dq += __shfl_xor_sync(0xffffffffu, dq, 8);
+        dk += __shfl_xor_sync(0xffffffffu, dk, 16);
+        dq += __shfl_xor_sync(0xffffffffu, dq, 16);
+        if (lane < STEP_COLS) { part[0][warp][l][col] = dk; part[1][warp][l][col] = dq; }
+    }
+    __syncthreads();
+    const float bv = bt * vt;
+    for (int l = 1; l < L; ++l) {
+        if (!live(l)) continue;
+        const float c = bt * ((part[0][0][l][col] + part[0][1][l][col]) + (part[0][2][l][col] + part[0][3][l][col]));
+#pragma unroll
+        for (int i = 0; i < KI; ++i) P[i][l] = eg * (P[i][l] - kr[i] * c);
+    }
+#pragma unroll
+    for (int i = 0; i < KI; ++i) P[i][0] = kr[i] * bv;
+    if (warp == 0) {                               // o = sum_l lambda_l e^g (q^T S_l - (q.k) c_l) + lambda_0 (q.k) beta v
+        float out = 0.f;
+        for (int l = 1 + (lane >> 3); l < L; l += 4)
+            if (live(l)) {
+                const float c = bt * ((part[0][0][l][col] + part[0][1][l][col]) + (part[0][2][l][col] + part[0][3][l][col]));
+                const float q = (part[1][0][l][col] + part[1][1][l][col]) + (part[1][2][l][col] + part[1][3][l][col]);
+                out += sLam[l] * (eg * (q - sQk * c));
             }
-            continue;
-        }
-        float val[KQ];
-        float dot = 0.f;
-#pragma unroll
-        for (int i = 0; i < KQ; ++i) {
-            val[i] = l == depth ? acc[i] : P[i][l];
-            dot += kr[i] * val[i];
-        }
-        dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-        dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-        const float c = bt * dot;
-        float qs = 0.f;
-#pragma unroll
-        for (int i = 0; i < KQ; ++i) {
-            const float nv = eg * (val[i] - kr[i] * c);
-            P[i][l] = nv;
-            qs += qr[i] * nv;
-        }
-        out += sLam[l] * qs;
+        out += __shfl_xor_sync(0xffffffffu, out, 8);
+        out += __shfl_xor_sync(0xffffffffu, out, 16);
+        if (lane < STEP_COLS) store_from_float(s.o, bh * VD + v0 + col, out + sLam[0] * (sQk * bv), s.qkv_dt);
     }
-    {
-        const float bv = bt * vt;
-        float qs = 0.f;
-#pragma unroll
-        for (int i = 0; i < KQ; ++i) {
-            const float nv = kr[i] * bv;
-            P[i][0] = nv;
-            qs += qr[i] * nv;
+    if (bulk) {
+        fence_async_shared();
+        __syncthreads();
+        if (tid < KD) {
+            bulk_s2g(gsrc + (size_t)tid * VD * L, slab + (size_t)tid * STEP_COLS * L, row_bytes);
+            bulk_commit();
         }
-        out += sLam[0] * qs;
+    } else {
+        __syncthreads();
+        for (int i = tid; i < KD * STEP_COLS * L; i += STEP_THREADS) {
+            const int r = i / (STEP_COLS * L);
+            gsrc[(size_t)r * VD * L + (i - r * STEP_COLS * L)] = slab[i];
+        }
     }
-    out += __shfl_xor_sync(0xffffffffu, out, 1);
-    out += __shfl_xor_sync(0xffffffffu, out, 2);
-    if (kq == 0) store_from_float(s.o, bh * VD + vv, out, s.qkv_dt);
+    if (tid == 0 && s.arrivals) {
+        const unsigned last = gridDim.x * gridDim.y - 1;
+        if (atomicInc(reinterpret_cast<unsigned*>(s.arrivals), last) == last) {    // wraps to zero for the next step
+            for (int l = 0; l < depth; ++l) s.counts[l] = 0;
+            if (depth > 0) s.counts[depth] = merged;
+            s.counts[0] = 1;
+        }
+    }
+    if (bulk && tid < KD) bulk_wait_read();
 }
 
 __global__ void hgdn_step_counts_kernel(int32_t* counts, int L) {
@@ -276,18 +476,21 @@ __global__ void hgdn_step_counts_kernel(int32_t* counts, int L) {
 
 template <int KD, int VD>
 int launch_hgdn_step(const StepArgs& s, cudaStream_t st) {
+    const int smem = KD * STEP_COLS * s.L * 4;     // at most 80 KB, beside 11 KB of static shared memory
+    if (smem > 36 * 1024 && cudaFuncSetAttribute(hgdn_step_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return LAMPA_ERR_CUDA;
     {
         ProfScope prof("hgdn_step", st);
-        hgdn_step_kernel<KD, VD><<<dim3(s.B, s.H), VD * 4, 0, st>>>(s);
+        hgdn_step_kernel<KD, VD><<<dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS, smem, st>>>(s);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
+    if (s.arrivals) return LAMPA_OK;
     hgdn_step_counts_kernel<<<1, 32, 0, st>>>(s.counts, s.L);
-    if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
-    return LAMPA_OK;
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
 #define LAMPA_INST(KD, VD)                                                                      \
-    template int launch_final_low<KD, VD>(const GdnArgs&, float*, int32_t*, cudaStream_t);      \
+    template int launch_hgdn_tail<KD, VD>(const GdnArgs&, const TailArgs&, cudaStream_t);       \
     template int launch_hgdn_step<KD, VD>(const StepArgs&, cudaStream_t);
 LAMPA_INST(64, 64)
 LAMPA_INST(32, 32)

@@ -216,12 +216,20 @@ class HState:
         self.states = torch.zeros(self.shape, dtype=dtype, device=device)
         self.counts = torch.zeros(self.max_num_levels, dtype=torch.int32, device=device)
 
+    def arrivals(self) -> torch.Tensor:
+        """The step kernel's arrival counter: one int32 of this state, zero between steps."""
+        a = getattr(self, "_arrivals", None)
+        if a is None or a.device != self.states.device:
+            a = self._arrivals = torch.zeros(1, dtype=torch.int32, device=self.states.device)
+        return a
+
     def reset_states(self) -> None:
         self.states.zero_()
 
     def to(self, dtype: Optional[torch.dtype] = None, device=None) -> "HState":
         new = HState.__new__(HState)
         new.__dict__.update(self.__dict__)
+        new._arrivals = None
         new.dtype = self.dtype if dtype is None else dtype
         new.device = self.device if device is None else torch.device(device)
         new.states = self.states.to(dtype=new.dtype, device=new.device)
@@ -289,10 +297,10 @@ def _hgdn_step(hstate: HState, q, k, v, g, beta, lam, use_l2norm: bool = True) -
                      use_l2norm=int(bool(use_l2norm)), scale=1.0)
     o = torch.empty(B, H, V, dtype=q.dtype, device=dev)
     st = L.status_word(dev)
-    rc = L.lib().lampa_hgdn_step(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                                 L.ptr(lam), L.ptr(hstate.states), L.ptr(hstate.counts), L.ptr(o),
-                                 L.ptr(st), L.stream_ptr(dev))
-    L.check(rc, "lampa_hgdn_step")
+    rc = L.lib().lampa_hgdn_step_counted(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
+                                         L.ptr(lam), L.ptr(hstate.states), L.ptr(hstate.counts),
+                                         L.ptr(hstate.arrivals()), L.ptr(o), L.ptr(st), L.stream_ptr(dev))
+    L.check(rc, "lampa_hgdn_step_counted")
     if L.debug_checks():
         L.check_status(dev)
     return o
@@ -301,22 +309,34 @@ def _hgdn_step(hstate: HState, q, k, v, g, beta, lam, use_l2norm: bool = True) -
 @torch.no_grad()
 def _hgdn_prefill(q, k, v, g, beta, lam, use_l2norm: bool = True):
     """(o, HState) after all T tokens: whole chunks through the chunkwise kernels, the remaining
-    T mod 64 tokens through the step kernel — the split hattention_prefill makes
-    (models/hattention/kernel.py:470-560)."""
+    T mod 64 tokens through the token recurrence — the split hattention_prefill makes
+    (models/hattention/kernel.py:470-560), in one call."""
+    dev, q, k, v, g, beta, lam, _ = _prep_inputs(q, k, v, g, beta, lam, None)
     B, T, H, K = q.shape
     V, Lv = v.shape[-1], lam.shape[-1]
-    dev = L.require_cuda(q, k, v, g, beta, lam)
     T0 = T - T % CHUNK
-    hstate = HState(2, HType.WEAK, HStruct.GDELTA, (B, H, K, V, Lv), torch.float32, dev)
+    if T0 > 0 and Lv < num_levels_required(T0):
+        raise ValueError(f"l has {Lv} levels, a sequence of {T0} tokens needs {num_levels_required(T0)}")
+    if K > 256:
+        raise NotImplementedError("current kernel does not support head dimension larger than 256.")
+    hstate = HState(2, HType.WEAK, HStruct.GDELTA, (B, H, K, V, Lv), torch.float32, dev, empty=True)
     o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
-    if T0 > 0:
-        o0, states, counts = _hgdn(q[:, :T0], k[:, :T0], v[:, :T0], g[:, :T0], beta[:, :T0], lam[:, :T0],
-                                   None, use_l2norm, want_state=True)
-        o[:, :T0] = o0
-        hstate.states = states
-        hstate.counts = counts[0].contiguous()
-    for t in range(T0, T):
-        o[:, t] = _hgdn_step(hstate, q[:, t], k[:, t], v[:, t], g[:, t], beta[:, t], lam[:, t], use_l2norm)
+    if T == 0:
+        hstate.states = torch.zeros(hstate.shape, dtype=torch.float32, device=dev)
+        hstate.counts = torch.zeros(Lv, dtype=torch.int32, device=dev)
+        return o, hstate
+    hstate.states = torch.empty(hstate.shape, dtype=torch.float32, device=dev)
+    hstate.counts = torch.empty(Lv, dtype=torch.int32, device=dev)
+    desc = _desc(q, v, g, lam, None, use_l2norm, 1.0)
+    desc.T = T0
+    ws = _workspace(desc, dev)
+    desc.T = T
+    rc = L.lib().lampa_hgdn_prefill(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta), L.ptr(lam),
+                                    L.ptr(o), L.ptr(ws), ws.numel(), L.ptr(hstate.states), L.ptr(hstate.counts),
+                                    L.ptr(L.status_word(dev)), L.stream_ptr(dev))
+    L.check(rc, "lampa_hgdn_prefill")
+    if L.debug_checks():
+        L.check_status(dev)
     return o, hstate
 
 
