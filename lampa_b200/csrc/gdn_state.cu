@@ -281,9 +281,11 @@ int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
 // walks the levels of its own element touches 4 bytes per sector and instruction: 148 us for 64 rows
 // x 8 heads of 64 x 64 x 17 levels (286 MB, 1.9 TB/s).  Here a CTA owns 8 state columns: their
 // K rows of 8 * L floats (544 bytes at L = 17) enter shared memory as bulk copies, are updated in
-// place and leave the same way.  Eight columns keep the slab at 35 KB, so that several CTAs per SM
-// overlap their copies with each other's arithmetic, and give even a single stream of 4 heads of 32
-// columns 16 CTAs.
+// place and leave the same way: 65 us (4.4 TB/s).  Eight columns keep the slab at 35 KB, so that
+// five CTAs per SM overlap their copies with each other's arithmetic, and give even a single stream
+// of 4 heads of 32 columns 16 CTAs.  Two rows per thread, not four: the arithmetic is a chain of
+// shared-memory round trips, and half the warps took 76 us.  16-byte cp.async and vector stores
+// instead of the bulk copies: 97 us.
 // -------------------------------------------------------------------------------------------------
 __device__ __forceinline__ int cascade_depth(const int32_t* counts, int L, int& merged, bool& overflow) {
     // levels 0 .. depth-1 move into level `depth`, which then holds `merged` tokens
@@ -306,14 +308,19 @@ __device__ __forceinline__ int cascade_depth(const int32_t* counts, int L, int& 
     return depth;
 }
 
-constexpr int STEP_COLS = 8, STEP_THREADS = 128, STEP_MAX_L = 40;
+constexpr int STEP_COLS = 8, STEP_MAX_L = 40, STEP_KI = 2;      // rows of a thread
+template <int KD> constexpr int STEP_THREADS = KD * STEP_COLS / STEP_KI;
+template <int KD> __host__ __device__ constexpr int step_smem(int L) {      // slab, partial sums, c
+    return (KD * STEP_COLS + 2 * (STEP_THREADS<KD> / 32) * STEP_COLS + STEP_COLS) * L * 4;
+}
 
 template <int KD, int VD>
-__global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
-    constexpr int KI = KD / 16;                  // rows kq + 4 warp + 16 i of a thread; lane = (kq, column)
+__global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s) {
+    constexpr int NT = STEP_THREADS<KD>, NW = NT / 32, KI = STEP_KI;        // lane = (4 rows, 8 columns)
     extern __shared__ __align__(16) float slab[];              // [KD][8][L]
+    float* part = slab + KD * STEP_COLS * s.L;                 // [2][warps][L][8]: k^T S and q^T S of every level
+    float* sC = part + 2 * NW * STEP_COLS * s.L;               // [L][8]: beta k^T S
     __shared__ float sK[KD], sQ[KD], sLam[STEP_MAX_L], sQk;
-    __shared__ float part[2][4][STEP_MAX_L][STEP_COLS];        // k^T S and q^T S of every level: one partial per warp
     __shared__ int32_t sCnt[STEP_MAX_L];
     __shared__ __align__(8) uint64_t bar;
     const int b = blockIdx.x / (VD / STEP_COLS), v0 = (blockIdx.x - b * (VD / STEP_COLS)) * STEP_COLS;
@@ -333,13 +340,13 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
     if (bulk) {
         if (tid < KD) bulk_g2s(slab + (size_t)tid * STEP_COLS * L, gsrc + (size_t)tid * VD * L, row_bytes, &bar);
     } else {
-        for (int i = tid; i < KD * STEP_COLS * L; i += STEP_THREADS) {
+        for (int i = tid; i < KD * STEP_COLS * L; i += NT) {
             const int r = i / (STEP_COLS * L);
             slab[i] = gsrc[(size_t)r * VD * L + (i - r * STEP_COLS * L)];
         }
     }
-    if (tid >= STEP_THREADS - L) {
-        const int l = tid - (STEP_THREADS - L);
+    if (tid >= NT - L) {
+        const int l = tid - (NT - L);
         sCnt[l] = s.counts[l];
         sLam[l] = load_as_float(s.lam, bh * L + l, s.lam_dt);
     }
@@ -387,15 +394,17 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
         if (tid == 0 && s.arrivals) atomicInc(reinterpret_cast<unsigned*>(s.arrivals), gridDim.x * gridDim.y - 1);
         return;
     }
-    const auto live = [&](int l) { return l == depth ? merged > 0 : (l > depth && sCnt[l] != 0); };
+    uint64_t live = 0;                             // levels >= 1 that hold tokens after the cascade
+    for (int l = max(depth, 1); l < L; ++l) live |= (uint64_t)(l == depth ? merged > 0 : sCnt[l] != 0) << l;
 
     float kr[KI], qr[KI];
     float* P[KI];
 #pragma unroll
     for (int i = 0; i < KI; ++i) {
-        kr[i] = sK[kq + 16 * i];
-        qr[i] = sQ[kq + 16 * i];
-        P[i] = slab + ((size_t)(kq + 16 * i) * STEP_COLS + col) * L;
+        const int r = kq + 4 * NW * i;
+        kr[i] = sK[r];
+        qr[i] = sQ[r];
+        P[i] = slab + ((size_t)r * STEP_COLS + col) * L;
     }
     if (depth > 0) {                               // levels 0 .. depth - 1 join level `depth`
 #pragma unroll
@@ -405,8 +414,8 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
             P[i][depth] = x;
         }
     }
-    for (int l = 1; l < L; ++l) {
-        if (!live(l)) continue;
+    for (uint64_t m = live; m; m &= m - 1) {
+        const int l = __ffsll((long long)m) - 1;
         float dk = 0.f, dq = 0.f;
 #pragma unroll
         for (int i = 0; i < KI; ++i) { const float x = P[i][l]; dk += kr[i] * x; dq += qr[i] * x; }
@@ -414,13 +423,22 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
         dq += __shfl_xor_sync(0xffffffffu, dq, 8);
         dk += __shfl_xor_sync(0xffffffffu, dk, 16);
         dq += __shfl_xor_sync(0xffffffffu, dq, 16);
-        if (lane < STEP_COLS) { part[0][warp][l][col] = dk; part[1][warp][l][col] = dq; }
+        if (lane < 2 * STEP_COLS) part[(((lane >> 3) * NW + warp) * L + l) * STEP_COLS + col] = lane < STEP_COLS ? dk : dq;
     }
     __syncthreads();
+    for (int i = tid; i < L * STEP_COLS; i += NT)
+        if ((live >> (i >> 3)) & 1) {
+            float c = 0.f, q = 0.f;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) { c += part[w * L * STEP_COLS + i]; q += part[(NW + w) * L * STEP_COLS + i]; }
+            sC[i] = bt * c;
+            part[i] = q;                           // read by this thread only so far
+        }
+    __syncthreads();
     const float bv = bt * vt;
-    for (int l = 1; l < L; ++l) {
-        if (!live(l)) continue;
-        const float c = bt * ((part[0][0][l][col] + part[0][1][l][col]) + (part[0][2][l][col] + part[0][3][l][col]));
+    for (uint64_t m = live; m; m &= m - 1) {
+        const int l = __ffsll((long long)m) - 1;
+        const float c = sC[l * STEP_COLS + col];
 #pragma unroll
         for (int i = 0; i < KI; ++i) P[i][l] = eg * (P[i][l] - kr[i] * c);
     }
@@ -429,11 +447,7 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
     if (warp == 0) {                               // o = sum_l lambda_l e^g (q^T S_l - (q.k) c_l) + lambda_0 (q.k) beta v
         float out = 0.f;
         for (int l = 1 + (lane >> 3); l < L; l += 4)
-            if (live(l)) {
-                const float c = bt * ((part[0][0][l][col] + part[0][1][l][col]) + (part[0][2][l][col] + part[0][3][l][col]));
-                const float q = (part[1][0][l][col] + part[1][1][l][col]) + (part[1][2][l][col] + part[1][3][l][col]);
-                out += sLam[l] * (eg * (q - sQk * c));
-            }
+            if ((live >> l) & 1) out += sLam[l] * (eg * (part[l * STEP_COLS + col] - sQk * sC[l * STEP_COLS + col]));
         out += __shfl_xor_sync(0xffffffffu, out, 8);
         out += __shfl_xor_sync(0xffffffffu, out, 16);
         if (lane < STEP_COLS) store_from_float(s.o, bh * VD + v0 + col, out + sLam[0] * (sQk * bv), s.qkv_dt);
@@ -447,7 +461,7 @@ __global__ void __launch_bounds__(STEP_THREADS) hgdn_step_kernel(StepArgs s) {
         }
     } else {
         __syncthreads();
-        for (int i = tid; i < KD * STEP_COLS * L; i += STEP_THREADS) {
+        for (int i = tid; i < KD * STEP_COLS * L; i += NT) {
             const int r = i / (STEP_COLS * L);
             gsrc[(size_t)r * VD * L + (i - r * STEP_COLS * L)] = slab[i];
         }
@@ -476,12 +490,12 @@ __global__ void hgdn_step_counts_kernel(int32_t* counts, int L) {
 
 template <int KD, int VD>
 int launch_hgdn_step(const StepArgs& s, cudaStream_t st) {
-    const int smem = KD * STEP_COLS * s.L * 4;     // at most 80 KB, beside 11 KB of static shared memory
-    if (smem > 36 * 1024 && cudaFuncSetAttribute(hgdn_step_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    const int smem = step_smem<KD>(s.L);           // at most 103 KB
+    if (smem > 44 * 1024 && cudaFuncSetAttribute(hgdn_step_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
     {
         ProfScope prof("hgdn_step", st);
-        hgdn_step_kernel<KD, VD><<<dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS, smem, st>>>(s);
+        hgdn_step_kernel<KD, VD><<<dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS<KD>, smem, st>>>(s);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     if (s.arrivals) return LAMPA_OK;

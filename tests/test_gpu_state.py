@@ -150,6 +150,52 @@ def test_prefill_with_ragged_tail_and_decode(lb, T, K, V):
     np.testing.assert_array_equal(to_np(hs.counts), cref1)
 
 
+@pytest.mark.parametrize("T,H,K,V,extra", [
+    (63, 1, 64, 64, 0),               # no whole chunk
+    (65, 3, 32, 32, 2),               # one tail token behind one chunk
+    (64 * 5 + 63, 1, 64, 64, 1),      # longest tail
+    (64 * 31 + 17, 1, 64, 64, 0),     # five chunk levels live
+    (64 * 511 + 5, 1, 16, 32, 0),     # nine
+])
+def test_prefill_tail_edges(lb, T, H, K, V, extra):
+    """Two rows of ragged prompts: outputs and states of the fp32 tail at the edges of its slots and lengths."""
+    from lampa_b200 import synth
+    Lv = lb.num_levels_required(T) + extra
+    rows = [synth.gdn_inputs(51 + i, T, H, K, V, L=Lv, g_shift=-5.0) for i in range(2)]
+    d = {k: torch.cat([r[k] for r in rows], 0).cuda() for k in rows[0]}
+    o, hs = lb.chunk_h_gated_delta_rule(d["q"], d["k"], d["v"], d["g"], d["lam"], d["beta"],
+                                        output_final_state=True, use_qk_l2norm_in_kernel=True)
+    for i, inp in enumerate(rows):
+        oref, sref, cref = _ref(inp)
+        assert_close_bf16(to_np(o[i]), oref, f"o row {i}")
+        _close_states(to_np(hs.states[i]), sref, f"states row {i}")
+        np.testing.assert_array_equal(to_np(hs.counts), cref)
+
+
+@pytest.mark.parametrize("K,V,Lv,shift", [(64, 64, 16, 0), (64, 64, 40, 0), (32, 32, 17, 1), (16, 32, 13, 0)])
+def test_decode_level_counts_and_unaligned_states(lb, K, V, Lv, shift):
+    """Decode steps for level counts of either parity, the largest one, and a state that is not 16-byte aligned."""
+    from lampa_b200 import synth
+    T, H, B = 70, 2, 3
+    rows = [synth.gdn_inputs(61 + i, T, H, K, V, L=Lv, g_shift=-3.0) for i in range(B)]
+    d = {k: torch.cat([r[k] for r in rows], 0).cuda() for k in rows[0]}
+    hs = lb.HState(2, lb.HType.WEAK, lb.HStruct.GDELTA, (B, H, K, V, Lv), torch.float32, "cuda:0")
+    n = hs.states.numel()
+    hs.states = torch.zeros(n + shift, device="cuda:0")[shift:].view(B, H, K, V, Lv)
+    outs = []
+    for t in range(T):
+        x = {k: v[:, t:t + 1] for k, v in d.items()}
+        o, hs = lb.chunk_h_gated_delta_rule(x["q"], x["k"], x["v"], x["g"], x["lam"], x["beta"], initial_state=hs,
+                                            output_final_state=True, use_qk_l2norm_in_kernel=True)
+        outs.append(o)
+    o = to_np(torch.cat(outs, 1))
+    for i, inp in enumerate(rows):
+        oref, sref, cref = _ref(inp)
+        assert_close_bf16(o[i], oref, f"o row {i}")
+        _close_states(to_np(hs.states[i]), sref, f"states row {i}")
+        np.testing.assert_array_equal(to_np(hs.counts), cref)
+
+
 def test_decode_from_empty_state_crosses_chunk_boundaries(lb):
     """130 decode steps from an empty state: every cascade depth up to level 8 occurs."""
     from lampa_b200 import synth
