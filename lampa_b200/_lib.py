@@ -96,6 +96,26 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+class _Native:
+    """The functions of _host.so (csrc/host.cpp), loaded on first use.  Each takes its arguments in the form the
+    kernels read and returns None for anything else, without side effects."""
+
+    def __getattr__(self, name: str):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise LampaError(f"the native host module is missing or does not load ({exc}): build it with "
+                             "`python -m lampa_b200.build` (there is no CPU or PyTorch fallback)") from exc
+        fn = getattr(_host, name)
+        setattr(self, name, fn)
+        return fn
+
+
+native = _Native()
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise LampaError(f"{what}: {lib().lampa_error_string(rc).decode()} ({rc})")
@@ -138,6 +158,14 @@ def status_word(dev: torch.device) -> torch.Tensor:
     if idx not in _status:
         _status[idx] = torch.zeros(4, dtype=torch.int32, device=dev)
     return _status[idx]
+
+
+def status_word_of(index: int) -> torch.Tensor:
+    return status_word(torch.device("cuda", index))
+
+
+def check_status_of(index: int) -> None:
+    check_status(torch.device("cuda", index))
 
 
 def check_status(dev: Optional[torch.device] = None) -> None:

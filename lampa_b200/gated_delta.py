@@ -12,7 +12,6 @@ on the current torch stream; there is no PyTorch or CPU fallback.
 """
 from __future__ import annotations
 
-import ctypes
 import enum
 import math
 import warnings
@@ -99,23 +98,6 @@ def _forward_only(*tensors) -> None:
             "call under torch.no_grad() or detach the inputs")
 
 
-def _desc(q, v, g, lam, cu_seqlens, use_l2norm, scale) -> L.GdnDesc:
-    B, T, H, K = q.shape
-    return L.GdnDesc(B=B, T=T, H=H, K=K, V=v.shape[-1], L=0 if lam is None else lam.shape[-1],
-                     nseq=0 if cu_seqlens is None else len(cu_seqlens) - 1,
-                     qkv_dtype=L.dtype_code(q.dtype), gb_dtype=L.dtype_code(g.dtype),
-                     lam_dtype=L.LAMPA_F32 if lam is None else L.dtype_code(lam.dtype),
-                     use_l2norm=int(bool(use_l2norm)), scale=float(scale))
-
-
-def _workspace(desc: L.GdnDesc, dev: torch.device) -> torch.Tensor:
-    n = ctypes.c_size_t(0)
-    L.check(L.lib().lampa_gdn_workspace_bytes(ctypes.byref(desc), ctypes.byref(n)), "lampa_gdn_workspace_bytes")
-    buf = torch.empty(max(n.value, 256) + 1024, dtype=torch.uint8, device=dev)
-    skip = (-buf.data_ptr()) % 1024          # the library wants a 1024-byte aligned workspace
-    return buf[skip: skip + max(n.value, 256)]
-
-
 def _prep_inputs(q, k, v, g, beta, lam, cu_seqlens):
     dev = L.require_cuda(q, k, v, g, beta, lam)          # cu_seqlens may live on the host: it is copied over
     if v.shape[:3] != q.shape[:3] or k.shape != q.shape or g.shape != q.shape[:3] or beta.shape != q.shape[:3]:
@@ -127,9 +109,18 @@ def _prep_inputs(q, k, v, g, beta, lam, cu_seqlens):
         if lam.shape[:3] != q.shape[:3]:
             raise ValueError("l must be [B,T,H,L]")
         lam = lam.contiguous()
+    for t in (q, g, lam):
+        if t is not None:
+            L.dtype_code(t.dtype)                         # TypeError for a type the kernels do not read
     if cu_seqlens is not None:
         cu_seqlens = cu_seqlens.to(device=dev, dtype=torch.int64).contiguous()
     return dev, q, k, v, g, beta, lam, cu_seqlens
+
+
+def _launched(result, what: str):
+    if result is None:
+        raise L.LampaError(f"{what}: {L.lib().lampa_error_string(-2).decode()} (-2)")
+    return result
 
 
 def chunk_gated_delta_rule(
@@ -152,11 +143,17 @@ def chunk_gated_delta_rule(
     fp32 or None).  fp32 q/k/v are rejected as in the reference (gated_delta_rule_ori.py:313):
     the tensor-core operands are bf16, so an fp32 call could not honour fp32 accuracy.
     """
+    compiling = torch.compiler.is_compiling()
+    if not compiling and not head_first:
+        r = L.native.gdn(q, k, v, g, beta, None, initial_state, cu_seqlens, None, scale,
+                         bool(use_qk_l2norm_in_kernel), bool(output_final_state), True)
+        if r is not None:
+            return r
     _common_checks(q, k, v, beta, head_first, cu_seqlens, initial_state)
     _forward_only(q, k, v, g, beta, initial_state)
     if scale is None:
         scale = k.shape[-1] ** -0.5
-    if torch.compiler.is_compiling():          # one opaque node in the traced graph (see torch_ops.py)
+    if compiling:          # one opaque node in the traced graph (see torch_ops.py)
         from . import torch_ops  # noqa: F401
         o, ht = torch.ops.lampa_b200.gdn_fwd(q, k, v, g, beta, float(scale), initial_state, cu_seqlens,
                                              bool(use_qk_l2norm_in_kernel))
@@ -179,18 +176,11 @@ def _gdn_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_se
         if tuple(initial_state.shape) != (N, H, K, V):
             raise ValueError(f"initial_state must be [{N},{H},{K},{V}]")
         h0 = initial_state.to(torch.float32).contiguous()
-    desc = _desc(q, v, g, None, cu, use_qk_l2norm_in_kernel, scale)
-    o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
-    ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
-    ws = _workspace(desc, dev)
-    st = L.status_word(dev)
-    rc = L.lib().lampa_gdn_fwd(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                               L.ptr(h0), L.ptr(cu), L.ptr(o), L.ptr(ht), L.ptr(ws), ws.numel(),
-                               L.ptr(st), L.stream_ptr(dev))
-    L.check(rc, "lampa_gdn_fwd")
-    if L.debug_checks():
-        L.check_status(dev)
-    return o, ht
+    if B * T == 0:
+        ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
+        return torch.empty(B, T, H, V, dtype=q.dtype, device=dev), ht
+    return _launched(L.native.gdn(q, k, v, g, beta, None, h0, cu, None, float(scale), bool(use_qk_l2norm_in_kernel),
+                                  bool(output_final_state), False), "lampa_gdn_fwd")
 
 
 class HState:
@@ -210,6 +200,7 @@ class HState:
         self.dtype = dtype
         self.device = torch.device(device)
         self.max_num_levels = self.shape[-1]
+        self._arrivals = None
         if empty:                      # the caller attaches tensors it already has
             self.states = self.counts = None
             return
@@ -218,7 +209,7 @@ class HState:
 
     def arrivals(self) -> torch.Tensor:
         """The step kernel's arrival counter: one int32 of this state, zero between steps."""
-        a = getattr(self, "_arrivals", None)
+        a = self._arrivals
         if a is None or a.device != self.states.device:
             a = self._arrivals = torch.zeros(1, dtype=torch.int32, device=self.states.device)
         return a
@@ -247,42 +238,26 @@ def _hgdn(q, k, v, g, beta, lam, cu_seqlens, use_l2norm, want_state: bool = Fals
         raise ValueError(f"l has {lam.shape[-1]} levels, a sequence of {T} tokens needs {num_levels_required(T)}")
     if K > 256:
         raise NotImplementedError("current kernel does not support head dimension larger than 256.")
-    desc = _desc(q, v, g, lam, cu, use_l2norm, 1.0)
-    o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
-    ws = _workspace(desc, dev)
-    st = L.status_word(dev)
-    if out_perm is None:
-        rc = L.lib().lampa_hgdn_fwd(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                                    L.ptr(lam), L.ptr(cu), L.ptr(o), L.ptr(ws), ws.numel(), L.ptr(st),
-                                    L.stream_ptr(dev))
-    else:
+    if out_perm is not None:
         L.require_cuda(out_perm)
         if out_perm.dtype != torch.int64 or out_perm.dim() != 1 or not out_perm.is_contiguous() or out_perm.numel() > B * T:
             raise ValueError("out_perm must be a contiguous int64 vector of at most B*T row indices")
-        rc = L.lib().lampa_hgdn_fwd_scatter(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                                            L.ptr(lam), L.ptr(cu), L.ptr(out_perm), out_perm.numel(), L.ptr(o),
-                                            L.ptr(ws), ws.numel(), L.ptr(st), L.stream_ptr(dev))
-    L.check(rc, "lampa_hgdn_fwd")
-    states = counts = None
-    if want_state:
-        N = B if cu is None else len(cu) - 1
-        Lv = lam.shape[-1]
-        states = torch.empty(N, H, K, V, Lv, dtype=torch.float32, device=dev)
-        counts = torch.empty(N, Lv, dtype=torch.int32, device=dev)
-        rc = L.lib().lampa_hgdn_final_state(ctypes.byref(desc), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                                            L.ptr(cu), L.ptr(ws), ws.numel(), L.ptr(states), L.ptr(counts),
-                                            L.ptr(st), L.stream_ptr(dev))
-        L.check(rc, "lampa_hgdn_final_state")
-    if L.debug_checks():
-        L.check_status(dev)
-    return (o, states, counts) if want_state else o
+    if B * T == 0:
+        o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
+        if not want_state:
+            return o
+        N, Lv = (B if cu is None else len(cu) - 1), lam.shape[-1]
+        return o, torch.empty(N, H, K, V, Lv, device=dev), torch.empty(N, Lv, dtype=torch.int32, device=dev)
+    r = _launched(L.native.gdn(q, k, v, g, beta, lam, None, cu, out_perm, None, bool(use_l2norm), want_state, False),
+                  "lampa_hgdn_fwd")
+    return r if want_state else r[0]
 
 
 @torch.no_grad()
 def _hgdn_step(hstate: HState, q, k, v, g, beta, lam, use_l2norm: bool = True) -> torch.Tensor:
     """One token per batch row: q,k [B,H,K]; v [B,H,V]; g,beta [B,H]; lam [B,H,L] (as given to
     the kernel, i.e. not divided by scale).  Updates hstate in place, returns o [B,H,V]."""
-    dev = L.require_cuda(q, k, v, g, beta, lam, hstate.states, hstate.counts)
+    L.require_cuda(q, k, v, g, beta, lam, hstate.states, hstate.counts)
     B, H, K = q.shape
     V = v.shape[-1]
     Lv = lam.shape[-1]
@@ -290,20 +265,11 @@ def _hgdn_step(hstate: HState, q, k, v, g, beta, lam, use_l2norm: bool = True) -
         raise ValueError(f"state must be fp32 [{B},{H},{K},{V},{Lv}]")
     if not hstate.states.is_contiguous():
         hstate.states = hstate.states.contiguous()
+    if not hstate.counts.is_contiguous():
+        hstate.counts = hstate.counts.contiguous()
     q, k, v, g, lam = (x.contiguous() for x in (q, k, v, g, lam))
     beta = beta.to(g.dtype).contiguous()
-    desc = L.GdnDesc(B=B, T=1, H=H, K=K, V=V, L=Lv, nseq=0, qkv_dtype=L.dtype_code(q.dtype),
-                     gb_dtype=L.dtype_code(g.dtype), lam_dtype=L.dtype_code(lam.dtype),
-                     use_l2norm=int(bool(use_l2norm)), scale=1.0)
-    o = torch.empty(B, H, V, dtype=q.dtype, device=dev)
-    st = L.status_word(dev)
-    rc = L.lib().lampa_hgdn_step_counted(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta),
-                                         L.ptr(lam), L.ptr(hstate.states), L.ptr(hstate.counts),
-                                         L.ptr(hstate.arrivals()), L.ptr(o), L.ptr(st), L.stream_ptr(dev))
-    L.check(rc, "lampa_hgdn_step_counted")
-    if L.debug_checks():
-        L.check_status(dev)
-    return o
+    return _launched(L.native.step(q, k, v, g, beta, lam, hstate.states, hstate.counts, hstate.arrivals(), False), "lampa_hgdn_step")
 
 
 @torch.no_grad()
@@ -319,25 +285,18 @@ def _hgdn_prefill(q, k, v, g, beta, lam, use_l2norm: bool = True):
         raise ValueError(f"l has {Lv} levels, a sequence of {T0} tokens needs {num_levels_required(T0)}")
     if K > 256:
         raise NotImplementedError("current kernel does not support head dimension larger than 256.")
-    hstate = HState(2, HType.WEAK, HStruct.GDELTA, (B, H, K, V, Lv), torch.float32, dev, empty=True)
-    o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
-    if T == 0:
-        hstate.states = torch.zeros(hstate.shape, dtype=torch.float32, device=dev)
-        hstate.counts = torch.zeros(Lv, dtype=torch.int32, device=dev)
-        return o, hstate
-    hstate.states = torch.empty(hstate.shape, dtype=torch.float32, device=dev)
-    hstate.counts = torch.empty(Lv, dtype=torch.int32, device=dev)
-    desc = _desc(q, v, g, lam, None, use_l2norm, 1.0)
-    desc.T = T0
-    ws = _workspace(desc, dev)
-    desc.T = T
-    rc = L.lib().lampa_hgdn_prefill(ctypes.byref(desc), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta), L.ptr(lam),
-                                    L.ptr(o), L.ptr(ws), ws.numel(), L.ptr(hstate.states), L.ptr(hstate.counts),
-                                    L.ptr(L.status_word(dev)), L.stream_ptr(dev))
-    L.check(rc, "lampa_hgdn_prefill")
-    if L.debug_checks():
-        L.check_status(dev)
-    return o, hstate
+    if B * T == 0:
+        return (torch.empty(B, T, H, V, dtype=q.dtype, device=dev),
+                HState(2, HType.WEAK, HStruct.GDELTA, (B, H, K, V, Lv), torch.float32, dev))
+    return _with_state(_launched(L.native.prefill(q, k, v, g, beta, lam, False), "lampa_hgdn_prefill"))
+
+
+def _with_state(r):
+    """(o, states, counts) -> (o, HState)"""
+    o, states, counts = r
+    hs = HState(2, HType.WEAK, HStruct.GDELTA, states.shape, torch.float32, states.device, empty=True)
+    hs.states, hs.counts = states, counts
+    return o, hs
 
 
 def chunk_h_gated_delta_rule(
@@ -375,6 +334,21 @@ def chunk_h_gated_delta_rule(
     Device-side problems (a wait that ran out, device-resident cu_seqlens that are malformed or
     need more levels than l has) are reported through `check_status()`.
     """
+    if use_qk_l2norm_in_kernel is True and not head_first and not torch.compiler.is_compiling():
+        # arguments the kernels read as they are; anything else falls through to the checks and conversions below
+        if initial_state is None:
+            if output_final_state is False or cu_seqlens is not None:
+                r = L.native.gdn(q, k, v, g, beta, l, None, cu_seqlens, out_perm, None, True, output_final_state is not False,
+                                 True)
+            else:
+                r = L.native.prefill(q, k, v, g, beta, l, True)
+            if r is not None:
+                return r if output_final_state is False else _with_state(r)
+        elif output_final_state is not False and cu_seqlens is None and type(initial_state) is HState:
+            r = L.native.step(q, k, v, g, beta, l, initial_state.states, initial_state.counts, initial_state.arrivals(),
+                              True)
+            if r is not None:
+                return r, initial_state
     _common_checks(q, k, v, beta, head_first, cu_seqlens, None)
     assert use_qk_l2norm_in_kernel is True
     _forward_only(q, k, v, g, l, beta)
@@ -388,10 +362,7 @@ def chunk_h_gated_delta_rule(
     if cu_seqlens is not None:
         if initial_state is not None:
             raise NotImplementedError("a decode step takes one token per batch row, not packed sequences")
-        o, states, counts = _hgdn(q, k, v, g, beta, l, cu_seqlens, True, want_state=True)
-        hs = HState(2, HType.WEAK, HStruct.GDELTA, tuple(states.shape), torch.float32, states.device, empty=True)
-        hs.states, hs.counts = states, counts
-        return o, hs
+        return _with_state(_hgdn(q, k, v, g, beta, l, cu_seqlens, True, want_state=True))
     if initial_state is None:
         return _hgdn_prefill(q, k, v, g, beta, l, True)
     if not all([q.ndim == 4, q.shape[1] == 1, k.ndim == 4, k.shape[1] == 1, v.ndim == 4, v.shape[1] == 1,

@@ -11,7 +11,6 @@ reference never computes.  All data movement and sorting runs in the CUDA librar
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -21,7 +20,6 @@ from . import _lib as L
 
 
 # ---- thin wrappers over the C ABI ------------------------------------------------------------------
-@torch.no_grad()
 def lsh_hash(x: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, w: float = 1.0, *,
              dim: Optional[int] = None, per_head_rows: bool = False, want_ids: bool = True,
              want_keys: bool = False, want_packed: bool = False):
@@ -32,11 +30,14 @@ def lsh_hash(x: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, w: float 
     Returns a dict with 'ids' int32 [rounds, heads, N], 'keys' fp32 [rounds, heads, N] (a.x),
     'packed' int32 [rounds, N] (sum_h ids << h) for the requested outputs.
     """
-    dev = L.require_cuda(x, alpha, beta)
+    L.require_cuda(x, alpha, beta)
     heads, d, rounds = alpha.shape
     dim = d if dim is None else dim
     if dim != d:
         raise ValueError("alpha's middle dimension must equal dim")
+    r = _hash(x, alpha, beta, w, per_head_rows, want_ids, want_keys, want_packed)
+    if r is not None:
+        return r
     # head-major rows that sit in padded storage (last stride 1, heads dense over the row pitch) are read in place
     in_place = (per_head_rows and x.dim() == 3 and x.dtype == torch.float32 and x.stride(2) == 1
                 and x.stride(1) >= x.shape[2] and x.stride(0) == x.stride(1) * x.shape[1])
@@ -49,28 +50,17 @@ def lsh_hash(x: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, w: float 
     if per_head_rows:
         if x.dim() != 3 or x.shape[0] != heads or x.shape[2] != dim:
             raise ValueError("x must be [heads, N, dim]")
-        N, row_stride, head_stride = x.shape[1], x.stride(1), x.stride(0)
     else:
         if x.dim() != 2 or x.shape[1] < dim:
             raise ValueError("x must be [N, row >= dim]")
-        N, row_stride, head_stride = x.shape[0], x.shape[1], 0
-    out = {}
-    ids = torch.empty(rounds, heads, N, dtype=torch.int32, device=dev) if want_ids else None
-    keys = torch.empty(rounds, heads, N, dtype=torch.float32, device=dev) if want_keys else None
-    packed = torch.empty(rounds, N, dtype=torch.int32, device=dev) if want_packed else None
-    rc = L.lib().lampa_lsh_hash(L.ptr(x), row_stride, head_stride, L.ptr(alpha), L.ptr(beta), float(w), N,
-                                heads, rounds, dim, L.ptr(ids), L.ptr(keys), L.ptr(packed), L.stream_ptr(dev))
-    L.check(rc, "lampa_lsh_hash")
-    if want_ids:
-        out["ids"] = ids
-    if want_keys:
-        out["keys"] = keys
-    if want_packed:
-        out["packed"] = packed
-    return out
+    return _hash(x, alpha, beta, w, per_head_rows, want_ids, want_keys, want_packed)
 
 
-@torch.no_grad()
+def _hash(x, alpha, beta, w, per_head_rows, want_ids, want_keys, want_packed):
+    r = L.native.lsh_hash(x, alpha, beta, float(w), bool(per_head_rows), bool(want_ids), bool(want_keys), bool(want_packed))
+    return None if r is None else {k: t for k, t in zip(("ids", "keys", "packed"), r) if t is not None}
+
+
 def segmented_sort(keys: torch.Tensor, seg_offsets: Optional[torch.Tensor] = None, nseg: Optional[int] = None,
                    init: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Stable ascending sort per segment of a flat int32 / fp32 key array.
@@ -79,15 +69,13 @@ def segmented_sort(keys: torch.Tensor, seg_offsets: Optional[torch.Tensor] = Non
     indices local to each segment.  With `init` (a starting order per segment) the result is
     init[stable_sort(keys[init])] — the norm pre-sort followed by the key sort of LSHOrdering.
     """
+    r = L.native.segsort(keys, seg_offsets, 1 if nseg is None else int(nseg), init)
+    if r is not None:
+        return r
     dev = L.require_cuda(keys, init)
-    if keys.dtype == torch.int32:
-        kt = L.LAMPA_KEY_I32
-    elif keys.dtype == torch.float32:
-        kt = L.LAMPA_KEY_F32
-    else:
+    if keys.dtype not in (torch.int32, torch.float32):
         raise TypeError("keys must be int32 or float32")
     flat = keys.contiguous().view(-1)
-    n = flat.numel()
     if seg_offsets is not None:
         seg_offsets = seg_offsets.to(device=dev, dtype=torch.int64).contiguous()
         nseg = seg_offsets.numel() - 1
@@ -95,20 +83,15 @@ def segmented_sort(keys: torch.Tensor, seg_offsets: Optional[torch.Tensor] = Non
         nseg = 1
     if init is not None:
         init = init.to(torch.int64).contiguous().view(-1)
-    perm = torch.empty(n, dtype=torch.int64, device=dev)
-    nb = ctypes.c_size_t(0)
-    L.check(L.lib().lampa_segsort_workspace_bytes(n, ctypes.byref(nb)), "lampa_segsort_workspace_bytes")
-    ws = torch.empty(nb.value, dtype=torch.uint8, device=dev)
-    rc = L.lib().lampa_segsort_stable(L.ptr(flat), kt, n, L.ptr(seg_offsets), nseg, L.ptr(init), L.ptr(perm),
-                                      L.ptr(ws), ws.numel(), L.ptr(L.status_word(dev)), L.stream_ptr(dev))
-    L.check(rc, "lampa_segsort_stable")
-    return perm
+    return L.native.segsort(flat, seg_offsets, int(nseg), init)
 
 
-@torch.no_grad()
 def permute_rows(src: torch.Tensor, perm: torch.Tensor, seg_offsets: Optional[torch.Tensor] = None,
                  nseg: int = 1, scatter: bool = False) -> torch.Tensor:
     """dst[s0+i] = src[s0+perm[s0+i]] per segment (or the scatter form); src is [rows, ...]."""
+    r = L.native.permute_rows(src, perm, seg_offsets, nseg, bool(scatter))
+    if r is not None:
+        return r
     dev = L.require_cuda(src, perm)
     src = src.contiguous()
     rows = perm.numel()
@@ -121,26 +104,20 @@ def permute_rows(src: torch.Tensor, perm: torch.Tensor, seg_offsets: Optional[to
     if seg_offsets is not None:
         seg_offsets = seg_offsets.to(device=dev, dtype=torch.int64).contiguous()
         nseg = seg_offsets.numel() - 1
-    dst = torch.empty_like(src)
-    rc = L.lib().lampa_permute_rows(L.ptr(src), L.ptr(perm), L.ptr(seg_offsets), nseg, rows, row_bytes,
-                                    int(scatter), L.ptr(dst), L.ptr(L.status_word(dev)), L.stream_ptr(dev))
-    L.check(rc, "lampa_permute_rows")
-    return dst
+    if rows == 0 or src.numel() == 0:
+        return torch.empty_like(src)
+    return L.native.permute_rows(src, perm, seg_offsets, nseg, bool(scatter))
 
 
 # ---- reference-named entry points ----------------------------------------------------------------------
-@torch.no_grad()
 def invert_permutation(perm: torch.Tensor) -> torch.Tensor:
     """perm: (..., n) -> inverse permutation along the last axis (hash_utils.py:46-57)."""
-    dev = L.require_cuda(perm)
+    r = L.native.invert_perm(perm)
+    if r is not None:
+        return r
+    L.require_cuda(perm)
     p = perm.to(torch.int64).contiguous()
-    n = p.shape[-1]
-    inv = torch.empty_like(p)
-    nseg = p.numel() // n if n else 1
-    rc = L.lib().lampa_invert_perm(L.ptr(p), None, max(nseg, 1), p.numel(), L.ptr(inv), L.ptr(L.status_word(dev)),
-                                   L.stream_ptr(dev))
-    L.check(rc, "lampa_invert_perm")
-    return inv
+    return L.native.invert_perm(p) if p.numel() else torch.empty_like(p)
 
 
 @torch.no_grad()
@@ -233,11 +210,14 @@ class LSHOrdering(nn.Module):
         return ordered, idx
 
 
-@torch.no_grad()
 def lsh_bucket_sort(x: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, w: float = 1.0,
                     seg_offsets: Optional[torch.Tensor] = None):
     """Integer pipeline of one packed batch: ids [rounds, heads, N] and, per (round, head) row and
     per event, the stable ascending permutation [rounds, heads, N] (int64, local to the event)."""
+    if seg_offsets is None:
+        r = L.native.bucket_sort(x, alpha, beta, float(w))
+        if r is not None:
+            return r
     ids = lsh_hash(x, alpha, beta, w)["ids"]
     rounds, heads, N = ids.shape
     if seg_offsets is None:

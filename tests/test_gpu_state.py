@@ -155,13 +155,13 @@ def test_prefill_with_ragged_tail_and_decode(lb, T, K, V):
     (65, 3, 32, 32, 2),               # one tail token behind one chunk
     (64 * 5 + 63, 1, 64, 64, 1),      # longest tail
     (64 * 31 + 17, 1, 64, 64, 0),     # five chunk levels live
-    (64 * 511 + 5, 1, 16, 32, 0),     # nine
+    (64 * 511 + 5, 1, 64, 64, 0),     # nine
 ])
 def test_prefill_tail_edges(lb, T, H, K, V, extra):
     """Two rows of ragged prompts: outputs and states of the fp32 tail at the edges of its slots and lengths."""
     from lampa_b200 import synth
     Lv = lb.num_levels_required(T) + extra
-    rows = [synth.gdn_inputs(51 + i, T, H, K, V, L=Lv, g_shift=-5.0) for i in range(2)]
+    rows = [synth.gdn_inputs(51 + i, T, H, K, V, L=Lv, g_shift=-3.0) for i in range(2)]
     d = {k: torch.cat([r[k] for r in rows], 0).cuda() for k in rows[0]}
     o, hs = lb.chunk_h_gated_delta_rule(d["q"], d["k"], d["v"], d["g"], d["lam"], d["beta"],
                                         output_final_state=True, use_qk_l2norm_in_kernel=True)
