@@ -14,8 +14,17 @@
 
 namespace lampa {
 
-constexpr int BLOCK_CHUNKS = 32;     // chunks per block of the block-parallel scan
-constexpr int BLOCK_LOG = 5;         // log2(BLOCK_CHUNKS): chunk levels 0..4 live inside a block
+// Chunks per block of the block-parallel scan, as a power of two: chunk levels 0 .. block_log - 1 live inside a block.
+// A block is a serial chain in the compose and output passes, the blocks of a sequence are one in the level pass, so
+// the critical path of a sequence of nch chunks is about nch / blocks * (0.65 + 1.45 us) + blocks * 0.9 us (K = V = 64):
+// 32-chunk blocks left 12 - 24 CTAs on the GPU for a 6000-token event (71 us at 4 heads, 30 us with 8).  The smallest
+// block that keeps a sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
+// beyond 1024 chunks there are blocks enough to fill the GPU, and smaller ones would only add composites to move.
+// The choice depends on the sequence alone, never on what else a call carries, so that a sequence's result does not.
+constexpr int BLOCK_CHUNKS = 32, BLOCK_LOG = 5;      // largest block
+constexpr int MIN_BLOCK_LOG = 3;                     // smallest
+__host__ __device__ __forceinline__ int block_log(int nch) { return nch <= 256 ? 3 : (nch <= 512 ? 4 : BLOCK_LOG); }
+__host__ __device__ __forceinline__ int blocks_of(int nch) { const int bl = block_log(nch); return (nch + (1 << bl) - 1) >> bl; }
 constexpr int NLW = 5;               // level states carried per warp in the hierarchical output pass
 constexpr int MAX_GROUPS = 3;        // 1 group of in-block levels + up to 2 groups of cross-block levels
 
@@ -91,7 +100,7 @@ __device__ __forceinline__ void stage_tick(const GdnArgs& a, int cta, int slot) 
 // Offset tables of equally long sequences, written by the first CTA of the preparation kernel for the passes that
 // follow it (the preparation kernel itself locates its chunks by arithmetic in that case).
 __device__ __forceinline__ void write_fixed_plan(const GdnArgs& a) {
-    const int bps = (a.fixed_cps + BLOCK_CHUNKS - 1) / BLOCK_CHUNKS;
+    const int bps = blocks_of(a.fixed_cps);
     for (int s = threadIdx.x; s <= a.nseq; s += blockDim.x) {
         const_cast<int64_t*>(a.tok_off)[s] = (int64_t)s * a.fixed_stride;
         const_cast<int32_t*>(a.chunk_off)[s] = s * a.fixed_cps;

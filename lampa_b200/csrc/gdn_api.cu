@@ -1,5 +1,6 @@
 // C ABI of the gated-delta forward: argument checks, workspace carve-up, kernel dispatch.
 #include "gdn.cuh"
+#include <algorithm>
 #include <cstdlib>
 
 using namespace lampa;
@@ -45,15 +46,19 @@ int make_layout(const lampa_gdn_desc* d, bool hier, Layout& l) {
     const int64_t ttot = (int64_t)d->B * d->T;
     // each sequence adds at most one ragged chunk and one ragged block
     const int64_t ncm = d->nseq > 0 ? ttot / CHUNK + l.nseq : (int64_t)d->B * ((d->T + CHUNK - 1) / CHUNK);
-    const int64_t nbm = d->nseq > 0 ? ncm / BLOCK_CHUNKS + l.nseq
-                                    : (int64_t)d->B * (((d->T + CHUNK - 1) / CHUNK + BLOCK_CHUNKS - 1) / BLOCK_CHUNKS);
-    if (ncm > (1 << 30) || nbm > 65535LL * 1024) return LAMPA_ERR_UNSUPPORTED;
+    if (ncm > (1 << 30)) return LAMPA_ERR_UNSUPPORTED;
+    // packed: at most one block per 8 chunks, and at most 32 or one per 32 chunks in any sequence (blocks_of)
+    const int64_t nbm = d->nseq > 0 ? std::min<int64_t>(ncm >> MIN_BLOCK_LOG, (ncm >> BLOCK_LOG) + (int64_t)l.nseq * 31) + l.nseq
+                                    : (int64_t)d->B * blocks_of((d->T + CHUNK - 1) / CHUNK);
+    if (nbm > 65535LL * 1024) return LAMPA_ERR_UNSUPPORTED;
     l.nc_max = (int)(ncm > 0 ? ncm : 1);
     l.nb_max = (int)(nbm > 0 ? nbm : 1);
     // longest possible sequence bounds the number of cross-block levels
     const int64_t longest = d->nseq > 0 ? (ttot + CHUNK - 1) / CHUNK : (d->T + CHUNK - 1) / CHUNK;
     const int nlev = longest > 1 ? ceil_log2_int((int)longest) : 0;
-    l.nhigh_max = hier ? (nlev > BLOCK_LOG ? nlev - BLOCK_LOG : 0) : 0;
+    // cross-block levels of any sequence up to that length: nlev - 3 up to 256 chunks, 5 up to 1024, then nlev - 5
+    const int nhigh = nlev <= MIN_BLOCK_LOG ? 0 : (nlev <= 8 ? nlev - MIN_BLOCK_LOG : (nlev <= 10 ? 5 : nlev - BLOCK_LOG));
+    l.nhigh_max = hier ? nhigh : 0;
     if (hier && 1 + (l.nhigh_max + NLW - 1) / NLW > MAX_GROUPS) return LAMPA_ERR_UNSUPPORTED;
     l.LC = hier ? (d->L > ELL0 ? d->L - ELL0 : 1) : 0;
     if (d->K == 64) fill_sizes<64, 64>(l);

@@ -25,7 +25,7 @@ __global__ void plan_kernel(PlanArgs p) {
         const int nch = (int)((len + CHUNK - 1) / CHUNK);
         if (p.hier && nch > 0 && ELL0 + ceil_log2_int(nch) > p.L) set_status(p.status, LAMPA_ERR_LEVELS, 1, s);
         c += nch;
-        b += (nch + BLOCK_CHUNKS - 1) / BLOCK_CHUNKS;
+        b += blocks_of(nch);
         p.chunk_off[s + 1] = c;
         p.block_off[s + 1] = b;
         if (s == p.nseq - 1) p.tok_off[s + 1] = t0 + len;

@@ -173,8 +173,9 @@ __global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
     const int seq = find_seq(a.block_off, a.nseq, gb);
     const int b = gb - a.block_off[seq];
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
-    const int c0 = a.chunk_off[seq] + b * BLOCK_CHUNKS;
-    const int nsteps = min(BLOCK_CHUNKS, nch - b * BLOCK_CHUNKS);
+    const int bc = 1 << block_log(nch);
+    const int c0 = a.chunk_off[seq] + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
 
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
 // -------------------------------------------------------------------------------------------------
 // level: scan of the block composites.  Plain rule: one state per (sequence, head), seeded by h0,
 // the state entering every block is stored and the last one is the final state.  Hierarchical:
-// one CTA per cross-block level lh (chunk level 5 + lh); the level collects blocks whose bit lh is
+// one CTA per cross-block level lh (chunk level block_log + lh); the level collects blocks whose bit lh is
 // 0, is read by blocks whose bit lh is 1 (its entry state is stored for those) and is cleared at
 // the end of each period of 2^(lh+1) blocks.
 // -------------------------------------------------------------------------------------------------
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
     if (HIER) {
         const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
         const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
-        if (lh >= nlev - BLOCK_LOG) return;
+        if (lh >= nlev - block_log(nch)) return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -341,21 +342,21 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int row0 = warp * 16;
-    const int n = nch - 1;
+    const int n = nch - 1, bl = block_log(nch);
     const bool live = nch > 0 && lev < 30 && ((n >> lev) & 1);
 
     float C[KD / 8][4];
     zero_state<KD>(C);
     if (live) {
         int c_first, half_end;
-        if (lev < BLOCK_LOG) {
+        if (lev < bl) {
             c_first = n & ~((2 << lev) - 1);
             half_end = c_first + (1 << lev);
         } else {
-            c_first = (n >> BLOCK_LOG) << BLOCK_LOG;
+            c_first = (n >> bl) << bl;
             half_end = c_first;
-            const int gb = a.block_off[seq] + (n >> BLOCK_LOG);
-            const float* e = a.entry + (((size_t)gb * a.nhigh_max + (lev - BLOCK_LOG)) * H + h) * R::STATE_FLOATS;
+            const int gb = a.block_off[seq] + (n >> bl);
+            const float* e = a.entry + (((size_t)gb * a.nhigh_max + (lev - bl)) * H + h) * R::STATE_FLOATS;
             load_slab_f32<KD>(C, e, KD, row0, lane);
         }
         Pipe<NST> pipe;
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
                 }
             if (c_first + i < half_end) load_slab_bf16<KD>(C, sBt, row0, lane);
             else zero_state<KD>(C);
-            if (i > 0 || lev >= BLOCK_LOG) {
+            if (i > 0 || lev >= bl) {
                 state_times_mt<KD, Tile<KD>>(C, sp, sM, lane);
                 state_times_mt<KD, Tile<KD>>(C, sl, sM, lane);
             }
@@ -418,9 +419,10 @@ __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
     const int seq = find_seq(a.block_off, a.nseq, gb);
     const int b = gb - a.block_off[seq];
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
-    const int c0 = a.chunk_off[seq] + b * BLOCK_CHUNKS;
-    const int nsteps = min(BLOCK_CHUNKS, nch - b * BLOCK_CHUNKS);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * BLOCK_CHUNKS * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int bc = 1 << block_log(nch);
+    const int c0 = a.chunk_off[seq] + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
+    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int row0 = warp * 16;
@@ -480,8 +482,8 @@ __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
 }
 
 // -------------------------------------------------------------------------------------------------
-// output, hierarchical rule.  Warp = (level group, slab).  Group 0 carries chunk levels 0..4, which
-// live and die inside the block; group gi >= 1 carries cross-block levels 5*(gi-1) .. +4, seeded
+// output, hierarchical rule.  Warp = (level group, slab).  Group 0 carries the chunk levels that
+// live and die inside the block (0 .. block_log - 1); group gi >= 1 carries cross-block levels 5*(gi-1) .. +4, seeded
 // from the level pass.  A level is read by chunk n when bit l of n is set:
 //     O_n += diag(lambda[:, 7 + l]) (Q~ S_l)
 // and then advances: cleared at the end of its period of 2^(l+1) chunks, otherwise
@@ -500,10 +502,11 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
     const int b = gb - a.block_off[seq];
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
-    const int nhigh = max(0, nlev - BLOCK_LOG);
-    const int c0 = a.chunk_off[seq] + b * BLOCK_CHUNKS;
-    const int nsteps = min(BLOCK_CHUNKS, nch - b * BLOCK_CHUNKS);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * BLOCK_CHUNKS * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int bl = block_log(nch), bc = 1 << bl;
+    const int nhigh = max(0, nlev - bl);
+    const int c0 = a.chunk_off[seq] + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
+    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int grp = warp / NS, slab = warp - grp * NS;
@@ -547,7 +550,7 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
         const __nv_bfloat16* sQt = reinterpret_cast<const __nv_bfloat16*>(st + R::QT_OFF);
         const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + R::OL_OFF);
         const float* sLam = reinterpret_cast<const float*>(st + R::LAM_OFF);
-        const int n = b * BLOCK_CHUNKS + i;
+        const int n = b * bc + i;
 
         float O[4][2][4];
 #pragma unroll
@@ -559,6 +562,7 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
         for (int x = 0; x < NLW; ++x) {
             bool do_read, do_mma, add_b, clear;
             int lam_row;
+            if (grp == 0 && x >= bl) continue;      // smaller blocks carry fewer levels of their own
             if (grp == 0) {
                 const int per = 2 << x, pos = n & (per - 1), bit = (n >> x) & 1;
                 do_read = bit != 0;
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
                 clear = false;
                 add_b = false;
                 do_mma = lv && (i + 1 < nsteps);
-                lam_row = BLOCK_LOG + (grp - 1) * NLW + x;
+                lam_row = bl + (grp - 1) * NLW + x;
             }
             if (lam_row >= a.LC) do_read = false;   // only reachable when the level check already failed
             uint32_t sp[KD / 16][4];

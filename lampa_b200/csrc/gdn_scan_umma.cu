@@ -1,9 +1,9 @@
 // Output passes on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM) for K = V = 64:
 // the hierarchical rule first, the plain rule (one state per head) at the end of the file.
 //
-// Per (block of 32 chunks, head) one CTA keeps every level state the block touches as rows of
+// Per (block of up to 32 chunks, head) one CTA keeps every level state the block touches as rows of
 // bf16 A operands in tensor memory: slot s holds S_l^T (64 rows v x 64 columns k), two slots
-// per 128-row operand ("pair").  Slots 0..4 are the chunk levels that live inside the block,
+// per 128-row operand ("pair").  The first block_log slots are the chunk levels that live inside the block,
 // the following ones the cross-block levels this block reads (seeded from the level pass).
 // A chunk is one record {M | Q~ | B^T | O_local | lambda}; its first 16 KB, the M and Q~ tiles back to
 // back, are a single 128-row K-major B operand, so ONE accumulating MMA per pair,
@@ -32,7 +32,7 @@ namespace lampa {
 namespace {
 
 constexpr int UKD = 64, UVD = 64;
-constexpr int UNP = 5;                       // pairs of slots: 5 in-block levels + up to 5 cross-block levels
+constexpr int UNP = 5;                       // pairs of slots: up to 5 in-block levels + up to 5 cross-block levels
 constexpr int UEPI_WARPS = 16;               // 4 warpgroups, each covering 16 state columns and 16 tokens of all 128 rows
 constexpr int UTHREADS = (UEPI_WARPS + 2) * 32;   // plus one control warp and one relay warp
 // An mbarrier poll costs the polling warp 200 - 300 cycles even when the phase is long complete, a hardware named
@@ -101,10 +101,11 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
     const int b = gb - a.block_off[seq];
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
-    const int nhigh = max(0, nlev - BLOCK_LOG);
-    const int c0 = a.chunk_off[seq] + b * BLOCK_CHUNKS;
-    const int nsteps = min(BLOCK_CHUNKS, nch - b * BLOCK_CHUNKS);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * BLOCK_CHUNKS * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int bl = block_log(nch), bc = 1 << bl;
+    const int nhigh = max(0, nlev - bl);
+    const int c0 = a.chunk_off[seq] + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
+    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int wg = warp >> 2;                          // 0..3: state columns / tokens 16*wg .. 16*wg+15; 4: control
     const int row = (warp & 3) * 32 + lane;            // TMEM lane = row of the pair's A operand
@@ -116,15 +117,16 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
     const char* rec0 = a.rec + ((size_t)c0 * H + h) * a.rec_bytes;
     const size_t rec_stride = (size_t)H * a.rec_bytes;
 
-    // cross-block levels this block reads, compacted into slots 5, 6, ...
+    // cross-block levels this block reads, compacted into slots bl, bl + 1, ...
     int nlive = 0;
     uint32_t live_pack = 0;                            // 4 bits per compact slot: the level index
     for (int lh = 0; lh < nhigh; ++lh)
         if ((b >> lh) & 1) { live_pack |= (uint32_t)lh << (4 * nlive); ++nlive; }
-    const int nslots = BLOCK_LOG + nlive;
+    const int nslots = bl + nlive;
     const int npairs = (nslots + 1) >> 1;
-    // accumulator buffers of 128 columns behind the operands: three where four pairs or fewer leave room for them
-    const int nbuf = npairs <= 4 ? 3 : 2, tm_d = npairs <= 4 ? 128 : TM_D;
+    // accumulator buffers of 128 columns behind the operands: three where four pairs or fewer leave room for them,
+    // never more than pairs (the hand-back of MMA m - nbuf must be the latest one of its pair)
+    const int nbuf = npairs <= 4 ? min(npairs, 3) : 2, tm_d = npairs <= 4 ? 128 : TM_D;
 
     if (tid == 0) {
 #pragma unroll
@@ -151,8 +153,8 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
             float x[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) x[i] = 0.f;
-            if (s >= BLOCK_LOG && s < nslots) {
-                const int lh = (live_pack >> (4 * (s - BLOCK_LOG))) & 15;
+            if (s >= bl && s < nslots) {
+                const int lh = (live_pack >> (4 * (s - bl))) & 15;
                 const float4* e = reinterpret_cast<const float4*>(
                     a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * UR::STATE_FLOATS + (size_t)v * UKD + 16 * part);
 #pragma unroll
@@ -242,11 +244,11 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
 #pragma unroll
         for (int p = 0; p < UNP; ++p) {
             const int s = 2 * p + u;
-            const int row = s < BLOCK_LOG ? s : BLOCK_LOG + (int)((live_pack >> (4 * max(s - BLOCK_LOG, 0))) & 15);
+            const int row = s < bl ? s : bl + (int)((live_pack >> (4 * max(s - bl, 0))) & 15);
             lam_pack |= (uint32_t)(row & 31) << (5 * p);
         }
         for (int s = 0; s < nslots; ++s) {
-            const int row = s < BLOCK_LOG ? s : BLOCK_LOG + (int)((live_pack >> (4 * (s - BLOCK_LOG))) & 15);
+            const int row = s < bl ? s : bl + (int)((live_pack >> (4 * (s - bl))) & 15);
             if (row < a.LC) slot_ok |= 1u << s;      // a missing row is only reachable when the level check already failed
         }
         int bufi = 0;                                // accumulator buffer of the next pair, in step with the control warp
@@ -254,14 +256,14 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
             const unsigned char* st = stage0 + (size_t)(i % UNST) * stage_bytes;
             const float* sLam = reinterpret_cast<const float*>(st + STAGE_TILES);
             const unsigned char* sBt = st + UR::BT_OFF;
-            const int n = b * BLOCK_CHUNKS + i;
+            const int n = b * bc + i;
             const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + UR::OL_OFF);
             // what this chunk does to each slot, as bit masks: in-block level s is read when bit s of n is
             // set and cleared when its period of 2^(s+1) chunks ends (all of bits 0..s set); the cross-block
             // slots are read by every chunk
-            const uint32_t low = (uint32_t)n & (BLOCK_CHUNKS - 1);
-            const uint32_t read_mask = (low | (~0u << BLOCK_LOG)) & slot_ok;
-            const uint32_t clear_mask = low & ~(low + 1u) & (BLOCK_CHUNKS - 1);      // trailing ones of n
+            const uint32_t low = (uint32_t)n & (bc - 1);
+            const uint32_t read_mask = (low | (~0u << bl)) & slot_ok;
+            const uint32_t clear_mask = low & ~(low + 1u) & (bc - 1);      // trailing ones of n
             uint4 bq0, bq1;                            // this row's 16 columns of B^T, shared by every level that collects in this chunk
 
             float oacc[16];
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
                 }
                 const int s = 2 * p + u;
                 const bool active = s < nslots;
-                const bool do_read = (read_mask >> s) & 1u, clear = (clear_mask >> s) & 1u, add_b = !((n >> s) & 1) && s < BLOCK_LOG;
+                const bool do_read = (read_mask >> s) & 1u, clear = (clear_mask >> s) & 1u, add_b = !((n >> s) & 1) && s < bl;
                 const int lam_row = (int)((lam_pack >> (5 * p)) & 31u);
                 const uint32_t tcol = tlane + (uint32_t)(tm_d + bufi * 128);
                 bufi = bufi + 1 == nbuf ? 0 : bufi + 1;
@@ -406,9 +408,10 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs
     const int seq = find_seq(a.block_off, a.nseq, gb);
     const int b = gb - a.block_off[seq];
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
-    const int c0 = a.chunk_off[seq] + b * BLOCK_CHUNKS;
-    const int nsteps = min(BLOCK_CHUNKS, nch - b * BLOCK_CHUNKS);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * BLOCK_CHUNKS * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int bc = 1 << block_log(nch);
+    const int c0 = a.chunk_off[seq] + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
+    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int sp = warp & 3, cq = (warp >> 2) & 3;     // lane quarter; 16 state columns and 16 tokens
     const int sub = lane >> 4, v = 16 * sp + (lane & 15);   // head of the pair, state row
@@ -606,12 +609,13 @@ int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st) {
     uo.nbs = 0;
     if (a.fixed_T > 0 && a.nseq > 0 && a.nb_max % a.nseq == 0 && a.nb_max / a.nseq <= 64) {
         uo.nbs = a.nb_max / a.nseq;
+        const int bl = block_log(a.fixed_cps);
         int n = 0;
         for (int pairs = UNP; pairs >= 0; --pairs)        // stable: block order kept inside a class
             for (int b = 0; b < uo.nbs; ++b) {
                 int live = 0;
                 for (int lh = 0; lh < a.nhigh_max; ++lh) live += (b >> lh) & 1;
-                if ((BLOCK_LOG + live + 1) / 2 == pairs) uo.order[n++] = (unsigned char)b;
+                if ((bl + live + 1) / 2 == pairs) uo.order[n++] = (unsigned char)b;
             }
         if (n != uo.nbs) uo.nbs = 0;
     }
