@@ -214,6 +214,18 @@ int lampa_segsort_stable(const void* keys, int32_t key_type, int64_t n_total,
                          int64_t* perm, void* ws, size_t ws_bytes, int32_t* status, void* stream);
 
 /*
+ * LSHOrdering.forward in one call: key = sum_c 2^c (coords . alpha[:, c]), rows ordered by norm, then stably by key,
+ * and gathered.
+ * Replaces: models/baselines/hmamba.py:306-353.
+ *   coords fp32 [B, n, dim], alpha fp32 [dim, num_hashes], points B * n rows of row_bytes (a multiple of 4);
+ *   idx int64 [B, n] (local to a batch row), ordered: the rows in that order.  Workspace 16-byte aligned.
+ */
+int lampa_lsh_ordering_workspace_bytes(int32_t B, int64_t n, size_t* bytes);
+int lampa_lsh_ordering(const float* coords, const float* alpha, int32_t dim, int32_t num_hashes, const void* points,
+                       int64_t row_bytes, int32_t B, int64_t n, int64_t* idx, void* ordered, void* ws, size_t ws_bytes,
+                       int32_t* status, void* stream);
+
+/*
  * lampa_segsort_stable for hosts that may not allocate device memory when they call it.
  * No counterpart in the reference (its sorts allocate through torch on every call).
  *

@@ -37,7 +37,8 @@ _lib: Optional[ctypes.CDLL] = None
 EXPORTS = ["lampa_version", "lampa_error_string", "lampa_gdn_workspace_bytes", "lampa_gdn_workspace_layout",
            "lampa_gdn_fwd", "lampa_hgdn_fwd", "lampa_hgdn_fwd_scatter", "lampa_hgdn_final_state", "lampa_hgdn_prefill",
            "lampa_hgdn_step", "lampa_hgdn_step_counted", "lampa_lsh_hash", "lampa_segsort_workspace_bytes",
-           "lampa_segsort_stable", "lampa_permute_rows", "lampa_invert_perm", "lampa_segsort_stable_static",
+           "lampa_segsort_stable", "lampa_lsh_ordering_workspace_bytes", "lampa_lsh_ordering",
+           "lampa_permute_rows", "lampa_invert_perm", "lampa_segsort_stable_static",
            "lampa_short_conv_fwd", "lampa_short_conv_step", "lampa_gate_inputs", "lampa_rmsnorm_gate", "lampa_add_rmsnorm",
            "lampa_row_range", "lampa_quantile_regions", "lampa_geo_keys",
            "lampa_bucket_rbf_attn", "lampa_bucket_attn_combine", "lampa_hept_prep_qk",
@@ -70,6 +71,8 @@ def lib() -> ctypes.CDLL:
         L.lampa_segsort_workspace_bytes.argtypes = [i64, ctypes.POINTER(sz)]
         L.lampa_segsort_stable.argtypes = [vp, i32, i64, vp, i32, vp, vp, vp, sz, vp, vp]
         L.lampa_segsort_stable_static.argtypes = [vp, i32, i64, vp, i32, vp, vp, vp, vp]
+        L.lampa_lsh_ordering_workspace_bytes.argtypes = [i32, i64, ctypes.POINTER(sz)]
+        L.lampa_lsh_ordering.argtypes = [vp, vp, i32, i32, vp, i64, i32, i64, vp, vp, vp, sz, vp, vp]
         L.lampa_permute_rows.argtypes = [vp, vp, vp, i32, i64, i64, i32, vp, vp, vp]
         L.lampa_invert_perm.argtypes = [vp, vp, i32, i64, vp, vp, vp]
         L.lampa_row_range.argtypes = [vp, vp, i32, i64, vp, vp, vp, vp]

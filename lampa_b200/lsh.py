@@ -197,17 +197,22 @@ class LSHOrdering(nn.Module):
         expo = torch.tensor([2.0 ** i for i in range(self.num_hashes)], device=coords.device)
         return (proj[:, 0, :] * expo[:, None]).sum(0).view(B, Ln)
 
-    @torch.no_grad()
     def forward(self, points: torch.Tensor, coords: torch.Tensor = None) -> Tuple[torch.Tensor, torch.Tensor]:
+        alpha = self.e2lsh.alpha
+        r = L.native.ordering(points, points if coords is None else coords, alpha)
+        if r is not None:
+            return r
         B, Ln, D = points.shape
         c = points if coords is None else coords
-        c = c.to(torch.float32)
-        keys = self.bucket_keys(c)
-        norm = c.norm(dim=-1)
-        norm_idx = segmented_sort(norm, nseg=B)
-        idx = segmented_sort(keys, nseg=B, init=norm_idx).view(B, Ln)
-        ordered = permute_rows(points.reshape(B * Ln, D), idx.view(-1), nseg=B).view(B, Ln, D)
-        return ordered, idx
+        L.require_cuda(points, c, alpha)
+        if points.numel() == 0:
+            return points.contiguous(), torch.empty(B, Ln, dtype=torch.int64, device=points.device)
+        if D * points.element_size() % 4:
+            raise ValueError("row size must be a multiple of 4 bytes")
+        if c.shape[:2] != points.shape[:2] or c.shape[2] != alpha.shape[1]:
+            raise ValueError("coords must be [B, L, C] with the C coordinates the layer was built for")
+        return L.native.ordering(points.detach().contiguous(), c.detach().to(torch.float32).contiguous(),
+                                 alpha.detach().to(torch.float32).contiguous())
 
 
 def lsh_bucket_sort(x: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, w: float = 1.0,

@@ -130,3 +130,20 @@ def test_reference_named_ops_against_golden(lb, golden_dir):
     np.testing.assert_array_equal(to_np(back), z["unsorted"])
     qh, kh, shift = lb.lsh_mapping(ordering.e2lsh, coords.reshape(1, B * Ln, C), coords.reshape(1, B * Ln, C))
     assert shift.shape == (3, 1, 1) and torch.equal(qh, kh)
+
+
+@pytest.mark.parametrize("B,n,C,D,nh", [(1, 1, 6, 3, 3), (2, 31, 3, 48, 3), (3, 33, 6, 5, 1), (1, 4097, 6, 24, 3),
+                                        (2, 8192, 4, 4, 6), (1, 8193, 6, 7, 3)])
+def test_ordering_layer_sizes(lb, B, n, C, D, nh):
+    """Both ways of ordering (counting, two radix sorts) at the edges of their ranges, with many equal points."""
+    rng = np.random.default_rng(n + C)
+    coords = rng.integers(-50, 51, (B, n, C)).astype(np.float32)  # exact sums in any order, equal keys
+    coords[:, n // 2:] = coords[:, :n - n // 2][:, ::-1]          # every second point again
+    points = torch.from_numpy(rng.standard_normal((B, n, D)).astype(np.float32))
+    layer = lb.LSHOrdering(C, num_hashes=nh).cuda()
+    layer.e2lsh.alpha.data.mul_(8).round_().div_(8)
+    ordered, idx = layer(points.cuda(), torch.from_numpy(coords).cuda())
+    alpha = to_np(layer.e2lsh.alpha)
+    for b in range(B):
+        np.testing.assert_array_equal(to_np(idx)[b], oracle.lsh_ordering(coords[b], alpha))
+    assert torch.equal(ordered.cpu(), points[torch.arange(B)[:, None], idx.cpu()])
