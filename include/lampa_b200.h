@@ -112,6 +112,13 @@ int lampa_hgdn_fwd(const lampa_gdn_desc* d, const void* q, const void* k, const 
                    const void* g, const void* beta, const void* lam, const int64_t* cu_seqlens,
                    void* o, void* ws, size_t ws_bytes, int32_t* status, void* stream);
 /*
+ * The same forward for a call whose descriptor, cu_seqlens and workspace are those of the previous lampa_hgdn_fwd on this
+ * workspace: its offset tables are used again (the layers of a model run the same packed batch one after the other).
+ */
+int lampa_hgdn_fwd_again(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
+                         const void* g, const void* beta, const void* lam, const int64_t* cu_seqlens,
+                         void* o, void* ws, size_t ws_bytes, int32_t* status, void* stream);
+/*
  * The same forward with the un-ordering of a sorted event folded into the output store.
  * Replaces: the mixer call followed by the gather with the inverse permutation that puts the rows of a sorted event
  * back in hit order (models/baselines/hmamba.py:451-455), without the second pass over o.
@@ -449,6 +456,44 @@ int lampa_debug_force_mma_sync(int on);
  * stay allocated while it is set.
  */
 int lampa_debug_set_tick_buffer(long long* ticks, int n_ctas);
+
+/*
+ * The dense half of a model block around the mixer, for d_model = 128, 4-tap short convolutions without bias, bf16 weights
+ * (matrices [out][in]) and heads with H * K = H * V = 128; LAMPA_ERR_UNSUPPORTED for anything else (the caller then
+ * composes the block from the other entry points).  `perm` int64 [n]: the block's order, local to each event of `cu`.
+ * Replaces, per block: models/hattention/modeling_gated_deltaproduct.py:1169-1199 and
+ * modeling_h_gated_deltanet.py:395-487 without the mixer call, with the ordering of models/baselines/hmamba.py:428-455.
+ */
+typedef struct lampa_model_mixer {
+    const void *q_w, *k_w, *v_w, *g_w;          /* [128][128] */
+    const void *a_w, *b_w;                      /* [H][128] */
+    const void *l_w;                            /* [H * L][128] */
+    const void *q_conv, *k_conv, *v_conv;       /* [128][4] */
+    const float *A_log, *dt_bias, *Lw;          /* [H], [H], [H * L] */
+    int32_t H, L;
+} lampa_model_mixer;
+typedef struct lampa_model_update_w {
+    const void *o_norm_w, *o_w;                 /* [head_dim] or NULL; [128][128] */
+    const void *up_w, *up_b, *down_w, *down_b;  /* [512][128], [512] or NULL, [128][512], [128] or NULL */
+    const float *mlp_norm_w, *next_norm_w;      /* [128]; NULL: no norm behind the block */
+    float o_eps, eps, next_eps;
+    int32_t head_dim;
+} lampa_model_update_w;
+/* x = W (hits * scale) + b [n][128] fp32, hs = rms_norm(x) * norm_w [n][128] bf16 (in_dim must be 24) */
+int lampa_model_encode(const float* hits, const float* scale, const float* weight, const float* bias, const float* norm_w,
+                       float eps, int64_t n, int32_t in_dim, int32_t d_model, float* x, void* hs, void* stream);
+/* hs rows gathered into the block's order -> q, k, v (convolved), gate [n][128] bf16, g, beta [n][H] fp32, lam [n][H][L] bf16 */
+int lampa_model_project(const lampa_model_mixer* w, const void* hs, const int64_t* perm, const int64_t* cu, int32_t nseq,
+                        int64_t n, void* q, void* k, void* v, void* gate, float* g, float* beta, void* lam,
+                        int32_t* status, void* stream);
+/* mixer output o and gate (ordered rows) -> residual stream x (hit rows, in place), next block's normed rows hs (hit rows) */
+int lampa_model_update(const lampa_model_update_w* w, const void* o, const void* gate, float* x, const int64_t* perm,
+                       const int64_t* cu, int32_t nseq, int64_t n, void* hs, int32_t* status, void* stream);
+/* out = x W^T + b [n][24] */
+int lampa_model_head(const float* x, const float* weight, const float* bias, int64_t n, int32_t d_model, int32_t out_dim,
+                     float* out, void* stream);
+/* segment offsets of `rounds` copies of a packed batch behind one another, int64 [rounds * nseq + 1] */
+int lampa_repeat_segments(const int64_t* cu, int32_t nseq, int32_t rounds, int64_t n, int64_t* out, void* stream);
 
 #ifdef __cplusplus
 }

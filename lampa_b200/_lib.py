@@ -42,7 +42,8 @@ EXPORTS = ["lampa_version", "lampa_error_string", "lampa_gdn_workspace_bytes", "
            "lampa_short_conv_fwd", "lampa_short_conv_step", "lampa_gate_inputs", "lampa_rmsnorm_gate", "lampa_add_rmsnorm",
            "lampa_row_range", "lampa_quantile_regions", "lampa_geo_keys",
            "lampa_bucket_rbf_attn", "lampa_bucket_attn_combine", "lampa_hept_prep_qk",
-           "lampa_profile_enable",
+           "lampa_hgdn_fwd_again", "lampa_model_encode", "lampa_model_project", "lampa_model_update", "lampa_model_head",
+           "lampa_repeat_segments", "lampa_profile_enable",
            "lampa_profile_read", "lampa_debug_set_poll_budget", "lampa_debug_set_tick_buffer",
            "lampa_debug_force_mma_sync"]
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/lampa_b200.h"
 
 namespace lampa {
@@ -206,6 +208,18 @@ __device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t by
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+
+// Opt-in to `bytes` of dynamic shared memory for a kernel, once per device (`ready`: one bit per device, static at the call).
+template <typename K>
+inline bool allow_smem(std::atomic<uint64_t>& ready, K kernel, int bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (bit && (ready.load(std::memory_order_relaxed) & bit)) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    ready.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+}
 
 // ---- sequence plan (device ints, built once per call from cu_seqlens) ---------------------------
 struct SeqPlan {

@@ -107,7 +107,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
 int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const void* v, const void* g,
         const void* beta, const void* lam, const float* h0, const int64_t* cu, void* o, float* ht,
         void* ws, size_t ws_bytes, int32_t* status, void* stream, const int64_t* out_perm = nullptr,
-        int64_t out_perm_rows = 0, int fixed_stride = 0) {
+        int64_t out_perm_rows = 0, int fixed_stride = 0, bool planned = false) {
     Layout l;
     int rc = make_layout(d, hier, l);
     if (rc != LAMPA_OK) return rc;
@@ -133,7 +133,9 @@ int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const 
     p.chunk_off = (int32_t*)a.chunk_off;
     p.block_off = (int32_t*)a.block_off;
     p.status = status;
-    if (cu) {
+    if (cu && planned) {
+        // the tables of the previous call
+    } else if (cu) {
         rc = launch_plan(p, st);
         if (rc != LAMPA_OK) return rc;
     } else {
@@ -229,6 +231,12 @@ extern "C" int lampa_hgdn_fwd(const lampa_gdn_desc* d, const void* q, const void
                               const void* g, const void* beta, const void* lam, const int64_t* cu_seqlens,
                               void* o, void* ws, size_t ws_bytes, int32_t* status, void* stream) {
     return run(d, true, q, k, v, g, beta, lam, nullptr, cu_seqlens, o, nullptr, ws, ws_bytes, status, stream);
+}
+
+extern "C" int lampa_hgdn_fwd_again(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
+                                    const void* g, const void* beta, const void* lam, const int64_t* cu_seqlens,
+                                    void* o, void* ws, size_t ws_bytes, int32_t* status, void* stream) {
+    return run(d, true, q, k, v, g, beta, lam, nullptr, cu_seqlens, o, nullptr, ws, ws_bytes, status, stream, nullptr, 0, 0, true);
 }
 
 extern "C" int lampa_hgdn_fwd_scatter(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,

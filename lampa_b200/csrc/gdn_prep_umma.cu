@@ -29,14 +29,13 @@
 // Replaces the per-chunk Triton kernels of the reference's forward:
 // fla_future/chunk_scaled_dot_kkt.py:14-74, solve_tril.py:221-276, fla_future/wy_fast.py:135-198,
 // chunkwise_hgdn.py:40-125 (intra-chunk output), fla_future/chunk_delta_h.py:384-462.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cstdlib>
 
 #include "gdn.cuh"
 #include "gdn_inv.cuh"
 #include "gdn_load.cuh"
 #include "profile.cuh"
+#include "tmap.cuh"
 #include "umma.cuh"
 
 namespace lampa {
@@ -61,16 +60,6 @@ inline int prep_umma_smem(int L, int lam_tma_bytes) {
     return S_LAM + (lam_tma_bytes > staged ? lam_tma_bytes : staged);
 }
 
-// 2-D tiled TMA load of one box into shared memory, completion on an mbarrier; x = innermost coordinate
-// (elements; x * element size must be a multiple of 16 bytes), y = row.  Single CTA, no multicast.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int32_t x, int32_t y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                 :: "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t x, int32_t y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n"
-                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
-}
 // tensor-memory columns (256 allocated): three 64-column accumulators and two 32-column A operands
 constexpr int T0 = 0, T1 = 64, T2 = 128, TA_P = 192, TA_R = 224;
 // one mbarrier per group of products issued together (commits complete in issue order, so the group's last one covers it)
@@ -567,33 +556,6 @@ __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, 
 
 }  // namespace
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
-static PFN_cuTensorMapEncodeTiled tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
-    }();
-    return fn;
-}
-
-// [rows][cols] 2-byte tensor, row pitch = cols elements, box of 64 rows x box_cols columns
-static bool make_map(CUtensorMap* m, const void* base, int dt, uint64_t rows, uint64_t cols, uint32_t box_cols, bool swizzle) {
-    PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * 2};
-    const cuuint32_t box[2] = {box_cols, (cuuint32_t)CHUNK};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(m, dt == LAMPA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base),
-               dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     if (a.qkv_dt == LAMPA_F32) return LAMPA_ERR_UNSUPPORTED;
     const uint64_t tokens = (uint64_t)a.total_tokens;
@@ -603,12 +565,12 @@ int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     const int smem = prep_umma_smem(hier ? a.L : 0, lam_tma ? lam_tile : 0);
     if (smem > 113 * 1024) return LAMPA_ERR_UNSUPPORTED;
     CUtensorMap tq, tk, tv, tl;
-    if (!make_map(&tq, a.q, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, true) ||
-        !make_map(&tk, a.k, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, true) ||
-        !make_map(&tv, a.v, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, true))
+    if (!make_map(&tq, a.q, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, CHUNK, true) ||
+        !make_map(&tk, a.k, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, CHUNK, true) ||
+        !make_map(&tv, a.v, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, CHUNK, true))
         return LAMPA_ERR_UNSUPPORTED;
     tl = tq;
-    if (lam_tma && !make_map(&tl, a.lam, a.lam_dt, tokens, (uint64_t)a.H * a.L, (uint32_t)(a.H * a.L), false)) return LAMPA_ERR_UNSUPPORTED;
+    if (lam_tma && !make_map(&tl, a.lam, a.lam_dt, tokens, (uint64_t)a.H * a.L, (uint32_t)(a.H * a.L), CHUNK, false)) return LAMPA_ERR_UNSUPPORTED;
     dim3 grid((a.H + 1) / 2, a.nc_max);
     ProfScope prof(hier ? "gdn_prep_hier" : "gdn_prep_plain", st);
     static const int nc = [] { const char* e = getenv("LAMPA_B200_PREP_COLS"); return (e && atoi(e) == 32) ? 32 : 16; }();

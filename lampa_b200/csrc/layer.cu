@@ -6,6 +6,7 @@
 // Reference: models/hattention/short_convolution.py (ShortConvolution.forward / step, kernels at
 // 39-112, 203-253, 484-502), models/hattention/modeling_h_gated_deltanet.py:151-166, 429-437,
 // models/hattention/fused_norm.py:40-112 (FusedRMSNormGated).
+#include "act.cuh"
 #include "common.cuh"
 #include "profile.cuh"
 #include <algorithm>
@@ -53,16 +54,6 @@ __device__ __forceinline__ void store_vec(void* p, size_t elem, const float (&x)
         u = *reinterpret_cast<const uint4*>(h);
     }
     *reinterpret_cast<uint4*>((char*)p + elem * (DT == LAMPA_F32 ? 4 : 2)) = u;
-}
-
-__device__ __forceinline__ float sigmoidf_(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-// log(1 + e^x) as max(x, 0) + log1p(e^-|x|); the log1p is the hardware log above 0.01 (absolute
-// error 2e-7) and its cubic Taylor polynomial below.  torch switches to x above 20, where the
-// two agree to fp32 rounding.
-__device__ __forceinline__ float softplusf_(float x) {
-    const float e = __expf(-fabsf(x));
-    const float l = e > 0.01f ? __logf(1.f + e) : e * (1.f - e * (0.5f - e * (1.f / 3.f)));
-    return fmaxf(x, 0.f) + l;
 }
 
 // Four channels of one token: 8 bytes of bf16 / fp16, 16 bytes of fp32.

@@ -1,0 +1,795 @@
+// The dense half of one model block around the hierarchical mixer, for d_model = 128 and bf16 layers: everything a block
+// does per row besides the mixer itself, in two kernels, so that no projection, hidden layer or norm makes a round trip
+// through HBM of its own.
+//
+//   project   gather the normed rows into the block's LSH order -> q, k, v, gate, a, b, l projections -> short causal
+//             convolutions + SiLU on q, k, v; g, beta, lambda from a, b, l     (modeling_h_gated_deltanet.py:395-450)
+//   update    gated norm of the mixer output -> o_proj -> residual add at the hit's row -> RMS norm -> MLP (up, GELU,
+//             down) -> residual add -> the next block's RMS norm               (481-487; modeling_gated_deltaproduct.py:
+//             1169-1199; the ordering around it: models/baselines/hmamba.py:428-455)
+//   encode    input scaling, first Linear and the first block's norm;  head: last Linear (both fp32, on CUDA cores)
+//
+// As separate library calls a block moved each row about 14 KB through HBM (projections, convolutions, gates, norms,
+// hidden layer, GELU, three residual passes): 5.3 ms per block for 2.05 M rows.  Here a row costs 1.4 KB in `project`
+// and 1.8 KB in `update`.  Both run two CTAs per SM: a CTA alternates between tensor-core products and epilogues that
+// cannot overlap inside one tile, and the other CTA fills the gaps.  Weights stream from L2 through a ring of 16 KB
+// stages (they do not fit beside the tiles at two CTAs per SM).
+#include "act.cuh"
+#include "common.cuh"
+#include "profile.cuh"
+#include "tmap.cuh"
+#include "umma.cuh"
+
+namespace lampa {
+
+namespace {
+
+constexpr int MD = 128;                      // model width
+constexpr int MST = 16384;                   // one weight stage: [128][64] or two [64][64] bf16 tiles, 128-byte swizzle
+constexpr int MNST = 3;
+constexpr int MWARPS = 8;                    // epilogue warps
+
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
+
+// Row r of the residual stream that position j of an ordered batch stands for (perm is local to j's event); -1 when the
+// permutation leaves the event.
+__device__ __forceinline__ int64_t ordered_row(const int64_t* __restrict__ cu, int nseq, const int64_t* __restrict__ perm,
+                                               int64_t j, int32_t* status, bool* first = nullptr) {
+    int lo = 0, hi = nseq;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(cu + mid) <= j) lo = mid; else hi = mid;
+    }
+    const int64_t s0 = __ldg(cu + lo), p = __ldg(perm + j);
+    if (first) *first = j == s0;
+    if ((uint64_t)p >= (uint64_t)(__ldg(cu + lo + 1) - s0)) {
+        set_status(status, LAMPA_ERR_BOUNDS, 40, (int)j);
+        return -1;
+    }
+    return s0 + p;
+}
+
+// bf16 element address inside a [rows][128] operand held as two swizzled [rows][64] halves of `half_bytes`
+__device__ __forceinline__ uint32_t op_off(int row, int col, int half_bytes) {
+    return (uint32_t)((col >> 6) * half_bytes + row * 128 + ((((col >> 3) & 7) ^ (row & 7)) << 4) + (col & 7) * 2);
+}
+
+}  // namespace
+
+// -------------------------------------------------------------------------------------------------
+// encode: x = W (hits * scale) + b, hs = rms_norm(x) w.  A lane keeps its 4 output columns of W in
+// registers, a warp takes 8 rows at a time through shared memory; 864 bytes per row move.
+// -------------------------------------------------------------------------------------------------
+constexpr int ENC_IN = 24;
+
+__global__ void __launch_bounds__(256) model_encode_kernel(const float* __restrict__ hits, const float* __restrict__ scale,
+                                                           const float* __restrict__ W, const float* __restrict__ bias,
+                                                           const float* __restrict__ nw, float eps, int64_t n,
+                                                           float* __restrict__ x, __nv_bfloat16* __restrict__ hs) {
+    __shared__ __align__(16) float rows[8][8 * ENC_IN];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float w[4][ENC_IN], b[4], g[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int i = 0; i < ENC_IN; ++i) w[c][i] = __ldg(W + (4 * lane + c) * ENC_IN + i);
+        b[c] = bias ? __ldg(bias + 4 * lane + c) : 0.f;
+        g[c] = __ldg(nw + 4 * lane + c);
+    }
+    float sc[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) sc[i] = __ldg(scale + (lane + 32 * i) % ENC_IN);
+    for (int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 8; r0 < n; r0 += (int64_t)gridDim.x * 64) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const int e = lane + 32 * i;
+            if (r0 + e / ENC_IN < n) rows[warp][e] = __ldg(hits + r0 * ENC_IN + e) * sc[i];
+        }
+        __syncwarp();
+        for (int r = 0; r < 8 && r0 + r < n; ++r) {
+            float y[4] = {b[0], b[1], b[2], b[3]};
+#pragma unroll
+            for (int i = 0; i < ENC_IN; i += 4) {
+                const float4 h = *reinterpret_cast<const float4*>(&rows[warp][r * ENC_IN + i]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    y[c] = fmaf(h.w, w[c][i + 3], fmaf(h.z, w[c][i + 2], fmaf(h.y, w[c][i + 1], fmaf(h.x, w[c][i], y[c]))));
+            }
+            float ss = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float rstd = 1.f / sqrtf(ss * (1.f / MD) + eps);
+            *reinterpret_cast<float4*>(x + (r0 + r) * MD + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
+            *reinterpret_cast<uint2*>(hs + (r0 + r) * MD + 4 * lane) =
+                make_uint2(pack_bf16x2(y[0] * rstd * g[0], y[1] * rstd * g[1]), pack_bf16x2(y[2] * rstd * g[2], y[3] * rstd * g[3]));
+        }
+    }
+}
+
+// -------------------------------------------------------------------------------------------------
+// head: out = x W^T + b, 24 outputs.  64 rows per CTA through shared memory; thread = (row, 6 outputs).
+// -------------------------------------------------------------------------------------------------
+constexpr int HEAD_OUT = 24, HEAD_PITCH = MD + 4;
+
+__global__ void __launch_bounds__(256) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
+                                                         const float* __restrict__ bias, int64_t n, float* __restrict__ out) {
+    __shared__ __align__(16) float sx[64 * HEAD_PITCH];
+    __shared__ __align__(16) float sw[HEAD_OUT * MD];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < HEAD_OUT * MD / 4; i += 256) reinterpret_cast<float4*>(sw)[i] = __ldg(reinterpret_cast<const float4*>(W) + i);
+    const int og = (tid & 3) * 6, row = tid >> 2;
+    float b[6];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) b[o] = bias ? __ldg(bias + og + o) : 0.f;
+    for (int64_t r0 = (int64_t)blockIdx.x * 64; r0 < n; r0 += (int64_t)gridDim.x * 64) {
+        __syncthreads();
+        const int m = (int)min((int64_t)64, n - r0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = tid + 256 * i, r = e >> 5, c = e & 31;
+            if (r < m) *reinterpret_cast<float4*>(sx + r * HEAD_PITCH + 4 * c) = __ldg(reinterpret_cast<const float4*>(x + (r0 + r) * MD) + c);
+        }
+        __syncthreads();
+        float y[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+        for (int c = 0; c < MD; c += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(sx + row * HEAD_PITCH + c);
+#pragma unroll
+            for (int o = 0; o < 6; ++o) {
+                const float4 w = *reinterpret_cast<const float4*>(sw + (og + o) * MD + c);
+                y[o] = fmaf(v.w, w.w, fmaf(v.z, w.z, fmaf(v.y, w.y, fmaf(v.x, w.x, y[o]))));
+            }
+        }
+        if (row < m)
+#pragma unroll
+            for (int o = 0; o < 6; o += 2)
+                *reinterpret_cast<float2*>(out + (r0 + row) * HEAD_OUT + og + o) = make_float2(y[o] + b[o], y[o + 1] + b[o + 1]);
+    }
+}
+
+// -------------------------------------------------------------------------------------------------
+// project.  A tile is 112 positions of the ordered batch with the 8 before them.  The products are
+// taken transposed, D[channel][position] = W x hs^T: a thread then owns one channel (tensor-memory
+// lane) and 56 consecutive positions in registers, which makes the 4-tap convolution a register
+// window.  Five blocks of 128 channels: q, k, v, gate, (a | b | l).  Results pass through a
+// [position][channel] tile in shared memory and leave as one bulk store per block (the rows of a
+// tile are contiguous in every output).
+// -------------------------------------------------------------------------------------------------
+constexpr int PJ_OUT = 112, PJ_ROWS = 128, PJ_HALO = 16;       // positions per tile; operand rows; the first output row
+constexpr int PJ_B = 2048;                                     // two swizzled [128][64] halves
+constexpr int PJ_W = PJ_B + 2 * MST;
+constexpr int PJ_ST = PJ_W + MNST * MST;                       // [112][128] bf16
+constexpr int PJ_SMEM = PJ_ST + PJ_OUT * MD * 2;
+constexpr int PJ_THREADS = (MWARPS + 1) * 32;
+constexpr int PJ_BLOCKS = 5;
+constexpr int PJ_ROW_B = 8, PJ_ROW_L = 16;                     // first weight row of b and l in the last block
+
+struct ProjArgs {
+    const __nv_bfloat16* hs; const int64_t* perm; const int64_t* cu; int nseq; int64_t n;
+    const __nv_bfloat16* conv[3];            // [128][4]
+    const float* A_log; const float* dt_bias; const float* Lw;
+    int H, L;
+    __nv_bfloat16* out[4];                   // q, k, v, gate [n][128]
+    float* g; float* beta; __nv_bfloat16* lam;   // [n][H], [n][H], [n][H * L]
+    int32_t* status; int budget;
+};
+
+__global__ void __launch_bounds__(PJ_THREADS, 2)
+model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
+                     const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg,
+                     const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
+                     const __grid_constant__ CUtensorMap ml) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);        // weight piece landed
+    uint64_t* mdone = full + MNST;                             // products of a block complete, by accumulator
+    uint64_t* dfree = mdone + 2;                               // accumulator read
+    uint64_t* bready = dfree + 2;                              // operand rows in place
+    uint64_t* drain = bready + 1;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 128);
+    uint32_t* sstart = reinterpret_cast<uint32_t*>(smem + 144);   // bit p: operand row p opens an event
+    int64_t* srow = reinterpret_cast<int64_t*>(smem + 1024);
+    unsigned char* sB = smem + PJ_B;
+    unsigned char* sW = smem + PJ_W;
+    unsigned char* sST = smem + PJ_ST;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t ntiles = (a.n + PJ_OUT - 1) / PJ_OUT;
+    const int mine = blockIdx.x < ntiles ? (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+
+    if (tid == 0) {
+        for (int s = 0; s < MNST; ++s) mbar_init(full + s, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(mdone + s, 1); mbar_init(dfree + s, MWARPS); }
+        mbar_init(bready, MWARPS);
+        mbar_init(drain, 1);
+        fence_mbar_init();
+    }
+    if (warp == 0) tmem_alloc(tslot, 256);
+    // operand rows before the halo are never written and never read back, but their products are formed: finite zeros
+    for (int i = tid; i < 2 * 8 * 8; i += PJ_THREADS)
+        *reinterpret_cast<uint4*>(sB + (i >> 6) * MST + (i & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t taddr = *tslot;
+    bool dead = false;
+
+    if (warp == MWARPS) {
+        if (lane == 0) {
+            const int npieces = mine * PJ_BLOCKS * 2;
+            int loaded = 0, landed = 0;
+            auto load = [&](int p) {                             // piece p: block (p / 2) % 5, half p & 1 of its 128 inputs
+                uint64_t* b = full + p % MNST;
+                unsigned char* dst = sW + (size_t)(p % MNST) * MST;
+                const int blk = (p >> 1) % PJ_BLOCKS, x = (p & 1) * 64;
+                if (blk < 4) {
+                    mbar_expect_tx(b, MST);
+                    tma_load_2d(dst, blk == 0 ? &mq : blk == 1 ? &mk : blk == 2 ? &mv : &mg, x, 0, b);
+                } else {
+                    mbar_expect_tx(b, (uint32_t)(2 * a.H + a.H * a.L) * 128);
+                    tma_load_2d(dst, &ma, x, 0, b);
+                    tma_load_2d(dst + PJ_ROW_B * 128, &mb, x, 0, b);
+                    tma_load_2d(dst + PJ_ROW_L * 128, &ml, x, 0, b);
+                }
+                loaded = p + 1;
+            };
+            for (int p = 0; p < MNST && p < npieces; ++p) load(p);
+            for (int t = 0; t < mine && !dead; ++t) {
+                mbar_wait(bready, (uint32_t)(t & 1), dead, a.status, 600, a.budget);
+                for (int m = 0; m < PJ_BLOCKS && !dead; ++m) {
+                    const int q = t * PJ_BLOCKS + m, buf = q & 1;
+                    if (q >= 2) mbar_wait(dfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 601, a.budget);
+                    for (int h = 0; h < 2 && !dead; ++h) {
+                        const int p = 2 * q + h;
+                        if (mbar_wait(full + p % MNST, (uint32_t)((p / MNST) & 1), dead, a.status, 602, a.budget)) landed = p + 1;
+                        if (dead) break;
+                        tc_fence_after();
+                        const uint64_t da = umma_desc_k128(smem_u32(sW + (size_t)(p % MNST) * MST));
+                        const uint64_t db = umma_desc_k128(smem_u32(sB + h * MST));
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umma_f16_ss(taddr + 128 * buf, da + 2 * kk, db + 2 * kk, umma_idesc(128, 128), h | kk ? 1u : 0u);
+                    }
+                    if (dead) break;
+                    umma_commit(mdone + buf);
+                    // the two stages of this block are free once its products are done
+                    mbar_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 603, a.budget);
+                    for (int p = 2 * q + MNST; p < 2 * q + MNST + 2 && p < npieces && !dead; ++p) load(p);
+                }
+            }
+            for (int p = landed; p < loaded; ++p) mbar_drain(full + p % MNST, (uint32_t)((p / MNST) & 1));
+            umma_commit(drain);
+            mbar_drain(drain, 0u);
+        }
+    } else {
+        const int quarter = warp & 3, half = warp >> 2;          // channels 32 quarter + lane; positions 56 half ..
+        const int ch = 32 * quarter + lane;
+        const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(PJ_HALO - 8 + 56 * half);
+        float cw[3][4];
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cw[m][i] = __bfloat162float(a.conv[m][ch * 4 + i]);
+        const int HL = a.H * a.L;
+        // last block: the channel is a (g), b (beta), l (lambda) or nothing; g and lambda are scale * softplus(mul x + add)
+        const bool is_a = ch < a.H, is_b = ch >= PJ_ROW_B && ch < PJ_ROW_B + a.H, is_l = ch >= PJ_ROW_L && ch < PJ_ROW_L + HL;
+        const float sp_scale = is_a ? -__expf(__ldg(a.A_log + ch)) : 1.f, sp_add = is_a ? __ldg(a.dt_bias + ch) : 0.f;
+        const float sp_mul = is_l ? __ldg(a.Lw + ch - PJ_ROW_L) : 1.f;
+
+        for (int t = 0; t < mine; ++t) {
+            const int64_t tile = blockIdx.x + (int64_t)t * gridDim.x, j0 = tile * PJ_OUT;
+            const int nv = (int)min((int64_t)PJ_OUT, a.n - j0);
+            // ---- the tile's rows of hs, in LSH order (the previous tile's products have all been waited for) ----
+            if (warp < 4) {
+                const int64_t j = j0 - PJ_HALO + tid;            // operand row tid
+                bool first = false;
+                int64_t r = -1;
+                if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.status, &first);
+                srow[tid] = r;
+                const uint32_t bits = __ballot_sync(0xffffffffu, first);
+                if (lane == 0) sstart[warp] = bits;
+            }
+            epi_sync();
+            for (int i = tid; i < (PJ_ROWS - 8) * 16; i += 256) {
+                const int row = 8 + (i >> 4), c = i & 15;
+                const int64_t r = srow[row];
+                unsigned char* dst = sB + op_off(row, 8 * c, MST);
+                if (r >= 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(smem_u32(dst)), "l"(a.hs + r * MD + 8 * c) : "memory");
+                else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bready);
+            // event starts of this thread's 56 positions and the 8 before: bit i = position i - 8
+            const int p0 = PJ_HALO - 8 + 56 * half;
+            uint64_t starts = 0;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const int sh = 32 * w - p0;
+                const uint64_t bits = sstart[w];
+                if (sh >= 0 && sh < 64) starts |= bits << sh;
+                else if (sh < 0 && sh > -32) starts |= bits >> -sh;
+            }
+            for (int m = 0; m < PJ_BLOCKS; ++m) {
+                const int q = t * PJ_BLOCKS + m, buf = q & 1;
+                mbar_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget);
+                tc_fence_after();
+                float x[2][32];
+                tmem_ld32(x[0], tl + 128 * buf);
+                tmem_ld32(x[1], tl + 128 * buf + 32);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(dfree + buf);
+                if (tid == 0) bulk_wait_read();                  // the staging tile has left
+                epi_sync();
+                auto X = [&](int i) -> float& { return x[i >> 5][i & 31]; };
+                __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(sST) + (size_t)(56 * half) * MD + ch;
+                if (m < 3) {
+                    float h1 = X(7), h2 = X(6), h3 = X(5);
+                    const float w0 = m == 0 ? cw[0][0] : m == 1 ? cw[1][0] : cw[2][0], w1 = m == 0 ? cw[0][1] : m == 1 ? cw[1][1] : cw[2][1];
+                    const float w2 = m == 0 ? cw[0][2] : m == 1 ? cw[1][2] : cw[2][2], w3 = m == 0 ? cw[0][3] : m == 1 ? cw[1][3] : cw[2][3];
+                    if (starts == 0) {
+#pragma unroll
+                        for (int i = 0; i < 56; ++i) {
+                            const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
+                            h3 = h2; h2 = h1; h1 = X(8 + i);
+                            st[i * MD] = __float2bfloat16_rn(v * sigmoidf_(v));
+                        }
+                    } else {                                     // an event opens here: its first taps are empty
+                        if ((starts >> 7) & 1) h2 = h3 = 0.f;
+                        if ((starts >> 6) & 1) h3 = 0.f;
+#pragma unroll
+                        for (int i = 0; i < 56; ++i) {
+                            if ((starts >> (8 + i)) & 1) h1 = h2 = h3 = 0.f;
+                            const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
+                            h3 = h2; h2 = h1; h1 = X(8 + i);
+                            st[i * MD] = __float2bfloat16_rn(v * sigmoidf_(v));
+                        }
+                    }
+                } else if (m == 3) {
+#pragma unroll
+                    for (int i = 0; i < 56; ++i) st[i * MD] = __float2bfloat16_rn(X(8 + i));
+                } else if (is_a || is_l) {
+                    __nv_bfloat16* sl = reinterpret_cast<__nv_bfloat16*>(sST) + (size_t)(56 * half) * HL + ch - PJ_ROW_L;
+                    float* gp = a.g + (j0 + 56 * half) * a.H + ch;
+#pragma unroll
+                    for (int i = 0; i < 56; ++i) {
+                        const float v = sp_scale * softplusf_(fmaf(sp_mul, X(8 + i), sp_add));
+                        if (is_l) sl[i * HL] = __float2bfloat16_rn(v);
+                        else if (56 * half + i < nv) gp[i * a.H] = v;
+                    }
+                } else if (is_b) {
+                    float* bp = a.beta + (j0 + 56 * half) * a.H + ch - PJ_ROW_B;
+#pragma unroll
+                    for (int i = 0; i < 56; ++i)
+                        if (56 * half + i < nv) bp[i * a.H] = sigmoidf_(X(8 + i));
+                }
+                fence_async_smem();
+                epi_sync();
+                const uint32_t bytes = (uint32_t)nv * (m < 4 ? MD : HL) * 2;
+                char* dst = m < 4 ? (char*)(m == 0 ? a.out[0] : m == 1 ? a.out[1] : m == 2 ? a.out[2] : a.out[3]) + j0 * MD * 2 : (char*)a.lam + j0 * HL * 2;
+                if (bytes % 16 == 0) {
+                    if (tid == 0) { bulk_s2g(dst, sST, bytes); bulk_commit(); }
+                } else {                                         // last rows of lambda: not whole 16-byte pieces
+                    for (int i = tid; i < nv * HL; i += 256) a.lam[j0 * HL + i] = reinterpret_cast<const __nv_bfloat16*>(sST)[i];
+                }
+            }
+        }
+        if (tid == 0) bulk_wait_read();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(taddr, 256);
+}
+
+// -------------------------------------------------------------------------------------------------
+// update.  A tile is 128 positions of the ordered batch.  Row-wise steps (gated norm, residual and
+// norm) give a warp 16 rows, four columns per lane; products leave tensor memory one row per lane and
+// go through the operand tile (bf16) to the row-wise layout.  The hidden layer never leaves the SM:
+// eight chunks of 64 hidden units, each up product -> bias, GELU -> bf16 operand -> accumulated into
+// the down product, the up product of the next chunk under the GELU of this one.
+// Bound by the epilogues' instruction issue (the GELU alone is 65 k elements per tile), not by HBM.
+// -------------------------------------------------------------------------------------------------
+constexpr int UP_ROWS = 128, UP_HID = 512, UP_CH = 64, UP_NCH = UP_HID / UP_CH;
+constexpr int UP_A = 1024;                                     // operand tile: two swizzled [128][64] halves
+constexpr int UP_H = UP_A + 2 * MST;                           // hidden operand, two buffers of [128][64]
+constexpr int UP_W = UP_H + 2 * MST;
+constexpr int UP_SMEM = UP_W + MNST * MST;                     // 113 KB: two CTAs fill an SM exactly
+constexpr int UP_THREADS = (MWARPS + 2) * 32;                  // + one warp issues products, one streams weights
+constexpr int UP_PIECES = 2 + 2 * UP_NCH;                      // o_proj halves, then up and down of every chunk
+constexpr int UT_UP = 0, UT_ACC = 128;                         // tensor-memory columns: two 64-column up accumulators; o_proj / down
+
+struct UpdateArgs {
+    const __nv_bfloat16* o; const __nv_bfloat16* gate; const __nv_bfloat16* o_norm_w; int head_dim;
+    float* x; const int64_t* perm; const int64_t* cu; int nseq; int64_t n;
+    const float* mlp_norm_w; const __nv_bfloat16* up_b; const __nv_bfloat16* down_b;
+    const float* next_norm_w; __nv_bfloat16* hs;             // NULL: last block, no norm behind it
+    float eps, next_eps, o_eps;
+    int32_t* status; int budget;
+};
+
+__global__ void __launch_bounds__(UP_THREADS, 2)
+model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const __grid_constant__ CUtensorMap mu,
+                    const __grid_constant__ CUtensorMap md) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);        // weight piece landed
+    uint64_t* wfree = full + MNST;                             // its products are done
+    uint64_t* aready = wfree + MNST;                           // operand tile written
+    uint64_t* macc = aready + 1;                               // o_proj / down complete
+    uint64_t* mup = macc + 1;                                  // up product complete, by accumulator
+    uint64_t* upfree = mup + 2;                                // up accumulator read
+    uint64_t* hready = upfree + 2;                             // hidden operand written
+    uint64_t* hfree = hready + 2;                              // hidden operand consumed
+    uint64_t* drain = hfree + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 256);
+    unsigned char* sA = smem + UP_A;
+    unsigned char* sH = smem + UP_H;
+    unsigned char* sW = smem + UP_W;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t ntiles = (a.n + UP_ROWS - 1) / UP_ROWS;
+    const int mine = blockIdx.x < ntiles ? (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+
+    if (tid == 0) {
+        for (int s = 0; s < MNST; ++s) { mbar_init(full + s, 1); mbar_init(wfree + s, 1); }
+        mbar_init(aready, MWARPS);
+        mbar_init(macc, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(mup + s, 1); mbar_init(upfree + s, MWARPS); mbar_init(hready + s, MWARPS); mbar_init(hfree + s, 1); }
+        mbar_init(drain, 1);
+        fence_mbar_init();
+    }
+    if (warp == 0) tmem_alloc(tslot, 256);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t taddr = *tslot;
+    bool dead = false;
+    const int npieces = mine * UP_PIECES;
+
+    if (warp == MWARPS + 1) {
+        // ---- weights: o_proj k-halves, then [64 hidden][128] of up and [128][64 hidden] of down, chunk by chunk ----
+        if (lane == 0) {
+            int p = 0;
+            for (; p < npieces; ++p) {
+                const int s = p % MNST, k = p % UP_PIECES;
+                if (p >= MNST && !mbar_wait(wfree + s, (uint32_t)((p / MNST - 1) & 1), dead, a.status, 620, a.budget)) break;
+                unsigned char* dst = sW + (size_t)s * MST;
+                mbar_expect_tx(full + s, MST);
+                if (k < 2) tma_load_2d(dst, &mo, 64 * k, 0, full + s);
+                else {
+                    // order of use: up 0, up 1, down 0, up 2, down 1, ..., up 7, down 6, down 7
+                    const int i = k - 2;
+                    const bool up = i == 0 || (i < 2 * UP_NCH - 1 && (i & 1));
+                    const int c = up ? (i + 1) / 2 : (i == 2 * UP_NCH - 1 ? UP_NCH - 1 : i / 2 - 1);
+                    if (up) {
+                        tma_load_2d(dst, &mu, 0, UP_CH * c, full + s);
+                        tma_load_2d(dst + MST / 2, &mu, 64, UP_CH * c, full + s);
+                    } else {
+                        tma_load_2d(dst, &md, UP_CH * c, 0, full + s);
+                    }
+                }
+            }
+            // nothing may land after the CTA has gone
+            for (int i = max(0, p - MNST); i < p; ++i) mbar_drain(full + i % MNST, (uint32_t)((i / MNST) & 1));
+        }
+    } else if (warp == MWARPS) {
+        // ---- products ----
+        if (lane == 0) {
+            int p = 0;
+            auto piece = [&]() -> uint32_t {                     // wait for the next weight piece
+                mbar_wait(full + p % MNST, (uint32_t)((p / MNST) & 1), dead, a.status, 621, a.budget);
+                tc_fence_after();
+                return smem_u32(sW + (size_t)(p % MNST) * MST);
+            };
+            for (int t = 0; t < mine && !dead; ++t) {
+                mbar_wait(aready, 0u, dead, a.status, 622, a.budget);           // two phases per tile: normed mixer rows, then normed residual rows
+                for (int h = 0; h < 2 && !dead; ++h) {
+                    const uint64_t db = umma_desc_k128(piece()), da = umma_desc_k128(smem_u32(sA + h * MST));
+                    if (dead) break;
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16_ss(taddr + UT_ACC, da + 2 * kk, db + 2 * kk, umma_idesc(128, 128), h | kk ? 1u : 0u);
+                    umma_commit(wfree + p % MNST);
+                    ++p;
+                }
+                if (dead) break;
+                umma_commit(macc);
+                mbar_wait(aready, 1u, dead, a.status, 623, a.budget);
+                auto up = [&](int c) {
+                    const int q = t * UP_NCH + c, buf = q & 1;
+                    if (q >= 2) mbar_wait(upfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 624, a.budget);
+                    const uint32_t w = piece();
+                    if (dead) return;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint64_t da = umma_desc_k128(smem_u32(sA + h * MST)), db = umma_desc_k128(w + h * (MST / 2));
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umma_f16_ss(taddr + UT_UP + 64 * buf, da + 2 * kk, db + 2 * kk, umma_idesc(128, 64), h | kk ? 1u : 0u);
+                    }
+                    umma_commit(wfree + p % MNST);
+                    umma_commit(mup + buf);
+                    ++p;
+                };
+                auto down = [&](int c) {
+                    const int q = t * UP_NCH + c, buf = q & 1;
+                    mbar_wait(hready + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 625, a.budget);
+                    const uint64_t db = umma_desc_k128(piece()), da = umma_desc_k128(smem_u32(sH + buf * MST));
+                    if (dead) return;
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16_ss(taddr + UT_ACC, da + 2 * kk, db + 2 * kk, umma_idesc(128, 128), c | kk ? 1u : 0u);
+                    umma_commit(wfree + p % MNST);
+                    umma_commit(hfree + buf);
+                    ++p;
+                };
+                up(0);
+                for (int c = 1; c < UP_NCH && !dead; ++c) { up(c); if (!dead) down(c - 1); }
+                if (!dead) down(UP_NCH - 1);
+                if (!dead) umma_commit(macc);
+            }
+            umma_commit(drain);
+            mbar_drain(drain, 0u);
+        }
+    } else {
+        const int quarter = warp & 3, half = warp >> 2;
+        const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16);
+        const int trow = 32 * quarter + lane;                    // this thread's row of an accumulator
+        const int lanes_per_head = a.head_dim >> 2;
+        float ow[4], mw[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            ow[c] = a.o_norm_w ? __bfloat162float(a.o_norm_w[(4 * lane + c) % a.head_dim]) : 1.f;
+            mw[c] = __ldg(a.mlp_norm_w + 4 * lane + c);
+        }
+        // accumulator half-row -> bf16 -> operand tile (row-wise readers pick it up there)
+        auto stage_acc = [&](const __nv_bfloat16* bias) {
+            float x[2][32];
+            tmem_ld32(x[0], tl + UT_ACC + 64 * half);
+            tmem_ld32(x[1], tl + UT_ACC + 64 * half + 32);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                float* v = &x[q >> 2][(q & 3) * 8];
+                if (bias) {
+                    const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + 64 * half) + q);
+                    const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { const float2 f = unpack_bf16x2(bw[e]); v[2 * e] += f.x; v[2 * e + 1] += f.y; }
+                }
+                *reinterpret_cast<uint4*>(sA + op_off(trow, 64 * half + 8 * q, MST)) =
+                    make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+            }
+        };
+        auto operand_ready = [&]() {
+            fence_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(aready);
+        };
+        for (int t = 0; t < mine; ++t) {
+            const int64_t j0 = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * UP_ROWS + 16 * warp;   // this warp's 16 rows
+            const int nr = (int)min((int64_t)16, max((int64_t)0, a.n - j0));
+            int64_t myrow = -1;
+            if (lane < nr) myrow = ordered_row(a.cu, a.nseq, a.perm, j0 + lane, a.status);
+            // ---- gated norm of the mixer's rows: the operand of o_proj ----
+#pragma unroll 1
+            for (int r0 = 0; r0 < 16; r0 += 4) {
+                uint2 ov[4], gv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool in = r0 + i < nr;
+                    ov[i] = in ? __ldg(reinterpret_cast<const uint2*>(a.o + (j0 + r0 + i) * MD) + lane) : make_uint2(0u, 0u);
+                    gv[i] = in ? __ldg(reinterpret_cast<const uint2*>(a.gate + (j0 + r0 + i) * MD) + lane) : make_uint2(0u, 0u);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 o0 = unpack_bf16x2(ov[i].x), o1 = unpack_bf16x2(ov[i].y), g0 = unpack_bf16x2(gv[i].x), g1 = unpack_bf16x2(gv[i].y);
+                    float ss = o0.x * o0.x + o0.y * o0.y + o1.x * o1.x + o1.y * o1.y;
+                    for (int o = lanes_per_head >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float rstd = 1.f / sqrtf(ss / (float)a.head_dim + a.o_eps);
+                    *reinterpret_cast<uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST)) =
+                        make_uint2(pack_bf16x2(o0.x * rstd * ow[0] * g0.x * sigmoidf_(g0.x), o0.y * rstd * ow[1] * g0.y * sigmoidf_(g0.y)),
+                                   pack_bf16x2(o1.x * rstd * ow[2] * g1.x * sigmoidf_(g1.x), o1.y * rstd * ow[3] * g1.y * sigmoidf_(g1.y)));
+                }
+            }
+            operand_ready();
+            // ---- x += o_proj at the hit's row, norm: the operand of the MLP ----
+            mbar_wait(macc, 0u, dead, a.status, 630, a.budget);
+            tc_fence_after();
+            stage_acc(nullptr);
+            epi_sync();
+#pragma unroll 1
+            for (int r0 = 0; r0 < 16; r0 += 8) {
+                float4 v[8];
+                int64_t rr[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    rr[i] = __shfl_sync(0xffffffffu, myrow, r0 + i);
+                    v[i] = rr[i] >= 0 ? *reinterpret_cast<const float4*>(a.x + rr[i] * MD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    uint2* op = reinterpret_cast<uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST));
+                    const float2 d0 = unpack_bf16x2(op->x), d1 = unpack_bf16x2(op->y);
+                    v[i].x += d0.x; v[i].y += d0.y; v[i].z += d1.x; v[i].w += d1.y;
+                    if (rr[i] >= 0) *reinterpret_cast<float4*>(a.x + rr[i] * MD + 4 * lane) = v[i];
+                    float ss = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float rstd = 1.f / sqrtf(ss * (1.f / MD) + a.eps);
+                    *op = make_uint2(pack_bf16x2(v[i].x * rstd * mw[0], v[i].y * rstd * mw[1]), pack_bf16x2(v[i].z * rstd * mw[2], v[i].w * rstd * mw[3]));
+                }
+            }
+            operand_ready();
+            // ---- hidden layer, 64 units at a time: this thread has 32 of its row ----
+#pragma unroll 1
+            for (int c = 0; c < UP_NCH; ++c) {
+                const int q = t * UP_NCH + c, buf = q & 1;
+                mbar_wait(mup + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 631, a.budget);
+                tc_fence_after();
+                float x[32];
+                tmem_ld32(x, tl + UT_UP + 64 * buf + 32 * half);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(upfree + buf);
+                if (a.up_b) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const uint4 b = __ldg(reinterpret_cast<const uint4*>(a.up_b + UP_CH * c + 32 * half) + e);
+                        const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(bw[k]); x[8 * e + 2 * k] += f.x; x[8 * e + 2 * k + 1] += f.y; }
+                    }
+                }
+                uint32_t w[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) w[e] = pack_bf16x2(geluf_(x[2 * e]), geluf_(x[2 * e + 1]));
+                if (q >= 2) mbar_wait(hfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 632, a.budget);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<uint4*>(sH + buf * MST + op_off(trow, 32 * half + 8 * e, 0)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(hready + buf);
+            }
+            // ---- x += MLP, the next block's norm ----
+            mbar_wait(macc, 1u, dead, a.status, 633, a.budget);
+            tc_fence_after();
+            stage_acc(a.down_b);
+            tc_fence_before();
+            epi_sync();
+#pragma unroll 1
+            for (int r0 = 0; r0 < 16; r0 += 8) {
+                float4 v[8];
+                int64_t rr[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    rr[i] = __shfl_sync(0xffffffffu, myrow, r0 + i);
+                    v[i] = rr[i] >= 0 ? *reinterpret_cast<const float4*>(a.x + rr[i] * MD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint2 op = *reinterpret_cast<const uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST));
+                    const float2 d0 = unpack_bf16x2(op.x), d1 = unpack_bf16x2(op.y);
+                    v[i].x += d0.x; v[i].y += d0.y; v[i].z += d1.x; v[i].w += d1.y;
+                    if (rr[i] < 0) continue;                     // warp-uniform
+                    *reinterpret_cast<float4*>(a.x + rr[i] * MD + 4 * lane) = v[i];
+                    if (!a.next_norm_w) continue;
+                    float ss = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float rstd = 1.f / sqrtf(ss * (1.f / MD) + a.next_eps);
+                    const float4 nw = __ldg(reinterpret_cast<const float4*>(a.next_norm_w) + lane);
+                    *reinterpret_cast<uint2*>(a.hs + rr[i] * MD + 4 * lane) =
+                        make_uint2(pack_bf16x2(v[i].x * rstd * nw.x, v[i].y * rstd * nw.y), pack_bf16x2(v[i].z * rstd * nw.z, v[i].w * rstd * nw.w));
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(taddr, 256);
+}
+
+static int sm_count() {
+    static const int sms = [] { int d = 0, n = 148; if (cudaGetDevice(&d) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d); return n; }();
+    return sms;
+}
+
+}  // namespace lampa
+
+using namespace lampa;
+
+extern "C" int lampa_model_encode(const float* hits, const float* scale, const float* weight, const float* bias,
+                                  const float* norm_w, float eps, int64_t n, int32_t in_dim, int32_t d_model, float* x,
+                                  void* hs, void* stream) {
+    if (n < 0 || !hits || !scale || !weight || !norm_w || !x || !hs) return LAMPA_ERR_ARG;
+    if (in_dim != ENC_IN || d_model != MD) return LAMPA_ERR_UNSUPPORTED;
+    if (n == 0) return LAMPA_OK;
+    ProfScope prof("model_encode", (cudaStream_t)stream);
+    const int64_t want = (n + 63) / 64, most = (int64_t)sm_count() * 4;
+    model_encode_kernel<<<(unsigned)(want < most ? want : most), 256, 0, (cudaStream_t)stream>>>(
+        hits, scale, weight, bias, norm_w, eps, n, x, (__nv_bfloat16*)hs);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+extern "C" int lampa_model_head(const float* x, const float* weight, const float* bias, int64_t n, int32_t d_model,
+                                int32_t out_dim, float* out, void* stream) {
+    if (n < 0 || !x || !weight || !out) return LAMPA_ERR_ARG;
+    if (out_dim != HEAD_OUT || d_model != MD) return LAMPA_ERR_UNSUPPORTED;
+    if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) return LAMPA_ERR_UNSUPPORTED;
+    if (n == 0) return LAMPA_OK;
+    ProfScope prof("model_head", (cudaStream_t)stream);
+    const int64_t want = (n + 63) / 64, most = (int64_t)sm_count() * 4;
+    model_head_kernel<<<(unsigned)(want < most ? want : most), 256, 0, (cudaStream_t)stream>>>(x, weight, bias, n, out);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, const int64_t* perm, const int64_t* cu, int32_t nseq,
+                                   int64_t n, void* q, void* k, void* v, void* gate, float* g, float* beta, void* lam,
+                                   int32_t* status, void* stream) {
+    if (!w || n < 0 || nseq <= 0) return LAMPA_ERR_ARG;
+    if (n == 0) return LAMPA_OK;
+    if (!hs || !perm || !cu || !q || !k || !v || !gate || !g || !beta || !lam) return LAMPA_ERR_ARG;
+    if (w->H <= 0 || w->H > PJ_ROW_L - PJ_ROW_B || w->L <= 0 || w->H * w->L > 128 - PJ_ROW_L || MD % w->H != 0) return LAMPA_ERR_UNSUPPORTED;
+    ProjArgs a;
+    a.hs = (const __nv_bfloat16*)hs; a.perm = perm; a.cu = cu; a.nseq = nseq; a.n = n;
+    a.conv[0] = (const __nv_bfloat16*)w->q_conv; a.conv[1] = (const __nv_bfloat16*)w->k_conv; a.conv[2] = (const __nv_bfloat16*)w->v_conv;
+    a.A_log = w->A_log; a.dt_bias = w->dt_bias; a.Lw = w->Lw; a.H = w->H; a.L = w->L;
+    a.out[0] = (__nv_bfloat16*)q; a.out[1] = (__nv_bfloat16*)k; a.out[2] = (__nv_bfloat16*)v; a.out[3] = (__nv_bfloat16*)gate;
+    a.g = g; a.beta = beta; a.lam = (__nv_bfloat16*)lam; a.status = status; a.budget = MBAR_POLLS;
+    for (const void* p : {w->q_w, w->k_w, w->v_w, w->g_w, w->a_w, w->b_w, w->l_w, hs, (const void*)q, (const void*)k, (const void*)v, (const void*)gate, (const void*)lam})
+        if (!p || ((uintptr_t)p & 15)) return LAMPA_ERR_UNSUPPORTED;
+    const void* mats[7] = {w->q_w, w->k_w, w->v_w, w->g_w, w->a_w, w->b_w, w->l_w};
+    const uint32_t rows[7] = {MD, MD, MD, MD, (uint32_t)w->H, (uint32_t)w->H, (uint32_t)(w->H * w->L)};
+    CUtensorMap m[7];
+    for (int i = 0; i < 7; ++i)
+        if (!make_map(&m[i], mats[i], LAMPA_BF16, rows[i], MD, 64, rows[i], true)) return LAMPA_ERR_UNSUPPORTED;
+    static std::atomic<uint64_t> ready{0};
+    if (!allow_smem(ready, model_project_kernel, PJ_SMEM)) return LAMPA_ERR_CUDA;
+    ProfScope prof("model_project", (cudaStream_t)stream);
+    const int64_t want = (n + PJ_OUT - 1) / PJ_OUT, most = (int64_t)sm_count() * 2;
+    model_project_kernel<<<(unsigned)(want < most ? want : most), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream>>>(a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+extern "C" int lampa_model_update(const lampa_model_update_w* w, const void* o, const void* gate, float* x, const int64_t* perm,
+                                  const int64_t* cu, int32_t nseq, int64_t n, void* hs, int32_t* status, void* stream) {
+    if (!w || n < 0 || nseq <= 0) return LAMPA_ERR_ARG;
+    if (n == 0) return LAMPA_OK;
+    if (!o || !gate || !x || !perm || !cu || (w->next_norm_w && !hs)) return LAMPA_ERR_ARG;
+    if (w->head_dim != 32 && w->head_dim != 64) return LAMPA_ERR_UNSUPPORTED;
+    for (const void* p : {w->o_w, w->up_w, w->down_w, o, gate, (const void*)x})
+        if (!p || ((uintptr_t)p & 15)) return LAMPA_ERR_UNSUPPORTED;
+    for (const void* p : {w->up_b, w->down_b, (const void*)w->next_norm_w, (const void*)hs})
+        if (p && ((uintptr_t)p & 15)) return LAMPA_ERR_UNSUPPORTED;
+    UpdateArgs a;
+    a.o = (const __nv_bfloat16*)o; a.gate = (const __nv_bfloat16*)gate; a.o_norm_w = (const __nv_bfloat16*)w->o_norm_w; a.head_dim = w->head_dim;
+    a.x = x; a.perm = perm; a.cu = cu; a.nseq = nseq; a.n = n;
+    a.mlp_norm_w = w->mlp_norm_w; a.up_b = (const __nv_bfloat16*)w->up_b; a.down_b = (const __nv_bfloat16*)w->down_b;
+    a.next_norm_w = w->next_norm_w; a.hs = (__nv_bfloat16*)hs;
+    a.eps = w->eps; a.next_eps = w->next_eps; a.o_eps = w->o_eps; a.status = status; a.budget = MBAR_POLLS;
+    CUtensorMap mo, mu, md;
+    if (!make_map(&mo, w->o_w, LAMPA_BF16, MD, MD, 64, MD, true) || !make_map(&mu, w->up_w, LAMPA_BF16, UP_HID, MD, 64, UP_CH, true) ||
+        !make_map(&md, w->down_w, LAMPA_BF16, MD, UP_HID, 64, MD, true))
+        return LAMPA_ERR_UNSUPPORTED;
+    static std::atomic<uint64_t> ready{0};
+    if (!allow_smem(ready, model_update_kernel, UP_SMEM)) return LAMPA_ERR_CUDA;
+    ProfScope prof("model_update", (cudaStream_t)stream);
+    const int64_t want = (n + UP_ROWS - 1) / UP_ROWS, most = (int64_t)sm_count() * 2;
+    model_update_kernel<<<(unsigned)(want < most ? want : most), UP_THREADS, UP_SMEM, (cudaStream_t)stream>>>(a, mo, mu, md);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+// Segment offsets of `rounds` copies of a packed batch behind one another: out[r * nseq + s] = r * n + cu[s], out[rounds * nseq] = rounds * n
+__global__ void model_segments_kernel(const int64_t* cu, int nseq, int rounds, int64_t n, int64_t* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < rounds * nseq) out[i] = (int64_t)(i / nseq) * n + cu[i % nseq];
+    else if (i == rounds * nseq) out[i] = (int64_t)rounds * n;
+}
+
+extern "C" int lampa_repeat_segments(const int64_t* cu, int32_t nseq, int32_t rounds, int64_t n, int64_t* out, void* stream) {
+    if (!cu || !out || nseq <= 0 || rounds <= 0) return LAMPA_ERR_ARG;
+    model_segments_kernel<<<(unsigned)((rounds * nseq) / 256 + 1), 256, 0, (cudaStream_t)stream>>>(cu, nseq, rounds, n, out);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}

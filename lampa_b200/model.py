@@ -11,8 +11,10 @@ Differences that the benchmark configuration asks for: the ordering is the integ
 mixer is the hierarchical rule with `cu_seqlens` (one hierarchy per event), the MLP is
 Linear-GELU-Linear, and a batch is many events packed back to back.
 
-Host side: torch (Linear, RMS norm, GELU, residuals).  Hashing, sorting, row movement, the
-short convolutions, gate inputs, the mixer and its gated norm run in the CUDA library.
+At d_model = 128 with bf16 blocks and heads of 32 or 64 the whole forward is one host call into the
+CUDA library: two kernels per block around the mixer (csrc/model.cu).  Other widths and modified
+blocks are composed here: torch for Linear and GELU; hashing, sorting, row movement, norms, the
+short convolutions, gate inputs, the mixer and its gated norm in the CUDA library.
 Forward only.
 """
 from __future__ import annotations
@@ -24,7 +26,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import sharding
+from . import _lib as L, sharding
 from .gated_delta import chunk_h_gated_delta_rule, num_levels_required
 from .layer import FusedRMSNormGated, ShortConvolution, add_rms_norm, gate_inputs
 from .lsh import lsh_hash, permute_rows, segmented_sort
@@ -182,9 +184,54 @@ class LSHGatedDelta(nn.Module):
         seg = torch.cat([offs, torch.full((1,), self.rounds * n, device=hits.device, dtype=torch.int64)])
         return segmented_sort(packed, seg_offsets=seg).view(self.rounds, n)
 
+    def _native_params(self):
+        """The parameters of every block in the order the native forward takes them, and the (block, output norm) eps
+        pairs; None when a block is not built the way its kernels are (custom or hooked submodules, other options)."""
+        params, eps = [], []
+        for blk in self.blocks._modules.values():
+            at = blk._modules.get("attn")
+            if type(blk) is not LSHGatedDeltaBlock or type(at) is not HGatedDeltaNet or blk.dtype != torch.bfloat16:
+                return None
+            if not (at.use_gate and at.use_short_conv and at.lambda_mode == "positive") or at._forward_hooks or at._forward_pre_hooks:
+                return None
+            am, ap, bp = at._modules, at._parameters, blk._parameters
+            lin = [am[k] for k in ("q_proj", "k_proj", "v_proj", "g_proj", "a_proj", "b_proj", "l_proj", "o_proj")]
+            mlp = [blk._modules["mlp_up"], blk._modules["mlp_down"]]
+            conv = [am[k] for k in ("q_conv1d", "k_conv1d", "v_conv1d")]
+            for m in lin + mlp + conv + [am["o_norm"]]:
+                if type(m) not in (nn.Linear, ShortConvolution, FusedRMSNormGated) or m._forward_hooks or m._forward_pre_hooks:
+                    return None
+            if any(m._parameters["bias"] is not None for m in lin):
+                return None
+            if any(c.bias is not None or c.activation is None or c.kernel_size[0] != 4 for c in conv) or am["o_norm"].activation == "sigmoid":
+                return None
+            params += [bp["attn_norm_weight"]] + [m._parameters["weight"] for m in lin[:7]] + [c._parameters["weight"] for c in conv]
+            params += [ap["A_log"], ap["dt_bias"], ap["L"], am["o_norm"]._parameters["weight"], lin[7]._parameters["weight"],
+                       bp["mlp_norm_weight"]]
+            for m in mlp:
+                params += [m._parameters["weight"], m._parameters["bias"]]
+            eps += [float(blk.eps), float(am["o_norm"].eps)]
+        return params, eps
+
+    def _native_forward(self, hits: torch.Tensor, cu: torch.Tensor):
+        """The whole forward behind one host call, for the widths the fused block kernels are built for (None otherwise)."""
+        enc, head = self._modules["encoder"], self._modules["head"]
+        if type(enc) is not nn.Linear or type(head) is not nn.Linear or enc._forward_hooks or head._forward_hooks:
+            return None
+        p = self._native_params()
+        if p is None:
+            return None
+        ep, hp = enc._parameters, head._parameters
+        top = (self._buffers["feature_scale"], ep["weight"], ep["bias"], self._parameters["lsh_alpha"],
+               self._parameters["lsh_beta"], hp["weight"], hp["bias"])
+        return L.native.model_forward(hits, cu, top, p[0], p[1], self.bucket_width)
+
     @torch.no_grad()
     def forward(self, hits: torch.Tensor, cu_seqlens: torch.Tensor) -> torch.Tensor:
         cu = cu_seqlens.to(device=hits.device, dtype=torch.int64)
+        out = self._native_forward(hits, cu) if hits.is_cuda and not torch.compiler.is_compiling() else None
+        if out is not None:
+            return out
         perms = self.orderings(hits, cu)
         x = self.encoder(hits * self.feature_scale)
         nb = len(self.blocks)
