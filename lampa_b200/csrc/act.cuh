@@ -14,21 +14,39 @@ __device__ __forceinline__ float softplusf_(float x) {
     return fmaxf(x, 0.f) + l;
 }
 
-// x Phi(x).  erfc(z) = (1 + a1 z + ... + a6 z^6)^-16 (Abramowitz & Stegun 7.1.28, error below 3e-7) on |x| / sqrt(2):
-// one reciprocal and ten multiply-adds, where erff costs twice that; the negative side comes out as 0.5 x erfc, without
-// the cancellation of 1 + erf.  Largest absolute difference from the exact function 7e-7.
-__device__ __forceinline__ float geluf_(float x) {
-    const float z = fabsf(x) * 0.70710678f;
-    float p = 0.0000430638f;
-    p = fmaf(p, z, 0.0002765672f);
-    p = fmaf(p, z, 0.0001520143f);
-    p = fmaf(p, z, 0.0092705272f);
-    p = fmaf(p, z, 0.0422820123f);
-    p = fmaf(p, z, 0.0705230784f);
-    p = fmaf(p, z, 1.f);
-    p *= p; p *= p; p *= p; p *= p;                       // overflows where erfc is far below the smallest float: 0
-    const float h = __fdividef(0.5f, p);
-    return x * (x < 0.f ? h : 1.f - h);
+__device__ __forceinline__ float rcp_approx(float x) {      // one instruction; for arguments of moderate size
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+    return y;
+}
+// sigmoid with the bare reciprocal: 1 + e^-x is at least 1, so the range handling of __fdividef has nothing to do
+__device__ __forceinline__ float sigmoid_fast(float x) { return rcp_approx(1.f + __expf(-x)); }
+
+// Two fp32 values in one 64-bit register and the packed arithmetic on them: one issue slot for two operations.
+struct F2 { uint64_t v; };
+__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};\n" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ void f2_get(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+
+// x Phi(x) of two values.  erfc(z) = (1 + a1 z + ... + a6 z^6)^-16 (Abramowitz & Stegun 7.1.28, error below 3e-7) with
+// z = |x| / sqrt(2); x Phi(x) = max(x, 0) - |x| erfc(z) / 2, which has no cancellation on either side.  19 instructions
+// for the pair; erff costs more than that for one.  Largest absolute difference from the exact function 7e-7.
+__device__ __forceinline__ void gelu_pair(float x0, float x1, float& y0, float& y1) {
+    const F2 z = f2(fabsf(x0) * 0.70710678f, fabsf(x1) * 0.70710678f);
+    F2 p = f2(0.0000430638f);
+    p = fma2(p, z, f2(0.0002765672f));
+    p = fma2(p, z, f2(0.0001520143f));
+    p = fma2(p, z, f2(0.0092705272f));
+    p = fma2(p, z, f2(0.0422820123f));
+    p = fma2(p, z, f2(0.0705230784f));
+    p = fma2(p, z, f2(1.f));
+    p = mul2(p, p); p = mul2(p, p); p = mul2(p, p); p = mul2(p, p);      // infinite where erfc is far below the smallest float
+    float p0, p1;
+    f2_get(p, p0, p1);
+    f2_get(fma2(mul2(z, f2(-0.70710678f)), f2(rcp_approx(p0), rcp_approx(p1)), f2(fmaxf(x0, 0.f), fmaxf(x1, 0.f))), y0, y1);
 }
 
 }  // namespace lampa

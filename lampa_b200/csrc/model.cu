@@ -87,64 +87,92 @@ __global__ void __launch_bounds__(256) model_encode_kernel(const float* __restri
             if (r0 + e / ENC_IN < n) rows[warp][e] = __ldg(hits + r0 * ENC_IN + e) * sc[i];
         }
         __syncwarp();
-        for (int r = 0; r < 8 && r0 + r < n; ++r) {
-            float y[4] = {b[0], b[1], b[2], b[3]};
+#pragma unroll 1
+        for (int q = 0; q < 8 && r0 + q < n; q += 4) {           // four rows at a time: their reductions overlap
+            float y[4][4], ss[4];
 #pragma unroll
-            for (int i = 0; i < ENC_IN; i += 4) {
-                const float4 h = *reinterpret_cast<const float4*>(&rows[warp][r * ENC_IN + i]);
+            for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    y[c] = fmaf(h.w, w[c][i + 3], fmaf(h.z, w[c][i + 2], fmaf(h.y, w[c][i + 1], fmaf(h.x, w[c][i], y[c]))));
+                for (int c = 0; c < 4; ++c) y[r][c] = b[c];
+#pragma unroll
+            for (int i = 0; i < ENC_IN; i += 4)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float4 h = *reinterpret_cast<const float4*>(&rows[warp][(q + r) * ENC_IN + i]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        y[r][c] = fmaf(h.w, w[c][i + 3], fmaf(h.z, w[c][i + 2], fmaf(h.y, w[c][i + 1], fmaf(h.x, w[c][i], y[r][c]))));
+                }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) ss[r] = y[r][0] * y[r][0] + y[r][1] * y[r][1] + y[r][2] * y[r][2] + y[r][3] * y[r][3];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (r0 + q + r >= n) break;
+                const float rstd = rsqrtf(ss[r] * (1.f / MD) + eps);
+                *reinterpret_cast<float4*>(x + (r0 + q + r) * MD + 4 * lane) = make_float4(y[r][0], y[r][1], y[r][2], y[r][3]);
+                *reinterpret_cast<uint2*>(hs + (r0 + q + r) * MD + 4 * lane) =
+                    make_uint2(pack_bf16x2(y[r][0] * rstd * g[0], y[r][1] * rstd * g[1]), pack_bf16x2(y[r][2] * rstd * g[2], y[r][3] * rstd * g[3]));
             }
-            float ss = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rstd = 1.f / sqrtf(ss * (1.f / MD) + eps);
-            *reinterpret_cast<float4*>(x + (r0 + r) * MD + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
-            *reinterpret_cast<uint2*>(hs + (r0 + r) * MD + 4 * lane) =
-                make_uint2(pack_bf16x2(y[0] * rstd * g[0], y[1] * rstd * g[1]), pack_bf16x2(y[2] * rstd * g[2], y[3] * rstd * g[3]));
         }
     }
 }
 
 // -------------------------------------------------------------------------------------------------
-// head: out = x W^T + b, 24 outputs.  64 rows per CTA through shared memory; thread = (row, 6 outputs).
+// head: out = x W^T + b, 24 outputs.  128 rows per CTA through shared memory; thread = 4 rows x 6
+// outputs, so that ten 16-byte loads feed 96 multiply-adds (one row per thread left it at the
+// shared-memory pipe).  608 bytes per row move.
 // -------------------------------------------------------------------------------------------------
-constexpr int HEAD_OUT = 24, HEAD_PITCH = MD + 4;
+constexpr int HEAD_OUT = 24, HEAD_PITCH = MD + 4, HEAD_ROWS = 128;
+constexpr int HEAD_SMEM = (HEAD_ROWS + HEAD_OUT) * HEAD_PITCH * 4;
 
-__global__ void __launch_bounds__(256) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
+__global__ void __launch_bounds__(128) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
                                                          const float* __restrict__ bias, int64_t n, float* __restrict__ out) {
-    __shared__ __align__(16) float sx[64 * HEAD_PITCH];
-    __shared__ __align__(16) float sw[HEAD_OUT * MD];
+    extern __shared__ __align__(16) float head_smem[];
+    float* sx = head_smem;                                   // [128][132]
+    float* sw = sx + HEAD_ROWS * HEAD_PITCH;                 // [24][132]
     const int tid = threadIdx.x;
-    for (int i = tid; i < HEAD_OUT * MD / 4; i += 256) reinterpret_cast<float4*>(sw)[i] = __ldg(reinterpret_cast<const float4*>(W) + i);
-    const int og = (tid & 3) * 6, row = tid >> 2;
-    float b[6];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) b[o] = bias ? __ldg(bias + og + o) : 0.f;
-    for (int64_t r0 = (int64_t)blockIdx.x * 64; r0 < n; r0 += (int64_t)gridDim.x * 64) {
+    for (int i = tid; i < HEAD_OUT * 32; i += 128)
+        *reinterpret_cast<float4*>(sw + (i >> 5) * HEAD_PITCH + 4 * (i & 31)) = __ldg(reinterpret_cast<const float4*>(W) + i);
+    const int og = (tid & 3) * 6, row = tid >> 2;            // rows row, row + 32, row + 64, row + 96
+    for (int64_t r0 = (int64_t)blockIdx.x * HEAD_ROWS; r0 < n; r0 += (int64_t)gridDim.x * HEAD_ROWS) {
         __syncthreads();
-        const int m = (int)min((int64_t)64, n - r0);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = tid + 256 * i, r = e >> 5, c = e & 31;
+        const int m = (int)min((int64_t)HEAD_ROWS, n - r0);
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+            const int r = 4 * i + (tid >> 5), c = tid & 31;
             if (r < m) *reinterpret_cast<float4*>(sx + r * HEAD_PITCH + 4 * c) = __ldg(reinterpret_cast<const float4*>(x + (r0 + r) * MD) + c);
         }
         __syncthreads();
-        float y[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int c = 0; c < MD; c += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(sx + row * HEAD_PITCH + c);
+        float y[4][6];
 #pragma unroll
-            for (int o = 0; o < 6; ++o) {
-                const float4 w = *reinterpret_cast<const float4*>(sw + (og + o) * MD + c);
-                y[o] = fmaf(v.w, w.w, fmaf(v.z, w.z, fmaf(v.y, w.y, fmaf(v.x, w.x, y[o]))));
-            }
+        for (int o = 0; o < 6; ++o) {
+            const float b = bias ? __ldg(bias + og + o) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i][o] = b;
         }
-        if (row < m)
+#pragma unroll 2
+        for (int c = 0; c < MD; c += 4) {
+            float4 v[4], w[6];
 #pragma unroll
-            for (int o = 0; o < 6; o += 2)
-                *reinterpret_cast<float2*>(out + (r0 + row) * HEAD_OUT + og + o) = make_float2(y[o] + b[o], y[o + 1] + b[o + 1]);
+            for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(sx + (row + 32 * i) * HEAD_PITCH + c);
+#pragma unroll
+            for (int o = 0; o < 6; ++o) w[o] = *reinterpret_cast<const float4*>(sw + (og + o) * HEAD_PITCH + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int o = 0; o < 6; ++o)
+                    y[i][o] = fmaf(v[i].w, w[o].w, fmaf(v[i].z, w[o].z, fmaf(v[i].y, w[o].y, fmaf(v[i].x, w[o].x, y[i][o]))));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (row + 32 * i < m)
+#pragma unroll
+                for (int o = 0; o < 6; o += 2)
+                    *reinterpret_cast<float2*>(out + (r0 + row + 32 * i) * HEAD_OUT + og + o) = make_float2(y[i][o], y[i][o + 1]);
     }
 }
 
@@ -163,7 +191,7 @@ constexpr int PJ_ST = PJ_W + MNST * MST;                       // [112][128] bf1
 constexpr int PJ_SMEM = PJ_ST + PJ_OUT * MD * 2;
 constexpr int PJ_THREADS = (MWARPS + 1) * 32;
 constexpr int PJ_BLOCKS = 5;
-constexpr int PJ_ROW_B = 8, PJ_ROW_L = 16;                     // first weight row of b and l in the last block
+constexpr int PJ_ROW_A = 112, PJ_ROW_B = 120;                  // weight rows of a and b in the last block, l from row 0: in warps of their own up to H * L = 96
 
 struct ProjArgs {
     const __nv_bfloat16* hs; const int64_t* perm; const int64_t* cu; int nseq; int64_t n;
@@ -227,9 +255,9 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                     tma_load_2d(dst, blk == 0 ? &mq : blk == 1 ? &mk : blk == 2 ? &mv : &mg, x, 0, b);
                 } else {
                     mbar_expect_tx(b, (uint32_t)(2 * a.H + a.H * a.L) * 128);
-                    tma_load_2d(dst, &ma, x, 0, b);
+                    tma_load_2d(dst + PJ_ROW_A * 128, &ma, x, 0, b);
                     tma_load_2d(dst + PJ_ROW_B * 128, &mb, x, 0, b);
-                    tma_load_2d(dst + PJ_ROW_L * 128, &ml, x, 0, b);
+                    tma_load_2d(dst, &ml, x, 0, b);
                 }
                 loaded = p + 1;
             };
@@ -272,9 +300,9 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             for (int i = 0; i < 4; ++i) cw[m][i] = __bfloat162float(a.conv[m][ch * 4 + i]);
         const int HL = a.H * a.L;
         // last block: the channel is a (g), b (beta), l (lambda) or nothing; g and lambda are scale * softplus(mul x + add)
-        const bool is_a = ch < a.H, is_b = ch >= PJ_ROW_B && ch < PJ_ROW_B + a.H, is_l = ch >= PJ_ROW_L && ch < PJ_ROW_L + HL;
-        const float sp_scale = is_a ? -__expf(__ldg(a.A_log + ch)) : 1.f, sp_add = is_a ? __ldg(a.dt_bias + ch) : 0.f;
-        const float sp_mul = is_l ? __ldg(a.Lw + ch - PJ_ROW_L) : 1.f;
+        const bool is_a = ch >= PJ_ROW_A && ch < PJ_ROW_A + a.H, is_b = ch >= PJ_ROW_B && ch < PJ_ROW_B + a.H, is_l = ch < HL;
+        const float sp_scale = is_a ? -__expf(__ldg(a.A_log + ch - PJ_ROW_A)) : 1.f, sp_add = is_a ? __ldg(a.dt_bias + ch - PJ_ROW_A) : 0.f;
+        const float sp_mul = is_l ? __ldg(a.Lw + ch) : 1.f;
 
         for (int t = 0; t < mine; ++t) {
             const int64_t tile = blockIdx.x + (int64_t)t * gridDim.x, j0 = tile * PJ_OUT;
@@ -321,49 +349,55 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dfree + buf);
-                if (tid == 0) bulk_wait_read();                  // the staging tile has left
-                epi_sync();
                 auto X = [&](int i) -> float& { return x[i >> 5][i & 31]; };
-                __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(sST) + (size_t)(56 * half) * MD + ch;
+                uint32_t w[28];                                  // the 56 results, packed before anybody waits for the staging tile
                 if (m < 3) {
                     float h1 = X(7), h2 = X(6), h3 = X(5);
                     const float w0 = m == 0 ? cw[0][0] : m == 1 ? cw[1][0] : cw[2][0], w1 = m == 0 ? cw[0][1] : m == 1 ? cw[1][1] : cw[2][1];
                     const float w2 = m == 0 ? cw[0][2] : m == 1 ? cw[1][2] : cw[2][2], w3 = m == 0 ? cw[0][3] : m == 1 ? cw[1][3] : cw[2][3];
+                    auto tap = [&](int i) {
+                        const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
+                        h3 = h2; h2 = h1; h1 = X(8 + i);
+                        return v * sigmoid_fast(v);
+                    };
                     if (starts == 0) {
 #pragma unroll
-                        for (int i = 0; i < 56; ++i) {
-                            const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
-                            h3 = h2; h2 = h1; h1 = X(8 + i);
-                            st[i * MD] = __float2bfloat16_rn(v * sigmoidf_(v));
-                        }
+                        for (int i = 0; i < 28; ++i) { const float u = tap(2 * i); w[i] = pack_bf16x2(u, tap(2 * i + 1)); }
                     } else {                                     // an event opens here: its first taps are empty
                         if ((starts >> 7) & 1) h2 = h3 = 0.f;
                         if ((starts >> 6) & 1) h3 = 0.f;
 #pragma unroll
-                        for (int i = 0; i < 56; ++i) {
-                            if ((starts >> (8 + i)) & 1) h1 = h2 = h3 = 0.f;
-                            const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
-                            h3 = h2; h2 = h1; h1 = X(8 + i);
-                            st[i * MD] = __float2bfloat16_rn(v * sigmoidf_(v));
+                        for (int i = 0; i < 28; ++i) {
+                            if ((starts >> (8 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
+                            const float u = tap(2 * i);
+                            if ((starts >> (9 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
+                            w[i] = pack_bf16x2(u, tap(2 * i + 1));
                         }
                     }
                 } else if (m == 3) {
 #pragma unroll
-                    for (int i = 0; i < 56; ++i) st[i * MD] = __float2bfloat16_rn(X(8 + i));
-                } else if (is_a || is_l) {
-                    __nv_bfloat16* sl = reinterpret_cast<__nv_bfloat16*>(sST) + (size_t)(56 * half) * HL + ch - PJ_ROW_L;
-                    float* gp = a.g + (j0 + 56 * half) * a.H + ch;
+                    for (int i = 0; i < 28; ++i) w[i] = pack_bf16x2(X(8 + 2 * i), X(9 + 2 * i));
+                } else if (is_l) {
 #pragma unroll
-                    for (int i = 0; i < 56; ++i) {
-                        const float v = sp_scale * softplusf_(fmaf(sp_mul, X(8 + i), sp_add));
-                        if (is_l) sl[i * HL] = __float2bfloat16_rn(v);
-                        else if (56 * half + i < nv) gp[i * a.H] = v;
-                    }
-                } else if (is_b) {
-                    float* bp = a.beta + (j0 + 56 * half) * a.H + ch - PJ_ROW_B;
+                    for (int i = 0; i < 28; ++i) w[i] = pack_bf16x2(softplusf_(sp_mul * X(8 + 2 * i)), softplusf_(sp_mul * X(9 + 2 * i)));
+                } else if (is_a || is_b) {                       // g and beta: straight to their rows
+                    float* gp = (is_a ? a.g + ch - PJ_ROW_A : a.beta + ch - PJ_ROW_B) + (j0 + 56 * half) * a.H;
 #pragma unroll
                     for (int i = 0; i < 56; ++i)
-                        if (56 * half + i < nv) bp[i * a.H] = sigmoidf_(X(8 + i));
+                        if (56 * half + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(X(8 + i) + sp_add) : sigmoid_fast(X(8 + i));
+                }
+                if (tid == 0) bulk_wait_read();                  // the previous results have left the staging tile
+                epi_sync();
+                if (m < 4 || is_l) {
+                    const int pitch = m < 4 ? MD : HL;
+                    uint16_t* st = reinterpret_cast<uint16_t*>(sST) + (size_t)(56 * half) * pitch + ch;
+                    if (m < 4) {
+#pragma unroll
+                        for (int i = 0; i < 28; ++i) { st[2 * i * MD] = (uint16_t)w[i]; st[(2 * i + 1) * MD] = (uint16_t)(w[i] >> 16); }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 28; ++i) { st[2 * i * HL] = (uint16_t)w[i]; st[(2 * i + 1) * HL] = (uint16_t)(w[i] >> 16); }
+                    }
                 }
                 fence_async_smem();
                 epi_sync();
@@ -536,6 +570,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
         const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16);
         const int trow = 32 * quarter + lane;                    // this thread's row of an accumulator
         const int lanes_per_head = a.head_dim >> 2;
+        const float inv_dim = 1.f / (float)a.head_dim;
         float ow[4], mw[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -586,10 +621,10 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     const float2 o0 = unpack_bf16x2(ov[i].x), o1 = unpack_bf16x2(ov[i].y), g0 = unpack_bf16x2(gv[i].x), g1 = unpack_bf16x2(gv[i].y);
                     float ss = o0.x * o0.x + o0.y * o0.y + o1.x * o1.x + o1.y * o1.y;
                     for (int o = lanes_per_head >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    const float rstd = 1.f / sqrtf(ss / (float)a.head_dim + a.o_eps);
+                    const float rstd = rsqrtf(ss * inv_dim + a.o_eps);
                     *reinterpret_cast<uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST)) =
-                        make_uint2(pack_bf16x2(o0.x * rstd * ow[0] * g0.x * sigmoidf_(g0.x), o0.y * rstd * ow[1] * g0.y * sigmoidf_(g0.y)),
-                                   pack_bf16x2(o1.x * rstd * ow[2] * g1.x * sigmoidf_(g1.x), o1.y * rstd * ow[3] * g1.y * sigmoidf_(g1.y)));
+                        make_uint2(pack_bf16x2(o0.x * rstd * ow[0] * g0.x * sigmoid_fast(g0.x), o0.y * rstd * ow[1] * g0.y * sigmoid_fast(g0.y)),
+                                   pack_bf16x2(o1.x * rstd * ow[2] * g1.x * sigmoid_fast(g1.x), o1.y * rstd * ow[3] * g1.y * sigmoid_fast(g1.y)));
                 }
             }
             operand_ready();
@@ -616,7 +651,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     float ss = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    const float rstd = 1.f / sqrtf(ss * (1.f / MD) + a.eps);
+                    const float rstd = rsqrtf(ss * (1.f / MD) + a.eps);
                     *op = make_uint2(pack_bf16x2(v[i].x * rstd * mw[0], v[i].y * rstd * mw[1]), pack_bf16x2(v[i].z * rstd * mw[2], v[i].w * rstd * mw[3]));
                 }
             }
@@ -643,7 +678,11 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                 }
                 uint32_t w[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) w[e] = pack_bf16x2(geluf_(x[2 * e]), geluf_(x[2 * e + 1]));
+                for (int e = 0; e < 16; ++e) {
+                    float y0, y1;
+                    gelu_pair(x[2 * e], x[2 * e + 1], y0, y1);
+                    w[e] = pack_bf16x2(y0, y1);
+                }
                 if (q >= 2) mbar_wait(hfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 632, a.budget);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
@@ -678,7 +717,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     float ss = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    const float rstd = 1.f / sqrtf(ss * (1.f / MD) + a.next_eps);
+                    const float rstd = rsqrtf(ss * (1.f / MD) + a.next_eps);
                     const float4 nw = __ldg(reinterpret_cast<const float4*>(a.next_norm_w) + lane);
                     *reinterpret_cast<uint2*>(a.hs + rr[i] * MD + 4 * lane) =
                         make_uint2(pack_bf16x2(v[i].x * rstd * nw.x, v[i].y * rstd * nw.y), pack_bf16x2(v[i].z * rstd * nw.z, v[i].w * rstd * nw.w));
@@ -720,8 +759,10 @@ extern "C" int lampa_model_head(const float* x, const float* weight, const float
     if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) return LAMPA_ERR_UNSUPPORTED;
     if (n == 0) return LAMPA_OK;
     ProfScope prof("model_head", (cudaStream_t)stream);
-    const int64_t want = (n + 63) / 64, most = (int64_t)sm_count() * 4;
-    model_head_kernel<<<(unsigned)(want < most ? want : most), 256, 0, (cudaStream_t)stream>>>(x, weight, bias, n, out);
+    static std::atomic<uint64_t> ready{0};
+    if (!allow_smem(ready, model_head_kernel, HEAD_SMEM)) return LAMPA_ERR_CUDA;
+    const int64_t want = (n + HEAD_ROWS - 1) / HEAD_ROWS, most = (int64_t)sm_count() * 2;
+    model_head_kernel<<<(unsigned)(want < most ? want : most), 128, HEAD_SMEM, (cudaStream_t)stream>>>(x, weight, bias, n, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -731,7 +772,7 @@ extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, c
     if (!w || n < 0 || nseq <= 0) return LAMPA_ERR_ARG;
     if (n == 0) return LAMPA_OK;
     if (!hs || !perm || !cu || !q || !k || !v || !gate || !g || !beta || !lam) return LAMPA_ERR_ARG;
-    if (w->H <= 0 || w->H > PJ_ROW_L - PJ_ROW_B || w->L <= 0 || w->H * w->L > 128 - PJ_ROW_L || MD % w->H != 0) return LAMPA_ERR_UNSUPPORTED;
+    if (w->H <= 0 || w->H > PJ_ROW_B - PJ_ROW_A || w->L <= 0 || w->H * w->L > PJ_ROW_A || MD % w->H != 0) return LAMPA_ERR_UNSUPPORTED;
     ProjArgs a;
     a.hs = (const __nv_bfloat16*)hs; a.perm = perm; a.cu = cu; a.nseq = nseq; a.n = n;
     a.conv[0] = (const __nv_bfloat16*)w->q_conv; a.conv[1] = (const __nv_bfloat16*)w->k_conv; a.conv[2] = (const __nv_bfloat16*)w->v_conv;
