@@ -5,13 +5,21 @@
 namespace lampa {
 
 __device__ __forceinline__ float sigmoidf_(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-// log(1 + e^x) as max(x, 0) + log1p(e^-|x|); the log1p is the hardware log above 0.01 (absolute
-// error 2e-7) and its cubic Taylor polynomial below.  torch switches to x above 20, where the
-// two agree to fp32 rounding.
+// log(1 + e^x) as max(x, 0) + log1p(e^-|x|).  log1p(e) = e P(e) on [0, 1] with P the degree-8 Chebyshev fit of log1p(e) / e:
+// relative error 2e-7 in fp32 and no branch (the hardware log below its accuracy limit needed one, which diverges in
+// nearly every warp).  torch switches to x above 20, where the two agree to fp32 rounding.
 __device__ __forceinline__ float softplusf_(float x) {
     const float e = __expf(-fabsf(x));
-    const float l = e > 0.01f ? __logf(1.f + e) : e * (1.f - e * (0.5f - e * (1.f / 3.f)));
-    return fmaxf(x, 0.f) + l;
+    float p = 0.005253457929939032f;
+    p = fmaf(p, e, -0.02958850748836994f);
+    p = fmaf(p, e, 0.07836166769266129f);
+    p = fmaf(p, e, -0.13674770295619965f);
+    p = fmaf(p, e, 0.19111430644989014f);
+    p = fmaf(p, e, -0.24844369292259216f);
+    p = fmaf(p, e, 0.33319270610809326f);
+    p = fmaf(p, e, -0.49999502301216125f);
+    p = fmaf(p, e, 1.f);
+    return fmaf(p, e, fmaxf(x, 0.f));
 }
 
 __device__ __forceinline__ float rcp_approx(float x) {      // one instruction; for arguments of moderate size

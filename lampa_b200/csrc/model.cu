@@ -27,9 +27,10 @@ namespace {
 constexpr int MD = 128;                      // model width
 constexpr int MST = 16384;                   // one weight stage: [128][64] or two [64][64] bf16 tiles, 128-byte swizzle
 constexpr int MNST = 3;
-constexpr int MWARPS = 8;                    // epilogue warps
+constexpr int MWARPS = 16;                   // epilogue warps: the epilogues are chains of latencies, 8 warps of twice the columns took 1.5 x as long
+constexpr int METHR = MWARPS * 32;
 
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;\n" :: "n"(METHR) : "memory"); }
 
 // Row r of the residual stream that position j of an ordered batch stands for (perm is local to j's event); -1 when the
 // permutation leaves the event.
@@ -179,12 +180,13 @@ __global__ void __launch_bounds__(128) model_head_kernel(const float* __restrict
 // -------------------------------------------------------------------------------------------------
 // project.  A tile is 112 positions of the ordered batch with the 8 before them.  The products are
 // taken transposed, D[channel][position] = W x hs^T: a thread then owns one channel (tensor-memory
-// lane) and 56 consecutive positions in registers, which makes the 4-tap convolution a register
+// lane) and 28 consecutive positions in registers, which makes the 4-tap convolution a register
 // window.  Five blocks of 128 channels: q, k, v, gate, (a | b | l).  Results pass through a
 // [position][channel] tile in shared memory and leave as one bulk store per block (the rows of a
 // tile are contiguous in every output).
 // -------------------------------------------------------------------------------------------------
 constexpr int PJ_OUT = 112, PJ_ROWS = 128, PJ_HALO = 16;       // positions per tile; operand rows; the first output row
+constexpr int PJ_PART = PJ_OUT / (MWARPS / 4);                 // positions of a thread
 constexpr int PJ_B = 2048;                                     // two swizzled [128][64] halves
 constexpr int PJ_W = PJ_B + 2 * MST;
 constexpr int PJ_ST = PJ_W + MNST * MST;                       // [112][128] bf16
@@ -290,14 +292,9 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             mbar_drain(drain, 0u);
         }
     } else {
-        const int quarter = warp & 3, half = warp >> 2;          // channels 32 quarter + lane; positions 56 half ..
+        const int quarter = warp & 3, part = warp >> 2;          // channels 32 quarter + lane; positions 28 part ..
         const int ch = 32 * quarter + lane;
-        const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(PJ_HALO - 8 + 56 * half);
-        float cw[3][4];
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cw[m][i] = __bfloat162float(a.conv[m][ch * 4 + i]);
+        const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(PJ_HALO - 4 + PJ_PART * part);
         const int HL = a.H * a.L;
         // last block: the channel is a (g), b (beta), l (lambda) or nothing; g and lambda are scale * softplus(mul x + add)
         const bool is_a = ch >= PJ_ROW_A && ch < PJ_ROW_A + a.H, is_b = ch >= PJ_ROW_B && ch < PJ_ROW_B + a.H, is_l = ch < HL;
@@ -318,7 +315,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 if (lane == 0) sstart[warp] = bits;
             }
             epi_sync();
-            for (int i = tid; i < (PJ_ROWS - 8) * 16; i += 256) {
+            for (int i = tid; i < (PJ_ROWS - 8) * 16; i += METHR) {
                 const int row = 8 + (i >> 4), c = i & 15;
                 const int64_t r = srow[row];
                 unsigned char* dst = sB + op_off(row, 8 * c, MST);
@@ -329,75 +326,67 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(bready);
-            // event starts of this thread's 56 positions and the 8 before: bit i = position i - 8
-            const int p0 = PJ_HALO - 8 + 56 * half;
-            uint64_t starts = 0;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const int sh = 32 * w - p0;
-                const uint64_t bits = sstart[w];
-                if (sh >= 0 && sh < 64) starts |= bits << sh;
-                else if (sh < 0 && sh > -32) starts |= bits >> -sh;
-            }
+            // event starts of this thread's 28 positions and the 4 before: bit i = operand row p0 + i
+            const int p0 = PJ_HALO - 4 + PJ_PART * part;
+            const uint32_t starts = __funnelshift_r(sstart[p0 >> 5], (p0 >> 5) < 3 ? sstart[(p0 >> 5) + 1] : 0u, p0 & 31);
             for (int m = 0; m < PJ_BLOCKS; ++m) {
                 const int q = t * PJ_BLOCKS + m, buf = q & 1;
+                uint2 taps = make_uint2(0u, 0u);                 // this channel's four taps
+                if (m < 3) taps = __ldg(reinterpret_cast<const uint2*>(m == 0 ? a.conv[0] : m == 1 ? a.conv[1] : a.conv[2]) + ch);
                 mbar_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget);
                 tc_fence_after();
-                float x[2][32];
-                tmem_ld32(x[0], tl + 128 * buf);
-                tmem_ld32(x[1], tl + 128 * buf + 32);
+                float x[32];                                     // X(i) = position i - 4
+                tmem_ld32(x, tl + 128 * buf);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dfree + buf);
-                auto X = [&](int i) -> float& { return x[i >> 5][i & 31]; };
-                uint32_t w[28];                                  // the 56 results, packed before anybody waits for the staging tile
+                uint32_t w[PJ_PART / 2];                         // the 28 results, packed before anybody waits for the staging tile
                 if (m < 3) {
-                    float h1 = X(7), h2 = X(6), h3 = X(5);
-                    const float w0 = m == 0 ? cw[0][0] : m == 1 ? cw[1][0] : cw[2][0], w1 = m == 0 ? cw[0][1] : m == 1 ? cw[1][1] : cw[2][1];
-                    const float w2 = m == 0 ? cw[0][2] : m == 1 ? cw[1][2] : cw[2][2], w3 = m == 0 ? cw[0][3] : m == 1 ? cw[1][3] : cw[2][3];
+                    float h1 = x[3], h2 = x[2], h3 = x[1];
+                    const float2 ta = unpack_bf16x2(taps.x), tb = unpack_bf16x2(taps.y);
+                    const float w0 = ta.x, w1 = ta.y, w2 = tb.x, w3 = tb.y;
                     auto tap = [&](int i) {
-                        const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * X(8 + i))));
-                        h3 = h2; h2 = h1; h1 = X(8 + i);
+                        const float v = fmaf(w0, h3, fmaf(w1, h2, fmaf(w2, h1, w3 * x[4 + i])));
+                        h3 = h2; h2 = h1; h1 = x[4 + i];
                         return v * sigmoid_fast(v);
                     };
                     if (starts == 0) {
 #pragma unroll
-                        for (int i = 0; i < 28; ++i) { const float u = tap(2 * i); w[i] = pack_bf16x2(u, tap(2 * i + 1)); }
+                        for (int i = 0; i < PJ_PART / 2; ++i) { const float u = tap(2 * i); w[i] = pack_bf16x2(u, tap(2 * i + 1)); }
                     } else {                                     // an event opens here: its first taps are empty
-                        if ((starts >> 7) & 1) h2 = h3 = 0.f;
-                        if ((starts >> 6) & 1) h3 = 0.f;
+                        if ((starts >> 3) & 1) h2 = h3 = 0.f;
+                        if ((starts >> 2) & 1) h3 = 0.f;
 #pragma unroll
-                        for (int i = 0; i < 28; ++i) {
-                            if ((starts >> (8 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
+                        for (int i = 0; i < PJ_PART / 2; ++i) {
+                            if ((starts >> (4 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
                             const float u = tap(2 * i);
-                            if ((starts >> (9 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
+                            if ((starts >> (5 + 2 * i)) & 1) h1 = h2 = h3 = 0.f;
                             w[i] = pack_bf16x2(u, tap(2 * i + 1));
                         }
                     }
                 } else if (m == 3) {
 #pragma unroll
-                    for (int i = 0; i < 28; ++i) w[i] = pack_bf16x2(X(8 + 2 * i), X(9 + 2 * i));
-                } else if (is_l) {
+                    for (int i = 0; i < PJ_PART / 2; ++i) w[i] = pack_bf16x2(x[4 + 2 * i], x[5 + 2 * i]);
+                } else if (quarter < 3 || is_l) {
 #pragma unroll
-                    for (int i = 0; i < 28; ++i) w[i] = pack_bf16x2(softplusf_(sp_mul * X(8 + 2 * i)), softplusf_(sp_mul * X(9 + 2 * i)));
+                    for (int i = 0; i < PJ_PART / 2; ++i) w[i] = pack_bf16x2(softplusf_(sp_mul * x[4 + 2 * i]), softplusf_(sp_mul * x[5 + 2 * i]));
                 } else if (is_a || is_b) {                       // g and beta: straight to their rows
-                    float* gp = (is_a ? a.g + ch - PJ_ROW_A : a.beta + ch - PJ_ROW_B) + (j0 + 56 * half) * a.H;
+                    float* gp = (is_a ? a.g + ch - PJ_ROW_A : a.beta + ch - PJ_ROW_B) + (j0 + PJ_PART * part) * a.H;
 #pragma unroll
-                    for (int i = 0; i < 56; ++i)
-                        if (56 * half + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(X(8 + i) + sp_add) : sigmoid_fast(X(8 + i));
+                    for (int i = 0; i < PJ_PART; ++i)
+                        if (PJ_PART * part + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(x[4 + i] + sp_add) : sigmoid_fast(x[4 + i]);
                 }
                 if (tid == 0) bulk_wait_read();                  // the previous results have left the staging tile
                 epi_sync();
-                if (m < 4 || is_l) {
-                    const int pitch = m < 4 ? MD : HL;
-                    uint16_t* st = reinterpret_cast<uint16_t*>(sST) + (size_t)(56 * half) * pitch + ch;
-                    if (m < 4) {
+                uint16_t* st = reinterpret_cast<uint16_t*>(sST) + ch;
+                if (m < 4) {
+                    st += PJ_PART * part * MD;
 #pragma unroll
-                        for (int i = 0; i < 28; ++i) { st[2 * i * MD] = (uint16_t)w[i]; st[(2 * i + 1) * MD] = (uint16_t)(w[i] >> 16); }
-                    } else {
+                    for (int i = 0; i < PJ_PART / 2; ++i) { st[2 * i * MD] = (uint16_t)w[i]; st[(2 * i + 1) * MD] = (uint16_t)(w[i] >> 16); }
+                } else if (is_l) {
+                    st += PJ_PART * part * HL;
 #pragma unroll
-                        for (int i = 0; i < 28; ++i) { st[2 * i * HL] = (uint16_t)w[i]; st[(2 * i + 1) * HL] = (uint16_t)(w[i] >> 16); }
-                    }
+                    for (int i = 0; i < PJ_PART / 2; ++i) { st[2 * i * HL] = (uint16_t)w[i]; st[(2 * i + 1) * HL] = (uint16_t)(w[i] >> 16); }
                 }
                 fence_async_smem();
                 epi_sync();
@@ -406,7 +395,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 if (bytes % 16 == 0) {
                     if (tid == 0) { bulk_s2g(dst, sST, bytes); bulk_commit(); }
                 } else {                                         // last rows of lambda: not whole 16-byte pieces
-                    for (int i = tid; i < nv * HL; i += 256) a.lam[j0 * HL + i] = reinterpret_cast<const __nv_bfloat16*>(sST)[i];
+                    for (int i = tid; i < nv * HL; i += METHR) a.lam[j0 * HL + i] = reinterpret_cast<const __nv_bfloat16*>(sST)[i];
                 }
             }
         }
@@ -419,13 +408,13 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
 
 // -------------------------------------------------------------------------------------------------
 // update.  A tile is 128 positions of the ordered batch.  Row-wise steps (gated norm, residual and
-// norm) give a warp 16 rows, four columns per lane; products leave tensor memory one row per lane and
+// norm) give a warp 8 rows, four columns per lane; products leave tensor memory one row per lane and
 // go through the operand tile (bf16) to the row-wise layout.  The hidden layer never leaves the SM:
 // eight chunks of 64 hidden units, each up product -> bias, GELU -> bf16 operand -> accumulated into
 // the down product, the up product of the next chunk under the GELU of this one.
 // Bound by the epilogues' instruction issue (the GELU alone is 65 k elements per tile), not by HBM.
 // -------------------------------------------------------------------------------------------------
-constexpr int UP_ROWS = 128, UP_HID = 512, UP_CH = 64, UP_NCH = UP_HID / UP_CH;
+constexpr int UP_ROWS = 128, UP_WROWS = UP_ROWS / MWARPS, UP_HID = 512, UP_CH = 64, UP_NCH = UP_HID / UP_CH;
 constexpr int UP_A = 1024;                                     // operand tile: two swizzled [128][64] halves
 constexpr int UP_H = UP_A + 2 * MST;                           // hidden operand, two buffers of [128][64]
 constexpr int UP_W = UP_H + 2 * MST;
@@ -566,7 +555,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             mbar_drain(drain, 0u);
         }
     } else {
-        const int quarter = warp & 3, half = warp >> 2;
+        const int quarter = warp & 3, part = warp >> 2;
         const uint32_t tl = taddr + ((uint32_t)(32 * quarter) << 16);
         const int trow = 32 * quarter + lane;                    // this thread's row of an accumulator
         const int lanes_per_head = a.head_dim >> 2;
@@ -577,21 +566,20 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             ow[c] = a.o_norm_w ? __bfloat162float(a.o_norm_w[(4 * lane + c) % a.head_dim]) : 1.f;
             mw[c] = __ldg(a.mlp_norm_w + 4 * lane + c);
         }
-        // accumulator half-row -> bf16 -> operand tile (row-wise readers pick it up there)
+        // accumulator quarter-row -> bf16 -> operand tile (row-wise readers pick it up there)
         auto stage_acc = [&](const __nv_bfloat16* bias) {
-            float x[2][32];
-            tmem_ld32(x[0], tl + UT_ACC + 64 * half);
-            tmem_ld32(x[1], tl + UT_ACC + 64 * half + 32);
+            float x[32];
+            tmem_ld32(x, tl + UT_ACC + 32 * part);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float* v = &x[q >> 2][(q & 3) * 8];
+            for (int q = 0; q < 4; ++q) {
+                float* v = &x[8 * q];
                 if (bias) {
-                    const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + 64 * half) + q);
+                    const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + 32 * part) + q);
                     const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) { const float2 f = unpack_bf16x2(bw[e]); v[2 * e] += f.x; v[2 * e + 1] += f.y; }
                 }
-                *reinterpret_cast<uint4*>(sA + op_off(trow, 64 * half + 8 * q, MST)) =
+                *reinterpret_cast<uint4*>(sA + op_off(trow, 32 * part + 8 * q, MST)) =
                     make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
             }
         };
@@ -602,13 +590,17 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             if (lane == 0) mbar_arrive(aready);
         };
         for (int t = 0; t < mine; ++t) {
-            const int64_t j0 = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * UP_ROWS + 16 * warp;   // this warp's 16 rows
-            const int nr = (int)min((int64_t)16, max((int64_t)0, a.n - j0));
+            const int64_t j0 = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * UP_ROWS + UP_WROWS * warp;   // this warp's rows
+            const int nr = (int)min((int64_t)UP_WROWS, max((int64_t)0, a.n - j0));
             int64_t myrow = -1;
             if (lane < nr) myrow = ordered_row(a.cu, a.nseq, a.perm, j0 + lane, a.status);
+            {   // the residual rows are wanted one product later: into L2 now (four lines each)
+                const int64_t pr = __shfl_sync(0xffffffffu, myrow, lane >> 2);
+                if (pr >= 0) asm volatile("prefetch.global.L2 [%0];\n" :: "l"(a.x + pr * MD + 32 * (lane & 3)));
+            }
             // ---- gated norm of the mixer's rows: the operand of o_proj ----
 #pragma unroll 1
-            for (int r0 = 0; r0 < 16; r0 += 4) {
+            for (int r0 = 0; r0 < UP_WROWS; r0 += 4) {
                 uint2 ov[4], gv[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -622,7 +614,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     float ss = o0.x * o0.x + o0.y * o0.y + o1.x * o1.x + o1.y * o1.y;
                     for (int o = lanes_per_head >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
                     const float rstd = rsqrtf(ss * inv_dim + a.o_eps);
-                    *reinterpret_cast<uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST)) =
+                    *reinterpret_cast<uint2*>(sA + op_off(UP_WROWS * warp + r0 + i, 4 * lane, MST)) =
                         make_uint2(pack_bf16x2(o0.x * rstd * ow[0] * g0.x * sigmoid_fast(g0.x), o0.y * rstd * ow[1] * g0.y * sigmoid_fast(g0.y)),
                                    pack_bf16x2(o1.x * rstd * ow[2] * g1.x * sigmoid_fast(g1.x), o1.y * rstd * ow[3] * g1.y * sigmoid_fast(g1.y)));
                 }
@@ -634,17 +626,17 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             stage_acc(nullptr);
             epi_sync();
 #pragma unroll 1
-            for (int r0 = 0; r0 < 16; r0 += 8) {
-                float4 v[8];
-                int64_t rr[8];
+            for (int r0 = 0; r0 < UP_WROWS; r0 += 4) {
+                float4 v[4];
+                int64_t rr[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     rr[i] = __shfl_sync(0xffffffffu, myrow, r0 + i);
                     v[i] = rr[i] >= 0 ? *reinterpret_cast<const float4*>(a.x + rr[i] * MD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    uint2* op = reinterpret_cast<uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST));
+                for (int i = 0; i < 4; ++i) {
+                    uint2* op = reinterpret_cast<uint2*>(sA + op_off(UP_WROWS * warp + r0 + i, 4 * lane, MST));
                     const float2 d0 = unpack_bf16x2(op->x), d1 = unpack_bf16x2(op->y);
                     v[i].x += d0.x; v[i].y += d0.y; v[i].z += d1.x; v[i].w += d1.y;
                     if (rr[i] >= 0) *reinterpret_cast<float4*>(a.x + rr[i] * MD + 4 * lane) = v[i];
@@ -656,37 +648,42 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                 }
             }
             operand_ready();
-            // ---- hidden layer, 64 units at a time: this thread has 32 of its row ----
+            // ---- hidden layer, 64 units at a time: this thread has 16 of its row ----
 #pragma unroll 1
             for (int c = 0; c < UP_NCH; ++c) {
                 const int q = t * UP_NCH + c, buf = q & 1;
+                uint4 bias[2];
+                bias[0] = bias[1] = make_uint4(0u, 0u, 0u, 0u);
+                if (a.up_b) {
+                    const uint4* bp = reinterpret_cast<const uint4*>(a.up_b + UP_CH * c + 16 * part);
+                    bias[0] = __ldg(bp);
+                    bias[1] = __ldg(bp + 1);
+                }
+                if (c == UP_NCH - 2 && t + 1 < mine) {           // the next tile's mixer and gate rows, on their way to L2
+                    const int64_t j = j0 + (int64_t)gridDim.x * UP_ROWS + (lane >> 2);
+                    const __nv_bfloat16* base = (lane & 2) ? a.gate : a.o;
+                    if (j < a.n) asm volatile("prefetch.global.L2 [%0];\n" :: "l"(base + j * MD + 64 * (lane & 1)));
+                }
                 mbar_wait(mup + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 631, a.budget);
                 tc_fence_after();
-                float x[32];
-                tmem_ld32(x, tl + UT_UP + 64 * buf + 32 * half);
+                float x[16];
+                tmem_ld16(x, tl + UT_UP + 64 * buf + 16 * part);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(upfree + buf);
-                if (a.up_b) {
+                const uint32_t bw[8] = {bias[0].x, bias[0].y, bias[0].z, bias[0].w, bias[1].x, bias[1].y, bias[1].z, bias[1].w};
+                uint32_t w[8];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const uint4 b = __ldg(reinterpret_cast<const uint4*>(a.up_b + UP_CH * c + 32 * half) + e);
-                        const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(bw[k]); x[8 * e + 2 * k] += f.x; x[8 * e + 2 * k + 1] += f.y; }
-                    }
-                }
-                uint32_t w[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < 8; ++e) {
+                    const float2 f = unpack_bf16x2(bw[e]);
                     float y0, y1;
-                    gelu_pair(x[2 * e], x[2 * e + 1], y0, y1);
+                    gelu_pair(x[2 * e] + f.x, x[2 * e + 1] + f.y, y0, y1);
                     w[e] = pack_bf16x2(y0, y1);
                 }
                 if (q >= 2) mbar_wait(hfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 632, a.budget);
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    *reinterpret_cast<uint4*>(sH + buf * MST + op_off(trow, 32 * half + 8 * e, 0)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+                for (int e = 0; e < 2; ++e)
+                    *reinterpret_cast<uint4*>(sH + buf * MST + op_off(trow, 16 * part + 8 * e, 0)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(hready + buf);
@@ -698,17 +695,17 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             tc_fence_before();
             epi_sync();
 #pragma unroll 1
-            for (int r0 = 0; r0 < 16; r0 += 8) {
-                float4 v[8];
-                int64_t rr[8];
+            for (int r0 = 0; r0 < UP_WROWS; r0 += 4) {
+                float4 v[4];
+                int64_t rr[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     rr[i] = __shfl_sync(0xffffffffu, myrow, r0 + i);
                     v[i] = rr[i] >= 0 ? *reinterpret_cast<const float4*>(a.x + rr[i] * MD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint2 op = *reinterpret_cast<const uint2*>(sA + op_off(16 * warp + r0 + i, 4 * lane, MST));
+                for (int i = 0; i < 4; ++i) {
+                    const uint2 op = *reinterpret_cast<const uint2*>(sA + op_off(UP_WROWS * warp + r0 + i, 4 * lane, MST));
                     const float2 d0 = unpack_bf16x2(op.x), d1 = unpack_bf16x2(op.y);
                     v[i].x += d0.x; v[i].y += d0.y; v[i].z += d1.x; v[i].w += d1.y;
                     if (rr[i] < 0) continue;                     // warp-uniform
@@ -781,6 +778,8 @@ extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, c
     a.g = g; a.beta = beta; a.lam = (__nv_bfloat16*)lam; a.status = status; a.budget = MBAR_POLLS;
     for (const void* p : {w->q_w, w->k_w, w->v_w, w->g_w, w->a_w, w->b_w, w->l_w, hs, (const void*)q, (const void*)k, (const void*)v, (const void*)gate, (const void*)lam})
         if (!p || ((uintptr_t)p & 15)) return LAMPA_ERR_UNSUPPORTED;
+    for (const void* p : {w->q_conv, w->k_conv, w->v_conv})
+        if (!p || ((uintptr_t)p & 7)) return LAMPA_ERR_UNSUPPORTED;
     const void* mats[7] = {w->q_w, w->k_w, w->v_w, w->g_w, w->a_w, w->b_w, w->l_w};
     const uint32_t rows[7] = {MD, MD, MD, MD, (uint32_t)w->H, (uint32_t)w->H, (uint32_t)(w->H * w->L)};
     CUtensorMap m[7];
