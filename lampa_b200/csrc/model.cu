@@ -32,6 +32,17 @@ constexpr int METHR = MWARPS * 32;
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;\n" :: "n"(METHR) : "memory"); }
 
+// Wait of the epilogue warps: one warp polls, the others join a hardware barrier (sixteen polling warps took a third of
+// the kernel's issue slots).  `also` runs in the polling warp before the barrier.
+template <class F>
+__device__ __forceinline__ void epi_wait(uint64_t* bar, uint32_t parity, bool& dead, int32_t* status, int where, int budget, F also) {
+    if (threadIdx.x < 32) {
+        mbar_wait(bar, parity, dead, status, where, budget);
+        also();
+    }
+    epi_sync();
+}
+
 // Row r of the residual stream that position j of an ordered batch stands for (perm is local to j's event); -1 when the
 // permutation leaves the event.
 __device__ __forceinline__ int64_t ordered_row(const int64_t* __restrict__ cu, int nseq, const int64_t* __restrict__ perm,
@@ -123,57 +134,56 @@ __global__ void __launch_bounds__(256) model_encode_kernel(const float* __restri
 }
 
 // -------------------------------------------------------------------------------------------------
-// head: out = x W^T + b, 24 outputs.  128 rows per CTA through shared memory; thread = 4 rows x 6
-// outputs, so that ten 16-byte loads feed 96 multiply-adds (one row per thread left it at the
-// shared-memory pipe).  608 bytes per row move.
+// head: out = x W^T + b, 24 outputs.  128 rows per CTA through shared memory; thread = 2 rows x 6
+// outputs, so that eight 16-byte loads feed 48 multiply-adds.  608 bytes per row move.
 // -------------------------------------------------------------------------------------------------
 constexpr int HEAD_OUT = 24, HEAD_PITCH = MD + 4, HEAD_ROWS = 128;
 constexpr int HEAD_SMEM = (HEAD_ROWS + HEAD_OUT) * HEAD_PITCH * 4;
 
-__global__ void __launch_bounds__(128) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
+__global__ void __launch_bounds__(256) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
                                                          const float* __restrict__ bias, int64_t n, float* __restrict__ out) {
     extern __shared__ __align__(16) float head_smem[];
     float* sx = head_smem;                                   // [128][132]
     float* sw = sx + HEAD_ROWS * HEAD_PITCH;                 // [24][132]
     const int tid = threadIdx.x;
-    for (int i = tid; i < HEAD_OUT * 32; i += 128)
+    for (int i = tid; i < HEAD_OUT * 32; i += 256)
         *reinterpret_cast<float4*>(sw + (i >> 5) * HEAD_PITCH + 4 * (i & 31)) = __ldg(reinterpret_cast<const float4*>(W) + i);
-    const int og = (tid & 3) * 6, row = tid >> 2;            // rows row, row + 32, row + 64, row + 96
+    const int og = (tid & 3) * 6, row = tid >> 2;            // rows row, row + 64
     for (int64_t r0 = (int64_t)blockIdx.x * HEAD_ROWS; r0 < n; r0 += (int64_t)gridDim.x * HEAD_ROWS) {
         __syncthreads();
         const int m = (int)min((int64_t)HEAD_ROWS, n - r0);
 #pragma unroll 8
-        for (int i = 0; i < 32; ++i) {
-            const int r = 4 * i + (tid >> 5), c = tid & 31;
+        for (int i = 0; i < 16; ++i) {
+            const int r = 8 * i + (tid >> 5), c = tid & 31;
             if (r < m) *reinterpret_cast<float4*>(sx + r * HEAD_PITCH + 4 * c) = __ldg(reinterpret_cast<const float4*>(x + (r0 + r) * MD) + c);
         }
         __syncthreads();
-        float y[4][6];
+        float y[2][6];
 #pragma unroll
         for (int o = 0; o < 6; ++o) {
             const float b = bias ? __ldg(bias + og + o) : 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) y[i][o] = b;
+            for (int i = 0; i < 2; ++i) y[i][o] = b;
         }
 #pragma unroll 2
         for (int c = 0; c < MD; c += 4) {
-            float4 v[4], w[6];
+            float4 v[2], w[6];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(sx + (row + 32 * i) * HEAD_PITCH + c);
+            for (int i = 0; i < 2; ++i) v[i] = *reinterpret_cast<const float4*>(sx + (row + 64 * i) * HEAD_PITCH + c);
 #pragma unroll
             for (int o = 0; o < 6; ++o) w[o] = *reinterpret_cast<const float4*>(sw + (og + o) * HEAD_PITCH + c);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int o = 0; o < 6; ++o)
                     y[i][o] = fmaf(v[i].w, w[o].w, fmaf(v[i].z, w[o].z, fmaf(v[i].y, w[o].y, fmaf(v[i].x, w[o].x, y[i][o]))));
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (row + 32 * i < m)
+        for (int i = 0; i < 2; ++i)
+            if (row + 64 * i < m)
 #pragma unroll
                 for (int o = 0; o < 6; o += 2)
-                    *reinterpret_cast<float2*>(out + (r0 + row + 32 * i) * HEAD_OUT + og + o) = make_float2(y[i][o], y[i][o + 1]);
+                    *reinterpret_cast<float2*>(out + (r0 + row + 64 * i) * HEAD_OUT + og + o) = make_float2(y[i][o], y[i][o + 1]);
     }
 }
 
@@ -333,14 +343,15 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 const int q = t * PJ_BLOCKS + m, buf = q & 1;
                 uint2 taps = make_uint2(0u, 0u);                 // this channel's four taps
                 if (m < 3) taps = __ldg(reinterpret_cast<const uint2*>(m == 0 ? a.conv[0] : m == 1 ? a.conv[1] : a.conv[2]) + ch);
-                mbar_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget);
+                // products complete, and the previous results have left the staging tile
+                epi_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget, [&] { if (tid == 0) bulk_wait_read(); });
                 tc_fence_after();
                 float x[32];                                     // X(i) = position i - 4
                 tmem_ld32(x, tl + 128 * buf);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dfree + buf);
-                uint32_t w[PJ_PART / 2];                         // the 28 results, packed before anybody waits for the staging tile
+                uint32_t w[PJ_PART / 2];                         // the 28 results
                 if (m < 3) {
                     float h1 = x[3], h2 = x[2], h3 = x[1];
                     const float2 ta = unpack_bf16x2(taps.x), tb = unpack_bf16x2(taps.y);
@@ -376,8 +387,6 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                     for (int i = 0; i < PJ_PART; ++i)
                         if (PJ_PART * part + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(x[4 + i] + sp_add) : sigmoid_fast(x[4 + i]);
                 }
-                if (tid == 0) bulk_wait_read();                  // the previous results have left the staging tile
-                epi_sync();
                 uint16_t* st = reinterpret_cast<uint16_t*>(sST) + ch;
                 if (m < 4) {
                     st += PJ_PART * part * MD;
@@ -621,7 +630,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             }
             operand_ready();
             // ---- x += o_proj at the hit's row, norm: the operand of the MLP ----
-            mbar_wait(macc, 0u, dead, a.status, 630, a.budget);
+            epi_wait(macc, 0u, dead, a.status, 630, a.budget, [] {});
             tc_fence_after();
             stage_acc(nullptr);
             epi_sync();
@@ -664,7 +673,10 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     const __nv_bfloat16* base = (lane & 2) ? a.gate : a.o;
                     if (j < a.n) asm volatile("prefetch.global.L2 [%0];\n" :: "l"(base + j * MD + 64 * (lane & 1)));
                 }
-                mbar_wait(mup + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 631, a.budget);
+                // up product complete, and the hidden operand of two chunks ago consumed
+                epi_wait(mup + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 631, a.budget, [&] {
+                    if (q >= 2) mbar_wait(hfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 632, a.budget);
+                });
                 tc_fence_after();
                 float x[16];
                 tmem_ld16(x, tl + UT_UP + 64 * buf + 16 * part);
@@ -680,7 +692,6 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                     gelu_pair(x[2 * e] + f.x, x[2 * e + 1] + f.y, y0, y1);
                     w[e] = pack_bf16x2(y0, y1);
                 }
-                if (q >= 2) mbar_wait(hfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 632, a.budget);
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
                     *reinterpret_cast<uint4*>(sH + buf * MST + op_off(trow, 16 * part + 8 * e, 0)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
@@ -689,7 +700,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
                 if (lane == 0) mbar_arrive(hready + buf);
             }
             // ---- x += MLP, the next block's norm ----
-            mbar_wait(macc, 1u, dead, a.status, 633, a.budget);
+            epi_wait(macc, 1u, dead, a.status, 633, a.budget, [] {});
             tc_fence_after();
             stage_acc(a.down_b);
             tc_fence_before();
@@ -759,7 +770,7 @@ extern "C" int lampa_model_head(const float* x, const float* weight, const float
     static std::atomic<uint64_t> ready{0};
     if (!allow_smem(ready, model_head_kernel, HEAD_SMEM)) return LAMPA_ERR_CUDA;
     const int64_t want = (n + HEAD_ROWS - 1) / HEAD_ROWS, most = (int64_t)sm_count() * 2;
-    model_head_kernel<<<(unsigned)(want < most ? want : most), 128, HEAD_SMEM, (cudaStream_t)stream>>>(x, weight, bias, n, out);
+    model_head_kernel<<<(unsigned)(want < most ? want : most), 256, HEAD_SMEM, (cudaStream_t)stream>>>(x, weight, bias, n, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
