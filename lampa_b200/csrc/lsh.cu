@@ -74,18 +74,21 @@ lsh_hash_kernel(const float* __restrict__ x, int64_t row_stride, int64_t head_st
 // (no flag spinning anywhere).  The cluster size is the largest one for which the occupancy
 // calculator reports all clusters resident at once: a cluster lives inside one GPC, and a size that
 // merely divides the SM count left a third of the clusters waiting for a second wave (103 us
-// against 57 us for the 24 x 60 000 keys of the benchmark).  Keys are reduced to (key - min) first,
-// so only ceil(bits(range)/8) passes run: two for the ~15-bit bucket ids of this workload.  A CTA
-// keeps its slice of the current pass in shared memory when it fits (filled by the histogram sweep,
-// read back by the scatter) and walks it in tiles of 4096 keys; a warp takes 128 consecutive keys
-// as four rounds of 32, ranking each round with ballots on top of a per-warp digit histogram, so
-// the order (round, lane) is the key order and the sort is stable.
+// against 57 us for 24 x 60 000 keys).  Keys are reduced to (key - min) first, so only as many
+// passes of up to 8 bits run as the key range needs: two for the ~15-bit bucket ids of an event.
+//
+// A CTA takes its slice in tiles of ITEMS * 1024 keys held in registers; a warp owns ITEMS * 32
+// consecutive keys and ranks them 32 at a time with one ballot per digit bit on top of its row of
+// digit counters, so the order (round, lane) is the key order and the sort is stable.  What bounds a
+// pass is instruction issue and its fixed chain of barriers, so the tile is as large as the slice
+// where it fits (the counters then double as the histogram: no separate sweep), the prefix over the
+// 32 warps' counters is one thread per digit (a warp-wide scan per digit cost as much as the
+// ranking), and the tile is grouped by digit in shared memory so that the writes are runs.
 // -------------------------------------------------------------------------------------------------
 constexpr int SORT_THREADS = 1024;
 constexpr int SORT_MAX_CL = 8;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-constexpr int SORT_ITEMS = 4;
-constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
+constexpr int SORT_MAX_ITEMS = 12;
 
 __device__ __forceinline__ uint32_t key_xform(const void* keys, int key_type, int64_t i) {
     uint32_t u = ((const uint32_t*)keys)[i];
@@ -95,11 +98,31 @@ __device__ __forceinline__ uint32_t key_xform(const void* keys, int key_type, in
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// exclusive prefix over 256 values held by threads 0..255 (one each); wtot: 8 words of shared memory.  All threads call it.
+__device__ __forceinline__ uint32_t prefix256(uint32_t v, uint32_t* wtot, int tid) {
+    const int lane = tid & 31, warp = tid >> 5;
+    uint32_t incl = v;
+    if (tid < 256) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wtot[warp] = incl;
+    }
+    __syncthreads();
+    if (tid < 256)
+        for (int w = 0; w < warp; ++w) incl += wtot[w];
+    return incl - v;
+}
+
+template <int ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS, 1)
 segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                const int64_t* __restrict__ seg, int nseg, const int64_t* __restrict__ init,
                int64_t* __restrict__ perm, uint32_t* kbuf0, uint32_t* kbuf1, uint32_t* ibuf0,
-               uint32_t* ibuf1, int cache_cap, int32_t* status) {
+               uint32_t* ibuf1, int32_t* status) {
+    constexpr int TILE = ITEMS * SORT_THREADS;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int ncl = (int)cluster.num_blocks();
@@ -115,58 +138,50 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
     }
     const int64_t per = (n + ncl - 1) / ncl;
     const int64_t lo = min((int64_t)rank * per, n), hi = min(lo + per, n);
+    const bool one_tile = hi - lo <= TILE;
 
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t dbase[256];
-    __shared__ uint32_t tile_tot[256];
-    __shared__ uint32_t wtot[8];
-    __shared__ uint32_t red[2];
-    __shared__ uint32_t wcount[SORT_WARPS][257];   // +1: a column (one digit across the warps) is conflict-free
-    __shared__ uint32_t tstart[256];
-    extern __shared__ uint32_t sort_dyn[];         // [SORT_TILE] keys, [SORT_TILE] indices of the tile, grouped by digit
+    __shared__ uint32_t hist[256], dbase[256], tstart[256], tile_tot[256];
+    __shared__ uint32_t wtot[8], red[2];
+    __shared__ __align__(16) uint16_t wcount[SORT_WARPS][256];
+    extern __shared__ uint32_t sort_dyn[];         // [TILE] keys, [TILE] indices of the tile, grouped by digit
     uint32_t* skey = sort_dyn;
-    uint32_t* sidx = sort_dyn + SORT_TILE;
-    // the CTA's slice (keys and indices of the current pass) stays in shared memory when it fits:
-    // the histogram sweep fills it and the scatter reads it back instead of going to L2 again
-    uint32_t* ckey = sort_dyn + 2 * SORT_TILE;
-    uint32_t* cidx = ckey + cache_cap;
-    const bool cached = (hi - lo) <= (int64_t)cache_cap;
+    uint32_t* sidx = sort_dyn + TILE;
+
+    uint32_t u[ITEMS], idx[ITEMS];
+    const int wpos = warp * (32 * ITEMS) + lane;   // of item 0; item `it` is 32 * it further
+    // keys of a tile in their current order: position i of the first pass holds element init[i]
+    auto load_tile = [&](int64_t t0, int p, const uint32_t* ksrc, const uint32_t* isrc, uint32_t base) {
+        if (p == 0) {
+#pragma unroll
+            for (int it = 0; it < ITEMS; ++it) {
+                const int64_t i = t0 + wpos + it * 32;
+                idx[it] = i < hi ? (init ? (uint32_t)init[s0 + i] : (uint32_t)i) : 0u;
+            }
+#pragma unroll
+            for (int it = 0; it < ITEMS; ++it) u[it] = t0 + wpos + it * 32 < hi ? key_xform(keys, key_type, s0 + idx[it]) - base : 0u;
+        } else {
+#pragma unroll
+            for (int it = 0; it < ITEMS; ++it) {
+                const int64_t i = t0 + wpos + it * 32;
+                u[it] = i < hi ? ksrc[s0 + i] : 0u;
+                idx[it] = i < hi ? isrc[s0 + i] : 0u;
+            }
+        }
+    };
 
     // ---- key range over the whole segment -------------------------------------------------------
     if (tid == 0) { red[0] = 0xFFFFFFFFu; red[1] = 0u; }
     __syncthreads();
     {
         uint32_t mn = 0xFFFFFFFFu, mx = 0u;
-        if (cached) {   // position i holds element init[i]; four independent loads in flight per thread
-            for (int64_t i0 = lo + tid; i0 < hi; i0 += 4 * SORT_THREADS) {
-                uint32_t ix[4], u[4];
+        for (int64_t t0 = lo; t0 < hi; t0 += TILE) {
+            load_tile(t0, 0, nullptr, nullptr, 0u);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t i = i0 + (int64_t)q * SORT_THREADS;
-                    ix[q] = i < hi ? (init ? (uint32_t)init[s0 + i] : (uint32_t)i) : 0u;
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t i = i0 + (int64_t)q * SORT_THREADS;
-                    u[q] = i < hi ? key_xform(keys, key_type, s0 + ix[q]) : 0u;
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t i = i0 + (int64_t)q * SORT_THREADS;
-                    if (i < hi) { ckey[i - lo] = u[q]; cidx[i - lo] = ix[q]; mn = min(mn, u[q]); mx = max(mx, u[q]); }
-                }
-            }
-        } else {
-            for (int64_t i = lo + tid; i < hi; i += SORT_THREADS) {
-                const uint32_t u = key_xform(keys, key_type, s0 + i);
-                mn = min(mn, u); mx = max(mx, u);
-            }
+            for (int it = 0; it < ITEMS; ++it)
+                if (t0 + wpos + it * 32 < hi) { mn = min(mn, u[it]); mx = max(mx, u[it]); }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) { atomicMin(&red[0], mn); atomicMax(&red[1], mx); }
     }
     __syncthreads();
@@ -179,173 +194,121 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
     const uint32_t range = (n > 0 && gmx >= gmn) ? (gmx - gmn) : 0u;
     const int bits = range ? (32 - __clz(range)) : 0;
     const int npass = (bits + 7) / 8;
+    const int width = npass ? (bits + npass - 1) / npass : 0;        // digits of equal width: fewer ballots than 8 + the rest
 
     if (npass == 0) {
         for (int64_t i = lo + tid; i < hi; i += SORT_THREADS) perm[s0 + i] = init ? init[s0 + i] : i;
     }
 
     for (int p = 0; p < npass; ++p) {
-        const int shift = 8 * p;
+        const int shift = width * p;
+        const uint32_t dmask = (1u << width) - 1u;
         const uint32_t* ksrc = (p & 1) ? kbuf0 : kbuf1;   // pass p reads what pass p-1 wrote
         const uint32_t* isrc = (p & 1) ? ibuf0 : ibuf1;
         uint32_t* kdst = (p & 1) ? kbuf1 : kbuf0;
         uint32_t* idst = (p & 1) ? ibuf1 : ibuf0;
         const bool last = (p == npass - 1);
+        uint32_t rnk[(ITEMS + 1) / 2];                    // two 16-bit ranks (within warp and digit) per word
+
+        // digit counters of a tile: rank of every key within its warp and digit, then the exclusive prefix over the warps
+        auto rank_tile = [&](int64_t t0) {
+            for (int z = tid; z < SORT_WARPS * 256 / 8; z += SORT_THREADS) reinterpret_cast<uint4*>(&wcount[0][0])[z] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+#pragma unroll
+            for (int it = 0; it < ITEMS; ++it) {
+                const bool valid = t0 + wpos + it * 32 < hi;
+                const uint32_t d = (u[it] >> shift) & dmask;
+                uint32_t m = __ballot_sync(0xffffffffu, valid);
+                if (m == 0u) { if (!(it & 1)) rnk[it >> 1] = 0u; continue; }         // warp-uniform: past the slice's end
+#pragma unroll
+                for (int bit = 0; bit < 8; ++bit) {
+                    const bool one = (d >> bit) & 1u;
+                    const uint32_t bal = __ballot_sync(0xffffffffu, one);
+                    m &= one ? bal : ~bal;
+                }
+                const uint32_t basecnt = valid ? wcount[warp][d] : 0u;
+                const uint32_t r = basecnt + __popc(m & ((1u << lane) - 1u));
+                if (it & 1) rnk[it >> 1] |= r << 16; else rnk[it >> 1] = r;
+                __syncwarp();
+                if (valid && (__ffs(m) - 1) == lane) wcount[warp][d] = (uint16_t)(basecnt + __popc(m));
+                __syncwarp();
+            }
+            __syncthreads();
+            if (tid < 256) {
+                uint32_t run = 0;
+#pragma unroll 8
+                for (int w = 0; w < SORT_WARPS; ++w) {
+                    const uint32_t c = wcount[w][tid];
+                    wcount[w][tid] = (uint16_t)run;
+                    run += c;
+                }
+                tile_tot[tid] = run;
+            }
+        };
 
         // (a) digit histogram of this CTA's slice
-        for (int d = tid; d < 256; d += SORT_THREADS) hist[d] = 0;
-        __syncthreads();
-        if (cached) {
-            for (int64_t i0 = lo + tid; i0 < hi; i0 += 4 * SORT_THREADS) {
-                uint32_t u[4], ix[4];
+        if (one_tile) {
+            if (p == 0) {                                 // still in registers from the range sweep
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t i = i0 + (int64_t)q * SORT_THREADS;
-                    u[q] = 0u; ix[q] = 0u;
-                    if (i < hi) {
-                        if (p == 0) u[q] = ckey[i - lo] - gmn;
-                        else { u[q] = ksrc[s0 + i]; ix[q] = isrc[s0 + i]; }
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t i = i0 + (int64_t)q * SORT_THREADS;
-                    if (i < hi) {
-                        ckey[i - lo] = u[q];
-                        if (p > 0) cidx[i - lo] = ix[q];
-                        atomicAdd(&hist[(u[q] >> shift) & 255u], 1u);
-                    }
-                }
+                for (int it = 0; it < ITEMS; ++it) u[it] -= gmn;
+            } else if (lo < hi) {
+                load_tile(lo, p, ksrc, isrc, gmn);
             }
+            rank_tile(lo);
+            if (tid < 256) hist[tid] = tile_tot[tid];
         } else {
-            for (int64_t i = lo + tid; i < hi; i += SORT_THREADS) {
-                uint32_t u;
-                if (p == 0) u = key_xform(keys, key_type, s0 + (init ? init[s0 + i] : i)) - gmn;   // position i holds element init[i]
-                else u = ksrc[s0 + i];
-                atomicAdd(&hist[(u >> shift) & 255u], 1u);
+            if (tid < 256) hist[tid] = 0;
+            __syncthreads();
+            for (int64_t t0 = lo; t0 < hi; t0 += TILE) {
+                load_tile(t0, p, ksrc, isrc, gmn);
+#pragma unroll
+                for (int it = 0; it < ITEMS; ++it)
+                    if (t0 + wpos + it * 32 < hi) atomicAdd(&hist[(u[it] >> shift) & dmask], 1u);
             }
         }
         __syncthreads();
         cluster.sync();
 
         // (b) where each digit of this slice starts in the segment
-        uint32_t tot = 0, before = 0, incl = 0;
-        if (tid < 256) {
+        uint32_t tot = 0, before = 0;
+        if (tid < 256)
             for (int r = 0; r < ncl; ++r) {
                 const uint32_t hv = cluster.map_shared_rank(hist, r)[tid];
                 tot += hv;
                 if (r < rank) before += hv;
             }
-            incl = tot;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (lane == 31) wtot[warp] = incl;
-        }
-        __syncthreads();
-        if (tid < 256) {
-            uint32_t off = 0;
-            for (int w2 = 0; w2 < warp; ++w2) off += wtot[w2];
-            dbase[tid] = off + incl - tot + before;
-        }
+        const uint32_t ex = prefix256(tot, wtot, tid);
+        if (tid < 256) dbase[tid] = ex + before;
         __syncthreads();
 
         // (c) stable scatter, tile by tile in slice order
-        for (int64_t t0 = lo; t0 < hi; t0 += SORT_TILE) {
-            uint32_t u[SORT_ITEMS], idx[SORT_ITEMS], rnk[SORT_ITEMS], dg[SORT_ITEMS];
-#pragma unroll
-            for (int it = 0; it < SORT_ITEMS; ++it) {
-                const int64_t i = t0 + warp * (32 * SORT_ITEMS) + it * 32 + lane;
-                u[it] = 0; idx[it] = 0;
-                if (i < hi) {
-                    if (cached) {
-                        u[it] = ckey[i - lo];
-                        idx[it] = cidx[i - lo];
-                    } else if (p == 0) {
-                        idx[it] = init ? (uint32_t)init[s0 + i] : (uint32_t)i;
-                        u[it] = key_xform(keys, key_type, s0 + idx[it]) - gmn;
-                    } else {
-                        u[it] = ksrc[s0 + i];
-                        idx[it] = isrc[s0 + i];
-                    }
-                    dg[it] = (u[it] >> shift) & 255u;
-                } else {
-                    dg[it] = 256u;
-                }
+        for (int64_t t0 = lo; t0 < hi; t0 += TILE) {
+            if (!one_tile) {
+                load_tile(t0, p, ksrc, isrc, gmn);
+                rank_tile(t0);
+                __syncthreads();
             }
-            for (int z = tid; z < SORT_WARPS * 257; z += SORT_THREADS) (&wcount[0][0])[z] = 0;
-            __syncthreads();
-#pragma unroll
-            for (int it = 0; it < SORT_ITEMS; ++it) {
-                // lanes holding the same digit: eight ballots (one per bit) instead of match.any
-                uint32_t m = 0xffffffffu;
-#pragma unroll
-                for (int bit = 0; bit < 9; ++bit) {
-                    const uint32_t bal = __ballot_sync(0xffffffffu, (dg[it] >> bit) & 1u);
-                    m &= ((dg[it] >> bit) & 1u) ? bal : ~bal;
-                }
-                const bool valid = dg[it] < 256u;
-                const uint32_t basecnt = valid ? wcount[warp][dg[it]] : 0u;
-                rnk[it] = basecnt + __popc(m & ((1u << lane) - 1u));
-                __syncwarp();
-                if (valid && (__ffs(m) - 1) == lane) wcount[warp][dg[it]] = basecnt + __popc(m);
-                __syncwarp();
-            }
-            __syncthreads();
-            // exclusive scan over the warps, per digit: warp w takes digits w, w + 32, ...; lane = source warp
-#pragma unroll
-            for (int q = 0; q < 256 / SORT_WARPS; ++q) {
-                const int d = warp + q * SORT_WARPS;
-                const uint32_t c = wcount[lane][d];
-                uint32_t incl2 = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl2, o);
-                    if (lane >= o) incl2 += y;
-                }
-                wcount[lane][d] = incl2 - c;
-                if (lane == 31) tile_tot[d] = incl2;
-            }
-            __syncthreads();
-            // where each digit starts inside the tile (exclusive scan of the tile's digit counts)
-            uint32_t tt = 0, ti = 0;
-            if (tid < 256) {
-                tt = tile_tot[tid];
-                ti = tt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, ti, o);
-                    if (lane >= o) ti += y;
-                }
-                if (lane == 31) wtot[warp] = ti;
-            }
-            __syncthreads();
-            if (tid < 256) {
-                uint32_t off = 0;
-                for (int w2 = 0; w2 < warp; ++w2) off += wtot[w2];
-                tstart[tid] = off + ti - tt;
-            }
+            const uint32_t ts = prefix256(tid < 256 ? tile_tot[tid] : 0u, wtot, tid);
+            if (tid < 256) tstart[tid] = ts;
             __syncthreads();
             // group the tile by digit in shared memory, so that the global writes below are runs of
             // consecutive addresses (a direct scatter costs one 32-byte sector per key)
 #pragma unroll
-            for (int it = 0; it < SORT_ITEMS; ++it) {
-                if (dg[it] < 256u) {
-                    const uint32_t lp = tstart[dg[it]] + wcount[warp][dg[it]] + rnk[it];
+            for (int it = 0; it < ITEMS; ++it)
+                if (t0 + wpos + it * 32 < hi) {
+                    const uint32_t d = (u[it] >> shift) & dmask;
+                    const uint32_t lp = tstart[d] + wcount[warp][d] + ((rnk[it >> 1] >> (16 * (it & 1))) & 0xffffu);
                     skey[lp] = u[it];
                     sidx[lp] = idx[it];
                 }
-            }
             __syncthreads();
-            const int ntile = (int)min((int64_t)SORT_TILE, hi - t0);
+            const int ntile = (int)min((int64_t)TILE, hi - t0);
 #pragma unroll
-            for (int it = 0; it < SORT_ITEMS; ++it) {
+            for (int it = 0; it < ITEMS; ++it) {
                 const int lp = it * SORT_THREADS + tid;
                 if (lp < ntile) {
                     const uint32_t ku = skey[lp], ki = sidx[lp];
-                    const uint32_t d = (ku >> shift) & 255u;
+                    const uint32_t d = (ku >> shift) & dmask;
                     const int64_t pos = (int64_t)dbase[d] + (lp - tstart[d]);
                     if (last) {
                         perm[s0 + pos] = (int64_t)ki;
@@ -355,12 +318,15 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                     }
                 }
             }
-            __syncthreads();
-            if (tid < 256) dbase[tid] += tile_tot[tid];
+            if (t0 + TILE < hi) {
+                __syncthreads();
+                if (tid < 256) dbase[tid] += tile_tot[tid];
+                __syncthreads();
+            }
         }
         cluster.sync();   // release/acquire at cluster scope: scattered keys visible to the peers; histograms free again
     }
-    cluster.sync();       // no CTA leaves while a peer may still read its shared memory
+    if (npass == 0) cluster.sync();       // no CTA leaves while a peer may still read its shared memory
 }
 
 // Upper bound of the cluster size for nseg segments: SMs / segments, at most 8 (the launcher lowers it until all fit).
@@ -373,19 +339,20 @@ static int sort_cluster_size(int nseg) {
     return cl;
 }
 
-// cudaOccupancyMaxActiveClusters for this kernel, remembered per (device, cluster size, cache size):
+// cudaOccupancyMaxActiveClusters for a kernel, remembered per (device, cluster size, tile):
 // the answer does not change and the query costs tens of microseconds of host time.
-static int clusters_resident(const cudaLaunchConfig_t& cfg, int cl, int cache_cap) {
+template <typename K>
+static int clusters_resident(K kernel, const cudaLaunchConfig_t& cfg, int cl, int items) {
     static std::mutex mu;
     static std::map<std::tuple<int, int, int>, int> memo;
     int dev = 0;
     cudaGetDevice(&dev);
-    const auto key = std::make_tuple(dev, cl, cache_cap);
+    const auto key = std::make_tuple(dev, cl, items);
     std::lock_guard<std::mutex> lk(mu);
     const auto it = memo.find(key);
     if (it != memo.end()) return it->second;
     int resident = 0;
-    if (cudaOccupancyMaxActiveClusters(&resident, segsort_kernel, &cfg) != cudaSuccess) resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess) resident = 0;
     memo[key] = resident;
     return resident;
 }
@@ -393,23 +360,27 @@ static int clusters_resident(const cudaLaunchConfig_t& cfg, int cl, int cache_ca
 static int launch_segsort(const void* keys, int key_type, int64_t n_total, const int64_t* seg, int nseg,
                           const int64_t* init, int64_t* perm, uint32_t* k0, uint32_t* k1, uint32_t* i0,
                           uint32_t* i1, int32_t* status, cudaStream_t st) {
-    if (cudaFuncSetAttribute(segsort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * SORT_TILE + 2 * 12288) * 4) != cudaSuccess)
-        return LAMPA_ERR_CUDA;
+    using Kernel = void (*)(const void*, int, int64_t, const int64_t*, int, const int64_t*, int64_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int32_t*);
+    static const Kernel kernels[] = {segsort_kernel<1>, segsort_kernel<2>, segsort_kernel<4>, segsort_kernel<8>, segsort_kernel<SORT_MAX_ITEMS>};
+    static const int item_counts[] = {1, 2, 4, 8, SORT_MAX_ITEMS};
+    static std::atomic<uint64_t> ready[5];
     // Cluster size: the largest one for which every segment's cluster is resident at the same time.
     // A cluster has to fit inside one GPC, so the SM count alone does not tell (148 SMs hold 24
     // clusters of 6 only if every GPC has 18 usable SMs): ask the occupancy calculator.
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    int cl = sort_cluster_size(nseg), cache_cap = 0;
+    int cl = sort_cluster_size(nseg), which = 0;
     for (;; --cl) {
-        // slice cache: the slice of an equal split, or twice the average slice when the segments are ragged
-        // (larger slices simply read from global memory), rounded up to 1 K keys, at most 12 K (96 KB)
+        // tile: the slice of an equal split, or twice the average slice when the segments are ragged (larger slices
+        // take several tiles), at most 12 keys per thread (96 KB)
         const int64_t avg = (n_total / (nseg > 0 ? nseg : 1) + cl - 1) / cl + 1;
         const int64_t want = seg ? 2 * avg : avg;
-        cache_cap = (int)std::min<int64_t>(12288, (want + 1023) / 1024 * 1024);
+        which = 0;
+        while (which < 4 && (int64_t)item_counts[which] * SORT_THREADS < want) ++which;
+        if (!allow_smem(ready[which], kernels[which], 2 * item_counts[which] * SORT_THREADS * 4)) return LAMPA_ERR_CUDA;
         cfg.gridDim = dim3((unsigned)nseg * cl, 1, 1);
         cfg.blockDim = dim3(SORT_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = (2 * SORT_TILE + 2 * (size_t)cache_cap) * sizeof(uint32_t);
+        cfg.dynamicSmemBytes = (size_t)2 * item_counts[which] * SORT_THREADS * 4;
         cfg.stream = st;
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = cl;
@@ -418,10 +389,9 @@ static int launch_segsort(const void* keys, int key_type, int64_t n_total, const
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         if (cl == 1) break;
-        if (clusters_resident(cfg, cl, cache_cap) >= nseg) break;
+        if (clusters_resident(kernels[which], cfg, cl, item_counts[which]) >= nseg) break;
     }
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, segsort_kernel, keys, key_type, n_total, seg, nseg, init, perm,
-                                             k0, k1, i0, i1, cache_cap, status);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], keys, key_type, n_total, seg, nseg, init, perm, k0, k1, i0, i1, status);
     return e == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
