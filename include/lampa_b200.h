@@ -458,6 +458,33 @@ int lampa_debug_force_mma_sync(int on);
 int lampa_debug_set_tick_buffer(long long* ticks, int n_ctas);
 
 /*
+ * Front of the attention layer in one pass: lampa_hept_prep_qk's rows (value given), the projections of lampa_lsh_hash with
+ * per-head rows, proj fp32 [2 (query, key)][rounds][heads][n], and per block of 32 hits the (min, max) of every row over
+ * both, part fp32 [rounds * heads][blocks][2] with blocks from lampa_hept_front_blocks.  alpha [heads, d + cd, rounds].
+ * Replaces: models/attention/hept.py:118-131 up to the keys.
+ */
+int lampa_hept_front_blocks(int64_t n, int64_t* blocks);
+int lampa_hept_front(const float* query, const float* key, const float* value, const float* scale, const float* coords,
+                     const float* alpha, int64_t n, int32_t heads, int32_t d, int32_t cd, int32_t rounds, int32_t ldq,
+                     int64_t raw_size, float* q_hat, float* k_hat, float* v_out, float* proj, float* part, void* stream);
+/*
+ * lampa_row_range + lampa_geo_keys for queries and keys in place over `proj` [2][rows][n], from the partial ranges above.
+ */
+int lampa_geo_keys_fused(float* proj, const float* part, int64_t blocks, const int64_t* rank_eta, const int64_t* rank_phi,
+                         const float* regions_eta, const float* regions_phi, int32_t rows, int64_t n, int64_t raw_size, void* stream);
+/*
+ * Region numbers of one event: pads the coordinates to n rows (zeros), ranks the first two columns (stable, +inf in the
+ * padding) and numbers the regions.
+ * Replaces: prepare_input (models/hattention/modeling_gated_deltaproduct.py:1200-1223) with quantile_partition
+ * (models/model_utils/hash_utils.py:14-27).
+ *   coords [raw][cols >= 2], regions [nc][2][nh]; padded [n][cols], regions_h [2][nc * nh], region_indices [2][nc * nh][n],
+ *   ranks and perm int64 [2][n], keys [2][n] scratch; ws: lampa_segsort_workspace_bytes(2 n).
+ */
+int lampa_region_inputs(const float* coords, int64_t raw, int64_t n, int32_t cols, const float* regions, int32_t nc,
+                        int32_t nh, float* padded, float* regions_h, float* region_indices, int64_t* ranks, int64_t* perm,
+                        float* keys, void* ws, size_t ws_bytes, int32_t* status, void* stream);
+
+/*
  * The dense half of a model block around the mixer, for d_model = 128, 4-tap short convolutions without bias, bf16 weights
  * (matrices [out][in]) and heads with H * K = H * V = 128; LAMPA_ERR_UNSUPPORTED for anything else (the caller then
  * composes the block from the other entry points).  `perm` int64 [n]: the block's order, local to each event of `cu`.

@@ -41,6 +41,7 @@ EXPORTS = ["lampa_version", "lampa_error_string", "lampa_gdn_workspace_bytes", "
            "lampa_permute_rows", "lampa_invert_perm", "lampa_segsort_stable_static",
            "lampa_short_conv_fwd", "lampa_short_conv_step", "lampa_gate_inputs", "lampa_rmsnorm_gate", "lampa_add_rmsnorm",
            "lampa_row_range", "lampa_quantile_regions", "lampa_geo_keys",
+           "lampa_hept_front_blocks", "lampa_hept_front", "lampa_geo_keys_fused", "lampa_region_inputs",
            "lampa_bucket_rbf_attn", "lampa_bucket_attn_combine", "lampa_hept_prep_qk",
            "lampa_hgdn_fwd_again", "lampa_model_encode", "lampa_model_project", "lampa_model_update", "lampa_model_head",
            "lampa_repeat_segments", "lampa_profile_enable",

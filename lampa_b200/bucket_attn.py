@@ -17,6 +17,7 @@ import torch
 
 from . import _lib as L
 from .geo import hept_positions
+from .lsh import E2LSH
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -158,6 +159,11 @@ def hept_attention_core(e2lsh, query: torch.Tensor, key: torch.Tensor, value: to
     """HEPTAttention.forward between the projections and `out_linear`: query, key, value
     [N, heads, d] (N padded to block_size), coords [N, r + 1] with the padded rows zeroed, `ranks`
     the (eta, phi) ranks of the hits (geo.region_inputs) -> [heads, N, d]."""
+    if type(e2lsh) is E2LSH and not e2lsh._forward_hooks and not e2lsh._forward_pre_hooks and w.is_cuda:
+        out = L.native.hept_core(e2lsh.alpha, query, key, value, _coord_scale(w.detach()), coords, regions_h, ranks[0], ranks[1],
+                                 int(raw_size), int(block_size))
+        if out is not None:
+            return out
     q_hat, k_hat, v = prep_qk(query, key, w, coords, value=value, raw_size=raw_size, head_major=True)
     q_pos, k_pos = hept_positions(e2lsh, q_hat, k_hat, regions_h, ranks, raw_size)
     return hept_bucket_attention(q_hat, k_hat, v, q_pos, k_pos, block_size)

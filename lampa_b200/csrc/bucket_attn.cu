@@ -264,16 +264,273 @@ __global__ void __launch_bounds__(BA_MAX_WARPS * 32, BA_QROWS == 4 ? 3 : 2) buck
     }
 }
 
-// out[row][col] = (sum over rounds of so) / (sum over rounds of denom), rounds added in order
+// -------------------------------------------------------------------------------------------------
+// Rows of at most 64 features: the same bucket on the tensor cores, at fp32 accuracy.  A float is
+// carried exactly by three bf16 pieces (hi + mid + lo, 8 significant bits each); of the nine products of
+// two such sums the six larger ones are issued (hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi, smallest
+// first), the other three are below 2^-24 of the result, and accumulation is fp32.  The FMA kernel above
+// is bound by instruction issue (64 k warp instructions per bucket, 71 % of the issue slots); this one
+// spends 2 k tensor-core instructions and 10 k others.
+// Warp = 16 query rows x all keys.  Keys and values are gathered, split once and kept as bf16 tiles in
+// shared memory; queries go from global memory straight into operand fragments, and the weights p from
+// their accumulators into the operand fragments of p V (the two layouts coincide), so that neither
+// touches shared memory.  Measured at the sizes above: 0.97 ms -> see bucket_attn's numbers in the table.
+// -------------------------------------------------------------------------------------------------
+struct Split3 { uint32_t h, m, l; };
+__device__ __forceinline__ Split3 split3(float x, float y) {
+    Split3 s;
+    s.h = pack_bf16x2(x, y);
+    const float2 h = unpack_bf16x2(s.h);
+    const float rx = x - h.x, ry = y - h.y;
+    s.m = pack_bf16x2(rx, ry);
+    const float2 m = unpack_bf16x2(s.m);
+    s.l = pack_bf16x2(rx - m.x, ry - m.y);
+    return s;
+}
+// c[i] += a b_i for operands in three pieces and NT column tiles (two per fragment); one product of every tile after the
+// other, so that consecutive instructions do not wait for each other's accumulator
+template <int NT>
+__device__ __forceinline__ void mma6(float (*c)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
+                                     const uint32_t (&bh)[(NT + 1) / 2][4], const uint32_t (&bm)[(NT + 1) / 2][4], const uint32_t (&bl)[(NT + 1) / 2][4]) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], al, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bl[i / 2][2 * (i & 1)], bl[i / 2][2 * (i & 1) + 1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], am, bm[i / 2][2 * (i & 1)], bm[i / 2][2 * (i & 1) + 1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], am, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bm[i / 2][2 * (i & 1)], bm[i / 2][2 * (i & 1) + 1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
+}
+__host__ __device__ inline int bam_keys(int bucket) { return (bucket + 15) & ~15; }
+template <int KQ, int NV>
+__host__ __device__ constexpr int bam_smem(int keys) { return 4 * 128 * 8 + keys * 3 * ((16 * KQ + 8) + (8 * ((NV + 1) & ~1) + 8)) * 2; }
+
+template <int KQ, int NV>      // 16-wide feature steps of q / k, 8-wide value column tiles
+__global__ void __launch_bounds__(256, 2) bucket_attn_mma_kernel(BucketAttnArgs a) {
+    constexpr int KP = 16 * KQ + 8, VP = 8 * ((NV + 1) & ~1) + 8;         // bf16 pitches: consecutive rows fall into different bank groups
+    extern __shared__ __align__(16) float ba_smem[];
+    const int bucket = a.bucket, keys = bam_keys(bucket), nthr = blockDim.x;     // nthr = 2 * keys
+    int64_t* sQpos = reinterpret_cast<int64_t*>(ba_smem);
+    int64_t* sKpos = sQpos + 128;
+    float* sKn = reinterpret_cast<float*>(sKpos + 128);      // -|k|^2 / 2
+    __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(ba_smem) + 4 * 128 * 8);   // [3][keys][KP]
+    __nv_bfloat16* sV = sK + 3 * keys * KP;                  // [3][keys][VP]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+
+    const int64_t nb = a.n / bucket;
+    const int64_t b = blockIdx.x % nb, hc = blockIdx.x / nb;
+    const int h = (int)(hc / a.rounds), c = (int)(hc % a.rounds);
+    const int64_t rh = (int64_t)c * a.heads + h;             // row of the positions and outputs
+    const int64_t row0 = b * bucket;
+    const float* qbase = a.q + c * a.in_round_stride_q + (size_t)h * a.n * a.ldq;
+    const float* kbase = a.k + c * a.in_round_stride_q + (size_t)h * a.n * a.ldq;
+    const float* vbase = a.v + c * a.in_round_stride_v + (size_t)h * a.n * a.ldv;
+
+    for (int j = tid; j < bucket; j += nthr) {
+        sQpos[j] = a.q_pos ? a.q_pos[rh * a.n + row0 + j] : row0 + j;
+        sKpos[j] = a.k_pos ? a.k_pos[rh * a.n + row0 + j] : row0 + j;
+    }
+    __syncthreads();
+    // ---- keys and values: eight lanes per row, four rows per lane group, all of their loads in flight at once ----
+    const int l8 = tid & 7, rstep = nthr >> 3;
+    {
+        float ss[4] = {0.f, 0.f, 0.f, 0.f};
+        float4 x[4], y[4];
+        auto fetch = [&](const float* base, int ld, int width, bool vec, int pc, float4 (&r)[4]) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int j = (tid >> 3) + it * rstep;
+                r[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j < bucket && 4 * pc < width) {
+                    const float* src = base + (size_t)sKpos[j] * ld + 4 * pc;
+                    if (vec) r[it] = __ldg(reinterpret_cast<const float4*>(src));
+                    else {
+                        r[it].x = __ldg(src);
+                        if (4 * pc + 1 < width) r[it].y = __ldg(src + 1);
+                        if (4 * pc + 2 < width) r[it].z = __ldg(src + 2);
+                        if (4 * pc + 3 < width) r[it].w = __ldg(src + 3);
+                    }
+                }
+            }
+        };
+        auto put = [&](__nv_bfloat16* base, int pitch, int pc, const float4 (&r)[4]) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int j = (tid >> 3) + it * rstep;
+                const Split3 p = split3(r[it].x, r[it].y), q = split3(r[it].z, r[it].w);
+                uint2* d = reinterpret_cast<uint2*>(base + j * pitch + 4 * pc);
+                d[0] = make_uint2(p.h, q.h);
+                d = reinterpret_cast<uint2*>(base + (keys + j) * pitch + 4 * pc);
+                d[0] = make_uint2(p.m, q.m);
+                d = reinterpret_cast<uint2*>(base + (2 * keys + j) * pitch + 4 * pc);
+                d[0] = make_uint2(p.l, q.l);
+            }
+        };
+        constexpr int NP = ((4 * KQ > 2 * NV ? 4 * KQ : 2 * NV) + 7) / 8;
+#pragma unroll
+        for (int pi = 0; pi < NP; ++pi) {
+            const int pc = l8 + 8 * pi;
+            if (8 * pi < 4 * KQ) fetch(kbase, a.ldq, a.dq, a.vec_qk, pc, x);
+            if (8 * pi < 2 * NV) fetch(vbase, a.ldv, a.dv, a.vec_v, pc, y);
+            if (8 * pi < 4 * KQ) {
+                put(sK, KP, pc, x);
+#pragma unroll
+                for (int it = 0; it < 4; ++it) {
+                    ss[it] = fmaf(x[it].x, x[it].x, ss[it]); ss[it] = fmaf(x[it].y, x[it].y, ss[it]);
+                    ss[it] = fmaf(x[it].z, x[it].z, ss[it]); ss[it] = fmaf(x[it].w, x[it].w, ss[it]);
+                }
+            }
+            if (8 * pi < 2 * NV) put(sV, VP, pc, y);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int it = 0; it < 4; ++it) ss[it] += __shfl_xor_sync(0xffffffffu, ss[it], o);
+        if (l8 == 0)
+#pragma unroll
+            for (int it = 0; it < 4; ++it) sKn[(tid >> 3) + it * rstep] = -0.5f * ss[it];
+    }
+    // ---- queries: this warp's 16 rows as operand fragments ----
+    const int m0 = 16 * warp;
+    uint32_t qh[KQ][4], qm[KQ][4], ql[KQ][4];
+    float qn[2] = {0.f, 0.f};
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int i = m0 + g + 8 * hh;
+        const float* src = qbase + (size_t)(i < bucket ? sQpos[i] : 0) * a.ldq;
+        float2 v[KQ][2];
+#pragma unroll
+        for (int kk = 0; kk < KQ; ++kk)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = 16 * kk + 8 * e + 2 * t;
+                v[kk][e] = make_float2(0.f, 0.f);
+                if (i < bucket && col < a.dq) {
+                    if (a.vec_qk) v[kk][e] = __ldg(reinterpret_cast<const float2*>(src + col));
+                    else { v[kk][e].x = __ldg(src + col); if (col + 1 < a.dq) v[kk][e].y = __ldg(src + col + 1); }
+                }
+            }
+#pragma unroll
+        for (int kk = 0; kk < KQ; ++kk)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                qn[hh] = fmaf(v[kk][e].x, v[kk][e].x, qn[hh]);
+                qn[hh] = fmaf(v[kk][e].y, v[kk][e].y, qn[hh]);
+                const Split3 s = split3(v[kk][e].x, v[kk][e].y);
+                qh[kk][hh + 2 * e] = s.h; qm[kk][hh + 2 * e] = s.m; ql[kk][hh + 2 * e] = s.l;
+            }
+        qn[hh] += __shfl_xor_sync(0xffffffffu, qn[hh], 1);
+        qn[hh] += __shfl_xor_sync(0xffffffffu, qn[hh], 2);
+        qn[hh] *= -0.5f;
+    }
+    __syncthreads();
+
+    const int mi = lane >> 3, r8 = lane & 7;
+    float o[NV][4], rowsum[2] = {0.f, 0.f};
+#pragma unroll
+    for (int nv = 0; nv < NV; ++nv) { o[nv][0] = o[nv][1] = o[nv][2] = o[nv][3] = 0.f; }
+    for (int n0 = 0; n0 < keys; n0 += 64) {
+        float acc[8][4];
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+#pragma unroll
+        for (int kk = 0; kk < KQ; ++kk)
+#pragma unroll
+            for (int nq = 0; nq < 2; ++nq) {                 // 32 keys: four column tiles
+                const int kb = n0 + 32 * nq;
+                if (kb >= keys) continue;
+                uint32_t bh[2][4], bm[2][4], bl[2][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {                // past the last 16 keys: the last ones again, results unused
+                    const uint32_t at = smem_u32(sK + (min(kb + 16 * x, keys - 16) + r8 + (mi >> 1) * 8) * KP + 16 * kk + (mi & 1) * 8);
+                    ldsm_x4(bh[x], at);
+                    ldsm_x4(bm[x], at + keys * KP * 2);
+                    ldsm_x4(bl[x], at + 2 * keys * KP * 2);
+                }
+                mma6<4>(&acc[4 * nq], qh[kk], qm[kk], ql[kk], bh, bm, bl);
+            }
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+            if (n0 + 16 * ks < keys) {
+                uint32_t ph[4], pm[4], pl[4];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int col = n0 + 16 * ks + 8 * e + 2 * t;
+                    const float2 kn = *reinterpret_cast<const float2*>(sKn + col);
+                    const bool in0 = col < bucket, in1 = col + 1 < bucket;
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const float p0 = in0 ? __expf(fminf((acc[2 * ks + e][2 * hh] + qn[hh]) + kn.x, 0.f)) : 0.f;
+                        const float p1 = in1 ? __expf(fminf((acc[2 * ks + e][2 * hh + 1] + qn[hh]) + kn.y, 0.f)) : 0.f;
+                        rowsum[hh] += p0 + p1;
+                        const Split3 s = split3(p0, p1);
+                        ph[2 * e + hh] = s.h; pm[2 * e + hh] = s.m; pl[2 * e + hh] = s.l;
+                    }
+                }
+#pragma unroll
+                for (int np = 0; np < NV; np += 4) {         // up to four column tiles at a time
+                    constexpr int NT = NV < 4 ? NV : 4;
+                    uint32_t bh[(NT + 1) / 2][4], bm[(NT + 1) / 2][4], bl[(NT + 1) / 2][4];
+#pragma unroll
+                    for (int x = 0; x < (NT + 1) / 2; ++x) {
+                        const uint32_t at = smem_u32(sV + (n0 + 16 * ks + r8 + (mi & 1) * 8) * VP + 8 * np + 16 * x + (mi >> 1) * 8);
+                        ldsm_x4_t(bh[x], at);
+                        ldsm_x4_t(bm[x], at + keys * VP * 2);
+                        ldsm_x4_t(bl[x], at + 2 * keys * VP * 2);
+                    }
+                    mma6<NT>(&o[np], ph, pm, pl, bh, bm, bl);
+                }
+            }
+    }
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        rowsum[hh] += __shfl_xor_sync(0xffffffffu, rowsum[hh], 1);
+        rowsum[hh] += __shfl_xor_sync(0xffffffffu, rowsum[hh], 2);
+        const int i = m0 + g + 8 * hh;
+        if (i >= bucket) continue;
+        const int64_t dst = a.scatter ? sQpos[i] : row0 + i;
+        float* orow = a.so + ((size_t)rh * a.n + dst) * a.dv;
+#pragma unroll
+        for (int nv = 0; nv < NV; ++nv) {
+            const int col = 8 * nv + 2 * t;
+            if (a.vec_store) {                               // dv % 4 == 0: the pair is inside and 8-byte aligned
+                if (col < a.dv) *reinterpret_cast<float2*>(orow + col) = make_float2(o[nv][2 * hh], o[nv][2 * hh + 1]);
+            } else {
+                if (col < a.dv) orow[col] = o[nv][2 * hh];
+                if (col + 1 < a.dv) orow[col + 1] = o[nv][2 * hh + 1];
+            }
+        }
+        if (t == 0) a.denom[(size_t)rh * a.n + dst] = rowsum[hh] + 1e-20f;
+    }
+}
+
+// out[row][col] = (sum over rounds of so) / (sum over rounds of denom), rounds added in order; V consecutive columns per thread
+template <int V>
 __global__ void __launch_bounds__(256)
 bucket_attn_combine_kernel(const float* __restrict__ so, const float* __restrict__ denom, int rounds,
                            int64_t rows, int dv, float* __restrict__ out) {
     const int64_t total = rows * dv;
-    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+    for (int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V; e < total; e += (int64_t)gridDim.x * 256 * V) {
         const int64_t row = e / dv;
-        float s = so[e], d = denom[row];
-        for (int c = 1; c < rounds; ++c) { s += so[(size_t)c * total + e]; d += denom[(size_t)c * rows + row]; }
-        out[e] = __fdiv_rn(s, d);
+        float s[V], d = denom[row];
+        if (V == 4) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(so + e));
+            s[0] = x.x; s[1 % V] = x.y; s[2 % V] = x.z; s[3 % V] = x.w;
+        } else s[0] = so[e];
+        for (int c = 1; c < rounds; ++c) {
+            if (V == 4) {
+                const float4 x = __ldg(reinterpret_cast<const float4*>(so + (size_t)c * total + e));
+                s[0] += x.x; s[1 % V] += x.y; s[2 % V] += x.z; s[3 % V] += x.w;
+            } else s[0] += so[(size_t)c * total + e];
+            d += denom[(size_t)c * rows + row];
+        }
+        if (V == 4)
+            *reinterpret_cast<float4*>(out + e) = make_float4(__fdiv_rn(s[0], d), __fdiv_rn(s[1 % V], d), __fdiv_rn(s[2 % V], d), __fdiv_rn(s[3 % V], d));
+        else out[e] = __fdiv_rn(s[0], d);
     }
 }
 
@@ -300,6 +557,91 @@ hept_prep_qk_kernel(const float* __restrict__ query, const float* __restrict__ k
             const float r = (live && col < d + cd) ? __fmul_rn(scale[h * cd + col - d], coords[(size_t)i * cd + col - d]) : 0.f;
             q_hat[e] = r;
             k_hat[e] = r;
+        }
+    }
+}
+
+// -------------------------------------------------------------------------------------------------
+// Front of the attention layer in one pass over the tokens: prep_qk's head-major rows (as above), the
+// E2LSH projections of both (operation order of lsh_hash_kernel), and per block of hits the smallest and
+// largest projection of every (round, head) row.  One after the other these passes read and wrote the
+// rows three times, and the generic hash walked a 128-byte row per lane (210 us for 480 000 rows); here a
+// CTA stages 32 tokens with all heads in shared memory, writes whole 4 KB runs per head, and a warp hashes
+// one head of its 32 hits.
+// -------------------------------------------------------------------------------------------------
+constexpr int HF_HITS = 32, HF_MAX_ROUNDS = 8;
+__host__ __device__ inline int hf_pitch(int heads, int d) { return heads * d | 1; }      // odd: a column of hits is conflict-free
+inline size_t hf_smem(int heads, int d, int cd, int rounds) {
+    return ((size_t)2 * HF_HITS * hf_pitch(heads, d) + HF_HITS * cd + (size_t)heads * cd + (size_t)heads * (d + cd) * rounds) * 4;
+}
+
+template <int R>
+__global__ void __launch_bounds__(256)
+hept_front_kernel(const float* __restrict__ query, const float* __restrict__ key, const float* __restrict__ value,
+                  const float* __restrict__ scale, const float* __restrict__ coords, const float* __restrict__ alpha,
+                  int64_t n, int heads, int d, int cd, int ldq, int64_t raw_size, float* __restrict__ q_hat,
+                  float* __restrict__ k_hat, float* __restrict__ v_out, float* __restrict__ proj, float2* __restrict__ part) {
+    extern __shared__ __align__(16) float hf[];
+    const int hd = heads * d, P = hf_pitch(heads, d), D = d + cd;
+    float* sq = hf;                             // [32][P] query rows, then key rows behind them
+    float* sk = sq + HF_HITS * P;
+    float* sc = sk + HF_HITS * P;               // [32][cd]
+    float* ss = sc + HF_HITS * cd;              // [heads][cd]
+    float* sa = ss + heads * cd;                // [heads][D][R]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * HF_HITS;
+    const int m = (int)max((int64_t)0, min((int64_t)HF_HITS, raw_size - i0));     // rows that hold a hit
+    const int rows = (int)min((int64_t)HF_HITS, n - i0);
+    for (int r = warp; r < HF_HITS; r += 8)
+        for (int c = lane; c < hd; c += 32) {
+            sq[r * P + c] = r < m ? __ldg(query + (i0 + r) * hd + c) : 0.f;
+            sk[r * P + c] = r < m ? __ldg(key + (i0 + r) * hd + c) : 0.f;
+            if (r < rows) {                     // values only change their layout
+                const int h = c / d;
+                v_out[((size_t)h * n + i0 + r) * d + c - h * d] = r < m ? __ldg(value + (i0 + r) * hd + c) : 0.f;
+            }
+        }
+    for (int e = tid; e < HF_HITS * cd; e += 256) sc[e] = e / cd < m ? __ldg(coords + i0 * cd + e) : 0.f;
+    for (int e = tid; e < heads * cd; e += 256) ss[e] = __ldg(scale + e);
+    for (int e = tid; e < heads * D * R; e += 256) sa[e] = __ldg(alpha + e);
+    __syncthreads();
+    for (int h = warp; h < heads; h += 8) {
+        for (int r = 0; r < rows; ++r)
+            for (int c = lane; c < ldq; c += 32) {
+                float x = 0.f, y = 0.f;
+                if (c < d) { x = sq[r * P + h * d + c]; y = sk[r * P + h * d + c]; }
+                else if (c < D && r < m) x = y = __fmul_rn(ss[h * cd + c - d], sc[r * cd + c - d]);
+                q_hat[((size_t)h * n + i0 + r) * ldq + c] = x;
+                k_hat[((size_t)h * n + i0 + r) * ldq + c] = y;
+            }
+        float aq[R], ak[R];
+        const float* al = sa + h * D * R;
+        for (int c = 0; c < D; ++c) {
+            float x, y;
+            if (c < d) { x = sq[lane * P + h * d + c]; y = sk[lane * P + h * d + c]; }
+            else x = y = lane < m ? __fmul_rn(ss[h * cd + c - d], sc[lane * cd + c - d]) : 0.f;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float w = al[c * R + r];
+                aq[r] = c == 0 ? __fmul_rn(x, w) : __fadd_rn(aq[r], __fmul_rn(x, w));
+                ak[r] = c == 0 ? __fmul_rn(y, w) : __fadd_rn(ak[r], __fmul_rn(y, w));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const size_t row = (size_t)r * heads + h;
+            float mn = INFINITY, mx = -INFINITY;
+            if (lane < rows) {
+                proj[row * n + i0 + lane] = aq[r];
+                proj[((size_t)R * heads + row) * n + i0 + lane] = ak[r];
+                mn = fminf(aq[r], ak[r]); mx = fmaxf(aq[r], ak[r]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            if (lane == 0) part[row * gridDim.x + blockIdx.x] = make_float2(mn, mx);
         }
     }
 }
@@ -350,6 +692,17 @@ extern "C" int lampa_bucket_rbf_attn(const float* q, const float* k, const float
     if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
     const int64_t units = (int64_t)rounds * heads * (n / bucket);
     if (units > 0x7fffffffLL) return LAMPA_ERR_UNSUPPORTED;
+    if (dq <= 64 && dv <= 64) {                            // what one 16-row warp tile holds in registers; wider rows stay on FMA
+        const int keys = bam_keys(bucket);
+        const bool q2 = dq <= 32, v3 = dv <= 24, v4 = dv <= 32;
+        auto mma = q2 ? (v3 ? bucket_attn_mma_kernel<2, 3> : v4 ? bucket_attn_mma_kernel<2, 4> : bucket_attn_mma_kernel<2, 8>)
+                      : (v4 ? bucket_attn_mma_kernel<4, 4> : bucket_attn_mma_kernel<4, 8>);
+        const int msmem = q2 ? (v4 ? bam_smem<2, 4>(keys) : bam_smem<2, 8>(keys)) : (v4 ? bam_smem<4, 4>(keys) : bam_smem<4, 8>(keys));
+        if (cudaFuncSetAttribute(mma, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem) != cudaSuccess) return LAMPA_ERR_CUDA;
+        ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
+        mma<<<(unsigned)units, 2 * keys, msmem, (cudaStream_t)stream>>>(a);
+        return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+    }
     auto kernel = wide ? bucket_rbf_attn_kernel<8> : bucket_rbf_attn_kernel<4>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
@@ -365,8 +718,10 @@ extern "C" int lampa_bucket_attn_combine(const float* so, const float* denom, in
     if (!so || !denom || !out) return LAMPA_ERR_ARG;
     ProfScope prof("bucket_attn_combine", (cudaStream_t)stream);
     const int64_t total = rows * dv;
-    const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    bucket_attn_combine_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(so, denom, rounds, rows, dv, out);
+    const bool v4 = dv % 4 == 0 && (((uintptr_t)so | (uintptr_t)out) & 15) == 0;
+    const unsigned grid = (unsigned)std::min<int64_t>((total / (v4 ? 4 : 1) + 255) / 256, 148 * 32);
+    if (v4) bucket_attn_combine_kernel<4><<<grid, 256, 0, (cudaStream_t)stream>>>(so, denom, rounds, rows, dv, out);
+    else bucket_attn_combine_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(so, denom, rounds, rows, dv, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -382,5 +737,31 @@ extern "C" int lampa_hept_prep_qk(const float* query, const float* key, const fl
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
     hept_prep_qk_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(query, key, value, scale, coords, n, heads, d, cd,
                                                                  ldq, raw_size, q_hat, k_hat, v_out);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+extern "C" int lampa_hept_front_blocks(int64_t n, int64_t* blocks) {
+    if (n < 0 || !blocks) return LAMPA_ERR_ARG;
+    *blocks = (n + HF_HITS - 1) / HF_HITS;
+    return LAMPA_OK;
+}
+
+extern "C" int lampa_hept_front(const float* query, const float* key, const float* value, const float* scale, const float* coords,
+                                const float* alpha, int64_t n, int32_t heads, int32_t d, int32_t cd, int32_t rounds, int32_t ldq,
+                                int64_t raw_size, float* q_hat, float* k_hat, float* v_out, float* proj, float* part, void* stream) {
+    if (n < 0 || heads <= 0 || d <= 0 || cd <= 0 || rounds <= 0 || raw_size < 0 || ldq < d + cd) return LAMPA_ERR_ARG;
+    if (n == 0) return LAMPA_OK;
+    if (!query || !key || !value || !scale || !coords || !alpha || !q_hat || !k_hat || !v_out || !proj || !part) return LAMPA_ERR_ARG;
+    const size_t smem = hf_smem(heads, d, cd, rounds);
+    if (rounds > HF_MAX_ROUNDS || smem > 200 * 1024) return LAMPA_ERR_UNSUPPORTED;
+    using K = void (*)(const float*, const float*, const float*, const float*, const float*, const float*, int64_t, int, int, int, int, int64_t,
+                       float*, float*, float*, float*, float2*);
+    static const K kernels[HF_MAX_ROUNDS] = {hept_front_kernel<1>, hept_front_kernel<2>, hept_front_kernel<3>, hept_front_kernel<4>,
+                                             hept_front_kernel<5>, hept_front_kernel<6>, hept_front_kernel<7>, hept_front_kernel<8>};
+    const K kernel = kernels[rounds - 1];
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LAMPA_ERR_CUDA;
+    ProfScope prof("hept_front", (cudaStream_t)stream);
+    kernel<<<(unsigned)((n + HF_HITS - 1) / HF_HITS), 256, smem, (cudaStream_t)stream>>>(query, key, value, scale, coords, alpha, n, heads, d, cd, ldq,
+                                                                                        raw_size, q_hat, k_hat, v_out, proj, (float2*)part);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }

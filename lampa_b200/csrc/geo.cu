@@ -110,9 +110,111 @@ geo_keys_kernel(const float* __restrict__ proj, const float* __restrict__ reg_et
     }
 }
 
+// The shifted sort keys of queries and keys in place over their projections [2][rows][n], with the range of each row taken
+// from the partial (min, max) pairs the projection pass left per block of hits: one launch instead of a range reduction
+// (one CTA per row) and two key passes.  Grid: (chunks of hits, rows).
+constexpr int GEO_CHUNK = 4096;
+
+__global__ void __launch_bounds__(512)
+geo_keys_fused_kernel(float* __restrict__ proj, const float2* __restrict__ part, int nblk, const int64_t* __restrict__ rank_eta,
+                      const int64_t* __restrict__ rank_phi, const float* __restrict__ regions_eta,
+                      const float* __restrict__ regions_phi, int rows, int64_t n, int64_t raw_size) {
+    __shared__ float smn[16], smx[16];
+    const int r = blockIdx.y, tid = threadIdx.x;
+    float mn = INFINITY, mx = -INFINITY;
+    for (int i = tid; i < nblk; i += 512) {
+        const float2 p = __ldg(part + (size_t)r * nblk + i);
+        mn = fminf(mn, p.x); mx = fmaxf(mx, p.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((tid & 31) == 0) { smn[tid >> 5] = mn; smx[tid >> 5] = mx; }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 16; ++w) { mn = fminf(mn, smn[w]); mx = fmaxf(mx, smx[w]); }
+    const float hs = __fsub_rn(mx, mn), ne = regions_eta[r], np = regions_phi[r], stride = __fadd_rn(ceilf(ne), 1.f);
+    const int64_t se = region_size_of(n, ne), sp = region_size_of(n, np);
+    const int64_t end = min((int64_t)(blockIdx.x + 1) * GEO_CHUNK, n);
+    for (int64_t i = (int64_t)blockIdx.x * GEO_CHUNK + tid; i < end; i += 512) {
+        // ranks and region sizes are below 2^31 for any n the sort takes at once: a 32-bit division
+        const float e = (float)((uint32_t)rank_eta[i] / (uint32_t)se) + 1.f, p = (float)((uint32_t)rank_phi[i] / (uint32_t)sp) + 1.f;
+        const float shift = __fadd_rn(__fmul_rn(__fmul_rn(p, hs), stride), __fmul_rn(e, hs));
+        const size_t at = (size_t)r * n + i, at2 = at + (size_t)rows * n;
+        proj[at] = __fadd_rn(i < raw_size ? proj[at] : INFINITY, shift);
+        proj[at2] = __fadd_rn(i < raw_size ? proj[at2] : INFINITY, shift);
+    }
+}
+
+// Padded coordinates (padding rows zero), the eta and phi columns of all rows as sort keys (+inf in the padding), and the
+// regions as [a][c * h].  One thread per padded row.
+__global__ void __launch_bounds__(GEO_THREADS)
+region_prepare_kernel(const float* __restrict__ coords, int64_t raw, int64_t n, int cols, const float* __restrict__ regions,
+                      int nc, int na, int nh, float* __restrict__ padded, float* __restrict__ keys, float* __restrict__ regions_h) {
+    const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
+    if (i < n) {
+        for (int c = 0; c < cols; ++c) {
+            const float x = i < raw ? coords[i * cols + c] : 0.f;
+            padded[i * cols + c] = x;
+            if (c < 2) keys[c * n + i] = i < raw ? x : INFINITY;
+        }
+    }
+    if (i < (int64_t)nc * na * nh) {                      // regions [c][a][h] -> [a][c][h]
+        const int hh = (int)(i % nh), rest = (int)(i / nh), cc = rest % nc, aa = rest / nc;
+        regions_h[i] = regions[((int64_t)cc * na + aa) * nh + hh];
+    }
+}
+
+// ranks of both coordinates and their region numbers: rank[perm[i]] = i, out[r][hit] for the `rows` rows of regions_h
+__global__ void __launch_bounds__(GEO_THREADS)
+region_ranks_kernel(const int64_t* __restrict__ perm, const float* __restrict__ regions_h, int rows, int64_t n,
+                    int64_t* __restrict__ rank, float* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
+    const int a = blockIdx.y;
+    if (i >= n) return;
+    const int64_t hit = perm[a * n + i];
+    rank[a * n + hit] = i;
+    for (int r = 0; r < rows; ++r)
+        out[((size_t)a * rows + r) * n + hit] = (float)((uint32_t)i / (uint32_t)region_size_of(n, regions_h[a * rows + r])) + 1.f;
+}
+
 }  // namespace lampa
 
 using namespace lampa;
+
+extern "C" int lampa_geo_keys_fused(float* proj, const float* part, int64_t blocks, const int64_t* rank_eta, const int64_t* rank_phi,
+                                    const float* regions_eta, const float* regions_phi, int32_t rows, int64_t n, int64_t raw_size, void* stream) {
+    if (rows <= 0 || rows > 65535 || n < 0 || n >= ((int64_t)1 << 31) || blocks <= 0 || blocks > INT32_MAX) return LAMPA_ERR_ARG;
+    if (n == 0) return LAMPA_OK;
+    if (!proj || !part || !rank_eta || !rank_phi || !regions_eta || !regions_phi) return LAMPA_ERR_ARG;
+    ProfScope prof("geo_keys", (cudaStream_t)stream);
+    geo_keys_fused_kernel<<<dim3((unsigned)((n + GEO_CHUNK - 1) / GEO_CHUNK), rows), 512, 0, (cudaStream_t)stream>>>(
+        proj, (const float2*)part, (int)blocks, rank_eta, rank_phi, regions_eta, regions_phi, rows, n, raw_size);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
+
+extern "C" int lampa_region_inputs(const float* coords, int64_t raw, int64_t n, int32_t cols, const float* regions, int32_t nc,
+                                   int32_t nh, float* padded, float* regions_h, float* region_indices, int64_t* ranks, int64_t* perm,
+                                   float* keys, void* ws, size_t ws_bytes, int32_t* status, void* stream) {
+    if (raw < 0 || n < raw || n >= ((int64_t)1 << 30) || cols < 2 || nc <= 0 || nh <= 0) return LAMPA_ERR_ARG;
+    if (n == 0) return LAMPA_OK;
+    if (!coords || !regions || !padded || !regions_h || !region_indices || !ranks || !perm || !keys || !ws) return LAMPA_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int rows = nc * nh;
+    const int64_t most = n > 2 * rows ? n : 2 * rows;
+    {
+        ProfScope prof("region_prepare", st);
+        region_prepare_kernel<<<(unsigned)((most + GEO_THREADS - 1) / GEO_THREADS), GEO_THREADS, 0, st>>>(coords, raw, n, cols, regions, nc, 2, nh, padded, keys, regions_h);
+        if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
+    }
+    const int rc = lampa_segsort_stable(keys, LAMPA_KEY_F32, 2 * n, nullptr, 2, nullptr, perm, ws, ws_bytes, status, stream);
+    if (rc != LAMPA_OK) return rc;
+    ProfScope prof("region_ranks", st);
+    region_ranks_kernel<<<dim3((unsigned)((n + GEO_THREADS - 1) / GEO_THREADS), 2), GEO_THREADS, 0, st>>>(perm, regions_h, rows, n, ranks, region_indices);
+    return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+}
 
 extern "C" int lampa_row_range(const float* a, const float* b, int32_t rows, int64_t n, float* mn,
                                float* mx, float* range, void* stream) {

@@ -281,6 +281,7 @@ PyObject* step(PyObject* const* a) {
 
 #include "host_lsh.inc"
 #include "host_model.inc"
+#include "host_hept.inc"
 
 template <PyObject* (*F)(PyObject* const*), int N>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -299,7 +300,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     ENTRY(gdn, 13), ENTRY(prefill, 7), ENTRY(step, 10),
     ENTRY(lsh_hash, 8), ENTRY(segsort, 4), ENTRY(permute_rows, 5), ENTRY(invert_perm, 1), ENTRY(bucket_sort, 4), ENTRY(ordering, 3),
-    ENTRY(model_forward, 6),
+    ENTRY(model_forward, 6), ENTRY(region_inputs, 3), ENTRY(hept_core, 11),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of lampa_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -110,6 +110,10 @@ def region_inputs(coords: torch.Tensor, regions: torch.Tensor, block_size: int):
     (padding rows zeroed, as the reference leaves them), raw_size, regions_h [a, c*h],
     region_indices [eta, phi] (fp32 [R, N]) and the two rank vectors they were made from."""
     dev = L.require_cuda(coords)
+    r = L.native.region_inputs(coords.detach().to(torch.float32).contiguous(), regions.detach().to(device=dev, dtype=torch.float32).contiguous(),
+                               int(block_size))
+    if r is not None:
+        return {"coords": r[0], "raw_size": coords.shape[0], "regions_h": r[1], "region_indices": [r[2], r[3]], "ranks": [r[4], r[5]]}
     raw = coords.shape[0]
     padded = pad_to_multiple(coords.to(torch.float32), block_size, dims=0, value=float("inf")).contiguous()
     rank_eta = ranks_of(padded[:, 0])
