@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BA_MAX_WARPS * 32, BA_QROWS == 4 ? 3 : 2) buck
 }
 
 // -------------------------------------------------------------------------------------------------
-// Rows of at most 64 features: the same bucket on the tensor cores, at fp32 accuracy.  A float is
+// Rows of at most 32 features: the same bucket on the tensor cores, at fp32 accuracy.  A float is
 // carried exactly by three bf16 pieces (hi + mid + lo, 8 significant bits each); of the nine products of
 // two such sums the six larger ones are issued (hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi, smallest
 // first), the other three are below 2^-24 of the result, and accumulation is fp32.  The FMA kernel above
@@ -287,30 +287,31 @@ __device__ __forceinline__ Split3 split3(float x, float y) {
     s.l = pack_bf16x2(rx - m.x, ry - m.y);
     return s;
 }
-// c[i] += a b_i for operands in three pieces and NT column tiles (two per fragment); one product of every tile after the
-// other, so that consecutive instructions do not wait for each other's accumulator
-template <int NT>
-__device__ __forceinline__ void mma6(float (*c)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
-                                     const uint32_t (&bh)[(NT + 1) / 2][4], const uint32_t (&bm)[(NT + 1) / 2][4], const uint32_t (&bl)[(NT + 1) / 2][4]) {
+// c[i] += a b_i for operands in three pieces and NT column tiles (two per fragment), one piece of b in registers at a time
+// (low first); `load` fetches the fragments of a piece.  Consecutive instructions go to different accumulators.
+template <int NT, class Load>
+__device__ __forceinline__ void mma6(float (*c)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4], Load load) {
+    uint32_t b[(NT + 1) / 2][4];
+    auto times = [&](const uint32_t (&x)[4]) {
 #pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], al, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bl[i / 2][2 * (i & 1)], bl[i / 2][2 * (i & 1) + 1]);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], am, bm[i / 2][2 * (i & 1)], bm[i / 2][2 * (i & 1) + 1]);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], am, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bm[i / 2][2 * (i & 1)], bm[i / 2][2 * (i & 1) + 1]);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) mma16816(c[i], ah, bh[i / 2][2 * (i & 1)], bh[i / 2][2 * (i & 1) + 1]);
+        for (int i = 0; i < NT; ++i) mma16816(c[i], x, b[i / 2][2 * (i & 1)], b[i / 2][2 * (i & 1) + 1]);
+    };
+    load(2, b);
+    times(ah);
+    load(1, b);
+    times(am);
+    times(ah);
+    load(0, b);
+    times(al);
+    times(am);
+    times(ah);
 }
 __host__ __device__ inline int bam_keys(int bucket) { return (bucket + 15) & ~15; }
 template <int KQ, int NV>
 __host__ __device__ constexpr int bam_smem(int keys) { return 4 * 128 * 8 + keys * 3 * ((16 * KQ + 8) + (8 * ((NV + 1) & ~1) + 8)) * 2; }
 
 template <int KQ, int NV>      // 16-wide feature steps of q / k, 8-wide value column tiles
-__global__ void __launch_bounds__(256, 2) bucket_attn_mma_kernel(BucketAttnArgs a) {
+__global__ void __launch_bounds__(256, 3) bucket_attn_mma_kernel(BucketAttnArgs a) {
     constexpr int KP = 16 * KQ + 8, VP = 8 * ((NV + 1) & ~1) + 8;         // bf16 pitches: consecutive rows fall into different bank groups
     extern __shared__ __align__(16) float ba_smem[];
     const int bucket = a.bucket, keys = bam_keys(bucket), nthr = blockDim.x;     // nthr = 2 * keys
@@ -392,7 +393,10 @@ __global__ void __launch_bounds__(256, 2) bucket_attn_mma_kernel(BucketAttnArgs 
             for (int it = 0; it < 4; ++it) ss[it] += __shfl_xor_sync(0xffffffffu, ss[it], o);
         if (l8 == 0)
 #pragma unroll
-            for (int it = 0; it < 4; ++it) sKn[(tid >> 3) + it * rstep] = -0.5f * ss[it];
+            for (int it = 0; it < 4; ++it) {
+                const int j = (tid >> 3) + it * rstep;
+                sKn[j] = j < bucket ? -0.5f * ss[it] : -INFINITY;
+            }
     }
     // ---- queries: this warp's 16 rows as operand fragments ----
     const int m0 = 16 * warp;
@@ -433,57 +437,41 @@ __global__ void __launch_bounds__(256, 2) bucket_attn_mma_kernel(BucketAttnArgs 
     float o[NV][4], rowsum[2] = {0.f, 0.f};
 #pragma unroll
     for (int nv = 0; nv < NV; ++nv) { o[nv][0] = o[nv][1] = o[nv][2] = o[nv][3] = 0.f; }
-    for (int n0 = 0; n0 < keys; n0 += 64) {
-        float acc[8][4];
+    for (int n0 = 0; n0 < keys; n0 += 32) {                  // 32 keys: four column tiles
+        float acc[4][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+        for (int nt = 0; nt < 4; ++nt) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+        const bool two = n0 + 16 < keys;                     // warp-uniform: the last step may hold 16 keys
 #pragma unroll
-        for (int kk = 0; kk < KQ; ++kk)
+        for (int kk = 0; kk < KQ; ++kk) {
+            const uint32_t at = smem_u32(sK + (n0 + r8 + (mi >> 1) * 8) * KP + 16 * kk + (mi & 1) * 8);
+            auto load1 = [&](int p, uint32_t (&b)[1][4]) { ldsm_x4(b[0], at + p * keys * KP * 2); };
+            auto load2 = [&](int p, uint32_t (&b)[2][4]) { ldsm_x4(b[0], at + p * keys * KP * 2); ldsm_x4(b[1], at + (p * keys + 16) * KP * 2); };
+            if (two) mma6<4>(acc, qh[kk], qm[kk], ql[kk], load2);
+            else mma6<2>(acc, qh[kk], qm[kk], ql[kk], load1);
+        }
 #pragma unroll
-            for (int nq = 0; nq < 2; ++nq) {                 // 32 keys: four column tiles
-                const int kb = n0 + 32 * nq;
-                if (kb >= keys) continue;
-                uint32_t bh[2][4], bm[2][4], bl[2][4];
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {                // past the last 16 keys: the last ones again, results unused
-                    const uint32_t at = smem_u32(sK + (min(kb + 16 * x, keys - 16) + r8 + (mi >> 1) * 8) * KP + 16 * kk + (mi & 1) * 8);
-                    ldsm_x4(bh[x], at);
-                    ldsm_x4(bm[x], at + keys * KP * 2);
-                    ldsm_x4(bl[x], at + 2 * keys * KP * 2);
-                }
-                mma6<4>(&acc[4 * nq], qh[kk], qm[kk], ql[kk], bh, bm, bl);
-            }
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-            if (n0 + 16 * ks < keys) {
+        for (int ks = 0; ks < 2; ++ks)
+            if (ks == 0 || two) {
                 uint32_t ph[4], pm[4], pl[4];
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int col = n0 + 16 * ks + 8 * e + 2 * t;
-                    const float2 kn = *reinterpret_cast<const float2*>(sKn + col);
-                    const bool in0 = col < bucket, in1 = col + 1 < bucket;
+                    const float2 kn = *reinterpret_cast<const float2*>(sKn + col);      // -inf past the bucket: weight 0
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
-                        const float p0 = in0 ? __expf(fminf((acc[2 * ks + e][2 * hh] + qn[hh]) + kn.x, 0.f)) : 0.f;
-                        const float p1 = in1 ? __expf(fminf((acc[2 * ks + e][2 * hh + 1] + qn[hh]) + kn.y, 0.f)) : 0.f;
+                        const float p0 = __expf(fminf((acc[2 * ks + e][2 * hh] + qn[hh]) + kn.x, 0.f));
+                        const float p1 = __expf(fminf((acc[2 * ks + e][2 * hh + 1] + qn[hh]) + kn.y, 0.f));
                         rowsum[hh] += p0 + p1;
                         const Split3 s = split3(p0, p1);
                         ph[2 * e + hh] = s.h; pm[2 * e + hh] = s.m; pl[2 * e + hh] = s.l;
                     }
                 }
+                const uint32_t at = smem_u32(sV + (n0 + 16 * ks + r8 + (mi & 1) * 8) * VP + (mi >> 1) * 8);
+                mma6<NV>(o, ph, pm, pl, [&](int p, uint32_t (&b)[(NV + 1) / 2][4]) {
 #pragma unroll
-                for (int np = 0; np < NV; np += 4) {         // up to four column tiles at a time
-                    constexpr int NT = NV < 4 ? NV : 4;
-                    uint32_t bh[(NT + 1) / 2][4], bm[(NT + 1) / 2][4], bl[(NT + 1) / 2][4];
-#pragma unroll
-                    for (int x = 0; x < (NT + 1) / 2; ++x) {
-                        const uint32_t at = smem_u32(sV + (n0 + 16 * ks + r8 + (mi & 1) * 8) * VP + 8 * np + 16 * x + (mi >> 1) * 8);
-                        ldsm_x4_t(bh[x], at);
-                        ldsm_x4_t(bm[x], at + keys * VP * 2);
-                        ldsm_x4_t(bl[x], at + 2 * keys * VP * 2);
-                    }
-                    mma6<NT>(&o[np], ph, pm, pl, bh, bm, bl);
-                }
+                    for (int x = 0; x < (NV + 1) / 2; ++x) ldsm_x4_t(b[x], at + (p * keys * VP + 16 * x) * 2);
+                });
             }
     }
 #pragma unroll
@@ -692,12 +680,12 @@ extern "C" int lampa_bucket_rbf_attn(const float* q, const float* k, const float
     if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
     const int64_t units = (int64_t)rounds * heads * (n / bucket);
     if (units > 0x7fffffffLL) return LAMPA_ERR_UNSUPPORTED;
-    if (dq <= 64 && dv <= 64) {                            // what one 16-row warp tile holds in registers; wider rows stay on FMA
+    // Rows of up to 32 features are what a warp's tile holds in registers at three CTAs per SM; with wider ones this kernel
+    // measured slower than FMA (dq 54 / dv 48: 1.78 against 1.65 ms), and a bucket of fewer than 33 hits leaves it two warps.
+    if (dq <= 32 && dv <= 32 && bucket > 32) {
         const int keys = bam_keys(bucket);
-        const bool q2 = dq <= 32, v3 = dv <= 24, v4 = dv <= 32;
-        auto mma = q2 ? (v3 ? bucket_attn_mma_kernel<2, 3> : v4 ? bucket_attn_mma_kernel<2, 4> : bucket_attn_mma_kernel<2, 8>)
-                      : (v4 ? bucket_attn_mma_kernel<4, 4> : bucket_attn_mma_kernel<4, 8>);
-        const int msmem = q2 ? (v4 ? bam_smem<2, 4>(keys) : bam_smem<2, 8>(keys)) : (v4 ? bam_smem<4, 4>(keys) : bam_smem<4, 8>(keys));
+        auto mma = dv <= 24 ? bucket_attn_mma_kernel<2, 3> : bucket_attn_mma_kernel<2, 4>;
+        const int msmem = bam_smem<2, 4>(keys);
         if (cudaFuncSetAttribute(mma, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem) != cudaSuccess) return LAMPA_ERR_CUDA;
         ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
         mma<<<(unsigned)units, 2 * keys, msmem, (cudaStream_t)stream>>>(a);
