@@ -563,7 +563,7 @@ inline size_t hf_smem(int heads, int d, int cd, int rounds) {
     return ((size_t)2 * HF_HITS * hf_pitch(heads, d) + HF_HITS * cd + (size_t)heads * cd + (size_t)heads * (d + cd) * rounds) * 4;
 }
 
-template <int R>
+template <int R, bool VEC>      // VEC: d and ldq are multiples of 4, everything 16-byte aligned
 __global__ void __launch_bounds__(256)
 hept_front_kernel(const float* __restrict__ query, const float* __restrict__ key, const float* __restrict__ value,
                   const float* __restrict__ scale, const float* __restrict__ coords, const float* __restrict__ alpha,
@@ -580,28 +580,75 @@ hept_front_kernel(const float* __restrict__ query, const float* __restrict__ key
     const int64_t i0 = (int64_t)blockIdx.x * HF_HITS;
     const int m = (int)max((int64_t)0, min((int64_t)HF_HITS, raw_size - i0));     // rows that hold a hit
     const int rows = (int)min((int64_t)HF_HITS, n - i0);
-    for (int r = warp; r < HF_HITS; r += 8)
-        for (int c = lane; c < hd; c += 32) {
-            sq[r * P + c] = r < m ? __ldg(query + (i0 + r) * hd + c) : 0.f;
-            sk[r * P + c] = r < m ? __ldg(key + (i0 + r) * hd + c) : 0.f;
-            if (r < rows) {                     // values only change their layout
-                const int h = c / d;
-                v_out[((size_t)h * n + i0 + r) * d + c - h * d] = r < m ? __ldg(value + (i0 + r) * hd + c) : 0.f;
+    if (VEC) {                                  // six 16-byte pieces of each input in flight per thread
+        const int hd4 = hd >> 2, d4 = d >> 2, total = HF_HITS * hd4, dr = 256 / hd4, dc = 256 - dr * hd4;
+        int r = tid / hd4, c = tid - r * hd4;
+        for (int e0 = tid; e0 < total; e0 += 6 * 256) {
+            float4 xq[6], xk[6], xv[6];
+            int rr[6], cc[6];
+#pragma unroll
+            for (int x = 0; x < 6; ++x) {
+                rr[x] = r; cc[x] = c;
+                const bool in = e0 + 256 * x < total && r < m;
+                const size_t at = (size_t)(i0 + r) * hd + 4 * c;
+                xq[x] = in ? __ldg(reinterpret_cast<const float4*>(query + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                xk[x] = in ? __ldg(reinterpret_cast<const float4*>(key + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                xv[x] = in ? __ldg(reinterpret_cast<const float4*>(value + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r += dr; c += dc;
+                if (c >= hd4) { c -= hd4; ++r; }
+            }
+#pragma unroll
+            for (int x = 0; x < 6; ++x) {
+                if (e0 + 256 * x >= total) break;
+                float* p = sq + rr[x] * P + 4 * cc[x];
+                p[0] = xq[x].x; p[1] = xq[x].y; p[2] = xq[x].z; p[3] = xq[x].w;
+                p = sk + rr[x] * P + 4 * cc[x];
+                p[0] = xk[x].x; p[1] = xk[x].y; p[2] = xk[x].z; p[3] = xk[x].w;
+                const int h = cc[x] / d4;       // values only change their layout
+                if (rr[x] < rows) *reinterpret_cast<float4*>(v_out + ((size_t)h * n + i0 + rr[x]) * d + 4 * (cc[x] - h * d4)) = xv[x];
             }
         }
+    } else
+        for (int r = warp; r < HF_HITS; r += 8)
+            for (int c = lane; c < hd; c += 32) {
+                sq[r * P + c] = r < m ? __ldg(query + (i0 + r) * hd + c) : 0.f;
+                sk[r * P + c] = r < m ? __ldg(key + (i0 + r) * hd + c) : 0.f;
+                if (r < rows) {
+                    const int h = c / d;
+                    v_out[((size_t)h * n + i0 + r) * d + c - h * d] = r < m ? __ldg(value + (i0 + r) * hd + c) : 0.f;
+                }
+            }
     for (int e = tid; e < HF_HITS * cd; e += 256) sc[e] = e / cd < m ? __ldg(coords + i0 * cd + e) : 0.f;
     for (int e = tid; e < heads * cd; e += 256) ss[e] = __ldg(scale + e);
     for (int e = tid; e < heads * D * R; e += 256) sa[e] = __ldg(alpha + e);
     __syncthreads();
     for (int h = warp; h < heads; h += 8) {
-        for (int r = 0; r < rows; ++r)
-            for (int c = lane; c < ldq; c += 32) {
-                float x = 0.f, y = 0.f;
-                if (c < d) { x = sq[r * P + h * d + c]; y = sk[r * P + h * d + c]; }
-                else if (c < D && r < m) x = y = __fmul_rn(ss[h * cd + c - d], sc[r * cd + c - d]);
-                q_hat[((size_t)h * n + i0 + r) * ldq + c] = x;
-                k_hat[((size_t)h * n + i0 + r) * ldq + c] = y;
+        if (VEC) {
+            const int w4 = ldq >> 2, dr = 32 / w4, dc = 32 - dr * w4;
+            int r = lane / w4, c = lane - r * w4;
+            while (r < rows) {
+                float x[4], y[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int col = 4 * c + e;
+                    if (col < d) { x[e] = sq[r * P + h * d + col]; y[e] = sk[r * P + h * d + col]; }
+                    else x[e] = y[e] = col < D && r < m ? __fmul_rn(ss[h * cd + col - d], sc[r * cd + col - d]) : 0.f;
+                }
+                const size_t at = ((size_t)h * n + i0 + r) * ldq + 4 * c;
+                *reinterpret_cast<float4*>(q_hat + at) = make_float4(x[0], x[1], x[2], x[3]);
+                *reinterpret_cast<float4*>(k_hat + at) = make_float4(y[0], y[1], y[2], y[3]);
+                r += dr; c += dc;
+                if (c >= w4) { c -= w4; ++r; }
             }
+        } else
+            for (int r = 0; r < rows; ++r)
+                for (int c = lane; c < ldq; c += 32) {
+                    float x = 0.f, y = 0.f;
+                    if (c < d) { x = sq[r * P + h * d + c]; y = sk[r * P + h * d + c]; }
+                    else if (c < D && r < m) x = y = __fmul_rn(ss[h * cd + c - d], sc[r * cd + c - d]);
+                    q_hat[((size_t)h * n + i0 + r) * ldq + c] = x;
+                    k_hat[((size_t)h * n + i0 + r) * ldq + c] = y;
+                }
         float aq[R], ak[R];
         const float* al = sa + h * D * R;
         for (int c = 0; c < D; ++c) {
@@ -744,9 +791,14 @@ extern "C" int lampa_hept_front(const float* query, const float* key, const floa
     if (rounds > HF_MAX_ROUNDS || smem > 200 * 1024) return LAMPA_ERR_UNSUPPORTED;
     using K = void (*)(const float*, const float*, const float*, const float*, const float*, const float*, int64_t, int, int, int, int, int64_t,
                        float*, float*, float*, float*, float2*);
-    static const K kernels[HF_MAX_ROUNDS] = {hept_front_kernel<1>, hept_front_kernel<2>, hept_front_kernel<3>, hept_front_kernel<4>,
-                                             hept_front_kernel<5>, hept_front_kernel<6>, hept_front_kernel<7>, hept_front_kernel<8>};
-    const K kernel = kernels[rounds - 1];
+    static const K kernels[2][HF_MAX_ROUNDS] = {
+        {hept_front_kernel<1, false>, hept_front_kernel<2, false>, hept_front_kernel<3, false>, hept_front_kernel<4, false>,
+         hept_front_kernel<5, false>, hept_front_kernel<6, false>, hept_front_kernel<7, false>, hept_front_kernel<8, false>},
+        {hept_front_kernel<1, true>, hept_front_kernel<2, true>, hept_front_kernel<3, true>, hept_front_kernel<4, true>,
+         hept_front_kernel<5, true>, hept_front_kernel<6, true>, hept_front_kernel<7, true>, hept_front_kernel<8, true>}};
+    const bool vec = d % 4 == 0 && ldq % 4 == 0 && heads * d <= 1024 &&
+                     (((uintptr_t)query | (uintptr_t)key | (uintptr_t)value | (uintptr_t)q_hat | (uintptr_t)k_hat | (uintptr_t)v_out) & 15) == 0;
+    const K kernel = kernels[vec][rounds - 1];
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LAMPA_ERR_CUDA;
     ProfScope prof("hept_front", (cudaStream_t)stream);
     kernel<<<(unsigned)((n + HF_HITS - 1) / HF_HITS), 256, smem, (cudaStream_t)stream>>>(query, key, value, scale, coords, alpha, n, heads, d, cd, ldq,

@@ -167,17 +167,19 @@ region_prepare_kernel(const float* __restrict__ coords, int64_t raw, int64_t n, 
     }
 }
 
-// ranks of both coordinates and their region numbers: rank[perm[i]] = i, out[r][hit] for the `rows` rows of regions_h
+// ranks of both coordinates: rank[perm[i]] = i; and, in hit order, their region numbers for the `rows` rows of regions_h
 __global__ void __launch_bounds__(GEO_THREADS)
-region_ranks_kernel(const int64_t* __restrict__ perm, const float* __restrict__ regions_h, int rows, int64_t n,
-                    int64_t* __restrict__ rank, float* __restrict__ out) {
+region_ranks_kernel(const int64_t* __restrict__ perm, int64_t n, int64_t* __restrict__ rank) {
+    const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x, at = blockIdx.y * n;
+    if (i < n) rank[at + perm[at + i]] = i;
+}
+__global__ void __launch_bounds__(GEO_THREADS)
+region_numbers_kernel(const int64_t* __restrict__ rank, const float* __restrict__ regions_h, int rows, int64_t n, float* __restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
     const int a = blockIdx.y;
     if (i >= n) return;
-    const int64_t hit = perm[a * n + i];
-    rank[a * n + hit] = i;
-    for (int r = 0; r < rows; ++r)
-        out[((size_t)a * rows + r) * n + hit] = (float)((uint32_t)i / (uint32_t)region_size_of(n, regions_h[a * rows + r])) + 1.f;
+    const uint32_t rk = (uint32_t)rank[a * n + i];
+    for (int r = 0; r < rows; ++r) out[((size_t)a * rows + r) * n + i] = (float)(rk / (uint32_t)region_size_of(n, regions_h[a * rows + r])) + 1.f;
 }
 
 }  // namespace lampa
@@ -212,7 +214,9 @@ extern "C" int lampa_region_inputs(const float* coords, int64_t raw, int64_t n, 
     const int rc = lampa_segsort_stable(keys, LAMPA_KEY_F32, 2 * n, nullptr, 2, nullptr, perm, ws, ws_bytes, status, stream);
     if (rc != LAMPA_OK) return rc;
     ProfScope prof("region_ranks", st);
-    region_ranks_kernel<<<dim3((unsigned)((n + GEO_THREADS - 1) / GEO_THREADS), 2), GEO_THREADS, 0, st>>>(perm, regions_h, rows, n, ranks, region_indices);
+    const dim3 grid((unsigned)((n + GEO_THREADS - 1) / GEO_THREADS), 2);
+    region_ranks_kernel<<<grid, GEO_THREADS, 0, st>>>(perm, n, ranks);
+    region_numbers_kernel<<<grid, GEO_THREADS, 0, st>>>(ranks, regions_h, rows, n, region_indices);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
