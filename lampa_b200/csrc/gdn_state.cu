@@ -9,6 +9,8 @@
 #include "gdn.cuh"
 #include "profile.cuh"
 
+#include <type_traits>
+
 namespace lampa {
 
 __device__ __forceinline__ float round_like(float x, int dt) {
@@ -43,6 +45,30 @@ __device__ __forceinline__ void half_warp_sum(float (&x)[N]) {
     for (int o = 1; o < 16; o <<= 1)
 #pragma unroll
         for (int i = 0; i < N; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], o);
+}
+
+// The same for many values: a butterfly that halves the number of values a lane carries at every step (15 shuffles for 16
+// values instead of 64), after which lane i of the half-warp has the sum of value i, and one shuffle hands each sum to all.
+template <int N>
+__device__ __forceinline__ void half_warp_sum_many(float (&x)[N], int lane) {
+#pragma unroll
+    for (int g = 0; g < N; g += 16) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = g + i < N ? x[g + i < N ? g + i : 0] : 0.f;
+#pragma unroll
+        for (int h = 8; h > 0; h >>= 1) {
+            const bool up = lane & h;
+#pragma unroll
+            for (int i = 0; i < h; ++i) {
+                const float give = up ? v[i] : v[i + h];
+                v[i] = (up ? v[i + h] : v[i]) + __shfl_xor_sync(0xffffffffu, give, h);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (g + i < N) x[g + i < N ? g + i : 0] = __shfl_sync(0xffffffffu, v[0], (lane & 16) | i);
+    }
 }
 
 template <int KD, int VD, int HS>
@@ -125,29 +151,42 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     if (nch > 0) {
         const int64_t t0 = tok0 + (int64_t)(nch - 1) * CHUNK;
         stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, a.tok_off[seq + 1] - t0), false);
-        for (int t = 0; t < CHUNK; ++t) {
-            if (t > 0) cascade_low(__ffs(t) - 1);
-            const float eg = sEg[t], bt = sBeta[t];
-            float kr[KI], dot[ELL0 - 1];
+        // After a whole chunk level l >= 1 holds tokens 64 - 2^l .. 63 - 2^(l-1), carried through the rest: one running
+        // state from its first token on, so that before token 32 there is one state to advance and six only at the end.
+        auto advance = [&](auto first, int t0, int t1) {         // levels first .. 6 have started
+            constexpr int F = decltype(first)::value, NLV = ELL0 - F;
+            for (int t = t0; t < t1; ++t) {
+                const float eg = sEg[t], bt = sBeta[t], bv = bt * sV[t * TAIL_COLS + col];
+                float kr[KI], dot[NLV];
 #pragma unroll
-            for (int i = 0; i < KI; ++i) kr[i] = sK[t * KD + kl + 16 * i];
+                for (int i = 0; i < KI; ++i) kr[i] = sK[t * KD + kl + 16 * i];
 #pragma unroll
-            for (int l = 1; l < ELL0; ++l) {
-                dot[l - 1] = 0.f;
+                for (int l = 0; l < NLV; ++l) {
+                    dot[l] = 0.f;
 #pragma unroll
-                for (int i = 0; i < KI; ++i) dot[l - 1] += kr[i] * S[l][i];
+                    for (int i = 0; i < KI; ++i) dot[l] += kr[i] * S[F + l][i];
+                }
+                half_warp_sum(dot);
+                const bool collect = t < CHUNK - (1 << (F - 1)); // the youngest of these levels is still taking tokens in
+#pragma unroll
+                for (int l = 0; l < NLV; ++l) {
+                    const float c = bt * dot[l];
+#pragma unroll
+                    for (int i = 0; i < KI; ++i) {
+                        S[F + l][i] = eg * (S[F + l][i] - kr[i] * c);
+                        if (l == 0 && collect) S[F][i] += kr[i] * bv;
+                    }
+                }
             }
-            half_warp_sum(dot);
+        };
+        advance(std::integral_constant<int, 6>{}, 0, 32);
+        advance(std::integral_constant<int, 5>{}, 32, 48);
+        advance(std::integral_constant<int, 4>{}, 48, 56);
+        advance(std::integral_constant<int, 3>{}, 56, 60);
+        advance(std::integral_constant<int, 2>{}, 60, 62);
+        advance(std::integral_constant<int, 1>{}, 62, 64);
 #pragma unroll
-            for (int l = 1; l < ELL0; ++l) {
-                const float c = bt * dot[l - 1];
-#pragma unroll
-                for (int i = 0; i < KI; ++i) S[l][i] = eg * (S[l][i] - kr[i] * c);
-            }
-            const float bv = bt * sV[t * TAIL_COLS + col];
-#pragma unroll
-            for (int i = 0; i < KI; ++i) S[0][i] = kr[i] * bv;
-        }
+        for (int i = 0; i < KI; ++i) S[0][i] = sK[63 * KD + kl + 16 * i] * (sBeta[63] * sV[63 * TAIL_COLS + col]);
     }
 
     float* st = ta.states + ((((size_t)seq * H + h) * KD + kl) * VD + vv) * L;     // row kl; row kl + 16 i is i * row16 further
@@ -195,7 +234,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 #pragma unroll
                     for (int i = 0; i < KI; ++i) dot[l] += kr[i] * (l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i]);
                 }
-                half_warp_sum(dot);
+                half_warp_sum_many(dot, lane);
                 const float* lam = sLam + t * L;
 #pragma unroll
                 for (int l = 1; l < ELL0; ++l) {

@@ -466,6 +466,23 @@ __device__ __forceinline__ uint32_t order_bits(float x) {          // key_xform 
 }
 // Operation order of a projection as in lsh_hash_kernel; the hashes are added in four interleaved partial sums,
 // which is the order torch.sum adds them in (fewer than four: simply left to right).
+// DIM, NH > 0: known to the compiler (the coordinates then stay in registers).
+template <int DIM, int NH>
+__device__ __forceinline__ void ordering_key_norm_fixed(const float* __restrict__ c, const float* alpha, float& key, float& norm) {
+    float x[DIM], ss = 0.f;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) { x[d] = __ldg(c + d); ss = fmaf(x[d], x[d], ss); }
+    norm = sqrtf(ss);
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < NH; ++j) {
+        float acc = __fmul_rn(x[0], alpha[j]);
+#pragma unroll
+        for (int d = 1; d < DIM; ++d) acc = __fadd_rn(acc, __fmul_rn(x[d], alpha[d * NH + j]));
+        part[j & 3] = __fadd_rn(part[j & 3], __fmul_rn(acc, (float)(1 << j)));
+    }
+    key = __fadd_rn(__fadd_rn(__fadd_rn(part[0], part[1]), part[2]), part[3]);
+}
 __device__ __forceinline__ float ordering_key(const float* __restrict__ c, int dim, const float* alpha, int nh) {
     float part[4] = {0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < nh; ++j) {
@@ -481,6 +498,7 @@ __device__ __forceinline__ float ordering_norm(const float* __restrict__ c, int 
     return sqrtf(ss);
 }
 
+template <int DIM, int NH>
 __global__ void __launch_bounds__(ORDER_THREADS)
 ordering_rank_kernel(const float* __restrict__ coords, const float* __restrict__ alpha, int dim, int nh,
                      const uint32_t* __restrict__ points, int row_words, int n, int64_t* __restrict__ idx,
@@ -495,16 +513,22 @@ ordering_rank_kernel(const float* __restrict__ coords, const float* __restrict__
     __syncthreads();
     for (int i = tid; i < n; i += ORDER_THREADS) {
         const float* c = coords + (s0 + i) * dim;
-        comp[i] = ((uint64_t)order_bits(ordering_key(c, dim, s_alpha, nh)) << 32) | order_bits(ordering_norm(c, dim));
+        float key, norm;
+        if (DIM > 0) ordering_key_norm_fixed<(DIM > 0 ? DIM : 1), NH>(c, s_alpha, key, norm);
+        else { key = ordering_key(c, dim, s_alpha, nh); norm = ordering_norm(c, dim); }
+        comp[i] = ((uint64_t)order_bits(key) << 32) | order_bits(norm);
     }
     __syncthreads();
     const int p = blockIdx.x * ORDER_POINTS + (tid >> 3), part = tid & 7;
     const uint64_t mine = p < n ? comp[p] : 0;
+    // before p an equal point counts, behind it only a smaller one does: two plain loops
     int cnt = 0;
-    for (int j = part; j < n; j += 8) {
-        const uint64_t c = comp[j];
-        cnt += (c < mine || (c == mine && j < p)) ? 1 : 0;
-    }
+    const int before = min(p, n);
+    int j = part;
+#pragma unroll 8
+    for (; j < before; j += 8) cnt += comp[j] <= mine ? 1 : 0;
+#pragma unroll 8
+    for (; j < n; j += 8) cnt += comp[j] < mine ? 1 : 0;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (part == 0) {
@@ -610,10 +634,11 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
     const int params = dim * num_hashes * 4;
     if (ordering_counts(B, n) && row_bytes <= (1 << 20)) {
         const int smem = (int)n * 8 + params;
-        if (smem > 47 * 1024 && cudaFuncSetAttribute(ordering_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        auto kernel = dim == 6 && num_hashes == 3 ? ordering_rank_kernel<6, 3> : ordering_rank_kernel<0, 0>;    // the layer's default, and any other
+        if (smem > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return LAMPA_ERR_CUDA;
         ProfScope prof("lsh_ordering", st);
-        ordering_rank_kernel<<<dim3((unsigned)((n + ORDER_POINTS - 1) / ORDER_POINTS), (unsigned)B), ORDER_THREADS, smem, st>>>(
+        kernel<<<dim3((unsigned)((n + ORDER_POINTS - 1) / ORDER_POINTS), (unsigned)B), ORDER_THREADS, smem, st>>>(
             coords, alpha, dim, num_hashes, (const uint32_t*)points, (int)(row_bytes / 4), (int)n, idx, (uint32_t*)ordered);
         return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
     }

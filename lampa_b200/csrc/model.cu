@@ -79,26 +79,38 @@ __global__ void __launch_bounds__(256) model_encode_kernel(const float* __restri
                                                            const float* __restrict__ nw, float eps, int64_t n,
                                                            float* __restrict__ x, __nv_bfloat16* __restrict__ hs) {
     __shared__ __align__(16) float rows[8][8 * ENC_IN];
+    __shared__ float sw[MD * (ENC_IN + 1)];                  // W through shared memory: a lane's four rows are 96 scattered words
+    for (int i = threadIdx.x; i < MD * ENC_IN; i += 256) sw[i / ENC_IN * (ENC_IN + 1) + i % ENC_IN] = __ldg(W + i);
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float w[4][ENC_IN], b[4], g[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
 #pragma unroll
-        for (int i = 0; i < ENC_IN; ++i) w[c][i] = __ldg(W + (4 * lane + c) * ENC_IN + i);
+        for (int i = 0; i < ENC_IN; ++i) w[c][i] = sw[(4 * lane + c) * (ENC_IN + 1) + i];
         b[c] = bias ? __ldg(bias + 4 * lane + c) : 0.f;
         g[c] = __ldg(nw + 4 * lane + c);
     }
     float sc[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) sc[i] = __ldg(scale + (lane + 32 * i) % ENC_IN);
-    for (int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 8; r0 < n; r0 += (int64_t)gridDim.x * 64) {
-        __syncwarp();
+    const int64_t step = (int64_t)gridDim.x * 64;
+    int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 8;
+    float ahead[6];                                          // the warp's next eight rows
+    auto fetch = [&](int64_t r) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
             const int e = lane + 32 * i;
-            if (r0 + e / ENC_IN < n) rows[warp][e] = __ldg(hits + r0 * ENC_IN + e) * sc[i];
+            ahead[i] = r + e / ENC_IN < n ? __ldg(hits + r * ENC_IN + e) : 0.f;
         }
+    };
+    fetch(r0);
+    for (; r0 < n; r0 += step) {
         __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 6; ++i) rows[warp][lane + 32 * i] = ahead[i] * sc[i];
+        __syncwarp();
+        fetch(r0 + step);
 #pragma unroll 1
         for (int q = 0; q < 8 && r0 + q < n; q += 4) {           // four rows at a time: their reductions overlap
             float y[4][4], ss[4];
