@@ -19,6 +19,28 @@ __device__ __forceinline__ float round_like(float x, int dt) {
     return x;
 }
 
+// Eight consecutive elements as floats (zeros where `live` is false): 16-byte loads where the base allows them
+__device__ __forceinline__ void load8_as_float(const void* p, size_t i, int dt, bool live, float (&x)[8]) {
+    if (!live) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = 0.f;
+    } else if (((uintptr_t)p & 15) != 0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = load_as_float(p, i + e, dt);
+    } else if (dt == LAMPA_F32) {
+        const float4 u = __ldg(reinterpret_cast<const float4*>((const float*)p + i)), v = __ldg(reinterpret_cast<const float4*>((const float*)p + i) + 1);
+        x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+    } else {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>((const uint16_t*)p + i));
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = dt == LAMPA_BF16 ? unpack_bf16x2(w[e]) : __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+            x[2 * e] = f.x; x[2 * e + 1] = f.y;
+        }
+    }
+}
+
 // -------------------------------------------------------------------------------------------------
 // End of a sequence, token by token in fp32: the token levels 0..6 after its last whole chunk (the
 // recurrence over that chunk from an empty state, as the reference's postprocess_prefill_hstate_
@@ -81,6 +103,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     float* sEg = sV + CHUNK * TAIL_COLS;         // [64]
     float* sBeta = sEg + CHUNK;                  // [64]
     float* sLam = sBeta + CHUNK;                 // [64][L] (tail only)
+    float* sOut = sLam + CHUNK * a.L;            // [63][8][17] terms of the outputs (tail only)
     const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col = 2 * warp + (lane >> 4), kl = lane & 15;
@@ -88,34 +111,34 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const int nch = ta.n0 >= 0 ? ta.n0 : a.chunk_off[seq + 1] - a.chunk_off[seq];
     const int64_t tok0 = ta.n0 >= 0 ? (int64_t)seq * a.fixed_stride : a.tok_off[seq];
 
-    // rows [t0, t0 + len) of the inputs as the kernel uses them; rows up to 64 become null tokens
+    // rows [t0, t0 + len) of the inputs as the kernel uses them; rows up to 64 become null tokens.  Eight elements per
+    // thread and step, K / 8 threads per row, every load in flight before the first is used.
     auto stage = [&](int64_t t0, int len, bool tail) {
-#pragma unroll 4
-        for (int r = warp; r < CHUNK; r += TAIL_THREADS / 32) {
-            float kx[(KD + 31) / 32], qx[(KD + 31) / 32];
+        constexpr int PPR = KD / 8, NIT = CHUNK * PPR / TAIL_THREADS;
+        float x[NIT][8], y[NIT][8];
+#pragma unroll
+        for (int it = 0; it < NIT; ++it) {
+            const int p = tid + it * TAIL_THREADS, r = p / PPR, c = (p % PPR) * 8;
+            const size_t at = ((size_t)(t0 + r) * H + h) * KD + c;
+            load8_as_float(a.k, at, a.qkv_dt, r < len, x[it]);
+            load8_as_float(a.q, at, a.qkv_dt, r < len && tail, y[it]);
+        }
+#pragma unroll
+        for (int it = 0; it < NIT; ++it) {
+            const int p = tid + it * TAIL_THREADS, r = p / PPR, c = (p % PPR) * 8;
             float sk = 0.f, sq = 0.f;
 #pragma unroll
-            for (int j = 0; j < (KD + 31) / 32; ++j) {
-                const int c = lane + 32 * j;
-                const bool in = r < len && c < KD;
-                kx[j] = in ? load_as_float(a.k, ((size_t)(t0 + r) * H + h) * KD + c, a.qkv_dt) : 0.f;
-                qx[j] = in && tail ? load_as_float(a.q, ((size_t)(t0 + r) * H + h) * KD + c, a.qkv_dt) : 0.f;
-                sk += kx[j] * kx[j];
-                sq += qx[j] * qx[j];
-            }
+            for (int e = 0; e < 8; ++e) { sk += x[it][e] * x[it][e]; sq += y[it][e] * y[it][e]; }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
+            for (int o = 1; o < PPR; o <<= 1) {
                 sk += __shfl_xor_sync(0xffffffffu, sk, o);
                 sq += __shfl_xor_sync(0xffffffffu, sq, o);
             }
             const float rk = rsqrtf(sk + 1e-6f), rq = rsqrtf(sq + 1e-6f);
 #pragma unroll
-            for (int j = 0; j < (KD + 31) / 32; ++j) {
-                const int c = lane + 32 * j;
-                if (c < KD) {
-                    sK[r * KD + c] = a.use_l2norm ? round_like(kx[j] * rk, a.qkv_dt) : kx[j];
-                    if (tail) sQ[r * KD + c] = a.use_l2norm ? qx[j] * rq : qx[j];
-                }
+            for (int e = 0; e < 8; ++e) {
+                sK[r * KD + c + e] = a.use_l2norm ? round_like(x[it][e] * rk, a.qkv_dt) : x[it][e];
+                if (tail) sQ[r * KD + c + e] = a.use_l2norm ? y[it][e] * rq : y[it][e];
             }
         }
         for (int i = tid; i < CHUNK * TAIL_COLS; i += TAIL_THREADS) {
@@ -218,6 +241,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             __syncthreads();                               // the last chunk's rows have been read
             const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
             stage(t0, ta.tail, true);
+            // A token's output is a sum over the half-warp too, but nothing in the recurrence waits for it: the lanes leave
+            // their terms in shared memory and all tokens are summed behind the loop.  The next token's rows are fetched
+            // while this one's sums are under way.
+            float kn[KI], qn[KI];
+#pragma unroll
+            for (int i = 0; i < KI; ++i) { kn[i] = sK[kl + 16 * i]; qn[i] = sQ[kl + 16 * i]; }
             for (int t = 0; t < ta.tail; ++t) {
                 if (t > 0) {
                     const int tz = __ffs(t) - 1;
@@ -225,39 +254,54 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                     cascade_low(tz);
                 }
                 const float eg = sEg[t], bt = sBeta[t];
-                float kr[KI], dot[ELL0 - 1 + HS], acc[KI];
+                float kr[KI], qr[KI], dot[ELL0 - 1 + HS], acc[KI];
+                const int tn = min(t + 1, CHUNK - 1);
 #pragma unroll
-                for (int i = 0; i < KI; ++i) { kr[i] = sK[t * KD + kl + 16 * i]; acc[i] = 0.f; }
+                for (int i = 0; i < KI; ++i) {
+                    kr[i] = kn[i]; qr[i] = qn[i]; acc[i] = 0.f;
+                    kn[i] = sK[tn * KD + kl + 16 * i]; qn[i] = sQ[tn * KD + kl + 16 * i];
+                }
 #pragma unroll
                 for (int l = 0; l < ELL0 - 1 + HS; ++l) {
                     dot[l] = 0.f;
 #pragma unroll
                     for (int i = 0; i < KI; ++i) dot[l] += kr[i] * (l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i]);
                 }
-                half_warp_sum_many(dot, lane);
                 const float* lam = sLam + t * L;
+                float lw[ELL0 + HS];
+#pragma unroll
+                for (int l = 0; l < ELL0; ++l) lw[l] = l < L ? lam[l] : 0.f;
+#pragma unroll
+                for (int s = 0; s < HS; ++s) lw[ELL0 + s] = lvl[s] >= 0 ? lam[lvl[s]] : 0.f;
+                const float bv = bt * sV[t * TAIL_COLS + col];
+                half_warp_sum_many(dot, lane);
 #pragma unroll
                 for (int l = 1; l < ELL0; ++l) {
-                    const float c = bt * dot[l - 1], w = l < L ? lam[l] : 0.f;
+                    const float c = bt * dot[l - 1];
 #pragma unroll
-                    for (int i = 0; i < KI; ++i) { S[l][i] = eg * (S[l][i] - kr[i] * c); acc[i] += w * S[l][i]; }
+                    for (int i = 0; i < KI; ++i) { S[l][i] = eg * (S[l][i] - kr[i] * c); acc[i] += lw[l] * S[l][i]; }
                 }
 #pragma unroll
                 for (int s = 0; s < HS; ++s) {
-                    const float c = bt * dot[ELL0 - 1 + s], w = lvl[s] >= 0 ? lam[lvl[s]] : 0.f;
+                    const float c = bt * dot[ELL0 - 1 + s];
 #pragma unroll
-                    for (int i = 0; i < KI; ++i) { X[s][i] = eg * (X[s][i] - kr[i] * c); acc[i] += w * X[s][i]; }
+                    for (int i = 0; i < KI; ++i) { X[s][i] = eg * (X[s][i] - kr[i] * c); acc[i] += lw[ELL0 + s] * X[s][i]; }
                 }
-                const float bv = bt * sV[t * TAIL_COLS + col];
-                float out[1] = {0.f};
+                float out = 0.f;
 #pragma unroll
                 for (int i = 0; i < KI; ++i) {
                     S[0][i] = kr[i] * bv;
-                    out[0] += sQ[t * KD + kl + 16 * i] * (acc[i] + lam[0] * S[0][i]);
+                    out += qr[i] * (acc[i] + lw[0] * S[0][i]);
                 }
-                half_warp_sum(out);
-                if (kl == 0) store_from_float(a.o, ((size_t)(t0 + t) * H + h) * VD + vv, out[0], a.qkv_dt);
+                sOut[(t * TAIL_COLS + col) * 17 + kl] = out;
                 done = t + 1;
+            }
+            __syncthreads();
+            for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS) {
+                float out = 0.f;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) out += sOut[i * 17 + e];
+                store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, out, a.qkv_dt);
             }
         }
         if (done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
@@ -299,7 +343,11 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
     const int slots = ta.tail > 0 ? __builtin_popcount((unsigned)ta.n0) : 0;
-    const size_t smem = (size_t)(CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L : 0)) * 4;   // at most 47 KB
+    const size_t smem = (size_t)(CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L + CHUNK * TAIL_COLS * 17 : 0)) * 4;   // at most 80 KB
+    constexpr int most = (CHUNK * (2 * KD + TAIL_COLS + 2) + CHUNK * 40 + CHUNK * TAIL_COLS * 17) * 4;
+    static std::atomic<uint64_t> ready[3];
+    if (!allow_smem(ready[0], hgdn_tail_kernel<KD, VD, 4>, most) || !allow_smem(ready[1], hgdn_tail_kernel<KD, VD, 8>, most) ||
+        !allow_smem(ready[2], hgdn_tail_kernel<KD, VD, 24>, most)) return LAMPA_ERR_CUDA;
     const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
     ProfScope prof("hgdn_tail", st);
     if (slots <= 4) hgdn_tail_kernel<KD, VD, 4><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
