@@ -135,12 +135,20 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 sq += __shfl_xor_sync(0xffffffffu, sq, o);
             }
             const float rk = rsqrtf(sk + 1e-6f), rq = rsqrtf(sq + 1e-6f);
+            if (a.use_l2norm) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                sK[r * KD + c + e] = a.use_l2norm ? round_like(x[it][e] * rk, a.qkv_dt) : x[it][e];
-                if (tail) sQ[r * KD + c + e] = a.use_l2norm ? y[it][e] * rq : y[it][e];
+                for (int e = 0; e < 8; ++e) { x[it][e] = round_like(x[it][e] * rk, a.qkv_dt); y[it][e] *= rq; }
+            }
+            float4* d = reinterpret_cast<float4*>(sK + r * KD + c);
+            d[0] = make_float4(x[it][0], x[it][1], x[it][2], x[it][3]);
+            d[1] = make_float4(x[it][4], x[it][5], x[it][6], x[it][7]);
+            if (tail) {
+                d = reinterpret_cast<float4*>(sQ + r * KD + c);
+                d[0] = make_float4(y[it][0], y[it][1], y[it][2], y[it][3]);
+                d[1] = make_float4(y[it][4], y[it][5], y[it][6], y[it][7]);
             }
         }
+#pragma unroll
         for (int i = tid; i < CHUNK * TAIL_COLS; i += TAIL_THREADS) {
             const int r = i / TAIL_COLS, c = i - r * TAIL_COLS;
             sV[i] = r < len ? load_as_float(a.v, ((size_t)(t0 + r) * H + h) * VD + v0 + c, a.qkv_dt) : 0.f;
@@ -149,11 +157,17 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             sEg[tid] = tid < len ? __expf(load_as_float(a.g, (size_t)(t0 + tid) * H + h, a.gb_dt)) : 1.f;
             sBeta[tid] = tid < len ? load_as_float(a.beta, (size_t)(t0 + tid) * H + h, a.gb_dt) : 0.f;
         }
-        if (tail)
-            for (int i = tid; i < len * L; i += TAIL_THREADS) {
-                const int r = i / L, l = i - r * L;
-                sLam[i] = load_as_float(a.lam, ((size_t)(t0 + r) * H + h) * L + l, a.lam_dt);
+        if (tail) {                             // two threads per token, up to twenty levels each
+            const int r = tid >> 1;
+            if (r < len) {
+                float w[20];
+#pragma unroll
+                for (int i = 0; i < 20; ++i) w[i] = (tid & 1) + 2 * i < L ? load_as_float(a.lam, ((size_t)(t0 + r) * H + h) * L + (tid & 1) + 2 * i, a.lam_dt) : 0.f;
+#pragma unroll
+                for (int i = 0; i < 20; ++i)
+                    if ((tid & 1) + 2 * i < L) sLam[r * L + (tid & 1) + 2 * i] = w[i];
             }
+        }
         __syncthreads();
     };
 
@@ -171,6 +185,30 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             }
     };
 
+    float* st = ta.states + ((((size_t)seq * H + h) * KD + kl) * VD + vv) * L;     // row kl; row kl + 16 i is i * row16 further
+    const size_t row16 = (size_t)16 * VD * L;
+    // chunk levels the tail continues from, on their way while the last chunk is run
+    float X[HS][KI];
+    int lvl[HS];
+    {
+        uint32_t rem = (uint32_t)nch;
+#pragma unroll
+        for (int s = 0; s < HS; ++s) {
+            lvl[s] = rem ? ELL0 + __ffs(rem) - 1 : -1;
+            rem &= rem - 1;
+        }
+    }
+    const bool room = nch == 0 || lvl[0] < L;    // the first cascade must not leave the last level
+#pragma unroll
+    for (int s = 0; s < HS; ++s)
+#pragma unroll
+        for (int i = 0; i < KI; ++i) X[s][i] = ta.tail > 0 && room && lvl[s] >= 0 && s > 0 ? st[i * row16 + lvl[s]] : 0.f;
+    if (ta.tail > 0 && room && nch > 0) {
+#pragma unroll
+        for (int i = 0; i < KI; ++i)
+            for (int l = ELL0; l < lvl[0]; ++l) X[0][i] += st[i * row16 + l];
+    }
+
     if (nch > 0) {
         const int64_t t0 = tok0 + (int64_t)(nch - 1) * CHUNK;
         stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, a.tok_off[seq + 1] - t0), false);
@@ -180,26 +218,25 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             constexpr int F = decltype(first)::value, NLV = ELL0 - F;
             for (int t = t0; t < t1; ++t) {
                 const float eg = sEg[t], bt = sBeta[t], bv = bt * sV[t * TAIL_COLS + col];
-                float kr[KI], dot[NLV];
+                float kr[KI], ek[KI], dot[NLV];
 #pragma unroll
-                for (int i = 0; i < KI; ++i) kr[i] = sK[t * KD + kl + 16 * i];
+                for (int i = 0; i < KI; ++i) { kr[i] = sK[t * KD + kl + 16 * i]; ek[i] = -eg * bt * kr[i]; }
+                const bool collect = t < CHUNK - (1 << (F - 1)); // the youngest of these levels is still taking tokens in
 #pragma unroll
                 for (int l = 0; l < NLV; ++l) {
                     dot[l] = 0.f;
 #pragma unroll
-                    for (int i = 0; i < KI; ++i) dot[l] += kr[i] * S[F + l][i];
-                }
-                half_warp_sum(dot);
-                const bool collect = t < CHUNK - (1 << (F - 1)); // the youngest of these levels is still taking tokens in
-#pragma unroll
-                for (int l = 0; l < NLV; ++l) {
-                    const float c = bt * dot[l];
-#pragma unroll
                     for (int i = 0; i < KI; ++i) {
-                        S[F + l][i] = eg * (S[F + l][i] - kr[i] * c);
+                        dot[l] += kr[i] * S[F + l][i];
+                        S[F + l][i] *= eg;                       // everything but the sum's term, before the sum is there
                         if (l == 0 && collect) S[F][i] += kr[i] * bv;
                     }
                 }
+                half_warp_sum(dot);
+#pragma unroll
+                for (int l = 0; l < NLV; ++l)
+#pragma unroll
+                    for (int i = 0; i < KI; ++i) S[F + l][i] = fmaf(ek[i], dot[l], S[F + l][i]);
             }
         };
         advance(std::integral_constant<int, 6>{}, 0, 32);
@@ -212,31 +249,14 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         for (int i = 0; i < KI; ++i) S[0][i] = sK[63 * KD + kl + 16 * i] * (sBeta[63] * sV[63 * TAIL_COLS + col]);
     }
 
-    float* st = ta.states + ((((size_t)seq * H + h) * KD + kl) * VD + vv) * L;     // row kl; row kl + 16 i is i * row16 further
-    const size_t row16 = (size_t)16 * VD * L;
-    float X[HS][KI];
-    int lvl[HS];
     int done = 0;                                // tail tokens taken in
     if (ta.tail > 0) {
-        uint32_t rem = (uint32_t)nch;
-#pragma unroll
-        for (int s = 0; s < HS; ++s) {
-            lvl[s] = rem ? ELL0 + __ffs(rem) - 1 : -1;
-            rem &= rem - 1;
-        }
-        const bool room = nch == 0 || lvl[0] < L;          // the first cascade must not leave the last level
         if (room) {
-#pragma unroll
-            for (int s = 0; s < HS; ++s)
-#pragma unroll
-                for (int i = 0; i < KI; ++i) X[s][i] = lvl[s] >= 0 && s > 0 ? st[i * row16 + lvl[s]] : 0.f;
             if (nch > 0) {
 #pragma unroll
-                for (int i = 0; i < KI; ++i) {
+                for (int i = 0; i < KI; ++i)
 #pragma unroll
                     for (int l = 0; l < ELL0; ++l) { X[0][i] += S[l][i]; S[l][i] = 0.f; }
-                    for (int l = ELL0; l < lvl[0]; ++l) X[0][i] += st[i * row16 + l];
-                }
             }
             __syncthreads();                               // the last chunk's rows have been read
             const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
@@ -254,18 +274,22 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                     cascade_low(tz);
                 }
                 const float eg = sEg[t], bt = sBeta[t];
-                float kr[KI], qr[KI], dot[ELL0 - 1 + HS], acc[KI];
+                float kr[KI], ek[KI], qr[KI], dot[ELL0 - 1 + HS], acc[KI];
                 const int tn = min(t + 1, CHUNK - 1);
 #pragma unroll
                 for (int i = 0; i < KI; ++i) {
-                    kr[i] = kn[i]; qr[i] = qn[i]; acc[i] = 0.f;
+                    kr[i] = kn[i]; qr[i] = qn[i]; acc[i] = 0.f; ek[i] = -eg * bt * kr[i];
                     kn[i] = sK[tn * KD + kl + 16 * i]; qn[i] = sQ[tn * KD + kl + 16 * i];
                 }
 #pragma unroll
                 for (int l = 0; l < ELL0 - 1 + HS; ++l) {
                     dot[l] = 0.f;
 #pragma unroll
-                    for (int i = 0; i < KI; ++i) dot[l] += kr[i] * (l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i]);
+                    for (int i = 0; i < KI; ++i) {
+                        float& x = l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i];
+                        dot[l] += kr[i] * x;
+                        x *= eg;                                 // everything but the sum's term, before the sum is there
+                    }
                 }
                 const float* lam = sLam + t * L;
                 float lw[ELL0 + HS];
@@ -276,17 +300,13 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 const float bv = bt * sV[t * TAIL_COLS + col];
                 half_warp_sum_many(dot, lane);
 #pragma unroll
-                for (int l = 1; l < ELL0; ++l) {
-                    const float c = bt * dot[l - 1];
+                for (int l = 0; l < ELL0 - 1 + HS; ++l)
 #pragma unroll
-                    for (int i = 0; i < KI; ++i) { S[l][i] = eg * (S[l][i] - kr[i] * c); acc[i] += lw[l] * S[l][i]; }
-                }
-#pragma unroll
-                for (int s = 0; s < HS; ++s) {
-                    const float c = bt * dot[ELL0 - 1 + s];
-#pragma unroll
-                    for (int i = 0; i < KI; ++i) { X[s][i] = eg * (X[s][i] - kr[i] * c); acc[i] += lw[ELL0 + s] * X[s][i]; }
-                }
+                    for (int i = 0; i < KI; ++i) {
+                        float& x = l < ELL0 - 1 ? S[l < ELL0 - 1 ? l + 1 : 0][i] : X[l < ELL0 - 1 ? 0 : l - ELL0 + 1][i];
+                        x = fmaf(ek[i], dot[l], x);
+                        acc[i] = fmaf(lw[l + 1], x, acc[i]);
+                    }
                 float out = 0.f;
 #pragma unroll
                 for (int i = 0; i < KI; ++i) {
@@ -307,23 +327,42 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         if (done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
     }
 
+    if (done > 0 && ((uintptr_t)ta.states & 15) == 0) {      // every level: the slab goes out as bulk copies of 8 columns x L
+        __syncthreads();
+        float* slab = tail_smem;                             // [KD][8][L] over everything staged
 #pragma unroll
-    for (int i = 0; i < KI; ++i) {
-#pragma unroll
-        for (int l = 0; l < ELL0; ++l)
-            if (l < L && (done > 0 || ta.tail == 0)) st[i * row16 + l] = S[l][i];
-        if (done > 0)
-            for (int l = ELL0; l < L; ++l) {
-                float x = 0.f;
-#pragma unroll
-                for (int s = 0; s < HS; ++s)
-                    if (lvl[s] == l) x = X[s][i];
-                st[i * row16 + l] = x;
-            }
-        else if (ta.tail > 0)                              // the tail was refused: the state after the whole chunks
+        for (int i = 0; i < KI; ++i) {
+            float* d = slab + ((kl + 16 * i) * TAIL_COLS + col) * L;
 #pragma unroll
             for (int l = 0; l < ELL0; ++l)
-                if (l < L) st[i * row16 + l] = S[l][i];
+                if (l < L) d[l] = S[l][i];
+            for (int l = ELL0; l < L; ++l) d[l] = 0.f;
+#pragma unroll
+            for (int s = 0; s < HS; ++s)
+                if (lvl[s] >= 0) d[lvl[s]] = X[s][i];
+        }
+        fence_async_shared();
+        __syncthreads();
+        if (tid < KD) {
+            bulk_s2g(ta.states + ((((size_t)seq * H + h) * KD + tid) * VD + v0) * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
+            bulk_commit();
+            bulk_wait_read();
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < KI; ++i) {
+#pragma unroll
+            for (int l = 0; l < ELL0; ++l)
+                if (l < L) st[i * row16 + l] = S[l][i];      // with a refused tail: the state after the whole chunks
+            if (done > 0)
+                for (int l = ELL0; l < L; ++l) {
+                    float x = 0.f;
+#pragma unroll
+                    for (int s = 0; s < HS; ++s)
+                        if (lvl[s] == l) x = X[s][i];
+                    st[i * row16 + l] = x;
+                }
+        }
     }
     if (h == 0 && blockIdx.z == 0 && tid == 0 && (ta.n0 < 0 || !ta.one_count || seq == 0)) {
         const int64_t n = (int64_t)nch * CHUNK + done;     // tokens held
@@ -343,8 +382,10 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
     const int slots = ta.tail > 0 ? __builtin_popcount((unsigned)ta.n0) : 0;
-    const size_t smem = (size_t)(CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L + CHUNK * TAIL_COLS * 17 : 0)) * 4;   // at most 80 KB
-    constexpr int most = (CHUNK * (2 * KD + TAIL_COLS + 2) + CHUNK * 40 + CHUNK * TAIL_COLS * 17) * 4;
+    const int staged = CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L + CHUNK * TAIL_COLS * 17 : 0);
+    const int slab = ta.tail > 0 ? KD * TAIL_COLS * a.L : 0;
+    const size_t smem = (size_t)(staged > slab ? staged : slab) * 4;
+    constexpr int most = 82 * 1024;                          // 64 x 64 heads at 40 levels
     static std::atomic<uint64_t> ready[3];
     if (!allow_smem(ready[0], hgdn_tail_kernel<KD, VD, 4>, most) || !allow_smem(ready[1], hgdn_tail_kernel<KD, VD, 8>, most) ||
         !allow_smem(ready[2], hgdn_tail_kernel<KD, VD, 24>, most)) return LAMPA_ERR_CUDA;
