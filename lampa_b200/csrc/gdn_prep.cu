@@ -49,8 +49,8 @@ struct PrepSmem {
     static constexpr int AW = V + CHUNK * VP * 2;                // bf16 [64][CP]   Awb = (I + A0)^-1 diag(beta)
     static constexpr int UH = AW + CHUNK * CP * 2;               // bf16 [64][VP]   diag(e^{Glast-G}) U
     static constexpr int AFTER_UH = UH + CHUNK * VP * 2, AFTER_SA = AW + CHUNK * PA * 4;   // the fp32 tile covers AW and UH
-    static constexpr int G = AFTER_UH > AFTER_SA ? AFTER_UH : AFTER_SA;   // fp32 [64] G, [64] beta, [64] e^G, [64] e^{Glast-G}
-    static constexpr int LAM = G + 4 * CHUNK * 4;                // fp32 [64][L+1]
+    static constexpr int G = AFTER_UH > AFTER_SA ? AFTER_UH : AFTER_SA;   // fp32 [64] G, [64] beta, [64] e^G, [64] e^{Glast-G}, [64] e^{G(end of the 8-block)-G}
+    static constexpr int LAM = G + 5 * CHUNK * 4;                // fp32 [64][L+1]
     static int bytes(int L) { return LAM + CHUNK * (L + 1) * 4; }
 };
 
@@ -62,7 +62,7 @@ struct PrepSmem {
 // (s = scale and lambda = 1 for the plain rule; s = 1 for the hierarchical one).  These equal
 // the definitions in gdn.cuh: every e^{G_last-G_tok} e^{G_tok} pair collapses to e^{G_last}.
 template <int KD, int VD, bool HIER>
-__global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
+__global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs a) {
     using S = PrepSmem<KD, VD>;
     using R = Rec<KD, VD>;
     constexpr int KP = S::KP, VP = S::VP, CP = S::CP;
@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
     float* sBeta = sG + CHUNK;
     float* sEG = sG + 2 * CHUNK;
     float* sEGl = sG + 3 * CHUNK;
+    float* sCF = sG + 4 * CHUNK;
     float* sLam = reinterpret_cast<float*>(smem + S::LAM);
 
     // head is the fastest grid index: the H CTAs of one chunk run together and between them read
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
         const float Gi = sG[tid], Gl = sG[CHUNK - 1];
         sEG[tid] = __expf(Gi);
         sEGl[tid] = __expf(Gl - Gi);
+        sCF[tid] = __expf(sG[tid | 7] - Gi);
     }
     char* rec = a.rec + ((size_t)c * H + h) * a.rec_bytes;
     if (HIER) {   // lambda of the chunk levels, transposed to [level][token] for the scan
@@ -300,27 +302,35 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
         {
             // level(i, j) = bit_length(i ^ j).  Off the diagonal 8x8 tile it depends on the tile only
             // (3 + bit_length(i/8 ^ j/8)): one lambda per (row, tile) serves both of the thread's columns.
+            // The decay splits the same way: e^{G_i - G_end(tile)} per (row, tile) times the column's decay to the end of
+            // its tile, both at most 1 - one exponential per row and tile instead of two per pair of elements.
             const float gi2[2] = {sG[m0 + gq], sG[m0 + gq + 8]};
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
-                const float2 gj = *reinterpret_cast<const float2*>(sG + nt * 8 + 2 * tq);
+                const float2 cf = *reinterpret_cast<const float2*>(sCF + nt * 8 + 2 * tq);
+                const float gend = sG[nt * 8 + 7];
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
                     const int it = (m0 >> 3) + hh;                     // the row's 8x8 tile index (warp-uniform)
                     float p0 = 0.f, p1 = 0.f;
                     if (nt <= it) {
-                        if (i >= j) p0 = racc[nt][2 * hh] * __expf(gi2[hh] - gj.x);
-                        if (i >= j + 1) p1 = racc[nt][2 * hh + 1] * __expf(gi2[hh] - gj.y);
-                        if (HIER) {
-                            if (nt < it) {
-                                const float lt = sLam[i * LP + 3 + (32 - __clz(it ^ nt))];
-                                p0 *= lt; p1 *= lt;
-                            } else {
+                        if (nt < it) {
+                            p0 = __expf(gi2[hh] - gend);
+                            if (HIER) p0 *= sLam[i * LP + 3 + (32 - __clz(it ^ nt))];
+                            p1 = p0 * cf.y;
+                            p0 *= cf.x;
+                        } else {
+                            const float2 gj = *reinterpret_cast<const float2*>(sG + nt * 8 + 2 * tq);
+                            if (i >= j) p0 = __expf(gi2[hh] - gj.x);
+                            if (i >= j + 1) p1 = __expf(gi2[hh] - gj.y);
+                            if (HIER) {
                                 p0 *= sLam[i * LP + (32 - __clz(i ^ j))];
                                 p1 *= sLam[i * LP + (32 - __clz(i ^ (j + 1)))];
                             }
                         }
+                        p0 *= racc[nt][2 * hh];
+                        p1 *= racc[nt][2 * hh + 1];
                     }
                     racc[nt][2 * hh] = p0;
                     racc[nt][2 * hh + 1] = p1;
@@ -346,30 +356,22 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
                         pack_bf16x2(osc * acc[nt][2 * hh], osc * acc[nt][2 * hh + 1]);
                 }
         }
-        // U^ = diag(e^{Glast-G}) (Awb .* E) V: the decay is applied to the A fragments in registers
+        // U^ = diag(e^{Glast-G}) (Awb .* E) V = (Awb diag(e^{Glast-G})) V: a column factor on the A fragments in registers
         {
             float acc[VD / 8][4];
             zero_acc<VD / 8>(acc);
-            const float g_lo = sG[m0 + gq], g_hi = sG[m0 + gq + 8];
-            const float fu[2] = {sEGl[m0 + gq], sEGl[m0 + gq + 8]};   // read before the stores to U^ below
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 if (kk * 16 < m0 + 16) {
                     uint32_t af[4];
                     load_a(af, sAw, CP, m0, kk * 16, lane);
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const int i = m0 + gq + (x & 1) * 8, j = kk * 16 + (x >> 1) * 8 + 2 * tq;
-                        const int it = (m0 >> 3) + (x & 1), jt = 2 * kk + (x >> 1);   // 8x8 tile of the row / of the columns
-                        if (jt > it) {
-                            af[x] = 0u;                                           // above the diagonal
-                        } else {
-                            const float gi = (x & 1) ? g_hi : g_lo;
-                            const float2 gj = *reinterpret_cast<const float2*>(sG + j);
-                            const float2 w = unpack_bf16x2(af[x]);
-                            const float u0 = (i >= j) ? w.x * __expf(gi - gj.x) : 0.f;
-                            const float u1 = (i >= j + 1) ? w.y * __expf(gi - gj.y) : 0.f;
-                            af[x] = pack_bf16x2(u0, u1);
+                    for (int x = 0; x < 2; ++x) {
+                        const float2 f = *reinterpret_cast<const float2*>(sEGl + kk * 16 + x * 8 + 2 * tq);
+#pragma unroll
+                        for (int y = 0; y < 2; ++y) {
+                            const float2 w = unpack_bf16x2(af[2 * x + y]);
+                            af[2 * x + y] = pack_bf16x2(w.x * f.x, w.y * f.y);
                         }
                     }
 #pragma unroll
@@ -386,8 +388,7 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_kernel(GdnArgs a) {
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    const float f = fu[hh];
-                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(f * acc[nt][2 * hh], f * acc[nt][2 * hh + 1]);
+                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(acc[nt][2 * hh], acc[nt][2 * hh + 1]);
                 }
         }
         // W = Awb K, written over this warp's own rows of Q (no longer needed)
