@@ -55,7 +55,8 @@ int make_layout(const lampa_gdn_desc* d, bool hier, Layout& l) {
     l.nb_max = (int)(nbm > 0 ? nbm : 1);
     // longest possible sequence bounds the number of cross-block levels
     const int64_t longest = d->nseq > 0 ? (ttot + CHUNK - 1) / CHUNK : (d->T + CHUNK - 1) / CHUNK;
-    const int nlev = longest > 1 ? ceil_log2_int((int)longest) : 0;
+    // (a packed call's longest sequence is only known on the device: at most all tokens, and no longer than L has levels for)
+    const int nlev = std::min(longest > 1 ? ceil_log2_int((int)longest) : 0, hier && d->nseq > 0 ? std::max(d->L - ELL0, 0) : 31);
     // cross-block levels of any sequence up to that length: nlev - 3 up to 256 chunks, 5 up to 1024, then nlev - 5
     const int nhigh = nlev <= MIN_BLOCK_LOG ? 0 : (nlev <= 8 ? nlev - MIN_BLOCK_LOG : (nlev <= 10 ? 5 : nlev - BLOCK_LOG));
     l.nhigh_max = hier ? nhigh : 0;

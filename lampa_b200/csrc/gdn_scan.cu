@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
     const int g = lane >> 2, t = lane & 3;
     const int row0 = warp * 16;
     const int n = nch - 1, bl = block_log(nch);
-    const bool live = nch > 0 && lev < 30 && ((n >> lev) & 1);
+    const bool live = nch > 0 && lev < 30 && ((n >> lev) & 1) && lev - bl < a.nhigh_max;
 
     float C[KD / 8][4];
     zero_state<KD>(C);
@@ -488,10 +488,16 @@ __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
 //     O_n += diag(lambda[:, 7 + l]) (Q~ S_l)
 // and then advances: cleared at the end of its period of 2^(l+1) chunks, otherwise
 //     S_l <- M S_l + [bit l of n == 0] B.
-// Partial outputs of groups >= 1 are added by group 0 through shared memory.
+// Partial outputs of groups >= 1 are added by group 0 through shared memory, in blocks that read any.
+//
+// Bound by the chain of one chunk's products and their shared-memory loads, so warps in flight decide:
+// at head dims up to 32 the registers are held to 168 for 12 warps per SM, whatever the split into groups
+// (3 spilled words).  16 warps (128 registers, two stages) spill and are slower, 1440 us.  One model block over
+// 64 events of 6,000 to 59,000 points: 2003 us with the registers unbounded and a group for every level of
+// the whole batch's length -> 968 us with this bound, the level count of L, and no sum over absent groups.
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD, int NG>
-__global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a) {
+__global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hier_kernel(GdnArgs a) {
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     constexpr int NS = VD / 16;
@@ -503,7 +509,7 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
     const int bl = block_log(nch), bc = 1 << bl;
-    const int nhigh = max(0, nlev - bl);
+    const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
     const int c0 = a.chunk_off[seq] + b * bc;
     const int nsteps = min(bc, nch - b * bc);
     const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
@@ -527,6 +533,13 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
     pipe.budget = a.poll_budget;
     float* red = reinterpret_cast<float*>(smem + 1024 + (size_t)NST * stage_bytes);   // [NG-1][NS][32 regs][32 lanes]
     pipe.start();
+
+    // groups of cross-block levels this block reads at all: the others have nothing to add to the sum over groups
+    uint32_t groups = 0;
+#pragma unroll
+    for (int gi = 1; gi < NG; ++gi)
+        if ((b & ((1 << min(nhigh, 30)) - 1)) >> ((gi - 1) * NLW) & ((1 << NLW) - 1)) groups |= 1u << gi;
+    const bool alone = groups == 0;                    // group 0 only: no second barrier per chunk
 
     float C[NLW][KD / 8][4];
     uint32_t live = 0;   // bit x: level x of this warp holds a state that matters
@@ -609,8 +622,8 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
             }
         }
 
-        if (NG > 1) {
-            if (grp > 0) {
+        if (NG > 1 && !alone) {
+            if ((groups >> grp) & 1) {
                 float* rd = red + ((size_t)(grp - 1) * NS + slab) * 1024 + lane;
 #pragma unroll
                 for (int mt = 0; mt < 4; ++mt)
@@ -624,6 +637,7 @@ __global__ void __launch_bounds__(NG * VD * 2, 1) gdn_out_hier_kernel(GdnArgs a)
         if (grp == 0) {
 #pragma unroll
             for (int gi = 1; gi < NG; ++gi) {
+                if (!((groups >> gi) & 1)) continue;
                 const float* rd = red + ((size_t)(gi - 1) * NS + slab) * 1024 + lane;
 #pragma unroll
                 for (int mt = 0; mt < 4; ++mt)

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
     const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
     const int bl = block_log(nch), bc = 1 << bl;
-    const int nhigh = max(0, nlev - bl);
+    const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
     const int c0 = a.chunk_off[seq] + b * bc;
     const int nsteps = min(bc, nch - b * bc);
     const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
