@@ -61,6 +61,17 @@ struct PrepSmem {
 //   O_local = s ((R .* E .* lambda[i][level(i,j)]) V)
 // (s = scale and lambda = 1 for the plain rule; s = 1 for the hierarchical one).  These equal
 // the definitions in gdn.cuh: every e^{G_last-G_tok} e^{G_tok} pair collapses to e^{G_last}.
+// eight accumulator tiles (16 x 64) as the A fragments of the next product
+__device__ __forceinline__ void pack_a(uint32_t (&f)[4][4], const float (&c)[8][4]) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        f[kk][0] = pack_bf16x2(c[2 * kk][0], c[2 * kk][1]);
+        f[kk][1] = pack_bf16x2(c[2 * kk][2], c[2 * kk][3]);
+        f[kk][2] = pack_bf16x2(c[2 * kk + 1][0], c[2 * kk + 1][1]);
+        f[kk][3] = pack_bf16x2(c[2 * kk + 1][2], c[2 * kk + 1][3]);
+    }
+}
+
 template <int KD, int VD, bool HIER>
 __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs a) {
     using S = PrepSmem<KD, VD>;
@@ -97,7 +108,10 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
     // Every global load of the chunk is issued before any of them is consumed (one DRAM round trip
     // instead of four), and the rows of a chunk some 600 CTAs ahead are pulled into L2.
     {
-        const int r = tid >> 1, half = tid & 1;
+        // two threads per row; at the 80-byte pitch of a 32-wide row the order 0, 1, 4, 5, 2, 3, 6, 7 puts the eight
+        // 16-byte stores of a phase in different banks
+        const int rl = tid >> 1, half = tid & 1;
+        const int r = KD == 64 ? rl : (rl & ~6) | ((rl & 2) << 1) | ((rl & 4) >> 1);
         const bool valid = r < len;
         const size_t tok = (size_t)(t0 + r);
         const bool two_byte = a.qkv_dt != LAMPA_F32;
@@ -201,6 +215,7 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
     }
 
     const int m0 = warp * 16;
+    uint32_t ra[4][4];                                       // tril(Q K^T), later R, as A fragments
     // ---- stage 1: Awb = (I + A0)^-1 diag(beta), A0 = tril(diag(beta) K K^T, -1) ---------------------
     // Blockwise, as the reference's solve_tril does (models/hattention/solve_tril.py:221-276): warp w
     // forms rows 16w.. of A0 on the tensor cores and inverts its own 16x16 diagonal block by fp32
@@ -213,92 +228,93 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
         constexpr int PA = S::PA;
         float* sA = reinterpret_cast<float*>(smem + S::AW);
         {
-            float acc[8][4];
+            float acc[8][4], racc[8][4];
             zero_acc<8>(acc);
-            warp_gemm<8, KD, false, false>(acc, sK, KP, m0, sK, KP, 0, lane, KD, m0 + 16);
+            zero_acc<8>(racc);
+#pragma unroll
+            for (int k0 = 0; k0 < KD; k0 += 16) {
+                uint32_t ak[4], aq[4];
+                load_a(ak, sK, KP, m0, k0, lane);
+                load_a(aq, sQ, KP, m0, k0, lane);
+#pragma unroll
+                for (int nt = 0; nt < 8; nt += 2)
+                    if (nt * 8 < m0 + 16) {
+                        uint32_t b[4];
+                        load_b(b, sK, KP, nt * 8, k0, lane);
+                        mma16816(acc[nt], ak, b[0], b[1]);
+                        mma16816(acc[nt + 1], ak, b[2], b[3]);
+                        mma16816(racc[nt], aq, b[0], b[1]);
+                        mma16816(racc[nt + 1], aq, b[2], b[3]);
+                    }
+            }
             const float b2[2] = {sBeta[m0 + gq], sBeta[m0 + gq + 8]};   // read before the stores below: they may alias for the compiler
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt)
+                if (nt * 8 < m0 + 16) {          // tiles above the diagonal are never read
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    const float bb = b2[hh];
-                    *reinterpret_cast<float2*>(sA + i * PA + j) =
-                        make_float2(i > j ? bb * acc[nt][2 * hh] : 0.f, i > j + 1 ? bb * acc[nt][2 * hh + 1] : 0.f);
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
+                        const float bb = b2[hh];
+                        *reinterpret_cast<float2*>(sA + i * PA + j) =
+                            make_float2(i > j ? bb * acc[nt][2 * hh] : 0.f, i > j + 1 ? bb * acc[nt][2 * hh + 1] : 0.f);
+                    }
+                    if (nt * 8 >= m0) {          // only the warp's two diagonal 8-column tiles can hold i < j
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int i = m0 + gq + (e >> 1) * 8, j = nt * 8 + 2 * tq + (e & 1);
+                            if (i < j) racc[nt][e] = 0.f;
+                        }
+                    }
                 }
+            pack_a(ra, racc);
         }
         __syncwarp();
         tril_inverse_64<PA>(sA, warp, lane);
-        {   // Awb = X diag(beta) as bf16, written over the front of the fp32 tile
+        {   // Awb = X diag(beta) as bf16, written over the front of the fp32 tile: the warp's own rows, up to the diagonal
             const int r = tid >> 1, half = tid & 1;
             uint32_t w[16];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float4 v = *reinterpret_cast<const float4*>(sA + r * PA + half * 32 + 4 * q);
-                const float4 b = *reinterpret_cast<const float4*>(sBeta + half * 32 + 4 * q);
-                w[2 * q] = pack_bf16x2(v.x * b.x, v.y * b.y);
-                w[2 * q + 1] = pack_bf16x2(v.z * b.z, v.w * b.w);
-            }
+            for (int p = 0; p < 2; ++p)
+                if (2 * p + half <= warp) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {      // 16 columns per thread and step: the two halves are four bank groups apart
+                        const float4 v = *reinterpret_cast<const float4*>(sA + r * PA + p * 32 + half * 16 + 4 * q);
+                        const float4 b = *reinterpret_cast<const float4*>(sBeta + p * 32 + half * 16 + 4 * q);
+                        w[8 * p + 2 * q] = pack_bf16x2(v.x * b.x, v.y * b.y);
+                        w[8 * p + 2 * q + 1] = pack_bf16x2(v.z * b.z, v.w * b.w);
+                    }
+                }
             __syncthreads();
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                reinterpret_cast<uint4*>(sAw + r * CP + half * 32)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+            for (int p = 0; p < 2; ++p)
+                if (2 * p + half <= warp) {
+                    uint4* d = reinterpret_cast<uint4*>(sAw + r * CP + p * 32 + half * 16);
+                    d[0] = make_uint4(w[8 * p], w[8 * p + 1], w[8 * p + 2], w[8 * p + 3]);
+                    d[1] = make_uint4(w[8 * p + 4], w[8 * p + 5], w[8 * p + 6], w[8 * p + 7]);
+                }
         }
         __syncthreads();
     }
     const float osc = HIER ? 1.f : a.scale;
     // ---- per-warp part (rows m0..m0+15 of everything; nothing leaves the warp) --------------------
     {
-        // tril(Q K^T) as A fragments, straight from its accumulators
-        uint32_t ra[4][4];
+        // R = tril(QK^T) Awb, kept as accumulators and re-used as an A operand twice
         float racc[8][4];
         zero_acc<8>(racc);
-        warp_gemm<8, KD, false, false>(racc, sQ, KP, m0, sK, KP, 0, lane, KD, m0 + 16);
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-            if (nt >= (m0 >> 3)) {       // only the warp's two diagonal 8-column tiles can hold i < j
+        for (int kk = 0; kk < 4; ++kk)
+            if (kk * 16 < m0 + 16) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int i = m0 + gq + (e >> 1) * 8, j = nt * 8 + 2 * tq + (e & 1);
-                    if (i < j) racc[nt][e] = 0.f;
+                for (int nt = 0; nt < 2 * kk + 2; nt += 2) {          // Awb is lower-triangular too
+                    uint32_t b[4];
+                    load_b_t(b, sAw, CP, nt * 8, kk * 16, lane);
+                    mma16816(racc[nt], ra[kk], b[0], b[1]);
+                    mma16816(racc[nt + 1], ra[kk], b[2], b[3]);
                 }
             }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            ra[kk][0] = pack_bf16x2(racc[2 * kk][0], racc[2 * kk][1]);
-            ra[kk][1] = pack_bf16x2(racc[2 * kk][2], racc[2 * kk][3]);
-            ra[kk][2] = pack_bf16x2(racc[2 * kk + 1][0], racc[2 * kk + 1][1]);
-            ra[kk][3] = pack_bf16x2(racc[2 * kk + 1][2], racc[2 * kk + 1][3]);
-        }
-        // R = tril(QK^T) Awb, kept as accumulators and re-used as an A operand twice
-        zero_acc<8>(racc);
-        warp_gemm_ra<8, 4, true>(racc, ra, sAw, CP, 0, lane, m0 + 16, m0 + 16);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            ra[kk][0] = pack_bf16x2(racc[2 * kk][0], racc[2 * kk][1]);
-            ra[kk][1] = pack_bf16x2(racc[2 * kk][2], racc[2 * kk][3]);
-            ra[kk][2] = pack_bf16x2(racc[2 * kk + 1][0], racc[2 * kk + 1][1]);
-            ra[kk][3] = pack_bf16x2(racc[2 * kk + 1][2], racc[2 * kk + 1][3]);
-        }
-        // Q~ = s e^G (Q - R K)
-        {
-            float acc[KD / 8][4];
-            zero_acc<KD / 8>(acc);
-            warp_gemm_ra<KD / 8, 4, true>(acc, ra, sK, KP, 0, lane, m0 + 16, KD);
-            __nv_bfloat16* gQ = reinterpret_cast<__nv_bfloat16*>(rec + R::QT_OFF);
-            const float fq[2] = {osc * sEG[m0 + gq], osc * sEG[m0 + gq + 8]};
-#pragma unroll
-            for (int nt = 0; nt < KD / 8; ++nt)
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    const float f = fq[hh];
-                    const float2 qv = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sQ + i * KP + j));
-                    *reinterpret_cast<uint32_t*>(gQ + R::T::off(i, j)) =
-                        pack_bf16x2(f * (qv.x - acc[nt][2 * hh]), f * (qv.y - acc[nt][2 * hh + 1]));
-                }
-        }
-        // Pm = R .* E .* lambda, as A fragments;  O_local = s Pm V
+        pack_a(ra, racc);
+        // Pm = R .* E .* lambda, as A fragments
+        uint32_t pa[4][4];
         {
             // level(i, j) = bit_length(i ^ j).  Off the diagonal 8x8 tile it depends on the tile only
             // (3 + bit_length(i/8 ^ j/8)): one lambda per (row, tile) serves both of the thread's columns.
@@ -336,30 +352,49 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
                     racc[nt][2 * hh + 1] = p1;
                 }
             }
+            pack_a(pa, racc);
+        }
+        // Q~ = s e^G (Q - R K) and W = Awb K: one pass over K's fragments.  W goes over this warp's own rows of Q.
+        {
+            float acc[KD / 8][4], wacc[KD / 8][4];
+            zero_acc<KD / 8>(acc);
+            zero_acc<KD / 8>(wacc);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                ra[kk][0] = pack_bf16x2(racc[2 * kk][0], racc[2 * kk][1]);
-                ra[kk][1] = pack_bf16x2(racc[2 * kk][2], racc[2 * kk][3]);
-                ra[kk][2] = pack_bf16x2(racc[2 * kk + 1][0], racc[2 * kk + 1][1]);
-                ra[kk][3] = pack_bf16x2(racc[2 * kk + 1][2], racc[2 * kk + 1][3]);
-            }
-            float acc[VD / 8][4];
-            zero_acc<VD / 8>(acc);
-            warp_gemm_ra<VD / 8, 4, true>(acc, ra, sV, VP, 0, lane, m0 + 16, VD);
-            __nv_bfloat16* gO = reinterpret_cast<__nv_bfloat16*>(rec + R::OL_OFF);
+            for (int kk = 0; kk < 4; ++kk)
+                if (kk * 16 < m0 + 16) {
+                    uint32_t af[4];
+                    load_a(af, sAw, CP, m0, kk * 16, lane);
 #pragma unroll
-            for (int nt = 0; nt < VD / 8; ++nt)
+                    for (int nt = 0; nt < KD / 8; nt += 2) {
+                        uint32_t b[4];
+                        load_b_t(b, sK, KP, nt * 8, kk * 16, lane);
+                        mma16816(acc[nt], ra[kk], b[0], b[1]);
+                        mma16816(acc[nt + 1], ra[kk], b[2], b[3]);
+                        mma16816(wacc[nt], af, b[0], b[1]);
+                        mma16816(wacc[nt + 1], af, b[2], b[3]);
+                    }
+                }
+            __nv_bfloat16* gQ = reinterpret_cast<__nv_bfloat16*>(rec + R::QT_OFF);
+            const float fq[2] = {osc * sEG[m0 + gq], osc * sEG[m0 + gq + 8]};
+#pragma unroll
+            for (int nt = 0; nt < KD / 8; ++nt)
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    *reinterpret_cast<uint32_t*>(gO + R::TV::off(i, j)) =
-                        pack_bf16x2(osc * acc[nt][2 * hh], osc * acc[nt][2 * hh + 1]);
+                    const float f = fq[hh];
+                    uint32_t* sq = reinterpret_cast<uint32_t*>(sQ + i * KP + j);   // read, then replaced, by this thread only
+                    const float2 qv = unpack_bf16x2(*sq);
+                    *sq = pack_bf16x2(wacc[nt][2 * hh], wacc[nt][2 * hh + 1]);
+                    *reinterpret_cast<uint32_t*>(gQ + R::T::off(i, j)) =
+                        pack_bf16x2(f * (qv.x - acc[nt][2 * hh]), f * (qv.y - acc[nt][2 * hh + 1]));
                 }
         }
-        // U^ = diag(e^{Glast-G}) (Awb .* E) V = (Awb diag(e^{Glast-G})) V: a column factor on the A fragments in registers
+        // O_local = s Pm V and U^ = diag(e^{Glast-G}) (Awb .* E) V = (Awb diag(e^{Glast-G})) V, a column factor on the
+        // A fragments in registers: one pass over V's fragments
         {
-            float acc[VD / 8][4];
+            float acc[VD / 8][4], uacc[VD / 8][4];
             zero_acc<VD / 8>(acc);
+            zero_acc<VD / 8>(uacc);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 if (kk * 16 < m0 + 16) {
@@ -378,31 +413,22 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
                     for (int nt = 0; nt < VD / 8; nt += 2) {
                         uint32_t b[4];
                         load_b_t(b, sV, VP, nt * 8, kk * 16, lane);
-                        mma16816(acc[nt], af, b[0], b[1]);
-                        mma16816(acc[nt + 1], af, b[2], b[3]);
+                        mma16816(acc[nt], pa[kk], b[0], b[1]);
+                        mma16816(acc[nt + 1], pa[kk], b[2], b[3]);
+                        mma16816(uacc[nt], af, b[0], b[1]);
+                        mma16816(uacc[nt + 1], af, b[2], b[3]);
                     }
                 }
             }
+            __nv_bfloat16* gO = reinterpret_cast<__nv_bfloat16*>(rec + R::OL_OFF);
 #pragma unroll
             for (int nt = 0; nt < VD / 8; ++nt)
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(acc[nt][2 * hh], acc[nt][2 * hh + 1]);
-                }
-        }
-        // W = Awb K, written over this warp's own rows of Q (no longer needed)
-        {
-            float acc[KD / 8][4];
-            zero_acc<KD / 8>(acc);
-            warp_gemm<KD / 8, CHUNK, false, true>(acc, sAw, CP, m0, sK, KP, 0, lane, m0 + 16, KD);
-            __syncwarp();
-#pragma unroll
-            for (int nt = 0; nt < KD / 8; ++nt)
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    *reinterpret_cast<uint32_t*>(sW + i * KP + j) = pack_bf16x2(acc[nt][2 * hh], acc[nt][2 * hh + 1]);
+                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(uacc[nt][2 * hh], uacc[nt][2 * hh + 1]);
+                    *reinterpret_cast<uint32_t*>(gO + R::TV::off(i, j)) =
+                        pack_bf16x2(osc * acc[nt][2 * hh], osc * acc[nt][2 * hh + 1]);
                 }
         }
     }
@@ -429,15 +455,16 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
                 *reinterpret_cast<uint32_t*>(stM + R::T::off(i, j)) = pack_bf16x2(m_0, m_1);
             }
     }
-    if (m0 < VD) {
+    const int v0 = KD <= 32 && VD <= 32 ? m0 - 32 : m0;      // two tiles of rows each: warps 0, 1 form M, warps 2, 3 form B^T
+    if (v0 >= 0 && v0 < VD) {
         float acc[KD / 8][4];
         zero_acc<KD / 8>(acc);
-        warp_gemm<KD / 8, CHUNK, true, true>(acc, sUh, VP, m0, sK, KP, 0, lane, CHUNK, KD);
+        warp_gemm<KD / 8, CHUNK, true, true>(acc, sUh, VP, v0, sK, KP, 0, lane, CHUNK, KD);
 #pragma unroll
         for (int nt = 0; nt < KD / 8; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
+                const int i = v0 + gq + hh * 8, j = nt * 8 + 2 * tq;
                 *reinterpret_cast<uint32_t*>(stB + R::T::off(i, j)) = pack_bf16x2(acc[nt][2 * hh], acc[nt][2 * hh + 1]);
             }
     }
