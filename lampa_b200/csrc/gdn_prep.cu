@@ -50,8 +50,8 @@ struct PrepSmem {
     static constexpr int UH = AW + CHUNK * CP * 2;               // bf16 [64][VP]   diag(e^{Glast-G}) U
     static constexpr int AFTER_UH = UH + CHUNK * VP * 2, AFTER_SA = AW + CHUNK * PA * 4;   // the fp32 tile covers AW and UH
     static constexpr int G = AFTER_UH > AFTER_SA ? AFTER_UH : AFTER_SA;   // fp32 [64] G, [64] beta, [64] e^G, [64] e^{Glast-G}, [64] e^{G(end of the 8-block)-G}
-    static constexpr int LAM = G + 5 * CHUNK * 4;                // fp32 [64][L+1]
-    static int bytes(int L) { return LAM + CHUNK * (L + 1) * 4; }
+    static constexpr int LAM = G + 5 * CHUNK * 4;                // fp32 [64][7]: the levels inside the chunk, an odd pitch
+    static constexpr int bytes(bool hier) { return LAM + (hier ? CHUNK * ELL0 * 4 : 0); }
 };
 
 // With beta folded into the columns of the inverse (Awb = (I + A0)^-1 diag(beta), Aub = Awb .* E):
@@ -61,19 +61,33 @@ struct PrepSmem {
 //   O_local = s ((R .* E .* lambda[i][level(i,j)]) V)
 // (s = scale and lambda = 1 for the plain rule; s = 1 for the hierarchical one).  These equal
 // the definitions in gdn.cuh: every e^{G_last-G_tok} e^{G_tok} pair collapses to e^{G_last}.
-// eight accumulator tiles (16 x 64) as the A fragments of the next product
-__device__ __forceinline__ void pack_a(uint32_t (&f)[4][4], const float (&c)[8][4]) {
+// Half of a token's lambda row (levels half, half + 2, ...): NIT loads in flight, then the chunk's own levels go to
+// shared memory and the others straight to the record's [level][token] table.
+template <int NIT>
+__device__ __forceinline__ void stage_lambda(const GdnArgs& a, size_t base, int half, bool valid, float* own, float* lamc) {
+    float lv[NIT];
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-        f[kk][0] = pack_bf16x2(c[2 * kk][0], c[2 * kk][1]);
-        f[kk][1] = pack_bf16x2(c[2 * kk][2], c[2 * kk][3]);
-        f[kk][2] = pack_bf16x2(c[2 * kk + 1][0], c[2 * kk + 1][1]);
-        f[kk][3] = pack_bf16x2(c[2 * kk + 1][2], c[2 * kk + 1][3]);
+    for (int i = 0; i < NIT; ++i) {
+        const int l = half + 2 * i;
+        lv[i] = (valid && l < a.L) ? load_as_float(a.lam, base + l, a.lam_dt) : 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < NIT; ++i) {
+        const int l = half + 2 * i;
+        if (l < ELL0) own[l] = lv[i];
+        else if (l < ELL0 + a.LC) lamc[(l - ELL0) * CHUNK] = lv[i];
+    }
+}
+// two accumulator tiles (16 x 16) as one A fragment of the next product
+__device__ __forceinline__ void pack_a(uint32_t (&f)[4], const float (&c0)[4], const float (&c1)[4]) {
+    f[0] = pack_bf16x2(c0[0], c0[1]);
+    f[1] = pack_bf16x2(c0[2], c0[3]);
+    f[2] = pack_bf16x2(c1[0], c1[1]);
+    f[3] = pack_bf16x2(c1[2], c1[3]);
 }
 
 template <int KD, int VD, bool HIER>
-__global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs a) {
+__global__ void __launch_bounds__(128, KD == 64 ? 4 : 6) gdn_prep_kernel(GdnArgs a) {
     using S = PrepSmem<KD, VD>;
     using R = Rec<KD, VD>;
     constexpr int KP = S::KP, VP = S::VP, CP = S::CP;
@@ -101,7 +115,7 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
     const int gq = lane >> 2, tq = lane & 3;
     const int64_t t0 = loc.t0;
     const int len = loc.len;
-    const int LP = a.L + 1;
+    char* rec = a.rec + ((size_t)c * H + h) * a.rec_bytes;
     if (h == 0) check_out_perm(a, t0, len);
 
     // ---- stage 0: loads, l2norm, cumulative decay -------------------------------------------------
@@ -128,9 +142,10 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
         }
         if (HIER) {   // all of the row's loads in flight before the first store; the unrolled length follows L
             const size_t lam_base = (tok * H + h) * a.L;
-            if (a.L <= 18) stage_lambda<9>(a.lam, a.lam_dt, lam_base, a.L, half, valid, sLam + r * LP);
-            else if (a.L <= 24) stage_lambda<12>(a.lam, a.lam_dt, lam_base, a.L, half, valid, sLam + r * LP);
-            else stage_lambda<20>(a.lam, a.lam_dt, lam_base, a.L, half, valid, sLam + r * LP);
+            float* lamc = reinterpret_cast<float*>(rec + R::LAM_OFF) + r;
+            if (a.L <= 18) stage_lambda<9>(a, lam_base, half, valid, sLam + r * ELL0, lamc);
+            else if (a.L <= 24) stage_lambda<12>(a, lam_base, half, valid, sLam + r * ELL0, lamc);
+            else stage_lambda<20>(a, lam_base, half, valid, sLam + r * ELL0, lamc);
         }
         if (h == 0) {   // L2 prefetch of the token rows (all heads) of a chunk ~80 chunks ahead
             ChunkLoc l2;
@@ -205,17 +220,8 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
         sEGl[tid] = __expf(Gl - Gi);
         sCF[tid] = __expf(sG[tid | 7] - Gi);
     }
-    char* rec = a.rec + ((size_t)c * H + h) * a.rec_bytes;
-    if (HIER) {   // lambda of the chunk levels, transposed to [level][token] for the scan
-        float* lamc = reinterpret_cast<float*>(rec + R::LAM_OFF);
-        for (int idx = tid; idx < a.LC * CHUNK; idx += 128) {
-            const int l = idx >> 6, r = idx & 63;
-            lamc[idx] = (ELL0 + l < a.L) ? sLam[r * LP + ELL0 + l] : 0.f;
-        }
-    }
-
     const int m0 = warp * 16;
-    uint32_t ra[4][4];                                       // tril(Q K^T), later R, as A fragments
+    uint32_t qk[4][4];                                       // tril(Q K^T) as A fragments
     // ---- stage 1: Awb = (I + A0)^-1 diag(beta), A0 = tril(diag(beta) K K^T, -1) ---------------------
     // Blockwise, as the reference's solve_tril does (models/hattention/solve_tril.py:221-276): warp w
     // forms rows 16w.. of A0 on the tensor cores and inverts its own 16x16 diagonal block by fp32
@@ -228,45 +234,45 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
         constexpr int PA = S::PA;
         float* sA = reinterpret_cast<float*>(smem + S::AW);
         {
-            float acc[8][4], racc[8][4];
-            zero_acc<8>(acc);
-            zero_acc<8>(racc);
+            uint32_t ak[KD / 16][4], aq[KD / 16][4];
 #pragma unroll
-            for (int k0 = 0; k0 < KD; k0 += 16) {
-                uint32_t ak[4], aq[4];
-                load_a(ak, sK, KP, m0, k0, lane);
-                load_a(aq, sQ, KP, m0, k0, lane);
-#pragma unroll
-                for (int nt = 0; nt < 8; nt += 2)
-                    if (nt * 8 < m0 + 16) {
-                        uint32_t b[4];
-                        load_b(b, sK, KP, nt * 8, k0, lane);
-                        mma16816(acc[nt], ak, b[0], b[1]);
-                        mma16816(acc[nt + 1], ak, b[2], b[3]);
-                        mma16816(racc[nt], aq, b[0], b[1]);
-                        mma16816(racc[nt + 1], aq, b[2], b[3]);
-                    }
+            for (int k = 0; k < KD / 16; ++k) {
+                load_a(ak[k], sK, KP, m0, 16 * k, lane);
+                load_a(aq[k], sQ, KP, m0, 16 * k, lane);
             }
             const float b2[2] = {sBeta[m0 + gq], sBeta[m0 + gq + 8]};   // read before the stores below: they may alias for the compiler
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt)
-                if (nt * 8 < m0 + 16) {          // tiles above the diagonal are never read
+            for (int np = 0; np < 4; ++np) {         // 16 columns at a time
+                float acc[2][4], racc[2][4];
+                zero_acc<2>(acc);
+                zero_acc<2>(racc);
+                if (np <= warp) {                    // tiles above the diagonal are never read
 #pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                        const float bb = b2[hh];
-                        *reinterpret_cast<float2*>(sA + i * PA + j) =
-                            make_float2(i > j ? bb * acc[nt][2 * hh] : 0.f, i > j + 1 ? bb * acc[nt][2 * hh + 1] : 0.f);
-                    }
-                    if (nt * 8 >= m0) {          // only the warp's two diagonal 8-column tiles can hold i < j
+                    for (int k = 0; k < KD / 16; ++k) {
+                        uint32_t b[4];
+                        load_b(b, sK, KP, np * 16, 16 * k, lane);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int i = m0 + gq + (e >> 1) * 8, j = nt * 8 + 2 * tq + (e & 1);
-                            if (i < j) racc[nt][e] = 0.f;
+                        for (int x = 0; x < 2; ++x) {
+                            mma16816(acc[x], ak[k], b[2 * x], b[2 * x + 1]);
+                            mma16816(racc[x], aq[k], b[2 * x], b[2 * x + 1]);
                         }
                     }
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int hh = 0; hh < 2; ++hh) {
+                            const int i = m0 + gq + hh * 8, j = np * 16 + x * 8 + 2 * tq;
+                            const float bb = b2[hh];
+                            *reinterpret_cast<float2*>(sA + i * PA + j) =
+                                make_float2(i > j ? bb * acc[x][2 * hh] : 0.f, i > j + 1 ? bb * acc[x][2 * hh + 1] : 0.f);
+                            if (np == warp) {        // only the warp's diagonal tile can hold i < j
+                                if (i < j) racc[x][2 * hh] = 0.f;
+                                if (i < j + 1) racc[x][2 * hh + 1] = 0.f;
+                            }
+                        }
                 }
-            pack_a(ra, racc);
+                pack_a(qk[np], racc[0], racc[1]);
+            }
         }
         __syncwarp();
         tril_inverse_64<PA>(sA, warp, lane);
@@ -298,137 +304,132 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
     const float osc = HIER ? 1.f : a.scale;
     // ---- per-warp part (rows m0..m0+15 of everything; nothing leaves the warp) --------------------
     {
-        // R = tril(QK^T) Awb, kept as accumulators and re-used as an A operand twice
-        float racc[8][4];
-        zero_acc<8>(racc);
+        // R = tril(QK^T) Awb, 16 columns at a time, and Pm = R .* E .* lambda, both as A fragments.
+        // level(i, j) = bit_length(i ^ j).  Off the diagonal 8x8 tile it depends on the tile only
+        // (3 + bit_length(i/8 ^ j/8)): one lambda per (row, tile) serves both of the thread's columns.
+        // The decay splits the same way: e^{G_i - G_end(tile)} per (row, tile) times the column's decay to the end of
+        // its tile, both at most 1 - one exponential per row and tile instead of two per pair of elements.
+        uint32_t ra[4][4], pa[4][4];
+        const float gi2[2] = {sG[m0 + gq], sG[m0 + gq + 8]};
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-            if (kk * 16 < m0 + 16) {
+        for (int np = 0; np < 4; ++np) {
+            float racc[2][4];
+            zero_acc<2>(racc);
 #pragma unroll
-                for (int nt = 0; nt < 2 * kk + 2; nt += 2) {          // Awb is lower-triangular too
+            for (int kk = np; kk < 4; ++kk)              // Awb is lower-triangular too
+                if (kk <= warp) {
                     uint32_t b[4];
-                    load_b_t(b, sAw, CP, nt * 8, kk * 16, lane);
-                    mma16816(racc[nt], ra[kk], b[0], b[1]);
-                    mma16816(racc[nt + 1], ra[kk], b[2], b[3]);
+                    load_b_t(b, sAw, CP, np * 16, kk * 16, lane);
+                    mma16816(racc[0], qk[kk], b[0], b[1]);
+                    mma16816(racc[1], qk[kk], b[2], b[3]);
                 }
-            }
-        pack_a(ra, racc);
-        // Pm = R .* E .* lambda, as A fragments
-        uint32_t pa[4][4];
-        {
-            // level(i, j) = bit_length(i ^ j).  Off the diagonal 8x8 tile it depends on the tile only
-            // (3 + bit_length(i/8 ^ j/8)): one lambda per (row, tile) serves both of the thread's columns.
-            // The decay splits the same way: e^{G_i - G_end(tile)} per (row, tile) times the column's decay to the end of
-            // its tile, both at most 1 - one exponential per row and tile instead of two per pair of elements.
-            const float gi2[2] = {sG[m0 + gq], sG[m0 + gq + 8]};
+            pack_a(ra[np], racc[0], racc[1]);
+            if (np <= warp) {
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                const float2 cf = *reinterpret_cast<const float2*>(sCF + nt * 8 + 2 * tq);
-                const float gend = sG[nt * 8 + 7];
+                for (int x = 0; x < 2; ++x) {
+                    const int nt = 2 * np + x, j = nt * 8 + 2 * tq;
+                    const float2 cf = *reinterpret_cast<const float2*>(sCF + j);
+                    const float gend = sG[nt * 8 + 7];
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    const int it = (m0 >> 3) + hh;                     // the row's 8x8 tile index (warp-uniform)
-                    float p0 = 0.f, p1 = 0.f;
-                    if (nt <= it) {
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int i = m0 + gq + hh * 8;
+                        const int it = (m0 >> 3) + hh;                     // the row's 8x8 tile index (warp-uniform)
+                        float p0 = 0.f, p1 = 0.f;
                         if (nt < it) {
                             p0 = __expf(gi2[hh] - gend);
-                            if (HIER) p0 *= sLam[i * LP + 3 + (32 - __clz(it ^ nt))];
+                            if (HIER) p0 *= sLam[i * ELL0 + 3 + (32 - __clz(it ^ nt))];
                             p1 = p0 * cf.y;
                             p0 *= cf.x;
-                        } else {
-                            const float2 gj = *reinterpret_cast<const float2*>(sG + nt * 8 + 2 * tq);
+                        } else if (nt == it) {
+                            const float2 gj = *reinterpret_cast<const float2*>(sG + j);
                             if (i >= j) p0 = __expf(gi2[hh] - gj.x);
                             if (i >= j + 1) p1 = __expf(gi2[hh] - gj.y);
                             if (HIER) {
-                                p0 *= sLam[i * LP + (32 - __clz(i ^ j))];
-                                p1 *= sLam[i * LP + (32 - __clz(i ^ (j + 1)))];
+                                p0 *= sLam[i * ELL0 + (32 - __clz(i ^ j))];
+                                p1 *= sLam[i * ELL0 + (32 - __clz(i ^ (j + 1)))];
                             }
                         }
-                        p0 *= racc[nt][2 * hh];
-                        p1 *= racc[nt][2 * hh + 1];
+                        racc[x][2 * hh] *= p0;
+                        racc[x][2 * hh + 1] *= p1;
                     }
-                    racc[nt][2 * hh] = p0;
-                    racc[nt][2 * hh + 1] = p1;
                 }
             }
-            pack_a(pa, racc);
+            pack_a(pa[np], racc[0], racc[1]);
         }
-        // Q~ = s e^G (Q - R K) and W = Awb K: one pass over K's fragments.  W goes over this warp's own rows of Q.
-        {
-            float acc[KD / 8][4], wacc[KD / 8][4];
-            zero_acc<KD / 8>(acc);
-            zero_acc<KD / 8>(wacc);
+        // Q~ = s e^G (Q - R K) and W = Awb K, 16 columns at a time over the same fragments of K.  W goes over this warp's
+        // own rows of Q.
+        __nv_bfloat16* gQ = reinterpret_cast<__nv_bfloat16*>(rec + R::QT_OFF);
+        const float fq[2] = {osc * sEG[m0 + gq], osc * sEG[m0 + gq + 8]};
+#pragma unroll
+        for (int np = 0; np < KD / 16; ++np) {
+            float acc[2][4], wacc[2][4];
+            zero_acc<2>(acc);
+            zero_acc<2>(wacc);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                if (kk * 16 < m0 + 16) {
-                    uint32_t af[4];
+                if (kk <= warp) {
+                    uint32_t af[4], b[4];
                     load_a(af, sAw, CP, m0, kk * 16, lane);
+                    load_b_t(b, sK, KP, np * 16, kk * 16, lane);
 #pragma unroll
-                    for (int nt = 0; nt < KD / 8; nt += 2) {
-                        uint32_t b[4];
-                        load_b_t(b, sK, KP, nt * 8, kk * 16, lane);
-                        mma16816(acc[nt], ra[kk], b[0], b[1]);
-                        mma16816(acc[nt + 1], ra[kk], b[2], b[3]);
-                        mma16816(wacc[nt], af, b[0], b[1]);
-                        mma16816(wacc[nt + 1], af, b[2], b[3]);
+                    for (int x = 0; x < 2; ++x) {
+                        mma16816(acc[x], ra[kk], b[2 * x], b[2 * x + 1]);
+                        mma16816(wacc[x], af, b[2 * x], b[2 * x + 1]);
                     }
                 }
-            __nv_bfloat16* gQ = reinterpret_cast<__nv_bfloat16*>(rec + R::QT_OFF);
-            const float fq[2] = {osc * sEG[m0 + gq], osc * sEG[m0 + gq + 8]};
 #pragma unroll
-            for (int nt = 0; nt < KD / 8; ++nt)
+            for (int x = 0; x < 2; ++x)
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    const float f = fq[hh];
+                    const int i = m0 + gq + hh * 8, j = np * 16 + x * 8 + 2 * tq;
                     uint32_t* sq = reinterpret_cast<uint32_t*>(sQ + i * KP + j);   // read, then replaced, by this thread only
                     const float2 qv = unpack_bf16x2(*sq);
-                    *sq = pack_bf16x2(wacc[nt][2 * hh], wacc[nt][2 * hh + 1]);
+                    *sq = pack_bf16x2(wacc[x][2 * hh], wacc[x][2 * hh + 1]);
                     *reinterpret_cast<uint32_t*>(gQ + R::T::off(i, j)) =
-                        pack_bf16x2(f * (qv.x - acc[nt][2 * hh]), f * (qv.y - acc[nt][2 * hh + 1]));
+                        pack_bf16x2(fq[hh] * (qv.x - acc[x][2 * hh]), fq[hh] * (qv.y - acc[x][2 * hh + 1]));
                 }
         }
         // O_local = s Pm V and U^ = diag(e^{Glast-G}) (Awb .* E) V = (Awb diag(e^{Glast-G})) V, a column factor on the
-        // A fragments in registers: one pass over V's fragments
-        {
-            float acc[VD / 8][4], uacc[VD / 8][4];
-            zero_acc<VD / 8>(acc);
-            zero_acc<VD / 8>(uacc);
+        // A fragments in registers, over the same fragments of V
+        __nv_bfloat16* gO = reinterpret_cast<__nv_bfloat16*>(rec + R::OL_OFF);
+        uint32_t (&ua)[4][4] = ra;                           // R is used up
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                if (kk * 16 < m0 + 16) {
-                    uint32_t af[4];
-                    load_a(af, sAw, CP, m0, kk * 16, lane);
+        for (int kk = 0; kk < 4; ++kk)
+            if (kk <= warp) {
+                load_a(ua[kk], sAw, CP, m0, kk * 16, lane);
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const float2 f = *reinterpret_cast<const float2*>(sEGl + kk * 16 + x * 8 + 2 * tq);
+                for (int x = 0; x < 2; ++x) {
+                    const float2 f = *reinterpret_cast<const float2*>(sEGl + kk * 16 + x * 8 + 2 * tq);
 #pragma unroll
-                        for (int y = 0; y < 2; ++y) {
-                            const float2 w = unpack_bf16x2(af[2 * x + y]);
-                            af[2 * x + y] = pack_bf16x2(w.x * f.x, w.y * f.y);
-                        }
-                    }
-#pragma unroll
-                    for (int nt = 0; nt < VD / 8; nt += 2) {
-                        uint32_t b[4];
-                        load_b_t(b, sV, VP, nt * 8, kk * 16, lane);
-                        mma16816(acc[nt], pa[kk], b[0], b[1]);
-                        mma16816(acc[nt + 1], pa[kk], b[2], b[3]);
-                        mma16816(uacc[nt], af, b[0], b[1]);
-                        mma16816(uacc[nt + 1], af, b[2], b[3]);
+                    for (int y = 0; y < 2; ++y) {
+                        const float2 w = unpack_bf16x2(ua[kk][2 * x + y]);
+                        ua[kk][2 * x + y] = pack_bf16x2(w.x * f.x, w.y * f.y);
                     }
                 }
             }
-            __nv_bfloat16* gO = reinterpret_cast<__nv_bfloat16*>(rec + R::OL_OFF);
 #pragma unroll
-            for (int nt = 0; nt < VD / 8; ++nt)
+        for (int np = 0; np < VD / 16; ++np) {
+            float acc[2][4], uacc[2][4];
+            zero_acc<2>(acc);
+            zero_acc<2>(uacc);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+                if (kk <= warp) {
+                    uint32_t b[4];
+                    load_b_t(b, sV, VP, np * 16, kk * 16, lane);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        mma16816(acc[x], pa[kk], b[2 * x], b[2 * x + 1]);
+                        mma16816(uacc[x], ua[kk], b[2 * x], b[2 * x + 1]);
+                    }
+                }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    const int i = m0 + gq + hh * 8, j = nt * 8 + 2 * tq;
-                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(uacc[nt][2 * hh], uacc[nt][2 * hh + 1]);
-                    *reinterpret_cast<uint32_t*>(gO + R::TV::off(i, j)) =
-                        pack_bf16x2(osc * acc[nt][2 * hh], osc * acc[nt][2 * hh + 1]);
+                    const int i = m0 + gq + hh * 8, j = np * 16 + x * 8 + 2 * tq;
+                    *reinterpret_cast<uint32_t*>(sUh + i * VP + j) = pack_bf16x2(uacc[x][2 * hh], uacc[x][2 * hh + 1]);
+                    *reinterpret_cast<uint32_t*>(gO + R::TV::off(i, j)) = pack_bf16x2(osc * acc[x][2 * hh], osc * acc[x][2 * hh + 1]);
                 }
         }
     }
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(128, KD == 64 ? 4 : 5) gdn_prep_kernel(GdnArgs
 template <int KD, int VD>
 int launch_prep(const GdnArgs& a, bool hier, cudaStream_t st) {
     using S = PrepSmem<KD, VD>;
-    const int smem = S::bytes(hier ? a.L : 0);
+    const int smem = S::bytes(hier);
     dim3 grid(a.H, a.nc_max);
     cudaError_t e;
     ProfScope prof(hier ? "gdn_prep_hier" : "gdn_prep_plain", st);
