@@ -13,8 +13,8 @@
 // row) and quarter of the columns, adds B^T where the level is collecting, clears it at the end of
 // its period and writes the bf16 row back into the A operand for the next chunk; then it scales
 // the level's contribution to its 16 tokens by lambda and accumulates it over the pairs.
-// Warp-specialised: 16 epilogue warps (warp = 32 rows x 16 state columns x 16 tokens; together they
-// also transpose the chunk's output through shared memory and store it with O_local added) and one
+// Warp-specialised: 16 epilogue warps (warp = 32 rows x 16 state columns x 16 tokens), four output warps that take the
+// chunk's output from them through shared memory and store it with O_local added, and one
 // control warp whose first lane streams the records in (bulk async copies, three stages) and issues
 // the MMAs.  The MMAs take the accumulator buffers in turn; one is issued as soon as every epilogue warp has
 // handed back the buffer it overwrites, which it does after rewriting the pair's operand and reading the
@@ -23,6 +23,7 @@
 // pair; every mbarrier wait is bounded, and a CTA whose wait ran out stops issuing copies and MMAs, lets
 // every warp walk through its remaining barriers in lockstep, waits for the copies and MMAs in flight
 // and only then frees its tensor memory.
+#include "act.cuh"
 #include "gdn.cuh"
 #include "profile.cuh"
 #include "umma.cuh"
@@ -34,11 +35,13 @@ namespace {
 constexpr int UKD = 64, UVD = 64;
 constexpr int UNP = 5;                       // pairs of slots: up to 5 in-block levels + up to 5 cross-block levels
 constexpr int UEPI_WARPS = 16;               // 4 warpgroups, each covering 16 state columns and 16 tokens of all 128 rows
-constexpr int UTHREADS = (UEPI_WARPS + 2) * 32;   // plus one control warp and one relay warp
+constexpr int UOUT_WARPS = 4;                 // hierarchical pass: warps that store the output
+constexpr int PTHREADS = (UEPI_WARPS + 2) * 32;   // plus one control warp and one relay warp
+constexpr int UTHREADS = PTHREADS + UOUT_WARPS * 32;
 // An mbarrier poll costs the polling warp 200 - 300 cycles even when the phase is long complete, a hardware named
 // barrier that everybody else has already reached about 30.  So only the relay warp polls the mbarriers the epilogue
 // depends on ("record landed", "pair's MMA complete") and passes each completion on through a named barrier that the
-// sixteen epilogue warps join (ids 5 + p; ids 1..4 belong to the output transpose), and the epilogue hands a pair's
+// sixteen epilogue warps join (ids 5 + p; ids 1..4 belong to the output tile), and the epilogue hands a pair's
 // accumulator back to the control warp the same way (ids 11 + p: sixteen warps arrive, the control warp waits).
 // Nobody can be left waiting at a named barrier: the relay's and the control lane's own waits are bounded and both
 // walk through every barrier whether or not a wait ran out, and the epilogue never waits for anything else.  Nobody
@@ -47,6 +50,11 @@ constexpr int UTHREADS = (UEPI_WARPS + 2) * 32;   // plus one control warp and o
 // arriving and running on.  (The plain-rule kernel below has one MMA group per chunk and hands its operands back
 // through an mbarrier: there the named barrier measured slower; its records alternate between ids 10 and 11.)
 constexpr int UNB_PAIR = 5, UNB_REC = 10, UNB_DFREE = 11, UNB_COUNT = (UEPI_WARPS + 1) * 32;
+// Hierarchical pass: the chunk's output tile (fp32, two buffers in turn) goes to the output warps at id 1 + buffer, and
+// comes back at id 3 + buffer.  Both sides wait for the other before they reuse a buffer, so neither can reach a barrier twice.
+constexpr int UNB_OFULL = 1, UNB_OFREE = 3, UNB_OCOUNT = (UEPI_WARPS + UOUT_WARPS) * 32;
+__device__ __forceinline__ void out_arrive(int id) { asm volatile("bar.arrive %0, %1;\n" :: "r"(id), "n"(UNB_OCOUNT) : "memory"); }
+__device__ __forceinline__ void out_sync(int id) { asm volatile("bar.sync %0, %1;\n" :: "r"(id), "n"(UNB_OCOUNT) : "memory"); }
 __device__ __forceinline__ void named_arrive(int id) { asm volatile("bar.arrive %0, %1;\n" :: "r"(id), "n"(UNB_COUNT) : "memory"); }
 __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;\n" :: "r"(id), "n"(UNB_COUNT) : "memory"); }
 __device__ __forceinline__ void relay_pass(int id, bool dead) { if (dead) named_sync(id); else named_arrive(id); }
@@ -76,10 +84,15 @@ struct UnitOrder {
     unsigned char order[64];    // block indices, most level pairs first
 };
 
+// A chunk's step is bound by the serial work of the epilogue warps (two tensor-memory round trips and two barriers per
+// pair), so nothing else is left to them: storing the output took 1840 of a step's 5250 cycles at four pairs, most of it
+// waiting for the scatter index, which four warps of their own now fetch a chunk ahead.  60,000 hits, 8 heads, 10 levels,
+// scattered output: 182 -> 150 us.  (Two output warps: 158 us, and 27 instead of 25 us for a 6,000-hit event; loading both
+// halves of the accumulator row at once: 166 - 217 us, the registers spill.)
 __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs a, UnitOrder uo) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM_BAR);      // record landed            (tx count)
-    uint64_t* sfree = full + UNST;                                      // stage consumed           (16 warps)
+    uint64_t* sfree = full + UNST;                                      // stage consumed           (16 + 4 warps)
     uint64_t* mdone = sfree + UNST;                                     // pair's MMA complete      (commit)
     uint64_t* drainb = mdone + UNP;                                     // every MMA issued has completed (commit at the end)
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + SM_BAR + 256);
@@ -107,7 +120,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
     const int nsteps = min(bc, nch - b * bc);
     const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wg = warp >> 2;                          // 0..3: state columns / tokens 16*wg .. 16*wg+15; 4: control
+    const int wg = warp >> 2;                          // 0..3: state columns / tokens 16*wg .. 16*wg+15
     const int row = (warp & 3) * 32 + lane;            // TMEM lane = row of the pair's A operand
     const int u = row >> 6, v = row & 63;              // which slot of the pair, which state row
     const int part = wg & 3;
@@ -130,7 +143,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
 
     if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < UNST; ++s) { mbar_init(full + s, 1); mbar_init(sfree + s, UEPI_WARPS); }
+        for (int s = 0; s < UNST; ++s) { mbar_init(full + s, 1); mbar_init(sfree + s, UEPI_WARPS + UOUT_WARPS); }
 #pragma unroll
         for (int p = 0; p < UNP; ++p) mbar_init(mdone + p, 1);
         mbar_init(drainb, 1);
@@ -225,7 +238,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
             umma_commit(drainb);
             mbar_drain(drainb, 0u);
         }
-    } else if (wg == 4) {
+    } else if (warp == UEPI_WARPS + 1) {
         // ---- relay warp (the second warp of this group): mbarrier completions -> named barriers ----
         // "record landed" travels with the first pair of the chunk.  A pair's barrier cannot be reached a second time
         // before every epilogue warp has left it: the pair's next MMA is only issued after its accumulator came back.
@@ -237,8 +250,63 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
                 relay_pass(UNB_PAIR + p, dead);
             }
         }
+    } else if (warp > UEPI_WARPS + 1) {
+        // ---- output warps: sum the two rows (levels) of the pairs, add O_local, store ----
+        // thread = (every 16th token, 4 + 4 output columns: 4c.. and 32 + 4c..): the eight lanes of a token read 128
+        // contiguous bytes of the tile per load, which is what keeps the 16-byte loads free of bank conflicts
+        const int ot = tid - PTHREADS, tok = ot >> 3, col = (ot & 7) * 4;
+        auto drain_tiles = [&](auto scat) {
+            // a scattered row's index is asked for one chunk ahead and looked at (see out_row) when its tile is there
+            int64_t next[4];
+            auto ask_rows = [&](int i) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int64_t t = tok0 + (int64_t)i * CHUNK + tok + 16 * q;
+                    next[q] = t >= tok_end ? -1 : t;
+                    if (decltype(scat)::value && t < tok_end && t < a.out_perm_rows) next[q] = a.out_perm[t];
+                }
+            };
+            ask_rows(0);
+            for (int i = 0; i < nsteps; ++i) {
+                const int64_t orow[4] = {next[0], next[1], next[2], next[3]};
+                ask_rows(i + 1);
+                const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(stage0 + (size_t)(i % UNST) * stage_bytes + UR::OL_OFF);
+                const float* sOTc = sOT + (i & 1) * (2 * 64 * 64);
+                out_sync(UNB_OFULL + (i & 1));
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if ((unsigned long long)orow[q] >= (unsigned long long)a.total_tokens) continue;
+                    const int tk = tok + 16 * q;
+                    const size_t idx = ((size_t)orow[q] * H + h) * UVD + col;
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        const float4 p0 = *reinterpret_cast<const float4*>(sOTc + (0 * 64 + tk) * 64 + col + 32 * x);
+                        const float4 q0 = *reinterpret_cast<const float4*>(sOTc + (1 * 64 + tk) * 64 + col + 32 * x);
+                        const uint2 ol = *reinterpret_cast<const uint2*>(sOl + UR::TV::off(tk, col + 32 * x));      // 4 bf16 of O_local
+                        const float2 oa = unpack_bf16x2(ol.x), ob = unpack_bf16x2(ol.y);
+                        const float r0 = p0.x + q0.x + oa.x, r1 = p0.y + q0.y + oa.y, r2 = p0.z + q0.z + ob.x, r3 = p0.w + q0.w + ob.y;
+                        if (a.qkv_dt == LAMPA_F32) {
+                            *reinterpret_cast<float4*>((float*)a.o + idx + 32 * x) = make_float4(r0, r1, r2, r3);
+                        } else {
+                            uint2 w;
+                            if (a.qkv_dt == LAMPA_BF16) { w.x = pack_bf16x2(r0, r1); w.y = pack_bf16x2(r2, r3); }
+                            else {
+                                const __half2 ha = __floats2half2_rn(r0, r1), hb = __floats2half2_rn(r2, r3);
+                                w.x = *reinterpret_cast<const uint32_t*>(&ha); w.y = *reinterpret_cast<const uint32_t*>(&hb);
+                            }
+                            *reinterpret_cast<uint2*>((uint16_t*)a.o + idx + 32 * x) = w;
+                        }
+                    }
+                }
+                if (i + 2 < nsteps) out_arrive(UNB_OFREE + (i & 1));      // nobody waits for the last two
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sfree + (i % UNST));           // O_local of this stage has been read
+            }
+        };
+        if (a.out_perm_rows > 0) drain_tiles(ScatterOn{}); else drain_tiles(ScatterOff{});
     } else {
         // ---- epilogue warps: every warp advances 16 state columns and reads 16 tokens of its 32 rows ----
+        // The loop over pairs is unrolled: barrier ids, bit positions and operand columns are constants in it.
         // per pair, the lambda row of this thread's slot, and the slots that exist and have a lambda row
         uint32_t lam_pack = 0, slot_ok = 0;          // 5 bits per pair: the lambda row of slot 2p + u
 #pragma unroll
@@ -251,26 +319,30 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
             const int row = s < bl ? s : bl + (int)((live_pack >> (4 * (s - bl))) & 15);
             if (row < a.LC) slot_ok |= 1u << s;      // a missing row is only reachable when the level check already failed
         }
-        int bufi = 0;                                // accumulator buffer of the next pair, in step with the control warp
+        const uint32_t tpart = tlane + (uint32_t)(tm_d + 16 * part);
+        uint32_t buf = 0;                            // first column of the next pair's accumulator, in step with the control warp
         for (int i = 0; i < nsteps; ++i) {
             const unsigned char* st = stage0 + (size_t)(i % UNST) * stage_bytes;
-            const float* sLam = reinterpret_cast<const float*>(st + STAGE_TILES);
+            const float* sLam = reinterpret_cast<const float*>(st + STAGE_TILES) + 16 * part;
             const unsigned char* sBt = st + UR::BT_OFF;
             const int n = b * bc + i;
-            const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + UR::OL_OFF);
-            // what this chunk does to each slot, as bit masks: in-block level s is read when bit s of n is
-            // set and cleared when its period of 2^(s+1) chunks ends (all of bits 0..s set); the cross-block
-            // slots are read by every chunk
+            // what this chunk does to each slot, as bit masks of this thread's slots (bit 2p = slot 2p + u): in-block level
+            // s is read when bit s of n is set, collects when it is not, and is cleared when its period of 2^(s+1) chunks
+            // ends (all of bits 0..s set); the cross-block slots are read by every chunk
             const uint32_t low = (uint32_t)n & (bc - 1);
-            const uint32_t read_mask = (low | (~0u << bl)) & slot_ok;
-            const uint32_t clear_mask = low & ~(low + 1u) & (bc - 1);      // trailing ones of n
+            const uint32_t read_mask = ((low | (~0u << bl)) & slot_ok) >> u;
+            const uint32_t clear_mask = (low & ~(low + 1u) & (bc - 1)) >> u;      // trailing ones of n
+            const uint32_t add_mask = (~low & (bc - 1)) >> u;
+            const uint32_t step_mask = i + 1 < nsteps ? ((1u << nslots) - 1u) >> u : 0u;   // the last chunk leaves no state
             uint4 bq0, bq1;                            // this row's 16 columns of B^T, shared by every level that collects in this chunk
 
-            float oacc[16];
+            F2 oacc[8];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) oacc[j] = 0.f;
+            for (int j = 0; j < 8; ++j) oacc[j].v = 0ull;
 
-            for (int p = 0; p < npairs; ++p) {
+#pragma unroll
+            for (int p = 0; p < UNP; ++p) {
+                if (p >= npairs) continue;
                 named_sync(UNB_PAIR + p);              // pair's MMA complete
                 tc_fence_after();
                 const uint32_t lockstep = *sdead;      // non-zero: a wait ran out somewhere, nobody runs ahead of anybody from here on
@@ -278,92 +350,59 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
                     bq0 = *reinterpret_cast<const uint4*>(sBt + v * 128 + (((2 * part) ^ (v & 7)) << 4));
                     bq1 = *reinterpret_cast<const uint4*>(sBt + v * 128 + (((2 * part + 1) ^ (v & 7)) << 4));
                 }
-                const int s = 2 * p + u;
-                const bool active = s < nslots;
-                const bool do_read = (read_mask >> s) & 1u, clear = (clear_mask >> s) & 1u, add_b = !((n >> s) & 1) && s < bl;
-                const int lam_row = (int)((lam_pack >> (5 * p)) & 31u);
-                const uint32_t tcol = tlane + (uint32_t)(tm_d + bufi * 128);
-                bufi = bufi + 1 == nbuf ? 0 : bufi + 1;
+                const uint32_t tcol = tpart + buf;
+                buf = buf == (uint32_t)(nbuf - 1) * 128u ? 0u : buf + 128u;
                 // state path first: the next chunk's MMA of this pair waits for it
-                if (active && i + 1 < nsteps) {
-                    float x[16];
-                    if (clear) {
+                if ((step_mask >> (2 * p)) & 1u) {
+                    uint32_t w[8];
+                    if ((clear_mask >> (2 * p)) & 1u) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) x[j] = 0.f;
+                        for (int c = 0; c < 8; ++c) w[c] = 0u;
                     } else {
-                        tmem_ld16(x, tcol + 16 * part);
-                        if (add_b) {
+                        float x[16];
+                        tmem_ld16(x, tcol);
+                        if ((add_mask >> (2 * p)) & 1u) {
                             const uint32_t bw[8] = {bq0.x, bq0.y, bq0.z, bq0.w, bq1.x, bq1.y, bq1.z, bq1.w};
 #pragma unroll
                             for (int c = 0; c < 8; ++c) {
                                 const float2 f = unpack_bf16x2(bw[c]);
-                                x[2 * c] += f.x; x[2 * c + 1] += f.y;
+                                f2_get(add2(f2(x[2 * c], x[2 * c + 1]), f2(f.x, f.y)), x[2 * c], x[2 * c + 1]);
                             }
                         }
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) w[c] = pack_bf16x2(x[2 * c], x[2 * c + 1]);
                     }
-                    tmem_st_bf16x16(tlane + TM_A + 32 * p + 8 * part, x);
+                    tmem_st8(tlane + TM_A + 32 * p + 8 * part, w);
                 }
                 // read path: lambda-weighted contribution of this level to 16 tokens
-                if (do_read) {
+                if ((read_mask >> (2 * p)) & 1u) {
                     float y[16];
-                    tmem_ld16(y, tcol + 64 + 16 * part);
-                    const float4* lr = reinterpret_cast<const float4*>(sLam + lam_row * CHUNK + 16 * part);
+                    tmem_ld16(y, tcol + 64);
+                    const float4* lr = reinterpret_cast<const float4*>(sLam + ((lam_pack >> (5 * p)) & 31u) * CHUNK);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float4 l4 = lr[j];
-                        oacc[4 * j] += l4.x * y[4 * j]; oacc[4 * j + 1] += l4.y * y[4 * j + 1];
-                        oacc[4 * j + 2] += l4.z * y[4 * j + 2]; oacc[4 * j + 3] += l4.w * y[4 * j + 3];
+                        oacc[2 * j] = fma2(f2(l4.x, l4.y), f2(y[4 * j], y[4 * j + 1]), oacc[2 * j]);
+                        oacc[2 * j + 1] = fma2(f2(l4.z, l4.w), f2(y[4 * j + 2], y[4 * j + 3]), oacc[2 * j + 1]);
                     }
                 }
                 tc_fence_before();
                 // operand rewritten, accumulator read: the control warp may go on
                 if (lockstep) named_sync(UNB_DFREE + p); else named_arrive(UNB_DFREE + p);
             }
-            // output: sum the two rows (levels) of the pairs through shared memory, add O_local, store.
-            // Tokens 16 wg .. 16 wg + 15 of the tile are written and read by warpgroup wg alone, so the barrier is the
-            // warpgroup's own.  The buffer alternates with the chunk: a warp that runs ahead writes the other buffer, and
-            // it cannot get two chunks ahead of a warp of its group that is still reading without passing that barrier.
+            // the output tile, [slot of the pair][token][v], goes to the output warps; its buffer was last read two chunks ago
             float* sOTc = sOT + (i & 1) * (2 * 64 * 64);
+            if (i >= 2) out_sync(UNB_OFREE + (i & 1));
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sOTc[(u * 64 + 16 * part + j) * 64 + v] = oacc[j];
-            switch (wg) {
-                case 0: asm volatile("bar.sync 1, 128;\n" ::: "memory"); break;
-                case 1: asm volatile("bar.sync 2, 128;\n" ::: "memory"); break;
-                case 2: asm volatile("bar.sync 3, 128;\n" ::: "memory"); break;
-                default: asm volatile("bar.sync 4, 128;\n" ::: "memory"); break;
+            for (int j = 0; j < 8; ++j) {
+                float lo, hi;
+                f2_get(oacc[j], lo, hi);
+                sOTc[(u * 64 + 16 * part + 2 * j) * 64 + v] = lo;
+                sOTc[(u * 64 + 16 * part + 2 * j + 1) * 64 + v] = hi;
             }
-            auto emit = [&](auto scat) {
-                // thread = (token, 4 + 4 output columns: 4c.. and 32 + 4c..): the eight lanes of a token read 128
-                // contiguous bytes of the tile per load, which is what keeps the 16-byte loads free of bank conflicts
-                const int tok = tid >> 3, col = (tid & 7) * 4;
-                const int64_t t_out = tok0 + (int64_t)i * CHUNK + tok;
-                const int64_t orow = t_out < tok_end ? out_row<decltype(scat)::value>(a, t_out) : -1;
-                if (orow >= 0) {
-                    const size_t idx = ((size_t)orow * H + h) * UVD + col;
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const float4 p0 = *reinterpret_cast<const float4*>(sOTc + (0 * 64 + tok) * 64 + col + 32 * q);
-                        const float4 q0 = *reinterpret_cast<const float4*>(sOTc + (1 * 64 + tok) * 64 + col + 32 * q);
-                        const uint2 ol = *reinterpret_cast<const uint2*>(sOl + UR::TV::off(tok, col + 32 * q));      // 4 bf16 of O_local
-                        const float2 oa = unpack_bf16x2(ol.x), ob = unpack_bf16x2(ol.y);
-                        const float r0 = p0.x + q0.x + oa.x, r1 = p0.y + q0.y + oa.y, r2 = p0.z + q0.z + ob.x, r3 = p0.w + q0.w + ob.y;
-                        if (a.qkv_dt == LAMPA_F32) {
-                            *reinterpret_cast<float4*>((float*)a.o + idx + 32 * q) = make_float4(r0, r1, r2, r3);
-                        } else {
-                            uint2 w;
-                            if (a.qkv_dt == LAMPA_BF16) { w.x = pack_bf16x2(r0, r1); w.y = pack_bf16x2(r2, r3); }
-                            else {
-                                const __half2 ha = __floats2half2_rn(r0, r1), hb = __floats2half2_rn(r2, r3);
-                                w.x = *reinterpret_cast<const uint32_t*>(&ha); w.y = *reinterpret_cast<const uint32_t*>(&hb);
-                            }
-                            *reinterpret_cast<uint2*>((uint16_t*)a.o + idx + 32 * q) = w;
-                        }
-                    }
-                }
-            };
-            if (a.out_perm_rows > 0) emit(ScatterOn{}); else emit(ScatterOff{});
+            out_arrive(UNB_OFULL + (i & 1));
             __syncwarp();
-            if (lane == 0) mbar_arrive(sfree + (i % UNST));   // B^T, lambda and O_local of this stage have been read
+            if (lane == 0) mbar_arrive(sfree + (i % UNST));   // B^T and lambda of this stage have been read
         }
     }
     tc_fence_before();
@@ -391,7 +430,7 @@ constexpr int PSM_STAGE = PSM_OT + 2 * 2 * 64 * 64 * 4;
 constexpr int PTM_A = 0, PTM_D = 64;         // tensor-memory columns (256 allocated)
 constexpr uint32_t PMMA_IDESC = umma_idesc(64, 128);
 
-__global__ void __launch_bounds__(UTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs a) {
+__global__ void __launch_bounds__(PTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM_BAR);      // records landed            (tx count)
     uint64_t* sfree = full + PNST;                                      // stage consumed            (16 warps)
@@ -629,7 +668,7 @@ int launch_out_plain_umma(const GdnArgs& a, cudaStream_t st) {
     if (cudaFuncSetAttribute(gdn_out_plain_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
     ProfScope prof("gdn_out_plain_umma", st);
-    gdn_out_plain_umma_kernel<<<dim3((unsigned)a.nb_max * ((a.H + 1) / 2)), UTHREADS, smem, st>>>(a);
+    gdn_out_plain_umma_kernel<<<dim3((unsigned)a.nb_max * ((a.H + 1) / 2)), PTHREADS, smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
