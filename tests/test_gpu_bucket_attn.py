@@ -211,3 +211,30 @@ def test_argument_errors(lb):
     big = torch.zeros(1, 1, 256, 8, device="cuda")
     with pytest.raises(lb.LampaError):
         lb.qkv_res(big, big, big)                                  # bucket of 256 > 128
+
+
+@pytest.mark.parametrize("N,block,H,C,dq,dv", [(66, 33, 1, 2, 32, 32), (128, 64, 2, 1, 1, 1), (130, 65, 1, 1, 16, 24),
+                                               (240, 80, 1, 2, 17, 25), (254, 127, 1, 1, 31, 8), (256, 128, 2, 1, 32, 9)])
+def test_tensor_core_tile_edges(lb, N, block, H, C, dq, dv):
+    """Bucket sizes and row widths around the 16-row, 16-feature and 8-column tiles of the tensor-core kernel."""
+    test_random_cases_against_checker(lb, N, block, H, C, dq, dv)
+
+
+@pytest.mark.parametrize("raw,block,heads,rounds,d,cd", [(128, 64, 2, 1, 23, 6), (1, 33, 1, 2, 8, 3), (301, 100, 3, 2, 26, 6),
+                                                         (205, 50, 2, 2, 33, 4)])
+def test_attention_core_sizes(lb, raw, block, heads, rounds, d, cd):
+    """The one-call layer against the composed one: odd widths, one hit, no padding rows, rows wider than a fragment."""
+    gen = torch.Generator().manual_seed(raw)
+    coords_raw = torch.randn(raw, cd, generator=gen)
+    w = torch.randn(heads, d, cd - 1, 5, generator=gen) * 0.3 - 0.8
+    torch.manual_seed(5)
+    regions = lb.get_regions(40, rounds, heads)
+    e2lsh = lb.E2LSH(n_hashes=rounds, n_heads=heads, dim=d + cd).cuda()
+    inp = lb.region_inputs(coords_raw.cuda(), regions, block)
+    query, key, value = (lb.pad_to_multiple(torch.randn(raw, heads, d, generator=gen) * 0.6, block, dims=0).cuda()
+                         for _ in range(3))
+    out = lb.hept_attention_core(e2lsh, query, key, value, w.cuda(), inp["coords"], inp["regions_h"], inp["ranks"], raw, block)
+    q_hat, k_hat, v = lb.prep_qk(query, key, w.cuda(), inp["coords"], value=value, raw_size=raw, head_major=True)
+    q_pos, k_pos = lb.hept_positions(e2lsh, q_hat, k_hat, inp["regions_h"], inp["ranks"], raw)
+    ref, _, _ = oracle.hept_bucket_attention(to_np(q_hat), to_np(k_hat), to_np(v), to_np(q_pos), to_np(k_pos), block)
+    _close(to_np(out)[:, :raw], ref[:, :raw], 5e-5, "attention core")

@@ -436,3 +436,25 @@ def test_output_scatter_equals_a_separate_row_scatter(lb, K, V, force_mma, monke
     keep = torch.ones(n, dtype=torch.bool, device="cuda")
     keep[5] = False
     assert torch.equal(out[0, perm[keep]], want[0, perm[keep]])
+
+
+@pytest.mark.parametrize("K,V,H,lens", [(64, 64, 3, (16384, 16385)), (64, 64, 2, (32769, 63)), (32, 32, 3, (16385, 65, 512)),
+                                        (16, 32, 2, (32769, 1))])
+def test_block_length_edges(lb, K, V, H, lens):
+    """Sequences at the lengths where the chunks per block change (256 and 512 chunks), packed together and with an odd
+    number of heads, through both rules; the hierarchical output also scattered."""
+    from lampa_b200 import synth
+    cu = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    T = int(cu[-1])
+    inp = synth.gdn_inputs(77 + T, T, H, K, V, L=lb.num_levels_required(max(lens)), g_shift=-5.0)
+    d = _cuda(inp)
+    cud = torch.from_numpy(cu).cuda()
+    o, _ = lb.chunk_gated_delta_rule(d["q"], d["k"], d["v"], d["g"], d["beta"], cu_seqlens=cud,
+                                     use_qk_l2norm_in_kernel=True)
+    assert_close_bf16(to_np(o[0]), _plain_ref(inp, cu=cu)[0], "o plain")
+    args = (d["q"], d["k"], d["v"], d["g"], d["lam"], d["beta"])
+    o, _ = lb.chunk_h_gated_delta_rule(*args, cu_seqlens=cud, use_qk_l2norm_in_kernel=True)
+    assert_close_bf16(to_np(o[0]), _hier_ref(inp, cu=cu), "o hier")
+    perm = torch.randperm(T, generator=torch.Generator().manual_seed(1)).cuda()
+    os_, _ = lb.chunk_h_gated_delta_rule(*args, cu_seqlens=cud, use_qk_l2norm_in_kernel=True, out_perm=perm)
+    assert torch.equal(os_[0][perm], o[0])

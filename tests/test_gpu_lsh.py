@@ -147,3 +147,14 @@ def test_ordering_layer_sizes(lb, B, n, C, D, nh):
     for b in range(B):
         np.testing.assert_array_equal(to_np(idx)[b], oracle.lsh_ordering(coords[b], alpha))
     assert torch.equal(ordered.cpu(), points[torch.arange(B)[:, None], idx.cpu()])
+
+
+@pytest.mark.parametrize("n", [8193, 16384, 32769, 65537, 98304, 98305, 200001])
+def test_sort_tile_edges(lb, n):
+    """One segment around the sizes where a CTA's keys per thread, and then its number of tiles, change; a short
+    segment beside it."""
+    rng = np.random.default_rng(n)
+    k = rng.integers(-2**31, 2**31 - 1, n + 77, dtype=np.int64).astype(np.int32)
+    seg = np.array([0, n, n + 77], np.int64)
+    got = to_np(lb.segmented_sort(_dev(torch.from_numpy(k)), seg_offsets=torch.from_numpy(seg)))
+    np.testing.assert_array_equal(got, oracle.segsort(k, seg))

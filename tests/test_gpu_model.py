@@ -89,3 +89,17 @@ def test_event_shards_reproduce_the_packed_forward(lb):
         assert rl <= 1e-3, (owned, mx, rl)
     with pytest.raises(ValueError):
         md.check_event_sizes([70000])
+
+
+@pytest.mark.parametrize("heads,head_dim", [(4, 32), (2, 64)])
+def test_fused_block_tile_edges(lb, heads, head_dim):
+    """Events that start and end inside, on and one past the fused kernels' row tiles; both head shapes they take."""
+    from lampa_b200.model import LSHGatedDelta
+    lengths = [111, 1, 113, 0, 128, 3, 224, 129]
+    hits, cu = _events(lengths, 31)
+    torch.manual_seed(3)
+    m = LSHGatedDelta(max_hits_per_event=1024, num_heads=heads, head_dim=head_dim, n_layers=2)
+    ref = model_oracle.forward(m, hits, cu)
+    out = m.to("cuda:0")(hits.to("cuda:0"), cu.to("cuda:0"))
+    lb.check_status()
+    assert_close_bf16(to_np(out), ref.numpy(), "model, events around the row tiles", max_abs_factor=4.0)
