@@ -18,11 +18,12 @@
 // value columns x a share of the keys).  The CTA has as many warps as finish the bucket's tiles in
 // whole rounds (7 for buckets of 100); three CTAs per SM at the layer's usual sizes, so that one
 // CTA's gather overlaps the others' arithmetic.  Arithmetic is fp32 FMA: the exponent is a
-// difference of large terms, which tensor-core input types cannot carry.
+// difference of large terms, which a single tensor-core operand type cannot carry.
 // Measured (60 000 hits, 3 rounds x 8 heads, buckets of 100, 30 + 24 features): the gather is what
 // bounds the kernel - with 4-byte pieces the copy instructions alone took 17 k of a CTA's 52 k
 // cycles (in-kernel counters), with 16-byte pieces and three CTAs per SM the kernel went from
-// 1.40 ms to 0.97 ms.
+// 1.40 ms to 0.97 ms.  Rows of at most 32 features in buckets of more than 32 take the tensor-core kernel
+// further down (0.47 ms).
 //
 // HBM traffic per (round, head, hit): the q, k, v rows once and the so row + denom once.
 #include "common.cuh"
@@ -274,7 +275,9 @@ __global__ void __launch_bounds__(BA_MAX_WARPS * 32, BA_QROWS == 4 ? 3 : 2) buck
 // Warp = 16 query rows x all keys.  Keys and values are gathered, split once and kept as bf16 tiles in
 // shared memory; queries go from global memory straight into operand fragments, and the weights p from
 // their accumulators into the operand fragments of p V (the two layouts coincide), so that neither
-// touches shared memory.  Measured at the sizes above: 0.97 ms -> see bucket_attn's numbers in the table.
+// touches shared memory.  60 000 hits, 3 rounds x 8 heads, buckets of 100, 30 + 24 features: 0.97 ms -> 0.47 ms.  Buckets of
+// at most 32 hits stay with the FMA kernel (two warps' worth of 16-row tiles), and so do wider rows: their fragments in
+// three pieces do not fit the registers and the kernel is slower than FMA there.
 // -------------------------------------------------------------------------------------------------
 struct Split3 { uint32_t h, m, l; };
 __device__ __forceinline__ Split3 split3(float x, float y) {
