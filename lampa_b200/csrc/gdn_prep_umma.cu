@@ -98,6 +98,9 @@ template <> __device__ __forceinline__ void tmem_st_n<8>(uint32_t taddr, const u
 __device__ __forceinline__ uint64_t desc_adv(uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); }
 
 // NC = columns of an accumulator row per thread: 32 (8 warps) or 16 (16 warps, half the registers).
+// Bound by barrier-separated phases that two CTAs per SM only partly fill, and inside a phase by the shared-memory pipe, a third of
+// whose cycles were bank conflicts: the row staging and the Awb conversion now meet none (T = 65,536, 8 heads: 212 -> 199 us).
+// A persistent form (static units, next tiles fetched a unit ahead) hides the loads but runs 229 us: the units of a slow SM queue up.
 template <bool HIER, int NC>
 __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, const __grid_constant__ CUtensorMap tq,
                                                                      const __grid_constant__ CUtensorMap tk,
@@ -192,7 +195,8 @@ __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, 
     uint32_t w[NC / 2];
     {
         // thread = (token r, head sub, part of the head's row)
-        const int r = tid / (2 * PARTS), sub = (tid / PARTS) & 1, part = tid & (PARTS - 1);
+        // (a quarter-warp's 16-byte accesses lie in rows r, r + 1 of one tile: the swizzle puts them in different banks)
+        const int sub = tid / (PT / 2), r = (tid % (PT / 2)) / PARTS, part = tid & (PARTS - 1);
         const int h = 2 * pair + sub;
         const bool valid = h < H && r < len;
         float gv = 0.f, bv = 0.f;
@@ -324,24 +328,43 @@ __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, 
     // ---- the inverse: warps 0..7 = (head, 16-row block) ---------------------------------------------
     tril_inverse_64<PA>(reinterpret_cast<float*>(smem + S_X) + ((warp >> 2) & 1) * CHUNK * PA, warp & 3, lane, warp < 8);
     stage_tick(a, cta, 4);
-    {   // Awb = X diag(beta) and Awb diag(e^{Gl-G}) as bf16 tiles over the front of the fp32 tiles
-        const int sb = tid / (PT / 2), r = (tid % (PT / 2)) / PARTS, part = tid & (PARTS - 1);
-        const float* sA = reinterpret_cast<const float*>(smem + S_X) + sb * CHUNK * PA + r * PA + part * NC;
-        uint32_t ws[NC / 2];
+    {   // Awb = X diag(beta) and Awb diag(e^{Gl-G}) as bf16 tiles over the front of the fp32 tiles.
+        // thread = (head, 8 columns, RPT rows): the column factors are read once per thread, and the two halves of a warp's
+        // column groups start at different 16 bytes, so that a quarter-warp's loads meet no bank twice
+        constexpr int RPT = 2 * CHUNK * 8 / PT;                        // rows per thread
+        const int c8 = tid & 7, rr = (tid >> 3) & (CHUNK / RPT - 1), sb = tid >> (RPT == 2 ? 8 : 7);
+        const int q0 = (c8 >> 2) & 1;
+        const float* sA = reinterpret_cast<const float*>(smem + S_X) + sb * CHUNK * PA + 8 * c8;
+        float4 b[2], e[2];
 #pragma unroll
-        for (int q = 0; q < NC / 4; ++q) {
-            const float4 v = *reinterpret_cast<const float4*>(sA + 4 * q);
-            const float4 b = *reinterpret_cast<const float4*>(sBeta(sb) + part * NC + 4 * q);
-            const float4 e = *reinterpret_cast<const float4*>(sEGl(sb) + part * NC + 4 * q);
-            const float y0 = v.x * b.x, y1 = v.y * b.y, y2 = v.z * b.z, y3 = v.w * b.w;
-            w[2 * q] = pack_bf16x2(y0, y1);
-            w[2 * q + 1] = pack_bf16x2(y2, y3);
-            ws[2 * q] = pack_bf16x2(y0 * e.x, y1 * e.y);
-            ws[2 * q + 1] = pack_bf16x2(y2 * e.z, y3 * e.w);
+        for (int q = 0; q < 2; ++q) {
+            b[q] = *reinterpret_cast<const float4*>(sBeta(sb) + 8 * c8 + 4 * (q ^ q0));
+            e[q] = *reinterpret_cast<const float4*>(sEGl(sb) + 8 * c8 + 4 * (q ^ q0));
+        }
+        uint4 wa[RPT], ws[RPT];
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+            const int r = rr + k * (CHUNK / RPT);
+            uint2 h[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)}, hs[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+            if (c8 <= (r >> 3)) {                                      // nothing above the diagonal
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 v = *reinterpret_cast<const float4*>(sA + r * PA + 4 * (q ^ q0));
+                    const float y0 = v.x * b[q].x, y1 = v.y * b[q].y, y2 = v.z * b[q].z, y3 = v.w * b[q].w;
+                    h[q] = make_uint2(pack_bf16x2(y0, y1), pack_bf16x2(y2, y3));
+                    hs[q] = make_uint2(pack_bf16x2(y0 * e[q].x, y1 * e[q].y), pack_bf16x2(y2 * e[q].z, y3 * e[q].w));
+                }
+            }
+            wa[k] = q0 ? make_uint4(h[1].x, h[1].y, h[0].x, h[0].y) : make_uint4(h[0].x, h[0].y, h[1].x, h[1].y);
+            ws[k] = q0 ? make_uint4(hs[1].x, hs[1].y, hs[0].x, hs[0].y) : make_uint4(hs[0].x, hs[0].y, hs[1].x, hs[1].y);
         }
         __syncthreads();
-        store_cols_swz<NC>(smem + S_X + sb * TILE, r, part * NCH, w);
-        store_cols_swz<NC>(smem + S_X + 2 * TILE + sb * TILE, r, part * NCH, ws);
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+            const int r = rr + k * (CHUNK / RPT), off = r * 128 + ((c8 ^ (r & 7)) << 4);
+            *reinterpret_cast<uint4*>(smem + S_X + sb * TILE + off) = wa[k];
+            *reinterpret_cast<uint4*>(smem + S_X + 2 * TILE + sb * TILE + off) = ws[k];
+        }
     }
     fence_async_smem();
     __syncthreads();
