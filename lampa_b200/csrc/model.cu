@@ -11,7 +11,7 @@
 //
 // As separate library calls a block moved each row about 14 KB through HBM (projections, convolutions, gates, norms,
 // hidden layer, GELU, three residual passes): 5.3 ms per block for 2.05 M rows.  Here a row costs 1.4 KB in `project`
-// and 1.8 KB in `update`: 1.67 + 2.0 ms.  Both run two CTAs per SM: a CTA alternates between tensor-core products and epilogues that
+// and 1.8 KB in `update`: 1.63 + 2.0 ms.  Both run two CTAs per SM: a CTA alternates between tensor-core products and epilogues that
 // cannot overlap inside one tile, and the other CTA fills the gaps.  Weights stream from L2 through a ring of 16 KB
 // stages (they do not fit beside the tiles at two CTAs per SM).
 #include "act.cuh"
@@ -323,20 +323,18 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
         const float sp_scale = is_a ? -__expf(__ldg(a.A_log + ch - PJ_ROW_A)) : 1.f, sp_add = is_a ? __ldg(a.dt_bias + ch - PJ_ROW_A) : 0.f;
         const float sp_mul = is_l ? __ldg(a.Lw + ch) : 1.f;
 
-        for (int t = 0; t < mine; ++t) {
-            const int64_t tile = blockIdx.x + (int64_t)t * gridDim.x, j0 = tile * PJ_OUT;
-            const int nv = (int)min((int64_t)PJ_OUT, a.n - j0);
-            // ---- the tile's rows of hs, in LSH order (the previous tile's products have all been waited for) ----
-            if (warp < 4) {
-                const int64_t j = j0 - PJ_HALO + tid;            // operand row tid
-                bool first = false;
-                int64_t r = -1;
-                if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.status, &first);
-                srow[tid] = r;
-                const uint32_t bits = __ballot_sync(0xffffffffu, first);
-                if (lane == 0) sstart[warp] = bits;
-            }
-            epi_sync();
+        // the rows of hs that tile t takes, in LSH order: found under the gate block of the tile before, fetched under its
+        // last epilogue (both are chains of dependent loads); 2.05 M rows: 1,667 -> 1,629 us
+        auto find_rows = [&](int t) {                            // warps 0..3
+            const int64_t j = (blockIdx.x + (int64_t)t * gridDim.x) * PJ_OUT - PJ_HALO + tid;            // operand row tid
+            bool first = false;
+            int64_t r = -1;
+            if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.status, &first);
+            srow[tid] = r;
+            const uint32_t bits = __ballot_sync(0xffffffffu, first);
+            if (lane == 0) sstart[warp] = bits;
+        };
+        auto fetch_rows = [&] {
             for (int i = tid; i < (PJ_ROWS - 8) * 16; i += METHR) {
                 const int row = 8 + (i >> 4), c = i & 15;
                 const int64_t r = srow[row];
@@ -344,7 +342,17 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 if (r >= 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(smem_u32(dst)), "l"(a.hs + r * MD + 8 * c) : "memory");
                 else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
             }
-            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        if (mine > 0) {
+            if (warp < 4) find_rows(0);
+            epi_sync();
+            fetch_rows();
+        }
+        for (int t = 0; t < mine; ++t) {
+            const int64_t tile = blockIdx.x + (int64_t)t * gridDim.x, j0 = tile * PJ_OUT;
+            const int nv = (int)min((int64_t)PJ_OUT, a.n - j0);
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(bready);
@@ -355,9 +363,9 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                 const int q = t * PJ_BLOCKS + m, buf = q & 1;
                 uint2 taps = make_uint2(0u, 0u);                 // this channel's four taps
                 if (m < 3) taps = __ldg(reinterpret_cast<const uint2*>(m == 0 ? a.conv[0] : m == 1 ? a.conv[1] : a.conv[2]) + ch);
-                // products complete, and the previous results have left the staging tile
-                epi_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget, [&] { if (tid == 0) bulk_wait_read(); });
+                epi_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget, [] {});      // products complete
                 tc_fence_after();
+                if (m == PJ_BLOCKS - 1 && t + 1 < mine) fetch_rows();        // the tile's last products: its operand is free
                 float x[32];                                     // X(i) = position i - 4
                 tmem_ld32(x, tl + 128 * buf);
                 tc_fence_before();
@@ -399,6 +407,9 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                     for (int i = 0; i < PJ_PART; ++i)
                         if (PJ_PART * part + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(x[4 + i] + sp_add) : sigmoid_fast(x[4 + i]);
                 }
+                if (m == 3 && t + 1 < mine && warp < 4) find_rows(t + 1);
+                if (tid == 0) bulk_wait_read();                  // the previous results have left the staging tile
+                epi_sync();
                 uint16_t* st = reinterpret_cast<uint16_t*>(sST) + ch;
                 if (m < 4) {
                     st += PJ_PART * part * MD;
