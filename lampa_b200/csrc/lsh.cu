@@ -310,6 +310,10 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                     const uint32_t ku = skey[lp], ki = sidx[lp];
                     const uint32_t d = (ku >> shift) & dmask;
                     const int64_t pos = (int64_t)dbase[d] + (lp - tstart[d]);
+                    // A slice of several tiles reads its keys twice, for the histogram and here.  Segments that overlap
+                    // (offsets that fall: the segment in between reports them) rewrite each other's keys in between, and
+                    // the counts no longer add up: nothing is written outside the segment all the same.
+                    if (pos >= n) continue;
                     if (last) {
                         perm[s0 + pos] = (int64_t)ki;
                     } else {

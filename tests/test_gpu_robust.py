@@ -119,3 +119,26 @@ def test_forward_only_ops_refuse_autograd(lb):
     with torch.no_grad():
         o, _ = lb.chunk_gated_delta_rule(q, q, q, g, g)
     assert not o.requires_grad
+
+
+def test_sort_of_overlapping_segments_stays_inside_them(lb):
+    """Offsets that fall make two segments of several tiles overlap: their passes rewrite each other's keys, the falling
+    one between them is reported, and nothing is written behind the permutation or the workspace."""
+    import ctypes
+    from lampa_b200 import _lib as L
+    n, pad = 400_000, 300_000
+    rng = np.random.default_rng(9)
+    keys = torch.from_numpy(rng.integers(-2**31, 2**31 - 1, n).astype(np.int32)).cuda()
+    seg = torch.tensor([0, 300_000, 100_000, n], dtype=torch.int64, device="cuda:0")
+    need = ctypes.c_size_t(0)
+    L.check(L.lib().lampa_segsort_workspace_bytes(n, ctypes.byref(need)), "workspace")
+    perm = torch.full((n + pad,), -7, dtype=torch.int64, device="cuda:0")
+    ws = torch.full((need.value + 4 * pad,), 0x5A, dtype=torch.uint8, device="cuda:0")
+    _status(lb)
+    st = L.status_word(torch.device("cuda:0"))
+    for _ in range(20):
+        L.check(L.lib().lampa_segsort_stable(L.ptr(keys), L.LAMPA_KEY_I32, n, L.ptr(seg), 3, None, L.ptr(perm), L.ptr(ws), need.value,
+                                             L.ptr(st), L.stream_ptr(torch.device("cuda:0"))), "lampa_segsort_stable")
+    vals = _status(lb)
+    assert vals[0] == L.ERR_BOUNDS and vals[1] == 12 and vals[2] == 1
+    assert bool((perm[n:] == -7).all()) and bool((ws[need.value:] == 0x5A).all())
