@@ -15,18 +15,34 @@ namespace lampa {
 constexpr int PLAN_THREADS = 256;
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(PlanArgs p) {
     __shared__ int2 wsum[PLAN_THREADS / 32];
+    __shared__ int64_t wtop[PLAN_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t total = (int64_t)p.B * p.T;
     int c0 = 0, b0 = 0;                                     // totals of the sequences before this pass
+    int64_t top0 = 0;                                       // largest offset inside the input before this pass
     if (threadIdx.x == 0) { p.chunk_off[0] = 0; p.block_off[0] = 0; }
     for (int s0 = 0; s0 < p.nseq; s0 += PLAN_THREADS) {
         const int s = s0 + threadIdx.x;
         int c = 0, b = 0;
+        const int64_t t0 = s >= p.nseq ? 0 : p.cu ? p.cu[s] : (int64_t)s * p.T;
+        // A sequence that begins before an earlier offset would take tokens of another one a second time: the chunks of
+        // all sequences together could then outnumber the records of the workspace.
+        int64_t top = t0 <= total ? t0 : 0;                 // (a negative offset is never the largest)
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) top = max(top, __shfl_up_sync(0xffffffffu, top, o));
+        if (lane == 31) wtop[warp] = top;
+        __syncthreads();
+        top = max(top, top0);
+#pragma unroll
+        for (int w = 0; w < PLAN_THREADS / 32; ++w) {
+            if (w < warp) top = max(top, wtop[w]);
+            top0 = max(top0, wtop[w]);
+        }
         if (s < p.nseq) {
-            const int64_t t0 = p.cu ? p.cu[s] : (int64_t)s * p.T;
             const int64_t t1 = p.cu ? p.cu[s + 1] : (int64_t)(s + 1) * p.T;
             p.tok_off[s] = t0;
             int64_t len = t1 - t0;
-            if (len < 0 || t0 < 0 || t1 > (int64_t)p.B * p.T) { set_status(p.status, LAMPA_ERR_BOUNDS, 1, s); len = 0; }
+            if (len < 0 || t0 < 0 || t1 > total || t0 < top) { set_status(p.status, LAMPA_ERR_BOUNDS, 1, s); len = 0; }
             c = (int)((len + CHUNK - 1) / CHUNK);
             if (p.hier && c > 0 && ELL0 + ceil_log2_int(c) > p.L) set_status(p.status, LAMPA_ERR_LEVELS, 1, s);
             b = blocks_of(c);

@@ -142,3 +142,49 @@ def test_sort_of_overlapping_segments_stays_inside_them(lb):
     vals = _status(lb)
     assert vals[0] == L.ERR_BOUNDS and vals[1] == 12 and vals[2] == 1
     assert bool((perm[n:] == -7).all()) and bool((ws[need.value:] == 0x5A).all())
+
+
+@pytest.mark.parametrize("K,hier", [(64, False), (64, True), (32, True)])
+def test_sequences_that_overlap_are_emptied(lb, K, hier):
+    """Offsets that fall and rise again: a sequence that begins before an earlier offset is emptied and reported, since its
+    chunks have no records, and the sequences in order give what they give alone."""
+    from lampa_b200 import _lib as L, synth
+    T, H = 640, 2
+    inp = synth.gdn_inputs(6, T, H, K, K, L=11, g_shift=-3.0)
+    d = {k: v.to("cuda:0") for k, v in inp.items()}
+    old = os.environ.pop("LAMPA_B200_CHECK", None)
+
+    def run(cu):
+        c = torch.tensor(cu, device="cuda:0")
+        if hier:
+            return lb.chunk_h_gated_delta_rule(d["q"], d["k"], d["v"], d["g"], d["lam"], d["beta"], cu_seqlens=c,
+                                               use_qk_l2norm_in_kernel=True)[0], None
+        return lb.chunk_gated_delta_rule(d["q"], d["k"], d["v"], d["g"], d["beta"], cu_seqlens=c, output_final_state=True,
+                                         use_qk_l2norm_in_kernel=True)
+
+    try:
+        _status(lb)
+        want, state = run([0, T])
+        assert _status(lb)[0] == 0
+        for cu in ([0, T, 0, T], [0, T, 64, T, 128, T, 0, T]):
+            got, st = run(cu)
+            vals = _status(lb)
+            assert vals[0] == L.ERR_BOUNDS and vals[1] == 1, vals
+            assert torch.equal(got, want)
+            assert st is None or (torch.equal(st[0], state[0]) and not st[1:].any())
+        # behind an offset that leaves the input, sequences in order are taken as before
+        got, _ = run([0, 256, T + 64, 320, T])
+        want, _ = run([0, 256, 256, 320, T])
+        assert torch.equal(got[:, :256], want[:, :256]) and torch.equal(got[:, 320:], want[:, 320:])
+        assert _status(lb)[0] == L.ERR_BOUNDS
+        # more sequences than the plan takes in one pass
+        cu = list(range(0, 600, 2)) + [T]
+        want, _ = run(cu)
+        assert _status(lb)[0] == 0
+        cu[290] = 10
+        got, _ = run(cu)
+        assert torch.equal(got[:, :578], want[:, :578]) and torch.equal(got[:, 582:], want[:, 582:])
+        assert _status(lb)[0] == L.ERR_BOUNDS
+    finally:
+        if old is not None:
+            os.environ["LAMPA_B200_CHECK"] = old
