@@ -43,18 +43,18 @@ __device__ __forceinline__ void epi_wait(uint64_t* bar, uint32_t parity, bool& d
     epi_sync();
 }
 
-// Row r of the residual stream that position j of an ordered batch stands for (perm is local to j's event); -1 when the
-// permutation leaves the event.
+// Row r of the residual stream of n rows that position j of an ordered batch stands for (perm is local to j's event); -1 when
+// the permutation leaves the event or the event's offsets, which nobody has checked before, leave the rows.
 __device__ __forceinline__ int64_t ordered_row(const int64_t* __restrict__ cu, int nseq, const int64_t* __restrict__ perm,
-                                               int64_t j, int32_t* status, bool* first = nullptr) {
+                                               int64_t j, int64_t n, int32_t* status, bool* first = nullptr) {
     int lo = 0, hi = nseq;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (__ldg(cu + mid) <= j) lo = mid; else hi = mid;
     }
-    const int64_t s0 = __ldg(cu + lo), p = __ldg(perm + j);
+    const int64_t s0 = __ldg(cu + lo), s1 = __ldg(cu + lo + 1), p = __ldg(perm + j);
     if (first) *first = j == s0;
-    if ((uint64_t)p >= (uint64_t)(__ldg(cu + lo + 1) - s0)) {
+    if (p < 0 || p >= s1 - s0 || s0 < 0 || s1 > n) {
         set_status(status, LAMPA_ERR_BOUNDS, 40, (int)j);
         return -1;
     }
@@ -329,7 +329,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             const int64_t j = (blockIdx.x + (int64_t)t * gridDim.x) * PJ_OUT - PJ_HALO + tid;            // operand row tid
             bool first = false;
             int64_t r = -1;
-            if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.status, &first);
+            if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.n, a.status, &first);
             srow[tid] = r;
             const uint32_t bits = __ballot_sync(0xffffffffu, first);
             if (lane == 0) sstart[warp] = bits;
@@ -625,7 +625,7 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
             const int64_t j0 = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * UP_ROWS + UP_WROWS * warp;   // this warp's rows
             const int nr = (int)min((int64_t)UP_WROWS, max((int64_t)0, a.n - j0));
             int64_t myrow = -1;
-            if (lane < nr) myrow = ordered_row(a.cu, a.nseq, a.perm, j0 + lane, a.status);
+            if (lane < nr) myrow = ordered_row(a.cu, a.nseq, a.perm, j0 + lane, a.n, a.status);
             {   // the residual rows are wanted one product later: into L2 now (four lines each)
                 const int64_t pr = __shfl_sync(0xffffffffu, myrow, lane >> 2);
                 if (pr >= 0) asm volatile("prefetch.global.L2 [%0];\n" :: "l"(a.x + pr * MD + 32 * (lane & 3)));

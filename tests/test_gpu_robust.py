@@ -188,3 +188,34 @@ def test_sequences_that_overlap_are_emptied(lb, K, hier):
     finally:
         if old is not None:
             os.environ["LAMPA_B200_CHECK"] = old
+
+
+def _model(lb, n):
+    from lampa_b200 import synth
+    from lampa_b200.model import LSHGatedDelta
+    torch.manual_seed(5)
+    return LSHGatedDelta(max_hits_per_event=4096, n_layers=3).to("cuda:0"), synth.detector_hits(17, n).to("cuda:0")
+
+
+@pytest.mark.parametrize("over", [50, 1 << 40])
+def test_model_rows_of_events_outside_the_input_are_skipped(lb, over):
+    """Device-resident event offsets whose inner entry lies behind or before the rows: no row is followed out of the
+    input, no block adds anything to a skipped row, and the call reports it."""
+    from lampa_b200 import _lib as L
+    n = 700
+    m, hits = _model(lb, n)
+    old = os.environ.pop("LAMPA_B200_CHECK", None)
+    try:
+        _status(lb)
+        with torch.no_grad():
+            x = m.head(m.encoder(hits * m.feature_scale))
+        for cu in ([0, n + over, n], [0, -over, n]):
+            got = m(hits, torch.tensor(cu, device="cuda:0"))
+            assert _status(lb)[0] == L.ERR_BOUNDS
+            # fp32 sums of 24 and 128 terms in another order
+            torch.testing.assert_close(got, x, rtol=1e-5, atol=1e-5)
+        m(hits, torch.tensor([0, n], device="cuda:0"))
+        assert _status(lb)[0] == 0
+    finally:
+        if old is not None:
+            os.environ["LAMPA_B200_CHECK"] = old
