@@ -513,13 +513,16 @@ int lampa_model_encode(const float* hits, const float* scale, const float* weigh
 int lampa_model_project(const lampa_model_mixer* w, const void* hs, const int64_t* perm, const int64_t* cu, int32_t nseq,
                         int64_t n, void* q, void* k, void* v, void* gate, float* g, float* beta, void* lam,
                         int32_t* status, void* stream);
-/* mixer output o and gate (ordered rows) -> residual stream x (hit rows, in place), next block's normed rows hs (hit rows) */
+/* mixer output o and gate (ordered rows) -> residual stream x (hit rows, in place), next block's normed rows hs (hit rows).
+ * In both, the rows of an event whose offsets leave [0, n], or whose permutation leaves the event, are skipped and reported as
+ * LAMPA_ERR_BOUNDS in `status`. */
 int lampa_model_update(const lampa_model_update_w* w, const void* o, const void* gate, float* x, const int64_t* perm,
                        const int64_t* cu, int32_t nseq, int64_t n, void* hs, int32_t* status, void* stream);
 /* out = x W^T + b [n][24] */
 int lampa_model_head(const float* x, const float* weight, const float* bias, int64_t n, int32_t d_model, int32_t out_dim,
                      float* out, void* stream);
-/* segment offsets of `rounds` copies of a packed batch behind one another, int64 [rounds * nseq + 1] */
+/* segment offsets of `rounds` copies of a packed batch behind one another, int64 [rounds * nseq + 1]; an offset outside
+ * [0, n], or below an earlier one, is replaced by the highest one before it, so that the segments never overlap */
 int lampa_repeat_segments(const int64_t* cu, int32_t nseq, int32_t rounds, int64_t n, int64_t* out, void* stream);
 
 #ifdef __cplusplus

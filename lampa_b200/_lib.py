@@ -88,6 +88,7 @@ def lib() -> ctypes.CDLL:
         L.lampa_gate_inputs.argtypes = [vp] * 7 + [i64, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp]
         L.lampa_rmsnorm_gate.argtypes = [vp, vp, vp, i64, i32, i32, i32, ctypes.c_float, i32, vp, vp]
         L.lampa_add_rmsnorm.argtypes = [vp, vp, i32, vp, vp, i32, i64, i32, vp, ctypes.c_float, i32, i32, vp, i32, vp, vp]
+        L.lampa_repeat_segments.argtypes = [vp, i32, i32, i64, vp, vp]
         L.lampa_profile_enable.argtypes = [ctypes.c_int]
         L.lampa_debug_set_poll_budget.argtypes = [ctypes.c_int]
         L.lampa_debug_force_mma_sync.argtypes = [ctypes.c_int]

@@ -221,6 +221,26 @@ inline bool allow_smem(std::atomic<uint64_t>& ready, K kernel, int bytes) {
     return true;
 }
 
+// Largest offset up to and including this thread's, over the threads of the CTA in order and, through `before`, the passes
+// before; offsets that leave [0, total] do not count.  A packed sequence in order begins at this offset.  All threads call it
+// (`wtop`: one word per warp, free again behind the caller's next barrier).
+template <int THREADS>
+__device__ __forceinline__ int64_t highest_offset(int64_t t, int64_t total, int64_t& before, int64_t* wtop) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t top = t <= total ? t : 0;                       // (a negative one is never the largest)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) top = max(top, __shfl_up_sync(0xffffffffu, top, o));
+    if (lane == 31) wtop[warp] = top;
+    __syncthreads();
+    top = max(top, before);
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) {
+        if (w < warp) top = max(top, wtop[w]);
+        before = max(before, wtop[w]);
+    }
+    return top;
+}
+
 // ---- sequence plan (device ints, built once per call from cu_seqlens) ---------------------------
 struct SeqPlan {
     const int64_t* tok_off;    // [nseq+1] token offsets

@@ -27,17 +27,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(PlanArgs p) {
         const int64_t t0 = s >= p.nseq ? 0 : p.cu ? p.cu[s] : (int64_t)s * p.T;
         // A sequence that begins before an earlier offset would take tokens of another one a second time: the chunks of
         // all sequences together could then outnumber the records of the workspace.
-        int64_t top = t0 <= total ? t0 : 0;                 // (a negative offset is never the largest)
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) top = max(top, __shfl_up_sync(0xffffffffu, top, o));
-        if (lane == 31) wtop[warp] = top;
-        __syncthreads();
-        top = max(top, top0);
-#pragma unroll
-        for (int w = 0; w < PLAN_THREADS / 32; ++w) {
-            if (w < warp) top = max(top, wtop[w]);
-            top0 = max(top0, wtop[w]);
-        }
+        const int64_t top = highest_offset<PLAN_THREADS>(t0, total, top0, wtop);
         if (s < p.nseq) {
             const int64_t t1 = p.cu ? p.cu[s + 1] : (int64_t)(s + 1) * p.T;
             p.tok_off[s] = t0;

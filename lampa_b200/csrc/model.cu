@@ -855,15 +855,25 @@ extern "C" int lampa_model_update(const lampa_model_update_w* w, const void* o, 
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
-// Segment offsets of `rounds` copies of a packed batch behind one another: out[r * nseq + s] = r * n + cu[s], out[rounds * nseq] = rounds * n
-static __global__ void model_segments_kernel(const int64_t* cu, int nseq, int rounds, int64_t n, int64_t* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < rounds * nseq) out[i] = (int64_t)(i / nseq) * n + cu[i % nseq];
-    else if (i == rounds * nseq) out[i] = (int64_t)rounds * n;
+// Segment offsets of `rounds` copies of a packed batch behind one another: out[r * nseq + s] = r * n + cu[s], out[rounds * nseq] = rounds * n.
+// An offset that leaves the batch, or falls, is moved to the highest one before it: the segments never overlap, so a bad event
+// reaches neither into the events beside it nor into another copy's.  One CTA per copy.
+constexpr int SEG_THREADS = 256;
+static __global__ void __launch_bounds__(SEG_THREADS) model_segments_kernel(const int64_t* cu, int nseq, int64_t n, int64_t* out) {
+    __shared__ int64_t wtop[SEG_THREADS / 32];
+    const int r = blockIdx.x;
+    int64_t before = 0;
+    for (int s0 = 0; s0 < nseq; s0 += SEG_THREADS) {
+        const int s = s0 + threadIdx.x;
+        const int64_t top = highest_offset<SEG_THREADS>(s < nseq ? cu[s] : 0, n, before, wtop);
+        if (s < nseq) out[(int64_t)r * nseq + s] = (int64_t)r * n + top;
+        __syncthreads();
+    }
+    if (r == gridDim.x - 1 && threadIdx.x == 0) out[(int64_t)gridDim.x * nseq] = (int64_t)gridDim.x * n;
 }
 
 extern "C" int lampa_repeat_segments(const int64_t* cu, int32_t nseq, int32_t rounds, int64_t n, int64_t* out, void* stream) {
     if (!cu || !out || nseq <= 0 || rounds <= 0) return LAMPA_ERR_ARG;
-    model_segments_kernel<<<(unsigned)((rounds * nseq) / 256 + 1), 256, 0, (cudaStream_t)stream>>>(cu, nseq, rounds, n, out);
+    model_segments_kernel<<<(unsigned)rounds, SEG_THREADS, 0, (cudaStream_t)stream>>>(cu, nseq, n, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }

@@ -180,8 +180,10 @@ class LSHGatedDelta(nn.Module):
         n = hits.shape[0]
         packed = lsh_hash(hits, self.lsh_alpha, self.lsh_beta, self.bucket_width, dim=self.coord_dim,
                           want_ids=False, want_packed=True)["packed"]                      # [rounds, N]
-        offs = (torch.arange(self.rounds, device=hits.device, dtype=torch.int64)[:, None] * n + cu[None, :-1]).reshape(-1)
-        seg = torch.cat([offs, torch.full((1,), self.rounds * n, device=hits.device, dtype=torch.int64)])
+        seg = torch.empty(self.rounds * (cu.numel() - 1) + 1, device=hits.device, dtype=torch.int64)
+        cu = cu.to(device=hits.device, dtype=torch.int64).contiguous()
+        L.check(L.lib().lampa_repeat_segments(L.ptr(cu), cu.numel() - 1, self.rounds, n, L.ptr(seg), L.stream_ptr(hits.device)),
+                "lampa_repeat_segments")
         return segmented_sort(packed, seg_offsets=seg).view(self.rounds, n)
 
     def _native_params(self):

@@ -219,3 +219,26 @@ def test_model_rows_of_events_outside_the_input_are_skipped(lb, over):
     finally:
         if old is not None:
             os.environ["LAMPA_B200_CHECK"] = old
+
+
+@pytest.mark.parametrize("bad", [[0, 300, 1200, 700], [-250, 0, 300, 700], [0, 300, -1, 700]])
+def test_model_events_beside_a_bad_one_are_unchanged(lb, bad):
+    """The orders of all rounds are one segmented sort: an offset that leaves the batch reaches into no other segment, and the
+    first event's 300 rows come out as they do beside a good one."""
+    from lampa_b200 import _lib as L
+    n = 700
+    m, hits = _model(lb, n)
+    old = os.environ.pop("LAMPA_B200_CHECK", None)
+    try:
+        _status(lb)
+        good = torch.tensor([0, 300, n], device="cuda:0")
+        want, order = m(hits, good), m.orderings(hits, good)
+        assert _status(lb)[0] == 0
+        cu = torch.tensor(bad, device="cuda:0")
+        for _ in range(10):
+            got, perm = m(hits, cu), m.orderings(hits, cu)
+            assert torch.equal(perm[:, :300], order[:, :300]) and torch.equal(got[:300], want[:300])
+        assert _status(lb)[0] == L.ERR_BOUNDS
+    finally:
+        if old is not None:
+            os.environ["LAMPA_B200_CHECK"] = old
