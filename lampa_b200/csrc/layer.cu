@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(128) short_conv_fwd_kernel(ConvArgs a) {
         bos = (t_begin / a.T) * a.T; eos = bos + a.T;
     }
     // window: win[i] = x[t - (W-1) + i]; slots 0 .. W-2 hold the history, slot W-1 the current token
+    // (device-resident offsets may be anything: a row outside the input reads as zero)
     float win[MW][NV];
 #pragma unroll
     for (int i = 0; i < MW; ++i)
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(128) short_conv_fwd_kernel(ConvArgs a) {
     for (int i = 0; i < MW - 1; ++i)
         if (i < W - 1) {
             const int64_t tt = t_begin - (W - 1) + i;
-            if (tt >= bos) unpack4(ldg4<DT>(a.x, (size_t)tt * a.D + d0), win[i], DT);
+            if (tt >= 0 && tt >= bos) unpack4(ldg4<DT>(a.x, (size_t)tt * a.D + d0), win[i], DT);
         }
     // all rows of the run are requested before the first one is used
     RawT raw[CONV_TOKENS];
@@ -228,9 +229,9 @@ __global__ void __launch_bounds__(128) short_conv_fwd_kernel(ConvArgs a) {
 }
 
 // Convolution state after a prefill: cache[n, d, w] = x[eos_n - W + w, d]; slots that would lie
-// before the sequence start are zeroed (zero_fill) or left as they are.
+// before the sequence start, or outside the n_tok rows of the input, are zeroed (zero_fill) or left as they are.
 __global__ void __launch_bounds__(256)
-short_conv_state_kernel(const void* x, const int64_t* cu, int64_t T, int nseq_packed, int N, int D, int W,
+short_conv_state_kernel(const void* x, const int64_t* cu, int64_t T, int64_t n_tok, int nseq_packed, int N, int D, int W,
                         int dt, int zero_fill, void* cache) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)N * D * W) return;
@@ -240,7 +241,7 @@ short_conv_state_kernel(const void* x, const int64_t* cu, int64_t T, int nseq_pa
     const int64_t bos = nseq_packed > 0 ? cu[n] : (int64_t)n * T;
     const int64_t eos = nseq_packed > 0 ? cu[n + 1] : bos + T;
     const int64_t t = eos - W + w;
-    if (t >= bos) store_from_float(cache, idx, load_as_float(x, (size_t)t * D + d, dt), dt);
+    if (t >= bos && t >= 0 && t < n_tok) store_from_float(cache, idx, load_as_float(x, (size_t)t * D + d, dt), dt);
     else if (zero_fill) store_from_float(cache, idx, 0.f, dt);
 }
 
@@ -584,7 +585,7 @@ extern "C" int lampa_short_conv_fwd(const void* x, const void* weight, const voi
     if (final_state) {
         const int N = nseq > 0 ? nseq : (int)B;
         const int64_t tot = (int64_t)N * D * W;
-        short_conv_state_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(x, cu_seqlens, T, nseq, N, D, W, dtype,
+        short_conv_state_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(x, cu_seqlens, T, a.n_tok, nseq, N, D, W, dtype,
                                                                             zero_fill, final_state);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }

@@ -242,3 +242,14 @@ def test_model_events_beside_a_bad_one_are_unchanged(lb, bad):
     finally:
         if old is not None:
             os.environ["LAMPA_B200_CHECK"] = old
+
+
+def test_short_conv_of_sequences_outside_the_input(lb):
+    """Device-resident offsets in front of and behind the rows: taps and final-state slots outside the input are zero."""
+    T, D, W = 100, 32, 4
+    conv = lb.ShortConvolution(D, W, device="cuda:0", dtype=torch.float32)
+    x = torch.randn(1, T, D, device="cuda:0")
+    want, _ = conv(x, cu_seqlens=torch.tensor([0, 40, T], device="cuda:0"))
+    got, state = conv(x, cu_seqlens=torch.tensor([-(1 << 36), 40, 1 << 40], device="cuda:0"), output_final_state=True)
+    assert torch.equal(got, want)                               # all rows have the taps of the sequence they lie in
+    assert torch.equal(state[0], x[0, 40 - W:40].T) and not state[1].any()
