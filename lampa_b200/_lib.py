@@ -10,6 +10,7 @@ import os
 from typing import Dict, Optional
 
 import torch
+from torch.nn.modules import module as _nn_module
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(_HERE, "liblampa_b200.so")
@@ -120,6 +121,14 @@ class _Native:
 
 
 native = _Native()
+
+
+def runs_own_forward(module: torch.nn.Module, cls: type) -> bool:
+    """Whether calling `module` would run `cls.forward` and nothing else: its work may then be done without the call.
+    A subclass, a replaced forward, and hooks of the module or of all modules have to run."""
+    return (type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks
+            and "forward" not in module.__dict__ and not _nn_module._global_forward_hooks
+            and not _nn_module._global_forward_pre_hooks)
 
 
 def check(rc: int, what: str) -> None:

@@ -192,18 +192,18 @@ class LSHGatedDelta(nn.Module):
         params, eps = [], []
         for blk in self.blocks._modules.values():
             at = blk._modules.get("attn")
-            if type(blk) is not LSHGatedDeltaBlock or type(at) is not HGatedDeltaNet or blk.dtype != torch.bfloat16:
+            if type(blk) is not LSHGatedDeltaBlock or "mix" in blk.__dict__ or blk.dtype != torch.bfloat16:
                 return None
-            if not (at.use_gate and at.use_short_conv and at.lambda_mode == "positive") or at._forward_hooks or at._forward_pre_hooks:
+            if not L.runs_own_forward(at, HGatedDeltaNet) or not (at.use_gate and at.use_short_conv and at.lambda_mode == "positive"):
                 return None
             am, ap, bp = at._modules, at._parameters, blk._parameters
             lin = [am[k] for k in ("q_proj", "k_proj", "v_proj", "g_proj", "a_proj", "b_proj", "l_proj", "o_proj")]
             mlp = [blk._modules["mlp_up"], blk._modules["mlp_down"]]
             conv = [am[k] for k in ("q_conv1d", "k_conv1d", "v_conv1d")]
-            for m in lin + mlp + conv + [am["o_norm"]]:
-                if type(m) not in (nn.Linear, ShortConvolution, FusedRMSNormGated) or m._forward_hooks or m._forward_pre_hooks:
-                    return None
-            if any(m._parameters["bias"] is not None for m in lin):
+            if not (all(L.runs_own_forward(m, nn.Linear) for m in lin + mlp) and all(L.runs_own_forward(m, ShortConvolution) for m in conv)
+                    and L.runs_own_forward(am["o_norm"], FusedRMSNormGated)):
+                return None
+            if any(m._parameters["bias"] is not None for m in lin + [am["o_norm"]]):
                 return None
             if any(c.bias is not None or c.activation is None or c.kernel_size[0] != 4 for c in conv) or am["o_norm"].activation == "sigmoid":
                 return None
@@ -218,7 +218,9 @@ class LSHGatedDelta(nn.Module):
     def _native_forward(self, hits: torch.Tensor, cu: torch.Tensor):
         """The whole forward behind one host call, for the widths the fused block kernels are built for (None otherwise)."""
         enc, head = self._modules["encoder"], self._modules["head"]
-        if type(enc) is not nn.Linear or type(head) is not nn.Linear or enc._forward_hooks or head._forward_hooks:
+        if not (L.runs_own_forward(enc, nn.Linear) and L.runs_own_forward(head, nn.Linear)):
+            return None
+        if type(self).orderings is not LSHGatedDelta.orderings or "orderings" in self.__dict__:
             return None
         p = self._native_params()
         if p is None:

@@ -103,3 +103,20 @@ def test_fused_block_tile_edges(lb, heads, head_dim):
     out = m.to("cuda:0")(hits.to("cuda:0"), cu.to("cuda:0"))
     lb.check_status()
     assert_close_bf16(to_np(out), ref.numpy(), "model, events around the row tiles", max_abs_factor=4.0)
+
+
+def test_hooked_submodules_run(lb):
+    """A pre-hook on the encoder and a hook on a block's projection run, and the composed forward agrees with the fused one."""
+    lengths = [300, 65]
+    hits, cu = _events(lengths, 13)
+    hits, cu = hits.to("cuda:0"), cu.to("cuda:0")
+    m = _model(4096).to("cuda:0")
+    fused = m(hits, cu)
+    seen = []
+    handles = [m.encoder.register_forward_pre_hook(lambda mod, a: seen.append("encoder")),
+               m.blocks[1].attn.q_proj.register_forward_hook(lambda mod, a, out: seen.append("q_proj"))]
+    got = m(hits, cu)
+    for h in handles:
+        h.remove()
+    assert seen == ["encoder", "q_proj"]
+    assert_close_bf16(to_np(got), to_np(fused), "composed against fused forward", max_abs_factor=4.0)

@@ -224,3 +224,54 @@ def test_dispatcher_entries_have_shape_functions():
     assert ht.shape == (4, H, K, V)
     o = torch.ops.lampa_b200.hgdn_fwd(q, k, v, g, beta, m(B, T, H, Lv), None, True)
     assert o.shape == (B, T, H, V) and o.dtype == torch.bfloat16
+
+
+def _native_taken(model, monkeypatch):
+    """Whether the model's forward hands this model to the host call (the call itself is replaced)."""
+    from lampa_b200 import _lib
+    taken = object()
+    monkeypatch.setattr(_lib.native, "model_forward", lambda *a: taken, raising=False)
+    return model._native_forward(torch.zeros(4, 24), torch.tensor([0, 4])) is taken
+
+
+def _hooked(kind):
+    return {"forward hook": lambda m: m.register_forward_hook(lambda *a: None),
+            "forward pre-hook": lambda m: m.register_forward_pre_hook(lambda *a: None),
+            "replaced forward": lambda m: setattr(m, "forward", lambda *a, **k: None),
+            "subclass": lambda m: setattr(m, "__class__", type("Sub", (type(m),), {}))}[kind]
+
+
+@pytest.mark.parametrize("kind", ["forward hook", "forward pre-hook", "replaced forward", "subclass"])
+def test_fused_model_leaves_modified_submodules_to_their_own_forward(kind, monkeypatch):
+    from lampa_b200.model import LSHGatedDelta
+    names = ["encoder", "head", "blocks.0.attn", "blocks.1.mlp_up", "blocks.0.mlp_down", "blocks.1.attn.q_proj", "blocks.0.attn.l_proj",
+             "blocks.0.attn.o_proj", "blocks.1.attn.v_conv1d", "blocks.0.attn.o_norm"]
+    assert _native_taken(LSHGatedDelta(n_layers=2), monkeypatch)
+    for name in names:
+        m = LSHGatedDelta(n_layers=2)
+        _hooked(kind)(m.get_submodule(name))
+        assert not _native_taken(m, monkeypatch), name
+
+
+def test_fused_model_leaves_global_hooks_and_overridden_methods_alone(monkeypatch):
+    from torch.nn.modules import module as nn_module
+    from lampa_b200.model import LSHGatedDelta
+    m = LSHGatedDelta(n_layers=1)
+    for register in (nn_module.register_module_forward_hook, nn_module.register_module_forward_pre_hook):
+        handle = register(lambda *a: None)
+        try:
+            assert not _native_taken(m, monkeypatch)
+        finally:
+            handle.remove()
+    assert _native_taken(m, monkeypatch)
+
+    class OwnOrder(LSHGatedDelta):
+        def orderings(self, hits, cu):
+            return super().orderings(hits, cu)
+
+    assert not _native_taken(OwnOrder(n_layers=1), monkeypatch)
+    m.blocks[0].mix = lambda *a, **k: None
+    assert not _native_taken(m, monkeypatch)
+    m = LSHGatedDelta(n_layers=1)
+    m.blocks[0].attn.o_norm.bias = torch.nn.Parameter(torch.zeros(32))     # the output norm refuses a bias
+    assert not _native_taken(m, monkeypatch)
