@@ -159,7 +159,7 @@ def hept_attention_core(e2lsh, query: torch.Tensor, key: torch.Tensor, value: to
     """HEPTAttention.forward between the projections and `out_linear`: query, key, value
     [N, heads, d] (N padded to block_size), coords [N, r + 1] with the padded rows zeroed, `ranks`
     the (eta, phi) ranks of the hits (geo.region_inputs) -> [heads, N, d]."""
-    if type(e2lsh) is E2LSH and not e2lsh._forward_hooks and not e2lsh._forward_pre_hooks and w.is_cuda:
+    if L.runs_own_forward(e2lsh, E2LSH) and w.is_cuda:
         out = L.native.hept_core(e2lsh.alpha, query, key, value, _coord_scale(w.detach()), coords, regions_h, ranks[0], ranks[1],
                                  int(raw_size), int(block_size))
         if out is not None:

@@ -238,3 +238,29 @@ def test_attention_core_sizes(lb, raw, block, heads, rounds, d, cd):
     q_pos, k_pos = lb.hept_positions(e2lsh, q_hat, k_hat, inp["regions_h"], inp["ranks"], raw)
     ref, _, _ = oracle.hept_bucket_attention(to_np(q_hat), to_np(k_hat), to_np(v), to_np(q_pos), to_np(k_pos), block)
     _close(to_np(out)[:, :raw], ref[:, :raw], 5e-5, "attention core")
+
+
+def test_attention_core_runs_a_modified_hash(lb):
+    """A replaced forward of the hash, and hooks of all modules, run instead of the one-call layer."""
+    from torch.nn.modules import module as nn_module
+    raw, block, heads, rounds, d, cd = 230, 50, 2, 2, 8, 4
+    gen = torch.Generator().manual_seed(3)
+    inp = lb.region_inputs(torch.randn(raw, cd, generator=gen).cuda(), lb.get_regions(20, rounds, heads), block)
+    query, key, value = (lb.pad_to_multiple(torch.randn(raw, heads, d, generator=gen) * 0.6, block, dims=0).cuda() for _ in range(3))
+    w = (torch.randn(heads, d, cd - 1, 5, generator=gen) * 0.3 - 0.8).cuda()
+    e2lsh = lb.E2LSH(n_hashes=rounds, n_heads=heads, dim=d + cd).cuda()
+
+    def core():
+        return lb.hept_attention_core(e2lsh, query, key, value, w, inp["coords"], inp["regions_h"], inp["ranks"], raw, block)
+
+    want, calls = core(), []
+    handle = nn_module.register_module_forward_hook(lambda mod, a, out: calls.append(mod))
+    try:
+        got = core()
+    finally:
+        handle.remove()
+    assert calls == [e2lsh, e2lsh]
+    _close(to_np(got)[:, :raw], to_np(want)[:, :raw], 5e-5, "composed against one-call layer")
+    e2lsh.forward = lambda vecs: calls.append("own") or type(e2lsh).forward(e2lsh, vecs)
+    _close(to_np(core())[:, :raw], to_np(want)[:, :raw], 5e-5, "composed against one-call layer")
+    assert calls[2:] == ["own", "own"]
