@@ -197,8 +197,19 @@ class LSHOrdering(nn.Module):
         expo = torch.tensor([2.0 ** i for i in range(self.num_hashes)], device=coords.device)
         return (proj[:, 0, :] * expo[:, None]).sum(0).view(B, Ln)
 
+    @torch.no_grad()
+    def _ordered_by(self, points: torch.Tensor, coords: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        """The order by the keys of a subclass: norms, two stable sorts and the gather as calls of their own."""
+        B, Ln, D = points.shape
+        c = coords.to(torch.float32)
+        by_norm = segmented_sort(c.norm(dim=-1), nseg=B)
+        idx = segmented_sort(self.bucket_keys(c), nseg=B, init=by_norm).view(B, Ln)
+        return permute_rows(points.reshape(B * Ln, D), idx.view(-1), nseg=B).view(B, Ln, D), idx
+
     def forward(self, points: torch.Tensor, coords: torch.Tensor = None) -> Tuple[torch.Tensor, torch.Tensor]:
         alpha = self.e2lsh.alpha
+        if type(self).bucket_keys is not LSHOrdering.bucket_keys or "bucket_keys" in self.__dict__:
+            return self._ordered_by(points, points if coords is None else coords)
         r = L.native.ordering(points, points if coords is None else coords, alpha)
         if r is not None:
             return r

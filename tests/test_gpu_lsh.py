@@ -158,3 +158,17 @@ def test_sort_tile_edges(lb, n):
     seg = np.array([0, n, n + 77], np.int64)
     got = to_np(lb.segmented_sort(_dev(torch.from_numpy(k)), seg_offsets=torch.from_numpy(seg)))
     np.testing.assert_array_equal(got, oracle.segsort(k, seg))
+
+
+def test_ordering_layer_with_keys_of_its_own(lb):
+    """A subclass's bucket_keys decide the order."""
+    class Falling(lb.LSHOrdering):
+        def bucket_keys(self, coords):
+            return -super().bucket_keys(coords)
+
+    gen = torch.Generator().manual_seed(4)
+    coords, points = torch.randn(2, 300, 4, generator=gen).cuda(), torch.randn(2, 300, 5, generator=gen).cuda()
+    layer = Falling(4).cuda()
+    ordered, idx = layer(points, coords)
+    want = layer.bucket_keys(coords).sort(dim=1, stable=True).indices      # distinct keys: the norms break no tie
+    assert torch.equal(idx, want) and torch.equal(ordered, points.gather(1, want[..., None].expand(-1, -1, 5)))
