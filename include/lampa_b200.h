@@ -436,7 +436,7 @@ int lampa_profile_read(char* names, size_t names_cap, float* total_ms, int32_t* 
 
 /*
  * Test hook (no counterpart in the reference): number of polls after which a device-side wait of
- * the gated-delta kernels gives up (default and maximum 2^22).  A test sets it to 0 to see the
+ * the gated-delta and model kernels gives up (default and maximum 2^22).  A test sets it to 0 to see the
  * give-up path without anything hanging: the kernels then return at once, results are undefined
  * and LAMPA_ERR_TIMEOUT is in the status word; copies and MMAs already in flight are still waited
  * for with the full budget before a CTA exits.  Process-wide; not for concurrent use.

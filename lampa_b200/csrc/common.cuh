@@ -176,8 +176,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // is left unbalanced.  A thread that has given up once (`dead`) does not wait again: it runs to the
 // end of its loop, issues nothing new and drains what it has in flight with mbar_drain.
 constexpr int MBAR_POLLS = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, bool& dead, int32_t* status, int where,
-                                          int budget = MBAR_POLLS) {
+int poll_budget();                 // of the launches that follow (host): MBAR_POLLS unless lampa_debug_set_poll_budget lowered it
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, bool& dead, int32_t* status, int where, int budget) {
     if (dead) return false;
     for (int i = 0; i < budget; ++i)
         if (mbar_try_wait(bar, parity)) return true;

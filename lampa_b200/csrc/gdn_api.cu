@@ -5,11 +5,15 @@
 
 using namespace lampa;
 
+namespace lampa {
+static int g_poll_budget = MBAR_POLLS;
+int poll_budget() { return g_poll_budget; }
+}  // namespace lampa
+
 namespace {
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-int g_poll_budget = MBAR_POLLS;   // see lampa_debug_set_poll_budget
 int g_force_mma_sync = 0;         // see lampa_debug_force_mma_sync
 long long* g_ticks = nullptr;     // see lampa_debug_set_tick_buffer
 int g_ticks_ctas = 0;
@@ -100,7 +104,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     a.status = status;
     static const int no_umma = [] { const char* e = getenv("LAMPA_B200_NO_UMMA"); return (e && e[0] == '1') ? 1 : 0; }();
     a.use_umma = (no_umma || g_force_mma_sync) ? 0 : 1;
-    a.poll_budget = g_poll_budget;
+    a.poll_budget = poll_budget();
     a.ticks = g_ticks;
     a.ticks_ctas = g_ticks_ctas;
 }
@@ -327,7 +331,7 @@ static int hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, cons
     s.qkv_dt = d->qkv_dtype; s.gb_dt = d->gb_dtype; s.lam_dt = d->lam_dtype;
     s.B = d->B; s.H = d->H; s.L = d->L; s.use_l2norm = d->use_l2norm;
     s.arrivals = arrivals;
-    s.poll_budget = g_poll_budget;
+    s.poll_budget = poll_budget();
     s.status = status;
     cudaStream_t st = (cudaStream_t)stream;
     if (d->K == 64) return launch_hgdn_step<64, 64>(s, st);

@@ -809,7 +809,7 @@ extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, c
     a.conv[0] = (const __nv_bfloat16*)w->q_conv; a.conv[1] = (const __nv_bfloat16*)w->k_conv; a.conv[2] = (const __nv_bfloat16*)w->v_conv;
     a.A_log = w->A_log; a.dt_bias = w->dt_bias; a.Lw = w->Lw; a.H = w->H; a.L = w->L;
     a.out[0] = (__nv_bfloat16*)q; a.out[1] = (__nv_bfloat16*)k; a.out[2] = (__nv_bfloat16*)v; a.out[3] = (__nv_bfloat16*)gate;
-    a.g = g; a.beta = beta; a.lam = (__nv_bfloat16*)lam; a.status = status; a.budget = MBAR_POLLS;
+    a.g = g; a.beta = beta; a.lam = (__nv_bfloat16*)lam; a.status = status; a.budget = poll_budget();
     for (const void* p : {w->q_w, w->k_w, w->v_w, w->g_w, w->a_w, w->b_w, w->l_w, hs, (const void*)q, (const void*)k, (const void*)v, (const void*)gate, (const void*)lam})
         if (!p || ((uintptr_t)p & 15)) return LAMPA_ERR_UNSUPPORTED;
     for (const void* p : {w->q_conv, w->k_conv, w->v_conv})
@@ -842,7 +842,7 @@ extern "C" int lampa_model_update(const lampa_model_update_w* w, const void* o, 
     a.x = x; a.perm = perm; a.cu = cu; a.nseq = nseq; a.n = n;
     a.mlp_norm_w = w->mlp_norm_w; a.up_b = (const __nv_bfloat16*)w->up_b; a.down_b = (const __nv_bfloat16*)w->down_b;
     a.next_norm_w = w->next_norm_w; a.hs = (__nv_bfloat16*)hs;
-    a.eps = w->eps; a.next_eps = w->next_eps; a.o_eps = w->o_eps; a.status = status; a.budget = MBAR_POLLS;
+    a.eps = w->eps; a.next_eps = w->next_eps; a.o_eps = w->o_eps; a.status = status; a.budget = poll_budget();
     CUtensorMap mo, mu, md;
     if (!make_map(&mo, w->o_w, LAMPA_BF16, MD, MD, 64, MD, true) || !make_map(&mu, w->up_w, LAMPA_BF16, UP_HID, MD, 64, UP_CH, true) ||
         !make_map(&md, w->down_w, LAMPA_BF16, MD, UP_HID, 64, MD, true))

@@ -253,3 +253,75 @@ def test_short_conv_of_sequences_outside_the_input(lb):
     got, state = conv(x, cu_seqlens=torch.tensor([-(1 << 36), 40, 1 << 40], device="cuda:0"), output_final_state=True)
     assert torch.equal(got, want)                               # all rows have the taps of the sequence they lie in
     assert torch.equal(state[0], x[0, 40 - W:40].T) and not state[1].any()
+
+
+def _model_structs(m):
+    """The two C structs of a model's first block, and what they point to."""
+    import ctypes
+    vp = ctypes.c_void_p
+
+    class Mixer(ctypes.Structure):
+        _fields_ = [(n, vp) for n in ("q_w", "k_w", "v_w", "g_w", "a_w", "b_w", "l_w", "q_conv", "k_conv", "v_conv",
+                                      "A_log", "dt_bias", "Lw")] + [("H", ctypes.c_int32), ("L", ctypes.c_int32)]
+
+    class Update(ctypes.Structure):
+        _fields_ = [(n, vp) for n in ("o_norm_w", "o_w", "up_w", "up_b", "down_w", "down_b", "mlp_norm_w", "next_norm_w")] + [
+            (n, ctypes.c_float) for n in ("o_eps", "eps", "next_eps")] + [("head_dim", ctypes.c_int32)]
+
+    b, at = m.blocks[0], m.blocks[0].attn
+    mix = Mixer(*(t.data_ptr() for t in (at.q_proj.weight, at.k_proj.weight, at.v_proj.weight, at.g_proj.weight, at.a_proj.weight,
+                                         at.b_proj.weight, at.l_proj.weight, at.q_conv1d.weight, at.k_conv1d.weight,
+                                         at.v_conv1d.weight, at.A_log, at.dt_bias, at.L)), at.num_heads, at.num_levels)
+    upd = Update(*(t.data_ptr() for t in (at.o_norm.weight, at.o_proj.weight, b.mlp_up.weight, b.mlp_up.bias, b.mlp_down.weight,
+                                          b.mlp_down.bias, b.mlp_norm_weight, m.blocks[1].attn_norm_weight)),
+                 at.o_norm.eps, b.eps, b.eps, at.head_dim)
+    return mix, upd
+
+
+@pytest.mark.parametrize("budget", [0, 1])
+def test_model_kernels_whose_waits_run_out_return(lb, budget):
+    """Both block kernels with several tiles per CTA: a wait that runs out is reported, the kernel drains and comes back, and
+    the next call is right."""
+    import ctypes
+    from lampa_b200 import _lib as L
+    n = 148 * 2 * 128 * 2 + 77                                  # every CTA has more than two tiles
+    m, _ = _model(lb, 1)
+    mix, upd = _model_structs(m)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    new = lambda *s, dt=torch.bfloat16: torch.randn(*s, generator=gen, device="cuda", dtype=torch.float32).to(dt)
+    hs, o, gate = new(n, 128), new(n, 128), new(n, 128)
+    x0 = new(n, 128, dt=torch.float32)
+    perm = torch.randperm(n, generator=gen, device="cuda")
+    cu = torch.tensor([0, n], device="cuda:0")
+    st, stream = L.status_word(torch.device("cuda:0")), L.stream_ptr(torch.device("cuda:0"))
+    lib = L.lib()
+    vp = ctypes.c_void_p
+
+    def project():
+        out = [torch.empty(n, 128, dtype=torch.bfloat16, device="cuda:0") for _ in range(4)]
+        out += [torch.empty(n, mix.H, device="cuda:0") for _ in range(2)]
+        out += [torch.empty(n, mix.H * mix.L, dtype=torch.bfloat16, device="cuda:0")]
+        L.check(lib.lampa_model_project(ctypes.byref(mix), vp(hs.data_ptr()), vp(perm.data_ptr()), vp(cu.data_ptr()), 1,
+                                        ctypes.c_int64(n), *(vp(t.data_ptr()) for t in out), vp(st.data_ptr()), vp(stream)), "project")
+        return out
+
+    def update():
+        x, y = x0.clone(), torch.empty_like(hs)
+        L.check(lib.lampa_model_update(ctypes.byref(upd), vp(o.data_ptr()), vp(gate.data_ptr()), vp(x.data_ptr()), vp(perm.data_ptr()),
+                                       vp(cu.data_ptr()), 1, ctypes.c_int64(n), vp(y.data_ptr()), vp(st.data_ptr()), vp(stream)), "update")
+        return [x, y]
+
+    _status(lb)
+    for call, waits in ((project, range(600, 620)), (update, range(620, 640))):
+        want = call()
+        assert _status(lb)[0] == 0
+        try:
+            assert lib.lampa_debug_set_poll_budget(budget) == 0
+            call()
+            vals = _status(lb)
+        finally:
+            lib.lampa_debug_set_poll_budget(1 << 22)
+        # a single poll may wait long enough in hardware to succeed
+        assert vals[0] == L.ERR_TIMEOUT and vals[1] in waits if budget == 0 else vals[0] in (0, L.ERR_TIMEOUT)
+        assert all(torch.equal(a, b) for a, b in zip(call(), want))
+        assert _status(lb)[0] == 0
