@@ -173,7 +173,9 @@ int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const void* k, co
  *   e^g (I - beta k k^T), level 0 becomes beta k v^T, counts[0] += 1;
  *   o = q^T sum_l lam_l S_l.  As in lampa_hgdn_fwd q and k are l2-normalised when
  *   d->use_l2norm and the result does not depend on d->scale.  A cascade that would leave the
- *   last level sets LAMPA_ERR_LEVELS in the status word and changes nothing.
+ *   last level sets LAMPA_ERR_LEVELS in the status word and changes nothing.  After
+ *   LAMPA_ERR_TIMEOUT (where = 32) counts are those before the step but parts of `states` may have
+ *   taken the token in: the state is not usable any more, and the outputs are undefined.
  */
 int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
                     const void* g, const void* beta, const void* lam, float* states,

@@ -186,7 +186,8 @@ def _gdn_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_se
 class HState:
     """Fenwick state of the hierarchical rule (models/hattention/recurrent.py:9-131): `states`
     [B,H,K,V,L] and `counts` [L] int32 (tokens held per level).  Always fp32 on the device; the
-    cascade / insert / dot methods of the reference live in the library's step kernel."""
+    cascade / insert / dot methods of the reference live in the library's step kernel.  A decode
+    step that reports a wait that ran out leaves `counts` as they were and `states` unusable."""
 
     def __init__(self, base: int, htype, hstruct, shape, dtype: torch.dtype, device, empty: bool = False) -> None:
         if getattr(htype, "name", htype) != "WEAK" or base != 2:

@@ -325,3 +325,53 @@ def test_model_kernels_whose_waits_run_out_return(lb, budget):
         assert vals[0] == L.ERR_TIMEOUT and vals[1] in waits if budget == 0 else vals[0] in (0, L.ERR_TIMEOUT)
         assert all(torch.equal(a, b) for a, b in zip(call(), want))
         assert _status(lb)[0] == 0
+
+
+@pytest.mark.parametrize("counted", [True, False])
+@pytest.mark.parametrize("budget", [0, 1])
+def test_decode_step_whose_wait_runs_out_leaves_the_counts(lb, counted, budget):
+    """The one-launch step and the one with a launch of its own for the counts: slabs that did not arrive in time are not
+    stepped, and then the counts are not either; the arrival counter is zero again for the next step."""
+    import ctypes
+    from lampa_b200 import _lib as L, synth
+    B, H, K, Lv = 16, 4, 64, 13
+    inp = {k: v.to("cuda:0") for k, v in synth.gdn_inputs(8, B, H, K, K, L=Lv, g_shift=-3.0).items()}
+    x = {k: v[0].contiguous() for k, v in inp.items()}                     # B rows of one token
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    states = torch.randn(B, H, K, K, Lv, generator=gen, device="cuda")
+    counts = torch.tensor([1, 1, 2, 0, 8] + [0] * (Lv - 5), dtype=torch.int32, device="cuda:0")
+    arrivals = torch.zeros(1, dtype=torch.int32, device="cuda:0")
+    desc = L.GdnDesc(B=B, T=1, H=H, K=K, V=K, L=Lv, nseq=0, qkv_dtype=L.dtype_code(x["q"].dtype), gb_dtype=L.dtype_code(x["g"].dtype),
+                     lam_dtype=L.dtype_code(x["lam"].dtype), use_l2norm=1, scale=1.0)
+    st, stream = L.status_word(torch.device("cuda:0")), L.stream_ptr(torch.device("cuda:0"))
+
+    def step(s, c):
+        o = torch.empty_like(x["v"])
+        a = [L.ptr(x[k]) for k in ("q", "k", "v", "g", "beta", "lam")] + [L.ptr(s), L.ptr(c)]
+        if counted:
+            rc = L.lib().lampa_hgdn_step_counted(ctypes.byref(desc), *a, L.ptr(arrivals), L.ptr(o), L.ptr(st), stream)
+        else:
+            rc = L.lib().lampa_hgdn_step(ctypes.byref(desc), *a, L.ptr(o), L.ptr(st), stream)
+        L.check(rc, "step")
+        return o
+
+    _status(lb)
+    want_s, want_c = states.clone(), counts.clone()
+    want = step(want_s, want_c)
+    assert _status(lb)[0] == 0 and want_c.tolist()[:5] == [1, 0, 0, 4, 8]
+    s, c = states.clone(), counts.clone()
+    try:
+        assert L.lib().lampa_debug_set_poll_budget(budget) == 0
+        step(s, c)
+        vals = _status(lb)
+    finally:
+        L.lib().lampa_debug_set_poll_budget(1 << 22)
+    assert arrivals.item() == 0
+    if budget == 0:
+        assert vals[0] == L.ERR_TIMEOUT and vals[1] == 32
+        assert torch.equal(s, states)
+    assert torch.equal(c, counts if vals[0] == L.ERR_TIMEOUT else want_c)    # one poll may wait long enough to succeed
+    s, c = states.clone(), counts.clone()
+    o = step(s, c)
+    assert _status(lb)[0] == 0 and arrivals.item() == 0
+    assert torch.equal(o, want) and torch.equal(s, want_s) and torch.equal(c, want_c)
