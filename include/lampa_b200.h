@@ -187,6 +187,13 @@ int lampa_hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const
 int lampa_hgdn_step_counted(const lampa_gdn_desc* d, const void* q, const void* k, const void* v,
                             const void* g, const void* beta, const void* lam, float* states,
                             int32_t* counts, int32_t* arrivals, void* o, int32_t* status, void* stream);
+/* lampa_hgdn_final_state and lampa_hgdn_prefill that also set that counter (or NULL) to zero for the steps to come */
+int lampa_hgdn_final_state_counted(const lampa_gdn_desc* d, const void* k, const void* v, const void* g,
+                                   const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
+                                   float* states, int32_t* counts, int32_t* arrivals, int32_t* status, void* stream);
+int lampa_hgdn_prefill_counted(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                               const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
+                               float* states, int32_t* counts, int32_t* arrivals, int32_t* status, void* stream);
 /*
  * E2LSH projection and integer bucket ids.
  * Replaces: E2LSH.forward (models/model_utils/hash_utils.py:359-371; copies in

@@ -37,7 +37,7 @@ class GdnDesc(ctypes.Structure):
 _lib: Optional[ctypes.CDLL] = None
 EXPORTS = ["lampa_version", "lampa_error_string", "lampa_gdn_workspace_bytes", "lampa_gdn_workspace_layout",
            "lampa_gdn_fwd", "lampa_hgdn_fwd", "lampa_hgdn_fwd_scatter", "lampa_hgdn_final_state", "lampa_hgdn_prefill",
-           "lampa_hgdn_step", "lampa_hgdn_step_counted", "lampa_lsh_hash", "lampa_segsort_workspace_bytes",
+           "lampa_hgdn_step", "lampa_hgdn_step_counted", "lampa_hgdn_final_state_counted", "lampa_hgdn_prefill_counted", "lampa_lsh_hash", "lampa_segsort_workspace_bytes",
            "lampa_segsort_stable", "lampa_lsh_ordering_workspace_bytes", "lampa_lsh_ordering",
            "lampa_permute_rows", "lampa_invert_perm", "lampa_segsort_stable_static",
            "lampa_short_conv_fwd", "lampa_short_conv_step", "lampa_gate_inputs", "lampa_rmsnorm_gate", "lampa_add_rmsnorm",
@@ -68,6 +68,8 @@ def lib() -> ctypes.CDLL:
         L.lampa_hgdn_fwd_scatter.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 8 + [i64, vp, vp, sz, vp, vp]
         L.lampa_hgdn_final_state.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 6 + [sz, vp, vp, vp, vp]
         L.lampa_hgdn_prefill.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 8 + [sz, vp, vp, vp, vp]
+        L.lampa_hgdn_final_state_counted.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 6 + [sz, vp, vp, vp, vp, vp]
+        L.lampa_hgdn_prefill_counted.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 8 + [sz, vp, vp, vp, vp, vp]
         L.lampa_hgdn_step.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 11
         L.lampa_hgdn_step_counted.argtypes = [ctypes.POINTER(GdnDesc)] + [vp] * 12
         L.lampa_lsh_hash.argtypes = [vp, i64, i64, vp, vp, ctypes.c_float, i64, i32, i32, i32, vp, vp, vp, vp]

@@ -175,6 +175,7 @@ struct TailArgs {
     int n0;                               // whole chunks of every sequence, or -1: from chunk_off, ragged chunks completed by null tokens
     int tail;                             // tokens behind them (only with n0 >= 0)
     int one_count;
+    int32_t* arrivals;                    // set to zero, or NULL: the arrival counter of the decode steps to come
 };
 template <int KD, int VD> int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st);
 

@@ -272,9 +272,9 @@ int final_state(const lampa_gdn_desc* d, const GdnArgs& a, const TailArgs& ta, c
 
 }  // namespace
 
-extern "C" int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v, const void* g,
-                                      const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
-                                      float* states, int32_t* counts, int32_t* status, void* stream) {
+extern "C" int lampa_hgdn_final_state_counted(const lampa_gdn_desc* d, const void* k, const void* v, const void* g,
+                                              const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
+                                              float* states, int32_t* counts, int32_t* arrivals, int32_t* status, void* stream) {
     Layout l;
     int rc = make_layout(d, true, l);
     if (rc != LAMPA_OK) return rc;
@@ -287,13 +287,19 @@ extern "C" int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, co
     fill_args(d, true, l, (char*)ws, cu_seqlens, status, a);
     a.k = k; a.v = v; a.g = g; a.beta = beta;
     TailArgs ta;
-    ta.states = states; ta.counts = counts; ta.n0 = -1; ta.tail = 0; ta.one_count = 0;
+    ta.states = states; ta.counts = counts; ta.n0 = -1; ta.tail = 0; ta.one_count = 0; ta.arrivals = arrivals;
     return final_state(d, a, ta, (cudaStream_t)stream);
 }
 
-extern "C" int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
-                                  const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
-                                  float* states, int32_t* counts, int32_t* status, void* stream) {
+extern "C" int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v, const void* g,
+                                      const void* beta, const int64_t* cu_seqlens, void* ws, size_t ws_bytes,
+                                      float* states, int32_t* counts, int32_t* status, void* stream) {
+    return lampa_hgdn_final_state_counted(d, k, v, g, beta, cu_seqlens, ws, ws_bytes, states, counts, nullptr, status, stream);
+}
+
+extern "C" int lampa_hgdn_prefill_counted(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                                          const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
+                                          float* states, int32_t* counts, int32_t* arrivals, int32_t* status, void* stream) {
     if (!d || d->nseq != 0) return LAMPA_ERR_ARG;
     Layout l;
     lampa_gdn_desc whole = *d;                           // the whole chunks of every row
@@ -312,8 +318,14 @@ extern "C" int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const 
     a.fixed_stride = d->T;
     a.q = q; a.k = k; a.v = v; a.g = g; a.beta = beta; a.lam = lam; a.o = o;
     TailArgs ta;
-    ta.states = states; ta.counts = counts; ta.n0 = whole.T / CHUNK; ta.tail = d->T - whole.T; ta.one_count = 1;
+    ta.states = states; ta.counts = counts; ta.n0 = whole.T / CHUNK; ta.tail = d->T - whole.T; ta.one_count = 1; ta.arrivals = arrivals;
     return final_state(d, a, ta, (cudaStream_t)stream);
+}
+
+extern "C" int lampa_hgdn_prefill(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,
+                                  const void* beta, const void* lam, void* o, void* ws, size_t ws_bytes,
+                                  float* states, int32_t* counts, int32_t* status, void* stream) {
+    return lampa_hgdn_prefill_counted(d, q, k, v, g, beta, lam, o, ws, ws_bytes, states, counts, nullptr, status, stream);
 }
 
 static int hgdn_step(const lampa_gdn_desc* d, const void* q, const void* k, const void* v, const void* g,

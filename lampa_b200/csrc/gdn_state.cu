@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             if (held) rem -= cap;
         }
         cn[0] = n > 0 ? 1 : 0;
+        if (seq == 0 && ta.arrivals) *ta.arrivals = 0;
         if (rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
     }
 }

@@ -172,8 +172,14 @@ bool mixer_args(PyObject* const* a, MixerArgs& m, bool entry) {
     return m.d.K <= 256;
 }
 
+// (o, states, counts, arrivals): the counts and, in the word behind them, the arrival counter of the decode steps
+PyObject* with_words(const Tensor& o, const Tensor& states, const Tensor& words, at::IntArrayRef counts) {
+    const int64_t n = words.numel() - 1;
+    return pack({wrap(o), wrap(states), wrap(words.narrow(0, 0, n).view(counts)), wrap(words.narrow(0, n, 1))});
+}
+
 // gdn(q, k, v, g, beta, lam|None, h0|None, cu|None, out_perm|None, scale|None, l2norm, want_state, entry)
-//   plain rule: (o, final state | None); hierarchical: (o, None), or (o, states, counts) with want_state
+//   plain rule: (o, final state | None); hierarchical: (o, None), or (o, states, counts, arrivals) with want_state
 PyObject* gdn(PyObject* const* a) {
     MixerArgs m;
     const bool entry = a[12] == Py_True;
@@ -214,19 +220,19 @@ PyObject* gdn(PyObject* const* a) {
     else
         check(lampa_hgdn_fwd(&m.d, ptr(m.q), ptr(m.k), ptr(m.v), ptr(m.g), ptr(m.beta), ptr(m.lam), (const int64_t*)ptr(cu),
                              o.data_ptr(), ws, bytes, c.status, c.stream), "lampa_hgdn_fwd");
-    Tensor states, counts;
-    if (want_state) {
-        states = empty({N, m.d.H, m.d.K, m.d.V, m.d.L}, at::kFloat, m.dev);
-        counts = empty({N, m.d.L}, at::kInt, m.dev);
-        check(lampa_hgdn_final_state(&m.d, ptr(m.k), ptr(m.v), ptr(m.g), ptr(m.beta), (const int64_t*)ptr(cu), ws, bytes,
-                                     (float*)states.data_ptr(), (int32_t*)counts.data_ptr(), c.status, c.stream), "lampa_hgdn_final_state");
+    if (!want_state) {
+        debug_check(c);
+        return pack({wrap(o), none()});
     }
+    Tensor states = empty({N, m.d.H, m.d.K, m.d.V, m.d.L}, at::kFloat, m.dev), words = empty({N * m.d.L + 1}, at::kInt, m.dev);
+    int32_t* counts = (int32_t*)words.data_ptr();
+    check(lampa_hgdn_final_state_counted(&m.d, ptr(m.k), ptr(m.v), ptr(m.g), ptr(m.beta), (const int64_t*)ptr(cu), ws, bytes,
+                                         (float*)states.data_ptr(), counts, counts + N * m.d.L, c.status, c.stream), "lampa_hgdn_final_state");
     debug_check(c);
-    if (!want_state) return pack({wrap(o), none()});
-    return pack({wrap(o), wrap(states), wrap(counts)});
+    return with_words(o, states, words, {N, m.d.L});
 }
 
-// prefill(q, k, v, g, beta, lam, entry) -> (o, states, counts [L])
+// prefill(q, k, v, g, beta, lam, entry) -> (o, states, counts [L], arrivals)
 PyObject* prefill(PyObject* const* a) {
     MixerArgs m;
     const bool entry = a[6] == Py_True;
@@ -241,11 +247,12 @@ PyObject* prefill(PyObject* const* a) {
     check(lampa_gdn_workspace_bytes(&whole, &bytes), "lampa_gdn_workspace_bytes");
     Tensor hold, o = empty({m.d.B, m.d.T, m.d.H, m.d.V}, m.q->scalar_type(), m.dev);
     void* ws = workspace(bytes, m.dev, hold);
-    Tensor states = empty({m.d.B, m.d.H, m.d.K, m.d.V, m.d.L}, at::kFloat, m.dev), counts = empty({m.d.L}, at::kInt, m.dev);
-    check(lampa_hgdn_prefill(&m.d, ptr(m.q), ptr(m.k), ptr(m.v), ptr(m.g), ptr(m.beta), ptr(m.lam), o.data_ptr(), ws, bytes,
-                             (float*)states.data_ptr(), (int32_t*)counts.data_ptr(), c.status, c.stream), "lampa_hgdn_prefill");
+    Tensor states = empty({m.d.B, m.d.H, m.d.K, m.d.V, m.d.L}, at::kFloat, m.dev), words = empty({m.d.L + 1}, at::kInt, m.dev);
+    int32_t* counts = (int32_t*)words.data_ptr();
+    check(lampa_hgdn_prefill_counted(&m.d, ptr(m.q), ptr(m.k), ptr(m.v), ptr(m.g), ptr(m.beta), ptr(m.lam), o.data_ptr(), ws, bytes,
+                                     (float*)states.data_ptr(), counts, counts + m.d.L, c.status, c.stream), "lampa_hgdn_prefill");
     debug_check(c);
-    return pack({wrap(o), wrap(states), wrap(counts)});
+    return with_words(o, states, words, {m.d.L});
 }
 
 // step(q, k, v, g, beta, lam, states, counts, arrivals, entry): one token per row, q [B,1,H,K] (or [B,H,K]) -> o of v's shape

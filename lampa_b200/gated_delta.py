@@ -206,10 +206,12 @@ class HState:
             self.states = self.counts = None
             return
         self.states = torch.zeros(self.shape, dtype=dtype, device=device)
-        self.counts = torch.zeros(self.max_num_levels, dtype=torch.int32, device=device)
+        words = torch.zeros(self.max_num_levels + 1, dtype=torch.int32, device=device)
+        self.counts, self._arrivals = words[:-1], words[-1:]
 
     def arrivals(self) -> torch.Tensor:
-        """The step kernel's arrival counter: one int32 of this state, zero between steps."""
+        """The step kernel's arrival counter: one int32 of this state, zero between steps.  It is made with the state; only a
+        state put together by hand, or moved by assignment, gets one here."""
         a = self._arrivals
         if a is None or a.device != self.states.device:
             a = self._arrivals = torch.zeros(1, dtype=torch.int32, device=self.states.device)
@@ -221,11 +223,11 @@ class HState:
     def to(self, dtype: Optional[torch.dtype] = None, device=None) -> "HState":
         new = HState.__new__(HState)
         new.__dict__.update(self.__dict__)
-        new._arrivals = None
         new.dtype = self.dtype if dtype is None else dtype
         new.device = self.device if device is None else torch.device(device)
         new.states = self.states.to(dtype=new.dtype, device=new.device)
         new.counts = self.counts.to(dtype=torch.int32, device=new.device)
+        new._arrivals = torch.zeros(1, dtype=torch.int32, device=new.states.device)
         return new
 
 
@@ -248,7 +250,8 @@ def _hgdn(q, k, v, g, beta, lam, cu_seqlens, use_l2norm, want_state: bool = Fals
         if not want_state:
             return o
         N, Lv = (B if cu is None else len(cu) - 1), lam.shape[-1]
-        return o, torch.empty(N, H, K, V, Lv, device=dev), torch.empty(N, Lv, dtype=torch.int32, device=dev)
+        return (o, torch.empty(N, H, K, V, Lv, device=dev), torch.empty(N, Lv, dtype=torch.int32, device=dev),
+                torch.zeros(1, dtype=torch.int32, device=dev))
     r = _launched(L.native.gdn(q, k, v, g, beta, lam, None, cu, out_perm, None, bool(use_l2norm), want_state, False),
                   "lampa_hgdn_fwd")
     return r if want_state else r[0]
@@ -293,10 +296,10 @@ def _hgdn_prefill(q, k, v, g, beta, lam, use_l2norm: bool = True):
 
 
 def _with_state(r):
-    """(o, states, counts) -> (o, HState)"""
-    o, states, counts = r
+    """(o, states, counts, arrivals) -> (o, HState)"""
+    o, states, counts, arrivals = r
     hs = HState(2, HType.WEAK, HStruct.GDELTA, states.shape, torch.float32, states.device, empty=True)
-    hs.states, hs.counts = states, counts
+    hs.states, hs.counts, hs._arrivals = states, counts, arrivals
     return o, hs
 
 

@@ -317,3 +317,29 @@ def test_final_state_of_packed_sequences_through_the_python_op(lb):
         assert_close_bf16(to_np(o[0, s:e]), oref, f"o of sequence {n}")
         np.testing.assert_array_equal(to_np(hs.counts[n]), cref)
         _close_states(to_np(hs.states[n]), sref, f"sequence {n}")
+
+
+def test_first_decode_step_prepares_nothing(lb):
+    """The arrival counter of the decode steps comes with the state, from whichever call made it: the first step asks the
+    allocator for as much as any other, and launches as much."""
+    from lampa_b200 import synth
+    H, K, Lv = 2, 32, 13
+    inp = _cuda(synth.gdn_inputs(7, 200, H, K, K, L=Lv, g_shift=-3.0))
+    part = lambda s: [inp[k][:, s] for k in ("q", "k", "v", "g", "lam", "beta")]
+    kw = dict(output_final_state=True, use_qk_l2norm_in_kernel=True)
+    made = [lb.chunk_h_gated_delta_rule(*(t.contiguous() for t in part(slice(0, 150))), **kw)[1],
+            lb.chunk_h_gated_delta_rule(*(t.contiguous() for t in part(slice(0, 128))), cu_seqlens=torch.tensor([0, 128]), **kw)[1],
+            lb.HState(2, lb.HType.WEAK, lb.HStruct.GDELTA, (1, H, K, K, Lv), torch.float32, "cuda:0")]
+    made.append(made[0].to(device="cuda:0"))
+    asked = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]
+    x = [t.contiguous() for t in part(slice(150, 151))]
+    lb.chunk_h_gated_delta_rule(*x, initial_state=lb.HState(2, lb.HType.WEAK, lb.HStruct.GDELTA, (1, H, K, K, Lv), torch.float32, "cuda:0"), **kw)
+    for state in made:
+        used = []
+        for _ in range(2):
+            before = asked()
+            o, _ = lb.chunk_h_gated_delta_rule(*x, initial_state=state, **kw)
+            used.append(asked() - before)
+        assert used == [1, 1], used                 # the output
+        assert state.arrivals().item() == 0
+    lb.check_status()
