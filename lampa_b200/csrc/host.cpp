@@ -272,7 +272,8 @@ PyObject* step(PyObject* const* a) {
     const int dt = dtype_code(*q), gdt = dtype_code(*g), ldt = dtype_code(*lam);
     if (B <= 0 || H <= 0 || dt < 0 || (entry && dt == LAMPA_F32) || gdt < 0 || ldt < 0) return none();
     if (k->scalar_type() != q->scalar_type() || v->scalar_type() != q->scalar_type() || beta->scalar_type() != g->scalar_type()) return none();
-    if (states->scalar_type() != at::kFloat || states->sizes() != at::IntArrayRef({B, H, K, V, L}) || counts->scalar_type() != at::kInt) return none();
+    if (states->scalar_type() != at::kFloat || states->sizes() != at::IntArrayRef({B, H, K, V, L}) || counts->scalar_type() != at::kInt ||
+        counts->numel() < L || arrivals->scalar_type() != at::kInt || arrivals->numel() < 1) return none();
     if (entry) warn_layout(1, H);
     const Call c = begin(*q);
     lampa_gdn_desc d;

@@ -267,6 +267,8 @@ def _hgdn_step(hstate: HState, q, k, v, g, beta, lam, use_l2norm: bool = True) -
     Lv = lam.shape[-1]
     if tuple(hstate.states.shape) != (B, H, K, V, Lv) or hstate.states.dtype != torch.float32:
         raise ValueError(f"state must be fp32 [{B},{H},{K},{V},{Lv}]")
+    if hstate.counts.dtype != torch.int32 or hstate.counts.numel() < Lv:
+        raise ValueError(f"counts must be int32 [{Lv}]")
     if not hstate.states.is_contiguous():
         hstate.states = hstate.states.contiguous()
     if not hstate.counts.is_contiguous():

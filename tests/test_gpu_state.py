@@ -343,3 +343,13 @@ def test_first_decode_step_prepares_nothing(lb):
         assert used == [1, 1], used                 # the output
         assert state.arrivals().item() == 0
     lb.check_status()
+
+
+def test_step_refuses_counts_that_are_too_few(lb):
+    H, K, Lv = 1, 32, 9
+    x, g, lam = torch.randn(1, 1, H, K, device="cuda:0").bfloat16(), torch.zeros(1, 1, H, device="cuda:0"), torch.ones(1, 1, H, Lv, device="cuda:0")
+    for counts in (torch.zeros(Lv - 1, dtype=torch.int32, device="cuda:0"), torch.zeros(Lv, dtype=torch.int64, device="cuda:0")):
+        hs = lb.HState(2, lb.HType.WEAK, lb.HStruct.GDELTA, (1, H, K, K, Lv), torch.float32, "cuda:0")
+        hs.counts = counts
+        with pytest.raises(ValueError):
+            lb.chunk_h_gated_delta_rule(x, x, x, g, lam, g, initial_state=hs, output_final_state=True, use_qk_l2norm_in_kernel=True)
