@@ -6,6 +6,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 
 #include "common.cuh"
 #include "profile.cuh"
@@ -459,7 +460,11 @@ invert_perm_kernel(const int64_t* __restrict__ perm, const int64_t* __restrict__
 // gather).  Here one launch does everything by counting: every CTA computes all keys of its segment
 // (24 bytes and ~50 flops per point, from L2), takes 32 points, eight lanes to a point, and counts
 // the points that come before each; the count is the point's position.  n^2 comparisons, but all in
-// parallel.
+// parallel.  The keys are half of it, and instruction issue bounds them: two points at a time, the
+// coordinates in registers, and loops over coordinates and hashes known to the compiler up to 8 and
+// 4.  4 x 1500 points with (coordinates, hashes) = (6, 3), (3, 3), (6, 4), (4, 6), (8, 8), (11, 3):
+// 8.7, 8.1, 9.0, 9.7, 12 and 13 us; with the hash count always a loop 9.3, 8.3, 9.5, 9.6, 12 and 12;
+// reading the coordinates again for every hash 11.7 for (3, 3) and 36 for (8, 8).
 // -------------------------------------------------------------------------------------------------
 constexpr int ORDER_THREADS = 256, ORDER_POINTS = ORDER_THREADS / 8, ORDER_MAX_N = 8192;
 
@@ -470,36 +475,76 @@ __device__ __forceinline__ uint32_t order_bits(float x) {          // key_xform 
 }
 // Operation order of a projection as in lsh_hash_kernel; the hashes are added in four interleaved partial sums,
 // which is the order torch.sum adds them in (fewer than four: simply left to right).
-// DIM, NH > 0: known to the compiler (the coordinates then stay in registers).
-template <int DIM, int NH>
-__device__ __forceinline__ void ordering_key_norm_fixed(const float* __restrict__ c, const float* alpha, float& key, float& norm) {
-    float x[DIM], ss = 0.f;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) { x[d] = __ldg(c + d); ss = fmaf(x[d], x[d], ss); }
-    norm = sqrtf(ss);
-    float part[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int j = 0; j < NH; ++j) {
-        float acc = __fmul_rn(x[0], alpha[j]);
-#pragma unroll
-        for (int d = 1; d < DIM; ++d) acc = __fadd_rn(acc, __fmul_rn(x[d], alpha[d * NH + j]));
-        part[j & 3] = __fadd_rn(part[j & 3], __fmul_rn(acc, (float)(1 << j)));
+// DIM > 0: rows of up to ORDER_REGS coordinates, read once and kept in registers through all hashes; wider rows (DIM = 0) are read
+// again for each four hashes.  NH > 0: up to four hashes, all at once (0: any number, four at a time).  alpha: [dim][nh4] in
+// shared memory, nh4 the hash count rounded up to four, padded with zeros that are not added.
+constexpr int ORDER_REGS = 8, ORDER_HASHES = 4;
+__device__ __forceinline__ void stage_alpha(const float* __restrict__ alpha, int dim, int nh, int nh4, float* s_alpha) {
+    for (int i = threadIdx.x; i < dim * nh4; i += blockDim.x) {
+        const int d = i / nh4, j = i - d * nh4;
+        s_alpha[i] = j < nh ? alpha[d * nh + j] : 0.f;
     }
-    key = __fadd_rn(__fadd_rn(__fadd_rn(part[0], part[1]), part[2]), part[3]);
 }
-__device__ __forceinline__ float ordering_key(const float* __restrict__ c, int dim, const float* alpha, int nh) {
-    float part[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < nh; ++j) {
-        float acc = __fmul_rn(__ldg(c), alpha[j]);
-        for (int d = 1; d < dim; ++d) acc = __fadd_rn(acc, __fmul_rn(__ldg(c + d), alpha[d * nh + j]));
-        part[j & 3] = __fadd_rn(part[j & 3], __fmul_rn(acc, __int_as_float((127 + min(j, 127)) << 23)));
+__device__ __forceinline__ float hash_weight(int j) { return __int_as_float((127 + min(j, 127)) << 23); }      // 2^j
+// NP points at c[0], c[1], ...: their loads and sums are independent chains.
+template <int DIM, int NH, int NP>
+__device__ __forceinline__ void ordering_key_norm(const float* const (&c)[NP], int dim, const float* s_alpha, int nh, int nh4, float (&key)[NP],
+                                                  float (&norm)[NP]) {
+    float x[NP][DIM > 0 ? DIM : 1], ss[NP], part[NP][4];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        ss[p] = part[p][0] = part[p][1] = part[p][2] = part[p][3] = 0.f;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) x[p][d] = __ldg(c[p] + d);
     }
-    return __fadd_rn(__fadd_rn(__fadd_rn(part[0], part[1]), part[2]), part[3]);
-}
-__device__ __forceinline__ float ordering_norm(const float* __restrict__ c, int dim) {
-    float ss = 0.f;
-    for (int d = 0; d < dim; ++d) { const float x = __ldg(c + d); ss = fmaf(x, x, ss); }
-    return sqrtf(ss);
+    if (DIM > 0) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) ss[p] = fmaf(x[p][d], x[p][d], ss[p]);
+    } else {
+        for (int d = 0; d < dim; ++d)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) { const float v = __ldg(c[p] + d); ss[p] = fmaf(v, v, ss[p]); }
+    }
+    auto hashes = [&](int j0) {
+        constexpr int U = NH > 0 ? NH : 4;
+        float acc[NP][U];
+        auto project = [&](int d, int p, float v, const float4& a) {
+            const float w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc[p][u] = d == 0 ? __fmul_rn(v, w[u]) : __fadd_rn(acc[p][u], __fmul_rn(v, w[u]));
+        };
+        const float4* ap = reinterpret_cast<const float4*>(s_alpha + j0);
+        if (DIM > 0) {
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                const float4 a = ap[d * (nh4 >> 2)];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) project(d, p, x[p][DIM > 0 ? d : 0], a);
+            }
+        } else {
+            for (int d = 0; d < dim; ++d) {
+                const float4 a = ap[d * (nh4 >> 2)];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) project(d, p, __ldg(c[p] + d), a);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (NH > 0 || j0 + u < nh) {
+                const float w = hash_weight(j0 + u);
+#pragma unroll
+                for (int p = 0; p < NP; ++p) part[p][u] = __fadd_rn(part[p][u], __fmul_rn(acc[p][u], w));
+            }
+    };
+    if (NH > 0) hashes(0);
+    else for (int j0 = 0; j0 < nh; j0 += 4) hashes(j0);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        norm[p] = sqrtf(ss[p]);
+        key[p] = __fadd_rn(__fadd_rn(__fadd_rn(part[p][0], part[p][1]), part[p][2]), part[p][3]);
+    }
 }
 
 template <int DIM, int NH>
@@ -508,19 +553,24 @@ ordering_rank_kernel(const float* __restrict__ coords, const float* __restrict__
                      const uint32_t* __restrict__ points, int row_words, int n, int64_t* __restrict__ idx,
                      uint32_t* __restrict__ ordered) {
     extern __shared__ __align__(16) unsigned char order_smem[];
-    uint64_t* comp = reinterpret_cast<uint64_t*>(order_smem);      // [n]: key, norm
-    float* s_alpha = reinterpret_cast<float*>(comp + n);
+    const int nh4 = NH > 0 ? 4 : (nh + 3) & ~3;
+    float* s_alpha = reinterpret_cast<float*>(order_smem);
+    uint64_t* comp = reinterpret_cast<uint64_t*>(s_alpha + dim * nh4);      // [n]: key, norm
     __shared__ int s_pos[ORDER_POINTS];
     const int tid = threadIdx.x;
     const int64_t s0 = (int64_t)blockIdx.y * n;
-    for (int i = tid; i < dim * nh; i += ORDER_THREADS) s_alpha[i] = alpha[i];
+    stage_alpha(alpha, dim, nh, nh4, s_alpha);
     __syncthreads();
-    for (int i = tid; i < n; i += ORDER_THREADS) {
-        const float* c = coords + (s0 + i) * dim;
-        float key, norm;
-        if (DIM > 0) ordering_key_norm_fixed<(DIM > 0 ? DIM : 1), NH>(c, s_alpha, key, norm);
-        else { key = ordering_key(c, dim, s_alpha, nh); norm = ordering_norm(c, dim); }
-        comp[i] = ((uint64_t)order_bits(key) << 32) | order_bits(norm);
+    constexpr int NP = 2;
+    for (int i0 = tid; i0 < n; i0 += NP * ORDER_THREADS) {
+        const float* c[NP];
+        float key[NP], norm[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) c[p] = coords + (s0 + min(i0 + p * ORDER_THREADS, n - 1)) * dim;
+        ordering_key_norm<DIM, NH, NP>(c, dim, s_alpha, nh, nh4, key, norm);
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            if (i0 + p * ORDER_THREADS < n) comp[i0 + p * ORDER_THREADS] = ((uint64_t)order_bits(key[p]) << 32) | order_bits(norm[p]);
     }
     __syncthreads();
     const int p = blockIdx.x * ORDER_POINTS + (tid >> 3), part = tid & 7;
@@ -547,17 +597,31 @@ ordering_rank_kernel(const float* __restrict__ coords, const float* __restrict__
     }
 }
 
+template <int DIM>
 __global__ void __launch_bounds__(256)
 ordering_keys_kernel(const float* __restrict__ coords, const float* __restrict__ alpha, int dim, int nh, int64_t n,
                      float* __restrict__ keys, float* __restrict__ norms) {
     extern __shared__ __align__(16) unsigned char order_smem[];
     float* s_alpha = reinterpret_cast<float*>(order_smem);
-    for (int i = threadIdx.x; i < dim * nh; i += 256) s_alpha[i] = alpha[i];
+    const int nh4 = (nh + 3) & ~3;
+    stage_alpha(alpha, dim, nh, nh4, s_alpha);
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
-    keys[i] = ordering_key(coords + i * dim, dim, s_alpha, nh);
-    norms[i] = ordering_norm(coords + i * dim, dim);
+    const float* const c[1] = {coords + i * dim};
+    float key[1], norm[1];
+    ordering_key_norm<DIM, 0, 1>(c, dim, s_alpha, nh, nh4, key, norm);
+    keys[i] = key[0];
+    norms[i] = norm[0];
+}
+
+// The copy for a coordinate and a hash count: both known to the compiler up to 8 and 4, then the coordinates alone, then neither.
+using OrderKernel = void (*)(const float*, const float*, int, int, const uint32_t*, int, int, int64_t*, uint32_t*);
+template <int... D>
+static OrderKernel order_kernel(int dim, int nh, std::integer_sequence<int, D...>) {
+    static const OrderKernel some[ORDER_REGS][ORDER_HASHES + 1] = {{ordering_rank_kernel<D + 1, 0>, ordering_rank_kernel<D + 1, 1>, ordering_rank_kernel<D + 1, 2>,
+                                                                    ordering_rank_kernel<D + 1, 3>, ordering_rank_kernel<D + 1, 4>}...};
+    return dim <= ORDER_REGS ? some[dim - 1][nh <= ORDER_HASHES ? nh : 0] : ordering_rank_kernel<0, 0>;
 }
 
 }  // namespace lampa
@@ -635,10 +699,10 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
     lampa_lsh_ordering_workspace_bytes(B, n, &need);
     if (ws_bytes < need || ((uintptr_t)ws & 15)) return LAMPA_ERR_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
-    const int params = dim * num_hashes * 4;
+    const int params = dim * ((num_hashes + 3) & ~3) * 4;
     if (ordering_counts(B, n) && row_bytes <= (1 << 20)) {
         const int smem = (int)n * 8 + params;
-        auto kernel = dim == 6 && num_hashes == 3 ? ordering_rank_kernel<6, 3> : ordering_rank_kernel<0, 0>;    // the layer's default, and any other
+        const OrderKernel kernel = order_kernel(dim, num_hashes, std::make_integer_sequence<int, ORDER_REGS>());
         if (smem > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return LAMPA_ERR_CUDA;
         ProfScope prof("lsh_ordering", st);
@@ -656,7 +720,13 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
     void* sws = (char*)by_norm + align_up((size_t)total * 8, 256);
     {
         ProfScope prof("lsh_ordering_keys", st);
-        ordering_keys_kernel<<<(unsigned)((total + 255) / 256), 256, params, st>>>(coords, alpha, dim, num_hashes, total, keys, norms);
+        using Kernel = void (*)(const float*, const float*, int, int, int64_t, float*, float*);
+        static const Kernel kernels[] = {ordering_keys_kernel<0>, ordering_keys_kernel<1>, ordering_keys_kernel<2>, ordering_keys_kernel<3>, ordering_keys_kernel<4>,
+                                         ordering_keys_kernel<5>, ordering_keys_kernel<6>, ordering_keys_kernel<7>, ordering_keys_kernel<8>};
+        const Kernel kernel = kernels[dim <= ORDER_REGS ? dim : 0];
+        if (params > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, params) != cudaSuccess)
+            return LAMPA_ERR_CUDA;
+        kernel<<<(unsigned)((total + 255) / 256), 256, params, st>>>(coords, alpha, dim, num_hashes, total, keys, norms);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     int rc = lampa_segsort_stable(norms, LAMPA_KEY_F32, total, nullptr, B, nullptr, by_norm, sws, sort, status, stream);

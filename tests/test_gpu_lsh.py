@@ -172,3 +172,11 @@ def test_ordering_layer_with_keys_of_its_own(lb):
     ordered, idx = layer(points, coords)
     want = layer.bucket_keys(coords).sort(dim=1, stable=True).indices      # distinct keys: the norms break no tie
     assert torch.equal(idx, want) and torch.equal(ordered, points.gather(1, want[..., None].expand(-1, -1, 5)))
+
+
+@pytest.mark.parametrize("n", [300, 8200])                        # counting, and two radix sorts
+@pytest.mark.parametrize("C,nh", [(1, 4), (2, 5), (4, 2), (5, 8), (7, 1), (8, 9), (9, 3), (12, 4), (3100, 1)])
+def test_ordering_layer_widths(lb, n, C, nh):
+    """Coordinate counts on both sides of what stays in registers (8) and the widest projections (shared memory beyond 48 KB),
+    hash counts around the groups of four."""
+    test_ordering_layer_sizes(lb, 1, n, C, 2, nh)
