@@ -21,7 +21,7 @@ namespace lampa {
 // block that keeps a sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
 // beyond 1024 chunks there are blocks enough to fill the GPU, and smaller ones would only add composites to move.
 // The choice depends on the sequence alone, never on what else a call carries, so that a sequence's result does not.
-constexpr int BLOCK_CHUNKS = 32, BLOCK_LOG = 5;      // largest block
+constexpr int BLOCK_LOG = 5;                         // largest block: 32 chunks
 constexpr int MIN_BLOCK_LOG = 3;                     // smallest
 __host__ __device__ __forceinline__ int block_log(int nch) { return nch <= 256 ? 3 : (nch <= 512 ? 4 : BLOCK_LOG); }
 __host__ __device__ __forceinline__ int blocks_of(int nch) { const int bl = block_log(nch); return (nch + (1 << bl) - 1) >> bl; }

@@ -220,7 +220,7 @@ extern "C" int lampa_gdn_workspace_layout(const lampa_gdn_desc* d, size_t out[12
     else if (d->K == 32) { using R = Rec<32, 32>; m = R::M_OFF; bt = R::BT_OFF; qt = R::QT_OFF; ol = R::OL_OFF; lam = R::LAM_OFF; }
     else { using R = Rec<16, 32>; m = R::M_OFF; bt = R::BT_OFF; qt = R::QT_OFF; ol = R::OL_OFF; lam = R::LAM_OFF; }
     out[0] = l.off_rec; out[1] = l.rec_bytes; out[2] = m; out[3] = bt; out[4] = qt; out[5] = ol; out[6] = lam;
-    out[7] = (size_t)l.LC; out[8] = (size_t)l.nc_max; out[9] = (size_t)BLOCK_CHUNKS;
+    out[7] = (size_t)l.LC; out[8] = (size_t)l.nc_max; out[9] = d->nseq > 0 ? 0 : (size_t)1 << block_log((d->T + CHUNK - 1) / CHUNK);
     out[10] = l.off_blk; out[11] = l.off_entry;
     return LAMPA_OK;
 }

@@ -39,6 +39,9 @@ def test_host_side_argument_errors_without_a_gpu():
     lay = (ctypes.c_size_t * 12)()
     assert lib.lampa_gdn_workspace_layout(ctypes.byref(ok), lay) == 0
     assert lay[1] % 128 == 0 and lay[7] == 10 and lay[9] == 32
+    for T, nseq, chunks in ((64, 0, 8), (256 * 64, 0, 8), (256 * 64 + 1, 0, 16), (512 * 64, 0, 16), (512 * 64 + 1, 0, 32), (61440, 3, 0)):
+        d = _lib.GdnDesc(B=1, T=T, H=8, K=64, V=64, L=17, nseq=nseq, qkv_dtype=0, gb_dtype=2, lam_dtype=0, use_l2norm=1, scale=0.1)
+        assert lib.lampa_gdn_workspace_layout(ctypes.byref(d), lay) == 0 and lay[9] == chunks, (T, nseq)
     assert lib.lampa_segsort_workspace_bytes(-1, ctypes.byref(n)) == -1
     assert lib.lampa_lsh_hash(None, 24, 0, None, None, 1.0, 10, 8, 3, 6, None, None, None, None) == -1
     assert lib.lampa_permute_rows(None, None, None, 1, 10, 6, 0, None, None, None) == -1            # row bytes not /4
