@@ -198,10 +198,6 @@ def check_status(dev: Optional[torch.device] = None) -> None:
                              f"(code {vals[0]}, where {vals[1]}, detail {vals[2]})")
 
 
-def debug_checks() -> bool:
-    return os.environ.get("LAMPA_B200_CHECK", "0") not in ("", "0")
-
-
 def profile_enable(on: bool) -> None:
     """Turn per-kernel CUDA-event timing inside the library on or off (clears earlier records)."""
     check(lib().lampa_profile_enable(int(on)), "lampa_profile_enable")

@@ -37,10 +37,6 @@ __device__ __forceinline__ void unpack_vec(const uint4& u, float (&x)[Vec16<DT>:
     }
 }
 template <int DT>
-__device__ __forceinline__ void load_vec(const void* p, size_t elem, float (&x)[Vec16<DT>::N]) {
-    unpack_vec<DT>(__ldg(reinterpret_cast<const uint4*>((const char*)p + elem * (DT == LAMPA_F32 ? 4 : 2))), x);
-}
-template <int DT>
 __device__ __forceinline__ void store_vec(void* p, size_t elem, const float (&x)[Vec16<DT>::N]) {
     uint4 u;
     if (DT == LAMPA_F32) {
