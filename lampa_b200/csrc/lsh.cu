@@ -284,10 +284,14 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
 
         // (c) stable scatter, tile by tile in slice order
         for (int64_t t0 = lo; t0 < hi; t0 += TILE) {
+            // A slice of several tiles reads its keys twice, for the histogram and here.  Segments that overlap (offsets that
+            // fall: the segment in between reports them) rewrite each other's keys in between, and the counts no longer add
+            // up: a tile whose keys would land behind the segment is not written.
+            bool outside = false;
             if (!one_tile) {
                 load_tile(t0, p, ksrc, isrc, gmn);
                 rank_tile(t0);
-                __syncthreads();
+                outside = __syncthreads_or(tid < 256 && (int64_t)dbase[tid] + tile_tot[tid] > n);
             }
             const uint32_t ts = prefix256(tid < 256 ? tile_tot[tid] : 0u, wtot, tid);
             if (tid < 256) tstart[tid] = ts;
@@ -303,7 +307,7 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                     sidx[lp] = idx[it];
                 }
             __syncthreads();
-            const int ntile = (int)min((int64_t)TILE, hi - t0);
+            const int ntile = outside ? 0 : (int)min((int64_t)TILE, hi - t0);
 #pragma unroll
             for (int it = 0; it < ITEMS; ++it) {
                 const int lp = it * SORT_THREADS + tid;
@@ -311,10 +315,6 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                     const uint32_t ku = skey[lp], ki = sidx[lp];
                     const uint32_t d = (ku >> shift) & dmask;
                     const int64_t pos = (int64_t)dbase[d] + (lp - tstart[d]);
-                    // A slice of several tiles reads its keys twice, for the histogram and here.  Segments that overlap
-                    // (offsets that fall: the segment in between reports them) rewrite each other's keys in between, and
-                    // the counts no longer add up: nothing is written outside the segment all the same.
-                    if (pos >= n) continue;
                     if (last) {
                         perm[s0 + pos] = (int64_t)ki;
                     } else {
