@@ -223,7 +223,8 @@ int lampa_segsort_workspace_bytes(int64_t n_total, size_t* bytes);
  * (models/attention/hept.py:138-143).
  *   keys: int32 or fp32 [n_total]; seg_offsets int64 [nseg+1] (device) or NULL for nseg equal
  *   segments of n_total/nseg keys; init: optional starting order per segment (local indices) —
- *   the result is init composed with the stable sort of keys[init], i.e. norm_idx[bk_idx].
+ *   the result is init composed with the stable sort of keys[init], i.e. norm_idx[bk_idx].  An entry outside its segment
+ *   stands for the segment's first element and sets LAMPA_ERR_BOUNDS in `status`.
  *   A segment whose offsets leave [0, n_total] is not sorted and sets LAMPA_ERR_BOUNDS in `status`.
  */
 int lampa_segsort_stable(const void* keys, int32_t key_type, int64_t n_total,

@@ -144,6 +144,26 @@ def test_sort_of_overlapping_segments_stays_inside_them(lb):
     assert bool((perm[n:] == -7).all()) and bool((ws[need.value:] == 0x5A).all())
 
 
+@pytest.mark.parametrize("n,flat", [(300, False), (60_000, False), (300, True)])
+def test_sort_starting_order_outside_its_segment(lb, n, flat):
+    """Entries of a starting order that leave their segment are reported and stand for its first element (`flat`: all keys are
+    equal and no pass is needed); the other segment is sorted as ever."""
+    from lampa_b200 import _lib as L
+    rng = np.random.default_rng(31)
+    keys = np.zeros(2 * n, np.float32) if flat else rng.standard_normal(2 * n).astype(np.float32)
+    init = np.stack([rng.permutation(n) for _ in range(2)])
+    bad = init.copy()
+    bad[1, [3, 17, n - 1]] = [n, -1, 1 << 40]
+    _status(lb)
+    got = to_np(lb.segmented_sort(torch.from_numpy(keys).cuda(), nseg=2, init=torch.from_numpy(bad.reshape(-1)).cuda()))
+    vals = _status(lb)
+    assert vals[0] == L.ERR_BOUNDS and vals[1] == 14 and vals[2] == 1
+    bad[1, [3, 17, n - 1]] = 0
+    for s in range(2):
+        k = keys[s * n:(s + 1) * n][bad[s]]
+        np.testing.assert_array_equal(got[s * n:(s + 1) * n], bad[s][np.argsort(k, kind="stable")])
+
+
 @pytest.mark.parametrize("K,hier", [(64, False), (64, True), (32, True)])
 def test_sequences_that_overlap_are_emptied(lb, K, hier):
     """Offsets that fall and rise again: a sequence that begins before an earlier offset is emptied and reported, since its
