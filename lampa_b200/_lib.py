@@ -83,6 +83,7 @@ def lib() -> ctypes.CDLL:
         L.lampa_row_range.argtypes = [vp, vp, i32, i64, vp, vp, vp, vp]
         L.lampa_quantile_regions.argtypes = [vp, vp, i32, i64, vp, vp]
         L.lampa_geo_keys.argtypes = [vp] * 8 + [i32, i64, i64, vp, vp]
+        L.lampa_geo_keys_fused.argtypes = [vp, vp, i64, vp, vp, vp, vp, i32, i64, i64, vp]
         L.lampa_bucket_rbf_attn.argtypes = [vp] * 5 + [i32, i32, i64, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]
         L.lampa_bucket_attn_combine.argtypes = [vp, vp, i32, i64, i32, vp, vp]
         L.lampa_hept_prep_qk.argtypes = [vp] * 5 + [i64, i32, i32, i32, i32, i64, vp, vp, vp, vp]

@@ -86,6 +86,9 @@ quantile_regions_kernel(const int64_t* __restrict__ rank, const float* __restric
         out[(size_t)r * n + i] = region_of(rk, region_size_of(n, num_regions[r]));
 }
 
+// The same for ranks of n < 2^31 hits by a 32-bit division: no rank reaches n, so a larger region is one of n hits.
+__device__ __forceinline__ uint32_t region_size32(int64_t n, float num_regions) { return (uint32_t)min(region_size_of(n, num_regions), n); }
+
 // out[r][i] = proj[r][i] (+inf for padded hits, 0 when proj is NULL) + shift[r][i]
 __global__ void __launch_bounds__(GEO_THREADS)
 geo_keys_kernel(const float* __restrict__ proj, const float* __restrict__ reg_eta,
@@ -136,11 +139,10 @@ geo_keys_fused_kernel(float* __restrict__ proj, const float2* __restrict__ part,
 #pragma unroll
     for (int w = 0; w < 16; ++w) { mn = fminf(mn, smn[w]); mx = fmaxf(mx, smx[w]); }
     const float hs = __fsub_rn(mx, mn), ne = regions_eta[r], np = regions_phi[r], stride = __fadd_rn(ceilf(ne), 1.f);
-    const int64_t se = region_size_of(n, ne), sp = region_size_of(n, np);
+    const uint32_t se = region_size32(n, ne), sp = region_size32(n, np);
     const int64_t end = min((int64_t)(blockIdx.x + 1) * GEO_CHUNK, n);
     for (int64_t i = (int64_t)blockIdx.x * GEO_CHUNK + tid; i < end; i += 512) {
-        // ranks and region sizes are below 2^31 for any n the sort takes at once: a 32-bit division
-        const float e = (float)((uint32_t)rank_eta[i] / (uint32_t)se) + 1.f, p = (float)((uint32_t)rank_phi[i] / (uint32_t)sp) + 1.f;
+        const float e = (float)((uint32_t)rank_eta[i] / se) + 1.f, p = (float)((uint32_t)rank_phi[i] / sp) + 1.f;
         const float shift = __fadd_rn(__fmul_rn(__fmul_rn(p, hs), stride), __fmul_rn(e, hs));
         const size_t at = (size_t)r * n + i, at2 = at + (size_t)rows * n;
         proj[at] = __fadd_rn(i < raw_size ? proj[at] : INFINITY, shift);
@@ -179,7 +181,7 @@ region_numbers_kernel(const int64_t* __restrict__ rank, const float* __restrict_
     const int a = blockIdx.y;
     if (i >= n) return;
     const uint32_t rk = (uint32_t)rank[a * n + i];
-    for (int r = 0; r < rows; ++r) out[((size_t)a * rows + r) * n + i] = (float)(rk / (uint32_t)region_size_of(n, regions_h[a * rows + r])) + 1.f;
+    for (int r = 0; r < rows; ++r) out[((size_t)a * rows + r) * n + i] = (float)(rk / region_size32(n, regions_h[a * rows + r])) + 1.f;
 }
 
 }  // namespace lampa

@@ -109,3 +109,31 @@ def test_against_numpy_checker(lb, n_raw, block, heads, rounds):
     code = rp * (np.ceil(regions_h[0])[:, None] + 1) + re
     along = np.take_along_axis(code, to_np(qpos).reshape(-1, n), 1)[:, :n_raw]
     assert (np.diff(along, axis=1) >= 0).all()
+
+
+@pytest.mark.parametrize("n", [1, 1000, 5000])
+def test_regions_larger_than_the_event(lb, n):
+    """Region counts far below one: regions of 2^32 hits and more are one region of all hits, in the numbers and in the fused
+    keys (both divide in 32 bits) as in the general key pass."""
+    from lampa_b200 import _lib as L
+    gen = torch.Generator().manual_seed(n)
+    coords = torch.randn(n, 2, generator=gen)
+    counts = torch.tensor([n * 2.0 ** -32, n * 2.0 ** -33, 1e-6, 0.5, 0.0, 7.0 + 1 / 3])
+    regions = torch.stack([counts, counts.flip(0)]).view(1, 2, -1)                 # [c, a, h]
+    inp = lb.region_inputs(coords.cuda(), regions.cuda(), 1)
+    for a in range(2):
+        got = to_np(inp["region_indices"][a])
+        np.testing.assert_array_equal(got, oracle.quantile_regions(oracle.segsort(coords[:, a].numpy().copy()), regions[0, a].numpy()))
+    rows, dev = counts.numel(), torch.device("cuda:0")
+    proj = torch.randn(2, rows, n, generator=gen).to(dev)
+    re, rp = (inp["regions_h"][a].contiguous() for a in range(2))
+    both = proj.permute(1, 0, 2).reshape(rows, -1)
+    part = torch.stack([both.amin(1), both.amax(1)], -1).contiguous()             # one block of (min, max) per row
+    hs = (part[:, 1] - part[:, 0]).contiguous()
+    want = torch.empty_like(proj)
+    ranks = [L.ptr(r) for r in inp["ranks"]]
+    for x in range(2):
+        L.check(L.lib().lampa_geo_keys(L.ptr(proj[x]), None, None, *ranks, L.ptr(re), L.ptr(rp), L.ptr(hs), rows, n, n, L.ptr(want[x]),
+                                       L.stream_ptr(dev)), "lampa_geo_keys")
+    L.check(L.lib().lampa_geo_keys_fused(L.ptr(proj), L.ptr(part), 1, *ranks, L.ptr(re), L.ptr(rp), rows, n, n, L.stream_ptr(dev)), "lampa_geo_keys_fused")
+    np.testing.assert_array_equal(to_np(proj), to_np(want))
