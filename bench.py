@@ -909,19 +909,13 @@ def run_hept(args):
     ms = out["bucket_rbf_attn"]["us_per_launch"] * 1e-3
     out["bucket_rbf_attn"]["fp32_tflops"] = flops / (ms * 1e-3) / 1e12
     total_ms = sum(o["us_per_launch"] for o in out.values()) * 1e-3
-    # fp32 FMA bound: no measured fp32 peak is written by the driver, so the denominator is the nominal
-    # 148 SMs x 128 FMA lanes x 2 flop x the maximum SM clock reported by NVML (1965 MHz on this pool)
-    try:
-        import pynvml
-        pynvml.nvmlInit()
-        mhz = float(pynvml.nvmlDeviceGetMaxClockInfo(pynvml.nvmlDeviceGetHandleByIndex(dev.index or 0),
-                                                     pynvml.NVML_CLOCK_SM))
-    except Exception:
-        mhz = 1965.0
-    peak = 148 * 128 * 2 * mhz * 1e6 / 1e12
-    roof = {"kernel": "bucket_rbf_attn", "bound": "fp32-fma", "achieved": out["bucket_rbf_attn"]["fp32_tflops"],
+    # rows of at most 32 features run on the tensor cores, each fp32 product as six bf16 products
+    pk = peaks()
+    peak = pk["bf16_tflops"] / 6
+    roof = {"kernel": "bucket_rbf_attn", "bound": "tensor", "achieved": out["bucket_rbf_attn"]["fp32_tflops"],
             "peak": peak, "unit": "TFLOP/s", "frac": out["bucket_rbf_attn"]["fp32_tflops"] / peak,
-            "peak_source": "nominal (SMs x lanes x 2 x max SM clock)", "traffic": 310.0e6 if n == 60000 else None}
+            "peak_source": pk["source"] + " bf16 over the six products of an fp32 one",
+            "traffic": profile_traffic().get("bucket_rbf_attn") if n == 60000 else None}
     print(json.dumps({"metric": "hits/sec, HEPT bucket attention", "value": n / (total_ms * 1e-3), "unit": "hits/s",
                       "roofline": roof,
                       "n_gpus": 1, "steps": args.steps, "dtype": "f32", "data": "synthetic",

@@ -113,10 +113,10 @@ __device__ __forceinline__ void pack_a(uint32_t (&f)[4], const float (&c0)[4], c
     f[3] = pack_bf16x2(c1[2], c1[3]);
 }
 
-// Bound by the shared-memory pipe (63 % busy) and issue slots (47 %) at head dims up to 32.  Every product is formed 16
-// columns at a time and products over the same fragments (K: KK^T and QK^T, Q~ and W; V: O_local and U^) share the pass:
-// whole 64-wide accumulators held it at 96 registers and five CTAs per SM.  Four packed sequences of 12,001 to 90,001
-// tokens, 6 heads, K = 16, V = 32: 319 -> 246 us.
+// Bound by the shared-memory pipe and issue slots at head dims up to 32 (69 and 58 % busy at K = 16, V = 32; 64 and 47 %
+// at K = V = 32 with levels).  Every product is formed 16 columns at a time and products over the same fragments (K: KK^T
+// and QK^T, Q~ and W; V: O_local and U^) share the pass: whole 64-wide accumulators held it at 96 registers and five CTAs
+// per SM.  Four packed sequences of 12,001 to 90,001 tokens, 6 heads, K = 16, V = 32: 319 -> 246 us.
 template <int KD, int VD, bool HIER>
 __global__ void __launch_bounds__(128, KD == 64 ? 4 : 6) gdn_prep_kernel(GdnArgs a) {
     using S = PrepSmem<KD, VD>;

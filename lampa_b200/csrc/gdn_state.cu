@@ -55,9 +55,10 @@ __device__ __forceinline__ void load8_as_float(const void* p, size_t i, int dt, 
 //
 // State columns are independent, so a half-warp owns one: lane kl has rows kl, kl + 16, ... of every
 // level in registers, a level's k^T S is K / 16 FMAs and four shuffles, and the levels of a token
-// are independent chains that hide each other's latency.  What bounds it is that chain, ~0.2 us per
-// token; with one CTA per (sequence, head) and a launch per tail token (61 us for the token levels
-// and 27 us per tail token) a 3001-token prompt spent 1.7 of its 1.9 ms on the device here.
+// are independent chains that hide each other's latency.  What bounds it is that chain, 0.3 us per
+// token of the last whole chunk and 0.4 us per token behind it (8 heads, K = V = 64: 19 us at 2944
+// tokens, 47 us at 3001); with one CTA per (sequence, head) and a launch per tail token (61 us for the
+// token levels and 27 us per tail token) a 3001-token prompt spent 1.7 of its 1.9 ms on the device here.
 // -------------------------------------------------------------------------------------------------
 constexpr int TAIL_COLS = 8, TAIL_THREADS = 128;
 
