@@ -120,7 +120,7 @@ class ClockSampler(threading.Thread):
                 "sm_max_mhz": float(self.max_sm), "reasons": reasons, "samples": len(inside)}
 
 
-# ---- CPU restatement of the reference path (checker code, timed as the baseline) ---------------------
+# ---- CPU restatement of the reference path (oracle code, timed as the baseline) ---------------------
 def cpu_pass(ev, n_tokens: int):
     """One pass of the path over the first n_tokens hits on the host cores; returns seconds."""
     from oracle import oracle
@@ -626,7 +626,7 @@ def model_measure(ms_, dev, rank, world, steps, warmup, e2e=True, profile=True):
 
 
 def model_cpu_baseline(n_hits=6000):
-    """The CPU statement of the model (tests/model_oracle.py over the CPU checker) on one small event."""
+    """The CPU statement of the model (tests/model_oracle.py over the CPU oracle) on one small event."""
     from lampa_b200 import synth
     from lampa_b200.model import LSHGatedDelta
     from oracle import oracle

@@ -18,7 +18,7 @@ namespace lampa {
 // -------------------------------------------------------------------------------------------------
 // Hash: one thread per hit.  Reads dim floats of the hit's row (for the detector rows of this
 // workload 24 B of a 96 B row: one 32 B sector) and writes rounds*heads ids, each coalesced across
-// the warp.  The operation order is a contract shared with the CPU checker (see the header).
+// the warp.  The operation order is a contract shared with the CPU oracle (see the header).
 // -------------------------------------------------------------------------------------------------
 constexpr int HASH_THREADS = 256;
 constexpr int HASH_MAX_PARAMS = 4096;   // heads*dim*rounds floats staged in shared memory

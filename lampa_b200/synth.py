@@ -5,7 +5,7 @@ available offline, so these generators stand in for it: hits on 10 cylindrical l
 (r = 30..1000 mm, phi ~ U(-pi, pi), z ~ U(-3000, 3000) mm) with a 24-float feature row
 [x, y, z, r, phi, eta, 18 x N(0,1)], and mixer inputs drawn as the benchmark configuration
 states (unit-norm q/k, v ~ N(0,1), beta = sigmoid(N), g = -softplus(N + shift), lambda = softplus(N)).
-Everything is drawn on the CPU from one torch.Generator so the CPU checker and the GPU see the
+Everything is drawn on the CPU from one torch.Generator so the CPU oracle and the GPU see the
 same numbers.
 """
 from __future__ import annotations

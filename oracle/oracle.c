@@ -2,7 +2,7 @@
  * TEST INFRASTRUCTURE ONLY — CPU restatement of the reference's algorithms for the
  * LSH ordering + (hierarchical) gated-delta forward path.  Nothing in the product
  * package may link or call this file; it exists so that tests, the smoke check and
- * the CPU-baseline leg of the benchmark have an independent checker.
+ * the CPU-baseline leg of the benchmark have an independent oracle.
  *
  * Parity status: pinned.  The reference ships no golden vectors for this path, so
  * the pin is against outputs of the reference's own pure-PyTorch code

@@ -1,6 +1,6 @@
 """CPU statement of lampa_b200.model.LSHGatedDelta for the parity tests: the same module's
 weights, torch on the CPU for the host-side layers (Linear, RMS norm, GELU) with the GPU's bf16
-rounding points, and the CPU checker (oracle/) in place of every library op."""
+rounding points, and the CPU oracle (oracle/) in place of every library op."""
 import numpy as np
 import torch
 import torch.nn.functional as F

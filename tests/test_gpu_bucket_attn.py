@@ -1,7 +1,7 @@
-"""GPU parity of the HEPT bucket attention through the C ABI, against the float64 checker and the
+"""GPU parity of the HEPT bucket attention through the C ABI, against the float64 oracle and the
 reference-generated fixture.
 
-Tolerance (fp32 kernel, float64 checker): |got - ref| <= 2e-5 * max(1, |ref|_inf) elementwise for
+Tolerance (fp32 kernel, float64 oracle): |got - ref| <= 2e-5 * max(1, |ref|_inf) elementwise for
 the weighted sums, relative 2e-5 for the denominators, 5e-5 for the quotient.  The exponent
 q.k - |q|^2/2 - |k|^2/2 is a difference of terms of size |q|^2 ~ 10 in these inputs, so its fp32
 rounding error (a few 1e-6 absolute) is the relative error of every weight.
@@ -84,9 +84,9 @@ def test_fixture_from_reference(lb, golden_dir):
     out_p = lb.hept_bucket_attention(q_hat, k_hat, v, _c(z["q_pos"]), _c(z["k_pos"]), block)
     _close(to_np(out_p), z["out"], 5e-5, "out from padded rows vs reference")
     ref_out, ref_o, ref_lg = oracle.hept_bucket_attention(z["q_hat"], z["k_hat"], z["v"], z["q_pos"], z["k_pos"], block)
-    _close(to_np(o), ref_o, 2e-5, "o vs checker")
-    _close_rel(to_np(lg), ref_lg, 2e-5, "logits vs checker")
-    _close(to_np(out), ref_out, 5e-5, "out vs checker")
+    _close(to_np(o), ref_o, 2e-5, "o vs oracle")
+    _close_rel(to_np(lg), ref_lg, 2e-5, "logits vs oracle")
+    _close(to_np(out), ref_out, 5e-5, "out vs oracle")
 
 
 CASES = [
@@ -165,7 +165,7 @@ def test_identical_points_and_far_points(lb):
 
 def test_attention_core_end_to_end(lb):
     """The layer's forward between the projections and the output projection: input preparation, region
-    shift, bucket orders and attention in one call, against the checker run on the positions the call
+    shift, bucket orders and attention in one call, against the oracle run on the positions the call
     itself produced (the positions have their own parity tests)."""
     raw, block, heads, rounds, d, cd, nw = 1130, 100, 4, 3, 24, 6, 5
     gen = torch.Generator().manual_seed(99)

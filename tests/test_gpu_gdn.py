@@ -1,4 +1,4 @@
-"""GPU parity of the gated-delta forward ops (through the C ABI) against the CPU checker.
+"""GPU parity of the gated-delta forward ops (through the C ABI) against the CPU oracle.
 
 Tolerance (bf16 operands, fp32 accumulation, against the fp32 token recurrence):
 max-abs <= 2e-2 * max(1, |ref|_inf) and relative L2 <= 1e-2.
@@ -207,7 +207,7 @@ def test_hier_golden_fixture_from_reference(lb, golden_dir):
         t = {k: torch.from_numpy(z[k])[None].cuda() for k in ("q", "k", "v", "g", "beta", "lam")}
         o, _ = lb.chunk_h_gated_delta_rule(t["q"].bfloat16(), t["k"].bfloat16(), t["v"].bfloat16(), t["g"], t["lam"],
                                            t["beta"], use_qk_l2norm_in_kernel=True)
-        # fixture inputs are fp32; compare against the checker on the bf16-rounded inputs and,
+        # fixture inputs are fp32; compare against the oracle on the bf16-rounded inputs and,
         # more loosely, against the reference's fp32 output itself
         ref_r = oracle.hgdn(to_np(t["q"].bfloat16()[0]), to_np(t["k"].bfloat16()[0]), to_np(t["v"].bfloat16()[0]),
                             z["g"], z["beta"], z["lam"], use_l2norm=True)[0]

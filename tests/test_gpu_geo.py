@@ -1,5 +1,5 @@
 """GPU parity of the region (geo) shift path through the C ABI: bit-exact against the numpy
-checker and the reference-generated fixture for ranks, regions, ranges, shifts and keys;
+oracle and the reference-generated fixture for ranks, regions, ranges, shifts and keys;
 positions agree wherever keys do not tie."""
 import os
 
@@ -87,7 +87,7 @@ def test_against_numpy_checker(lb, n_raw, block, heads, rounds):
     q = torch.zeros(heads, n, dim); q[:, :n_raw] = torch.randn(heads, n_raw, dim, generator=gen)
     k = torch.zeros(heads, n, dim); k[:, :n_raw] = torch.randn(heads, n_raw, dim, generator=gen)
     e2 = lb.E2LSH(n_hashes=rounds, n_heads=heads, dim=dim).cuda()
-    # checker
+    # oracle
     padded = np.full((n, 2), np.inf, np.float32); padded[:n_raw] = coords.numpy()
     se, sp = oracle.segsort(padded[:, 0]), oracle.segsort(padded[:, 1])
     regions_h = regions.numpy().transpose(1, 0, 2).reshape(2, -1)

@@ -1,5 +1,5 @@
 """GPU parity of the layer's producers / consumers (short convolution, gate inputs, gated RMS
-norm) through the C ABI, against the numpy checker and the reference-generated fixture.
+norm) through the C ABI, against the numpy oracle and the reference-generated fixture.
 
 Tolerance: fp32 storage 1e-5 (relative + absolute; the kernels use the fast exp); bf16 storage:
 one bf16 ulp of the fp32 result (2^-8 relative) plus 1e-3 absolute.

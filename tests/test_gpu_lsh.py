@@ -1,4 +1,4 @@
-"""GPU parity of the ordering kernels (through the C ABI) against the CPU checker: bit-exact."""
+"""GPU parity of the ordering kernels (through the C ABI) against the CPU oracle: bit-exact."""
 import os
 
 import numpy as np

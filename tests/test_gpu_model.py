@@ -1,5 +1,5 @@
 """GPU parity of the packed, event-sharded model forward (benchmark configuration 4) against its
-CPU statement (tests/model_oracle.py: the same weights, the CPU checker for every library op).
+CPU statement (tests/model_oracle.py: the same weights, the CPU oracle for every library op).
 
 Orderings: bit-exact.  Every block alone, fed with the CPU statement's own input to that block:
 the op tolerance (max-abs 2e-2, see tests/util.max_abs_bound, and relative L2 1e-2).  The whole

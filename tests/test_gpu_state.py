@@ -1,5 +1,5 @@
 """GPU parity of the hierarchical rule's Fenwick state (prefill final state and decode step),
-through the C ABI, against the CPU checker's token recurrence.
+through the C ABI, against the CPU oracle's token recurrence.
 
 Outputs: the bf16 tolerance of the forward tests (tests/util.assert_close_bf16).
 States: the whole tensor [H, K, V, L] within max-abs 2e-2 of its largest value and relative L2
@@ -37,7 +37,7 @@ def _cuda(d):
 
 
 def _close_level(got, ref, what, floor):
-    """One level against the checker, rescaled first (strongly decayed levels sit near 1e-30,
+    """One level against the oracle, rescaled first (strongly decayed levels sit near 1e-30,
     where squaring for the L2 norm would underflow)."""
     m = max(float(np.abs(ref).max()), floor)
     if m < 1e-35:

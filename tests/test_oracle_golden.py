@@ -33,7 +33,7 @@ def test_hier_and_plain_match_reference_recurrence(golden_dir, name):
 def test_hier_matches_reference_chunkwise_statement(golden_dir):
     """Second pin: the reference's own chunkwise statement (hgdn_minimal, hssd_minimal.py:462-493)
     at T = 4096 -- 64 chunks, two blocks of 32, one cross-block level -- against the token
-    recurrence of the checker, both fp32."""
+    recurrence of the oracle, both fp32."""
     from tests.util import minimal_fixture_inputs
     z = np.load(os.path.join(golden_dir, "hgdn_minimal_T4096_H2_K32_V32_L13.npz"))
     q, k, v, beta, g, lam = (x.numpy() for x in minimal_fixture_inputs(z))

@@ -30,7 +30,7 @@ def max_abs_bound(rmax: float) -> float:
 
 
 def assert_close_bf16(got, ref, what="", max_abs_factor: float = 1.0):
-    """Tolerance of the build target for bf16 runs against the fp32 checker: max-abs <= 2e-2
+    """Tolerance of the build target for bf16 runs against the fp32 oracle: max-abs <= 2e-2
     (see max_abs_bound for values above 2) and relative L2 <= 1e-2."""
     mx, rl = err_stats(got, ref)
     rmax = float(np.abs(ref).max())
