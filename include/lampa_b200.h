@@ -415,6 +415,12 @@ int lampa_bucket_rbf_attn(const float* q, const float* k, const float* v, const 
                           const int64_t* k_pos, int32_t rounds, int32_t heads, int64_t n, int32_t bucket,
                           int32_t dq, int32_t dv, int32_t ldq, int32_t ldv, int32_t inputs_per_round,
                           int32_t scatter, float* so, float* denom, void* stream);
+/* The same with a status word: a position outside [0, n) sets LAMPA_ERR_BOUNDS.  In either form such a hit
+ * stands for hit 0: nothing is read or written outside the arrays, and the rows of its bucket and of hit 0 are undefined. */
+int lampa_bucket_rbf_attn_checked(const float* q, const float* k, const float* v, const int64_t* q_pos,
+                          const int64_t* k_pos, int32_t rounds, int32_t heads, int64_t n, int32_t bucket,
+                          int32_t dq, int32_t dv, int32_t ldq, int32_t ldv, int32_t inputs_per_round,
+                          int32_t scatter, float* so, float* denom, int32_t* status, void* stream);
 /*
  * out[row][:] = (sum over rounds of so[r][row][:]) / (sum over rounds of denom[r][row]), rounds added
  * in order.  rows = heads * n.  Replaces: `o.sum(dim=0) / logits.sum(dim=0)` (hept.py:151).

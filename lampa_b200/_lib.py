@@ -43,7 +43,7 @@ EXPORTS = ["lampa_version", "lampa_error_string", "lampa_gdn_workspace_bytes", "
            "lampa_short_conv_fwd", "lampa_short_conv_step", "lampa_gate_inputs", "lampa_rmsnorm_gate", "lampa_add_rmsnorm",
            "lampa_row_range", "lampa_quantile_regions", "lampa_geo_keys",
            "lampa_hept_front_blocks", "lampa_hept_front", "lampa_geo_keys_fused", "lampa_region_inputs",
-           "lampa_bucket_rbf_attn", "lampa_bucket_attn_combine", "lampa_hept_prep_qk",
+           "lampa_bucket_rbf_attn", "lampa_bucket_rbf_attn_checked", "lampa_bucket_attn_combine", "lampa_hept_prep_qk",
            "lampa_hgdn_fwd_again", "lampa_model_encode", "lampa_model_project", "lampa_model_update", "lampa_model_head",
            "lampa_repeat_segments", "lampa_profile_enable",
            "lampa_profile_read", "lampa_debug_set_poll_budget", "lampa_debug_set_tick_buffer",
@@ -85,6 +85,7 @@ def lib() -> ctypes.CDLL:
         L.lampa_geo_keys.argtypes = [vp] * 8 + [i32, i64, i64, vp, vp]
         L.lampa_geo_keys_fused.argtypes = [vp, vp, i64, vp, vp, vp, vp, i32, i64, i64, vp]
         L.lampa_bucket_rbf_attn.argtypes = [vp] * 5 + [i32, i32, i64, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]
+        L.lampa_bucket_rbf_attn_checked.argtypes = [vp] * 5 + [i32, i32, i64, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp]
         L.lampa_bucket_attn_combine.argtypes = [vp, vp, i32, i64, i32, vp, vp]
         L.lampa_hept_prep_qk.argtypes = [vp] * 5 + [i64, i32, i32, i32, i32, i64, vp, vp, vp, vp]
         L.lampa_short_conv_fwd.argtypes = [vp, vp, vp, vp, vp, i32, i64, i64, i32, i32, i32, i32, i32, vp, vp, i32, vp]

@@ -103,8 +103,9 @@ def hept_bucket_attention(q_hat: torch.Tensor, k_hat: torch.Tensor, value: torch
     so = torch.empty(rounds, heads, n, dv, dtype=torch.float32, device=dev)
     denom = torch.empty(rounds, heads, n, 1, dtype=torch.float32, device=dev)
     s = L.stream_ptr(dev)
-    rc = L.lib().lampa_bucket_rbf_attn(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(qp), L.ptr(kp), rounds, heads, n,
-                                       int(block_size), dq, dv, ldq, ldv, 0, 1, L.ptr(so), L.ptr(denom), s)
+    rc = L.lib().lampa_bucket_rbf_attn_checked(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(qp), L.ptr(kp), rounds, heads, n,
+                                               int(block_size), dq, dv, ldq, ldv, 0, 1, L.ptr(so), L.ptr(denom),
+                                               L.ptr(L.status_word(dev)), s)
     L.check(rc, "lampa_bucket_rbf_attn")
     out = torch.empty(heads, n, dv, dtype=torch.float32, device=dev)
     L.check(L.lib().lampa_bucket_attn_combine(L.ptr(so), L.ptr(denom), rounds, heads * n, dv, L.ptr(out), s),

@@ -144,6 +144,35 @@ def test_sort_of_overlapping_segments_stays_inside_them(lb):
     assert bool((perm[n:] == -7).all()) and bool((ws[need.value:] == 0x5A).all())
 
 
+@pytest.mark.parametrize("bucket,dq,dv", [(100, 30, 24), (25, 30, 24), (50, 41, 40)])
+def test_bucket_positions_outside_the_hits(lb, bucket, dq, dv):
+    """Bucket positions that leave the hits are reported and not followed, on the tensor-core kernel and the FMA one (small
+    buckets, wide rows with whole and ragged pieces): the other buckets' rows come out as without them."""
+    from lampa_b200 import _lib as L
+    heads, n = 2, 4 * bucket
+    gen = torch.Generator().manual_seed(bucket)
+    q, k = (torch.randn(heads, n, dq, generator=gen).cuda() * 0.3 for _ in range(2))
+    v = torch.randn(heads, n, dv, generator=gen).cuda()
+    qp, kp = (torch.stack([torch.randperm(n, generator=gen) for _ in range(heads)]).unsqueeze(0).cuda() for _ in range(2))
+    want = lb.hept_bucket_attention(q, k, v, qp, kp, bucket)
+    old = os.environ.pop("LAMPA_B200_CHECK", None)
+    try:
+        assert _status(lb)[0] == 0
+        for which in (qp, kp):
+            bad = which.clone()
+            bad[0, 0, :3] = torch.tensor([n, -1, 1 << 40])              # first bucket of the first head
+            got = lb.hept_bucket_attention(q, k, v, *((bad, kp) if which is qp else (qp, bad)), bucket)
+            vals = _status(lb)
+            assert vals[0] == L.ERR_BOUNDS and vals[1] == 50 and vals[2] < 3
+            assert torch.equal(got[1], want[1])
+            others = qp[0, 0, bucket:]
+            others = others[others != 0]                               # a bad entry stands for hit 0
+            assert torch.equal(got[0][others], want[0][others])
+    finally:
+        if old is not None:
+            os.environ["LAMPA_B200_CHECK"] = old
+
+
 @pytest.mark.parametrize("n,flat", [(300, False), (60_000, False), (300, True)])
 def test_sort_starting_order_outside_its_segment(lb, n, flat):
     """Entries of a starting order that leave their segment are reported and stand for its first element (`flat`: all keys are
