@@ -94,6 +94,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Measured at 60 000 hits, 3 x 8: dq 54 / dv 48 1.25 ms with 4 rows against 1.62 with 8; dq 102 / dv 96 3.63 against 3.40.
 template <int BA_QROWS>
 __global__ void __launch_bounds__(BA_MAX_WARPS * 32, BA_QROWS == 4 ? 3 : 2) bucket_rbf_attn_kernel(BucketAttnArgs a) {
+    if (chain_wait()) return;
     extern __shared__ __align__(16) float ba_smem[];
     const int dq4 = a.dq4, pk = a.pk, pv = a.pv, bucket = a.bucket;
     const int nthr = blockDim.x, nwarps = nthr >> 5;
@@ -331,6 +332,7 @@ __host__ __device__ constexpr int bam_smem(int keys) { return 4 * 128 * 8 + keys
 
 template <int KQ, int NV>      // 16-wide feature steps of q / k, 8-wide value column tiles
 __global__ void __launch_bounds__(256, 3) bucket_attn_mma_kernel(BucketAttnArgs a) {
+    if (chain_wait()) return;
     constexpr int KP = 16 * KQ + 8, VP = 8 * ((NV + 1) & ~1) + 8;         // bf16 pitches: consecutive rows fall into different bank groups
     extern __shared__ __align__(16) float ba_smem[];
     const int bucket = a.bucket, keys = bam_keys(bucket), nthr = blockDim.x;     // nthr = 2 * keys
@@ -522,6 +524,7 @@ template <int V>
 __global__ void __launch_bounds__(256)
 bucket_attn_combine_kernel(const float* __restrict__ so, const float* __restrict__ denom, int rounds,
                            int64_t rows, int dv, float* __restrict__ out) {
+    if (chain_wait()) return;
     const int64_t total = rows * dv;
     for (int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V; e < total; e += (int64_t)gridDim.x * 256 * V) {
         const int64_t row = e / dv;
@@ -550,6 +553,7 @@ hept_prep_qk_kernel(const float* __restrict__ query, const float* __restrict__ k
                     const float* __restrict__ scale, const float* __restrict__ coords, int64_t n, int heads,
                     int d, int cd, int ldq, int64_t raw_size, float* __restrict__ q_hat, float* __restrict__ k_hat,
                     float* __restrict__ v_out) {
+    if (chain_wait()) return;
     const int dq = ldq;                       // columns d + cd .. ldq - 1 are zero padding
     const int64_t total = (int64_t)heads * n * dq;
     for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
@@ -590,6 +594,7 @@ hept_front_kernel(const float* __restrict__ query, const float* __restrict__ key
                   const float* __restrict__ scale, const float* __restrict__ coords, const float* __restrict__ alpha,
                   int64_t n, int heads, int d, int cd, int ldq, int64_t raw_size, float* __restrict__ q_hat,
                   float* __restrict__ k_hat, float* __restrict__ v_out, float* __restrict__ proj, float2* __restrict__ part) {
+    if (chain_wait()) return;
     extern __shared__ __align__(16) float hf[];
     const int hd = heads * d, P = hf_pitch(heads, d), D = d + cd;
     float* sq = hf;                             // [32][P] query rows, then key rows behind them
@@ -765,14 +770,14 @@ extern "C" int lampa_bucket_rbf_attn_checked(const float* q, const float* k, con
         const int msmem = bam_smem<2, 4>(keys);
         if (cudaFuncSetAttribute(mma, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem) != cudaSuccess) return LAMPA_ERR_CUDA;
         ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
-        mma<<<(unsigned)units, 2 * keys, msmem, (cudaStream_t)stream>>>(a);
+        launch_chained(mma, (unsigned)units, 2 * keys, msmem, (cudaStream_t)stream, a);
         return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
     }
     auto kernel = wide ? bucket_rbf_attn_kernel<8> : bucket_rbf_attn_kernel<4>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
     ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
-    kernel<<<(unsigned)units, warps * 32, smem, (cudaStream_t)stream>>>(a);
+    launch_chained(kernel, (unsigned)units, warps * 32, smem, (cudaStream_t)stream, a);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -785,8 +790,8 @@ extern "C" int lampa_bucket_attn_combine(const float* so, const float* denom, in
     const int64_t total = rows * dv;
     const bool v4 = dv % 4 == 0 && (((uintptr_t)so | (uintptr_t)out) & 15) == 0;
     const unsigned grid = (unsigned)std::min<int64_t>((total / (v4 ? 4 : 1) + 255) / 256, 148 * 32);
-    if (v4) bucket_attn_combine_kernel<4><<<grid, 256, 0, (cudaStream_t)stream>>>(so, denom, rounds, rows, dv, out);
-    else bucket_attn_combine_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(so, denom, rounds, rows, dv, out);
+    if (v4) launch_chained(bucket_attn_combine_kernel<4>, grid, 256, 0, (cudaStream_t)stream, so, denom, rounds, rows, dv, out);
+    else launch_chained(bucket_attn_combine_kernel<1>, grid, 256, 0, (cudaStream_t)stream, so, denom, rounds, rows, dv, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -800,7 +805,7 @@ extern "C" int lampa_hept_prep_qk(const float* query, const float* key, const fl
     ProfScope prof("hept_prep_qk", (cudaStream_t)stream);
     const int64_t total = (int64_t)heads * n * ldq;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    hept_prep_qk_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(query, key, value, scale, coords, n, heads, d, cd,
+    launch_chained(hept_prep_qk_kernel, grid, 256, 0, (cudaStream_t)stream, query, key, value, scale, coords, n, heads, d, cd,
                                                                  ldq, raw_size, q_hat, k_hat, v_out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
@@ -831,7 +836,7 @@ extern "C" int lampa_hept_front(const float* query, const float* key, const floa
     const K kernel = kernels[vec][rounds - 1];
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LAMPA_ERR_CUDA;
     ProfScope prof("hept_front", (cudaStream_t)stream);
-    kernel<<<(unsigned)((n + HF_HITS - 1) / HF_HITS), 256, smem, (cudaStream_t)stream>>>(query, key, value, scale, coords, alpha, n, heads, d, cd, ldq,
+    launch_chained(kernel, (unsigned)((n + HF_HITS - 1) / HF_HITS), 256, smem, (cudaStream_t)stream, query, key, value, scale, coords, alpha, n, heads, d, cd, ldq,
                                                                                         raw_size, q_hat, k_hat, v_out, proj, (float2*)part);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }

@@ -14,6 +14,7 @@ namespace lampa {
 // One CTA, a thread per sequence and a running sum over the CTA (one thread walking 64 sequences: 26 us, now 6.5).
 constexpr int PLAN_THREADS = 256;
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(PlanArgs p) {
+    if (chain_wait()) return;
     __shared__ int2 wsum[PLAN_THREADS / 32];
     __shared__ int64_t wtop[PLAN_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(PlanArgs p) {
 
 int launch_plan(const PlanArgs& p, cudaStream_t st) {
     ProfScope prof("gdn_plan", st);
-    plan_kernel<<<1, PLAN_THREADS, 0, st>>>(p);
+    launch_chained(plan_kernel, 1, PLAN_THREADS, 0, st, p);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -119,6 +120,7 @@ __device__ __forceinline__ void pack_a(uint32_t (&f)[4], const float (&c0)[4], c
 // per SM.  Four packed sequences of 12,001 to 90,001 tokens, 6 heads, K = 16, V = 32: 319 -> 246 us.
 template <int KD, int VD, bool HIER>
 __global__ void __launch_bounds__(128, KD == 64 ? 4 : 6) gdn_prep_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     using S = PrepSmem<KD, VD>;
     using R = Rec<KD, VD>;
     constexpr int KP = S::KP, VP = S::VP, CP = S::CP;
@@ -520,11 +522,11 @@ int launch_prep(const GdnArgs& a, bool hier, cudaStream_t st) {
     if (hier) {
         e = cudaFuncSetAttribute(gdn_prep_kernel<KD, VD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return LAMPA_ERR_CUDA;
-        gdn_prep_kernel<KD, VD, true><<<grid, 128, smem, st>>>(a);
+        launch_chained(gdn_prep_kernel<KD, VD, true>, grid, 128, smem, st, a);
     } else {
         e = cudaFuncSetAttribute(gdn_prep_kernel<KD, VD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return LAMPA_ERR_CUDA;
-        gdn_prep_kernel<KD, VD, false><<<grid, 128, smem, st>>>(a);
+        launch_chained(gdn_prep_kernel<KD, VD, false>, grid, 128, smem, st, a);
     }
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }

@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, 
                                                                      const __grid_constant__ CUtensorMap tk,
                                                                      const __grid_constant__ CUtensorMap tv,
                                                                      const __grid_constant__ CUtensorMap tl, int lam_tma) {
+    if (chain_wait()) return;
     using R = Rec<64, 64>;
     constexpr int PT = 8192 / NC;                 // threads
     constexpr int PARTS = 64 / NC;                // threads per row of 64
@@ -601,7 +602,7 @@ int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     do {                                                                                                               \
         if (cudaFuncSetAttribute(gdn_prep_umma_kernel<HIER_, NC_>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) \
             return LAMPA_ERR_CUDA;                                                                                     \
-        gdn_prep_umma_kernel<HIER_, NC_><<<grid, 8192 / NC_, smem, st>>>(a, tq, tk, tv, tl, HIER_ ? lam_tma : 0);        \
+        launch_chained(gdn_prep_umma_kernel<HIER_, NC_>, grid, 8192 / NC_, smem, st, a, tq, tk, tv, tl, HIER_ ? lam_tma : 0);        \
     } while (0)
     if (hier) { if (nc == 32) LAMPA_LAUNCH_PREP(true, 32); else LAMPA_LAUNCH_PREP(true, 16); }
     else { if (nc == 32) LAMPA_LAUNCH_PREP(false, 32); else LAMPA_LAUNCH_PREP(false, 16); }

@@ -164,6 +164,7 @@ struct Pipe {
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
 __global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     constexpr int NS = VD / 16;
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD, bool HIER>
 __global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -334,6 +336,7 @@ __global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
 __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, float* states) {
+    if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -411,6 +414,7 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
 __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -498,6 +502,7 @@ __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD, int NG>
 __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hier_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     constexpr int NS = VD / 16;
@@ -686,7 +691,7 @@ static int launch_compose(const GdnArgs& a, cudaStream_t st) {
     const int smem = 1024 + 3 * R::PRE_BYTES;
     LAMPA_TRY(set_smem(gdn_compose_kernel<KD, VD>, smem));
     ProfScope prof("gdn_compose", st);
-    gdn_compose_kernel<KD, VD><<<dim3(a.nb_max, a.H), (KD + VD) * 2, smem, st>>>(a);
+    launch_chained(gdn_compose_kernel<KD, VD>, dim3(a.nb_max, a.H), (KD + VD) * 2, smem, st, a);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
 }
@@ -699,7 +704,7 @@ int launch_scan_plain(const GdnArgs& a, cudaStream_t st) {
         const int smem = 1024 + 3 * R::BLK_BYTES;
         LAMPA_TRY(set_smem(gdn_level_kernel<KD, VD, false>, smem));
         ProfScope prof("gdn_level_plain", st);
-        gdn_level_kernel<KD, VD, false><<<dim3(a.nseq, a.H, 1), VD * 2, smem, st>>>(a);
+        launch_chained(gdn_level_kernel<KD, VD, false>, dim3(a.nseq, a.H, 1), VD * 2, smem, st, a);
         LAMPA_LAUNCHED();
     }
     if (KD == 64 && VD == 64 && a.use_umma) return launch_out_plain_umma(a, st);
@@ -707,7 +712,7 @@ int launch_scan_plain(const GdnArgs& a, cudaStream_t st) {
         const int smem = 1024 + 3 * R::LAM_OFF;
         LAMPA_TRY(set_smem(gdn_out_plain_kernel<KD, VD>, smem));
         ProfScope prof("gdn_out_plain", st);
-        gdn_out_plain_kernel<KD, VD><<<dim3(a.nb_max, a.H), VD * 2, smem, st>>>(a);
+        launch_chained(gdn_out_plain_kernel<KD, VD>, dim3(a.nb_max, a.H), VD * 2, smem, st, a);
         LAMPA_LAUNCHED();
     }
     return LAMPA_OK;
@@ -721,7 +726,7 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
     if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
     LAMPA_TRY(set_smem(gdn_out_hier_kernel<KD, VD, NG>, smem));
     ProfScope prof("gdn_out_hier", st);
-    gdn_out_hier_kernel<KD, VD, NG><<<dim3(a.nb_max, a.H), NG * VD * 2, smem, st>>>(a);
+    launch_chained(gdn_out_hier_kernel<KD, VD, NG>, dim3(a.nb_max, a.H), NG * VD * 2, smem, st, a);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
 }
@@ -736,7 +741,7 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
         const int smem = 1024 + 3 * R::BLK_BYTES;
         LAMPA_TRY(set_smem(gdn_level_kernel<KD, VD, true>, smem));
         ProfScope prof("gdn_level_hier", st);
-        gdn_level_kernel<KD, VD, true><<<dim3(a.nseq, a.H, a.nhigh_max), VD * 2, smem, st>>>(a);
+        launch_chained(gdn_level_kernel<KD, VD, true>, dim3(a.nseq, a.H, a.nhigh_max), VD * 2, smem, st, a);
         LAMPA_LAUNCHED();
     }
     if (KD == 64 && VD == 64 && a.nhigh_max <= 5 && a.use_umma) return launch_out_hier_umma(a, st);
@@ -752,7 +757,7 @@ int launch_final_high(const GdnArgs& a, float* states, cudaStream_t st) {
     const int smem = 1024 + 3 * R::PRE_BYTES;
     LAMPA_TRY(set_smem(hgdn_final_high_kernel<KD, VD>, smem));
     ProfScope prof("hgdn_final_high", st);
-    hgdn_final_high_kernel<KD, VD><<<dim3(a.nseq, a.H, a.L - ELL0), VD * 2, smem, st>>>(a, states);
+    launch_chained(hgdn_final_high_kernel<KD, VD>, dim3(a.nseq, a.H, a.L - ELL0), VD * 2, smem, st, a, states);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
 }

@@ -90,6 +90,7 @@ struct UnitOrder {
 // scattered output: 182 -> 150 us.  (Two output warps: 158 us, and 27 instead of 25 us for a 6,000-hit event; loading both
 // halves of the accumulator row at once: 166 - 217 us, the registers spill.)
 __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs a, UnitOrder uo) {
+    if (chain_wait()) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM_BAR);      // record landed            (tx count)
     uint64_t* sfree = full + UNST;                                      // stage consumed           (16 + 4 warps)
@@ -431,6 +432,7 @@ constexpr int PTM_A = 0, PTM_D = 64;         // tensor-memory columns (256 alloc
 constexpr uint32_t PMMA_IDESC = umma_idesc(64, 128);
 
 __global__ void __launch_bounds__(PTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs a) {
+    if (chain_wait()) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM_BAR);      // records landed            (tx count)
     uint64_t* sfree = full + PNST;                                      // stage consumed            (16 warps)
@@ -659,7 +661,7 @@ int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st) {
         if (n != uo.nbs) uo.nbs = 0;
     }
     ProfScope prof("gdn_out_hier_umma", st);
-    gdn_out_hier_umma_kernel<<<dim3((unsigned)a.nb_max * a.H), UTHREADS, smem, st>>>(a, uo);
+    launch_chained(gdn_out_hier_umma_kernel, dim3((unsigned)a.nb_max * a.H), UTHREADS, smem, st, a, uo);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -668,7 +670,7 @@ int launch_out_plain_umma(const GdnArgs& a, cudaStream_t st) {
     if (cudaFuncSetAttribute(gdn_out_plain_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
     ProfScope prof("gdn_out_plain_umma", st);
-    gdn_out_plain_umma_kernel<<<dim3((unsigned)a.nb_max * ((a.H + 1) / 2)), PTHREADS, smem, st>>>(a);
+    launch_chained(gdn_out_plain_umma_kernel, dim3((unsigned)a.nb_max * ((a.H + 1) / 2)), PTHREADS, smem, st, a);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 

@@ -96,6 +96,7 @@ __device__ __forceinline__ void half_warp_sum_many(float (&x)[N], int lane) {
 
 template <int KD, int VD, int HS>
 __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, TailArgs ta) {
+    if (chain_wait()) return;
     constexpr int KI = KD / 16;
     extern __shared__ __align__(16) float tail_smem[];
     float* sK = tail_smem;                       // [64][KD], normalised
@@ -393,9 +394,9 @@ int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
         !allow_smem(ready[2], hgdn_tail_kernel<KD, VD, 24>, most)) return LAMPA_ERR_CUDA;
     const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
     ProfScope prof("hgdn_tail", st);
-    if (slots <= 4) hgdn_tail_kernel<KD, VD, 4><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
-    else if (slots <= 8) hgdn_tail_kernel<KD, VD, 8><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
-    else hgdn_tail_kernel<KD, VD, 24><<<grid, TAIL_THREADS, smem, st>>>(a, ta);
+    if (slots <= 4) launch_chained(hgdn_tail_kernel<KD, VD, 4>, grid, TAIL_THREADS, smem, st, a, ta);
+    else if (slots <= 8) launch_chained(hgdn_tail_kernel<KD, VD, 8>, grid, TAIL_THREADS, smem, st, a, ta);
+    else launch_chained(hgdn_tail_kernel<KD, VD, 24>, grid, TAIL_THREADS, smem, st, a, ta);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -451,6 +452,7 @@ template <int KD> __host__ __device__ constexpr int step_smem(int L) {      // s
 
 template <int KD, int VD>
 __global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s) {
+    if (chain_wait()) return;
     constexpr int NT = STEP_THREADS<KD>, NW = NT / 32, KI = STEP_KI;        // lane = (4 rows, 8 columns)
     extern __shared__ __align__(16) float slab[];              // [KD][8][L]
     float* part = slab + KD * STEP_COLS * s.L;                 // [2][warps][L][8]: k^T S and q^T S of every level
@@ -617,6 +619,7 @@ __global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s)
 }
 
 __global__ void hgdn_step_counts_kernel(int32_t* counts, int L) {
+    if (chain_wait()) return;
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const uint32_t c0 = (uint32_t)counts[0];
     if (c0 & STEP_LATE) { counts[0] = (int32_t)(c0 & ~STEP_LATE); return; }
@@ -636,11 +639,11 @@ int launch_hgdn_step(const StepArgs& s, cudaStream_t st) {
         return LAMPA_ERR_CUDA;
     {
         ProfScope prof("hgdn_step", st);
-        hgdn_step_kernel<KD, VD><<<dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS<KD>, smem, st>>>(s);
+        launch_chained(hgdn_step_kernel<KD, VD>, dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS<KD>, smem, st, s);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     if (s.arrivals) return LAMPA_OK;
-    hgdn_step_counts_kernel<<<1, 32, 0, st>>>(s.counts, s.L);
+    launch_chained(hgdn_step_counts_kernel, 1, 32, 0, st, s.counts, s.L);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 

@@ -96,6 +96,7 @@ geo_keys_kernel(const float* __restrict__ proj, const float* __restrict__ reg_et
                 const int64_t* __restrict__ rank_phi, const float* __restrict__ regions_eta,
                 const float* __restrict__ regions_phi, const float* __restrict__ hash_shift,
                 int rows, int64_t n, int64_t raw_size, float* __restrict__ out) {
+    if (chain_wait()) return;
     const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
     if (i >= n) return;
     int64_t re = 0, rp = 0;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(512)
 geo_keys_fused_kernel(float* __restrict__ proj, const float2* __restrict__ part, int nblk, const int64_t* __restrict__ rank_eta,
                       const int64_t* __restrict__ rank_phi, const float* __restrict__ regions_eta,
                       const float* __restrict__ regions_phi, int rows, int64_t n, int64_t raw_size) {
+    if (chain_wait()) return;
     __shared__ float smn[16], smx[16];
     const int r = blockIdx.y, tid = threadIdx.x;
     float mn = INFINITY, mx = -INFINITY;
@@ -155,6 +157,7 @@ geo_keys_fused_kernel(float* __restrict__ proj, const float2* __restrict__ part,
 __global__ void __launch_bounds__(GEO_THREADS)
 region_prepare_kernel(const float* __restrict__ coords, int64_t raw, int64_t n, int cols, const float* __restrict__ regions,
                       int nc, int na, int nh, float* __restrict__ padded, float* __restrict__ keys, float* __restrict__ regions_h) {
+    if (chain_wait()) return;
     const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
     if (i < n) {
         for (int c = 0; c < cols; ++c) {
@@ -172,11 +175,13 @@ region_prepare_kernel(const float* __restrict__ coords, int64_t raw, int64_t n, 
 // ranks of both coordinates: rank[perm[i]] = i; and, in hit order, their region numbers for the `rows` rows of regions_h
 __global__ void __launch_bounds__(GEO_THREADS)
 region_ranks_kernel(const int64_t* __restrict__ perm, int64_t n, int64_t* __restrict__ rank) {
+    if (chain_wait()) return;
     const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x, at = blockIdx.y * n;
     if (i < n) rank[at + perm[at + i]] = i;
 }
 __global__ void __launch_bounds__(GEO_THREADS)
 region_numbers_kernel(const int64_t* __restrict__ rank, const float* __restrict__ regions_h, int rows, int64_t n, float* __restrict__ out) {
+    if (chain_wait()) return;
     const int64_t i = (int64_t)blockIdx.x * GEO_THREADS + threadIdx.x;
     const int a = blockIdx.y;
     if (i >= n) return;
@@ -194,7 +199,7 @@ extern "C" int lampa_geo_keys_fused(float* proj, const float* part, int64_t bloc
     if (n == 0) return LAMPA_OK;
     if (!proj || !part || !rank_eta || !rank_phi || !regions_eta || !regions_phi) return LAMPA_ERR_ARG;
     ProfScope prof("geo_keys", (cudaStream_t)stream);
-    geo_keys_fused_kernel<<<dim3((unsigned)((n + GEO_CHUNK - 1) / GEO_CHUNK), rows), 512, 0, (cudaStream_t)stream>>>(
+    launch_chained(geo_keys_fused_kernel, dim3((unsigned)((n + GEO_CHUNK - 1) / GEO_CHUNK), rows), 512, 0, (cudaStream_t)stream,
         proj, (const float2*)part, (int)blocks, rank_eta, rank_phi, regions_eta, regions_phi, rows, n, raw_size);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
@@ -210,15 +215,15 @@ extern "C" int lampa_region_inputs(const float* coords, int64_t raw, int64_t n, 
     const int64_t most = n > 2 * rows ? n : 2 * rows;
     {
         ProfScope prof("region_prepare", st);
-        region_prepare_kernel<<<(unsigned)((most + GEO_THREADS - 1) / GEO_THREADS), GEO_THREADS, 0, st>>>(coords, raw, n, cols, regions, nc, 2, nh, padded, keys, regions_h);
+        launch_chained(region_prepare_kernel, (unsigned)((most + GEO_THREADS - 1) / GEO_THREADS), GEO_THREADS, 0, st, coords, raw, n, cols, regions, nc, 2, nh, padded, keys, regions_h);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     const int rc = lampa_segsort_stable(keys, LAMPA_KEY_F32, 2 * n, nullptr, 2, nullptr, perm, ws, ws_bytes, status, stream);
     if (rc != LAMPA_OK) return rc;
     ProfScope prof("region_ranks", st);
     const dim3 grid((unsigned)((n + GEO_THREADS - 1) / GEO_THREADS), 2);
-    region_ranks_kernel<<<grid, GEO_THREADS, 0, st>>>(perm, n, ranks);
-    region_numbers_kernel<<<grid, GEO_THREADS, 0, st>>>(ranks, regions_h, rows, n, region_indices);
+    launch_chained(region_ranks_kernel, grid, GEO_THREADS, 0, st, perm, n, ranks);
+    launch_chained(region_numbers_kernel, grid, GEO_THREADS, 0, st, ranks, regions_h, rows, n, region_indices);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -253,7 +258,7 @@ extern "C" int lampa_geo_keys(const float* proj, const float* reg_eta, const flo
     if (!from_regions && !from_ranks) return LAMPA_ERR_ARG;
     ProfScope prof("geo_keys", (cudaStream_t)stream);
     const unsigned grid = (unsigned)((n + GEO_THREADS - 1) / GEO_THREADS);
-    geo_keys_kernel<<<grid, GEO_THREADS, 0, (cudaStream_t)stream>>>(
+    launch_chained(geo_keys_kernel, grid, GEO_THREADS, 0, (cudaStream_t)stream,
         proj, from_regions ? reg_eta : nullptr, from_regions ? reg_phi : nullptr, rank_eta, rank_phi,
         regions_eta, regions_phi, hash_shift, rows, n, raw_size, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;

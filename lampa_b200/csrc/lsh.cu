@@ -29,6 +29,7 @@ lsh_hash_kernel(const float* __restrict__ x, int64_t row_stride, int64_t head_st
                 const float* __restrict__ alpha, const float* __restrict__ beta, float w, int64_t N,
                 int heads, int rounds, int dim, int32_t* __restrict__ ids, float* __restrict__ keys,
                 int32_t* __restrict__ packed) {
+    if (chain_wait()) return;
     __shared__ float s_alpha[HASH_MAX_PARAMS];
     __shared__ float s_beta[64];
     const int np = heads * dim * rounds;
@@ -126,6 +127,7 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                const int64_t* __restrict__ seg, int nseg, const int64_t* __restrict__ init,
                int64_t* __restrict__ perm, uint32_t* kbuf0, uint32_t* kbuf1, uint32_t* ibuf0,
                uint32_t* ibuf1, int32_t* status) {
+    if (chain_wait()) return;
     constexpr int TILE = ITEMS * SORT_THREADS;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
@@ -388,7 +390,7 @@ static int launch_segsort(const void* keys, int key_type, int64_t n_total, const
     // A cluster has to fit inside one GPC, so the SM count alone does not tell (148 SMs hold 24
     // clusters of 6 only if every GPC has 18 usable SMs): ask the occupancy calculator.
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     int cl = sort_cluster_size(nseg), which = 0;
     for (;; --cl) {
         // tile: the slice of an equal split, or twice the average slice when the segments are ragged (larger slices
@@ -407,10 +409,12 @@ static int launch_segsort(const void* keys, int key_type, int64_t n_total, const
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 1;                    // the occupancy query knows clusters only
         if (cl == 1) break;
         if (clusters_resident(kernels[which], cfg, cl, 2 * item_counts[which] + (init != nullptr)) >= nseg) break;
     }
+    attr[1] = chained_attribute();
+    cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], keys, key_type, n_total, seg, nseg, init, perm, k0, k1, i0, i1, status);
     return e == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
@@ -434,6 +438,7 @@ __global__ void __launch_bounds__(256)
 permute_rows_kernel(const VEC* __restrict__ src, const int64_t* __restrict__ perm,
                     const int64_t* __restrict__ seg, int nseg, int64_t n_rows, int64_t units_per_row,
                     int scatter, VEC* __restrict__ dst, int32_t* status) {
+    if (chain_wait()) return;
     const int64_t total = n_rows * units_per_row;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total;
          u += (int64_t)gridDim.x * blockDim.x) {
@@ -455,6 +460,7 @@ permute_rows_kernel(const VEC* __restrict__ src, const int64_t* __restrict__ per
 __global__ void __launch_bounds__(256)
 invert_perm_kernel(const int64_t* __restrict__ perm, const int64_t* __restrict__ seg, int nseg,
                    int64_t n_total, int64_t* __restrict__ inv, int32_t* status) {
+    if (chain_wait()) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_total;
          i += (int64_t)gridDim.x * blockDim.x) {
         int64_t s0, len;
@@ -567,6 +573,7 @@ __global__ void __launch_bounds__(ORDER_THREADS)
 ordering_rank_kernel(const float* __restrict__ coords, const float* __restrict__ alpha, int dim, int nh,
                      const uint32_t* __restrict__ points, int row_words, int n, int64_t* __restrict__ idx,
                      uint32_t* __restrict__ ordered) {
+    if (chain_wait()) return;
     extern __shared__ __align__(16) unsigned char order_smem[];
     const int nh4 = NH > 0 ? 4 : (nh + 3) & ~3;
     float* s_alpha = reinterpret_cast<float*>(order_smem);
@@ -616,6 +623,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 ordering_keys_kernel(const float* __restrict__ coords, const float* __restrict__ alpha, int dim, int nh, int64_t n,
                      float* __restrict__ keys, float* __restrict__ norms) {
+    if (chain_wait()) return;
     extern __shared__ __align__(16) unsigned char order_smem[];
     float* s_alpha = reinterpret_cast<float*>(order_smem);
     const int nh4 = (nh + 3) & ~3;
@@ -656,9 +664,9 @@ extern "C" int lampa_lsh_hash(const float* x, int64_t row_stride, int64_t head_s
     const unsigned grid = (unsigned)((N + HASH_THREADS - 1) / HASH_THREADS);
     ProfScope prof("lsh_hash", st);
     if (dim == 6 && head_stride == 0)
-        lsh_hash_kernel<6><<<grid, HASH_THREADS, 0, st>>>(x, row_stride, head_stride, alpha, beta, w, N, heads, rounds, dim, ids, keys, packed);
+        launch_chained(lsh_hash_kernel<6>, grid, HASH_THREADS, 0, st, x, row_stride, head_stride, alpha, beta, w, N, heads, rounds, dim, ids, keys, packed);
     else
-        lsh_hash_kernel<0><<<grid, HASH_THREADS, 0, st>>>(x, row_stride, head_stride, alpha, beta, w, N, heads, rounds, dim, ids, keys, packed);
+        launch_chained(lsh_hash_kernel<0>, grid, HASH_THREADS, 0, st, x, row_stride, head_stride, alpha, beta, w, N, heads, rounds, dim, ids, keys, packed);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -721,7 +729,7 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
         if (smem > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return LAMPA_ERR_CUDA;
         ProfScope prof("lsh_ordering", st);
-        kernel<<<dim3((unsigned)((n + ORDER_POINTS - 1) / ORDER_POINTS), (unsigned)B), ORDER_THREADS, smem, st>>>(
+        launch_chained(kernel, dim3((unsigned)((n + ORDER_POINTS - 1) / ORDER_POINTS), (unsigned)B), ORDER_THREADS, smem, st,
             coords, alpha, dim, num_hashes, (const uint32_t*)points, (int)(row_bytes / 4), (int)n, idx, (uint32_t*)ordered);
         return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
     }
@@ -741,7 +749,7 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
         const Kernel kernel = kernels[dim <= ORDER_REGS ? dim : 0];
         if (params > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, params) != cudaSuccess)
             return LAMPA_ERR_CUDA;
-        kernel<<<(unsigned)((total + 255) / 256), 256, params, st>>>(coords, alpha, dim, num_hashes, total, keys, norms);
+        launch_chained(kernel, (unsigned)((total + 255) / 256), 256, params, st, coords, alpha, dim, num_hashes, total, keys, norms);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     int rc = lampa_segsort_stable(norms, LAMPA_KEY_F32, total, nullptr, B, nullptr, by_norm, sws, sort, status, stream);
@@ -764,9 +772,9 @@ extern "C" int lampa_permute_rows(const void* src, const int64_t* perm, const in
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 32);
     ProfScope prof("permute_rows", st);
     if (v16)
-        permute_rows_kernel<uint4><<<grid, 256, 0, st>>>((const uint4*)src, perm, seg_offsets, nseg, n_rows, upr, scatter, (uint4*)dst, status);
+        launch_chained(permute_rows_kernel<uint4>, grid, 256, 0, st, (const uint4*)src, perm, seg_offsets, nseg, n_rows, upr, scatter, (uint4*)dst, status);
     else
-        permute_rows_kernel<uint32_t><<<grid, 256, 0, st>>>((const uint32_t*)src, perm, seg_offsets, nseg, n_rows, upr, scatter, (uint32_t*)dst, status);
+        launch_chained(permute_rows_kernel<uint32_t>, grid, 256, 0, st, (const uint32_t*)src, perm, seg_offsets, nseg, n_rows, upr, scatter, (uint32_t*)dst, status);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -778,7 +786,7 @@ extern "C" int lampa_invert_perm(const int64_t* perm, const int64_t* seg_offsets
     if (!seg_offsets && n_total % nseg != 0) return LAMPA_ERR_ARG;
     const unsigned grid = (unsigned)std::min<int64_t>((n_total + 255) / 256, 148 * 32);
     ProfScope prof("invert_perm", (cudaStream_t)stream);
-    invert_perm_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(perm, seg_offsets, nseg, n_total, inv, status);
+    launch_chained(invert_perm_kernel, grid, 256, 0, (cudaStream_t)stream, perm, seg_offsets, nseg, n_total, inv, status);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 

@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(256) model_encode_kernel(const float* __restri
                                                            const float* __restrict__ W, const float* __restrict__ bias,
                                                            const float* __restrict__ nw, float eps, int64_t n,
                                                            float* __restrict__ x, __nv_bfloat16* __restrict__ hs) {
+    if (chain_wait()) return;
     __shared__ __align__(16) float rows[8][8 * ENC_IN];
     __shared__ float sw[MD * (ENC_IN + 1)];                  // W through shared memory: a lane's four rows are 96 scattered words
     for (int i = threadIdx.x; i < MD * ENC_IN; i += 256) sw[i / ENC_IN * (ENC_IN + 1) + i % ENC_IN] = __ldg(W + i);
@@ -154,6 +155,7 @@ constexpr int HEAD_SMEM = (HEAD_ROWS + HEAD_OUT) * HEAD_PITCH * 4;
 
 __global__ void __launch_bounds__(256) model_head_kernel(const float* __restrict__ x, const float* __restrict__ W,
                                                          const float* __restrict__ bias, int64_t n, float* __restrict__ out) {
+    if (chain_wait()) return;
     extern __shared__ __align__(16) float head_smem[];
     float* sx = head_smem;                                   // [128][132]
     float* sw = sx + HEAD_ROWS * HEAD_PITCH;                 // [24][132]
@@ -232,6 +234,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                      const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg,
                      const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
                      const __grid_constant__ CUtensorMap ml) {
+    if (chain_wait()) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);        // weight piece landed
     uint64_t* mdone = full + MNST;                             // products of a block complete, by accumulator
@@ -467,6 +470,7 @@ struct UpdateArgs {
 __global__ void __launch_bounds__(UP_THREADS, 2)
 model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const __grid_constant__ CUtensorMap mu,
                     const __grid_constant__ CUtensorMap md) {
+    if (chain_wait()) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);        // weight piece landed
     uint64_t* wfree = full + MNST;                             // its products are done
@@ -778,7 +782,7 @@ extern "C" int lampa_model_encode(const float* hits, const float* scale, const f
     if (n == 0) return LAMPA_OK;
     ProfScope prof("model_encode", (cudaStream_t)stream);
     const int64_t want = (n + 63) / 64, most = (int64_t)sm_count() * 4;
-    model_encode_kernel<<<(unsigned)(want < most ? want : most), 256, 0, (cudaStream_t)stream>>>(
+    launch_chained(model_encode_kernel, (unsigned)(want < most ? want : most), 256, 0, (cudaStream_t)stream,
         hits, scale, weight, bias, norm_w, eps, n, x, (__nv_bfloat16*)hs);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
@@ -793,7 +797,7 @@ extern "C" int lampa_model_head(const float* x, const float* weight, const float
     static std::atomic<uint64_t> ready{0};
     if (!allow_smem(ready, model_head_kernel, HEAD_SMEM)) return LAMPA_ERR_CUDA;
     const int64_t want = (n + HEAD_ROWS - 1) / HEAD_ROWS, most = (int64_t)sm_count() * 2;
-    model_head_kernel<<<(unsigned)(want < most ? want : most), 256, HEAD_SMEM, (cudaStream_t)stream>>>(x, weight, bias, n, out);
+    launch_chained(model_head_kernel, (unsigned)(want < most ? want : most), 256, HEAD_SMEM, (cudaStream_t)stream, x, weight, bias, n, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -823,7 +827,7 @@ extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, c
     if (!allow_smem(ready, model_project_kernel, PJ_SMEM)) return LAMPA_ERR_CUDA;
     ProfScope prof("model_project", (cudaStream_t)stream);
     const int64_t want = (n + PJ_OUT - 1) / PJ_OUT, most = (int64_t)sm_count() * 2;
-    model_project_kernel<<<(unsigned)(want < most ? want : most), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream>>>(a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
+    launch_chained(model_project_kernel, (unsigned)(want < most ? want : most), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream, a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -851,7 +855,7 @@ extern "C" int lampa_model_update(const lampa_model_update_w* w, const void* o, 
     if (!allow_smem(ready, model_update_kernel, UP_SMEM)) return LAMPA_ERR_CUDA;
     ProfScope prof("model_update", (cudaStream_t)stream);
     const int64_t want = (n + UP_ROWS - 1) / UP_ROWS, most = (int64_t)sm_count() * 2;
-    model_update_kernel<<<(unsigned)(want < most ? want : most), UP_THREADS, UP_SMEM, (cudaStream_t)stream>>>(a, mo, mu, md);
+    launch_chained(model_update_kernel, (unsigned)(want < most ? want : most), UP_THREADS, UP_SMEM, (cudaStream_t)stream, a, mo, mu, md);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
@@ -860,6 +864,7 @@ extern "C" int lampa_model_update(const lampa_model_update_w* w, const void* o, 
 // reaches neither into the events beside it nor into another copy's.  One CTA per copy.
 constexpr int SEG_THREADS = 256;
 static __global__ void __launch_bounds__(SEG_THREADS) model_segments_kernel(const int64_t* cu, int nseq, int64_t n, int64_t* out) {
+    if (chain_wait()) return;
     __shared__ int64_t wtop[SEG_THREADS / 32];
     const int r = blockIdx.x;
     int64_t before = 0;
@@ -874,6 +879,6 @@ static __global__ void __launch_bounds__(SEG_THREADS) model_segments_kernel(cons
 
 extern "C" int lampa_repeat_segments(const int64_t* cu, int32_t nseq, int32_t rounds, int64_t n, int64_t* out, void* stream) {
     if (!cu || !out || nseq <= 0 || rounds <= 0) return LAMPA_ERR_ARG;
-    model_segments_kernel<<<(unsigned)rounds, SEG_THREADS, 0, (cudaStream_t)stream>>>(cu, nseq, n, out);
+    launch_chained(model_segments_kernel, (unsigned)rounds, SEG_THREADS, 0, (cudaStream_t)stream, cu, nseq, n, out);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
