@@ -221,6 +221,13 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 blo
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// SMs of the current device
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    return n;
+}
+
 // Opt-in to `bytes` of dynamic shared memory for a kernel, once per device (`ready`: one bit per device, static at the call).
 template <typename K>
 inline bool allow_smem(std::atomic<uint64_t>& ready, K kernel, int bytes) {

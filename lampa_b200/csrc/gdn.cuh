@@ -44,7 +44,6 @@ struct Tile {
 template <int KD, int VD>
 struct Rec {
     using T = Tile<KD>;
-    static constexpr int KP = KD + 8;                 // padded bf16 row pitch (block composites)
     using TV = Tile<VD>;                              // layout of O_local[token][v]: a V-wide bf16 tile
     static constexpr int M_OFF = 0;
     static constexpr int M_BYTES = T::bytes(KD);      // M[k_out][k_in]
@@ -58,13 +57,20 @@ struct Rec {
     static constexpr int PRE_BYTES = OL_OFF;          // M, Q~, B^T: what the compose pass streams
     static constexpr int ALIGN = T::SWZ ? 1024 : 128; // records and shared-memory stages
     __host__ __device__ static constexpr int bytes(int LC) { return LAM_OFF + LC * CHUNK * 4; }
-    // block composite: Mblk[k_out][k_in] bf16 (padded pitch), then Bblk^T[v][k] fp32 (pitch KD + 8)
-    static constexpr int BP = KD + 8;
+    // block composite, in the order in which the lanes of the level pass take it (16 bytes per lane, whole lines per warp):
+    // Mblk as bf16 B fragments [k_in / 16][k_out / 16][lane][4 words], then Bblk^T as an fp32 state
     static constexpr int BLK_M_OFF = 0;
-    static constexpr int BLK_M_BYTES = KD * KP * 2;
+    static constexpr int BLK_M_BYTES = KD * KD * 2;
     static constexpr int BLK_B_OFF = BLK_M_BYTES;
-    static constexpr int BLK_BYTES = BLK_M_BYTES + VD * BP * 4;
-    static constexpr int STATE_FLOATS = VD * KD;      // an S^T[v][k] fp32 state
+    static constexpr int BLK_BYTES = BLK_M_BYTES + VD * KD * 4;
+    // An fp32 state S^T[v][k] (entry states, Bblk^T) is kept as the accumulators of a warp's 16 rows hold it: element (v, k) at
+    // state_at().  A warp moves its slab in KD / 8 instructions of whole 128-byte lines (row-major it was 16 instructions of 8
+    // sectors each, 480 of the level pass's 1560 cycles per block), and a row's 16 columns 16p .. 16p + 15 are 64 contiguous
+    // bytes: four pieces of 16, piece t holding columns 2t, 2t + 1, 8 + 2t, 9 + 2t.
+    static constexpr int STATE_FLOATS = VD * KD;
+    __host__ __device__ static constexpr int state_at(int v, int k) {
+        return ((((v >> 4) * (KD / 16) + (k >> 4)) * 2 + ((v >> 3) & 1)) * 32 + (v & 7) * 4 + ((k >> 1) & 3)) * 4 + ((k >> 3) & 1) * 2 + (k & 1);
+    }
 };
 
 struct GdnArgs {
@@ -79,10 +85,9 @@ struct GdnArgs {
     int fixed_T;        // tokens per sequence when there is no cu_seqlens (0 otherwise)
     int fixed_stride;   // tokens from one sequence to the next in that case (fixed_T, or more when a prompt's tail is left to hgdn_tail)
     int fixed_cps;      // chunks per sequence in that case: positions follow by arithmetic, no plan loads
-    int plan_inline;    // no cu_seqlens: the first preparation CTA writes the offset tables below (no separate launch)
     int nc_max, nb_max, nhigh_max;
     long long total_tokens;  // B * T of the call (rows of the token-major inputs)
-    const int64_t* tok_off; const int32_t* chunk_off; const int32_t* block_off;
+    const int64_t* tok_off; const int32_t* chunk_off; const int32_t* block_off;   // offset tables of a packed call (plan_kernel)
     char* rec; size_t rec_bytes;          // per (chunk, head) records
     char* blk;                            // per (block, head) composites
     float* entry;                         // entry states: plain [nb][H][V][K]; hier [nb][nhigh][H][V][K]
@@ -95,17 +100,6 @@ struct GdnArgs {
 // Stage clock of a preparation CTA: thread 0 of the first `ticks_ctas` CTAs stores clock64() in its slot.
 __device__ __forceinline__ void stage_tick(const GdnArgs& a, int cta, int slot) {
     if (a.ticks != nullptr && threadIdx.x == 0 && cta < a.ticks_ctas) a.ticks[(size_t)cta * 16 + slot] = clock64();
-}
-
-// Offset tables of equally long sequences, written by the first CTA of the preparation kernel for the passes that
-// follow it (the preparation kernel itself locates its chunks by arithmetic in that case).
-__device__ __forceinline__ void write_fixed_plan(const GdnArgs& a) {
-    const int bps = blocks_of(a.fixed_cps);
-    for (int s = threadIdx.x; s <= a.nseq; s += blockDim.x) {
-        const_cast<int64_t*>(a.tok_off)[s] = (int64_t)s * a.fixed_stride;
-        const_cast<int32_t*>(a.chunk_off)[s] = s * a.fixed_cps;
-        const_cast<int32_t*>(a.block_off)[s] = s * bps;
-    }
 }
 
 struct PlanArgs {
@@ -133,6 +127,43 @@ __device__ __forceinline__ bool locate_chunk(const GdnArgs& a, int c, ChunkLoc& 
     loc.seq = find_seq(a.chunk_off, a.nseq, c);
     loc.t0 = a.tok_off[loc.seq] + (int64_t)(c - a.chunk_off[loc.seq]) * CHUNK;
     loc.len = (int)min((int64_t)CHUNK, a.tok_off[loc.seq + 1] - loc.t0);
+    return true;
+}
+
+// The chunks, blocks and tokens of a sequence.  Equally long sequences follow by arithmetic: the dependent loads of the offset
+// tables are the first thing a CTA of the scan would wait for (about 1 us of a pass that is 10 to 20 us long).
+struct SeqLoc { int nch, c0, nblk, gb0; int64_t tok0, tok_end; };
+__device__ __forceinline__ SeqLoc locate_seq(const GdnArgs& a, int seq) {
+    SeqLoc s;
+    if (a.fixed_T > 0) {
+        s.nch = a.fixed_cps;
+        s.c0 = seq * a.fixed_cps;
+        s.nblk = blocks_of(a.fixed_cps);
+        s.gb0 = seq * s.nblk;
+        s.tok0 = (int64_t)seq * a.fixed_stride;
+        s.tok_end = s.tok0 + a.fixed_T;
+    } else {
+        s.c0 = a.chunk_off[seq];
+        s.nch = a.chunk_off[seq + 1] - s.c0;
+        s.gb0 = a.block_off[seq];
+        s.nblk = a.block_off[seq + 1] - s.gb0;
+        s.tok0 = a.tok_off[seq];
+        s.tok_end = a.tok_off[seq + 1];
+    }
+    return s;
+}
+// Where block slot gb lives: its sequence and its place in it.  False for unused slots.
+__device__ __forceinline__ bool locate_block(const GdnArgs& a, int gb, SeqLoc& s, int& b) {
+    int seq;
+    if (a.fixed_T > 0) {
+        seq = gb / blocks_of(a.fixed_cps);
+        if (seq >= a.nseq) return false;
+    } else {
+        if (gb >= a.block_off[a.nseq]) return false;
+        seq = find_seq(a.block_off, a.nseq, gb);
+    }
+    s = locate_seq(a, seq);
+    b = gb - s.gb0;
     return true;
 }
 

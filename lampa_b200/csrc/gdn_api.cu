@@ -92,7 +92,6 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     a.fixed_T = cu ? 0 : d->T;
     a.fixed_stride = a.fixed_T;
     a.fixed_cps = cu ? 0 : (d->T + CHUNK - 1) / CHUNK;
-    a.plan_inline = 0;
     a.total_tokens = (long long)d->B * d->T;
     a.nseq = l.nseq; a.nc_max = l.nc_max; a.nb_max = l.nb_max; a.nhigh_max = l.nhigh_max;
     a.tok_off = (int64_t*)(base + l.off_tok);
@@ -143,8 +142,6 @@ int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const 
     } else if (cu) {
         rc = launch_plan(p, st);
         if (rc != LAMPA_OK) return rc;
-    } else {
-        a.plan_inline = 1;         // equally long sequences: the preparation kernel writes the tables itself
     }
 
 #define LAMPA_DISPATCH(KD, VD)                                         \

@@ -129,7 +129,6 @@ __global__ void __launch_bounds__(8192 / NC, 2) gdn_prep_umma_kernel(GdnArgs a, 
         return sLam[(sb * CHUNK + r) * (a.L + 1) + lev];
     };
     ChunkLoc loc;
-    if (a.plan_inline && blockIdx.x == 0 && blockIdx.y == 0) write_fixed_plan(a);
     if (!locate_chunk(a, c, loc)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t t0 = loc.t0;

@@ -8,9 +8,16 @@
 //   level   : per (sequence, head[, level])  scan the block composites -> state entering each block
 //   output  : per (block, head)  re-run the block from its entry state(s) and emit the outputs
 // Everything a warp owns is a 16-row slab of S^T kept in mma accumulator registers; the slab is
-// re-used as the A operand (S^T M^T) and as the B operand (Q~ S) without leaving registers, so
-// slabs never synchronise with each other.  Records stream through shared memory by bulk async
-// copies (cp.async.bulk + mbarrier), a few chunks ahead of the math.
+// re-used as the A operand (S^T M^T) and as the B operand (Q~ S) without leaving registers.
+// Records stream through shared memory by bulk async copies (cp.async.bulk + mbarrier), a few
+// chunks ahead of the math, issued by a warp of their own.
+//
+// These passes are serial chains, a product per step whose result is the next one's operand: what
+// bounds them is the latency of a step.  The product itself is 373 cycles for a slab of 16 x 64 on
+// an otherwise idle scheduler; a __syncthreads, a poll of a completed mbarrier by every warp, and a
+// state moved in 8-byte pieces added 60, 170 - 260 and 480 (level pass: 1560 cycles per block).
+// Hence one warp polls, the others meet it at a named barrier, and states and composites are laid
+// out in the order of the accumulator registers.
 #include "gdn.cuh"
 #include "profile.cuh"
 
@@ -36,16 +43,9 @@ __device__ __forceinline__ void pack_state(const float (&C)[KD / 8][4], uint32_t
     }
 }
 
-// Element offset inside a bf16 tile: TL is Tile<KD> (record tiles, swizzled for KD = 64) or Padded<KD>
-// (block composites).
-template <int KD>
-struct Padded {
-    __device__ static constexpr int off(int r, int c) { return r * (KD + 8) + c; }
-};
-
-// C += slab * M^T, with sM[k_out][k_in]
-template <int KD, class TL>
-__device__ __forceinline__ void state_times_mt(float (&C)[KD / 8][4], const uint32_t (&sp)[KD / 16][4],
+// C += slab * M^T for NX slabs, with the record tile sM[k_out][k_in]
+template <int KD, int NX>
+__device__ __forceinline__ void state_times_mt(float (&C)[NX][KD / 8][4], const uint32_t (&sp)[NX][KD / 16][4],
                                                const __nv_bfloat16* sM, int lane) {
     const int mi = lane >> 3, r = lane & 7;
 #pragma unroll
@@ -53,61 +53,97 @@ __device__ __forceinline__ void state_times_mt(float (&C)[KD / 8][4], const uint
 #pragma unroll
         for (int nt = 0; nt < KD / 8; nt += 2) {
             uint32_t b[4];
-            ldsm_x4(b, smem_u32(sM + TL::off(nt * 8 + r + (mi >> 1) * 8, kk * 16 + (mi & 1) * 8)));
-            mma16816(C[nt], sp[kk], b[0], b[1]);
-            mma16816(C[nt + 1], sp[kk], b[2], b[3]);
+            ldsm_x4(b, smem_u32(sM + Tile<KD>::off(nt * 8 + r + (mi >> 1) * 8, kk * 16 + (mi & 1) * 8)));
+#pragma unroll
+            for (int x = 0; x < NX; ++x) {
+                mma16816(C[x][nt], sp[x][kk], b[0], b[1]);
+                mma16816(C[x][nt + 1], sp[x][kk], b[2], b[3]);
+            }
         }
     }
 }
-
-// C = rows row0+g, row0+g+8 of a bf16 [rows][KD] record tile
 template <int KD>
-__device__ __forceinline__ void load_slab_bf16(float (&C)[KD / 8][4], const __nv_bfloat16* s, int row0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int nt = 0; nt < KD / 8; ++nt) {
-        const float2 lo = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(s + Tile<KD>::off(row0 + g, nt * 8 + 2 * t)));
-        const float2 hi = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(s + Tile<KD>::off(row0 + g + 8, nt * 8 + 2 * t)));
-        C[nt][0] = lo.x; C[nt][1] = lo.y; C[nt][2] = hi.x; C[nt][3] = hi.y;
-    }
+__device__ __forceinline__ void state_times_mt(float (&C)[KD / 8][4], const uint32_t (&sp)[KD / 16][4],
+                                               const __nv_bfloat16* sM, int lane) {
+    state_times_mt<KD, 1>(reinterpret_cast<float (&)[1][KD / 8][4]>(C), reinterpret_cast<const uint32_t (&)[1][KD / 16][4]>(sp), sM, lane);
 }
-// same from / to an fp32 [rows][pitch] tile (shared or global)
+// The same with a block composite's Mblk, which is stored as the fragments themselves
 template <int KD>
-__device__ __forceinline__ void load_slab_f32(float (&C)[KD / 8][4], const float* s, int pitch, int row0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int nt = 0; nt < KD / 8; ++nt) {
-        const float2 lo = *reinterpret_cast<const float2*>(s + (size_t)(row0 + g) * pitch + nt * 8 + 2 * t);
-        const float2 hi = *reinterpret_cast<const float2*>(s + (size_t)(row0 + g + 8) * pitch + nt * 8 + 2 * t);
-        C[nt][0] = lo.x; C[nt][1] = lo.y; C[nt][2] = hi.x; C[nt][3] = hi.y;
-    }
-}
-template <int KD>
-__device__ __forceinline__ void store_slab_f32(const float (&C)[KD / 8][4], float* s, int pitch, int row0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int nt = 0; nt < KD / 8; ++nt) {
-        *reinterpret_cast<float2*>(s + (size_t)(row0 + g) * pitch + nt * 8 + 2 * t) = make_float2(C[nt][0], C[nt][1]);
-        *reinterpret_cast<float2*>(s + (size_t)(row0 + g + 8) * pitch + nt * 8 + 2 * t) = make_float2(C[nt][2], C[nt][3]);
-    }
-}
-
-// tmp (16 tokens x 16 state columns of this slab) = Q~[16*mt .. +16, :] * S
-template <int KD>
-__device__ __forceinline__ void read_tile(float (&tmp)[2][4], const uint32_t (&sp)[KD / 16][4],
-                                          const __nv_bfloat16* sQt, int mt, int lane) {
-    tmp[0][0] = tmp[0][1] = tmp[0][2] = tmp[0][3] = 0.f;
-    tmp[1][0] = tmp[1][1] = tmp[1][2] = tmp[1][3] = 0.f;
+__device__ __forceinline__ void state_times_mblk(float (&C)[KD / 8][4], const uint32_t (&sp)[KD / 16][4], const uint4* sM, int lane) {
 #pragma unroll
     for (int kk = 0; kk < KD / 16; ++kk) {
-        uint32_t a[4];
-        {
-            const int mi = lane >> 3, r = lane & 7;
-            ldsm_x4(a, smem_u32(sQt + Tile<KD>::off(mt * 16 + r + (mi & 1) * 8, kk * 16 + (mi >> 1) * 8)));
+#pragma unroll
+        for (int np = 0; np < KD / 16; ++np) {
+            const uint4 b = sM[(kk * (KD / 16) + np) * 32 + lane];
+            mma16816(C[2 * np], sp[kk], b.x, b.y);
+            mma16816(C[2 * np + 1], sp[kk], b.z, b.w);
         }
-        mma16816(tmp[0], a, sp[kk][0], sp[kk][2]);
-        mma16816(tmp[1], a, sp[kk][1], sp[kk][3]);
     }
+}
+// 8 x 8 bf16 tile across the warp, transposed
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+    return y;
+}
+
+// C = rows row0 .. row0 + 15 of a bf16 [rows][KD] record tile
+template <int KD>
+__device__ __forceinline__ void load_slab_bf16(float (&C)[KD / 8][4], const __nv_bfloat16* s, int row0, int lane) {
+    const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int p = 0; p < KD / 16; ++p) {
+        uint32_t w[4];
+        ldsm_x4(w, smem_u32(s + Tile<KD>::off(row0 + r + (mi & 1) * 8, 16 * p + (mi >> 1) * 8)));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 f = unpack_bf16x2(w[q]);
+            C[2 * p + (q >> 1)][2 * (q & 1)] = f.x;
+            C[2 * p + (q >> 1)][2 * (q & 1) + 1] = f.y;
+        }
+    }
+}
+// slab `slab` of an fp32 state (Rec::state_at) in shared or global memory
+template <int KD>
+__device__ __forceinline__ void load_slab_f32(float (&C)[KD / 8][4], const float* s, int slab, int lane) {
+    const float4* p4 = reinterpret_cast<const float4*>(s) + slab * (KD / 8) * 32 + lane;
+#pragma unroll
+    for (int p = 0; p < KD / 16; ++p)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const float4 f = p4[(2 * p + hh) * 32];
+            C[2 * p][2 * hh] = f.x; C[2 * p][2 * hh + 1] = f.y; C[2 * p + 1][2 * hh] = f.z; C[2 * p + 1][2 * hh + 1] = f.w;
+        }
+}
+template <int KD>
+__device__ __forceinline__ void store_slab_f32(const float (&C)[KD / 8][4], float* s, int slab, int lane) {
+    float4* p4 = reinterpret_cast<float4*>(s) + slab * (KD / 8) * 32 + lane;
+#pragma unroll
+    for (int p = 0; p < KD / 16; ++p)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh)
+            p4[(2 * p + hh) * 32] = make_float4(C[2 * p][2 * hh], C[2 * p][2 * hh + 1], C[2 * p + 1][2 * hh], C[2 * p + 1][2 * hh + 1]);
+}
+
+// tmp[x] (16 tokens x 16 state columns of this slab) = Q~[16 (mt + x) .. +16, :] * S for NM row tiles: 2 NM independent chains
+// of KD / 16 dependent products
+template <int KD, int NM>
+__device__ __forceinline__ void read_tiles(float (&tmp)[NM][2][4], const uint32_t (&sp)[KD / 16][4],
+                                           const __nv_bfloat16* sQt, int mt, int lane) {
+    const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int x = 0; x < NM; ++x)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) { tmp[x][nt][0] = tmp[x][nt][1] = tmp[x][nt][2] = tmp[x][nt][3] = 0.f; }
+#pragma unroll
+    for (int kk = 0; kk < KD / 16; ++kk)
+#pragma unroll
+        for (int x = 0; x < NM; ++x) {
+            uint32_t a[4];
+            ldsm_x4(a, smem_u32(sQt + Tile<KD>::off((mt + x) * 16 + r + (mi & 1) * 8, kk * 16 + (mi >> 1) * 8)));
+            mma16816(tmp[x][0], a, sp[kk][0], sp[kk][2]);
+            mma16816(tmp[x][1], a, sp[kk][1], sp[kk][3]);
+        }
 }
 
 // ---- record pipeline: thread 0 issues bulk copies NST-1 steps ahead; everyone waits on the
@@ -159,79 +195,169 @@ struct Pipe {
     }
 };
 
+// ---- the same pipeline with a warp of its own for the copies.  Steps come in groups of GRP with one mbarrier, which only that
+// warp polls; a group begins with one named barrier of all NT threads, which says that its records have landed and that
+// everybody is done with the group before, whose stage is refilled then.  (A poll and a copy cost the warp 170 and 150 - 350
+// cycles: with one record to a group that is as long as a short step.)  A wait that runs out is recorded and everybody walks
+// on to the end.
+template <int NST, int NT, int GRP>
+struct Feed {
+    uint64_t* bar;
+    unsigned char* stage;
+    int step_bytes;      // distance between steps in shared memory
+    const char* src;     // record of step 0
+    size_t src_stride;   // bytes between consecutive steps' records
+    uint32_t copy_bytes;
+    int nsteps;
+    int32_t* status;
+    int budget;          // polls per wait
+    size_t src2;         // a second piece of every record: where it begins in the record, and its bytes (0: none).  It lands
+    uint32_t copy2;      // behind the first one in the stage
+
+    static __device__ __forceinline__ void meet() { asm volatile("bar.sync 1, %0;\n" :: "n"(NT) : "memory"); }
+    __device__ __forceinline__ int groups() const { return (nsteps + GRP - 1) / GRP; }
+    __device__ __forceinline__ void issue(int grp) const {                       // the whole warp, a lane to a step
+        const int lane = threadIdx.x & 31, step = grp * GRP + lane;
+        uint64_t* b = bar + (grp % NST);
+        if (lane == 0) mbar_expect_tx(b, (uint32_t)min(GRP, nsteps - step) * (copy_bytes + copy2));
+        __syncwarp();
+        if (lane < GRP && step < nsteps) {
+            unsigned char* dst = stage + (size_t)((grp % NST) * GRP + lane) * step_bytes;
+            const char* from = src + (size_t)step * src_stride;
+            bulk_g2s(dst, from, copy_bytes, b);
+            if (copy2 > 0) bulk_g2s(dst + copy_bytes, from + src2, copy2, b);
+        }
+    }
+    // All threads, before anything else; `producer`: the warp that goes on to produce()
+    __device__ __forceinline__ void start(bool producer) const {
+        if (!producer) return;
+        if ((threadIdx.x & 31) == 0) {
+            for (int s = 0; s < NST; ++s) mbar_init(bar + s, 1);
+            fence_mbar_init();
+        }
+        __syncwarp();
+        for (int s = 0; s < NST && s < groups(); ++s) issue(s);
+    }
+    // The producer warp.  `extra`: barriers behind the last step
+    __device__ __forceinline__ void produce(int extra = 0) const {
+        bool dead = false;
+        const int ng = groups();
+        int issued = ng < NST ? ng : NST, landed = 0;
+        for (int i = 0; i < ng; ++i) {
+            if (mbar_wait(bar + (i % NST), (uint32_t)((i / NST) & 1), dead, status, 100 + (i & 0xffff), budget)) landed = i + 1;
+            dead = __any_sync(0xffffffffu, dead);
+            meet();
+            if (!dead && i > 0 && i - 1 + NST < ng) { issue(i - 1 + NST); issued = i + NST; }
+        }
+        for (int i = 0; i < extra; ++i) meet();
+        // copies that were started but never seen complete (only after a wait gave up) land before the CTA's memory is given back
+        for (int s = landed; s < issued; ++s) mbar_drain(bar + (s % NST), (uint32_t)((s / NST) & 1));
+    }
+    // Everybody else, at the top of step i: where its record is
+    __device__ __forceinline__ const unsigned char* step(int i) const {
+        if (GRP == 1 || i % GRP == 0) meet();
+        return stage + (size_t)(GRP == 1 ? i % NST : i % (NST * GRP)) * step_bytes;
+    }
+};
+
 // -------------------------------------------------------------------------------------------------
-// compose: (Mblk, Bblk) of one block of chunks
+// compose: (Mblk, Bblk) of one block of chunks.  Slabs 0 .. VD / 16 - 1 run S from zero, the KD / 16 slabs behind them P from
+// the identity; SPW slabs to a warp.  A slab's 32 products of a step take 290 cycles of a scheduler and its fragments of M 64
+// cycles of the SM's shared-memory pipe, so with one slab to a warp the eight warps of a block spend as long on reading M
+// eight times as on the products.  Two slabs to a warp share the fragments (SPLIT = 1).  SPLIT = 2: S and P in CTAs of their
+// own, one slab to a warp and one warp to a scheduler: the shortest step, where all halves run at once on SMs of their own.
 // -------------------------------------------------------------------------------------------------
-template <int KD, int VD>
-__global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
+template <int KD, int VD, int SPLIT>
+struct Compose {
+    static constexpr int SLABS_S = VD / 16, SLABS_P = KD / 16;
+    static constexpr int SPW = SPLIT == 1 && KD == 64 ? 2 : 1;
+    static constexpr int SLABS = SPLIT == 1 ? SLABS_S + SLABS_P : (SLABS_S > SLABS_P ? SLABS_S : SLABS_P);
+    static constexpr int NW = SLABS / SPW;
+    static constexpr int GRP = SPLIT == 1 ? 1 : 2, NST = SPLIT == 1 ? 3 : 4;       // 74 KB: three CTAs to an SM; 197 KB: one
+    static_assert(SLABS % SPW == 0 && SLABS_S % SPW == 0, "a warp's slabs are of one kind");
+};
+
+template <int KD, int VD, int SPLIT>
+__global__ void __launch_bounds__(Compose<KD, VD, SPLIT>::NW * 32 + 32) gdn_compose_kernel(GdnArgs a) {
     if (chain_wait()) return;
     using R = Rec<KD, VD>;
-    constexpr int NST = 3;
-    constexpr int NS = VD / 16;
+    using G = Compose<KD, VD, SPLIT>;
+    constexpr int NW = G::NW, SPW = G::SPW, NS = G::SLABS_S;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int gb = blockIdx.x, h = blockIdx.y;
-    if (gb >= a.block_off[a.nseq]) return;
-    const int seq = find_seq(a.block_off, a.nseq, gb);
-    const int b = gb - a.block_off[seq];
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
+    const int nch = sq.nch;
     const int bc = 1 << block_log(nch);
-    const int c0 = a.chunk_off[seq] + b * bc;
+    const int c0 = sq.c0 + b * bc;
     const int nsteps = min(bc, nch - b * bc);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
+    const bool only_p = SPLIT == 2 && blockIdx.z == 1;
 
-    Pipe<NST> pipe;
-    pipe.bar = reinterpret_cast<uint64_t*>(smem);
-    pipe.stage = smem + 1024;
-    pipe.stage_bytes = R::PRE_BYTES;
-    pipe.src = a.rec + ((size_t)c0 * a.H + h) * a.rec_bytes;
-    pipe.src_stride = (size_t)a.H * a.rec_bytes;
-    pipe.copy_bytes = R::PRE_BYTES;
-    pipe.nsteps = nsteps;
-    pipe.dead = false;
-    pipe.status = a.status;
-    pipe.budget = a.poll_budget;
-    pipe.start();
-
-    const bool is_s = warp < NS;
-    const int row0 = is_s ? warp * 16 : (warp - NS) * 16;
-    float C[KD / 8][4];
-    zero_state<KD>(C);
-    if (!is_s) {
-#pragma unroll
-        for (int nt = 0; nt < KD / 8; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (row0 + g + (e >> 1) * 8 == nt * 8 + 2 * t + (e & 1)) C[nt][e] = 1.f;
+    Feed<G::NST, NW * 32 + 32, G::GRP> feed;
+    feed.bar = reinterpret_cast<uint64_t*>(smem);
+    feed.stage = smem + 1024;
+    feed.step_bytes = R::M_BYTES + R::BT_BYTES;
+    feed.src = a.rec + ((size_t)c0 * a.H + h) * a.rec_bytes;
+    feed.src_stride = (size_t)a.H * a.rec_bytes;
+    feed.copy_bytes = R::M_BYTES;
+    feed.src2 = R::BT_OFF;
+    feed.copy2 = only_p ? 0 : R::BT_BYTES;
+    feed.nsteps = nsteps;
+    feed.status = a.status;
+    feed.budget = a.poll_budget;
+    feed.start(warp == NW);
+    if (warp == NW) {
+        feed.produce();
+        return;
     }
-    for (int i = 0; i < nsteps; ++i) {
-        const unsigned char* st = pipe.acquire(i);
-        const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
-        const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
-        uint32_t sp[KD / 16][4];
-        pack_state<KD>(C, sp);
-        if (is_s) {
-            load_slab_bf16<KD>(C, sBt, row0, lane);
-            if (i > 0) state_times_mt<KD, Tile<KD>>(C, sp, sM, lane);
-        } else {
-            zero_state<KD>(C);
-            state_times_mt<KD, Tile<KD>>(C, sp, sM, lane);
+    const int slot = (only_p ? NS : 0) + warp * SPW;
+    const bool is_s = slot < NS;
+    if (slot >= (SPLIT == 2 && !only_p ? NS : NS + G::SLABS_P)) {      // a half with fewer slabs than warps
+        for (int i = 0; i < nsteps; ++i) feed.step(i);
+        return;
+    }
+    const int slab = is_s ? slot : slot - NS;
+    float C[SPW][KD / 8][4];
+#pragma unroll
+    for (int x = 0; x < SPW; ++x) {
+        zero_state<KD>(C[x]);
+        if (!is_s) {
+#pragma unroll
+            for (int nt = 0; nt < KD / 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (16 * (slab + x) + g + (e >> 1) * 8 == nt * 8 + 2 * t + (e & 1)) C[x][nt][e] = 1.f;
         }
     }
-    pipe.finish();
+    for (int i = 0; i < nsteps; ++i) {
+        const unsigned char* st = feed.step(i);
+        const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st);
+        const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::M_BYTES);
+        uint32_t sp[SPW][KD / 16][4];
+#pragma unroll
+        for (int x = 0; x < SPW; ++x) {
+            pack_state<KD>(C[x], sp[x]);
+            if (is_s) load_slab_bf16<KD>(C[x], sBt, 16 * (slab + x), lane);
+            else zero_state<KD>(C[x]);
+        }
+        if (i > 0 || !is_s) state_times_mt<KD, SPW>(C, sp, sM, lane);
+    }
     char* blk = a.blk + ((size_t)gb * a.H + h) * R::BLK_BYTES;
-    if (is_s) {
-        store_slab_f32<KD>(C, reinterpret_cast<float*>(blk + R::BLK_B_OFF), R::BP, row0, lane);
-    } else {
-        // registers hold P^T (row = k_in, col = k_out); Mblk is stored as P[k_out][k_in]
-        __nv_bfloat16* gm = reinterpret_cast<__nv_bfloat16*>(blk + R::BLK_M_OFF);
 #pragma unroll
-        for (int nt = 0; nt < KD / 8; ++nt)
+    for (int x = 0; x < SPW; ++x) {
+        if (is_s) {
+            store_slab_f32<KD>(C[x], reinterpret_cast<float*>(blk + R::BLK_B_OFF), slab + x, lane);
+        } else {
+            // registers hold P^T (row = k_in, col = k_out): its 8 x 8 tiles transposed are the fragments the level pass takes
+            uint4* gm = reinterpret_cast<uint4*>(blk + R::BLK_M_OFF) + (slab + x) * (KD / 16) * 32 + lane;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int kin = row0 + g + (e >> 1) * 8, kout = nt * 8 + 2 * t + (e & 1);
-                gm[kout * R::KP + kin] = __float2bfloat16_rn(C[nt][e]);   // block composites keep the padded pitch
-            }
+            for (int q = 0; q < KD / 16; ++q)
+                gm[q * 32] = make_uint4(transpose8x8(pack_bf16x2(C[x][2 * q][0], C[x][2 * q][1])), transpose8x8(pack_bf16x2(C[x][2 * q][2], C[x][2 * q][3])),
+                                        transpose8x8(pack_bf16x2(C[x][2 * q + 1][0], C[x][2 * q + 1][1])), transpose8x8(pack_bf16x2(C[x][2 * q + 1][2], C[x][2 * q + 1][3])));
+        }
     }
 }
 
@@ -241,37 +367,54 @@ __global__ void __launch_bounds__((KD + VD) * 2) gdn_compose_kernel(GdnArgs a) {
 // one CTA per cross-block level lh (chunk level block_log + lh); the level collects blocks whose bit lh is
 // 0, is read by blocks whose bit lh is 1 (its entry state is stored for those) and is cleared at
 // the end of each period of 2^(lh+1) blocks.
+//
+// NW slabs of 16 state rows to a CTA.  With all four of a 64 x 64 head in one CTA the shared-memory and store pipes of the SM are
+// the longest part of a step (M read four times, the state written: 640 of 1220 cycles); slabs never meet, so where that leaves
+// SMs idle every slab gets a CTA.
 // -------------------------------------------------------------------------------------------------
-template <int KD, int VD, bool HIER>
-__global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
+template <int KD, int NW>
+struct LevelSmem {
+    static constexpr int STEP = KD * KD * 2 + NW * 16 * KD * 4;      // Mblk and the slabs' rows of Bblk^T
+    static constexpr int NST = KD == 64 ? 4 : 3, GRP = KD < 64 ? 4 : (NW == 1 ? 2 : 1);
+    static constexpr int bytes = 1024 + NST * GRP * STEP;            // 99 KB at K = V = 64, either way: two CTAs to an SM
+};
+
+template <int KD, int VD, bool HIER, int NW>
+__global__ void __launch_bounds__(NW * 32 + 32) gdn_level_kernel(GdnArgs a) {
     if (chain_wait()) return;
     using R = Rec<KD, VD>;
-    constexpr int NST = 3;
+    using S = LevelSmem<KD, NW>;
+    constexpr int PARTS = VD / 16 / NW;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int seq = blockIdx.x, h = blockIdx.y, lh = blockIdx.z, H = a.H;
-    const int nblk = a.block_off[seq + 1] - a.block_off[seq];
-    const int gb0 = a.block_off[seq];
+    const int seq = blockIdx.x, h = blockIdx.y, lh = blockIdx.z / PARTS, H = a.H;
+    const SeqLoc sq = locate_seq(a, seq);
+    const int nblk = sq.nblk, gb0 = sq.gb0;
     if (HIER) {
-        const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+        const int nch = sq.nch;
         const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
         if (lh >= nlev - block_log(nch)) return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int row0 = warp * 16;
+    const int slab0 = (blockIdx.z - lh * PARTS) * NW, slab = slab0 + warp, row0 = slab * 16;
 
-    Pipe<NST> pipe;
-    pipe.bar = reinterpret_cast<uint64_t*>(smem);
-    pipe.stage = smem + 1024;
-    pipe.stage_bytes = R::BLK_BYTES;
-    pipe.src = a.blk + ((size_t)gb0 * H + h) * R::BLK_BYTES;
-    pipe.src_stride = (size_t)H * R::BLK_BYTES;
-    pipe.copy_bytes = R::BLK_BYTES;
-    pipe.nsteps = nblk;
-    pipe.dead = false;
-    pipe.status = a.status;
-    pipe.budget = a.poll_budget;
-    pipe.start();
+    Feed<S::NST, NW * 32 + 32, S::GRP> feed;
+    feed.bar = reinterpret_cast<uint64_t*>(smem);
+    feed.stage = smem + 1024;
+    feed.step_bytes = S::STEP;
+    feed.src = a.blk + ((size_t)gb0 * H + h) * R::BLK_BYTES;
+    feed.src_stride = (size_t)H * R::BLK_BYTES;
+    feed.copy_bytes = PARTS == 1 ? R::BLK_BYTES : R::BLK_M_BYTES;
+    feed.src2 = R::BLK_B_OFF + (size_t)slab0 * 16 * KD * 4;
+    feed.copy2 = PARTS == 1 ? 0 : NW * 16 * KD * 4;
+    feed.nsteps = nblk;
+    feed.status = a.status;
+    feed.budget = a.poll_budget;
+    feed.start(warp == NW);
+    if (warp == NW) {
+        feed.produce();
+        return;
+    }
 
     float C[KD / 8][4];
     zero_state<KD>(C);
@@ -286,34 +429,29 @@ __global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
         nonzero = true;
     }
     for (int b = 0; b < nblk; ++b) {
-        const unsigned char* st = pipe.acquire(b);
-        const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::BLK_M_OFF);
-        const float* sB = reinterpret_cast<const float*>(st + R::BLK_B_OFF);
+        const unsigned char* st = feed.step(b);
+        const uint4* sM = reinterpret_cast<const uint4*>(st);
+        const float* sB = reinterpret_cast<const float*>(st + R::BLK_M_BYTES);
         uint32_t sp[KD / 16][4];
         if (!HIER) {
-            float* e = a.entry + ((size_t)(gb0 + b) * H + h) * R::STATE_FLOATS;
-            store_slab_f32<KD>(C, e, KD, row0, lane);
+            store_slab_f32<KD>(C, a.entry + ((size_t)(gb0 + b) * H + h) * R::STATE_FLOATS, slab, lane);
             pack_state<KD>(C, sp);
-            load_slab_f32<KD>(C, sB, R::BP, row0, lane);
-            if (nonzero) state_times_mt<KD, Padded<KD>>(C, sp, sM, lane);
+            load_slab_f32<KD>(C, sB, warp, lane);
+            if (nonzero) state_times_mblk<KD>(C, sp, sM, lane);
             nonzero = true;
         } else {
             const int period = 2 << lh, pos = b & (period - 1), bit = (b >> lh) & 1;
-            if (bit) {
-                float* e = a.entry + (((size_t)(gb0 + b) * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS;
-                store_slab_f32<KD>(C, e, KD, row0, lane);
-            }
+            if (bit) store_slab_f32<KD>(C, a.entry + (((size_t)(gb0 + b) * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, slab, lane);
             if (pos == period - 1) {
                 zero_state<KD>(C);
             } else {
                 pack_state<KD>(C, sp);
-                if (bit == 0) load_slab_f32<KD>(C, sB, R::BP, row0, lane);
+                if (bit == 0) load_slab_f32<KD>(C, sB, warp, lane);
                 else zero_state<KD>(C);
-                if (pos != 0) state_times_mt<KD, Padded<KD>>(C, sp, sM, lane);
+                if (pos != 0) state_times_mblk<KD>(C, sp, sM, lane);
             }
         }
     }
-    pipe.finish();
     if (!HIER && a.ht != nullptr) {
         float* ht = a.ht + ((size_t)seq * H + h) * KD * VD;
 #pragma unroll
@@ -335,13 +473,14 @@ __global__ void __launch_bounds__(VD * 2) gdn_level_kernel(GdnArgs a) {
 // pass stored for the last block.  states is [N][H][K][V][L] fp32; unoccupied levels are zeroed.
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
-__global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, float* states) {
+__global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a, float* states) {
     if (chain_wait()) return;
     using R = Rec<KD, VD>;
-    constexpr int NST = 3;
+    constexpr int NST = 3, NW = VD / 16;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int seq = blockIdx.x, h = blockIdx.y, lev = blockIdx.z, H = a.H;
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    const SeqLoc sq = locate_seq(a, seq);
+    const int nch = sq.nch;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int row0 = warp * 16;
@@ -351,31 +490,30 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
     float C[KD / 8][4];
     zero_state<KD>(C);
     if (live) {
-        int c_first, half_end;
-        if (lev < bl) {
-            c_first = n & ~((2 << lev) - 1);
-            half_end = c_first + (1 << lev);
-        } else {
-            c_first = (n >> bl) << bl;
-            half_end = c_first;
-            const int gb = a.block_off[seq] + (n >> bl);
-            const float* e = a.entry + (((size_t)gb * a.nhigh_max + (lev - bl)) * H + h) * R::STATE_FLOATS;
-            load_slab_f32<KD>(C, e, KD, row0, lane);
+        const int c_first = lev < bl ? n & ~((2 << lev) - 1) : (n >> bl) << bl;
+        const int half_end = lev < bl ? c_first + (1 << lev) : c_first;
+        Feed<NST, NW * 32 + 32, 1> feed;
+        feed.bar = reinterpret_cast<uint64_t*>(smem);
+        feed.stage = smem + 1024;
+        feed.step_bytes = R::PRE_BYTES;
+        feed.src = a.rec + ((size_t)(sq.c0 + c_first) * H + h) * a.rec_bytes;
+        feed.src_stride = (size_t)H * a.rec_bytes;
+        feed.copy_bytes = R::PRE_BYTES;
+        feed.nsteps = n - c_first + 1;
+        feed.status = a.status;
+        feed.budget = a.poll_budget;
+        feed.copy2 = 0;
+        feed.start(warp == NW);
+        if (warp == NW) {
+            feed.produce();
+            return;
         }
-        Pipe<NST> pipe;
-        pipe.bar = reinterpret_cast<uint64_t*>(smem);
-        pipe.stage = smem + 1024;
-        pipe.stage_bytes = R::PRE_BYTES;
-        pipe.src = a.rec + ((size_t)(a.chunk_off[seq] + c_first) * H + h) * a.rec_bytes;
-        pipe.src_stride = (size_t)H * a.rec_bytes;
-        pipe.copy_bytes = R::PRE_BYTES;
-        pipe.nsteps = n - c_first + 1;
-        pipe.dead = false;
-        pipe.status = a.status;
-        pipe.budget = a.poll_budget;
-        pipe.start();
-        for (int i = 0; i < pipe.nsteps; ++i) {
-            const unsigned char* st = pipe.acquire(i);
+        if (lev >= bl) {
+            const int gb = sq.gb0 + (n >> bl);
+            load_slab_f32<KD>(C, a.entry + (((size_t)gb * a.nhigh_max + (lev - bl)) * H + h) * R::STATE_FLOATS, warp, lane);
+        }
+        for (int i = 0; i < feed.nsteps; ++i) {
+            const unsigned char* st = feed.step(i);
             const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
             const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
             // the state enters the tensor core as bf16 hi + bf16 lo (two products), so that re-rounding
@@ -393,12 +531,12 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
             if (c_first + i < half_end) load_slab_bf16<KD>(C, sBt, row0, lane);
             else zero_state<KD>(C);
             if (i > 0 || lev >= bl) {
-                state_times_mt<KD, Tile<KD>>(C, sp, sM, lane);
-                state_times_mt<KD, Tile<KD>>(C, sl, sM, lane);
+                state_times_mt<KD>(C, sp, sM, lane);
+                state_times_mt<KD>(C, sl, sM, lane);
             }
         }
-        pipe.finish();
     }
+    if (warp == NW) return;
     float* dst = states + ((size_t)seq * H + h) * KD * VD * a.L + ELL0 + lev;
 #pragma unroll
     for (int nt = 0; nt < KD / 8; ++nt)
@@ -411,78 +549,122 @@ __global__ void __launch_bounds__(VD * 2) hgdn_final_high_kernel(GdnArgs a, floa
 
 // -------------------------------------------------------------------------------------------------
 // output, plain rule:  O_n = O_local + Q~ S_n ;  S_{n+1} = M S_n + B
+// VD / 16 slab warps, the copying warp, and one that stores: a chunk's output goes through a [token][v] tile in shared memory
+// and leaves as whole rows, under the next chunk's products.  (fp32 outputs go straight from the registers.)
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
-__global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
+struct OutPlainSmem {
+    static constexpr int NST = 3;
+    static constexpr int PITCH = VD * 2 + 16;            // output tile: 16-byte pieces, a row's pairs in banks of their own
+    static constexpr int TILE = 1024, STAGE = TILE + (CHUNK * PITCH + 1023) / 1024 * 1024;
+    static constexpr int bytes = STAGE + NST * Rec<KD, VD>::LAM_OFF;
+};
+
+template <int KD, int VD>
+__global__ void __launch_bounds__(VD * 2 + 64) gdn_out_plain_kernel(GdnArgs a) {
     if (chain_wait()) return;
     using R = Rec<KD, VD>;
-    constexpr int NST = 3;
+    using S = OutPlainSmem<KD, VD>;
+    constexpr int NST = S::NST, NW = VD / 16;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int gb = blockIdx.x, h = blockIdx.y, H = a.H;
-    if (gb >= a.block_off[a.nseq]) return;
-    const int seq = find_seq(a.block_off, a.nseq, gb);
-    const int b = gb - a.block_off[seq];
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
+    const int nch = sq.nch;
     const int bc = 1 << block_log(nch);
-    const int c0 = a.chunk_off[seq] + b * bc;
+    const int c0 = sq.c0 + b * bc;
     const int nsteps = min(bc, nch - b * bc);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int64_t tok0 = sq.tok0 + (int64_t)b * bc * CHUNK, tok_end = sq.tok_end;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int row0 = warp * 16;
+    const bool direct = a.qkv_dt == LAMPA_F32;
+    unsigned char* tile = smem + S::TILE;
 
-    Pipe<NST> pipe;
-    pipe.bar = reinterpret_cast<uint64_t*>(smem);
-    pipe.stage = smem + 1024;
-    pipe.stage_bytes = R::LAM_OFF;
-    pipe.src = a.rec + ((size_t)c0 * H + h) * a.rec_bytes;
-    pipe.src_stride = (size_t)H * a.rec_bytes;
-    pipe.copy_bytes = R::LAM_OFF;
-    pipe.nsteps = nsteps;
-    pipe.dead = false;
-    pipe.status = a.status;
-    pipe.budget = a.poll_budget;
-    pipe.start();
-
+    Feed<NST, NW * 32 + 64, 1> feed;
+    feed.bar = reinterpret_cast<uint64_t*>(smem);
+    feed.stage = smem + S::STAGE;
+    feed.step_bytes = R::LAM_OFF;
+    feed.src = a.rec + ((size_t)c0 * H + h) * a.rec_bytes;
+    feed.src_stride = (size_t)H * a.rec_bytes;
+    feed.copy_bytes = R::LAM_OFF;
+    feed.nsteps = nsteps;
+    feed.status = a.status;
+    feed.budget = a.poll_budget;
+    feed.copy2 = 0;
+    feed.start(warp == NW);
+    auto tile_free = [] { asm volatile("bar.sync 2, %0;\n" :: "n"(NW * 32 + 32) : "memory"); };      // slab warps, joined by the storing warp
+    if (warp == NW) {
+        feed.produce(1);
+        return;
+    }
+    if (warp == NW + 1) {
+        for (int i = 0; i <= nsteps; ++i) {
+            feed.step(i);                              // tile i - 1 is written
+            if (i == 0) continue;
+            if (!direct) {
+                const int64_t t0 = tok0 + (int64_t)(i - 1) * CHUNK;
+                constexpr int LPR = VD / 8;                // lanes to a token's row
+#pragma unroll
+                for (int r = 0; r < CHUNK; r += 32 / LPR) {
+                    const int tk = r + lane / LPR, c = lane % LPR;
+                    const uint4 w = *reinterpret_cast<const uint4*>(tile + tk * S::PITCH + 16 * c);
+                    if (t0 + tk < tok_end) *reinterpret_cast<uint4*>((uint16_t*)a.o + ((size_t)(t0 + tk) * H + h) * VD + 8 * c) = w;
+                }
+                __syncwarp();
+            }
+            if (i < nsteps) asm volatile("bar.arrive 2, %0;\n" :: "n"(NW * 32 + 32) : "memory");
+        }
+        return;
+    }
     float C[KD / 8][4];
-    load_slab_f32<KD>(C, a.entry + ((size_t)gb * H + h) * R::STATE_FLOATS, KD, row0, lane);
+    load_slab_f32<KD>(C, a.entry + ((size_t)gb * H + h) * R::STATE_FLOATS, warp, lane);
     for (int i = 0; i < nsteps; ++i) {
-        const unsigned char* st = pipe.acquire(i);
+        const unsigned char* st = feed.step(i);
         const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
         const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
         const __nv_bfloat16* sQt = reinterpret_cast<const __nv_bfloat16*>(st + R::QT_OFF);
         const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + R::OL_OFF);
         uint32_t sp[KD / 16][4];
         pack_state<KD>(C, sp);
-        const int64_t t0 = tok0 + (int64_t)i * CHUNK;
-        auto emit = [&](auto scat) {
-#pragma unroll
-            for (int mt = 0; mt < 4; ++mt) {
-                float tmp[2][4];
-                read_tile<KD>(tmp, sp, sQt, mt, lane);
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int r = mt * 16 + g + hh * 8;
-                    const int64_t orow = t0 + r < tok_end ? out_row<decltype(scat)::value>(a, t0 + r) : -1;
-                    if (orow >= 0) {
-#pragma unroll
-                        for (int nt = 0; nt < 2; ++nt) {
-                            const int col = row0 + nt * 8 + 2 * t;
-                            const float2 ol = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sOl + R::TV::off(r, col)));
-                            store_out2(a.o, a.qkv_dt, ((size_t)orow * H + h) * VD + col,
-                                       ol.x + tmp[nt][2 * hh], ol.y + tmp[nt][2 * hh + 1]);
-                        }
-                    }
-                }
-            }
-        };
-        if (a.out_perm_rows > 0) emit(ScatterOn{}); else emit(ScatterOff{});
-        if (i + 1 < nsteps) {
+        if (i + 1 < nsteps) {                          // the state first: the next step waits for it
             load_slab_bf16<KD>(C, sBt, row0, lane);
-            state_times_mt<KD, Tile<KD>>(C, sp, sM, lane);
+            state_times_mt<KD>(C, sp, sM, lane);
+        }
+        float o[4][2][4];
+        read_tiles<KD, 4>(o, sp, sQt, 0, lane);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    const float2 ol = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sOl + R::TV::off(mt * 16 + g + hh * 8, row0 + nt * 8 + 2 * t)));
+                    o[mt][nt][2 * hh] += ol.x;
+                    o[mt][nt][2 * hh + 1] += ol.y;
+                }
+        if (i > 0) tile_free();
+        const int64_t t0 = tok0 + (int64_t)i * CHUNK;
+        auto emit = [&](auto put) {
+#pragma unroll
+            for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) put(mt * 16 + g + hh * 8, row0 + nt * 8 + 2 * t, o[mt][nt][2 * hh], o[mt][nt][2 * hh + 1]);
+        };
+        if (a.qkv_dt == LAMPA_BF16) {
+            emit([&](int r, int col, float x, float y) { *reinterpret_cast<uint32_t*>(tile + r * S::PITCH + 2 * col) = pack_bf16x2(x, y); });
+        } else if (!direct) {
+            emit([&](int r, int col, float x, float y) { *reinterpret_cast<__half2*>(tile + r * S::PITCH + 2 * col) = __floats2half2_rn(x, y); });
+        } else {
+            emit([&](int r, int col, float x, float y) {
+                if (t0 + r < tok_end) *reinterpret_cast<float2*>((float*)a.o + ((size_t)(t0 + r) * H + h) * VD + col) = make_float2(x, y);
+            });
         }
     }
-    pipe.finish();
+    feed.step(nsteps);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -500,6 +682,8 @@ __global__ void __launch_bounds__(VD * 2) gdn_out_plain_kernel(GdnArgs a) {
 // 64 events of 6,000 to 59,000 points: 2003 us with the registers unbounded and a group for every level of
 // the whole batch's length -> 968 us with this bound, the level count of L, and no sum over absent groups.
 // -------------------------------------------------------------------------------------------------
+constexpr int HIER_TILES = 4;
+
 template <int KD, int VD, int NG>
 __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hier_kernel(GdnArgs a) {
     if (chain_wait()) return;
@@ -508,16 +692,16 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
     constexpr int NS = VD / 16;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int gb = blockIdx.x, h = blockIdx.y, H = a.H;
-    if (gb >= a.block_off[a.nseq]) return;
-    const int seq = find_seq(a.block_off, a.nseq, gb);
-    const int b = gb - a.block_off[seq];
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
+    const int nch = sq.nch;
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
     const int bl = block_log(nch), bc = 1 << bl;
     const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
-    const int c0 = a.chunk_off[seq] + b * bc;
+    const int c0 = sq.c0 + b * bc;
     const int nsteps = min(bc, nch - b * bc);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int64_t tok0 = sq.tok0 + (int64_t)b * bc * CHUNK, tok_end = sq.tok_end;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int grp = warp / NS, slab = warp - grp * NS;
@@ -556,7 +740,7 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
             const int lh = (grp - 1) * NLW + x;
             if (lh < nhigh && ((b >> lh) & 1)) {
                 live |= 1u << x;
-                load_slab_f32<KD>(C[x], a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, KD, row0, lane);
+                load_slab_f32<KD>(C[x], a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, slab, lane);
             }
         }
     }
@@ -602,14 +786,18 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
             if (do_read) {
                 const float* lr = sLam + lam_row * CHUNK;
 #pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    float tmp[2][4];
-                    read_tile<KD>(tmp, sp, sQt, mt, lane);
-                    const float l0 = lr[mt * 16 + g], l1 = lr[mt * 16 + g + 8];
+                for (int m2 = 0; m2 < 4; m2 += HIER_TILES) {
+                    float tmp[HIER_TILES][2][4];
+                    read_tiles<KD, HIER_TILES>(tmp, sp, sQt, m2, lane);
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) {
-                        O[mt][nt][0] += l0 * tmp[nt][0]; O[mt][nt][1] += l0 * tmp[nt][1];
-                        O[mt][nt][2] += l1 * tmp[nt][2]; O[mt][nt][3] += l1 * tmp[nt][3];
+                    for (int x = 0; x < HIER_TILES; ++x) {
+                        const int mt = m2 + x;
+                        const float l0 = lr[mt * 16 + g], l1 = lr[mt * 16 + g + 8];
+#pragma unroll
+                        for (int nt = 0; nt < 2; ++nt) {
+                            O[mt][nt][0] += l0 * tmp[x][nt][0]; O[mt][nt][1] += l0 * tmp[x][nt][1];
+                            O[mt][nt][2] += l1 * tmp[x][nt][2]; O[mt][nt][3] += l1 * tmp[x][nt][3];
+                        }
                     }
                 }
             }
@@ -619,11 +807,11 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
                 } else {
                     if (add_b) load_slab_bf16<KD>(C[x], sBt, row0, lane);
                     else zero_state<KD>(C[x]);
-                    if (do_mma) state_times_mt<KD, Tile<KD>>(C[x], sp, sM, lane);
+                    if (do_mma) state_times_mt<KD>(C[x], sp, sM, lane);
                 }
             } else if (do_mma) {
                 zero_state<KD>(C[x]);
-                state_times_mt<KD, Tile<KD>>(C[x], sp, sM, lane);
+                state_times_mt<KD>(C[x], sp, sM, lane);
             }
         }
 
@@ -685,34 +873,47 @@ static int set_smem(KernelT kern, int bytes) {
 #define LAMPA_TRY(x) do { int rc_ = (x); if (rc_ != LAMPA_OK) return rc_; } while (0)
 #define LAMPA_LAUNCHED() do { if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA; } while (0)
 
-template <int KD, int VD>
-static int launch_compose(const GdnArgs& a, cudaStream_t st) {
+template <int KD, int VD, int SPLIT>
+static int launch_compose_split(const GdnArgs& a, cudaStream_t st) {
     using R = Rec<KD, VD>;
-    const int smem = 1024 + 3 * R::PRE_BYTES;
-    LAMPA_TRY(set_smem(gdn_compose_kernel<KD, VD>, smem));
+    using G = Compose<KD, VD, SPLIT>;
+    const int smem = 1024 + G::NST * G::GRP * (R::M_BYTES + R::BT_BYTES);
+    LAMPA_TRY(set_smem(gdn_compose_kernel<KD, VD, SPLIT>, smem));
     ProfScope prof("gdn_compose", st);
-    launch_chained(gdn_compose_kernel<KD, VD>, dim3(a.nb_max, a.H), (KD + VD) * 2, smem, st, a);
+    launch_chained(gdn_compose_kernel<KD, VD, SPLIT>, dim3(a.nb_max, a.H, SPLIT), G::NW * 32 + 32, smem, st, a);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
+}
+template <int KD, int VD>
+static int launch_compose(const GdnArgs& a, cudaStream_t st) {
+    return (int64_t)a.nb_max * a.H * 2 <= sm_count() ? launch_compose_split<KD, VD, 2>(a, st) : launch_compose_split<KD, VD, 1>(a, st);
+}
+
+template <int KD, int VD, bool HIER, int NW>
+static int launch_level_slabs(const GdnArgs& a, int levels, cudaStream_t st) {
+    const int smem = LevelSmem<KD, NW>::bytes;
+    LAMPA_TRY(set_smem(gdn_level_kernel<KD, VD, HIER, NW>, smem));
+    ProfScope prof(HIER ? "gdn_level_hier" : "gdn_level_plain", st);
+    launch_chained(gdn_level_kernel<KD, VD, HIER, NW>, dim3(a.nseq, a.H, levels * (VD / 16 / NW)), NW * 32 + 32, smem, st, a);
+    LAMPA_LAUNCHED();
+    return LAMPA_OK;
+}
+template <int KD, int VD, bool HIER>
+static int launch_level(const GdnArgs& a, int levels, cudaStream_t st) {
+    return (int64_t)a.nseq * a.H * levels * (VD / 16) <= 2 * sm_count() ? launch_level_slabs<KD, VD, HIER, 1>(a, levels, st)
+                                                                       : launch_level_slabs<KD, VD, HIER, VD / 16>(a, levels, st);
 }
 
 template <int KD, int VD>
 int launch_scan_plain(const GdnArgs& a, cudaStream_t st) {
-    using R = Rec<KD, VD>;
     LAMPA_TRY((launch_compose<KD, VD>(a, st)));
-    {
-        const int smem = 1024 + 3 * R::BLK_BYTES;
-        LAMPA_TRY(set_smem(gdn_level_kernel<KD, VD, false>, smem));
-        ProfScope prof("gdn_level_plain", st);
-        launch_chained(gdn_level_kernel<KD, VD, false>, dim3(a.nseq, a.H, 1), VD * 2, smem, st, a);
-        LAMPA_LAUNCHED();
-    }
+    LAMPA_TRY((launch_level<KD, VD, false>(a, 1, st)));
     if (KD == 64 && VD == 64 && a.use_umma) return launch_out_plain_umma(a, st);
     {
-        const int smem = 1024 + 3 * R::LAM_OFF;
+        const int smem = OutPlainSmem<KD, VD>::bytes;
         LAMPA_TRY(set_smem(gdn_out_plain_kernel<KD, VD>, smem));
         ProfScope prof("gdn_out_plain", st);
-        launch_chained(gdn_out_plain_kernel<KD, VD>, dim3(a.nb_max, a.H), VD * 2, smem, st, a);
+        launch_chained(gdn_out_plain_kernel<KD, VD>, dim3(a.nb_max, a.H), VD * 2 + 64, smem, st, a);
         LAMPA_LAUNCHED();
     }
     return LAMPA_OK;
@@ -733,16 +934,11 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
 
 template <int KD, int VD>
 int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
-    using R = Rec<KD, VD>;
     const int ng = 1 + (a.nhigh_max + NLW - 1) / NLW;
     if (ng > MAX_GROUPS) return LAMPA_ERR_UNSUPPORTED;
     if (a.nhigh_max > 0) {
         LAMPA_TRY((launch_compose<KD, VD>(a, st)));
-        const int smem = 1024 + 3 * R::BLK_BYTES;
-        LAMPA_TRY(set_smem(gdn_level_kernel<KD, VD, true>, smem));
-        ProfScope prof("gdn_level_hier", st);
-        launch_chained(gdn_level_kernel<KD, VD, true>, dim3(a.nseq, a.H, a.nhigh_max), VD * 2, smem, st, a);
-        LAMPA_LAUNCHED();
+        LAMPA_TRY((launch_level<KD, VD, true>(a, a.nhigh_max, st)));
     }
     if (KD == 64 && VD == 64 && a.nhigh_max <= 5 && a.use_umma) return launch_out_hier_umma(a, st);
     if (ng == 1) return launch_out_hier<KD, VD, 1>(a, st);
@@ -757,7 +953,7 @@ int launch_final_high(const GdnArgs& a, float* states, cudaStream_t st) {
     const int smem = 1024 + 3 * R::PRE_BYTES;
     LAMPA_TRY(set_smem(hgdn_final_high_kernel<KD, VD>, smem));
     ProfScope prof("hgdn_final_high", st);
-    launch_chained(hgdn_final_high_kernel<KD, VD>, dim3(a.nseq, a.H, a.L - ELL0), VD * 2, smem, st, a, states);
+    launch_chained(hgdn_final_high_kernel<KD, VD>, dim3(a.nseq, a.H, a.L - ELL0), VD * 2 + 32, smem, st, a, states);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
 }

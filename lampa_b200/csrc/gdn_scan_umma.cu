@@ -76,6 +76,16 @@ __host__ __device__ constexpr int ustage_bytes(int LC) { return (STAGE_TILES + L
 // instruction descriptor: D fp32, A/B bf16, both K-major, M = 128, N = 128
 constexpr uint32_t UMMA_IDESC = umma_idesc(128, 128);
 
+// columns 16p .. 16p + 15 of row v of an entry state
+__device__ __forceinline__ void load_state16(float (&x)[16], const float* state, int v, int p) {
+    const float4* e = reinterpret_cast<const float4*>(state + UR::state_at(v, 16 * p));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 f = e[i];
+        x[2 * i] = f.x; x[2 * i + 1] = f.y; x[8 + 2 * i] = f.z; x[9 + 2 * i] = f.w;
+    }
+}
+
 // Launch order of the (block, head) units.  A unit's time grows with the number of level pairs it
 // carries (3 to 5, from the set bits of its block index), and 240 units on 148 SMs leave the second
 // round partly empty: handing the long units out first lets the short ones fill the tail.
@@ -110,16 +120,16 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
         gb = blockIdx.x % a.nb_max;
         h = blockIdx.x / a.nb_max;
     }
-    if (gb >= a.block_off[a.nseq]) return;
-    const int seq = find_seq(a.block_off, a.nseq, gb);
-    const int b = gb - a.block_off[seq];
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
+    const int nch = sq.nch;
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
     const int bl = block_log(nch), bc = 1 << bl;
     const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
-    const int c0 = a.chunk_off[seq] + b * bc;
+    const int c0 = sq.c0 + b * bc;
     const int nsteps = min(bc, nch - b * bc);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int64_t tok0 = sq.tok0 + (int64_t)b * bc * CHUNK, tok_end = sq.tok_end;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int wg = warp >> 2;                          // 0..3: state columns / tokens 16*wg .. 16*wg+15
     const int row = (warp & 3) * 32 + lane;            // TMEM lane = row of the pair's A operand
@@ -169,13 +179,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
             for (int i = 0; i < 16; ++i) x[i] = 0.f;
             if (s >= bl && s < nslots) {
                 const int lh = (live_pack >> (4 * (s - bl))) & 15;
-                const float4* e = reinterpret_cast<const float4*>(
-                    a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * UR::STATE_FLOATS + (size_t)v * UKD + 16 * part);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 f = e[i];
-                    x[4 * i] = f.x; x[4 * i + 1] = f.y; x[4 * i + 2] = f.z; x[4 * i + 3] = f.w;
-                }
+                load_state16(x, a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * UR::STATE_FLOATS, v, part);
             }
             tmem_st_bf16x16(tlane + TM_A + 32 * p + 8 * part, x);
         }
@@ -444,15 +448,15 @@ __global__ void __launch_bounds__(PTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs
 
     const int H = a.H, npair = (H + 1) / 2;
     const int gb = blockIdx.x / npair, h0 = 2 * (blockIdx.x % npair);
-    if (gb >= a.block_off[a.nseq]) return;
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
     const int nheads = min(2, H - h0);
-    const int seq = find_seq(a.block_off, a.nseq, gb);
-    const int b = gb - a.block_off[seq];
-    const int nch = a.chunk_off[seq + 1] - a.chunk_off[seq];
+    const int nch = sq.nch;
     const int bc = 1 << block_log(nch);
-    const int c0 = a.chunk_off[seq] + b * bc;
+    const int c0 = sq.c0 + b * bc;
     const int nsteps = min(bc, nch - b * bc);
-    const int64_t tok0 = a.tok_off[seq] + (int64_t)b * bc * CHUNK, tok_end = a.tok_off[seq + 1];
+    const int64_t tok0 = sq.tok0 + (int64_t)b * bc * CHUNK, tok_end = sq.tok_end;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int sp = warp & 3, cq = (warp >> 2) & 3;     // lane quarter; 16 state columns and 16 tokens
     const int sub = lane >> 4, v = 16 * sp + (lane & 15);   // head of the pair, state row
@@ -481,12 +485,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) gdn_out_plain_umma_kernel(GdnArgs
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = 0.f;
         if (sub < nheads) {
-            const float4* e = reinterpret_cast<const float4*>(a.entry + ((size_t)gb * H + h0 + sub) * UR::STATE_FLOATS + (size_t)v * UKD + 16 * cq);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 f = e[i];
-                x[4 * i] = f.x; x[4 * i + 1] = f.y; x[4 * i + 2] = f.z; x[4 * i + 3] = f.w;
-            }
+            load_state16(x, a.entry + ((size_t)gb * H + h0 + sub) * UR::STATE_FLOATS, v, cq);
         }
         tmem_st_bf16x16(tlane + PTM_A + 8 * cq, x);
     }

@@ -110,8 +110,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col = 2 * warp + (lane >> 4), kl = lane & 15;
     const int v0 = blockIdx.z * TAIL_COLS, vv = v0 + col;
-    const int nch = ta.n0 >= 0 ? ta.n0 : a.chunk_off[seq + 1] - a.chunk_off[seq];
-    const int64_t tok0 = ta.n0 >= 0 ? (int64_t)seq * a.fixed_stride : a.tok_off[seq];
+    int nch = ta.n0;
+    int64_t tok0 = (int64_t)seq * a.fixed_stride, tok_end = 0;
+    if (ta.n0 < 0) {
+        const SeqLoc sq = locate_seq(a, seq);
+        nch = sq.nch; tok0 = sq.tok0; tok_end = sq.tok_end;
+    }
 
     // rows [t0, t0 + len) of the inputs as the kernel uses them; rows up to 64 become null tokens.  Eight elements per
     // thread and step, K / 8 threads per row, every load in flight before the first is used.
@@ -213,7 +217,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 
     if (nch > 0) {
         const int64_t t0 = tok0 + (int64_t)(nch - 1) * CHUNK;
-        stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, a.tok_off[seq + 1] - t0), false);
+        stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - t0), false);
         // After a whole chunk level l >= 1 holds tokens 64 - 2^l .. 63 - 2^(l-1), carried through the rest: one running
         // state from its first token on, so that before token 32 there is one state to advance and six only at the end.
         auto advance = [&](auto first, int t0, int t1) {         // levels first .. 6 have started

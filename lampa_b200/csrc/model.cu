@@ -765,11 +765,6 @@ model_update_kernel(UpdateArgs a, const __grid_constant__ CUtensorMap mo, const 
     if (warp == 0) tmem_dealloc(taddr, 256);
 }
 
-static int sm_count() {
-    static const int sms = [] { int d = 0, n = 148; if (cudaGetDevice(&d) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d); return n; }();
-    return sms;
-}
-
 }  // namespace lampa
 
 using namespace lampa;
