@@ -197,7 +197,6 @@ __device__ __forceinline__ void store_out2(void* o, int dt, size_t idx, float x,
 }
 
 int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st);
-int launch_out_plain_umma(const GdnArgs& a, cudaStream_t st);  // K = V = 64
 int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st);   // K = V = 64, 2-byte q/k/v
 template <int KD, int VD> int launch_final_high(const GdnArgs& a, float* states, cudaStream_t st);
 // The end of every sequence in fp32 (gdn_state.cu): token levels of the state, and the tokens behind the last whole chunk.

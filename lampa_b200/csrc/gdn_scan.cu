@@ -551,6 +551,10 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
 // output, plain rule:  O_n = O_local + Q~ S_n ;  S_{n+1} = M S_n + B
 // VD / 16 slab warps, the copying warp, and one that stores: a chunk's output goes through a [token][v] tile in shared memory
 // and leaves as whole rows, under the next chunk's products.  (fp32 outputs go straight from the registers.)
+// Bound by streaming the records where the blocks fill the GPU (65,536 tokens, 8 heads: 56 us for 317 MB, 5.7 TB/s of the
+// measured 6.5), by the step of a block elsewhere: about 1000 cycles, 64 products of a warp among them.  The same pass on
+// tcgen05 (state in tensor memory, an epilogue of 16 warps around one MMA per chunk) needs two hand-overs per chunk and
+// took 2800 cycles: 18.8 us against 14.7 at 6,144 tokens and 4 heads, 60.4 against 59.9 at 65,536 and 8.
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
 struct OutPlainSmem {
@@ -908,14 +912,11 @@ template <int KD, int VD>
 int launch_scan_plain(const GdnArgs& a, cudaStream_t st) {
     LAMPA_TRY((launch_compose<KD, VD>(a, st)));
     LAMPA_TRY((launch_level<KD, VD, false>(a, 1, st)));
-    if (KD == 64 && VD == 64 && a.use_umma) return launch_out_plain_umma(a, st);
-    {
-        const int smem = OutPlainSmem<KD, VD>::bytes;
-        LAMPA_TRY(set_smem(gdn_out_plain_kernel<KD, VD>, smem));
-        ProfScope prof("gdn_out_plain", st);
-        launch_chained(gdn_out_plain_kernel<KD, VD>, dim3(a.nb_max, a.H), VD * 2 + 64, smem, st, a);
-        LAMPA_LAUNCHED();
-    }
+    const int smem = OutPlainSmem<KD, VD>::bytes;
+    LAMPA_TRY(set_smem(gdn_out_plain_kernel<KD, VD>, smem));
+    ProfScope prof("gdn_out_plain", st);
+    launch_chained(gdn_out_plain_kernel<KD, VD>, dim3(a.nb_max, a.H), VD * 2 + 64, smem, st, a);
+    LAMPA_LAUNCHED();
     return LAMPA_OK;
 }
 
