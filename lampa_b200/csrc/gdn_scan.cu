@@ -265,7 +265,8 @@ struct Feed {
 // the identity; SPW slabs to a warp.  A slab's 32 products of a step take 290 cycles of a scheduler and its fragments of M 64
 // cycles of the SM's shared-memory pipe, so with one slab to a warp the eight warps of a block spend as long on reading M
 // eight times as on the products.  Two slabs to a warp share the fragments (SPLIT = 1).  SPLIT = 2: S and P in CTAs of their
-// own, one slab to a warp and one warp to a scheduler: the shortest step, where all halves run at once on SMs of their own.
+// own, one slab to a warp and one warp to a scheduler: the shortest step, taken while the halves of all blocks come to at most
+// two to an SM (12 blocks of 8 chunks, 8 heads: 12.2 -> 10.7 us; 4 heads, one to an SM: 11.3 -> 10.7).
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD, int SPLIT>
 struct Compose {
@@ -273,7 +274,7 @@ struct Compose {
     static constexpr int SPW = SPLIT == 1 && KD == 64 ? 2 : 1;
     static constexpr int SLABS = SPLIT == 1 ? SLABS_S + SLABS_P : (SLABS_S > SLABS_P ? SLABS_S : SLABS_P);
     static constexpr int NW = SLABS / SPW;
-    static constexpr int GRP = SPLIT == 1 ? 1 : 2, NST = SPLIT == 1 ? 3 : 4;       // 74 KB: three CTAs to an SM; 197 KB: one
+    static constexpr int GRP = 1, NST = 3;       // 74 KB: three CTAs to an SM
     static_assert(SLABS % SPW == 0 && SLABS_S % SPW == 0, "a warp's slabs are of one kind");
 };
 
@@ -890,7 +891,7 @@ static int launch_compose_split(const GdnArgs& a, cudaStream_t st) {
 }
 template <int KD, int VD>
 static int launch_compose(const GdnArgs& a, cudaStream_t st) {
-    return (int64_t)a.nb_max * a.H * 2 <= sm_count() ? launch_compose_split<KD, VD, 2>(a, st) : launch_compose_split<KD, VD, 1>(a, st);
+    return (int64_t)a.nb_max * a.H <= sm_count() ? launch_compose_split<KD, VD, 2>(a, st) : launch_compose_split<KD, VD, 1>(a, st);
 }
 
 template <int KD, int VD, bool HIER, int NW>
