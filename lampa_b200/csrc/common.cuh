@@ -195,13 +195,17 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 // `if (chain_wait()) return;` makes all that follows depend on it, so that no load that counts as invariant
 // (const __restrict__, __ldg) can be moved in front of it.
 // 6,144 tokens, 4 heads: 58.4 -> 50.5 us over four launches; one 9,001-hit event through the model: 475 -> 420 over 27.
-// (No kernel signals earlier, griddepcontrol.launch_dependents: the next grid then fills the SMs that happen to be free,
-// two or three CTAs to an SM beside idle ones: 56 and 447 us, and 486 instead of 463 for a 60,000-hit event.)
+// A kernel may let the next one start before its own end (chain_signal, once all its CTAs have passed it or left).  That is
+// for kernels that leave most of the GPU idle and for a next one that can do without them: everywhere else the next grid only
+// fills the SMs that happen to be free, two or three CTAs to an SM beside idle ones (56 and 447 us, and 486 instead of 463 for a
+// 60,000-hit event).  chain_signal comes behind chain_wait: what the kernel was waiting for is complete for the next one
+// too, which may read it (from L2) before its own wait.  That one still waits before it ends, so that its end means theirs.
 __device__ __forceinline__ bool chain_wait() {
     uint32_t never;
     asm volatile("griddepcontrol.wait;\n mov.u32 %0, 0;\n" : "=r"(never) :: "memory");
     return never != 0;
 }
+__device__ __forceinline__ void chain_signal() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 inline cudaLaunchAttribute chained_attribute() {
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -94,6 +94,7 @@ struct GdnArgs {
     int32_t* status;
     int use_umma;                         // tcgen05 kernels where they exist (K = V = 64)
     int poll_budget;                      // polls before a device wait gives up (MBAR_POLLS unless a test lowers it)
+    int signal;                           // a prefill's output pass and chunk levels let the next kernel in (chain_signal)
     long long* ticks; int ticks_ctas;     // stage clocks for tuning: [ticks_ctas][16] or NULL (lampa_debug_set_tick_buffer)
 };
 
@@ -206,6 +207,7 @@ struct TailArgs {
     int tail;                             // tokens behind them (only with n0 >= 0)
     int one_count;
     int32_t* arrivals;                    // set to zero, or NULL: the arrival counter of the decode steps to come
+    int early;                            // this call's kernels in front signal early (GdnArgs::signal)
 };
 template <int KD, int VD> int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st);
 

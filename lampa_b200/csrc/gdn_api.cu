@@ -104,6 +104,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     static const int no_umma = [] { const char* e = getenv("LAMPA_B200_NO_UMMA"); return (e && e[0] == '1') ? 1 : 0; }();
     a.use_umma = (no_umma || g_force_mma_sync) ? 0 : 1;
     a.poll_budget = poll_budget();
+    a.signal = 0;
     a.ticks = g_ticks;
     a.ticks_ctas = g_ticks_ctas;
 }
@@ -111,7 +112,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
 int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const void* v, const void* g,
         const void* beta, const void* lam, const float* h0, const int64_t* cu, void* o, float* ht,
         void* ws, size_t ws_bytes, int32_t* status, void* stream, const int64_t* out_perm = nullptr,
-        int64_t out_perm_rows = 0, int fixed_stride = 0, bool planned = false) {
+        int64_t out_perm_rows = 0, int fixed_stride = 0, bool planned = false, bool signal = false) {
     Layout l;
     int rc = make_layout(d, hier, l);
     if (rc != LAMPA_OK) return rc;
@@ -129,6 +130,7 @@ int run(const lampa_gdn_desc* d, bool hier, const void* q, const void* k, const 
     fill_args(d, hier, l, base, cu, status, a);
     a.q = q; a.k = k; a.v = v; a.g = g; a.beta = beta; a.lam = lam; a.h0 = h0; a.ht = ht; a.o = o;
     a.out_perm = out_perm; a.out_perm_rows = out_perm ? out_perm_rows : 0;
+    a.signal = signal ? 1 : 0;
     if (fixed_stride > 0) { a.fixed_stride = fixed_stride; a.total_tokens = (long long)d->B * fixed_stride; }
 
     PlanArgs p;
@@ -284,7 +286,7 @@ extern "C" int lampa_hgdn_final_state_counted(const lampa_gdn_desc* d, const voi
     fill_args(d, true, l, (char*)ws, cu_seqlens, status, a);
     a.k = k; a.v = v; a.g = g; a.beta = beta;
     TailArgs ta;
-    ta.states = states; ta.counts = counts; ta.n0 = -1; ta.tail = 0; ta.one_count = 0; ta.arrivals = arrivals;
+    ta.states = states; ta.counts = counts; ta.n0 = -1; ta.tail = 0; ta.one_count = 0; ta.arrivals = arrivals; ta.early = 0;
     return final_state(d, a, ta, (cudaStream_t)stream);
 }
 
@@ -307,7 +309,7 @@ extern "C" int lampa_hgdn_prefill_counted(const lampa_gdn_desc* d, const void* q
     if (!q || !k || !v || !g || !beta || !lam || !o || !ws || !states || !counts) return LAMPA_ERR_ARG;
     if (whole.T > 0 && d->L < ELL0) return LAMPA_ERR_LEVELS;
     if (whole.T > 0) {
-        rc = run(&whole, true, q, k, v, g, beta, lam, nullptr, nullptr, o, nullptr, ws, ws_bytes, status, stream, nullptr, 0, d->T);
+        rc = run(&whole, true, q, k, v, g, beta, lam, nullptr, nullptr, o, nullptr, ws, ws_bytes, status, stream, nullptr, 0, d->T, false, true);
         if (rc != LAMPA_OK) return rc;
     }
     GdnArgs a;
@@ -316,6 +318,7 @@ extern "C" int lampa_hgdn_prefill_counted(const lampa_gdn_desc* d, const void* q
     a.q = q; a.k = k; a.v = v; a.g = g; a.beta = beta; a.lam = lam; a.o = o;
     TailArgs ta;
     ta.states = states; ta.counts = counts; ta.n0 = whole.T / CHUNK; ta.tail = d->T - whole.T; ta.one_count = 1; ta.arrivals = arrivals;
+    a.signal = ta.early = whole.T > 0;                   // the output pass has signalled, and everything in front of it is complete
     return final_state(d, a, ta, (cudaStream_t)stream);
 }
 

@@ -104,14 +104,14 @@ __device__ __forceinline__ void load_slab_bf16(float (&C)[KD / 8][4], const __nv
     }
 }
 // slab `slab` of an fp32 state (Rec::state_at) in shared or global memory
-template <int KD>
+template <int KD, bool GLOBAL = false>
 __device__ __forceinline__ void load_slab_f32(float (&C)[KD / 8][4], const float* s, int slab, int lane) {
     const float4* p4 = reinterpret_cast<const float4*>(s) + slab * (KD / 8) * 32 + lane;
 #pragma unroll
     for (int p = 0; p < KD / 16; ++p)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-            const float4 f = p4[(2 * p + hh) * 32];
+            const float4 f = GLOBAL ? __ldcg(p4 + (2 * p + hh) * 32) : p4[(2 * p + hh) * 32];
             C[2 * p][2 * hh] = f.x; C[2 * p][2 * hh + 1] = f.y; C[2 * p + 1][2 * hh] = f.z; C[2 * p + 1][2 * hh + 1] = f.w;
         }
 }
@@ -475,7 +475,10 @@ __global__ void __launch_bounds__(NW * 32 + 32) gdn_level_kernel(GdnArgs a) {
 // -------------------------------------------------------------------------------------------------
 template <int KD, int VD>
 __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a, float* states) {
-    if (chain_wait()) return;
+    // In a prefill the output pass in front lets this one in at its start: it needs nothing of that pass, only what was complete
+    // before it, so it runs beside it, signals in turn and waits at its end.
+    if (a.signal) chain_signal();
+    else if (chain_wait()) return;
     using R = Rec<KD, VD>;
     constexpr int NST = 3, NW = VD / 16;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -507,11 +510,12 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
         feed.start(warp == NW);
         if (warp == NW) {
             feed.produce();
+            if (a.signal) (void)chain_wait();
             return;
         }
         if (lev >= bl) {
             const int gb = sq.gb0 + (n >> bl);
-            load_slab_f32<KD>(C, a.entry + (((size_t)gb * a.nhigh_max + (lev - bl)) * H + h) * R::STATE_FLOATS, warp, lane);
+            load_slab_f32<KD, true>(C, a.entry + (((size_t)gb * a.nhigh_max + (lev - bl)) * H + h) * R::STATE_FLOATS, warp, lane);
         }
         for (int i = 0; i < feed.nsteps; ++i) {
             const unsigned char* st = feed.step(i);
@@ -537,6 +541,7 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
             }
         }
     }
+    if (a.signal && chain_wait()) return;
     if (warp == NW) return;
     float* dst = states + ((size_t)seq * H + h) * KD * VD * a.L + ELL0 + lev;
 #pragma unroll
@@ -624,7 +629,7 @@ __global__ void __launch_bounds__(VD * 2 + 64) gdn_out_plain_kernel(GdnArgs a) {
         return;
     }
     float C[KD / 8][4];
-    load_slab_f32<KD>(C, a.entry + ((size_t)gb * H + h) * R::STATE_FLOATS, warp, lane);
+    load_slab_f32<KD, true>(C, a.entry + ((size_t)gb * H + h) * R::STATE_FLOATS, warp, lane);
     for (int i = 0; i < nsteps; ++i) {
         const unsigned char* st = feed.step(i);
         const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
@@ -692,6 +697,7 @@ constexpr int HIER_TILES = 4;
 template <int KD, int VD, int NG>
 __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hier_kernel(GdnArgs a) {
     if (chain_wait()) return;
+    if (a.signal) chain_signal();
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     constexpr int NS = VD / 16;
@@ -745,7 +751,7 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
             const int lh = (grp - 1) * NLW + x;
             if (lh < nhigh && ((b >> lh) & 1)) {
                 live |= 1u << x;
-                load_slab_f32<KD>(C[x], a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, slab, lane);
+                load_slab_f32<KD, true>(C[x], a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, slab, lane);
             }
         }
     }

@@ -19,19 +19,44 @@ __device__ __forceinline__ float round_like(float x, int dt) {
     return x;
 }
 
+// Elements as they lie in memory, and what they stand for: the loads of a phase are all in flight before the first is looked at.
+// From L2, past an L1 that may hold what an earlier kernel read there: the tail reads its inputs while the kernel in front
+// of it still runs.
+__device__ __forceinline__ uint32_t load_raw(const void* p, size_t i, int dt, bool live) {
+    uint32_t u = 0u;
+    if (live && dt == LAMPA_F32) u = __ldcg((const unsigned int*)p + i);
+    if (live && dt != LAMPA_F32) u = __ldcg((const unsigned short*)p + i);
+    return u;
+}
+__device__ __forceinline__ float raw_float(uint32_t u, int dt) {
+    return dt == LAMPA_F32 ? __uint_as_float(u) : dt == LAMPA_BF16 ? __uint_as_float(u << 16) : __half2float(__ushort_as_half((unsigned short)u));
+}
+// eight consecutive 2-byte elements of a 16-byte aligned tensor
+__device__ __forceinline__ uint4 load8_raw(const void* p, size_t i, bool live) {
+    return live ? __ldcg(reinterpret_cast<const uint4*>((const uint16_t*)p + i)) : make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ void raw_floats(const uint4& u, int dt, float (&x)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 f = dt == LAMPA_BF16 ? unpack_bf16x2(w[e]) : __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+        x[2 * e] = f.x; x[2 * e + 1] = f.y;
+    }
+}
+
 // Eight consecutive elements as floats (zeros where `live` is false): 16-byte loads where the base allows them
-__device__ __forceinline__ void load8_as_float(const void* p, size_t i, int dt, bool live, float (&x)[8]) {
+__device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, bool live, float (&x)[8]) {
     if (!live) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) x[e] = 0.f;
     } else if (((uintptr_t)p & 15) != 0) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = load_as_float(p, i + e, dt);
+        for (int e = 0; e < 8; ++e) x[e] = raw_float(load_raw(p, i + e, dt, true), dt);
     } else if (dt == LAMPA_F32) {
-        const float4 u = __ldg(reinterpret_cast<const float4*>((const float*)p + i)), v = __ldg(reinterpret_cast<const float4*>((const float*)p + i) + 1);
+        const float4 u = __ldcg(reinterpret_cast<const float4*>((const float*)p + i)), v = __ldcg(reinterpret_cast<const float4*>((const float*)p + i) + 1);
         x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
     } else {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>((const uint16_t*)p + i));
+        const uint4 u = __ldcg(reinterpret_cast<const uint4*>((const uint16_t*)p + i));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -42,16 +67,565 @@ __device__ __forceinline__ void load8_as_float(const void* p, size_t i, int dt, 
 }
 
 // -------------------------------------------------------------------------------------------------
-// End of a sequence, token by token in fp32: the token levels 0..6 after its last whole chunk (the
-// recurrence over that chunk from an empty state, as the reference's postprocess_prefill_hstate_
-// does, models/hattention/kernel.py:377-466), then, for a prefill, the T mod 64 tokens behind it with
-// all levels and their outputs (what the reference hands to its step function, kernel.py:470-560).
-// Inside one chunk the cascade is fixed: before token t > 0, levels 0..tz(t) collapse into level
-// tz(t) + 1 (tz = trailing zeros); before the first token behind n0 chunks, the token levels and the
-// trailing full chunk levels collapse into level 7 + tz(n0), after which the live chunk levels are
-// the set bits of n0 and do not change any more: they sit in HS register slots, in bit order.
-// Without a tail a ragged last chunk (cu_seqlens) is completed with null tokens (k = v = 0,
-// beta = 0, g = 0).  Also writes counts.
+// End of a sequence, in fp32: the token levels 0..6 after its last whole chunk (the recurrence over that
+// chunk from an empty state, as the reference's postprocess_prefill_hstate_ does,
+// models/hattention/kernel.py:377-466), then, for a prefill, the T mod 64 tokens behind it with all levels
+// and their outputs (what the reference hands to its step function, kernel.py:470-560).
+// Inside one chunk the cascade is fixed: after r tokens level l >= 1 holds 2^(l-1) tokens exactly when bit
+// l-1 of r - 1 is set, the older ones higher up, and level 0 the last token.  Before the first token behind
+// n0 chunks, the token levels and the trailing full chunk levels collapse into level 7 + tz(n0), after which
+// the live chunk levels are the set bits of n0 and do not change any more ("slots", in bit order).
+// Without a tail a ragged last chunk (cu_seqlens) is completed with null tokens (k = v = 0, beta = 0, g = 0).
+// Also writes counts.
+//
+// 64 tokens at a time in closed form instead of one after the other.  With G the running sum of g and
+// E_ij = e^{G_i - G_j} (j <= i), the states are independent linear recurrences with the same transitions:
+//     T = (I + tril(diag(beta) K K^T .* E, -1))^-1 diag(beta)          R = (tril(Q K^T) .* E) T
+//     a level that holds tokens j in J:   S = K^T diag(e^{Gl-G}) T[:, J] V[J]
+//     a slot that enters with X:          X <- e^{Gl} X - K^T diag(e^{Gl-G}) T diag(e^G) K X
+//     o_i = sum_j lambda[i, bit_length(i^j)] R_ij v_j + sum_slots lambda[i, slot] (e^{G_i} q_i X - (R diag(e^G) K X)_i)
+// all of it fp32 multiply-adds (no operand is rounded, G is summed in double so that E is exact to fp32).
+// A CTA takes eight state columns of a (sequence, head); T and R do not depend on the column and are formed
+// by each: 1.5 M multiply-adds per CTA, two halves of the CTA on the last chunk and the tail side by side.
+// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 34 us, of which 20 - 25 run beside the
+// output pass (launch_chained): the call 95 -> 77 us.  What bounds it is the shared-memory pipe (a 16-byte load of a warp
+// returns 512 bytes, four cycles, for 16 multiply-adds of four).
+// -------------------------------------------------------------------------------------------------
+constexpr int TAIL_COLS = 8, TAIL_THREADS = 512, TAIL_GRP = 256, TAIL_BATCH = 4;      // states formed at a time
+constexpr int TAIL_AP = CHUNK + 4, TAIL_XP = TAIL_BATCH * TAIL_COLS + 4;              // pitches of 64- and 32-wide rows
+
+template <int KD>
+struct TailSmem {                                            // offsets in floats
+    static constexpr int KP = KD + 4;
+    static constexpr int SCAL = 2 * CHUNK + 3 * CHUNK;       // G (double), e^G, e^{Gl-G}, beta
+    static constexpr int CH = CHUNK * KP + CHUNK * TAIL_AP + CHUNK * TAIL_COLS + SCAL;       // k, A -> T, v, scalars of one chunk
+    static constexpr int K_ = 0, A_ = CHUNK * KP, V_ = A_ + CHUNK * TAIL_AP, S_ = V_ + CHUNK * TAIL_COLS;
+    static constexpr int Z = CH;                             // [64][XP]
+    static constexpr int SUM = Z + CHUNK * TAIL_XP;          // [KD][8] all tokens of the last chunk
+    static constexpr int B = SUM + KD * TAIL_COLS;           // (tail only) the tail's chunk
+    static constexpr int Q = B + CH;                         // [64][KP]
+    static constexpr int P = Q + CHUNK * KP;                 // [64][AP], then R
+    static constexpr int OUT = P + CHUNK * TAIL_AP;          // [64][8]
+    static constexpr int LAM = OUT + CHUNK * TAIL_COLS;      // [64][L], then the slab [KD][8][L]
+    static constexpr int X = 0, D = KD * TAIL_XP;            // slots and K X over the last chunk's k and T, which are done with by then
+    static_assert(KD * TAIL_XP + CHUNK * TAIL_XP <= V_, "slots must fit");
+    static_assert(CH % 4 == 0 && Q % 4 == 0 && LAM % 4 == 0, "16-byte rows");
+    __host__ __device__ static constexpr int floats(bool tail, int L) { return tail ? LAM + (CHUNK * L + 3) / 4 * 4 + KD * TAIL_COLS * L : B; }
+};
+
+__device__ __forceinline__ void tail_meet(int grp) { asm volatile("bar.sync %0, %1;\n" :: "r"(grp + 1), "n"(TAIL_GRP) : "memory"); }
+
+// In place: A (strictly lower triangular, fp32 [64][AP]) -> (I + A)^-1 diag(beta).  The 256 threads of a group.
+__device__ __forceinline__ void tail_inverse(float* A, const float* beta, int t, int grp) {
+    constexpr int AP = TAIL_AP;
+    if (t < CHUNK) {                                         // diagonal blocks by substitution, a thread to a column
+        const int m0 = t & ~15, cc = t & 15;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float s0 = i == cc ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+            for (int q = 0; q < (i + 3) / 4; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(A + (m0 + i) * AP + m0 + 4 * q);
+                const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (4 * q + u < i) { if (u & 1) s1 -= e[u] * x[4 * q + u]; else s0 -= e[u] * x[4 * q + u]; }
+            }
+            x[i] = s0 + s1;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) A[(m0 + i) * AP + m0 + cc] = x[i];
+    }
+    tail_meet(grp);
+    // X_ba = -X_bb (A_ba X_aa) for blocks of W = 16, then 32; the inner product waits in the mirror image above the diagonal.
+    // The sums run over whole rows: what they need not take in is zero.
+    auto corner = [&](auto width) {
+        constexpr int W = decltype(width)::value;
+        constexpr int per = W * W / 4, np = 32 / W;          // threads (4 columns each) and pairs
+        const bool on = t < per * np;
+        const int p = t / per, u = t - p * per, r = u / (W / 4), c = (u % (W / 4)) * 4;
+        const int a0 = 2 * W * p, b0 = a0 + W;
+        auto product = [&](const float* left, const float* right) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int k = 0; k < W; k += 4) {
+                const float4 f4 = *reinterpret_cast<const float4*>(left + k);
+                const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 v = *reinterpret_cast<const float4*>(right + (k + q) * AP);
+                    s.x = fmaf(f[q], v.x, s.x); s.y = fmaf(f[q], v.y, s.y); s.z = fmaf(f[q], v.z, s.z); s.w = fmaf(f[q], v.w, s.w);
+                }
+            }
+            return s;
+        };
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on) s = product(A + (b0 + r) * AP + a0, A + a0 * AP + a0 + c);
+        if (on) *reinterpret_cast<float4*>(A + (a0 + r) * AP + b0 + c) = s;
+        tail_meet(grp);
+        if (on) s = product(A + (b0 + r) * AP + b0, A + a0 * AP + b0 + c);
+        if (on) *reinterpret_cast<float4*>(A + (b0 + r) * AP + a0 + c) = make_float4(-s.x, -s.y, -s.z, -s.w);
+        tail_meet(grp);
+        if (on) *reinterpret_cast<float4*>(A + (a0 + r) * AP + b0 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        tail_meet(grp);
+    };
+    corner(std::integral_constant<int, 16>{});
+    corner(std::integral_constant<int, 32>{});
+    for (int i = t; i < CHUNK * 16; i += TAIL_GRP) {
+        float4* p = reinterpret_cast<float4*>(A + (i >> 4) * AP + 4 * (i & 15));
+        const float4 b = *reinterpret_cast<const float4*>(beta + 4 * (i & 15));
+        float4 v = *p;
+        v.x *= b.x; v.y *= b.y; v.z *= b.z; v.w *= b.w;
+        *p = v;
+    }
+    tail_meet(grp);
+}
+
+template <int KD, int VD>
+__global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, TailArgs ta) {
+    // In a prefill the kernels in front let this one in early: until it waits it reads the call's inputs alone.
+    if (!ta.early && chain_wait()) return;
+    using M = TailSmem<KD>;
+    constexpr int KP = M::KP, AP = TAIL_AP, XP = TAIL_XP;
+    extern __shared__ __align__(16) float sm[];
+    const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
+    const int tid = threadIdx.x, lane = tid & 31, grp = tid / TAIL_GRP, t = tid % TAIL_GRP;
+    const int v0 = blockIdx.z * TAIL_COLS;
+    int nch = ta.n0;
+    int64_t tok0 = (int64_t)seq * a.fixed_stride, tok_end = 0;
+    if (ta.n0 < 0) {
+        const SeqLoc sq = locate_seq(a, seq);
+        nch = sq.nch; tok0 = sq.tok0; tok_end = sq.tok_end;
+    }
+    const int lvl0 = nch > 0 ? ELL0 + __ffs(nch) - 1 : -1;   // the slot that takes in the last chunk's tokens
+    const bool room = nch == 0 || lvl0 < L;                  // the first cascade must not leave the last level
+    const bool tailed = ta.tail > 0 && room;
+    // tokens of the tail that are taken in: before token t > 0 levels 0..tz(t) move up one, which ends with the last level
+    const int done = tailed ? min(ta.tail, L < ELL0 ? 1 << (L - 1) : CHUNK) : 0;
+    const size_t bh = (size_t)seq * H + h;
+    float* st = ta.states + (bh * KD * VD + v0) * L;         // row k: VD * L floats further each
+    // the chunk a thread group works on: the last whole one, or the tail
+    float* ch = sm + (grp == 0 ? 0 : M::B);
+    float *sK = ch + M::K_, *sA = ch + M::A_, *sV = ch + M::V_;
+    double* sG = reinterpret_cast<double*>(ch + M::S_);
+    float *sEg = ch + M::S_ + 2 * CHUNK, *sEl = sEg + CHUNK, *sBeta = sEl + CHUNK;
+    float *sQ = sm + M::Q, *sP = sm + M::P, *sOut = sm + M::OUT, *sLam = sm + M::LAM, *slab = sLam + (CHUNK * L + 3) / 4 * 4;
+    float *sZ = sm + M::Z, *sSum = sm + M::SUM;
+
+    // chunk levels the tail continues from: slot (tid / 8) % 4 of a batch, column tid % 8, rows tid / 32 + 16 i
+    auto slot_level = [&](int s) {                           // level of slot s (bit order), or -1
+        uint32_t rem = (uint32_t)nch;
+        for (int i = 0; i < s; ++i) rem &= rem - 1;
+        return rem ? ELL0 + __ffs(rem) - 1 : -1;
+    };
+    const int xs = (tid >> 3) & 3, xv = tid & 7, xk = tid >> 5;
+    constexpr int XR = (KD + 15) / 16;
+    float xr[XR];
+    auto fetch_slots = [&](int s0) {
+        const int l = slot_level(s0 + xs);
+#pragma unroll
+        for (int i = 0; i < XR; ++i) {
+            const float* p = st + ((size_t)(xk + 16 * i) * VD + xv) * L;
+            xr[i] = 0.f;
+            if (l < 0) continue;
+            if (l != lvl0) xr[i] = __ldcg(p + l);
+            else for (int q = ELL0; q < l; ++q) xr[i] += __ldcg(p + q);
+        }
+    };
+    const bool mine = grp == 0 ? nch > 0 : tailed;
+    if (mine) {
+        const bool tail = grp == 1;
+        const int64_t t0 = tok0 + (int64_t)(tail ? nch : nch - 1) * CHUNK;
+        const int len = tail ? done : (ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - t0));
+        // rows as the kernel uses them, rows up to 64 null tokens: eight elements per thread and step, KD / 8 threads per row; every
+        // load is in flight before the first is used
+        constexpr int PPR = KD / 8, NIT = (CHUNK * PPR + TAIL_GRP - 1) / TAIL_GRP, NV = CHUNK * TAIL_COLS / TAIL_GRP, NL = 4;
+        const bool fast = a.qkv_dt != LAMPA_F32 && (((uintptr_t)a.k | (uintptr_t)a.q) & 15) == 0;
+        uint4 kw[NIT], qw[NIT];
+        uint32_t vv[NV], lv[NL];
+        if (fast) {
+#pragma unroll
+            for (int it = 0; it < NIT; ++it) {
+                const int p = t + it * TAIL_GRP, r = p / PPR;
+                const size_t at = ((size_t)(t0 + r) * H + h) * KD + (p % PPR) * 8;
+                kw[it] = load8_raw(a.k, at, r < len);
+                qw[it] = load8_raw(a.q, at, r < len && tail);
+            }
+        }
+        const uint32_t g0w = load_raw(a.g, (size_t)(t0 + 2 * t) * H + h, a.gb_dt, 2 * t < len);
+        const uint32_t g1w = load_raw(a.g, (size_t)(t0 + 2 * t + 1) * H + h, a.gb_dt, 2 * t + 1 < len);
+        const uint32_t btw = load_raw(a.beta, (size_t)(t0 + t) * H + h, a.gb_dt, t < len);
+#pragma unroll
+        for (int it = 0; it < NV; ++it) {
+            const int p = t + it * TAIL_GRP, r = p / TAIL_COLS;
+            vv[it] = load_raw(a.v, ((size_t)(t0 + r) * H + h) * VD + v0 + p % TAIL_COLS, a.qkv_dt, r < len);
+        }
+        const int nlam = tail ? len * L : 0;
+        auto lam_load = [&](int p) { return load_raw(a.lam, ((size_t)(t0 + p / L) * H + h) * L + p % L, a.lam_dt, p < nlam); };
+#pragma unroll
+        for (int it = 0; it < NL; ++it) lv[it] = lam_load(t + it * TAIL_GRP);
+        const float g0 = raw_float(g0w, a.gb_dt), g1 = raw_float(g1w, a.gb_dt), bt = raw_float(btw, a.gb_dt);
+        if (t < CHUNK) sBeta[t] = bt;
+#pragma unroll
+        for (int it = 0; it < NV; ++it) sV[t + it * TAIL_GRP] = raw_float(vv[it], a.qkv_dt);
+#pragma unroll
+        for (int it = 0; it < NIT; ++it) {
+            const int p = t + it * TAIL_GRP, r = p / PPR, c = (p % PPR) * 8;
+            if (p >= CHUNK * PPR) break;                     // whole warps
+            float x[8], y[8];
+            if (fast) {
+                raw_floats(kw[it], a.qkv_dt, x);
+                raw_floats(qw[it], a.qkv_dt, y);
+            } else {
+                const size_t at = ((size_t)(t0 + r) * H + h) * KD + c;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    x[e] = raw_float(load_raw(a.k, at + e, a.qkv_dt, r < len), a.qkv_dt);
+                    y[e] = raw_float(load_raw(a.q, at + e, a.qkv_dt, r < len && tail), a.qkv_dt);
+                }
+            }
+            float sk = 0.f, sq = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { sk += x[e] * x[e]; sq += y[e] * y[e]; }
+#pragma unroll
+            for (int o = 1; o < PPR; o <<= 1) {
+                sk += __shfl_xor_sync(0xffffffffu, sk, o);
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            }
+            if (a.use_l2norm) {
+                const float rk = rsqrtf(sk + 1e-6f), rq = rsqrtf(sq + 1e-6f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { x[e] = round_like(x[e] * rk, a.qkv_dt); y[e] *= rq; }
+            }
+            float4* d = reinterpret_cast<float4*>(sK + r * KP + c);
+            d[0] = make_float4(x[0], x[1], x[2], x[3]);
+            d[1] = make_float4(x[4], x[5], x[6], x[7]);
+            if (tail) {
+                d = reinterpret_cast<float4*>(sQ + r * KP + c);
+                d[0] = make_float4(y[0], y[1], y[2], y[3]);
+                d[1] = make_float4(y[4], y[5], y[6], y[7]);
+            }
+        }
+#pragma unroll
+        for (int it = 0; it < NL; ++it)
+            if (t + it * TAIL_GRP < nlam) sLam[t + it * TAIL_GRP] = raw_float(lv[it], a.lam_dt);
+        for (int p = t + NL * TAIL_GRP; p < nlam; p += TAIL_GRP) sLam[p] = raw_float(lam_load(p), a.lam_dt);      // more than 16 levels
+        if (t < 32) {
+            double cs = (double)g0 + (double)g1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u = __shfl_up_sync(0xffffffffu, cs, o);
+                if (lane >= o) cs += u;
+            }
+            const double last = __shfl_sync(0xffffffffu, cs, 31);
+            sG[2 * t] = cs - (double)g1; sG[2 * t + 1] = cs;
+            sEg[2 * t] = __expf((float)(cs - (double)g1)); sEg[2 * t + 1] = __expf((float)cs);
+            sEl[2 * t] = __expf((float)(last - (cs - (double)g1))); sEl[2 * t + 1] = __expf((float)(last - cs));
+        }
+        tail_meet(grp);
+        {   // A = tril(diag(beta) K K^T .* E, -1), P = tril(Q K^T .* E): rows ti + 16 x, columns tj + 16 y of the blocks y <= x
+            const int ti = t >> 4, tj = t & 15;
+            float kk[10], qk[10];
+#pragma unroll
+            for (int e = 0; e < 10; ++e) kk[e] = qk[e] = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < KD; c += 4) {
+                float4 ki[4], kj[4], qi[4];
+#pragma unroll
+                for (int x4 = 0; x4 < 4; ++x4) {
+                    ki[x4] = *reinterpret_cast<const float4*>(sK + (ti + 16 * x4) * KP + c);
+                    kj[x4] = *reinterpret_cast<const float4*>(sK + (tj + 16 * x4) * KP + c);
+                    if (tail) qi[x4] = *reinterpret_cast<const float4*>(sQ + (ti + 16 * x4) * KP + c);
+                }
+                int e = 0;
+#pragma unroll
+                for (int xi = 0; xi < 4; ++xi)
+#pragma unroll
+                    for (int yj = 0; yj <= xi; ++yj, ++e) {
+                        kk[e] = fmaf(ki[xi].w, kj[yj].w, fmaf(ki[xi].z, kj[yj].z, fmaf(ki[xi].y, kj[yj].y, fmaf(ki[xi].x, kj[yj].x, kk[e]))));
+                        if (tail) qk[e] = fmaf(qi[xi].w, kj[yj].w, fmaf(qi[xi].z, kj[yj].z, fmaf(qi[xi].y, kj[yj].y, fmaf(qi[xi].x, kj[yj].x, qk[e]))));
+                    }
+            }
+            int e = 0;
+#pragma unroll
+            for (int xi = 0; xi < 4; ++xi)
+#pragma unroll
+                for (int yj = 0; yj < 4; ++yj) {
+                    const int i = ti + 16 * xi, j = tj + 16 * yj;
+                    float av = 0.f, pv = 0.f;
+                    if (yj <= xi) {
+                        const float f = j <= i ? __expf((float)(sG[i] - sG[j])) : 0.f;
+                        if (j < i) av = sBeta[i] * kk[e] * f;
+                        pv = qk[e] * f;
+                        ++e;
+                    }
+                    sA[i * AP + j] = av;
+                    if (tail) sP[i * AP + j] = pv;
+                }
+        }
+        tail_meet(grp);
+        tail_inverse(sA, sBeta, t, grp);
+        if (!tail && tailed) {                               // all tokens of the last chunk as one state: they join a slot
+            {
+                const int i = t >> 2, jg = t & 3;            // row i, all columns, every fourth token
+                float u[TAIL_COLS];
+#pragma unroll
+                for (int v = 0; v < TAIL_COLS; ++v) u[v] = 0.f;
+#pragma unroll 4
+                for (int j = jg; j < CHUNK; j += 4) {        // T is zero above the diagonal
+                    const float f = sA[i * AP + j];
+                    const float4 p = *reinterpret_cast<const float4*>(sV + j * TAIL_COLS), q = *reinterpret_cast<const float4*>(sV + j * TAIL_COLS + 4);
+                    u[0] = fmaf(f, p.x, u[0]); u[1] = fmaf(f, p.y, u[1]); u[2] = fmaf(f, p.z, u[2]); u[3] = fmaf(f, p.w, u[3]);
+                    u[4] = fmaf(f, q.x, u[4]); u[5] = fmaf(f, q.y, u[5]); u[6] = fmaf(f, q.z, u[6]); u[7] = fmaf(f, q.w, u[7]);
+                }
+#pragma unroll
+                for (int v = 0; v < TAIL_COLS; ++v) {
+                    u[v] += __shfl_xor_sync(0xffffffffu, u[v], 1);
+                    u[v] += __shfl_xor_sync(0xffffffffu, u[v], 2);
+                }
+                const float el = sEl[i];
+                if (jg < 2) *reinterpret_cast<float4*>(sZ + i * XP + 4 * jg) = jg == 0 ? make_float4(el * u[0], el * u[1], el * u[2], el * u[3])
+                                                                                    : make_float4(el * u[4], el * u[5], el * u[6], el * u[7]);
+            }
+            tail_meet(grp);
+            for (int o = t; o < KD * 4; o += TAIL_GRP) {     // row k, two columns
+                const int k = o >> 2, v = (o & 3) * 2;
+                float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+                for (int i = 0; i < CHUNK; ++i) {
+                    const float f = sK[i * KP + k];
+                    const float2 z = *reinterpret_cast<const float2*>(sZ + i * XP + v);
+                    s0 = fmaf(f, z.x, s0); s1 = fmaf(f, z.y, s1);
+                }
+                *reinterpret_cast<float2*>(sSum + k * TAIL_COLS + v) = make_float2(s0, s1);
+            }
+        }
+    }
+    __syncthreads();
+    if (ta.early && !tailed) (void)chain_wait();             // the states are written from here on
+    // from here on everybody works on the tail's chunk, or on the last whole one when there is no tail
+    const float* cs = sm + (tailed ? M::B : 0);
+    const float *cK = cs + M::K_, *cT = cs + M::A_, *cV = cs + M::V_, *cEg = cs + M::S_ + 2 * CHUNK, *cEl = cEg + CHUNK;
+    const int r_all = tailed ? done : (nch > 0 ? CHUNK : 0);
+    const int row = tid >> 3, c8 = tid & 7;                  // row; four of 32 columns: state c8 / 2 of the batch, its half c8 % 2
+
+    // where a state element of the result goes: the slab, which leaves at the end, or (no tail) the state itself
+    auto put = [&](int k, int v, int l, float x) {
+        if (tailed) slab[(k * TAIL_COLS + v) * L + l] = x;
+        else st[((size_t)k * VD + v) * L + l] = x;
+    };
+    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z; thread = four rows k, four columns, every fourth token
+    auto kt_product = [&](const float* X, auto level_of) {
+        if (tid < KD * 8) {
+            const int ig = tid & 3, c = (tid >> 2) & 7, k0 = (tid >> 5) * 4;
+            float acc[4][4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) { acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f; }
+#pragma unroll 4
+            for (int i = ig; i < CHUNK; i += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(cK + i * KP + k0);
+                const float4 z4 = *reinterpret_cast<const float4*>(sZ + i * XP + 4 * c);
+                const float kx[4] = {k4.x, k4.y, k4.z, k4.w}, zx[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) acc[x][y] = fmaf(kx[x], zx[y], acc[x][y]);
+            }
+            float half[2][4], res[4];                        // summed over the four token groups, lane ig left with row ig
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const float give = ig & 2 ? acc[x][y] : acc[x + 2][y];
+                    half[x][y] = (ig & 2 ? acc[x + 2][y] : acc[x][y]) + __shfl_xor_sync(0xffffffffu, give, 2);
+                }
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const float give = ig & 1 ? half[0][y] : half[1][y];
+                res[y] = (ig & 1 ? half[1][y] : half[0][y]) + __shfl_xor_sync(0xffffffffu, give, 1);
+            }
+            const int l = level_of(c >> 1), k = k0 + ig;
+            if (l >= 0 && l < L) {
+                const float egl = cEg[CHUNK - 1];
+#pragma unroll
+                for (int y = 0; y < 4; ++y) put(k, 4 * (c & 1) + y, l, X ? egl * X[k * XP + 4 * c + y] - res[y] : res[y]);
+            }
+        }
+    };
+
+    if (tailed) {
+        for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
+        // R = P T: thread = (row, eight columns); both are lower triangular
+        float4 s[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll 2
+        for (int k = 8 * c8; k <= row; k += 4) {
+            const float4 p4 = *reinterpret_cast<const float4*>(sP + row * AP + k);
+            const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 v = *reinterpret_cast<const float4*>(cT + (k + u) * AP + 8 * c8 + 4 * q);
+                    s[q].x = fmaf(p[u], v.x, s[q].x); s[q].y = fmaf(p[u], v.y, s[q].y); s[q].z = fmaf(p[u], v.z, s[q].z); s[q].w = fmaf(p[u], v.w, s[q].w);
+                }
+        }
+        __syncthreads();
+        *reinterpret_cast<float4*>(sP + row * AP + 8 * c8) = s[0];
+        *reinterpret_cast<float4*>(sP + row * AP + 8 * c8 + 4) = s[1];
+        __syncthreads();
+        // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
+        // row i reads are the 2^(l-1) below the highest set bit they differ in
+        {
+            const int hf = (tid >> 2) & 1, jg = tid & 3;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < done) {
+                for (int l = 0; l < ELL0 && l < L; ++l) {
+                    if (l > 0 && !((row >> (l - 1)) & 1)) continue;
+                    const int j0 = l == 0 ? row : (row >> l) << l, j1 = l == 0 ? row + 1 : j0 + (1 << (l - 1));
+                    float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int j = j0 + jg; j < j1; j += 4) {
+                        const float f = sP[row * AP + j];
+                        const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * hf);
+                        u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
+                    }
+                    const float w = sLam[row * L + l];
+                    o.x = fmaf(w, u.x, o.x); o.y = fmaf(w, u.y, o.y); o.z = fmaf(w, u.z, o.z); o.w = fmaf(w, u.w, o.w);
+                }
+            }
+#pragma unroll
+            for (int d = 1; d < 4; d <<= 1) {
+                o.x += __shfl_xor_sync(0xffffffffu, o.x, d); o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
+                o.z += __shfl_xor_sync(0xffffffffu, o.z, d); o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
+            }
+            if (jg == 0) *reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * hf) = o;
+        }
+    }
+    // token levels that hold tokens, four at a time: bit l of `held`
+    const uint32_t held = r_all > 0 ? (uint32_t)(r_all - 1) << 1 | 1u : 0u;
+    auto nth = [](uint32_t m, int n) {                       // its n-th level, or -1
+        for (int i = 0; i < n; ++i) m &= m - 1;
+        return m ? __ffs(m) - 1 : -1;
+    };
+    if (!tailed)                                             // the slab is zero where no level is
+        for (int i = tid; i < KD * TAIL_COLS * 8; i += TAIL_THREADS) {
+            const int l = i & 7;
+            if (l < ELL0 && l < L && !((held >> l) & 1)) put(i >> 6, (i >> 3) & 7, l, 0.f);
+        }
+    for (int n0 = 0; n0 < __popc(held); n0 += TAIL_BATCH) {
+        const int l = nth(held, n0 + (c8 >> 1));
+        const int j0 = l < 0 ? 0 : l == 0 ? r_all - 1 : ((r_all - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? r_all : j0 + (1 << (l - 1));
+        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int je = min(j1, row + 1);
+#pragma unroll 4
+        for (int j = j0; j < je; ++j) {
+            const float f = cT[row * AP + j];
+            const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * (c8 & 1));
+            u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
+        }
+        const float el = cEl[row];
+        *reinterpret_cast<float4*>(sZ + row * XP + 4 * c8) = make_float4(el * u.x, el * u.y, el * u.z, el * u.w);
+        __syncthreads();
+        kt_product(nullptr, [&](int x) { return nth(held, n0 + x); });
+        __syncthreads();
+    }
+    if (ta.early && tailed) (void)chain_wait();              // the chunk levels are there
+    if (tailed) {
+        float *sX = sm + M::X, *sD = sm + M::D;
+        const int nslot = __popc((uint32_t)nch);
+        for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
+            fetch_slots(s0);
+#pragma unroll
+            for (int i = 0; i < XR; ++i)
+                sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs == 0 ? sSum[(xk + 16 * i) * TAIL_COLS + xv] : 0.f);
+            __syncthreads();
+            float4 d = make_float4(0.f, 0.f, 0.f, 0.f), y = d;
+#pragma unroll 2
+            for (int k = 0; k < KD; k += 4) {                // K X and Q X
+                const float4 k4 = *reinterpret_cast<const float4*>(cK + row * KP + k), q4 = *reinterpret_cast<const float4*>(sQ + row * KP + k);
+                const float kx[4] = {k4.x, k4.y, k4.z, k4.w}, qx[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float4 x = *reinterpret_cast<const float4*>(sX + (k + u) * XP + 4 * c8);
+                    d.x = fmaf(kx[u], x.x, d.x); d.y = fmaf(kx[u], x.y, d.y); d.z = fmaf(kx[u], x.z, d.z); d.w = fmaf(kx[u], x.w, d.w);
+                    y.x = fmaf(qx[u], x.x, y.x); y.y = fmaf(qx[u], x.y, y.y); y.z = fmaf(qx[u], x.z, y.z); y.w = fmaf(qx[u], x.w, y.w);
+                }
+            }
+            const float eg = cEg[row];
+            *reinterpret_cast<float4*>(sD + row * XP + 4 * c8) = make_float4(eg * d.x, eg * d.y, eg * d.z, eg * d.w);
+            y = make_float4(eg * y.x, eg * y.y, eg * y.z, eg * y.w);
+            __syncthreads();
+            float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int j = 0; j <= row; j += 4) {              // T and R times that; both rows are zero behind the diagonal
+                const float4 t4 = *reinterpret_cast<const float4*>(cT + row * AP + j), r4 = *reinterpret_cast<const float4*>(sP + row * AP + j);
+                const float tx[4] = {t4.x, t4.y, t4.z, t4.w}, rx[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float4 x = *reinterpret_cast<const float4*>(sD + (j + u) * XP + 4 * c8);
+                    z.x = fmaf(tx[u], x.x, z.x); z.y = fmaf(tx[u], x.y, z.y); z.z = fmaf(tx[u], x.z, z.z); z.w = fmaf(tx[u], x.w, z.w);
+                    y.x = fmaf(-rx[u], x.x, y.x); y.y = fmaf(-rx[u], x.y, y.y); y.z = fmaf(-rx[u], x.z, y.z); y.w = fmaf(-rx[u], x.w, y.w);
+                }
+            }
+            const float el = cEl[row];
+            *reinterpret_cast<float4*>(sZ + row * XP + 4 * c8) = make_float4(el * z.x, el * z.y, el * z.z, el * z.w);
+            const int l = slot_level(s0 + (c8 >> 1));
+            const float w = l >= 0 && row < done ? sLam[row * L + l] : 0.f;
+            y = make_float4(w * y.x, w * y.y, w * y.z, w * y.w);
+#pragma unroll
+            for (int o = 2; o < 8; o <<= 1) {                // over the slots of the batch
+                y.x += __shfl_xor_sync(0xffffffffu, y.x, o); y.y += __shfl_xor_sync(0xffffffffu, y.y, o);
+                y.z += __shfl_xor_sync(0xffffffffu, y.z, o); y.w += __shfl_xor_sync(0xffffffffu, y.w, o);
+            }
+            if (c8 < 2) {
+                float4* o = reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * c8);
+                *o = make_float4(o->x + y.x, o->y + y.y, o->z + y.z, o->w + y.w);
+            }
+            __syncthreads();
+            kt_product(sX, [&](int s) { return slot_level(s0 + s); });
+            __syncthreads();
+        }
+        const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
+        for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
+            store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, sOut[i], a.qkv_dt);
+        if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
+            fence_async_shared();
+            __syncthreads();
+            if (tid < KD) {
+                bulk_s2g(st + (size_t)tid * VD * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
+                bulk_commit();
+                bulk_wait_read();
+            }
+        } else {
+            __syncthreads();
+            for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) {
+                const int k = i / (TAIL_COLS * L);
+                st[(size_t)k * VD * L + (i - k * TAIL_COLS * L)] = slab[i];
+            }
+        }
+    }
+    if (ta.tail > 0 && done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
+    if (h == 0 && blockIdx.z == 0 && tid == 0 && (ta.n0 < 0 || !ta.one_count || seq == 0)) {
+        const int64_t n = (int64_t)nch * CHUNK + done;     // tokens held
+        int32_t* cn = ta.counts + (size_t)seq * L;
+        int64_t rem = n > 0 ? n - 1 : 0;
+        for (int l = L - 1; l >= 1; --l) {
+            const int64_t cap = l - 1 < 40 ? (int64_t)1 << (l - 1) : (int64_t)1 << 40;
+            const bool held = n > 0 && rem >= cap;
+            cn[l] = held ? (int32_t)cap : 0;
+            if (held) rem -= cap;
+        }
+        cn[0] = n > 0 ? 1 : 0;
+        if (seq == 0 && ta.arrivals) *ta.arrivals = 0;
+        if (rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
+    }
+}
+
+// -------------------------------------------------------------------------------------------------
+// The same token by token, for what the closed form is not faster at (launch_hgdn_tail).
+// Before token t > 0 of a chunk, levels 0..tz(t) collapse into level tz(t) + 1 (tz = trailing zeros); the live chunk levels sit
+// in HS register slots, in bit order.
 //
 // State columns are independent, so a half-warp owns one: lane kl has rows kl, kl + 16, ... of every
 // level in registers, a level's k^T S is K / 16 FMAs and four shuffles, and the levels of a token
@@ -60,7 +634,7 @@ __device__ __forceinline__ void load8_as_float(const void* p, size_t i, int dt, 
 // tokens, 47 us at 3001); with one CTA per (sequence, head) and a launch per tail token (61 us for the
 // token levels and 27 us per tail token) a 3001-token prompt spent 1.7 of its 1.9 ms on the device here.
 // -------------------------------------------------------------------------------------------------
-constexpr int TAIL_COLS = 8, TAIL_THREADS = 128;
+constexpr int STEPS_THREADS = 128;
 
 template <int N>
 __device__ __forceinline__ void half_warp_sum(float (&x)[N]) {
@@ -95,8 +669,8 @@ __device__ __forceinline__ void half_warp_sum_many(float (&x)[N], int lane) {
 }
 
 template <int KD, int VD, int HS>
-__global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, TailArgs ta) {
-    if (chain_wait()) return;
+__global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs a, TailArgs ta) {
+    if (!ta.early && chain_wait()) return;               // see above: only the inputs are read before the wait
     constexpr int KI = KD / 16;
     extern __shared__ __align__(16) float tail_smem[];
     float* sK = tail_smem;                       // [64][KD], normalised
@@ -117,21 +691,22 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         nch = sq.nch; tok0 = sq.tok0; tok_end = sq.tok_end;
     }
 
+    auto input = [](const void* p, size_t i, int dt) { return raw_float(load_raw(p, i, dt, true), dt); };
     // rows [t0, t0 + len) of the inputs as the kernel uses them; rows up to 64 become null tokens.  Eight elements per
     // thread and step, K / 8 threads per row, every load in flight before the first is used.
     auto stage = [&](int64_t t0, int len, bool tail) {
-        constexpr int PPR = KD / 8, NIT = CHUNK * PPR / TAIL_THREADS;
+        constexpr int PPR = KD / 8, NIT = CHUNK * PPR / STEPS_THREADS;
         float x[NIT][8], y[NIT][8];
 #pragma unroll
         for (int it = 0; it < NIT; ++it) {
-            const int p = tid + it * TAIL_THREADS, r = p / PPR, c = (p % PPR) * 8;
+            const int p = tid + it * STEPS_THREADS, r = p / PPR, c = (p % PPR) * 8;
             const size_t at = ((size_t)(t0 + r) * H + h) * KD + c;
-            load8_as_float(a.k, at, a.qkv_dt, r < len, x[it]);
-            load8_as_float(a.q, at, a.qkv_dt, r < len && tail, y[it]);
+            load8_float(a.k, at, a.qkv_dt, r < len, x[it]);
+            load8_float(a.q, at, a.qkv_dt, r < len && tail, y[it]);
         }
 #pragma unroll
         for (int it = 0; it < NIT; ++it) {
-            const int p = tid + it * TAIL_THREADS, r = p / PPR, c = (p % PPR) * 8;
+            const int p = tid + it * STEPS_THREADS, r = p / PPR, c = (p % PPR) * 8;
             float sk = 0.f, sq = 0.f;
 #pragma unroll
             for (int e = 0; e < 8; ++e) { sk += x[it][e] * x[it][e]; sq += y[it][e] * y[it][e]; }
@@ -155,20 +730,20 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             }
         }
 #pragma unroll
-        for (int i = tid; i < CHUNK * TAIL_COLS; i += TAIL_THREADS) {
+        for (int i = tid; i < CHUNK * TAIL_COLS; i += STEPS_THREADS) {
             const int r = i / TAIL_COLS, c = i - r * TAIL_COLS;
-            sV[i] = r < len ? load_as_float(a.v, ((size_t)(t0 + r) * H + h) * VD + v0 + c, a.qkv_dt) : 0.f;
+            sV[i] = r < len ? input(a.v, ((size_t)(t0 + r) * H + h) * VD + v0 + c, a.qkv_dt) : 0.f;
         }
         if (tid < CHUNK) {
-            sEg[tid] = tid < len ? __expf(load_as_float(a.g, (size_t)(t0 + tid) * H + h, a.gb_dt)) : 1.f;
-            sBeta[tid] = tid < len ? load_as_float(a.beta, (size_t)(t0 + tid) * H + h, a.gb_dt) : 0.f;
+            sEg[tid] = tid < len ? __expf(input(a.g, (size_t)(t0 + tid) * H + h, a.gb_dt)) : 1.f;
+            sBeta[tid] = tid < len ? input(a.beta, (size_t)(t0 + tid) * H + h, a.gb_dt) : 0.f;
         }
         if (tail) {                             // two threads per token, up to twenty levels each
             const int r = tid >> 1;
             if (r < len) {
                 float w[20];
 #pragma unroll
-                for (int i = 0; i < 20; ++i) w[i] = (tid & 1) + 2 * i < L ? load_as_float(a.lam, ((size_t)(t0 + r) * H + h) * L + (tid & 1) + 2 * i, a.lam_dt) : 0.f;
+                for (int i = 0; i < 20; ++i) w[i] = (tid & 1) + 2 * i < L ? input(a.lam, ((size_t)(t0 + r) * H + h) * L + (tid & 1) + 2 * i, a.lam_dt) : 0.f;
 #pragma unroll
                 for (int i = 0; i < 20; ++i)
                     if ((tid & 1) + 2 * i < L) sLam[r * L + (tid & 1) + 2 * i] = w[i];
@@ -193,7 +768,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 
     float* st = ta.states + ((((size_t)seq * H + h) * KD + kl) * VD + vv) * L;     // row kl; row kl + 16 i is i * row16 further
     const size_t row16 = (size_t)16 * VD * L;
-    // chunk levels the tail continues from, on their way while the last chunk is run
+    // chunk levels the tail continues from
     float X[HS][KI];
     int lvl[HS];
     {
@@ -205,16 +780,6 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         }
     }
     const bool room = nch == 0 || lvl[0] < L;    // the first cascade must not leave the last level
-#pragma unroll
-    for (int s = 0; s < HS; ++s)
-#pragma unroll
-        for (int i = 0; i < KI; ++i) X[s][i] = ta.tail > 0 && room && lvl[s] >= 0 && s > 0 ? st[i * row16 + lvl[s]] : 0.f;
-    if (ta.tail > 0 && room && nch > 0) {
-#pragma unroll
-        for (int i = 0; i < KI; ++i)
-            for (int l = ELL0; l < lvl[0]; ++l) X[0][i] += st[i * row16 + l];
-    }
-
     if (nch > 0) {
         const int64_t t0 = tok0 + (int64_t)(nch - 1) * CHUNK;
         stage(t0, ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - t0), false);
@@ -253,6 +818,17 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         advance(std::integral_constant<int, 1>{}, 62, 64);
 #pragma unroll
         for (int i = 0; i < KI; ++i) S[0][i] = sK[63 * KD + kl + 16 * i] * (sBeta[63] * sV[63 * TAIL_COLS + col]);
+    }
+
+    if (ta.early) (void)chain_wait();            // the chunk levels are there
+#pragma unroll
+    for (int s = 0; s < HS; ++s)
+#pragma unroll
+        for (int i = 0; i < KI; ++i) X[s][i] = ta.tail > 0 && room && lvl[s] >= 0 && s > 0 ? st[i * row16 + lvl[s]] : 0.f;
+    if (ta.tail > 0 && room && nch > 0) {
+#pragma unroll
+        for (int i = 0; i < KI; ++i)
+            for (int l = ELL0; l < lvl[0]; ++l) X[0][i] += st[i * row16 + l];
     }
 
     int done = 0;                                // tail tokens taken in
@@ -323,7 +899,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 done = t + 1;
             }
             __syncthreads();
-            for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS) {
+            for (int i = tid; i < done * TAIL_COLS; i += STEPS_THREADS) {
                 float out = 0.f;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) out += sOut[i * 17 + e];
@@ -386,21 +962,35 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     }
 }
 
+// The closed form takes 34 us whatever the tail (8 heads, K = V = 64; 14 us without one), a CTA to an SM; the steps 19 us and 0.4 us per
+// token behind the last chunk, any number of CTAs.  Both begin beside the output pass.  Whole calls of 2,944 tokens and a tail:
+// steps 63 us at 2, 77 at 22 tokens, closed form 86 - 87 from 32 to 62, without a tail 60 instead of 66; past one CTA to an SM
+// it would take a second round.
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
+    const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
+    ProfScope prof("hgdn_tail", st);
+    if ((ta.tail == 0 || ta.tail >= 48) && (int64_t)a.nseq * a.H * (VD / TAIL_COLS) <= sm_count()) {
+        using M = TailSmem<KD>;
+        const int smem = M::floats(ta.tail > 0, a.L) * 4;
+        constexpr int most = M::floats(true, 40) * 4;
+        static_assert(most <= 227 * 1024, "shared memory of an SM");
+        static std::atomic<uint64_t> ready;
+        if (!allow_smem(ready, hgdn_tail_kernel<KD, VD>, most)) return LAMPA_ERR_CUDA;
+        launch_chained(hgdn_tail_kernel<KD, VD>, grid, TAIL_THREADS, smem, st, a, ta);
+        return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
+    }
     const int slots = ta.tail > 0 ? __builtin_popcount((unsigned)ta.n0) : 0;
     const int staged = CHUNK * (2 * KD + TAIL_COLS + 2) + (ta.tail > 0 ? CHUNK * a.L + CHUNK * TAIL_COLS * 17 : 0);
     const int slab = ta.tail > 0 ? KD * TAIL_COLS * a.L : 0;
     const size_t smem = (size_t)(staged > slab ? staged : slab) * 4;
     constexpr int most = 82 * 1024;                          // 64 x 64 heads at 40 levels
     static std::atomic<uint64_t> ready[3];
-    if (!allow_smem(ready[0], hgdn_tail_kernel<KD, VD, 4>, most) || !allow_smem(ready[1], hgdn_tail_kernel<KD, VD, 8>, most) ||
-        !allow_smem(ready[2], hgdn_tail_kernel<KD, VD, 24>, most)) return LAMPA_ERR_CUDA;
-    const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
-    ProfScope prof("hgdn_tail", st);
-    if (slots <= 4) launch_chained(hgdn_tail_kernel<KD, VD, 4>, grid, TAIL_THREADS, smem, st, a, ta);
-    else if (slots <= 8) launch_chained(hgdn_tail_kernel<KD, VD, 8>, grid, TAIL_THREADS, smem, st, a, ta);
-    else launch_chained(hgdn_tail_kernel<KD, VD, 24>, grid, TAIL_THREADS, smem, st, a, ta);
+    if (!allow_smem(ready[0], hgdn_tail_steps_kernel<KD, VD, 4>, most) || !allow_smem(ready[1], hgdn_tail_steps_kernel<KD, VD, 8>, most) ||
+        !allow_smem(ready[2], hgdn_tail_steps_kernel<KD, VD, 24>, most)) return LAMPA_ERR_CUDA;
+    if (slots <= 4) launch_chained(hgdn_tail_steps_kernel<KD, VD, 4>, grid, STEPS_THREADS, smem, st, a, ta);
+    else if (slots <= 8) launch_chained(hgdn_tail_steps_kernel<KD, VD, 8>, grid, STEPS_THREADS, smem, st, a, ta);
+    else launch_chained(hgdn_tail_steps_kernel<KD, VD, 24>, grid, STEPS_THREADS, smem, st, a, ta);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 

@@ -1,0 +1,59 @@
+"""The end of a prompt (the last whole chunk's tokens and the T mod 64 behind it) is fp32 arithmetic up to the output's type:
+prompts short enough that no chunk level has gone through a bf16 record, against the token recurrence in float64."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+import lampa_b200
+
+pytestmark = pytest.mark.gpu
+
+
+def _fenwick64(q, k, v, g, b, lam):
+    T, K = k.shape
+    L = lam.shape[1]
+    S = torch.zeros(L, K, v.shape[1], dtype=torch.float64)
+    o = torch.zeros(T, v.shape[1], dtype=torch.float64)
+    for t in range(T):
+        if t:
+            tz = (t & -t).bit_length() - 1
+            S[tz + 1] += S[: tz + 1].sum(0)
+            S[: tz + 1] = 0
+        S = torch.exp(g[t]) * (S - b[t] * k[t][None, :, None] * (k[t] @ S)[:, None, :])
+        S[0] += b[t] * torch.outer(k[t], v[t])
+        o[t] = torch.einsum("l,k,lkv->v", lam[t], q[t], S)
+    return o, S.permute(1, 2, 0)
+
+
+# first and last token of a chunk, a chunk with nothing, one token and all but one behind it, fewer levels than a chunk has,
+# more levels than the loads of one pass take (16), decays that leave nothing of a chunk; fp16 rows; tails on either side of 48, from
+# where on they are taken in at once
+@pytest.mark.parametrize("K,V", [(64, 64), (32, 32), (16, 32)])
+@pytest.mark.parametrize("T,L,shift,dt", [(1, 1, -3.0, torch.bfloat16), (4, 3, -3.0, torch.bfloat16), (63, 7, -3.0, torch.float16),
+                                          (64, 9, -3.0, torch.bfloat16), (65, 9, 2.0, torch.bfloat16), (127, 8, -3.0, torch.bfloat16),
+                                          (100, 40, -5.0, torch.float16), (111, 9, -3.0, torch.bfloat16), (112, 17, -3.0, torch.bfloat16),
+                                          (121, 40, -5.0, torch.float16), (126, 17, 2.0, torch.bfloat16)])
+def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
+    B, H = 2, 3
+    gen = torch.Generator().manual_seed(T * 64 + K)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    q, k, v = F.normalize(rn(B, T, H, K), dim=-1).to(dt), F.normalize(rn(B, T, H, K), dim=-1).to(dt), rn(B, T, H, V).to(dt)
+    g, b, lam = -F.softplus(rn(B, T, H) + shift), torch.sigmoid(rn(B, T, H)), F.softplus(rn(B, T, H, L))
+    o, st = lampa_b200.chunk_h_gated_delta_rule(q.cuda(), k.cuda(), v.cuda(), g.cuda(), lam.cuda(), b.cuda(),
+                                                output_final_state=True, use_qk_l2norm_in_kernel=True)
+    lampa_b200.check_status(torch.device("cuda:0"))
+    kn = (k.float() * torch.rsqrt((k.float() ** 2).sum(-1, keepdim=True) + 1e-6)).to(dt)      # k is rounded, q is not
+    qn = q.double() * torch.rsqrt((q.double() ** 2).sum(-1, keepdim=True) + 1e-6)
+    n0 = T - T % 64
+    for i in range(B):
+        for h in range(H):
+            ro, rs = _fenwick64(*(x[i, :, h].double() for x in (qn, kn, v, g, b, lam)))
+            d = st.states[i, h].cpu().double() - rs
+            # a state is a sum over up to 128 tokens, each through a few dozen fp32 operations of relative error 2^-24; 1e-6 is 16 of them
+            assert d.norm() <= 1e-6 * rs.norm(), (float(d.norm()), float(rs.norm()))
+            if T > n0:
+                e = o[i, n0:, h].cpu().double() - ro[n0:]
+                eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11                          # rounding of the output, half an ulp
+                assert (e.abs() <= eps * ro[n0:].abs() + 2e-6 * ro[n0:].abs().max()).all()
+    want = [1 if T > 0 else 0] + [(1 << (l - 1)) if ((T - 1) >> (l - 1)) & 1 else 0 for l in range(1, L)]
+    assert st.counts.view(-1)[:L].tolist() == want
