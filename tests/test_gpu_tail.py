@@ -49,11 +49,14 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
         for h in range(H):
             ro, rs = _fenwick64(*(x[i, :, h].double() for x in (qn, kn, v, g, b, lam)))
             d = st.states[i, h].cpu().double() - rs
-            # a state is a sum over up to 128 tokens, each through a few dozen fp32 operations of relative error 2^-24; 1e-6 is 16 of them
-            assert d.norm() <= 1e-6 * rs.norm(), (float(d.norm()), float(rs.norm()))
+            # One decay factor is exp to two ulp, 2^-22.  At once (no tail, or one of 48 tokens and more) an element goes through one such
+            # factor and a few dozen roundings of 2^-24: four times 2^-22.  Token by token it goes through one factor per token, and
+            # their errors may all point the same way.
+            bound = 2.0 ** -22 * (4 if T == n0 or T - n0 >= 48 else max(4, T))
+            assert d.norm() <= bound * rs.norm(), (float(d.norm()), float(rs.norm()))
             if T > n0:
                 e = o[i, n0:, h].cpu().double() - ro[n0:]
                 eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11                          # rounding of the output, half an ulp
-                assert (e.abs() <= eps * ro[n0:].abs() + 2e-6 * ro[n0:].abs().max()).all()
+                assert (e.abs() <= eps * ro[n0:].abs() + 2 * bound * ro[n0:].abs().max()).all()
     want = [1 if T > 0 else 0] + [(1 << (l - 1)) if ((T - 1) >> (l - 1)) & 1 else 0 for l in range(1, L)]
     assert st.counts.view(-1)[:L].tolist() == want
