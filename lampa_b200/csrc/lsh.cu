@@ -70,14 +70,14 @@ lsh_hash_kernel(const float* __restrict__ x, int64_t row_stride, int64_t head_st
 }
 
 // -------------------------------------------------------------------------------------------------
-// Segmented stable LSD radix sort.  One thread-block cluster (up to 8 CTAs) per segment: each CTA
+// Segmented stable LSD radix sort.  One thread-block cluster (up to 16 CTAs) per segment: each CTA
 // owns a contiguous slice of the segment in its current order, digit histograms are exchanged
 // through distributed shared memory, and the passes are separated by the hardware cluster barrier
 // (no flag spinning anywhere).  The cluster size is the largest one for which the occupancy
 // calculator reports all clusters resident at once: a cluster lives inside one GPC, and a size that
 // merely divides the SM count left a third of the clusters waiting for a second wave (24 x 60 000
 // keys: 103 us against 57 us then; 45 us with the tile as large as the slice).  Keys are reduced to
-// (key - min) first, so only as many passes of up to 8 bits run as the key range needs: two for the
+// (key - min) first, so only as many passes of 8 or 9 bits run as the key range needs: two for the
 // ~15-bit bucket ids of an event.
 //
 // A CTA takes its slice in tiles of ITEMS * 1024 keys held in registers; a warp owns ITEMS * 32
@@ -89,7 +89,8 @@ lsh_hash_kernel(const float* __restrict__ x, int64_t row_stride, int64_t head_st
 // ranking), and the tile is grouped by digit in shared memory so that the writes are runs.
 // -------------------------------------------------------------------------------------------------
 constexpr int SORT_THREADS = 1024;
-constexpr int SORT_MAX_CL = 8;
+constexpr int SORT_MAX_CL = 16;          // beyond 8 the kernel opts in (non-portable cluster size)
+constexpr int SORT_DIGITS = 512;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int SORT_MAX_ITEMS = 12;
 
@@ -101,11 +102,12 @@ __device__ __forceinline__ uint32_t key_xform(const void* keys, int key_type, in
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// exclusive prefix over 256 values held by threads 0..255 (one each); wtot: 8 words of shared memory.  All threads call it.
-__device__ __forceinline__ uint32_t prefix256(uint32_t v, uint32_t* wtot, int tid) {
+// exclusive prefix over n values (a multiple of 32, at most 512) held by threads 0..n - 1; wtot: a word per warp of them in shared
+// memory.  All threads call it.
+__device__ __forceinline__ uint32_t prefix_digits(uint32_t v, uint32_t* wtot, int tid, int n) {
     const int lane = tid & 31, warp = tid >> 5;
     uint32_t incl = v;
-    if (tid < 256) {
+    if (tid < n) {
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -114,7 +116,7 @@ __device__ __forceinline__ uint32_t prefix256(uint32_t v, uint32_t* wtot, int ti
         if (lane == 31) wtot[warp] = incl;
     }
     __syncthreads();
-    if (tid < 256)
+    if (tid < n)
         for (int w = 0; w < warp; ++w) incl += wtot[w];
     return incl - v;
 }
@@ -146,9 +148,9 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
     const int64_t lo = min((int64_t)rank * per, n), hi = min(lo + per, n);
     const bool one_tile = hi - lo <= TILE;
 
-    __shared__ uint32_t hist[256], dbase[256], tstart[256], tile_tot[256];
-    __shared__ uint32_t wtot[8], red[2];
-    __shared__ __align__(16) uint16_t wcount[SORT_WARPS][256];
+    __shared__ uint32_t hist[SORT_DIGITS], dbase[SORT_DIGITS], tstart[SORT_DIGITS], tile_tot[SORT_DIGITS];
+    __shared__ uint32_t wtot[SORT_DIGITS / 32], red[2];
+    __shared__ __align__(16) uint16_t wcount[SORT_WARPS][SORT_DIGITS];
     extern __shared__ uint32_t sort_dyn[];         // [TILE] keys, [TILE] indices of the tile, grouped by digit
     uint32_t* skey = sort_dyn;
     uint32_t* sidx = sort_dyn + TILE;
@@ -208,8 +210,11 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
     }
     const uint32_t range = (n > 0 && gmx >= gmn) ? (gmx - gmn) : 0u;
     const int bits = range ? (32 - __clz(range)) : 0;
-    const int npass = (bits + 7) / 8;
-    const int width = npass ? (bits + npass - 1) / npass : 0;        // digits of equal width: fewer ballots than 8 + the rest
+    // Digits of up to eight bits, or of nine where that saves a pass (24 segments of 60,000 keys of 26 bits: 68.6 us with four
+    // passes of seven bits, 57.6 with three of nine); of equal width.
+    const int npass = (bits + 8) / 9 < (bits + 7) / 8 ? (bits + 8) / 9 : (bits + 7) / 8;
+    const int width = npass ? (bits + npass - 1) / npass : 0;
+    const int ndig = max(32, 1 << width);
 
     if (npass == 0) {
         for (int64_t i = lo + tid; i < hi; i += SORT_THREADS) perm[s0 + i] = INIT ? (int64_t)starting(i) : i;
@@ -227,7 +232,7 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
 
         // digit counters of a tile: rank of every key within its warp and digit, then the exclusive prefix over the warps
         auto rank_tile = [&](int64_t t0) {
-            for (int z = tid; z < SORT_WARPS * 256 / 8; z += SORT_THREADS) reinterpret_cast<uint4*>(&wcount[0][0])[z] = make_uint4(0u, 0u, 0u, 0u);
+            for (int z = lane * 8; z < ndig; z += 256) *reinterpret_cast<uint4*>(&wcount[warp][z]) = make_uint4(0u, 0u, 0u, 0u);      // the warp's own row
             __syncthreads();
 #pragma unroll
             for (int it = 0; it < ITEMS; ++it) {
@@ -241,6 +246,10 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                     const uint32_t bal = __ballot_sync(0xffffffffu, one);
                     m &= one ? bal : ~bal;
                 }
+                if (width > 8) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, d & 256u);
+                    m &= (d & 256u) ? bal : ~bal;
+                }
                 const uint32_t basecnt = valid ? wcount[warp][d] : 0u;
                 const uint32_t r = basecnt + __popc(m & ((1u << lane) - 1u));
                 if (it & 1) rnk[it >> 1] |= r << 16; else rnk[it >> 1] = r;
@@ -249,7 +258,7 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                 __syncwarp();
             }
             __syncthreads();
-            if (tid < 256) {
+            if (tid < ndig) {
                 uint32_t run = 0;
 #pragma unroll 8
                 for (int w = 0; w < SORT_WARPS; ++w) {
@@ -270,9 +279,9 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
                 load_tile(lo, p, ksrc, isrc, gmn);
             }
             rank_tile(lo);
-            if (tid < 256) hist[tid] = tile_tot[tid];
+            if (tid < ndig) hist[tid] = tile_tot[tid];
         } else {
-            if (tid < 256) hist[tid] = 0;
+            if (tid < ndig) hist[tid] = 0;
             __syncthreads();
             for (int64_t t0 = lo; t0 < hi; t0 += TILE) {
                 load_tile(t0, p, ksrc, isrc, gmn);
@@ -286,14 +295,14 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
 
         // (b) where each digit of this slice starts in the segment
         uint32_t tot = 0, before = 0;
-        if (tid < 256)
+        if (tid < ndig)
             for (int r = 0; r < ncl; ++r) {
                 const uint32_t hv = cluster.map_shared_rank(hist, r)[tid];
                 tot += hv;
                 if (r < rank) before += hv;
             }
-        const uint32_t ex = prefix256(tot, wtot, tid);
-        if (tid < 256) dbase[tid] = ex + before;
+        const uint32_t ex = prefix_digits(tot, wtot, tid, ndig);
+        if (tid < ndig) dbase[tid] = ex + before;
         __syncthreads();
 
         // (c) stable scatter, tile by tile in slice order
@@ -305,10 +314,10 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
             if (!one_tile) {
                 load_tile(t0, p, ksrc, isrc, gmn);
                 rank_tile(t0);
-                outside = __syncthreads_or(tid < 256 && (int64_t)dbase[tid] + tile_tot[tid] > n);
+                outside = __syncthreads_or(tid < ndig && (int64_t)dbase[tid] + tile_tot[tid] > n);
             }
-            const uint32_t ts = prefix256(tid < 256 ? tile_tot[tid] : 0u, wtot, tid);
-            if (tid < 256) tstart[tid] = ts;
+            const uint32_t ts = prefix_digits(tid < ndig ? tile_tot[tid] : 0u, wtot, tid, ndig);
+            if (tid < ndig) tstart[tid] = ts;
             __syncthreads();
             // group the tile by digit in shared memory, so that the global writes below are runs of
             // consecutive addresses (a direct scatter costs one 32-byte sector per key)
@@ -339,7 +348,7 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
             }
             if (t0 + TILE < hi) {
                 __syncthreads();
-                if (tid < 256) dbase[tid] += tile_tot[tid];
+                if (tid < ndig) dbase[tid] += tile_tot[tid];
                 __syncthreads();
             }
         }
@@ -348,12 +357,13 @@ segsort_kernel(const void* __restrict__ keys, int key_type, int64_t n_total,
     if (npass == 0) cluster.sync();       // no CTA leaves while a peer may still read its shared memory
 }
 
-// Upper bound of the cluster size for nseg segments: SMs / segments, at most 8 (the launcher lowers it until all fit).
-static int sort_cluster_size(int nseg) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int cl = sms / (nseg > 0 ? nseg : 1);
-    if (cl > SORT_MAX_CL) cl = SORT_MAX_CL;
+// Upper bound of the cluster size: SMs / segments (the launcher lowers it until all fit), at most 8, or 16 where eight slices would
+// be longer than 4096 keys.  2 x 60,000 keys: 50 us in slices of 7,500 and 37 in slices of 3,750; 4 x 20,000 28.5 and 30, 3 x 9,001
+// 14.5 and 16.9, since a cluster barrier of sixteen costs more than half a short slice.
+static int sort_cluster_size(int nseg, int64_t avg_keys) {
+    int cl = sm_count() / (nseg > 0 ? nseg : 1);
+    const int most = avg_keys > 8 * 4096 ? SORT_MAX_CL : 8;
+    if (cl > most) cl = most;
     if (cl < 1) cl = 1;
     return cl;
 }
@@ -391,7 +401,7 @@ static int launch_segsort(const void* keys, int key_type, int64_t n_total, const
     // clusters of 6 only if every GPC has 18 usable SMs): ask the occupancy calculator.
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    int cl = sort_cluster_size(nseg), which = 0;
+    int cl = sort_cluster_size(nseg, n_total / (nseg > 0 ? nseg : 1)), which = 0;
     for (;; --cl) {
         // tile: the slice of an equal split, or twice the average slice when the segments are ragged (larger slices
         // take several tiles), at most 12 keys per thread (96 KB)
@@ -400,6 +410,7 @@ static int launch_segsort(const void* keys, int key_type, int64_t n_total, const
         which = 0;
         while (which < 4 && (int64_t)item_counts[which] * SORT_THREADS < want) ++which;
         if (!allow_smem(ready[init != nullptr][which], kernels[which], 2 * item_counts[which] * SORT_THREADS * 4)) return LAMPA_ERR_CUDA;
+        if (cl > 8 && cudaFuncSetAttribute(kernels[which], cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return LAMPA_ERR_CUDA;
         cfg.gridDim = dim3((unsigned)nseg * cl, 1, 1);
         cfg.blockDim = dim3(SORT_THREADS, 1, 1);
         cfg.dynamicSmemBytes = (size_t)2 * item_counts[which] * SORT_THREADS * 4;
