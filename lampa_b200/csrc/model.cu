@@ -229,6 +229,9 @@ struct ProjArgs {
     int32_t* status; int budget;
 };
 
+// PARTS > 1: the blocks of a tile shared out over CTAs of their own, for batches whose tiles leave SMs idle: a tile is then one or two
+// blocks long instead of five (9,001 rows, 81 tiles: 24 -> 19 us).
+template <int PARTS>
 __global__ void __launch_bounds__(PJ_THREADS, 2)
 model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                      const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg,
@@ -249,7 +252,10 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
     unsigned char* sST = smem + PJ_ST;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t ntiles = (a.n + PJ_OUT - 1) / PJ_OUT;
-    const int mine = blockIdx.x < ntiles ? (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+    const int cta = blockIdx.x / PARTS, ctas = gridDim.x / PARTS, piece = blockIdx.x % PARTS;
+    constexpr int PER = (PJ_BLOCKS + PARTS - 1) / PARTS;            // blocks of a part; the last one has the rest
+    const int m0 = PARTS == 1 ? 0 : piece * PER, m1 = PARTS == 1 ? PJ_BLOCKS : min(m0 + PER, PJ_BLOCKS), nb = m1 - m0;
+    const int mine = cta < ntiles ? (int)((ntiles - cta + ctas - 1) / ctas) : 0;
 
     if (tid == 0) {
         for (int s = 0; s < MNST; ++s) mbar_init(full + s, 1);
@@ -271,12 +277,12 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
 
     if (warp == MWARPS) {
         if (lane == 0) {
-            const int npieces = mine * PJ_BLOCKS * 2;
+            const int npieces = mine * nb * 2;
             int loaded = 0, landed = 0;
             auto load = [&](int p) {                             // piece p: block (p / 2) % 5, half p & 1 of its 128 inputs
                 uint64_t* b = full + p % MNST;
                 unsigned char* dst = sW + (size_t)(p % MNST) * MST;
-                const int blk = (p >> 1) % PJ_BLOCKS, x = (p & 1) * 64;
+                const int blk = m0 + (p >> 1) % nb, x = (p & 1) * 64;
                 if (blk < 4) {
                     mbar_expect_tx(b, MST);
                     tma_load_2d(dst, blk == 0 ? &mq : blk == 1 ? &mk : blk == 2 ? &mv : &mg, x, 0, b);
@@ -291,8 +297,8 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             for (int p = 0; p < MNST && p < npieces; ++p) load(p);
             for (int t = 0; t < mine && !dead; ++t) {
                 mbar_wait(bready, (uint32_t)(t & 1), dead, a.status, 600, a.budget);
-                for (int m = 0; m < PJ_BLOCKS && !dead; ++m) {
-                    const int q = t * PJ_BLOCKS + m, buf = q & 1;
+                for (int m = m0; m < m1 && !dead; ++m) {
+                    const int q = t * nb + m - m0, buf = q & 1;
                     if (q >= 2) mbar_wait(dfree + buf, (uint32_t)(((q >> 1) - 1) & 1), dead, a.status, 601, a.budget);
                     for (int h = 0; h < 2 && !dead; ++h) {
                         const int p = 2 * q + h;
@@ -329,7 +335,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
         // the rows of hs that tile t takes, in LSH order: found under the gate block of the tile before, fetched under its
         // last epilogue (both are chains of dependent loads); 2.05 M rows: 1,667 -> 1,629 us
         auto find_rows = [&](int t) {                            // warps 0..3
-            const int64_t j = (blockIdx.x + (int64_t)t * gridDim.x) * PJ_OUT - PJ_HALO + tid;            // operand row tid
+            const int64_t j = (cta + (int64_t)t * ctas) * PJ_OUT - PJ_HALO + tid;            // operand row tid
             bool first = false;
             int64_t r = -1;
             if (tid >= 8 && j >= 0 && j < a.n) r = ordered_row(a.cu, a.nseq, a.perm, j, a.n, a.status, &first);
@@ -353,7 +359,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             fetch_rows();
         }
         for (int t = 0; t < mine; ++t) {
-            const int64_t tile = blockIdx.x + (int64_t)t * gridDim.x, j0 = tile * PJ_OUT;
+            const int64_t tile = cta + (int64_t)t * ctas, j0 = tile * PJ_OUT;
             const int nv = (int)min((int64_t)PJ_OUT, a.n - j0);
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             fence_async_smem();
@@ -362,13 +368,13 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
             // event starts of this thread's 28 positions and the 4 before: bit i = operand row p0 + i
             const int p0 = PJ_HALO - 4 + PJ_PART * part;
             const uint32_t starts = __funnelshift_r(sstart[p0 >> 5], (p0 >> 5) < 3 ? sstart[(p0 >> 5) + 1] : 0u, p0 & 31);
-            for (int m = 0; m < PJ_BLOCKS; ++m) {
-                const int q = t * PJ_BLOCKS + m, buf = q & 1;
+            for (int m = m0; m < m1; ++m) {
+                const int q = t * nb + m - m0, buf = q & 1;
                 uint2 taps = make_uint2(0u, 0u);                 // this channel's four taps
                 if (m < 3) taps = __ldg(reinterpret_cast<const uint2*>(m == 0 ? a.conv[0] : m == 1 ? a.conv[1] : a.conv[2]) + ch);
                 epi_wait(mdone + buf, (uint32_t)((q >> 1) & 1), dead, a.status, 610, a.budget, [] {});      // products complete
                 tc_fence_after();
-                if (m == PJ_BLOCKS - 1 && t + 1 < mine) fetch_rows();        // the tile's last products: its operand is free
+                if (PARTS == 1 && m == PJ_BLOCKS - 1 && t + 1 < mine) fetch_rows();        // the tile's last products: its operand is free
                 float x[32];                                     // X(i) = position i - 4
                 tmem_ld32(x, tl + 128 * buf);
                 tc_fence_before();
@@ -410,7 +416,7 @@ model_project_kernel(ProjArgs a, const __grid_constant__ CUtensorMap mq, const _
                     for (int i = 0; i < PJ_PART; ++i)
                         if (PJ_PART * part + i < nv) gp[i * a.H] = is_a ? sp_scale * softplusf_(x[4 + i] + sp_add) : sigmoid_fast(x[4 + i]);
                 }
-                if (m == 3 && t + 1 < mine && warp < 4) find_rows(t + 1);
+                if (PARTS == 1 && m == 3 && t + 1 < mine && warp < 4) find_rows(t + 1);      // (shared-out tiles: one to a CTA)
                 if (tid == 0) bulk_wait_read();                  // the previous results have left the staging tile
                 epi_sync();
                 uint16_t* st = reinterpret_cast<uint16_t*>(sST) + ch;
@@ -818,11 +824,15 @@ extern "C" int lampa_model_project(const lampa_model_mixer* w, const void* hs, c
     CUtensorMap m[7];
     for (int i = 0; i < 7; ++i)
         if (!make_map(&m[i], mats[i], LAMPA_BF16, rows[i], MD, 64, rows[i], true)) return LAMPA_ERR_UNSUPPORTED;
-    static std::atomic<uint64_t> ready{0};
-    if (!allow_smem(ready, model_project_kernel, PJ_SMEM)) return LAMPA_ERR_CUDA;
+    static std::atomic<uint64_t> ready[3];
+    if (!allow_smem(ready[0], model_project_kernel<1>, PJ_SMEM) || !allow_smem(ready[1], model_project_kernel<2>, PJ_SMEM) ||
+        !allow_smem(ready[2], model_project_kernel<3>, PJ_SMEM)) return LAMPA_ERR_CUDA;
     ProfScope prof("model_project", (cudaStream_t)stream);
     const int64_t want = (n + PJ_OUT - 1) / PJ_OUT, most = (int64_t)sm_count() * 2;
-    launch_chained(model_project_kernel, (unsigned)(want < most ? want : most), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream, a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
+    // as many parts as all run at once, two CTAs to an SM
+    if (3 * want <= most) launch_chained(model_project_kernel<3>, (unsigned)(3 * want), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream, a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
+    else if (2 * want <= most) launch_chained(model_project_kernel<2>, (unsigned)(2 * want), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream, a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
+    else launch_chained(model_project_kernel<1>, (unsigned)(want < most ? want : most), PJ_THREADS, PJ_SMEM, (cudaStream_t)stream, a, m[0], m[1], m[2], m[3], m[4], m[5], m[6]);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
 }
 
