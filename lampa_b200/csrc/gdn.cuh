@@ -86,6 +86,7 @@ struct GdnArgs {
     int fixed_stride;   // tokens from one sequence to the next in that case (fixed_T, or more when a prompt's tail is left to hgdn_tail)
     int fixed_cps;      // chunks per sequence in that case: positions follow by arithmetic, no plan loads
     int nc_max, nb_max, nhigh_max;
+    int nlev_max;       // chunk levels of the longest sequence there can be
     long long total_tokens;  // B * T of the call (rows of the token-major inputs)
     const int64_t* tok_off; const int32_t* chunk_off; const int32_t* block_off;   // offset tables of a packed call (plan_kernel)
     char* rec; size_t rec_bytes;          // per (chunk, head) records

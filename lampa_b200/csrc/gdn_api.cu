@@ -19,7 +19,7 @@ long long* g_ticks = nullptr;     // see lampa_debug_set_tick_buffer
 int g_ticks_ctas = 0;
 
 struct Layout {
-    int nseq, nc_max, nb_max, nhigh_max, LC;
+    int nseq, nc_max, nb_max, nhigh_max, nlev_max, LC;
     size_t rec_bytes, blk_bytes, state_bytes;
     size_t off_tok, off_chunk, off_block, off_rec, off_blk, off_entry, total;
 };
@@ -64,6 +64,7 @@ int make_layout(const lampa_gdn_desc* d, bool hier, Layout& l) {
     // cross-block levels of any sequence up to that length: nlev - 3 up to 256 chunks, 5 up to 1024, then nlev - 5
     const int nhigh = nlev <= MIN_BLOCK_LOG ? 0 : (nlev <= 8 ? nlev - MIN_BLOCK_LOG : (nlev <= 10 ? 5 : nlev - BLOCK_LOG));
     l.nhigh_max = hier ? nhigh : 0;
+    l.nlev_max = nlev;
     if (hier && 1 + (l.nhigh_max + NLW - 1) / NLW > MAX_GROUPS) return LAMPA_ERR_UNSUPPORTED;
     l.LC = hier ? (d->L > ELL0 ? d->L - ELL0 : 1) : 0;
     if (d->K == 64) fill_sizes<64, 64>(l);
@@ -93,7 +94,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     a.fixed_stride = a.fixed_T;
     a.fixed_cps = cu ? 0 : (d->T + CHUNK - 1) / CHUNK;
     a.total_tokens = (long long)d->B * d->T;
-    a.nseq = l.nseq; a.nc_max = l.nc_max; a.nb_max = l.nb_max; a.nhigh_max = l.nhigh_max;
+    a.nseq = l.nseq; a.nc_max = l.nc_max; a.nb_max = l.nb_max; a.nhigh_max = l.nhigh_max; a.nlev_max = l.nlev_max;
     a.tok_off = (int64_t*)(base + l.off_tok);
     a.chunk_off = (int32_t*)(base + l.off_chunk);
     a.block_off = (int32_t*)(base + l.off_block);

@@ -200,7 +200,9 @@ struct Pipe {
 // everybody is done with the group before, whose stage is refilled then.  (A poll and a copy cost the warp 170 and 150 - 350
 // cycles: with one record to a group that is as long as a short step.)  A wait that runs out is recorded and everybody walks
 // on to the end.
-template <int NST, int NT, int GRP>
+// LAG: groups that a stage stays untouched behind its own (1: until everybody has moved on; 2: one group more, for warps that
+// follow a step behind).  NT = 0: every thread of the CTA.
+template <int NST, int NT, int GRP, int LAG = 1>
 struct Feed {
     uint64_t* bar;
     unsigned char* stage;
@@ -214,7 +216,10 @@ struct Feed {
     size_t src2;         // a second piece of every record: where it begins in the record, and its bytes (0: none).  It lands
     uint32_t copy2;      // behind the first one in the stage
 
-    static __device__ __forceinline__ void meet() { asm volatile("bar.sync 1, %0;\n" :: "n"(NT) : "memory"); }
+    static __device__ __forceinline__ void meet() {
+        if (NT == 0) asm volatile("bar.sync 1;\n" ::: "memory");
+        else asm volatile("bar.sync 1, %0;\n" :: "n"(NT == 0 ? 32 : NT) : "memory");
+    }
     __device__ __forceinline__ int groups() const { return (nsteps + GRP - 1) / GRP; }
     __device__ __forceinline__ void issue(int grp) const {                       // the whole warp, a lane to a step
         const int lane = threadIdx.x & 31, step = grp * GRP + lane;
@@ -247,7 +252,7 @@ struct Feed {
             if (mbar_wait(bar + (i % NST), (uint32_t)((i / NST) & 1), dead, status, 100 + (i & 0xffff), budget)) landed = i + 1;
             dead = __any_sync(0xffffffffu, dead);
             meet();
-            if (!dead && i > 0 && i - 1 + NST < ng) { issue(i - 1 + NST); issued = i + NST; }
+            if (!dead && i >= LAG && i - LAG + NST < ng) { issue(i - LAG + NST); issued = i - LAG + NST + 1; }
         }
         for (int i = 0; i < extra; ++i) meet();
         // copies that were started but never seen complete (only after a wait gave up) land before the CTA's memory is given back
@@ -875,6 +880,202 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
     pipe.finish();
 }
 
+// -------------------------------------------------------------------------------------------------
+// The same for head dims up to 32 with the levels spread over warps: a warp carries two levels of a 16-column slab (level
+// slots p and p + pairs of those the block has: its own first, then the cross-block ones it reads), leaves their sum in shared
+// memory in its own register order, and four warps a chunk behind add the partial sums and O_local and store.
+// A block's chunk is then two levels deep instead of five, with no barrier but the one at its top.  15 warps and 150 KB, a CTA to an
+// SM: taken while the blocks of all heads are at most one to an SM (one event of 9,001 points, 72 CTAs: 25 -> 19 us, two events
+// 509 -> 480 us for the whole model; three events, two rounds: 620 against 622; 64 events: 960 against 1270 us a pass).
+// -------------------------------------------------------------------------------------------------
+constexpr int LV_SUM = 4, LV_MAX_PAIRS = 5, LV_MAX_THREADS = (2 * LV_MAX_PAIRS + 1 + LV_SUM) * 32;
+
+template <int KD, int VD>
+struct LevelsSmem {
+    static constexpr int NST = 4;
+    static constexpr int PART = 1024;                        // partial sums [2][pairs][slabs][8][32 lanes][4], behind the barriers
+    static int stage(int LC) { return (Rec<KD, VD>::bytes(LC) + 127) / 128 * 128; }
+    static int bytes(int LC, int pairs) { return PART + 2 * pairs * 2 * 4096 + NST * stage(LC); }
+};
+
+template <int KD, int VD>
+__global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs a, int pairs) {
+    if (chain_wait()) return;
+    if (a.signal) chain_signal();
+    using R = Rec<KD, VD>;
+    using S = LevelsSmem<KD, VD>;
+    constexpr int NS = VD / 16;
+    static_assert(NS == 2, "two slabs");
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int gb = blockIdx.x, h = blockIdx.y, H = a.H;
+    SeqLoc sq;
+    int b;
+    if (!locate_block(a, gb, sq, b)) return;
+    const int nch = sq.nch;
+    const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
+    const int bl = block_log(nch), bc = 1 << bl;
+    const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
+    const int c0 = sq.c0 + b * bc;
+    const int nsteps = min(bc, nch - b * bc);
+    const int64_t tok0 = sq.tok0 + (int64_t)b * bc * CHUNK, tok_end = sq.tok_end;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    float4* part = reinterpret_cast<float4*>(smem + S::PART);
+    const int buf_stride = pairs * NS * 256;                    // float4 of one chunk's partial sums
+
+    Feed<S::NST, 0, 1, 2> feed;
+    feed.bar = reinterpret_cast<uint64_t*>(smem);
+    feed.stage = smem + S::PART + 2 * pairs * NS * 4096;
+    feed.step_bytes = (R::bytes(a.LC) + 127) / 128 * 128;
+    feed.src = a.rec + ((size_t)c0 * H + h) * a.rec_bytes;
+    feed.src_stride = (size_t)H * a.rec_bytes;
+    feed.copy_bytes = R::bytes(a.LC);
+    feed.nsteps = nsteps;
+    feed.status = a.status;
+    feed.budget = a.poll_budget;
+    feed.copy2 = 0;
+    const int producer = pairs * NS;
+    feed.start(warp == producer);
+    if (warp == producer) {
+        feed.produce(1);
+        return;
+    }
+    // the block's level slots: its own levels, then the cross-block levels it reads
+    const uint32_t cross = (uint32_t)b & ((1u << min(nhigh, 30)) - 1u);
+    const int nslots = bl + __popc(cross);
+    auto nth_cross = [&](int k) {
+        uint32_t m = cross;
+        for (int i = 0; i < k; ++i) m &= m - 1;
+        return __ffs(m) - 1;
+    };
+    // slots read in chunk n, as a mask of pairs that leave a partial sum
+    auto read_slot = [&](int s, int n) { return s < nslots && (s >= bl || ((n >> s) & 1)); };
+    if (warp > producer) {
+        // ---- sums: warp = (slab, two of the four row tiles), a chunk behind ----
+        const int w = warp - producer - 1, slab = w & 1, mt0 = (w >> 1) * 2, row0 = 16 * slab;
+        const unsigned char* st = nullptr;
+        for (int i = 0; i <= nsteps; ++i) {
+            const unsigned char* now = feed.step(i);          // chunk i - 1 is in its partial sums
+            if (i > 0) {
+                const int n = b * bc + i - 1;
+                float o[2][2][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) { o[x][nt][0] = o[x][nt][1] = o[x][nt][2] = o[x][nt][3] = 0.f; }
+                const float4* p0 = part + ((i - 1) & 1) * buf_stride + slab * 256 + lane;
+                for (int p = 0; p < pairs; ++p) {
+                    if (!read_slot(p, n) && !read_slot(p + pairs, n)) continue;
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int nt = 0; nt < 2; ++nt) {
+                            const float4 f = p0[p * NS * 256 + ((mt0 + x) * 2 + nt) * 32];
+                            o[x][nt][0] += f.x; o[x][nt][1] += f.y; o[x][nt][2] += f.z; o[x][nt][3] += f.w;
+                        }
+                }
+                const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + R::OL_OFF);
+                const int64_t t0 = tok0 + (int64_t)(i - 1) * CHUNK;
+                auto emit = [&](auto scat) {
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int hh = 0; hh < 2; ++hh) {
+                            const int r = (mt0 + x) * 16 + g + hh * 8;
+                            const int64_t orow = t0 + r < tok_end ? out_row<decltype(scat)::value>(a, t0 + r) : -1;
+                            if (orow >= 0) {
+#pragma unroll
+                                for (int nt = 0; nt < 2; ++nt) {
+                                    const int col = row0 + nt * 8 + 2 * t;
+                                    const float2 ol = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sOl + R::TV::off(r, col)));
+                                    store_out2(a.o, a.qkv_dt, ((size_t)orow * H + h) * VD + col, ol.x + o[x][nt][2 * hh], ol.y + o[x][nt][2 * hh + 1]);
+                                }
+                            }
+                        }
+                };
+                if (a.out_perm_rows > 0) emit(ScatterOn{}); else emit(ScatterOff{});
+            }
+            st = now;
+        }
+        return;
+    }
+    // ---- levels: warp = (pair, slab) ----
+    const int pair = warp / NS, slab = warp - pair * NS, row0 = 16 * slab;
+    float C[2][KD / 8][4];
+    int lam_row[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const int s = pair + x * pairs;
+        zero_state<KD>(C[x]);
+        lam_row[x] = s;
+        if (s >= bl && s < nslots) {
+            const int lh = nth_cross(s - bl);
+            lam_row[x] = bl + lh;
+            load_slab_f32<KD, true>(C[x], a.entry + (((size_t)gb * a.nhigh_max + lh) * H + h) * R::STATE_FLOATS, slab, lane);
+        }
+    }
+    for (int i = 0; i < nsteps; ++i) {
+        const unsigned char* st = feed.step(i);
+        const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
+        const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
+        const __nv_bfloat16* sQt = reinterpret_cast<const __nv_bfloat16*>(st + R::QT_OFF);
+        const float* sLam = reinterpret_cast<const float*>(st + R::LAM_OFF);
+        const int n = b * bc + i;
+        const bool more = i + 1 < nsteps;
+        uint32_t sp[2][KD / 16][4];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int s = pair + x * pairs;
+            if (s >= nslots) continue;
+            pack_state<KD>(C[x], sp[x]);
+            if (!more) continue;
+            if (s < bl) {
+                const int per = 2 << s, pos = n & (per - 1);
+                if (((n >> s) & 1) == 0) load_slab_bf16<KD>(C[x], sBt, row0, lane);      // collects
+                else zero_state<KD>(C[x]);
+                if (pos != per - 1 && pos != 0) state_times_mt<KD>(C[x], sp[x], sM, lane);      // cleared at the end of its period
+            } else {
+                zero_state<KD>(C[x]);
+                state_times_mt<KD>(C[x], sp[x], sM, lane);
+            }
+        }
+        float O[4][2][4];
+        bool any = false;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int s = pair + x * pairs;
+            if (!read_slot(s, n)) continue;
+            float tmp[4][2][4];
+            read_tiles<KD, 4>(tmp, sp[x], sQt, 0, lane);
+            const bool has = lam_row[x] < a.LC;               // a missing row is only reachable when the level check already failed
+            const float* lr = sLam + (has ? lam_row[x] : 0) * CHUNK;
+#pragma unroll
+            for (int mt = 0; mt < 4; ++mt) {
+                const float l0 = has ? lr[mt * 16 + g] : 0.f, l1 = has ? lr[mt * 16 + g + 8] : 0.f;
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    if (any) {
+                        O[mt][nt][0] += l0 * tmp[mt][nt][0]; O[mt][nt][1] += l0 * tmp[mt][nt][1];
+                        O[mt][nt][2] += l1 * tmp[mt][nt][2]; O[mt][nt][3] += l1 * tmp[mt][nt][3];
+                    } else {
+                        O[mt][nt][0] = l0 * tmp[mt][nt][0]; O[mt][nt][1] = l0 * tmp[mt][nt][1];
+                        O[mt][nt][2] = l1 * tmp[mt][nt][2]; O[mt][nt][3] = l1 * tmp[mt][nt][3];
+                    }
+                }
+            }
+            any = true;
+        }
+        if (any) {
+            float4* d = part + (i & 1) * buf_stride + (pair * NS + slab) * 256 + lane;
+#pragma unroll
+            for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) d[(mt * 2 + nt) * 32] = make_float4(O[mt][nt][0], O[mt][nt][1], O[mt][nt][2], O[mt][nt][3]);
+        }
+    }
+    feed.step(nsteps);
+}
+
 // ---- launchers ------------------------------------------------------------------------------------
 template <typename KernelT>
 static int set_smem(KernelT kern, int bytes) {
@@ -941,6 +1142,16 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
 }
 
 template <int KD, int VD>
+static int launch_out_levels(const GdnArgs& a, int pairs, cudaStream_t st) {
+    const int smem = LevelsSmem<KD, VD>::bytes(a.LC, pairs);
+    LAMPA_TRY(set_smem(gdn_out_levels_kernel<KD, VD>, smem));
+    ProfScope prof("gdn_out_hier", st);
+    launch_chained(gdn_out_levels_kernel<KD, VD>, dim3(a.nb_max, a.H), (2 * pairs + 1 + LV_SUM) * 32, smem, st, a, pairs);
+    LAMPA_LAUNCHED();
+    return LAMPA_OK;
+}
+
+template <int KD, int VD>
 int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
     const int ng = 1 + (a.nhigh_max + NLW - 1) / NLW;
     if (ng > MAX_GROUPS) return LAMPA_ERR_UNSUPPORTED;
@@ -949,6 +1160,10 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
         LAMPA_TRY((launch_level<KD, VD, true>(a, a.nhigh_max, st)));
     }
     if (KD == 64 && VD == 64 && a.nhigh_max <= 5 && a.use_umma) return launch_out_hier_umma(a, st);
+    if constexpr (KD <= 32) {
+        const int pairs = ((a.nlev_max > MIN_BLOCK_LOG ? a.nlev_max : MIN_BLOCK_LOG) + 1) / 2;      // a block has at most a slot per level of its sequence
+        if ((int64_t)a.nb_max * a.H <= sm_count() && pairs <= LV_MAX_PAIRS && LevelsSmem<KD, VD>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD>(a, pairs, st);
+    }
     if (ng == 1) return launch_out_hier<KD, VD, 1>(a, st);
     if (ng == 2) return launch_out_hier<KD, VD, 2>(a, st);
     return launch_out_hier<KD, VD, 3>(a, st);

@@ -65,3 +65,13 @@ def test_fp16_rows(K, V, T):
     inp = synth.gdn_inputs(33, T, 3, K, V, g_shift=-3.0)
     o, _ = _call(inp, 0, dt=torch.float16)
     assert_close_bf16(o, _ref(inp, 0)[0], "o fp16")
+
+
+# blocks x heads at most 148 and above it: levels shared out over warps, or five to a warp; a sequence of one block, a ragged one,
+# blocks of 8, 16 and 32 chunks
+@pytest.mark.parametrize("K,V", [(32, 32), (16, 32)])
+@pytest.mark.parametrize("T,H", [(64 * 3, 1), (64 * 8 * 9 + 5, 3), (64 * 256, 4), (64 * 300, 6), (64 * 304, 8), (64 * 520, 2)])
+def test_levels_by_warp(K, V, T, H):
+    from lampa_b200 import synth
+    inp = synth.gdn_inputs(34, T, H, K, V, L=18, g_shift=-4.0)
+    assert_close_bf16(_call(inp, 18)[0], _ref(inp, 18)[0], f"o, levels {T}x{H}")
