@@ -8,6 +8,7 @@
 // holds one token and level l >= 1 holds 2^(l-1) tokens exactly when bit l-1 of T - 1 is set.
 #include "gdn.cuh"
 #include "profile.cuh"
+#include "tmap.cuh"
 
 #include <type_traits>
 
@@ -1009,12 +1010,13 @@ int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
 // time, but they alternate inside every 32-byte sector, so the whole tensor moves.  A thread that
 // walks the levels of its own element touches 4 bytes per sector and instruction: 148 us for 64 rows
 // x 8 heads of 64 x 64 x 17 levels (286 MB, 1.9 TB/s).  Here a CTA owns 8 state columns: their
-// K rows of 8 * L floats (544 bytes at L = 17) enter shared memory as bulk copies, are updated in
-// place and leave the same way: 65 us (4.4 TB/s).  Eight columns keep the slab at 35 KB, so that
-// five CTAs per SM overlap their copies with each other's arithmetic, and give even a single stream
-// of 4 heads of 32 columns 16 CTAs.  Two rows per thread, not four: the arithmetic is a chain of
-// shared-memory round trips, and half the warps took 76 us.  16-byte cp.async and vector stores
-// instead of the bulk copies: 97 us.
+// K rows of 8 * L floats (544 bytes at L = 17) enter shared memory as one tiled copy, are updated in
+// place and leave the same way: 56 us (5.1 TB/s, 78 % of the measured copy).  A bulk copy per row, 64 in and
+// 64 out, kept the copy unit busier than the memory: 61 us, and 7.9 instead of 6.9 for four rows.
+// Eight columns keep the slab at 35 KB, so that five CTAs per SM overlap their copies with each
+// other's arithmetic, and give even a single stream of 4 heads of 32 columns 16 CTAs.  Two rows per
+// thread, not four: the arithmetic is a chain of shared-memory round trips, and half the warps took
+// 76 us (against 65 then).  16-byte cp.async and vector stores instead of the bulk copies: 97 us.
 // -------------------------------------------------------------------------------------------------
 __device__ __forceinline__ int cascade_depth(const int32_t* counts, int L, int& merged, bool& overflow) {
     // levels 0 .. depth-1 move into level `depth`, which then holds `merged` tokens
@@ -1045,10 +1047,10 @@ template <int KD> __host__ __device__ constexpr int step_smem(int L) {      // s
 }
 
 template <int KD, int VD>
-__global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s) {
+__global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s, const __grid_constant__ CUtensorMap map, int tiled) {
     if (chain_wait()) return;
     constexpr int NT = STEP_THREADS<KD>, NW = NT / 32, KI = STEP_KI;        // lane = (4 rows, 8 columns)
-    extern __shared__ __align__(16) float slab[];              // [KD][8][L]
+    extern __shared__ __align__(128) float slab[];              // [KD][8][L]
     float* part = slab + KD * STEP_COLS * s.L;                 // [2][warps][L][8]: k^T S and q^T S of every level
     float* sC = part + 2 * NW * STEP_COLS * s.L;               // [L][8]: beta k^T S
     __shared__ float sK[KD], sQ[KD], sLam[STEP_MAX_L], sQk;
@@ -1068,7 +1070,9 @@ __global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s)
         if (bulk) mbar_expect_tx(&bar, KD * row_bytes);
     }
     __syncthreads();
-    if (bulk) {
+    if (tiled) {
+        if (tid == 0) tma_load_2d(slab, &map, v0 * L, (int32_t)(bh * KD), &bar);
+    } else if (bulk) {
         if (tid < KD) bulk_g2s(slab + (size_t)tid * STEP_COLS * L, gsrc + (size_t)tid * VD * L, row_bytes, &bar);
     } else {
         for (int i = tid; i < KD * STEP_COLS * L; i += NT) {
@@ -1197,7 +1201,9 @@ __global__ void __launch_bounds__(STEP_THREADS<KD>) hgdn_step_kernel(StepArgs s)
     if (bulk) {
         fence_async_shared();
         __syncthreads();
-        if (tid < KD) {
+        if (tiled) {
+            if (tid == 0) { tma_store_2d(&map, v0 * L, (int32_t)(bh * KD), slab); bulk_commit(); }
+        } else if (tid < KD) {
             bulk_s2g(gsrc + (size_t)tid * VD * L, slab + (size_t)tid * STEP_COLS * L, row_bytes);
             bulk_commit();
         }
@@ -1231,9 +1237,14 @@ int launch_hgdn_step(const StepArgs& s, cudaStream_t st) {
     const int smem = step_smem<KD>(s.L);           // at most 103 KB
     if (smem > 44 * 1024 && cudaFuncSetAttribute(hgdn_step_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
+    // one tiled copy per slab, up to 32 levels (a box is at most 256 elements wide)
+    CUtensorMap map = {};
+    const int64_t rows = (int64_t)s.B * s.H * KD;
+    const int tiled = ((uintptr_t)s.states & 15) == 0 && STEP_COLS * s.L <= 256 && rows <= INT32_MAX &&
+                      make_map(&map, s.states, LAMPA_F32, (uint64_t)rows, (uint64_t)VD * s.L, STEP_COLS * s.L, KD, false);
     {
         ProfScope prof("hgdn_step", st);
-        launch_chained(hgdn_step_kernel<KD, VD>, dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS<KD>, smem, st, s);
+        launch_chained(hgdn_step_kernel<KD, VD>, dim3((unsigned)s.B * (VD / STEP_COLS), s.H), STEP_THREADS<KD>, smem, st, s, map, tiled);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
     }
     if (s.arrivals) return LAMPA_OK;

@@ -1,4 +1,4 @@
-// Tiled TMA loads: tensor maps of row-major 2-byte matrices, and the copy of one box.
+// Tiled TMA copies: tensor maps of row-major matrices, and the copy of one box.
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -12,6 +12,11 @@ namespace lampa {
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int32_t x, int32_t y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
                  :: "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+}
+// one box from shared memory (inside the tensor: x, y >= 0), part of the bulk group of the issuing thread
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int32_t x, int32_t y, const void* src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n"
+                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(src)) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t x, int32_t y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n"
@@ -31,15 +36,17 @@ inline PFN_cuTensorMapEncodeTiled tensor_map_encoder() {
     return fn;
 }
 
-// [rows][cols] 2-byte tensor, row pitch = cols elements, box of box_rows x box_cols
+// [rows][cols] tensor, row pitch = cols elements, box of box_rows x box_cols
 inline bool make_map(CUtensorMap* m, const void* base, int dt, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows, bool swizzle) {
     PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
     if (!enc) return false;
     const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * 2};
+    const cuuint64_t strides[1] = {cols * (cuuint64_t)dtype_bytes(dt)};
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    return enc(m, dt == LAMPA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base),
+    const CUtensorMapDataType type = dt == LAMPA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : dt == LAMPA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                                                                                 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    return enc(m, type, 2, const_cast<void*>(base),
                dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;

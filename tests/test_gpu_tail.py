@@ -60,3 +60,28 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
                 assert (e.abs() <= eps * ro[n0:].abs() + 2 * bound * ro[n0:].abs().max()).all()
     want = [1 if T > 0 else 0] + [(1 << (l - 1)) if ((T - 1) >> (l - 1)) & 1 else 0 for l in range(1, L)]
     assert st.counts.view(-1)[:L].tolist() == want
+
+
+# one tiled copy per slab up to 32 levels, row by row beyond; more slabs than fit the GPU at once, and few
+@pytest.mark.parametrize("K,V,H,B,L", [(64, 64, 4, 10, 17), (64, 64, 1, 37, 32), (64, 64, 1, 37, 33), (32, 32, 4, 19, 9), (16, 32, 8, 12, 17)])
+def test_steps_of_large_batches(K, V, H, B, L):
+    """Every row of a batch is stepped as it is alone, bit for bit."""
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+
+    def draw(T):
+        return (rn(B, T, H, K).bfloat16(), rn(B, T, H, K).bfloat16(), rn(B, T, H, V).bfloat16(), -F.softplus(rn(B, T, H) - 3),
+                F.softplus(rn(B, T, H, L)), torch.sigmoid(rn(B, T, H)))
+
+    def run(x, state=None):
+        return lampa_b200.chunk_h_gated_delta_rule(*x, initial_state=state, output_final_state=True, use_qk_l2norm_in_kernel=True)
+
+    prompt, steps = draw(70), [draw(1) for _ in range(5)]
+    _, state = run(prompt)
+    rows = [run([t[i : i + 1].contiguous() for t in prompt])[1] for i in range(B)]
+    for x in steps:
+        o, state = run(x, state)
+        for i in range(B):
+            oi, rows[i] = run([t[i : i + 1].contiguous() for t in x], rows[i])
+            assert torch.equal(o[i], oi[0]) and torch.equal(state.states[i], rows[i].states[0])
+    lampa_b200.check_status(torch.device("cuda:0"))
