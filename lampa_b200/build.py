@@ -13,7 +13,7 @@ SO = os.path.join(HERE, "liblampa_b200.so")
 HOST_SO = os.path.join(HERE, "_host.so")
 HOST_SOURCES = ["host.cpp", "host_lsh.inc", "host_model.inc", "host_hept.inc"]
 SOURCES = ["lsh.cu", "geo.cu", "layer.cu", "model.cu", "bucket_attn.cu", "gdn_prep.cu", "gdn_prep_umma.cu", "gdn_scan.cu", "gdn_scan_umma.cu", "gdn_state.cu", "gdn_api.cu", "profile.cu"]
-HEADERS = ["common.cuh", "gdn.cuh", "gdn_inv.cuh", "gdn_load.cuh", "umma.cuh", "tmap.cuh", "act.cuh", "profile.cuh", os.path.join("..", "..", "include", "lampa_b200.h")]
+HEADERS = ["common.cuh", "gdn.cuh", "gdn_inv.cuh", "gdn_load.cuh", "umma.cuh", "tmap.cuh", "act.cuh", "split3.cuh", "profile.cuh", os.path.join("..", "..", "include", "lampa_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
 

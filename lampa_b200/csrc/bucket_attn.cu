@@ -27,6 +27,7 @@
 //
 // HBM traffic per (round, head, hit): the q, k, v rows once and the so row + denom once.
 #include "common.cuh"
+#include "split3.cuh"
 #include "profile.cuh"
 #include <algorithm>
 
@@ -296,17 +297,6 @@ __global__ void __launch_bounds__(BA_MAX_WARPS * 32, BA_QROWS == 4 ? 3 : 2) buck
 // at most 32 hits stay with the FMA kernel (two warps' worth of 16-row tiles), and so do wider rows: their fragments in
 // three pieces do not fit the registers and the kernel is slower than FMA there.
 // -------------------------------------------------------------------------------------------------
-struct Split3 { uint32_t h, m, l; };
-__device__ __forceinline__ Split3 split3(float x, float y) {
-    Split3 s;
-    s.h = pack_bf16x2(x, y);
-    const float2 h = unpack_bf16x2(s.h);
-    const float rx = x - h.x, ry = y - h.y;
-    s.m = pack_bf16x2(rx, ry);
-    const float2 m = unpack_bf16x2(s.m);
-    s.l = pack_bf16x2(rx - m.x, ry - m.y);
-    return s;
-}
 // c[i] += a b_i for operands in three pieces and NT column tiles (two per fragment), one piece of b in registers at a time
 // (low first); `load` fetches the fragments of a piece.  Consecutive instructions go to different accumulators.
 template <int NT, class Load>

@@ -199,7 +199,7 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 // for kernels that leave most of the GPU idle and for a next one that can do without them: everywhere else the next grid only
 // fills the SMs that happen to be free, two or three CTAs to an SM beside idle ones (56 and 447 us, and 486 instead of 463 for a
 // 60,000-hit event).  chain_signal comes behind chain_wait: what the kernel was waiting for is complete for the next one
-// too, which may read it (from L2) before its own wait.  That one still waits before it ends, so that its end means theirs.
+// too, which may read it (from L2) before its own wait.  A CTA of that one still waits before it ends, so that its end means theirs.
 __device__ __forceinline__ bool chain_wait() {
     uint32_t never;
     asm volatile("griddepcontrol.wait;\n mov.u32 %0, 0;\n" : "=r"(never) :: "memory");

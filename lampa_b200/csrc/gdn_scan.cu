@@ -481,7 +481,8 @@ __global__ void __launch_bounds__(NW * 32 + 32) gdn_level_kernel(GdnArgs a) {
 template <int KD, int VD>
 __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a, float* states) {
     // In a prefill the output pass in front lets this one in at its start: it needs nothing of that pass, only what was complete
-    // before it, so it runs beside it, signals in turn and waits at its end.
+    // before it, so it runs beside it and signals in turn.  One CTA waits at its end, which keeps the grid's end behind that pass's;
+    // the others give their SMs to the prompt's tail.
     if (a.signal) chain_signal();
     else if (chain_wait()) return;
     using R = Rec<KD, VD>;
@@ -504,18 +505,18 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
         Feed<NST, NW * 32 + 32, 1> feed;
         feed.bar = reinterpret_cast<uint64_t*>(smem);
         feed.stage = smem + 1024;
-        feed.step_bytes = R::PRE_BYTES;
+        feed.step_bytes = R::M_BYTES + R::BT_BYTES;
         feed.src = a.rec + ((size_t)(sq.c0 + c_first) * H + h) * a.rec_bytes;
         feed.src_stride = (size_t)H * a.rec_bytes;
-        feed.copy_bytes = R::PRE_BYTES;
+        feed.copy_bytes = R::M_BYTES;
+        feed.src2 = R::BT_OFF;
         feed.nsteps = n - c_first + 1;
         feed.status = a.status;
         feed.budget = a.poll_budget;
-        feed.copy2 = 0;
+        feed.copy2 = R::BT_BYTES;
         feed.start(warp == NW);
         if (warp == NW) {
             feed.produce();
-            if (a.signal) (void)chain_wait();
             return;
         }
         if (lev >= bl) {
@@ -524,8 +525,8 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
         }
         for (int i = 0; i < feed.nsteps; ++i) {
             const unsigned char* st = feed.step(i);
-            const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
-            const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
+            const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st);
+            const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::M_BYTES);
             // the state enters the tensor core as bf16 hi + bf16 lo (two products), so that re-rounding
             // it at every chunk does not accumulate in the state handed to the caller
             uint32_t sp[KD / 16][4], sl[KD / 16][4];
@@ -546,8 +547,8 @@ __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a,
             }
         }
     }
-    if (a.signal && chain_wait()) return;
     if (warp == NW) return;
+    if (a.signal && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && chain_wait()) return;
     float* dst = states + ((size_t)seq * H + h) * KD * VD * a.L + ELL0 + lev;
 #pragma unroll
     for (int nt = 0; nt < KD / 8; ++nt)
@@ -1173,7 +1174,7 @@ template <int KD, int VD>
 int launch_final_high(const GdnArgs& a, float* states, cudaStream_t st) {
     using R = Rec<KD, VD>;
     if (a.L <= ELL0) return LAMPA_OK;
-    const int smem = 1024 + 3 * R::PRE_BYTES;
+    const int smem = 1024 + 3 * (R::M_BYTES + R::BT_BYTES);
     LAMPA_TRY(set_smem(hgdn_final_high_kernel<KD, VD>, smem));
     ProfScope prof("hgdn_final_high", st);
     launch_chained(hgdn_final_high_kernel<KD, VD>, dim3(a.nseq, a.H, a.L - ELL0), VD * 2 + 32, smem, st, a, states);

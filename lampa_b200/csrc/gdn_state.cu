@@ -8,6 +8,7 @@
 // holds one token and level l >= 1 holds 2^(l-1) tokens exactly when bit l-1 of T - 1 is set.
 #include "gdn.cuh"
 #include "profile.cuh"
+#include "split3.cuh"
 #include "tmap.cuh"
 
 #include <type_traits>
@@ -108,8 +109,9 @@ struct TailSmem {                                            // offsets in float
     static constexpr int P = Q + CHUNK * KP;                 // [64][AP], then R
     static constexpr int OUT = P + CHUNK * TAIL_AP;          // [64][8]
     static constexpr int LAM = OUT + CHUNK * TAIL_COLS;      // [64][L], then the slab [KD][8][L]
-    static constexpr int X = 0, D = KD * TAIL_XP;            // slots and K X over the last chunk's k and T, which are done with by then
-    static_assert(KD * TAIL_XP + CHUNK * TAIL_XP <= V_, "slots must fit");
+    // slots, K X, and what a batch of slots adds to the outputs, over the last chunk, which is done with by then
+    static constexpr int X = 0, D = KD * TAIL_XP, Y = D + CHUNK * TAIL_XP;
+    static_assert(Y + CHUNK * TAIL_XP <= CH, "slots must fit");
     static_assert(CH % 4 == 0 && Q % 4 == 0 && LAM % 4 == 0, "16-byte rows");
     __host__ __device__ static constexpr int floats(bool tail, int L) { return tail ? LAM + (CHUNK * L + 3) / 4 * 4 + KD * TAIL_COLS * L : B; }
 };
@@ -140,36 +142,29 @@ __device__ __forceinline__ void tail_inverse(float* A, const float* beta, int t,
         for (int i = 0; i < 16; ++i) A[(m0 + i) * AP + m0 + cc] = x[i];
     }
     tail_meet(grp);
-    // X_ba = -X_bb (A_ba X_aa) for blocks of W = 16, then 32; the inner product waits in the mirror image above the diagonal.
-    // The sums run over whole rows: what they need not take in is zero.
+    // X_ba = -X_bb (A_ba X_aa) for blocks of W = 16, then 32; the inner product waits in the mirror image above the diagonal.  A warp
+    // forms a tile of 16 x 8.
     auto corner = [&](auto width) {
-        constexpr int W = decltype(width)::value;
-        constexpr int per = W * W / 4, np = 32 / W;          // threads (4 columns each) and pairs
-        const bool on = t < per * np;
-        const int p = t / per, u = t - p * per, r = u / (W / 4), c = (u % (W / 4)) * 4;
-        const int a0 = 2 * W * p, b0 = a0 + W;
-        auto product = [&](const float* left, const float* right) {
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int k = 0; k < W; k += 4) {
-                const float4 f4 = *reinterpret_cast<const float4*>(left + k);
-                const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+        constexpr int W = decltype(width)::value, MT = W / 16, NT = W / 8;
+        const int w = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
+        const bool on = w < (32 / W) * MT * NT;              // (pair, row tile, column tile)
+        const int p = w / (MT * NT), mt = (w / NT) % MT, n0 = (w % NT) * 8, a0 = 2 * W * p, b0 = a0 + W;
+        auto product = [&](const float* left, const float* right, float* dst, float sign) {
+            if (!on) return;
+            float c[1][1][4] = {};
+            const float* const l1[1] = {left};
+            tile_product3<1, 1, false, false>(c, l1, AP, 16 * mt, right, AP, n0, 1, 0, W, lane);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 v = *reinterpret_cast<const float4*>(right + (k + q) * AP);
-                    s.x = fmaf(f[q], v.x, s.x); s.y = fmaf(f[q], v.y, s.y); s.z = fmaf(f[q], v.z, s.z); s.w = fmaf(f[q], v.w, s.w);
-                }
-            }
-            return s;
+            for (int hh = 0; hh < 2; ++hh)
+                *reinterpret_cast<float2*>(dst + (16 * mt + gq + 8 * hh) * AP + n0 + 2 * tq) = make_float2(sign * c[0][0][2 * hh], sign * c[0][0][2 * hh + 1]);
         };
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (on) s = product(A + (b0 + r) * AP + a0, A + a0 * AP + a0 + c);
-        if (on) *reinterpret_cast<float4*>(A + (a0 + r) * AP + b0 + c) = s;
+        product(A + b0 * AP + a0, A + a0 * AP + a0, A + a0 * AP + b0, 1.f);
         tail_meet(grp);
-        if (on) s = product(A + (b0 + r) * AP + b0, A + a0 * AP + b0 + c);
-        if (on) *reinterpret_cast<float4*>(A + (b0 + r) * AP + a0 + c) = make_float4(-s.x, -s.y, -s.z, -s.w);
+        product(A + b0 * AP + b0, A + a0 * AP + b0, A + b0 * AP + a0, -1.f);
         tail_meet(grp);
-        if (on) *reinterpret_cast<float4*>(A + (a0 + r) * AP + b0 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) *reinterpret_cast<float2*>(A + (a0 + 16 * mt + gq + 8 * hh) * AP + b0 + n0 + 2 * tq) = make_float2(0.f, 0.f);
         tail_meet(grp);
     };
     corner(std::integral_constant<int, 16>{});
@@ -192,7 +187,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     constexpr int KP = M::KP, AP = TAIL_AP, XP = TAIL_XP;
     extern __shared__ __align__(16) float sm[];
     const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
-    const int tid = threadIdx.x, lane = tid & 31, grp = tid / TAIL_GRP, t = tid % TAIL_GRP;
+    const int tid = threadIdx.x, lane = tid & 31, gq = lane >> 2, tq = lane & 3, grp = tid / TAIL_GRP, t = tid % TAIL_GRP;
     const int v0 = blockIdx.z * TAIL_COLS;
     int nch = ta.n0;
     int64_t tok0 = (int64_t)seq * a.fixed_stride, tok_end = 0;
@@ -267,7 +262,9 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         auto lam_load = [&](int p) { return load_raw(a.lam, ((size_t)(t0 + p / L) * H + h) * L + p % L, a.lam_dt, p < nlam); };
 #pragma unroll
         for (int it = 0; it < NL; ++it) lv[it] = lam_load(t + it * TAIL_GRP);
-        const float g0 = raw_float(g0w, a.gb_dt), g1 = raw_float(g1w, a.gb_dt), bt = raw_float(btw, a.gb_dt);
+        // e^g is zero far above -1e5; a g of minus infinity would make differences of G undefined
+        auto decay = [&](uint32_t w) { const float g = raw_float(w, a.gb_dt); return g < -1e5f ? -1e5f : g; };
+        const float g0 = decay(g0w), g1 = decay(g1w), bt = raw_float(btw, a.gb_dt);
         if (t < CHUNK) sBeta[t] = bt;
 #pragma unroll
         for (int it = 0; it < NV; ++it) sV[t + it * TAIL_GRP] = raw_float(vv[it], a.qkv_dt);
@@ -326,81 +323,62 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             sEl[2 * t] = __expf((float)(last - (cs - (double)g1))); sEl[2 * t + 1] = __expf((float)(last - cs));
         }
         tail_meet(grp);
-        {   // A = tril(diag(beta) K K^T .* E, -1), P = tril(Q K^T .* E): rows ti + 16 x, columns tj + 16 y of the blocks y <= x
-            const int ti = t >> 4, tj = t & 15;
-            float kk[10], qk[10];
+        {   // A = tril(diag(beta) K K^T .* E, -1), P = tril(Q K^T .* E): warp = (16 rows, half of the column tiles up to the diagonal)
+            const int mt = (t >> 5) & 3, half = t >> 7, cnt = mt + 1, n0 = 8 * half * cnt;
+            float c[2][4][4];
 #pragma unroll
-            for (int e = 0; e < 10; ++e) kk[e] = qk[e] = 0.f;
-#pragma unroll 1
-            for (int c = 0; c < KD; c += 4) {
-                float4 ki[4], kj[4], qi[4];
+            for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int x4 = 0; x4 < 4; ++x4) {
-                    ki[x4] = *reinterpret_cast<const float4*>(sK + (ti + 16 * x4) * KP + c);
-                    kj[x4] = *reinterpret_cast<const float4*>(sK + (tj + 16 * x4) * KP + c);
-                    if (tail) qi[x4] = *reinterpret_cast<const float4*>(sQ + (ti + 16 * x4) * KP + c);
-                }
-                int e = 0;
-#pragma unroll
-                for (int xi = 0; xi < 4; ++xi)
-#pragma unroll
-                    for (int yj = 0; yj <= xi; ++yj, ++e) {
-                        kk[e] = fmaf(ki[xi].w, kj[yj].w, fmaf(ki[xi].z, kj[yj].z, fmaf(ki[xi].y, kj[yj].y, fmaf(ki[xi].x, kj[yj].x, kk[e]))));
-                        if (tail) qk[e] = fmaf(qi[xi].w, kj[yj].w, fmaf(qi[xi].z, kj[yj].z, fmaf(qi[xi].y, kj[yj].y, fmaf(qi[xi].x, kj[yj].x, qk[e]))));
-                    }
+                for (int nt = 0; nt < 4; ++nt) { c[x][nt][0] = c[x][nt][1] = c[x][nt][2] = c[x][nt][3] = 0.f; }
+            if (tail) {
+                const float* const kq[2] = {sK, sQ};
+                tile_product3<2, 4, false, true>(c, kq, KP, 16 * mt, sK, KP, n0, cnt, 0, KD, lane);
+            } else {
+                const float* const k1[1] = {sK};
+                tile_product3<1, 4, false, true>(reinterpret_cast<float (&)[1][4][4]>(c), k1, KP, 16 * mt, sK, KP, n0, cnt, 0, KD, lane);
             }
-            int e = 0;
 #pragma unroll
-            for (int xi = 0; xi < 4; ++xi)
+            for (int nt = 0; nt < 4; ++nt) {
+                if (nt >= cnt) break;
 #pragma unroll
-                for (int yj = 0; yj < 4; ++yj) {
-                    const int i = ti + 16 * xi, j = tj + 16 * yj;
-                    float av = 0.f, pv = 0.f;
-                    if (yj <= xi) {
-                        const float f = j <= i ? __expf((float)(sG[i] - sG[j])) : 0.f;
-                        if (j < i) av = sBeta[i] * kk[e] * f;
-                        pv = qk[e] * f;
-                        ++e;
-                    }
-                    sA[i * AP + j] = av;
-                    if (tail) sP[i * AP + j] = pv;
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * mt + gq + 8 * hh, j = n0 + 8 * nt + 2 * tq;
+                    const float f0 = j <= i ? __expf((float)(sG[i] - sG[j])) : 0.f, f1 = j + 1 <= i ? __expf((float)(sG[i] - sG[j + 1])) : 0.f;
+                    const float bi = sBeta[i];
+                    *reinterpret_cast<float2*>(sA + i * AP + j) = make_float2(j < i ? bi * c[0][nt][2 * hh] * f0 : 0.f, j + 1 < i ? bi * c[0][nt][2 * hh + 1] * f1 : 0.f);
+                    if (tail) *reinterpret_cast<float2*>(sP + i * AP + j) = make_float2(c[1][nt][2 * hh] * f0, c[1][nt][2 * hh + 1] * f1);
+                }
+            }
+            for (int u = 2 * cnt + half; u < 8; u += 2)      // nothing above the diagonal
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int at = (16 * mt + gq + 8 * hh) * AP + 8 * u + 2 * tq;
+                    *reinterpret_cast<float2*>(sA + at) = make_float2(0.f, 0.f);
+                    if (tail) *reinterpret_cast<float2*>(sP + at) = make_float2(0.f, 0.f);
                 }
         }
         tail_meet(grp);
         tail_inverse(sA, sBeta, t, grp);
         if (!tail && tailed) {                               // all tokens of the last chunk as one state: they join a slot
-            {
-                const int i = t >> 2, jg = t & 3;            // row i, all columns, every fourth token
-                float u[TAIL_COLS];
+            const int w = t >> 5;
+            if (w < 4) {
+                float c[1][1][4] = {};
+                const float* const T1[1] = {sA};
+                tile_product3<1, 1, false, false>(c, T1, AP, 16 * w, sV, TAIL_COLS, 0, 1, 0, 16 * w + 16, lane);
 #pragma unroll
-                for (int v = 0; v < TAIL_COLS; ++v) u[v] = 0.f;
-#pragma unroll 4
-                for (int j = jg; j < CHUNK; j += 4) {        // T is zero above the diagonal
-                    const float f = sA[i * AP + j];
-                    const float4 p = *reinterpret_cast<const float4*>(sV + j * TAIL_COLS), q = *reinterpret_cast<const float4*>(sV + j * TAIL_COLS + 4);
-                    u[0] = fmaf(f, p.x, u[0]); u[1] = fmaf(f, p.y, u[1]); u[2] = fmaf(f, p.z, u[2]); u[3] = fmaf(f, p.w, u[3]);
-                    u[4] = fmaf(f, q.x, u[4]); u[5] = fmaf(f, q.y, u[5]); u[6] = fmaf(f, q.z, u[6]); u[7] = fmaf(f, q.w, u[7]);
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * w + gq + 8 * hh;
+                    *reinterpret_cast<float2*>(sZ + i * XP + 2 * tq) = make_float2(sEl[i] * c[0][0][2 * hh], sEl[i] * c[0][0][2 * hh + 1]);
                 }
-#pragma unroll
-                for (int v = 0; v < TAIL_COLS; ++v) {
-                    u[v] += __shfl_xor_sync(0xffffffffu, u[v], 1);
-                    u[v] += __shfl_xor_sync(0xffffffffu, u[v], 2);
-                }
-                const float el = sEl[i];
-                if (jg < 2) *reinterpret_cast<float4*>(sZ + i * XP + 4 * jg) = jg == 0 ? make_float4(el * u[0], el * u[1], el * u[2], el * u[3])
-                                                                                    : make_float4(el * u[4], el * u[5], el * u[6], el * u[7]);
             }
             tail_meet(grp);
-            for (int o = t; o < KD * 4; o += TAIL_GRP) {     // row k, two columns
-                const int k = o >> 2, v = (o & 3) * 2;
-                float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-                for (int i = 0; i < CHUNK; ++i) {
-                    const float f = sK[i * KP + k];
-                    const float2 z = *reinterpret_cast<const float2*>(sZ + i * XP + v);
-                    s0 = fmaf(f, z.x, s0); s1 = fmaf(f, z.y, s1);
-                }
-                *reinterpret_cast<float2*>(sSum + k * TAIL_COLS + v) = make_float2(s0, s1);
+            if (w < KD / 16) {
+                float c[1][1][4] = {};
+                const float* const k1[1] = {sK};
+                tile_product3<1, 1, true, false>(c, k1, KP, 16 * w, sZ, XP, 0, 1, 0, CHUNK, lane);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+                    *reinterpret_cast<float2*>(sSum + (16 * w + gq + 8 * hh) * TAIL_COLS + 2 * tq) = make_float2(c[0][0][2 * hh], c[0][0][2 * hh + 1]);
             }
         }
     }
@@ -410,71 +388,43 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const float* cs = sm + (tailed ? M::B : 0);
     const float *cK = cs + M::K_, *cT = cs + M::A_, *cV = cs + M::V_, *cEg = cs + M::S_ + 2 * CHUNK, *cEl = cEg + CHUNK;
     const int r_all = tailed ? done : (nch > 0 ? CHUNK : 0);
-    const int row = tid >> 3, c8 = tid & 7;                  // row; four of 32 columns: state c8 / 2 of the batch, its half c8 % 2
+    const int row = tid >> 3, c8 = tid & 7;                  // row and column of what goes element by element
+    const int warp = tid >> 5, mt = warp & 3, nt = warp >> 2;       // products: 16 rows, and eight columns: state nt of a batch
 
     // where a state element of the result goes: the slab, which leaves at the end, or (no tail) the state itself
     auto put = [&](int k, int v, int l, float x) {
         if (tailed) slab[(k * TAIL_COLS + v) * L + l] = x;
         else st[((size_t)k * VD + v) * L + l] = x;
     };
-    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z; thread = four rows k, four columns, every fourth token
-    auto kt_product = [&](const float* X, auto level_of) {
-        if (tid < KD * 8) {
-            const int ig = tid & 3, c = (tid >> 2) & 7, k0 = (tid >> 5) * 4;
-            float acc[4][4];
+    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z, state nt to level l
+    auto kt_product = [&](const float* X, int l) {
+        if (mt >= KD / 16 || l < 0 || l >= L) return;        // (warp-uniform)
+        float c[1][1][4] = {};
+        const float* const k1[1] = {cK};
+        tile_product3<1, 1, true, false>(c, k1, KP, 16 * mt, sZ, XP, 8 * nt, 1, 0, CHUNK, lane);
+        const float egl = cEg[CHUNK - 1];
 #pragma unroll
-            for (int x = 0; x < 4; ++x) { acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f; }
-#pragma unroll 4
-            for (int i = ig; i < CHUNK; i += 4) {
-                const float4 k4 = *reinterpret_cast<const float4*>(cK + i * KP + k0);
-                const float4 z4 = *reinterpret_cast<const float4*>(sZ + i * XP + 4 * c);
-                const float kx[4] = {k4.x, k4.y, k4.z, k4.w}, zx[4] = {z4.x, z4.y, z4.z, z4.w};
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) acc[x][y] = fmaf(kx[x], zx[y], acc[x][y]);
-            }
-            float half[2][4], res[4];                        // summed over the four token groups, lane ig left with row ig
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-                for (int y = 0; y < 4; ++y) {
-                    const float give = ig & 2 ? acc[x][y] : acc[x + 2][y];
-                    half[x][y] = (ig & 2 ? acc[x + 2][y] : acc[x][y]) + __shfl_xor_sync(0xffffffffu, give, 2);
-                }
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                const float give = ig & 1 ? half[0][y] : half[1][y];
-                res[y] = (ig & 1 ? half[1][y] : half[0][y]) + __shfl_xor_sync(0xffffffffu, give, 1);
-            }
-            const int l = level_of(c >> 1), k = k0 + ig;
-            if (l >= 0 && l < L) {
-                const float egl = cEg[CHUNK - 1];
-#pragma unroll
-                for (int y = 0; y < 4; ++y) put(k, 4 * (c & 1) + y, l, X ? egl * X[k * XP + 4 * c + y] - res[y] : res[y]);
-            }
+        for (int e = 0; e < 4; ++e) {
+            const int k = 16 * mt + gq + 8 * (e >> 1), v = 2 * tq + (e & 1);
+            put(k, v, l, X ? egl * X[k * XP + 8 * nt + v] - c[0][0][e] : c[0][0][e]);
         }
     };
 
     if (tailed) {
         for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
-        // R = P T: thread = (row, eight columns); both are lower triangular
-        float4 s[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll 2
-        for (int k = 8 * c8; k <= row; k += 4) {
-            const float4 p4 = *reinterpret_cast<const float4*>(sP + row * AP + k);
-            const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+        // R = P T, both lower triangular: warp = (16 rows, column tiles nt and nt + 4)
+        float c[2][1][1][4] = {};
+        const float* const P1[1] = {sP};
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const float4 v = *reinterpret_cast<const float4*>(cT + (k + u) * AP + 8 * c8 + 4 * q);
-                    s[q].x = fmaf(p[u], v.x, s[q].x); s[q].y = fmaf(p[u], v.y, s[q].y); s[q].z = fmaf(p[u], v.z, s[q].z); s[q].w = fmaf(p[u], v.w, s[q].w);
-                }
-        }
+        for (int x = 0; x < 2; ++x)
+            if (nt + 4 * x <= 2 * mt + 1)
+                tile_product3<1, 1, false, false>(c[x], P1, AP, 16 * mt, cT, AP, 8 * (nt + 4 * x), 1, (nt + 4 * x) / 2 * 16, 16 * mt + 16, lane);
         __syncthreads();
-        *reinterpret_cast<float4*>(sP + row * AP + 8 * c8) = s[0];
-        *reinterpret_cast<float4*>(sP + row * AP + 8 * c8 + 4) = s[1];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+                *reinterpret_cast<float2*>(sP + (16 * mt + gq + 8 * hh) * AP + 8 * (nt + 4 * x) + 2 * tq) = make_float2(c[x][0][0][2 * hh], c[x][0][0][2 * hh + 1]);
         __syncthreads();
         // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
         // row i reads are the 2^(l-1) below the highest set bit they differ in
@@ -515,25 +465,23 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             if (l < ELL0 && l < L && !((held >> l) & 1)) put(i >> 6, (i >> 3) & 7, l, 0.f);
         }
     for (int n0 = 0; n0 < __popc(held); n0 += TAIL_BATCH) {
-        const int l = nth(held, n0 + (c8 >> 1));
+        const int l = nth(held, n0 + nt);
         const int j0 = l < 0 ? 0 : l == 0 ? r_all - 1 : ((r_all - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? r_all : j0 + (1 << (l - 1));
-        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int je = min(j1, row + 1);
-#pragma unroll 4
-        for (int j = j0; j < je; ++j) {
-            const float f = cT[row * AP + j];
-            const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * (c8 & 1));
-            u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
+        float c[1][1][4] = {};
+        const float* const T1[1] = {cT};
+        tile_product3<1, 1, false, false>(c, T1, AP, 16 * mt, cV, TAIL_COLS, 0, 1, j0 & ~15, min(16 * mt + 16, (j1 + 15) & ~15), lane, j0, j1);
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int i = 16 * mt + gq + 8 * hh;
+            *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
         }
-        const float el = cEl[row];
-        *reinterpret_cast<float4*>(sZ + row * XP + 4 * c8) = make_float4(el * u.x, el * u.y, el * u.z, el * u.w);
         __syncthreads();
-        kt_product(nullptr, [&](int x) { return nth(held, n0 + x); });
+        kt_product(nullptr, l);
         __syncthreads();
     }
     if (ta.early && tailed) (void)chain_wait();              // the chunk levels are there
     if (tailed) {
-        float *sX = sm + M::X, *sD = sm + M::D;
+        float *sX = sm + M::X, *sD = sm + M::D, *sY = sm + M::Y;
         const int nslot = __popc((uint32_t)nch);
         for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
             fetch_slots(s0);
@@ -541,50 +489,39 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             for (int i = 0; i < XR; ++i)
                 sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs == 0 ? sSum[(xk + 16 * i) * TAIL_COLS + xv] : 0.f);
             __syncthreads();
-            float4 d = make_float4(0.f, 0.f, 0.f, 0.f), y = d;
-#pragma unroll 2
-            for (int k = 0; k < KD; k += 4) {                // K X and Q X
-                const float4 k4 = *reinterpret_cast<const float4*>(cK + row * KP + k), q4 = *reinterpret_cast<const float4*>(sQ + row * KP + k);
-                const float kx[4] = {k4.x, k4.y, k4.z, k4.w}, qx[4] = {q4.x, q4.y, q4.z, q4.w};
+            const int l = slot_level(s0 + nt);
+            float y[4];
+            {   // K X and Q X
+                float c[2][1][4] = {};
+                const float* const kq[2] = {cK, sQ};
+                tile_product3<2, 1, false, false>(c, kq, KP, 16 * mt, sX, XP, 8 * nt, 1, 0, KD, lane);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float4 x = *reinterpret_cast<const float4*>(sX + (k + u) * XP + 4 * c8);
-                    d.x = fmaf(kx[u], x.x, d.x); d.y = fmaf(kx[u], x.y, d.y); d.z = fmaf(kx[u], x.z, d.z); d.w = fmaf(kx[u], x.w, d.w);
-                    y.x = fmaf(qx[u], x.x, y.x); y.y = fmaf(qx[u], x.y, y.y); y.z = fmaf(qx[u], x.z, y.z); y.w = fmaf(qx[u], x.w, y.w);
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * mt + gq + 8 * hh;
+                    *reinterpret_cast<float2*>(sD + i * XP + 8 * nt + 2 * tq) = make_float2(cEg[i] * c[0][0][2 * hh], cEg[i] * c[0][0][2 * hh + 1]);
+                    y[2 * hh] = cEg[i] * c[1][0][2 * hh];
+                    y[2 * hh + 1] = cEg[i] * c[1][0][2 * hh + 1];
                 }
             }
-            const float eg = cEg[row];
-            *reinterpret_cast<float4*>(sD + row * XP + 4 * c8) = make_float4(eg * d.x, eg * d.y, eg * d.z, eg * d.w);
-            y = make_float4(eg * y.x, eg * y.y, eg * y.z, eg * y.w);
             __syncthreads();
-            float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-            for (int j = 0; j <= row; j += 4) {              // T and R times that; both rows are zero behind the diagonal
-                const float4 t4 = *reinterpret_cast<const float4*>(cT + row * AP + j), r4 = *reinterpret_cast<const float4*>(sP + row * AP + j);
-                const float tx[4] = {t4.x, t4.y, t4.z, t4.w}, rx[4] = {r4.x, r4.y, r4.z, r4.w};
+            {   // T and R times that
+                float c[2][1][4] = {};
+                const float* const tr[2] = {cT, sP};
+                tile_product3<2, 1, false, false>(c, tr, AP, 16 * mt, sD, XP, 8 * nt, 1, 0, 16 * mt + 16, lane);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float4 x = *reinterpret_cast<const float4*>(sD + (j + u) * XP + 4 * c8);
-                    z.x = fmaf(tx[u], x.x, z.x); z.y = fmaf(tx[u], x.y, z.y); z.z = fmaf(tx[u], x.z, z.z); z.w = fmaf(tx[u], x.w, z.w);
-                    y.x = fmaf(-rx[u], x.x, y.x); y.y = fmaf(-rx[u], x.y, y.y); y.z = fmaf(-rx[u], x.z, y.z); y.w = fmaf(-rx[u], x.w, y.w);
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * mt + gq + 8 * hh;
+                    const float w = l >= 0 && i < done ? sLam[i * L + l] : 0.f;
+                    *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
+                    *reinterpret_cast<float2*>(sY + i * XP + 8 * nt + 2 * tq) = make_float2(w * (y[2 * hh] - c[1][0][2 * hh]), w * (y[2 * hh + 1] - c[1][0][2 * hh + 1]));
                 }
             }
-            const float el = cEl[row];
-            *reinterpret_cast<float4*>(sZ + row * XP + 4 * c8) = make_float4(el * z.x, el * z.y, el * z.z, el * z.w);
-            const int l = slot_level(s0 + (c8 >> 1));
-            const float w = l >= 0 && row < done ? sLam[row * L + l] : 0.f;
-            y = make_float4(w * y.x, w * y.y, w * y.z, w * y.w);
-#pragma unroll
-            for (int o = 2; o < 8; o <<= 1) {                // over the slots of the batch
-                y.x += __shfl_xor_sync(0xffffffffu, y.x, o); y.y += __shfl_xor_sync(0xffffffffu, y.y, o);
-                y.z += __shfl_xor_sync(0xffffffffu, y.z, o); y.w += __shfl_xor_sync(0xffffffffu, y.w, o);
-            }
-            if (c8 < 2) {
-                float4* o = reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * c8);
-                *o = make_float4(o->x + y.x, o->y + y.y, o->z + y.z, o->w + y.w);
-            }
             __syncthreads();
-            kt_product(sX, [&](int s) { return slot_level(s0 + s); });
+            {
+                const float* p = sY + row * XP + c8;         // the slots of the batch
+                sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
+            }
+            kt_product(sX, l);
             __syncthreads();
         }
         const int64_t t0 = tok0 + (int64_t)nch * CHUNK;

@@ -62,6 +62,26 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
     assert st.counts.view(-1)[:L].tolist() == want
 
 
+@pytest.mark.parametrize("T", [50, 64, 114])
+def test_a_decay_of_minus_infinity_forgets(T):
+    """Whatever came before a token with g = -inf is gone, and nothing else changes (T <= 64 of it in the tail's own arithmetic)."""
+    H, K, V, L = 2, 32, 32, 9
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    n = T - 20                                               # inside the last chunk or the tail
+    x = [rn(1, T, H, K).bfloat16(), rn(1, T, H, K).bfloat16(), rn(1, T, H, V).bfloat16(), -F.softplus(rn(1, T, H)), F.softplus(rn(1, T, H, L)),
+         torch.sigmoid(rn(1, T, H))]
+    kw = dict(output_final_state=True, use_qk_l2norm_in_kernel=True)
+    x[3][:, n] = -200.0                                      # e^-200 is zero in fp32
+    o1, s1 = lampa_b200.chunk_h_gated_delta_rule(*x, **kw)
+    if T < 64:                                               # (whole chunks go through the chunkwise kernels, which take finite decays)
+        x[3][:, n] = float("-inf")
+    o2, s2 = lampa_b200.chunk_h_gated_delta_rule(*x, **kw)
+    assert torch.isfinite(o2).all() and torch.isfinite(s2.states).all()
+    assert torch.equal(o1, o2) or (o1.float() - o2.float()).norm() <= 1e-2 * o1.float().norm()
+    assert (s1.states - s2.states).norm() <= 1e-6 * s1.states.norm()
+
+
 # one tiled copy per slab up to 32 levels, row by row beyond; more slabs than fit the GPU at once, and few
 @pytest.mark.parametrize("K,V,H,B,L", [(64, 64, 4, 10, 17), (64, 64, 1, 37, 32), (64, 64, 1, 37, 33), (32, 32, 4, 19, 9), (16, 32, 8, 12, 17)])
 def test_steps_of_large_batches(K, V, H, B, L):
