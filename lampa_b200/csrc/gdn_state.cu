@@ -86,12 +86,14 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 //     a level that holds tokens j in J:   S = K^T diag(e^{Gl-G}) T[:, J] V[J]
 //     a slot that enters with X:          X <- e^{Gl} X - K^T diag(e^{Gl-G}) T diag(e^G) K X
 //     o_i = sum_j lambda[i, bit_length(i^j)] R_ij v_j + sum_slots lambda[i, slot] (e^{G_i} q_i X - (R diag(e^G) K X)_i)
-// all of it fp32 multiply-adds (no operand is rounded, G is summed in double so that E is exact to fp32).
-// A CTA takes eight state columns of a (sequence, head); T and R do not depend on the column and are formed
-// by each: 1.5 M multiply-adds per CTA, two halves of the CTA on the last chunk and the tail side by side.
-// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 34 us, of which 20 - 25 run beside the
-// output pass (launch_chained): the call 95 -> 77 us.  What bounds it is the shared-memory pipe (a 16-byte load of a warp
-// returns 512 bytes, four cycles, for 16 multiply-adds of four).
+// all of it at fp32 accuracy: the products on the tensor cores with every operand in three bf16 pieces (split3.cuh), the 16 x 16
+// diagonal blocks of the inverse by substitution, and G summed in double so that E is exact to fp32.
+// A CTA takes eight state columns of a (sequence, head); T and R do not depend on the column and are
+// formed by each, two halves of the CTA on the last chunk and the tail side by side.
+// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
+// pass (launch_chained): the call 95 -> 63 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
+// a few hundred products.  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
+// cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (68 us the call).
 // -------------------------------------------------------------------------------------------------
 constexpr int TAIL_COLS = 8, TAIL_THREADS = 512, TAIL_GRP = 256, TAIL_BATCH = 4;      // states formed at a time
 constexpr int TAIL_AP = CHUNK + 4, TAIL_XP = TAIL_BATCH * TAIL_COLS + 4;              // pitches of 64- and 32-wide rows
@@ -900,15 +902,16 @@ __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs 
     }
 }
 
-// The closed form takes 34 us whatever the tail (8 heads, K = V = 64; 14 us without one), a CTA to an SM; the steps 19 us and 0.4 us per
-// token behind the last chunk, any number of CTAs.  Both begin beside the output pass.  Whole calls of 2,944 tokens and a tail:
-// steps 63 us at 2, 77 at 22 tokens, closed form 86 - 87 from 32 to 62, without a tail 60 instead of 66; past one CTA to an SM
-// it would take a second round.
+// The closed form takes 30 us whatever the tail (8 heads, K = V = 64; 12 us without one), a CTA to an SM; the steps 19 us and 0.4 us
+// per token behind the last chunk (0.25 at head dims up to 32), any number of CTAs.  Both begin beside the output pass.  Whole
+// calls of 2,944 tokens and a tail, steps against closed form: 63 and 63 us at 2 and 18 tokens, 77 and 70 at 22, 84 and 72 at 32;
+// without a tail 66 and 58.  6 heads of 16 and 32: 320 tokens and 30 30 and 35 us, 256 and 44 39 and 39.  Past one CTA to an SM the
+// closed form would take a second round.
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
     const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
     ProfScope prof("hgdn_tail", st);
-    if ((ta.tail == 0 || ta.tail >= 48) && (int64_t)a.nseq * a.H * (VD / TAIL_COLS) <= sm_count()) {
+    if ((ta.tail == 0 || ta.tail >= (KD == 64 ? 16 : 48)) && (int64_t)a.nseq * a.H * (VD / TAIL_COLS) <= sm_count()) {
         using M = TailSmem<KD>;
         const int smem = M::floats(ta.tail > 0, a.L) * 4;
         constexpr int most = M::floats(true, 40) * 4;
