@@ -16,9 +16,10 @@ namespace lampa {
 
 // Chunks per block of the block-parallel scan, as a power of two: chunk levels 0 .. block_log - 1 live inside a block.
 // A block is a serial chain in the compose and output passes, the blocks of a sequence are one in the level pass, so
-// the critical path of a sequence of nch chunks is about nch / blocks * (0.65 + 1.45 us) + blocks * 0.9 us (K = V = 64):
-// 32-chunk blocks left 12 - 24 CTAs on the GPU for a 6000-token event (71 us at 4 heads, 30 us with 8).  The smallest
-// block that keeps a sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
+// the critical path of a sequence of nch chunks is about nch / blocks * (0.35 + 0.5 to 2.5 us) + blocks * 0.3 us (K = V = 64, plain
+// to hierarchical output; 0.65 + 1.45 and 0.9 us when the line was drawn, and on the same side of it): 32-chunk blocks left
+// 12 - 24 CTAs on the GPU for a 6000-token event (71 us at 4 heads, 30 us with 8).  The smallest block that keeps a
+// sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
 // beyond 1024 chunks there are blocks enough to fill the GPU, and smaller ones would only add composites to move.
 // The choice depends on the sequence alone, never on what else a call carries, so that a sequence's result does not.
 constexpr int BLOCK_LOG = 5;                         // largest block: 32 chunks
