@@ -711,7 +711,7 @@ def run_plain(args):
     n_ch = (T + 63) // 64
     rec = 4 * 8192                                        # M, Q~, B^T, O_local: bf16 [64][64] each
     alg = {"gdn_prep_plain": T * (nh * (2 * K + V) * 2 + 2 * nh * 4) + nh * n_ch * rec,
-           "gdn_compose": nh * n_ch * 3 * 8192,
+           "gdn_compose": nh * n_ch * 2 * 8192,             # M and B^T
            "gdn_out_plain": nh * n_ch * rec + T * nh * V * 2}
     kernels = {}
     for n, r in prof.items():

@@ -92,7 +92,7 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // formed by each, two halves of the CTA on the last chunk and the tail side by side.
 // 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
 // pass (launch_chained): the call 95 -> 63 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
-// a few hundred products.  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
+// a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
 // cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (68 us the call).
 // -------------------------------------------------------------------------------------------------
 constexpr int TAIL_COLS = 8, TAIL_THREADS = 512, TAIL_GRP = 256, TAIL_BATCH = 4;      // states formed at a time
