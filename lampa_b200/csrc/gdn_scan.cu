@@ -146,6 +146,13 @@ __device__ __forceinline__ void read_tiles(float (&tmp)[NM][2][4], const uint32_
         }
 }
 
+// o (a row tile's 8 columns) += a level's term: its weights for the rows g and g + 8 of the tile, and Q~ S.  One rounding per level, in
+// the order of the levels, in every kernel that adds them: a sequence's outputs do not depend on which one it meets.
+__device__ __forceinline__ void add_level(float (&o)[4], float l0, float l1, float x, float y, float z, float w) {
+    o[0] = __fmaf_rn(l0, x, o[0]); o[1] = __fmaf_rn(l0, y, o[1]);
+    o[2] = __fmaf_rn(l1, z, o[2]); o[3] = __fmaf_rn(l1, w, o[3]);
+}
+
 // ---- record pipeline: thread 0 issues bulk copies NST-1 steps ahead; everyone waits on the
 // stage's mbarrier.  The __syncthreads at the top of a step frees the stage consumed last step.
 template <int NST>
@@ -811,10 +818,7 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
                         const int mt = m2 + x;
                         const float l0 = lr[mt * 16 + g], l1 = lr[mt * 16 + g + 8];
 #pragma unroll
-                        for (int nt = 0; nt < 2; ++nt) {
-                            O[mt][nt][0] += l0 * tmp[x][nt][0]; O[mt][nt][1] += l0 * tmp[x][nt][1];
-                            O[mt][nt][2] += l1 * tmp[x][nt][2]; O[mt][nt][3] += l1 * tmp[x][nt][3];
-                        }
+                        for (int nt = 0; nt < 2; ++nt) add_level(O[mt][nt], l0, l1, tmp[x][nt][0], tmp[x][nt][1], tmp[x][nt][2], tmp[x][nt][3]);
                     }
                 }
             }
@@ -883,28 +887,29 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
 
 // -------------------------------------------------------------------------------------------------
 // The same for head dims up to 32 with the levels spread over warps: a warp carries two levels of a 16-column slab (level
-// slots p and p + pairs of those the block has: its own first, then the cross-block ones it reads), leaves their sum in shared
-// memory in its own register order, and four warps a chunk behind add the partial sums and O_local and store.
-// A block's chunk is then two levels deep instead of five, with no barrier but the one at its top.  15 warps and 150 KB, a CTA to an
-// SM: taken while the blocks of all heads are at most one to an SM (one event of 9,001 points, 72 CTAs: 25 -> 19 us, two events
+// slots p and p + pairs of those the block has: its own first, then the cross-block ones it reads), leaves their Q~ S in shared
+// memory in its own register order, and eight warps a chunk behind add the terms, in the order of gdn_out_hier_kernel and so with
+// its results to the bit, add O_local and store.
+// A block's chunk is then two levels deep instead of five, with no barrier but the one at its top.  17 warps and 200 KB, a CTA to an
+// SM: taken while the blocks of all heads are at most one to an SM (one event of 9,001 points, 72 CTAs: 25 -> 21 us; two events
 // 509 -> 480 us for the whole model; three events, two rounds: 620 against 622; 64 events: 960 against 1270 us a pass).
 // -------------------------------------------------------------------------------------------------
-constexpr int LV_SUM = 4, LV_MAX_PAIRS = 5, LV_MAX_THREADS = (2 * LV_MAX_PAIRS + 1 + LV_SUM) * 32;
+constexpr int LV_SUM = 8, LV_MAX_PAIRS = 5, LV_MAX_THREADS = (2 * LV_MAX_PAIRS + 1 + LV_SUM) * 32;
 
-template <int KD, int VD>
+template <int KD, int VD, int STAGES>
 struct LevelsSmem {
-    static constexpr int NST = 4;
-    static constexpr int PART = 1024;                        // partial sums [2][pairs][slabs][8][32 lanes][4], behind the barriers
+    static constexpr int NST = STAGES;
+    static constexpr int PART = 1024;                        // Q~ S of the levels [2][slots][slabs][8][32 lanes][4], behind the barriers
     static int stage(int LC) { return (Rec<KD, VD>::bytes(LC) + 127) / 128 * 128; }
-    static int bytes(int LC, int pairs) { return PART + 2 * pairs * 2 * 4096 + NST * stage(LC); }
+    static int bytes(int LC, int pairs) { return PART + 2 * 2 * pairs * 2 * 4096 + NST * stage(LC); }
 };
 
-template <int KD, int VD>
+template <int KD, int VD, int STAGES>
 __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs a, int pairs) {
     if (chain_wait()) return;
     if (a.signal) chain_signal();
     using R = Rec<KD, VD>;
-    using S = LevelsSmem<KD, VD>;
+    using S = LevelsSmem<KD, VD, STAGES>;
     constexpr int NS = VD / 16;
     static_assert(NS == 2, "two slabs");
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -922,11 +927,11 @@ __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     float4* part = reinterpret_cast<float4*>(smem + S::PART);
-    const int buf_stride = pairs * NS * 256;                    // float4 of one chunk's partial sums
+    const int buf_stride = 2 * pairs * NS * 256;                // float4 of one chunk's terms
 
     Feed<S::NST, 0, 1, 2> feed;
     feed.bar = reinterpret_cast<uint64_t*>(smem);
-    feed.stage = smem + S::PART + 2 * pairs * NS * 4096;
+    feed.stage = smem + S::PART + 4 * pairs * NS * 4096;
     feed.step_bytes = (R::bytes(a.LC) + 127) / 128 * 128;
     feed.src = a.rec + ((size_t)c0 * H + h) * a.rec_bytes;
     feed.src_stride = (size_t)H * a.rec_bytes;
@@ -949,50 +954,57 @@ __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs 
         for (int i = 0; i < k; ++i) m &= m - 1;
         return __ffs(m) - 1;
     };
-    // slots read in chunk n, as a mask of pairs that leave a partial sum
-    auto read_slot = [&](int s, int n) { return s < nslots && (s >= bl || ((n >> s) & 1)); };
+    // slots read in chunk n (a missing lambda row is only reachable when the level check already failed)
+    auto read_slot = [&](int s, int lam_row, int n) { return s < nslots && lam_row < a.LC && (s >= bl || ((n >> s) & 1)); };
     if (warp > producer) {
-        // ---- sums: warp = (slab, two of the four row tiles), a chunk behind ----
-        const int w = warp - producer - 1, slab = w & 1, mt0 = (w >> 1) * 2, row0 = 16 * slab;
+        // ---- sums: warp = (slab, row tile), a chunk behind ----
+        const int w = warp - producer - 1, slab = w & 1, mt = w >> 1, row0 = 16 * slab;
         const unsigned char* st = nullptr;
         for (int i = 0; i <= nsteps; ++i) {
-            const unsigned char* now = feed.step(i);          // chunk i - 1 is in its partial sums
+            const unsigned char* now = feed.step(i);          // the terms of chunk i - 1 are there
             if (i > 0) {
                 const int n = b * bc + i - 1;
-                float o[2][2][4];
+                const float4* p0 = part + ((i - 1) & 1) * buf_stride + slab * 256 + mt * 64 + lane;
+                const float* lam = reinterpret_cast<const float*>(st + R::LAM_OFF) + mt * 16 + g;
+                auto add_slot = [&](float (&x)[2][4], int s, int row) {
+                    const float l0 = lam[row * CHUNK], l1 = lam[row * CHUNK + 8];
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+                    for (int nt = 0; nt < 2; ++nt) {
+                        const float4 f = p0[s * NS * 256 + nt * 32];
+                        add_level(x[nt], l0, l1, f.x, f.y, f.z, f.w);
+                    }
+                };
+                float o[2][4] = {};
+                for (int s = 0; s < bl; ++s)
+                    if (read_slot(s, s, n)) add_slot(o, s, s);
+                // the cross-block levels by the groups of gdn_out_hier_kernel
+                uint32_t m = cross;
+                for (int s = bl; m != 0;) {
+                    const int grp = (__ffs(m) - 1) / NLW;
+                    float oc[2][4] = {};
+                    for (; m != 0 && (__ffs(m) - 1) / NLW == grp; m &= m - 1, ++s) {
+                        const int row = bl + __ffs(m) - 1;
+                        if (read_slot(s, row, n)) add_slot(oc, s, row);
+                    }
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) { o[x][nt][0] = o[x][nt][1] = o[x][nt][2] = o[x][nt][3] = 0.f; }
-                const float4* p0 = part + ((i - 1) & 1) * buf_stride + slab * 256 + lane;
-                for (int p = 0; p < pairs; ++p) {
-                    if (!read_slot(p, n) && !read_slot(p + pairs, n)) continue;
-#pragma unroll
-                    for (int x = 0; x < 2; ++x)
-#pragma unroll
-                        for (int nt = 0; nt < 2; ++nt) {
-                            const float4 f = p0[p * NS * 256 + ((mt0 + x) * 2 + nt) * 32];
-                            o[x][nt][0] += f.x; o[x][nt][1] += f.y; o[x][nt][2] += f.z; o[x][nt][3] += f.w;
-                        }
+                    for (int e = 0; e < 8; ++e) o[e >> 2][e & 3] += oc[e >> 2][e & 3];
                 }
                 const __nv_bfloat16* sOl = reinterpret_cast<const __nv_bfloat16*>(st + R::OL_OFF);
                 const int64_t t0 = tok0 + (int64_t)(i - 1) * CHUNK;
                 auto emit = [&](auto scat) {
 #pragma unroll
-                    for (int x = 0; x < 2; ++x)
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int r = mt * 16 + g + hh * 8;
+                        const int64_t orow = t0 + r < tok_end ? out_row<decltype(scat)::value>(a, t0 + r) : -1;
+                        if (orow >= 0) {
 #pragma unroll
-                        for (int hh = 0; hh < 2; ++hh) {
-                            const int r = (mt0 + x) * 16 + g + hh * 8;
-                            const int64_t orow = t0 + r < tok_end ? out_row<decltype(scat)::value>(a, t0 + r) : -1;
-                            if (orow >= 0) {
-#pragma unroll
-                                for (int nt = 0; nt < 2; ++nt) {
-                                    const int col = row0 + nt * 8 + 2 * t;
-                                    const float2 ol = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sOl + R::TV::off(r, col)));
-                                    store_out2(a.o, a.qkv_dt, ((size_t)orow * H + h) * VD + col, ol.x + o[x][nt][2 * hh], ol.y + o[x][nt][2 * hh + 1]);
-                                }
+                            for (int nt = 0; nt < 2; ++nt) {
+                                const int col = row0 + nt * 8 + 2 * t;
+                                const float2 ol = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(sOl + R::TV::off(r, col)));
+                                store_out2(a.o, a.qkv_dt, ((size_t)orow * H + h) * VD + col, ol.x + o[nt][2 * hh], ol.y + o[nt][2 * hh + 1]);
                             }
                         }
+                    }
                 };
                 if (a.out_perm_rows > 0) emit(ScatterOn{}); else emit(ScatterOff{});
             }
@@ -1020,7 +1032,6 @@ __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs 
         const __nv_bfloat16* sM = reinterpret_cast<const __nv_bfloat16*>(st + R::M_OFF);
         const __nv_bfloat16* sBt = reinterpret_cast<const __nv_bfloat16*>(st + R::BT_OFF);
         const __nv_bfloat16* sQt = reinterpret_cast<const __nv_bfloat16*>(st + R::QT_OFF);
-        const float* sLam = reinterpret_cast<const float*>(st + R::LAM_OFF);
         const int n = b * bc + i;
         const bool more = i + 1 < nsteps;
         uint32_t sp[2][KD / 16][4];
@@ -1040,38 +1051,17 @@ __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs 
                 state_times_mt<KD>(C[x], sp[x], sM, lane);
             }
         }
-        float O[4][2][4];
-        bool any = false;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const int s = pair + x * pairs;
-            if (!read_slot(s, n)) continue;
+            if (!read_slot(s, lam_row[x], n)) continue;
             float tmp[4][2][4];
             read_tiles<KD, 4>(tmp, sp[x], sQt, 0, lane);
-            const bool has = lam_row[x] < a.LC;               // a missing row is only reachable when the level check already failed
-            const float* lr = sLam + (has ? lam_row[x] : 0) * CHUNK;
-#pragma unroll
-            for (int mt = 0; mt < 4; ++mt) {
-                const float l0 = has ? lr[mt * 16 + g] : 0.f, l1 = has ? lr[mt * 16 + g + 8] : 0.f;
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    if (any) {
-                        O[mt][nt][0] += l0 * tmp[mt][nt][0]; O[mt][nt][1] += l0 * tmp[mt][nt][1];
-                        O[mt][nt][2] += l1 * tmp[mt][nt][2]; O[mt][nt][3] += l1 * tmp[mt][nt][3];
-                    } else {
-                        O[mt][nt][0] = l0 * tmp[mt][nt][0]; O[mt][nt][1] = l0 * tmp[mt][nt][1];
-                        O[mt][nt][2] = l1 * tmp[mt][nt][2]; O[mt][nt][3] = l1 * tmp[mt][nt][3];
-                    }
-                }
-            }
-            any = true;
-        }
-        if (any) {
-            float4* d = part + (i & 1) * buf_stride + (pair * NS + slab) * 256 + lane;
+            float4* d = part + (i & 1) * buf_stride + (s * NS + slab) * 256 + lane;
 #pragma unroll
             for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) d[(mt * 2 + nt) * 32] = make_float4(O[mt][nt][0], O[mt][nt][1], O[mt][nt][2], O[mt][nt][3]);
+                for (int nt = 0; nt < 2; ++nt) d[(mt * 2 + nt) * 32] = make_float4(tmp[mt][nt][0], tmp[mt][nt][1], tmp[mt][nt][2], tmp[mt][nt][3]);
         }
     }
     feed.step(nsteps);
@@ -1142,12 +1132,12 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
     return LAMPA_OK;
 }
 
-template <int KD, int VD>
+template <int KD, int VD, int STAGES>
 static int launch_out_levels(const GdnArgs& a, int pairs, cudaStream_t st) {
-    const int smem = LevelsSmem<KD, VD>::bytes(a.LC, pairs);
-    LAMPA_TRY(set_smem(gdn_out_levels_kernel<KD, VD>, smem));
+    const int smem = LevelsSmem<KD, VD, STAGES>::bytes(a.LC, pairs);
+    LAMPA_TRY(set_smem(gdn_out_levels_kernel<KD, VD, STAGES>, smem));
     ProfScope prof("gdn_out_hier", st);
-    launch_chained(gdn_out_levels_kernel<KD, VD>, dim3(a.nb_max, a.H), (2 * pairs + 1 + LV_SUM) * 32, smem, st, a, pairs);
+    launch_chained(gdn_out_levels_kernel<KD, VD, STAGES>, dim3(a.nb_max, a.H), (2 * pairs + 1 + LV_SUM) * 32, smem, st, a, pairs);
     LAMPA_LAUNCHED();
     return LAMPA_OK;
 }
@@ -1163,7 +1153,10 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
     if (KD == 64 && VD == 64 && a.nhigh_max <= 5 && a.use_umma) return launch_out_hier_umma(a, st);
     if constexpr (KD <= 32) {
         const int pairs = ((a.nlev_max > MIN_BLOCK_LOG ? a.nlev_max : MIN_BLOCK_LOG) + 1) / 2;      // a block has at most a slot per level of its sequence
-        if ((int64_t)a.nb_max * a.H <= sm_count() && pairs <= LV_MAX_PAIRS && LevelsSmem<KD, VD>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD>(a, pairs, st);
+        if ((int64_t)a.nb_max * a.H <= sm_count() && pairs <= LV_MAX_PAIRS) {
+            if (LevelsSmem<KD, VD, 4>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD, 4>(a, pairs, st);
+            if (LevelsSmem<KD, VD, 3>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD, 3>(a, pairs, st);
+        }
     }
     if (ng == 1) return launch_out_hier<KD, VD, 1>(a, st);
     if (ng == 2) return launch_out_hier<KD, VD, 2>(a, st);
