@@ -21,12 +21,15 @@ namespace lampa {
 // 12 - 24 CTAs on the GPU for a 6000-token event (71 us at 4 heads, 30 us with 8).  The smallest block that keeps a
 // sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
 // beyond 1024 chunks there are blocks enough to fill the GPU, and smaller ones would only add composites to move.
-// The choice depends on the sequence alone, never on what else a call carries, so that a sequence's result does not.
+// The choice depends on the sequence alone, never on what else a call carries, and so does every other one that changes the order
+// of a sum (which output pass a sequence meets: launch_scan_hier): a sequence's results are the same bits alone, in a batch, packed
+// and in a slice of its heads.
 constexpr int BLOCK_LOG = 5;                         // largest block: 32 chunks
 constexpr int MIN_BLOCK_LOG = 3;                     // smallest
 __host__ __device__ __forceinline__ int block_log(int nch) { return nch <= 256 ? 3 : (nch <= 512 ? 4 : BLOCK_LOG); }
 __host__ __device__ __forceinline__ int blocks_of(int nch) { const int bl = block_log(nch); return (nch + (1 << bl) - 1) >> bl; }
 constexpr int NLW = 5;               // level states carried per warp in the hierarchical output pass
+constexpr int UMMA_LEVELS = BLOCK_LOG + 5;   // chunk levels that the tcgen05 output pass carries: 1024 chunks
 constexpr int MAX_GROUPS = 3;        // 1 group of in-block levels + up to 2 groups of cross-block levels
 
 // Layout of a K-wide bf16 tile ([rows][KD]) inside a record.  For KD = 64 rows are dense 128-byte
@@ -96,6 +99,7 @@ struct GdnArgs {
     int32_t* status;
     int use_umma;                         // tcgen05 kernels where they exist (K = V = 64)
     int poll_budget;                      // polls before a device wait gives up (MBAR_POLLS unless a test lowers it)
+    int long_only, short_only;            // output pass: only sequences of more (of at most) UMMA_LEVELS chunk levels
     int signal;                           // a prefill's output pass and chunk levels let the next kernel in (chain_signal)
     long long* ticks; int ticks_ctas;     // stage clocks for tuning: [ticks_ctas][16] or NULL (lampa_debug_set_tick_buffer)
 };

@@ -105,6 +105,7 @@ void fill_args(const lampa_gdn_desc* d, bool hier, const Layout& l, char* base, 
     static const int no_umma = [] { const char* e = getenv("LAMPA_B200_NO_UMMA"); return (e && e[0] == '1') ? 1 : 0; }();
     a.use_umma = (no_umma || g_force_mma_sync) ? 0 : 1;
     a.poll_budget = poll_budget();
+    a.long_only = a.short_only = 0;
     a.signal = 0;
     a.ticks = g_ticks;
     a.ticks_ctas = g_ticks_ctas;

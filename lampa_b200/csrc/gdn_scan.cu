@@ -721,6 +721,7 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
     if (!locate_block(a, gb, sq, b)) return;
     const int nch = sq.nch;
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
+    if (a.long_only && nlev <= UMMA_LEVELS) return;
     const int bl = block_log(nch), bc = 1 << bl;
     const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
     const int c0 = sq.c0 + b * bc;
@@ -1150,7 +1151,17 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
         LAMPA_TRY((launch_compose<KD, VD>(a, st)));
         LAMPA_TRY((launch_level<KD, VD, true>(a, a.nhigh_max, st)));
     }
-    if (KD == 64 && VD == 64 && a.nhigh_max <= 5 && a.use_umma) return launch_out_hier_umma(a, st);
+    // The two passes add in different orders, so a sequence's own length decides.  A packed call knows it on the device only: where it
+    // may hold sequences of more levels than the tcgen05 pass carries, both run, each on its sequences.
+    GdnArgs rest = a;
+    if (KD == 64 && VD == 64 && a.use_umma) {
+        if (a.nlev_max <= UMMA_LEVELS) return launch_out_hier_umma(a, st);
+        if (a.fixed_T == 0) {
+            GdnArgs shorts = a;
+            shorts.short_only = rest.long_only = 1;
+            LAMPA_TRY(launch_out_hier_umma(shorts, st));
+        }
+    }
     if constexpr (KD <= 32) {
         const int pairs = ((a.nlev_max > MIN_BLOCK_LOG ? a.nlev_max : MIN_BLOCK_LOG) + 1) / 2;      // a block has at most a slot per level of its sequence
         if ((int64_t)a.nb_max * a.H <= sm_count() && pairs <= LV_MAX_PAIRS) {
@@ -1158,9 +1169,9 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
             if (LevelsSmem<KD, VD, 3>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD, 3>(a, pairs, st);
         }
     }
-    if (ng == 1) return launch_out_hier<KD, VD, 1>(a, st);
-    if (ng == 2) return launch_out_hier<KD, VD, 2>(a, st);
-    return launch_out_hier<KD, VD, 3>(a, st);
+    if (ng == 1) return launch_out_hier<KD, VD, 1>(rest, st);
+    if (ng == 2) return launch_out_hier<KD, VD, 2>(rest, st);
+    return launch_out_hier<KD, VD, 3>(rest, st);
 }
 
 template <int KD, int VD>

@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
     if (!locate_block(a, gb, sq, b)) return;
     const int nch = sq.nch;
     const int nlev = nch > 1 ? ceil_log2_int(nch) : 0;
+    if (a.short_only && nlev > UMMA_LEVELS) return;
     const int bl = block_log(nch), bc = 1 << bl;
     const int nhigh = min(max(0, nlev - bl), a.nhigh_max);     // more only when the level check has already failed
     const int c0 = sq.c0 + b * bc;
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
 
 int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st) {
     const int smem = SM_STAGE + UNST * ustage_bytes(a.LC);
-    if (smem > 227 * 1024 || a.nhigh_max > UNP) return LAMPA_ERR_UNSUPPORTED;
+    if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
     if (cudaFuncSetAttribute(gdn_out_hier_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return LAMPA_ERR_CUDA;
     UnitOrder uo;

@@ -33,7 +33,7 @@ def _heads(x, a, b):
 @pytest.mark.parametrize("K,V", [(64, 64), (32, 32), (16, 32)])
 @pytest.mark.parametrize("T,H,B", [(128, 4, 40), (9001, 8, 4), (64 * 300 - 3, 6, 3), (64 * 520, 8, 2)])
 def test_alone_batched_packed_and_by_head(K, V, T, H, B):
-    L = 17
+    L = 18                                            # packed: up to 2048 chunks, twice what the 64 x 64 pass on tcgen05 carries
     rows = [_draw(10 * T + i, T, H, K, V, L) for i in range(B)]
     batch = [torch.cat(t) for t in zip(*rows)]
     cu = torch.arange(B + 1, dtype=torch.int64, device="cuda") * T
@@ -48,6 +48,18 @@ def test_alone_batched_packed_and_by_head(K, V, T, H, B):
             assert torch.equal(op(rows[i], torch.tensor([0, T], device="cuda"))[0], alone)
         for a, b in ((0, 1), (1, H)):
             assert torch.equal(op(_heads(rows[0], a, b))[0], together[:1, :, a:b])
+    lampa_b200.check_status(torch.device("cuda:0"))
+
+
+def test_short_and_long_sequences_packed():
+    """64 x 64 heads: a sequence of more than 65,536 tokens beside shorter ones, an empty one among them."""
+    H, L, lens = 2, 18, [700, 65600, 0, 33280, 65536, 1]
+    rows = [_draw(7 + i, n, H, 64, 64, L) for i, n in enumerate(lens)]
+    cu = torch.tensor([0] + lens).cumsum(0)
+    together, _ = _hier([torch.cat(t, dim=1) for t in zip(*rows)], cu.cuda())
+    for i, n in enumerate(lens):
+        if n > 0:
+            assert torch.equal(_hier(rows[i])[0], together[:, cu[i] : cu[i + 1]]), n
     lampa_b200.check_status(torch.device("cuda:0"))
 
 
