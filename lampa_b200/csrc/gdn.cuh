@@ -22,8 +22,8 @@ namespace lampa {
 // sequence at 32 blocks or fewer is taken, i.e. 8 chunks up to 256 chunks, 16 up to 512, then 32:
 // beyond 1024 chunks there are blocks enough to fill the GPU, and smaller ones would only add composites to move.
 // The choice depends on the sequence alone, never on what else a call carries, and so does every other one that changes the order
-// of a sum (which output pass a sequence meets: launch_scan_hier): a sequence's results are the same bits alone, in a batch, packed
-// and in a slice of its heads.
+// of a sum (which output pass a sequence meets, launch_scan_hier; which form takes a prompt's tail, launch_hgdn_tail): a sequence's
+// results are the same bits alone, in a batch, packed and in a slice of its heads.
 constexpr int BLOCK_LOG = 5;                         // largest block: 32 chunks
 constexpr int MIN_BLOCK_LOG = 3;                     // smallest
 __host__ __device__ __forceinline__ int block_log(int nch) { return nch <= 256 ? 3 : (nch <= 512 ? 4 : BLOCK_LOG); }
@@ -214,6 +214,7 @@ struct TailArgs {
     int one_count;
     int32_t* arrivals;                    // set to zero, or NULL: the arrival counter of the decode steps to come
     int early;                            // this call's kernels in front signal early (GdnArgs::signal)
+    int slabs = 1;                        // eight state columns each: what a CTA of the closed form works through
 };
 template <int KD, int VD> int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st);
 

@@ -88,10 +88,11 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 //     o_i = sum_j lambda[i, bit_length(i^j)] R_ij v_j + sum_slots lambda[i, slot] (e^{G_i} q_i X - (R diag(e^G) K X)_i)
 // all of it at fp32 accuracy: the products on the tensor cores with every operand in three bf16 pieces (split3.cuh), the 16 x 16
 // diagonal blocks of the inverse by substitution, and G summed in double so that E is exact to fp32.
-// A CTA takes eight state columns of a (sequence, head); T and R do not depend on the column and are
-// formed by each, two halves of the CTA on the last chunk and the tail side by side.
+// A CTA takes eight state columns of a (sequence, head) after the other, as many as leave one CTA to an SM (one set of eight while
+// there are SMs for all); T and R do not depend on the column and are formed once by each CTA, two halves of it on the last
+// chunk and the tail side by side.  A column's arithmetic is the same whichever CTA has it.
 // 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
-// pass (launch_chained): the call 95 -> 63 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
+// pass (launch_chained): the call 95 -> 65 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
 // cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (68 us the call).
 // -------------------------------------------------------------------------------------------------
@@ -105,17 +106,17 @@ struct TailSmem {                                            // offsets in float
     static constexpr int CH = CHUNK * KP + CHUNK * TAIL_AP + CHUNK * TAIL_COLS + SCAL;       // k, A -> T, v, scalars of one chunk
     static constexpr int K_ = 0, A_ = CHUNK * KP, V_ = A_ + CHUNK * TAIL_AP, S_ = V_ + CHUNK * TAIL_COLS;
     static constexpr int Z = CH;                             // [64][XP]
-    static constexpr int SUM = Z + CHUNK * TAIL_XP;          // [KD][8] all tokens of the last chunk
-    static constexpr int B = SUM + KD * TAIL_COLS;           // (tail only) the tail's chunk
+    static constexpr int B = Z + CHUNK * TAIL_XP;            // (tail only) the tail's chunk
     static constexpr int Q = B + CH;                         // [64][KP]
     static constexpr int P = Q + CHUNK * KP;                 // [64][AP], then R
     static constexpr int OUT = P + CHUNK * TAIL_AP;          // [64][8]
-    static constexpr int LAM = OUT + CHUNK * TAIL_COLS;      // [64][L], then the slab [KD][8][L]
+    static constexpr int LAM = OUT + CHUNK * TAIL_COLS;      // [64][L], then the slab [KD][8][L], then [slabs][KD][8] all tokens of the last chunk
     // slots, K X, and what a batch of slots adds to the outputs, over the last chunk, which is done with by then
     static constexpr int X = 0, D = KD * TAIL_XP, Y = D + CHUNK * TAIL_XP;
     static_assert(Y + CHUNK * TAIL_XP <= CH, "slots must fit");
     static_assert(CH % 4 == 0 && Q % 4 == 0 && LAM % 4 == 0, "16-byte rows");
-    __host__ __device__ static constexpr int floats(bool tail, int L) { return tail ? LAM + (CHUNK * L + 3) / 4 * 4 + KD * TAIL_COLS * L : B; }
+    __host__ __device__ static constexpr int sum(int L) { return LAM + (CHUNK * L + 3) / 4 * 4 + KD * TAIL_COLS * L; }
+    __host__ __device__ static constexpr int floats(bool tail, int L, int slabs) { return tail ? sum(L) + slabs * KD * TAIL_COLS : B; }
 };
 
 __device__ __forceinline__ void tail_meet(int grp) { asm volatile("bar.sync %0, %1;\n" :: "r"(grp + 1), "n"(TAIL_GRP) : "memory"); }
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     extern __shared__ __align__(16) float sm[];
     const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
     const int tid = threadIdx.x, lane = tid & 31, gq = lane >> 2, tq = lane & 3, grp = tid / TAIL_GRP, t = tid % TAIL_GRP;
-    const int v0 = blockIdx.z * TAIL_COLS;
+    int v0 = blockIdx.z * ta.slabs * TAIL_COLS;              // the first of the state columns that are being worked on
     int nch = ta.n0;
     int64_t tok0 = (int64_t)seq * a.fixed_stride, tok_end = 0;
     if (ta.n0 < 0) {
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     double* sG = reinterpret_cast<double*>(ch + M::S_);
     float *sEg = ch + M::S_ + 2 * CHUNK, *sEl = sEg + CHUNK, *sBeta = sEl + CHUNK;
     float *sQ = sm + M::Q, *sP = sm + M::P, *sOut = sm + M::OUT, *sLam = sm + M::LAM, *slab = sLam + (CHUNK * L + 3) / 4 * 4;
-    float *sZ = sm + M::Z, *sSum = sm + M::SUM;
+    float *sZ = sm + M::Z, *sSum = sm + M::sum(L);
 
     // chunk levels the tail continues from: slot (tid / 8) % 4 of a batch, column tid % 8, rows tid / 32 + 16 i
     auto slot_level = [&](int s) {                           // level of slot s (bit order), or -1
@@ -230,6 +231,13 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             if (l < 0) continue;
             if (l != lvl0) xr[i] = __ldcg(p + l);
             else for (int q = ELL0; q < l; ++q) xr[i] += __ldcg(p + q);
+        }
+    };
+    // v of `len` tokens from t0 on, columns c0 .. c0 + 7, rows up to 64 null tokens; n threads
+    auto stage_values = [&](float* d, int i, int n, int64_t t0, int len, int c0) {
+        for (; i < CHUNK * TAIL_COLS; i += n) {
+            const int r = i / TAIL_COLS;
+            d[i] = raw_float(load_raw(a.v, ((size_t)(t0 + r) * H + h) * VD + c0 + i % TAIL_COLS, a.qkv_dt, r < len), a.qkv_dt);
         }
     };
     const bool mine = grp == 0 ? nch > 0 : tailed;
@@ -361,8 +369,13 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         }
         tail_meet(grp);
         tail_inverse(sA, sBeta, t, grp);
-        if (!tail && tailed) {                               // all tokens of the last chunk as one state: they join a slot
+        for (int s = 0; s < ta.slabs && !tail && tailed; ++s) {      // all tokens of the last chunk as one state: they join a slot
             const int w = t >> 5;
+            if (s > 0) {
+                tail_meet(grp);
+                stage_values(sV, t, TAIL_GRP, t0, len, v0 + s * TAIL_COLS);
+                tail_meet(grp);
+            }
             if (w < 4) {
                 float c[1][1][4] = {};
                 const float* const T1[1] = {sA};
@@ -380,7 +393,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 tile_product3<1, 1, true, false>(c, k1, KP, 16 * w, sZ, XP, 0, 1, 0, CHUNK, lane);
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh)
-                    *reinterpret_cast<float2*>(sSum + (16 * w + gq + 8 * hh) * TAIL_COLS + 2 * tq) = make_float2(c[0][0][2 * hh], c[0][0][2 * hh + 1]);
+                    *reinterpret_cast<float2*>(sSum + (s * KD + 16 * w + gq + 8 * hh) * TAIL_COLS + 2 * tq) = make_float2(c[0][0][2 * hh], c[0][0][2 * hh + 1]);
             }
         }
     }
@@ -390,6 +403,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const float* cs = sm + (tailed ? M::B : 0);
     const float *cK = cs + M::K_, *cT = cs + M::A_, *cV = cs + M::V_, *cEg = cs + M::S_ + 2 * CHUNK, *cEl = cEg + CHUNK;
     const int r_all = tailed ? done : (nch > 0 ? CHUNK : 0);
+    const int len_all = tailed ? done : nch == 0 ? 0 : ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - tok0 - (int64_t)(nch - 1) * CHUNK);
     const int row = tid >> 3, c8 = tid & 7;                  // row and column of what goes element by element
     const int warp = tid >> 5, mt = warp & 3, nt = warp >> 2;       // products: 16 rows, and eight columns: state nt of a batch
 
@@ -413,7 +427,6 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     };
 
     if (tailed) {
-        for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
         // R = P T, both lower triangular: warp = (16 rows, column tiles nt and nt + 4)
         float c[2][1][1][4] = {};
         const float* const P1[1] = {sP};
@@ -428,120 +441,132 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             for (int hh = 0; hh < 2; ++hh)
                 *reinterpret_cast<float2*>(sP + (16 * mt + gq + 8 * hh) * AP + 8 * (nt + 4 * x) + 2 * tq) = make_float2(c[x][0][0][2 * hh], c[x][0][0][2 * hh + 1]);
         __syncthreads();
-        // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
-        // row i reads are the 2^(l-1) below the highest set bit they differ in
-        {
-            const int hf = (tid >> 2) & 1, jg = tid & 3;
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < done) {
-                for (int l = 0; l < ELL0 && l < L; ++l) {
-                    if (l > 0 && !((row >> (l - 1)) & 1)) continue;
-                    const int j0 = l == 0 ? row : (row >> l) << l, j1 = l == 0 ? row + 1 : j0 + (1 << (l - 1));
-                    float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int j = j0 + jg; j < j1; j += 4) {
-                        const float f = sP[row * AP + j];
-                        const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * hf);
-                        u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
-                    }
-                    const float w = sLam[row * L + l];
-                    o.x = fmaf(w, u.x, o.x); o.y = fmaf(w, u.y, o.y); o.z = fmaf(w, u.z, o.z); o.w = fmaf(w, u.w, o.w);
-                }
-            }
-#pragma unroll
-            for (int d = 1; d < 4; d <<= 1) {
-                o.x += __shfl_xor_sync(0xffffffffu, o.x, d); o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
-                o.z += __shfl_xor_sync(0xffffffffu, o.z, d); o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
-            }
-            if (jg == 0) *reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * hf) = o;
-        }
     }
-    // token levels that hold tokens, four at a time: bit l of `held`
-    const uint32_t held = r_all > 0 ? (uint32_t)(r_all - 1) << 1 | 1u : 0u;
-    auto nth = [](uint32_t m, int n) {                       // its n-th level, or -1
-        for (int i = 0; i < n; ++i) m &= m - 1;
-        return m ? __ffs(m) - 1 : -1;
-    };
-    if (!tailed)                                             // the slab is zero where no level is
-        for (int i = tid; i < KD * TAIL_COLS * 8; i += TAIL_THREADS) {
-            const int l = i & 7;
-            if (l < ELL0 && l < L && !((held >> l) & 1)) put(i >> 6, (i >> 3) & 7, l, 0.f);
+    for (int s = 0; s < ta.slabs; ++s) {                     // eight state columns at a time
+        if (s > 0) {
+            __syncthreads();                                 // the slab before is done with
+            v0 += TAIL_COLS;
+            st += TAIL_COLS * L;
+            stage_values(const_cast<float*>(cV), tid, TAIL_THREADS, tok0 + (int64_t)(tailed ? nch : nch - 1) * CHUNK, len_all, v0);
+            __syncthreads();
         }
-    for (int n0 = 0; n0 < __popc(held); n0 += TAIL_BATCH) {
-        const int l = nth(held, n0 + nt);
-        const int j0 = l < 0 ? 0 : l == 0 ? r_all - 1 : ((r_all - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? r_all : j0 + (1 << (l - 1));
-        float c[1][1][4] = {};
-        const float* const T1[1] = {cT};
-        tile_product3<1, 1, false, false>(c, T1, AP, 16 * mt, cV, TAIL_COLS, 0, 1, j0 & ~15, min(16 * mt + 16, (j1 + 15) & ~15), lane, j0, j1);
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int i = 16 * mt + gq + 8 * hh;
-            *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
-        }
-        __syncthreads();
-        kt_product(nullptr, l);
-        __syncthreads();
-    }
-    if (ta.early && tailed) (void)chain_wait();              // the chunk levels are there
-    if (tailed) {
-        float *sX = sm + M::X, *sD = sm + M::D, *sY = sm + M::Y;
-        const int nslot = __popc((uint32_t)nch);
-        for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
-            fetch_slots(s0);
-#pragma unroll
-            for (int i = 0; i < XR; ++i)
-                sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs == 0 ? sSum[(xk + 16 * i) * TAIL_COLS + xv] : 0.f);
-            __syncthreads();
-            const int l = slot_level(s0 + nt);
-            float y[4];
-            {   // K X and Q X
-                float c[2][1][4] = {};
-                const float* const kq[2] = {cK, sQ};
-                tile_product3<2, 1, false, false>(c, kq, KP, 16 * mt, sX, XP, 8 * nt, 1, 0, KD, lane);
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = 16 * mt + gq + 8 * hh;
-                    *reinterpret_cast<float2*>(sD + i * XP + 8 * nt + 2 * tq) = make_float2(cEg[i] * c[0][0][2 * hh], cEg[i] * c[0][0][2 * hh + 1]);
-                    y[2 * hh] = cEg[i] * c[1][0][2 * hh];
-                    y[2 * hh + 1] = cEg[i] * c[1][0][2 * hh + 1];
-                }
-            }
-            __syncthreads();
-            {   // T and R times that
-                float c[2][1][4] = {};
-                const float* const tr[2] = {cT, sP};
-                tile_product3<2, 1, false, false>(c, tr, AP, 16 * mt, sD, XP, 8 * nt, 1, 0, 16 * mt + 16, lane);
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int i = 16 * mt + gq + 8 * hh;
-                    const float w = l >= 0 && i < done ? sLam[i * L + l] : 0.f;
-                    *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
-                    *reinterpret_cast<float2*>(sY + i * XP + 8 * nt + 2 * tq) = make_float2(w * (y[2 * hh] - c[1][0][2 * hh]), w * (y[2 * hh + 1] - c[1][0][2 * hh + 1]));
-                }
-            }
-            __syncthreads();
+        if (tailed) {
+            for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
+            // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
+            // row i reads are the 2^(l-1) below the highest set bit they differ in
             {
-                const float* p = sY + row * XP + c8;         // the slots of the batch
-                sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
+                const int hf = (tid >> 2) & 1, jg = tid & 3;
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (row < done) {
+                    for (int l = 0; l < ELL0 && l < L; ++l) {
+                        if (l > 0 && !((row >> (l - 1)) & 1)) continue;
+                        const int j0 = l == 0 ? row : (row >> l) << l, j1 = l == 0 ? row + 1 : j0 + (1 << (l - 1));
+                        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int j = j0 + jg; j < j1; j += 4) {
+                            const float f = sP[row * AP + j];
+                            const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * hf);
+                            u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
+                        }
+                        const float w = sLam[row * L + l];
+                        o.x = fmaf(w, u.x, o.x); o.y = fmaf(w, u.y, o.y); o.z = fmaf(w, u.z, o.z); o.w = fmaf(w, u.w, o.w);
+                    }
+                }
+#pragma unroll
+                for (int d = 1; d < 4; d <<= 1) {
+                    o.x += __shfl_xor_sync(0xffffffffu, o.x, d); o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
+                    o.z += __shfl_xor_sync(0xffffffffu, o.z, d); o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
+                }
+                if (jg == 0) *reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * hf) = o;
             }
-            kt_product(sX, l);
+        }
+        // token levels that hold tokens, four at a time: bit l of `held`
+        const uint32_t held = r_all > 0 ? (uint32_t)(r_all - 1) << 1 | 1u : 0u;
+        auto nth = [](uint32_t m, int n) {                       // its n-th level, or -1
+            for (int i = 0; i < n; ++i) m &= m - 1;
+            return m ? __ffs(m) - 1 : -1;
+        };
+        if (!tailed)                                             // the slab is zero where no level is
+            for (int i = tid; i < KD * TAIL_COLS * 8; i += TAIL_THREADS) {
+                const int l = i & 7;
+                if (l < ELL0 && l < L && !((held >> l) & 1)) put(i >> 6, (i >> 3) & 7, l, 0.f);
+            }
+        for (int n0 = 0; n0 < __popc(held); n0 += TAIL_BATCH) {
+            const int l = nth(held, n0 + nt);
+            const int j0 = l < 0 ? 0 : l == 0 ? r_all - 1 : ((r_all - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? r_all : j0 + (1 << (l - 1));
+            float c[1][1][4] = {};
+            const float* const T1[1] = {cT};
+            tile_product3<1, 1, false, false>(c, T1, AP, 16 * mt, cV, TAIL_COLS, 0, 1, j0 & ~15, min(16 * mt + 16, (j1 + 15) & ~15), lane, j0, j1);
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = 16 * mt + gq + 8 * hh;
+                *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
+            }
+            __syncthreads();
+            kt_product(nullptr, l);
             __syncthreads();
         }
-        const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
-        for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
-            store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, sOut[i], a.qkv_dt);
-        if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
-            fence_async_shared();
-            __syncthreads();
-            if (tid < KD) {
-                bulk_s2g(st + (size_t)tid * VD * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
-                bulk_commit();
-                bulk_wait_read();
+        if (s == 0 && ta.early && tailed) (void)chain_wait();        // the chunk levels are there
+        if (tailed) {
+            float *sX = sm + M::X, *sD = sm + M::D, *sY = sm + M::Y;
+            const int nslot = __popc((uint32_t)nch);
+            for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
+                fetch_slots(s0);
+#pragma unroll
+                for (int i = 0; i < XR; ++i)
+                    sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs == 0 ? sSum[(s * KD + xk + 16 * i) * TAIL_COLS + xv] : 0.f);
+                __syncthreads();
+                const int l = slot_level(s0 + nt);
+                float y[4];
+                {   // K X and Q X
+                    float c[2][1][4] = {};
+                    const float* const kq[2] = {cK, sQ};
+                    tile_product3<2, 1, false, false>(c, kq, KP, 16 * mt, sX, XP, 8 * nt, 1, 0, KD, lane);
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int i = 16 * mt + gq + 8 * hh;
+                        *reinterpret_cast<float2*>(sD + i * XP + 8 * nt + 2 * tq) = make_float2(cEg[i] * c[0][0][2 * hh], cEg[i] * c[0][0][2 * hh + 1]);
+                        y[2 * hh] = cEg[i] * c[1][0][2 * hh];
+                        y[2 * hh + 1] = cEg[i] * c[1][0][2 * hh + 1];
+                    }
+                }
+                __syncthreads();
+                {   // T and R times that
+                    float c[2][1][4] = {};
+                    const float* const tr[2] = {cT, sP};
+                    tile_product3<2, 1, false, false>(c, tr, AP, 16 * mt, sD, XP, 8 * nt, 1, 0, 16 * mt + 16, lane);
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int i = 16 * mt + gq + 8 * hh;
+                        const float w = l >= 0 && i < done ? sLam[i * L + l] : 0.f;
+                        *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
+                        *reinterpret_cast<float2*>(sY + i * XP + 8 * nt + 2 * tq) = make_float2(w * (y[2 * hh] - c[1][0][2 * hh]), w * (y[2 * hh + 1] - c[1][0][2 * hh + 1]));
+                    }
+                }
+                __syncthreads();
+                {
+                    const float* p = sY + row * XP + c8;         // the slots of the batch
+                    sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
+                }
+                kt_product(sX, l);
+                __syncthreads();
             }
-        } else {
-            __syncthreads();
-            for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) {
-                const int k = i / (TAIL_COLS * L);
-                st[(size_t)k * VD * L + (i - k * TAIL_COLS * L)] = slab[i];
+            const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
+            for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
+                store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, sOut[i], a.qkv_dt);
+            if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
+                fence_async_shared();
+                __syncthreads();
+                if (tid < KD) {
+                    bulk_s2g(st + (size_t)tid * VD * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
+                    bulk_commit();
+                    bulk_wait_read();
+                }
+            } else {
+                __syncthreads();
+                for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) {
+                    const int k = i / (TAIL_COLS * L);
+                    st[(size_t)k * VD * L + (i - k * TAIL_COLS * L)] = slab[i];
+                }
             }
         }
     }
@@ -902,23 +927,28 @@ __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs 
     }
 }
 
-// The closed form takes 30 us whatever the tail (8 heads, K = V = 64; 12 us without one), a CTA to an SM; the steps 19 us and 0.4 us
-// per token behind the last chunk (0.25 at head dims up to 32), any number of CTAs.  Both begin beside the output pass.  Whole
-// calls of 2,944 tokens and a tail, steps against closed form: 63 and 63 us at 2 and 18 tokens, 77 and 70 at 22, 84 and 72 at 32;
-// without a tail 66 and 58.  6 heads of 16 and 32: 320 tokens and 30 30 and 35 us, 256 and 44 39 and 39.  Past one CTA to an SM the
-// closed form would take a second round.
+// Which form takes a tail follows from the tail alone, because the two do not round alike: a prompt's state and outputs are the
+// same alone and in a batch.  The closed form takes 30 us whatever the tail (8 heads, K = V = 64; 12 us without one), a CTA to an SM;
+// the steps 19 us and 0.4 us per token behind the last chunk (0.25 at head dims up to 32), any number of CTAs.  Both begin beside
+// the output pass.  Whole calls of 2,944 tokens and a tail, steps against closed form: 63 and 63 us at 2 and 18 tokens, 77 and 70 at
+// 22, 84 and 72 at 32; without a tail 66 and 58.  6 heads of 16 and 32: 320 tokens and 30 30 and 35 us, 256 and 44 39 and 39.
+// In batches a CTA of the closed form works through several slabs: 8 heads of 64, 704 tokens and 16, 32 and 60 behind
+// them, 71, 83 and 103 us by steps and 91, 93 and 93 at once for four prompts, 359, 409 and 503 against 497, 507 and 513 for 32; without
+// a tail 55 and 65 us, 279 and 317.
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
-    const dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
+    dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
     ProfScope prof("hgdn_tail", st);
-    if ((ta.tail == 0 || ta.tail >= (KD == 64 ? 16 : 48)) && (int64_t)a.nseq * a.H * (VD / TAIL_COLS) <= sm_count()) {
+    if (ta.tail == 0 || ta.tail >= (KD == 64 ? 16 : 48)) {
         using M = TailSmem<KD>;
-        const int smem = M::floats(ta.tail > 0, a.L) * 4;
-        constexpr int most = M::floats(true, 40) * 4;
+        TailArgs tc = ta;
+        while ((int64_t)a.nseq * a.H * grid.z > sm_count() && grid.z > 1) { grid.z /= 2; tc.slabs *= 2; }
+        const int smem = M::floats(ta.tail > 0, a.L, tc.slabs) * 4;
+        constexpr int most = M::floats(true, 40, VD / TAIL_COLS) * 4;
         static_assert(most <= 227 * 1024, "shared memory of an SM");
         static std::atomic<uint64_t> ready;
         if (!allow_smem(ready, hgdn_tail_kernel<KD, VD>, most)) return LAMPA_ERR_CUDA;
-        launch_chained(hgdn_tail_kernel<KD, VD>, grid, TAIL_THREADS, smem, st, a, ta);
+        launch_chained(hgdn_tail_kernel<KD, VD>, grid, TAIL_THREADS, smem, st, a, tc);
         return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
     }
     const int slots = ta.tail > 0 ? __builtin_popcount((unsigned)ta.n0) : 0;

@@ -75,3 +75,20 @@ def test_model_event_alone_and_in_a_batch():
     full = m(torch.cat(hits), cu.cuda())
     for i, n in enumerate(lengths):
         assert torch.equal(m(hits[i], torch.tensor([0, n], device="cuda")), full[cu[i] : cu[i + 1]]), n
+
+
+# tails of nothing, of either form of the tail kernel (16 tokens and more at once at K = 64, 48 at smaller heads) and of 63; a prompt
+# alone has a CTA per eight state columns, the batches have CTAs that work through several
+@pytest.mark.parametrize("K,V,H,B", [(64, 64, 8, 3), (64, 64, 8, 24), (32, 32, 8, 6), (16, 32, 8, 40), (64, 64, 2, 40)])
+@pytest.mark.parametrize("T", [57, 128, 143, 144, 191, 320 + 31])
+def test_prompts_alone_and_in_a_batch(K, V, H, B, T):
+    L = 12
+    rows = [_draw(10 * T + i, T, H, K, V, L) for i in range(B)]
+    o, st = _hier([torch.cat(t) for t in zip(*rows)], state=True)
+    for i in (0, B - 1):
+        oi, si = _hier(rows[i], state=True)
+        assert torch.equal(oi[0], o[i]) and torch.equal(si.states[0], st.states[i])
+    for a, b in ((0, 1), (1, H)):
+        oh, sh = _hier(_heads(rows[0], a, b), state=True)
+        assert torch.equal(oh[0], o[0, :, a:b]) and torch.equal(sh.states[0], st.states[0, a:b])
+    lampa_b200.check_status(torch.device("cuda:0"))
