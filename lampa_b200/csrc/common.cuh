@@ -198,14 +198,35 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 // A kernel may let the next one start before its own end (chain_signal, once all its CTAs have passed it or left).  That is
 // for kernels that leave most of the GPU idle and for a next one that can do without them: everywhere else the next grid only
 // fills the SMs that happen to be free, two or three CTAs to an SM beside idle ones (56 and 447 us, and 486 instead of 463 for a
-// 60,000-hit event).  chain_signal comes behind chain_wait: what the kernel was waiting for is complete for the next one
-// too, which may read it (from L2) before its own wait.  A CTA of that one still waits before it ends, so that its end means theirs.
+// 60,000-hit event).  chain_signal comes behind chain_wait: what the kernel was waiting for is complete then.  The next one may use
+// it before its own wait only where chain_seen() says so, and a CTA of it still waits before it ends, so that its end means
+// theirs.  That a grid has been let in orders no memory by itself: the first thread of the signalling kernel, for which griddepcontrol.wait
+// has made all of it visible, therefore leaves the call's number in a word of the call's workspace with a release, and a
+// kernel that reads that number with an acquire comes behind it in the memory model's causality order.  One that does not find
+// it waits as any other.  (The last kernel of the call clears the word behind its wait: a replayed call has the same number.)
 __device__ __forceinline__ bool chain_wait() {
     uint32_t never;
     asm volatile("griddepcontrol.wait;\n mov.u32 %0, 0;\n" : "=r"(never) :: "memory");
     return never != 0;
 }
 __device__ __forceinline__ void chain_signal() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// All threads of the grid, behind chain_wait().  One thread signals for its CTA: the first one's word is out by then.
+__device__ __forceinline__ void chain_signal(unsigned long long* word, unsigned long long call) {
+    if (threadIdx.x != 0) return;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+        asm volatile("st.release.gpu.global.u64 [%0], %1;\n" :: "l"(word), "l"(call) : "memory");
+        __threadfence();
+    }
+    chain_signal();
+}
+// All threads of a CTA: whether what was complete in front of the kernel that signalled with `call` may be used, by bulk copies too
+__device__ __forceinline__ bool chain_seen(const unsigned long long* word, unsigned long long call) {
+    unsigned long long v = 0;
+    if (threadIdx.x == 0) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(word) : "memory");
+    const bool seen = __syncthreads_or(threadIdx.x == 0 && v == call) != 0;
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+    return seen;
+}
 inline cudaLaunchAttribute chained_attribute() {
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

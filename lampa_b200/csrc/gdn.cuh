@@ -100,7 +100,8 @@ struct GdnArgs {
     int use_umma;                         // tcgen05 kernels where they exist (K = V = 64)
     int poll_budget;                      // polls before a device wait gives up (MBAR_POLLS unless a test lowers it)
     int long_only, short_only;            // output pass: only sequences of more (of at most) UMMA_LEVELS chunk levels
-    int signal;                           // a prefill's output pass and chunk levels let the next kernel in (chain_signal)
+    unsigned long long signal;            // a prefill's number, or 0: its output pass and chunk levels let the next kernel in (chain_signal)
+    unsigned long long* signal_word;
     long long* ticks; int ticks_ctas;     // stage clocks for tuning: [ticks_ctas][16] or NULL (lampa_debug_set_tick_buffer)
 };
 

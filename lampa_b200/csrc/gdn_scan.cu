@@ -488,10 +488,14 @@ __global__ void __launch_bounds__(NW * 32 + 32) gdn_level_kernel(GdnArgs a) {
 template <int KD, int VD>
 __global__ void __launch_bounds__(VD * 2 + 32) hgdn_final_high_kernel(GdnArgs a, float* states) {
     // In a prefill the output pass in front lets this one in at its start: it needs nothing of that pass, only what was complete
-    // before it, so it runs beside it and signals in turn.  One CTA waits at its end, which keeps the grid's end behind that pass's;
+    // before it (chain_seen), so it runs beside it and signals in turn.  One CTA waits at its end, which keeps the grid's end behind that pass's;
     // the others give their SMs to the prompt's tail.
-    if (a.signal) chain_signal();
-    else if (chain_wait()) return;
+    if (a.signal) {
+        chain_signal();
+        if (!chain_seen(a.signal_word, a.signal) && chain_wait()) return;
+    } else if (chain_wait()) {
+        return;
+    }
     using R = Rec<KD, VD>;
     constexpr int NST = 3, NW = VD / 16;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -710,7 +714,7 @@ constexpr int HIER_TILES = 4;
 template <int KD, int VD, int NG>
 __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hier_kernel(GdnArgs a) {
     if (chain_wait()) return;
-    if (a.signal) chain_signal();
+    if (a.signal) chain_signal(a.signal_word, a.signal);
     using R = Rec<KD, VD>;
     constexpr int NST = 3;
     constexpr int NS = VD / 16;
@@ -908,7 +912,7 @@ struct LevelsSmem {
 template <int KD, int VD, int STAGES>
 __global__ void __launch_bounds__(LV_MAX_THREADS) gdn_out_levels_kernel(GdnArgs a, int pairs) {
     if (chain_wait()) return;
-    if (a.signal) chain_signal();
+    if (a.signal) chain_signal(a.signal_word, a.signal);
     using R = Rec<KD, VD>;
     using S = LevelsSmem<KD, VD, STAGES>;
     constexpr int NS = VD / 16;

@@ -99,7 +99,7 @@ struct UnitOrder {
 // halves of the accumulator row at once: 166 - 217 us, the registers spill.)
 __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs a, UnitOrder uo) {
     if (chain_wait()) return;
-    if (a.signal) chain_signal();
+    if (a.signal) chain_signal(a.signal_word, a.signal);
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM_BAR);      // record landed            (tx count)
     uint64_t* sfree = full + UNST;                                      // stage consumed           (16 + 4 warps)

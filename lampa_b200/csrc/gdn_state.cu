@@ -92,7 +92,7 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // there are SMs for all); T and R do not depend on the column and are formed once by each CTA, two halves of it on the last
 // chunk and the tail side by side.  A column's arithmetic is the same whichever CTA has it.
 // 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
-// pass (launch_chained): the call 95 -> 65 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
+// pass (launch_chained): the call 95 -> 67 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
 // cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (68 us the call).
 // -------------------------------------------------------------------------------------------------
@@ -185,7 +185,7 @@ __device__ __forceinline__ void tail_inverse(float* A, const float* beta, int t,
 template <int KD, int VD>
 __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, TailArgs ta) {
     // In a prefill the kernels in front let this one in early: until it waits it reads the call's inputs alone.
-    if (!ta.early && chain_wait()) return;
+    if (!(ta.early && chain_seen(a.signal_word, a.signal)) && chain_wait()) return;
     using M = TailSmem<KD>;
     constexpr int KP = M::KP, AP = TAIL_AP, XP = TAIL_XP;
     extern __shared__ __align__(16) float sm[];
@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         }
         cn[0] = n > 0 ? 1 : 0;
         if (seq == 0 && ta.arrivals) *ta.arrivals = 0;
+        if (ta.early) *a.signal_word = 0;                  // behind the wait
         if (rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
     }
 }
@@ -635,7 +636,7 @@ __device__ __forceinline__ void half_warp_sum_many(float (&x)[N], int lane) {
 
 template <int KD, int VD, int HS>
 __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs a, TailArgs ta) {
-    if (!ta.early && chain_wait()) return;               // see above: only the inputs are read before the wait
+    if (!(ta.early && chain_seen(a.signal_word, a.signal)) && chain_wait()) return;      // see above: only the inputs are read before the wait
     constexpr int KI = KD / 16;
     extern __shared__ __align__(16) float tail_smem[];
     float* sK = tail_smem;                       // [64][KD], normalised
@@ -923,6 +924,7 @@ __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs 
         }
         cn[0] = n > 0 ? 1 : 0;
         if (seq == 0 && ta.arrivals) *ta.arrivals = 0;
+        if (ta.early) *a.signal_word = 0;                  // behind the wait
         if (rem != 0) set_status(a.status, LAMPA_ERR_LEVELS, 30, seq);
     }
 }

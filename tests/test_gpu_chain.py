@@ -72,3 +72,60 @@ def test_steps_behind_one_another():
         runs.append((torch.stack(outs), st.states.clone(), st.counts.clone()))
     for a, b in zip(*runs):
         assert torch.equal(a, b)
+
+
+def _prompts(T, H, K, V, n):
+    L = lampa_b200.num_levels_required(max(T, 64))
+    sets = [_inputs(20 + s, 1, T, H, K, V, L) for s in range(n)]
+    want = []
+    for x in sets:
+        torch.cuda.synchronize()
+        o, st = _mixer(x, output_final_state=True)
+        torch.cuda.synchronize()
+        want.append((o.clone(), st.states.clone(), st.counts.clone()))
+    return sets, want
+
+
+# a prompt whose tail is taken in at once, token by token, and none; more CTAs than fit the GPU
+@pytest.mark.parametrize("T,H,K,V", [(700, 4, 64, 64), (3001, 8, 64, 64), (643, 4, 64, 64), (1024, 8, 64, 64), (5003, 2, 32, 32), (700, 40, 16, 32)])
+def test_prefill_replayed(T, H, K, V):
+    """The end of a prompt begins beside its output pass, in a replayed graph too, where every replay has the same number."""
+    sets, want = _prompts(T, H, K, V, 3)
+    buf = [t.clone() for t in sets[0]]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        _mixer(buf, output_final_state=True)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            rows = [t + 0 for t in buf]                      # written right in front of the call
+            o, st = _mixer(rows, output_final_state=True)
+        got = []
+        for _ in range(4):
+            for x in sets:
+                for b, t in zip(buf, x):
+                    b.copy_(t)
+                graph.replay()
+                got.append((o.clone(), st.states.clone(), st.counts.clone()))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        for a, b in zip(g, want[i % 3]):
+            assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("T,H,K,V", [(700, 4, 64, 64), (3001, 8, 64, 64), (5003, 2, 32, 32)])
+def test_prefills_beside_one_another(T, H, K, V):
+    """Prompts on three streams, their kernels among one another's on the same SMs; each writes its inputs right before its call."""
+    sets, want = _prompts(T, H, K, V, 3)
+    streams = [torch.cuda.Stream() for _ in sets]
+    got = [[] for _ in sets]
+    torch.cuda.synchronize()
+    for _ in range(6):
+        for i, (s, x) in enumerate(zip(streams, sets)):
+            with torch.cuda.stream(s):
+                o, st = _mixer([t + 0 for t in x], output_final_state=True)
+                got[i].append((o, st.states, st.counts))
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        for r in g:
+            for a, b in zip(r, w):
+                assert torch.equal(a, b)
