@@ -749,7 +749,7 @@ extern "C" int lampa_bucket_rbf_attn_checked(const float* q, const float* k, con
     plan(4, warps, smem);
     const bool wide = smem > 113 * 1024;                   // not even two CTAs of 4-row tiles fit an SM
     if (wide) plan(8, warps, smem);
-    if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
+    if (smem > MAX_SMEM) return LAMPA_ERR_UNSUPPORTED;
     const int64_t units = (int64_t)rounds * heads * (n / bucket);
     if (units > 0x7fffffffLL) return LAMPA_ERR_UNSUPPORTED;
     // Rows of up to 32 features are what a warp's tile holds in registers at three CTAs per SM; with wider ones this kernel
@@ -758,14 +758,13 @@ extern "C" int lampa_bucket_rbf_attn_checked(const float* q, const float* k, con
         const int keys = bam_keys(bucket);
         auto mma = dv <= 24 ? bucket_attn_mma_kernel<2, 3> : bucket_attn_mma_kernel<2, 4>;
         const int msmem = bam_smem<2, 4>(keys);
-        if (cudaFuncSetAttribute(mma, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem) != cudaSuccess) return LAMPA_ERR_CUDA;
+        if (cudaFuncSetAttribute(mma, cudaFuncAttributeMaxDynamicSharedMemorySize, bam_smem<2, 4>(BA_MAX_BUCKET)) != cudaSuccess) return LAMPA_ERR_CUDA;
         ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
         launch_chained(mma, (unsigned)units, 2 * keys, msmem, (cudaStream_t)stream, a);
         return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
     }
     auto kernel = wide ? bucket_rbf_attn_kernel<8> : bucket_rbf_attn_kernel<4>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return LAMPA_ERR_CUDA;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM) != cudaSuccess) return LAMPA_ERR_CUDA;
     ProfScope prof("bucket_rbf_attn", (cudaStream_t)stream);
     launch_chained(kernel, (unsigned)units, warps * 32, smem, (cudaStream_t)stream, a);
     return cudaGetLastError() == cudaSuccess ? LAMPA_OK : LAMPA_ERR_CUDA;
@@ -813,7 +812,8 @@ extern "C" int lampa_hept_front(const float* query, const float* key, const floa
     if (n == 0) return LAMPA_OK;
     if (!query || !key || !value || !scale || !coords || !alpha || !q_hat || !k_hat || !v_out || !proj || !part) return LAMPA_ERR_ARG;
     const size_t smem = hf_smem(heads, d, cd, rounds);
-    if (rounds > HF_MAX_ROUNDS || smem > 200 * 1024) return LAMPA_ERR_UNSUPPORTED;
+    constexpr int most = 200 * 1024;
+    if (rounds > HF_MAX_ROUNDS || smem > most) return LAMPA_ERR_UNSUPPORTED;
     using K = void (*)(const float*, const float*, const float*, const float*, const float*, const float*, int64_t, int, int, int, int, int64_t,
                        float*, float*, float*, float*, float2*);
     static const K kernels[2][HF_MAX_ROUNDS] = {
@@ -824,7 +824,7 @@ extern "C" int lampa_hept_front(const float* query, const float* key, const floa
     const bool vec = d % 4 == 0 && ldq % 4 == 0 && heads * d <= 1024 &&
                      (((uintptr_t)query | (uintptr_t)key | (uintptr_t)value | (uintptr_t)q_hat | (uintptr_t)k_hat | (uintptr_t)v_out) & 15) == 0;
     const K kernel = kernels[vec][rounds - 1];
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LAMPA_ERR_CUDA;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return LAMPA_ERR_CUDA;
     ProfScope prof("hept_front", (cudaStream_t)stream);
     launch_chained(kernel, (unsigned)((n + HF_HITS - 1) / HF_HITS), 256, smem, (cudaStream_t)stream, query, key, value, scale, coords, alpha, n, heads, d, cd, ldq,
                                                                                         raw_size, q_hat, k_hat, v_out, proj, (float2*)part);

@@ -254,6 +254,9 @@ inline int sm_count() {
 }
 
 // Opt-in to `bytes` of dynamic shared memory for a kernel, once per device (`ready`: one bit per device, static at the call).
+// The opt-in is the kernel's, not the launch's: where the size varies, every call opts in to the largest one that the entry point
+// accepts, or a thread with a smaller size would take the opt-in of another one's launch back in front of it.
+constexpr int MAX_SMEM = 227 * 1024;                     // dynamic shared memory of a kernel that has no other
 template <typename K>
 inline bool allow_smem(std::atomic<uint64_t>& ready, K kernel, int bytes) {
     int dev = 0;

@@ -586,7 +586,8 @@ int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     const int lam_tile = hier ? CHUNK * a.H * a.L * 2 : 0;
     const int lam_tma = hier && a.lam_dt != LAMPA_F32 && (a.H * a.L) % 8 == 0 && a.H * a.L <= 256 && lam_tile <= LAM_TMA_MAX;
     const int smem = prep_umma_smem(hier ? a.L : 0, lam_tma ? lam_tile : 0);
-    if (smem > 113 * 1024) return LAMPA_ERR_UNSUPPORTED;
+    constexpr int most = 113 * 1024;
+    if (smem > most) return LAMPA_ERR_UNSUPPORTED;
     CUtensorMap tq, tk, tv, tl;
     if (!make_map(&tq, a.q, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, CHUNK, true) ||
         !make_map(&tk, a.k, a.qkv_dt, tokens, (uint64_t)a.H * 64, 64, CHUNK, true) ||
@@ -599,8 +600,8 @@ int launch_prep_umma(const GdnArgs& a, bool hier, cudaStream_t st) {
     static const int nc = [] { const char* e = getenv("LAMPA_B200_PREP_COLS"); return (e && atoi(e) == 32) ? 32 : 16; }();
 #define LAMPA_LAUNCH_PREP(HIER_, NC_)                                                                                  \
     do {                                                                                                               \
-        if (cudaFuncSetAttribute(gdn_prep_umma_kernel<HIER_, NC_>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) \
-            return LAMPA_ERR_CUDA;                                                                                     \
+        static std::atomic<uint64_t> ready;                                                                            \
+        if (!allow_smem(ready, gdn_prep_umma_kernel<HIER_, NC_>, most)) return LAMPA_ERR_CUDA;                         \
         launch_chained(gdn_prep_umma_kernel<HIER_, NC_>, grid, 8192 / NC_, smem, st, a, tq, tk, tv, tl, HIER_ ? lam_tma : 0);        \
     } while (0)
     if (hier) { if (nc == 32) LAMPA_LAUNCH_PREP(true, 32); else LAMPA_LAUNCH_PREP(true, 16); }

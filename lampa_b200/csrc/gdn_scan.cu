@@ -1129,8 +1129,8 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
     using R = Rec<KD, VD>;
     const int stage = (R::bytes(a.LC) + 1023) / 1024 * 1024;
     const int smem = 1024 + 3 * stage + (NG - 1) * (VD / 16) * 4096;
-    if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
-    LAMPA_TRY(set_smem(gdn_out_hier_kernel<KD, VD, NG>, smem));
+    if (smem > MAX_SMEM) return LAMPA_ERR_UNSUPPORTED;
+    LAMPA_TRY(set_smem(gdn_out_hier_kernel<KD, VD, NG>, MAX_SMEM));
     ProfScope prof("gdn_out_hier", st);
     launch_chained(gdn_out_hier_kernel<KD, VD, NG>, dim3(a.nb_max, a.H), NG * VD * 2, smem, st, a);
     LAMPA_LAUNCHED();
@@ -1140,7 +1140,7 @@ static int launch_out_hier(const GdnArgs& a, cudaStream_t st) {
 template <int KD, int VD, int STAGES>
 static int launch_out_levels(const GdnArgs& a, int pairs, cudaStream_t st) {
     const int smem = LevelsSmem<KD, VD, STAGES>::bytes(a.LC, pairs);
-    LAMPA_TRY(set_smem(gdn_out_levels_kernel<KD, VD, STAGES>, smem));
+    LAMPA_TRY(set_smem(gdn_out_levels_kernel<KD, VD, STAGES>, MAX_SMEM));
     ProfScope prof("gdn_out_hier", st);
     launch_chained(gdn_out_levels_kernel<KD, VD, STAGES>, dim3(a.nb_max, a.H), (2 * pairs + 1 + LV_SUM) * 32, smem, st, a, pairs);
     LAMPA_LAUNCHED();
@@ -1169,8 +1169,8 @@ int launch_scan_hier(const GdnArgs& a, cudaStream_t st) {
     if constexpr (KD <= 32) {
         const int pairs = ((a.nlev_max > MIN_BLOCK_LOG ? a.nlev_max : MIN_BLOCK_LOG) + 1) / 2;      // a block has at most a slot per level of its sequence
         if ((int64_t)a.nb_max * a.H <= sm_count() && pairs <= LV_MAX_PAIRS) {
-            if (LevelsSmem<KD, VD, 4>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD, 4>(a, pairs, st);
-            if (LevelsSmem<KD, VD, 3>::bytes(a.LC, pairs) <= 227 * 1024) return launch_out_levels<KD, VD, 3>(a, pairs, st);
+            if (LevelsSmem<KD, VD, 4>::bytes(a.LC, pairs) <= MAX_SMEM) return launch_out_levels<KD, VD, 4>(a, pairs, st);
+            if (LevelsSmem<KD, VD, 3>::bytes(a.LC, pairs) <= MAX_SMEM) return launch_out_levels<KD, VD, 3>(a, pairs, st);
         }
     }
     if (ng == 1) return launch_out_hier<KD, VD, 1>(rest, st);

@@ -419,9 +419,9 @@ __global__ void __launch_bounds__(UTHREADS, 1) gdn_out_hier_umma_kernel(GdnArgs 
 
 int launch_out_hier_umma(const GdnArgs& a, cudaStream_t st) {
     const int smem = SM_STAGE + UNST * ustage_bytes(a.LC);
-    if (smem > 227 * 1024) return LAMPA_ERR_UNSUPPORTED;
-    if (cudaFuncSetAttribute(gdn_out_hier_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return LAMPA_ERR_CUDA;
+    if (smem > MAX_SMEM) return LAMPA_ERR_UNSUPPORTED;
+    static std::atomic<uint64_t> ready;
+    if (!allow_smem(ready, gdn_out_hier_umma_kernel, MAX_SMEM)) return LAMPA_ERR_CUDA;
     UnitOrder uo;
     uo.nbs = 0;
     if (a.fixed_T > 0 && a.nseq > 0 && a.nb_max % a.nseq == 0 && a.nb_max / a.nseq <= 64) {

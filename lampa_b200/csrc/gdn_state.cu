@@ -1206,9 +1206,9 @@ __global__ void hgdn_step_counts_kernel(int32_t* counts, int L) {
 
 template <int KD, int VD>
 int launch_hgdn_step(const StepArgs& s, cudaStream_t st) {
-    const int smem = step_smem<KD>(s.L);           // at most 103 KB
-    if (smem > 44 * 1024 && cudaFuncSetAttribute(hgdn_step_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return LAMPA_ERR_CUDA;
+    const int smem = step_smem<KD>(s.L);
+    static std::atomic<uint64_t> ready;
+    if (!allow_smem(ready, hgdn_step_kernel<KD, VD>, step_smem<KD>(STEP_MAX_L))) return LAMPA_ERR_CUDA;      // 103 KB
     // one tiled copy per slab, up to 32 levels (a box is at most 256 elements wide)
     CUtensorMap map = {};
     const int64_t rows = (int64_t)s.B * s.H * KD;

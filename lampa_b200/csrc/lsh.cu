@@ -739,10 +739,11 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
     if (ws_bytes < need || ((uintptr_t)ws & 15)) return LAMPA_ERR_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
     const int params = dim * ((num_hashes + 3) & ~3) * 4;
+    constexpr int params_most = 4 * HASH_MAX_PARAMS * 4;                 // one hash to a coordinate, padded to four
     if (ordering_counts(B, n) && row_bytes <= (1 << 20)) {
         const int smem = (int)n * 8 + params;
         const OrderKernel kernel = order_kernel(dim, num_hashes, std::make_integer_sequence<int, ORDER_REGS>());
-        if (smem > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        if (smem > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_MAX_N * 8 + params_most) != cudaSuccess)
             return LAMPA_ERR_CUDA;
         ProfScope prof("lsh_ordering", st);
         launch_chained(kernel, dim3((unsigned)((n + ORDER_POINTS - 1) / ORDER_POINTS), (unsigned)B), ORDER_THREADS, smem, st,
@@ -763,7 +764,7 @@ extern "C" int lampa_lsh_ordering(const float* coords, const float* alpha, int32
         static const Kernel kernels[] = {ordering_keys_kernel<0>, ordering_keys_kernel<1>, ordering_keys_kernel<2>, ordering_keys_kernel<3>, ordering_keys_kernel<4>,
                                          ordering_keys_kernel<5>, ordering_keys_kernel<6>, ordering_keys_kernel<7>, ordering_keys_kernel<8>};
         const Kernel kernel = kernels[dim <= ORDER_REGS ? dim : 0];
-        if (params > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, params) != cudaSuccess)
+        if (params > 47 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, params_most) != cudaSuccess)
             return LAMPA_ERR_CUDA;
         launch_chained(kernel, (unsigned)((total + 255) / 256), 256, params, st, coords, alpha, dim, num_hashes, total, keys, norms);
         if (cudaGetLastError() != cudaSuccess) return LAMPA_ERR_CUDA;
