@@ -46,6 +46,8 @@ __device__ __forceinline__ void raw_floats(const uint4& u, int dt, float (&x)[8]
     }
 }
 
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
 // Eight consecutive elements as floats (zeros where `live` is false): 16-byte loads where the base allows them
 __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, bool live, float (&x)[8]) {
     if (!live) {
@@ -91,6 +93,10 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // A CTA takes eight state columns of a (sequence, head) after the other, as many as leave one CTA to an SM (one set of eight while
 // there are SMs for all); T and R do not depend on the column and are formed once by each CTA, two halves of it on the last
 // chunk and the tail side by side.  A column's arithmetic is the same whichever CTA has it.
+// A k, beta or e^g that is not finite enters as zero (g: as one), or the zeros above a diagonal times its row would reach outputs of
+// tokens before it.  What the recurrence makes of it is filled in: with a k or beta the states that hold the token or
+// older ones are NaN from then on, with a g those that hold older ones, and so are the outputs, which read them all.  (q, v and
+// lambda reach only what they belong to.)
 // 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
 // pass (launch_chained): the call 95 -> 67 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
@@ -102,7 +108,8 @@ constexpr int TAIL_AP = CHUNK + 4, TAIL_XP = TAIL_BATCH * TAIL_COLS + 4;        
 template <int KD>
 struct TailSmem {                                            // offsets in floats
     static constexpr int KP = KD + 4;
-    static constexpr int SCAL = 2 * CHUNK + 3 * CHUNK;       // G (double), e^G, e^{Gl-G}, beta
+    static constexpr int LOST = 2 * CHUNK + 3 * CHUNK;       // behind G (double), e^G, e^{Gl-G}, beta
+    static constexpr int SCAL = LOST + 3 * CHUNK / 4;        // [3][64] bytes: whether a token's k, g or beta is not finite
     static constexpr int CH = CHUNK * KP + CHUNK * TAIL_AP + CHUNK * TAIL_COLS + SCAL;       // k, A -> T, v, scalars of one chunk
     static constexpr int K_ = 0, A_ = CHUNK * KP, V_ = A_ + CHUNK * TAIL_AP, S_ = V_ + CHUNK * TAIL_COLS;
     static constexpr int Z = CH;                             // [64][XP]
@@ -273,9 +280,18 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 #pragma unroll
         for (int it = 0; it < NL; ++it) lv[it] = lam_load(t + it * TAIL_GRP);
         // e^g is zero far above -1e5; a g of minus infinity would make differences of G undefined
-        auto decay = [&](uint32_t w) { const float g = raw_float(w, a.gb_dt); return g < -1e5f ? -1e5f : g; };
-        const float g0 = decay(g0w), g1 = decay(g1w), bt = raw_float(btw, a.gb_dt);
-        if (t < CHUNK) sBeta[t] = bt;
+        auto decay = [&](uint32_t w, bool& bad) {
+            const float g = raw_float(w, a.gb_dt);
+            bad = !finite(__expf(g));
+            return bad ? 0.f : g < -1e5f ? -1e5f : g;
+        };
+        unsigned char* bad = reinterpret_cast<unsigned char*>(ch + M::S_ + M::LOST);
+        bool bad0, bad1;
+        const float g0 = decay(g0w, bad0), g1 = decay(g1w, bad1), bt = raw_float(btw, a.gb_dt);
+        if (t < CHUNK) {
+            sBeta[t] = finite(bt) ? bt : 0.f;
+            bad[2 * CHUNK + t] = !finite(bt);
+        }
 #pragma unroll
         for (int it = 0; it < NV; ++it) sV[t + it * TAIL_GRP] = raw_float(vv[it], a.qkv_dt);
 #pragma unroll
@@ -307,6 +323,14 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 #pragma unroll
                 for (int e = 0; e < 8; ++e) { x[e] = round_like(x[e] * rk, a.qkv_dt); y[e] *= rq; }
             }
+            bool any = false;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) any |= !finite(x[e]);
+            any = (__ballot_sync(0xffffffffu, any) >> (lane & ~(PPR - 1)) & ((1u << PPR) - 1u)) != 0;
+            if (c == 0) bad[r] = any;
+            if (any)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = 0.f;
             float4* d = reinterpret_cast<float4*>(sK + r * KP + c);
             d[0] = make_float4(x[0], x[1], x[2], x[3]);
             d[1] = make_float4(x[4], x[5], x[6], x[7]);
@@ -328,6 +352,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 if (lane >= o) cs += u;
             }
             const double last = __shfl_sync(0xffffffffu, cs, 31);
+            bad[CHUNK + 2 * t] = bad0; bad[CHUNK + 2 * t + 1] = bad1;
             sG[2 * t] = cs - (double)g1; sG[2 * t + 1] = cs;
             sEg[2 * t] = __expf((float)(cs - (double)g1)); sEg[2 * t + 1] = __expf((float)cs);
             sEl[2 * t] = __expf((float)(last - (cs - (double)g1))); sEl[2 * t + 1] = __expf((float)(last - cs));
@@ -406,14 +431,29 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const int len_all = tailed ? done : nch == 0 ? 0 : ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - tok0 - (int64_t)(nch - 1) * CHUNK);
     const int row = tid >> 3, c8 = tid & 7;                  // row and column of what goes element by element
     const int warp = tid >> 5, mt = warp & 3, nt = warp >> 2;       // products: 16 rows, and eight columns: state nt of a batch
+    // tokens of a chunk with a k or beta that is not finite, and with such a g, as masks; and what they take with them
+    struct Lost { unsigned long long kb, g; };
+    auto lost_tokens = [&](const float* c) {
+        const unsigned char* f = reinterpret_cast<const unsigned char*>(c + M::S_ + M::LOST) + lane;
+        Lost m;
+        m.kb = (unsigned long long)__ballot_sync(0xffffffffu, f[32] | f[2 * CHUNK + 32]) << 32 | __ballot_sync(0xffffffffu, f[0] | f[2 * CHUNK]);
+        m.g = (unsigned long long)__ballot_sync(0xffffffffu, f[CHUNK + 32]) << 32 | __ballot_sync(0xffffffffu, f[CHUNK]);
+        return m;
+    };
+    const Lost lost = r_all > 0 ? lost_tokens(cs) : Lost{0, 0}, before = tailed && nch > 0 ? lost_tokens(sm) : Lost{0, 0};
+    const unsigned long long lost_out = lost.kb | (nch > 0 ? lost.g : lost.g & ~1ull), lost_in = lost.kb | lost.g >> 1;
+    const int first_lost = lost_out ? __ffsll((long long)lost_out) - 1 : CHUNK;      // outputs from this token on
+    const int last_lost = lost_in ? 63 - __clzll((long long)lost_in) : -1;           // states with a token up to this one
+    const bool lost_slots = (lost.kb | lost.g) != 0, lost_before = (before.kb | before.g >> 1) != 0;
+    const float nan = __int_as_float(0x7fffffff);
 
     // where a state element of the result goes: the slab, which leaves at the end, or (no tail) the state itself
     auto put = [&](int k, int v, int l, float x) {
         if (tailed) slab[(k * TAIL_COLS + v) * L + l] = x;
         else st[((size_t)k * VD + v) * L + l] = x;
     };
-    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z, state nt to level l
-    auto kt_product = [&](const float* X, int l) {
+    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z, state nt to level l, or what is left of it (`gone`: nothing)
+    auto kt_product = [&](const float* X, int l, bool gone) {
         if (mt >= KD / 16 || l < 0 || l >= L) return;        // (warp-uniform)
         float c[1][1][4] = {};
         const float* const k1[1] = {cK};
@@ -422,7 +462,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int k = 16 * mt + gq + 8 * (e >> 1), v = 2 * tq + (e & 1);
-            put(k, v, l, X ? egl * X[k * XP + 8 * nt + v] - c[0][0][e] : c[0][0][e]);
+            put(k, v, l, gone ? nan : X ? egl * X[k * XP + 8 * nt + v] - c[0][0][e] : c[0][0][e]);
         }
     };
 
@@ -502,7 +542,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
             }
             __syncthreads();
-            kt_product(nullptr, l);
+            kt_product(nullptr, l, j0 <= last_lost);
             __syncthreads();
         }
         if (s == 0 && ta.early && tailed) (void)chain_wait();        // the chunk levels are there
@@ -513,7 +553,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                 fetch_slots(s0);
 #pragma unroll
                 for (int i = 0; i < XR; ++i)
-                    sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs == 0 ? sSum[(s * KD + xk + 16 * i) * TAIL_COLS + xv] : 0.f);
+                    sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs != 0 ? 0.f : lost_before ? nan : sSum[(s * KD + xk + 16 * i) * TAIL_COLS + xv]);
                 __syncthreads();
                 const int l = slot_level(s0 + nt);
                 float y[4];
@@ -547,12 +587,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
                     const float* p = sY + row * XP + c8;         // the slots of the batch
                     sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
                 }
-                kt_product(sX, l);
+                kt_product(sX, l, lost_slots);
                 __syncthreads();
             }
             const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
             for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
-                store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, sOut[i], a.qkv_dt);
+                store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, i / TAIL_COLS < first_lost ? sOut[i] : nan, a.qkv_dt);
             if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
                 fence_async_shared();
                 __syncthreads();

@@ -63,6 +63,52 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
     assert st.counts.view(-1)[:L].tolist() == want
 
 
+# a tail taken in at once behind a whole chunk, a prompt that is nothing but such a tail, and one that ends with a whole chunk; the
+# token that carries the value: in the tail, its first one, one of the last whole chunk, the first of all
+@pytest.mark.parametrize("K,V", [(64, 64), (32, 32), (16, 32)])
+@pytest.mark.parametrize("T,n", [(121, 101), (121, 64), (121, 40), (57, 33), (57, 0), (64, 50), (700, 690)])
+@pytest.mark.parametrize("what,value", [("q", "nan"), ("k", "nan"), ("k", "inf"), ("v", "nan"), ("v", "inf"), ("g", "nan"), ("g", "inf"), ("beta", "nan"),
+                                        ("beta", "inf"), ("lam", "nan")])
+def test_values_that_are_not_finite_reach_what_comes_after(K, V, T, n, what, value):
+    """A NaN or an infinity at token n: outputs and states are finite exactly where the token recurrence has them finite, outputs in
+    front of token n stay as they were, and so does the other head."""
+    H, L = 2, 12
+    gen = torch.Generator().manual_seed(T + K)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    x = dict(q=rn(1, T, H, K).bfloat16(), k=rn(1, T, H, K).bfloat16(), v=rn(1, T, H, V).bfloat16(), g=-F.softplus(rn(1, T, H) - 3),
+             lam=F.softplus(rn(1, T, H, L)), beta=torch.sigmoid(rn(1, T, H)))
+
+    def run():
+        o, st = lampa_b200.chunk_h_gated_delta_rule(*(t.cuda() for t in x.values()), output_final_state=True, use_qk_l2norm_in_kernel=True)
+        lampa_b200.check_status(torch.device("cuda:0"))
+        return o[0].float().cpu(), st.states[0].cpu()
+
+    o1, s1 = run()
+    at = (0, n, 0, 3) if x[what].dim() == 4 else (0, n, 0)
+    if what == "lam":
+        at = (0, n, 0, 0)                                    # the level of the token itself, which every output reads
+    x[what][at] = float(value)
+    o2, s2 = run()
+    # what the recurrence makes of it: the first and last of the tokens whose states are lost, and the outputs, which read all states
+    lost = {"q": None, "lam": None, "v": (n, n), "k": (0, n), "beta": (0, n), "g": (0, n - 1) if n > 0 else None}[what]
+    rows, cols = torch.zeros(T, V, dtype=torch.bool), slice(3, 4) if what == "v" else slice(None)
+    rows[n : T if lost else n if what == "g" else n + 1, cols] = True
+    # tokens of level l of the state: the older ones higher up, 2^(l-1) where bit l - 1 of T - 1 is set
+    want, end = torch.zeros(K, V, L, dtype=torch.bool), 0
+    for l in range(L - 1, -1, -1):
+        size = 1 if l == 0 else (1 << (l - 1)) if ((T - 1) >> (l - 1)) & 1 else 0
+        if size and lost and end <= lost[1] and lost[0] < end + size:
+            want[:, cols, l] = True
+        end += size
+    n0 = T - T % 64                                          # outputs of whole chunks are not the tail's
+    assert torch.equal(~torch.isfinite(o2[n0:, 0]), rows[n0:])
+    assert torch.equal(~torch.isfinite(s2[0]), want)
+    # what stays finite is what it was
+    assert torch.equal(s2[1], s1[1]) and torch.equal(o2[n0:, 1], o1[n0:, 1])
+    assert torch.equal(o2[n0:, 0][~rows[n0:]], o1[n0:, 0][~rows[n0:]])
+    assert torch.equal(s2[0][~want], s1[0][~want])
+
+
 @pytest.mark.parametrize("T", [50, 64, 114])
 def test_a_decay_of_minus_infinity_forgets(T):
     """Whatever came before a token with g = -inf is gone, and nothing else changes (T <= 64 of it in the tail's own arithmetic)."""
