@@ -156,6 +156,10 @@ def test_prefill_with_ragged_tail_and_decode(lb, T, K, V):
     (64 * 5 + 63, 1, 64, 64, 1),      # longest tail
     (64 * 31 + 17, 1, 64, 64, 0),     # five chunk levels live
     (64 * 511 + 5, 1, 64, 64, 0),     # nine
+    # tails taken in at once at head dims up to 32 (48 tokens and more), behind two live chunk levels, an even number of chunks, and
+    # five levels, one more than a batch of slots (at K = 16 the bf16 transitions leave older levels less than these bounds ask for:
+    # test_a_tail_is_decode_steps looks at what the tail does to them)
+    (64 * 5 + 63, 2, 32, 32, 1), (64 * 6 + 50, 2, 32, 32, 0), (64 * 31 + 50, 1, 32, 32, 0), (64 * 6 + 50, 2, 16, 32, 0),
 ])
 def test_prefill_tail_edges(lb, T, H, K, V, extra):
     """Two rows of ragged prompts: outputs and states of the fp32 tail at the edges of its slots and lengths."""

@@ -50,7 +50,7 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
         for h in range(H):
             ro, rs = _fenwick64(*(x[i, :, h].double() for x in (qn, kn, v, g, b, lam)))
             d = st.states[i, h].cpu().double() - rs
-            # One decay factor is exp to two ulp, 2^-22.  At once (no tail, or one of 48 tokens and more) an element goes through one such
+            # One decay factor is exp to two ulp, 2^-22.  At once (no tail, or one of 16 or 48 tokens and more) an element goes through one such
             # factor and a few dozen roundings of 2^-24: four times 2^-22.  Token by token it goes through one factor per token, and
             # their errors may all point the same way.
             bound = 2.0 ** -22 * (4 if T == n0 or T - n0 >= (16 if K == 64 else 48) else max(4, T))
@@ -61,6 +61,44 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
                 assert (e.abs() <= eps * ro[n0:].abs() + 2 * bound * ro[n0:].abs().max()).all()
     want = [1 if T > 0 else 0] + [(1 << (l - 1)) if ((T - 1) >> (l - 1)) & 1 else 0 for l in range(1, L)]
     assert st.counts.view(-1)[:L].tolist() == want
+
+
+# one chunk level live, two, an even number of chunks, five (one more than a batch of slots) and nine
+@pytest.mark.parametrize("K,V", [(64, 64), (32, 32), (16, 32)])
+@pytest.mark.parametrize("chunks,tail", [(2, 50), (5, 63), (6, 50), (31, 50), (511, 57)])
+def test_a_tail_is_decode_steps(K, V, chunks, tail):
+    """A tail taken in at once continues from the chunk levels as decode steps from the whole chunks' state do."""
+    B, H, n0 = 2, 2, 64 * chunks
+    T = n0 + tail
+    L = lampa_b200.num_levels_required(T) + 1
+    gen = torch.Generator(device="cuda").manual_seed(T + K)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x = [rn(B, T, H, K).bfloat16(), rn(B, T, H, K).bfloat16(), rn(B, T, H, V).bfloat16(), -F.softplus(rn(B, T, H) - 3), F.softplus(rn(B, T, H, L)),
+         torch.sigmoid(rn(B, T, H))]
+
+    def run(a, b, state=None):
+        return lampa_b200.chunk_h_gated_delta_rule(*(t[:, a:b].contiguous() for t in x), initial_state=state, output_final_state=True,
+                                                   use_qk_l2norm_in_kernel=True)
+
+    o, st = run(0, T)
+    _, steps = run(0, n0)
+    start = steps.states.flatten(2).norm(dim=-1)              # per row and head
+    outs = []
+    for t in range(n0, T):
+        ot, steps = run(t, t + 1, steps)
+        outs.append(ot)
+    lampa_b200.check_status(torch.device("cuda:0"))
+    assert torch.equal(st.counts, steps.counts)
+    # A token's transition is a contraction, entered with an error of a few 2^-24 and one decay factor to 2^-22: 2^-21 of the state
+    # per token, of the steps and of the closed form, on states that grow by their token (at most |v|) each.
+    bound = 2 * tail * 2.0 ** -21 * (start + x[2].float()[:, n0:].norm(dim=-1).amax(1))
+    d = (st.states - steps.states).flatten(2, 3).norm(dim=2)        # per row, head and level
+    assert (d <= bound[..., None]).all(), float((d / bound[..., None]).max())
+    want = torch.cat(outs, 1).float()
+    # both are rounded to bf16 (half a step each, 2^-8 of the value at most)
+    lam = x[4][:, n0:].amax(-1)
+    limit = 2.0 ** -7 * want.abs() + (x[0].float()[:, n0:].norm(dim=-1).clamp(max=1.0) * lam * L ** 0.5 * bound[:, None])[..., None]
+    assert ((o[:, n0:].float() - want).abs() <= limit).all()
 
 
 # a tail taken in at once behind a whole chunk, a prompt that is nothing but such a tail, and one that ends with a whole chunk; the
@@ -109,24 +147,34 @@ def test_values_that_are_not_finite_reach_what_comes_after(K, V, T, n, what, val
     assert torch.equal(s2[0][~want], s1[0][~want])
 
 
-@pytest.mark.parametrize("T", [50, 64, 114])
-def test_a_decay_of_minus_infinity_forgets(T):
-    """Whatever came before a token with g = -inf is gone, and nothing else changes (T <= 64 of it in the tail's own arithmetic)."""
-    H, K, V, L = 2, 32, 32, 9
+# in the tail, taken in at once (64 x 64) and token by token, with no whole chunk, one, and several chunk levels in front
+@pytest.mark.parametrize("K,V", [(64, 64), (32, 32)])
+@pytest.mark.parametrize("T", [40, 57, 114, 64 * 7 + 40])
+def test_a_decay_of_minus_infinity_forgets(T, K, V):
+    """Whatever came before a token with g = -inf is gone, and nothing else changes.  (The tail's own arithmetic: whole chunks go
+    through the chunkwise kernels, which take finite decays.)"""
+    H, L = 2, 12
     gen = torch.Generator(device="cuda").manual_seed(T)
     rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
-    n = T - 20                                               # inside the last chunk or the tail
+    n0, n = T - T % 64, T - 20
     x = [rn(1, T, H, K).bfloat16(), rn(1, T, H, K).bfloat16(), rn(1, T, H, V).bfloat16(), -F.softplus(rn(1, T, H)), F.softplus(rn(1, T, H, L)),
          torch.sigmoid(rn(1, T, H))]
-    kw = dict(output_final_state=True, use_qk_l2norm_in_kernel=True)
+    assert n >= n0
+    run = lambda: lampa_b200.chunk_h_gated_delta_rule(*x, output_final_state=True, use_qk_l2norm_in_kernel=True)
     x[3][:, n] = -200.0                                      # e^-200 is zero in fp32
-    o1, s1 = lampa_b200.chunk_h_gated_delta_rule(*x, **kw)
-    if T < 64:                                               # (whole chunks go through the chunkwise kernels, which take finite decays)
-        x[3][:, n] = float("-inf")
-    o2, s2 = lampa_b200.chunk_h_gated_delta_rule(*x, **kw)
+    o1, s1 = run()
+    x[3][:, n] = float("-inf")
+    o2, s2 = run()
     assert torch.isfinite(o2).all() and torch.isfinite(s2.states).all()
     assert torch.equal(o1, o2) or (o1.float() - o2.float()).norm() <= 1e-2 * o1.float().norm()
     assert (s1.states - s2.states).norm() <= 1e-6 * s1.states.norm()
+    for i in (1, 2):                                         # other keys and values before token n
+        x[i][:, :n] = rn(*x[i][:, :n].shape).bfloat16()
+    o3, s3 = run()
+    assert not torch.equal(o3[:, :n], o2[:, :n])
+    # Forgotten to the bit where a decay enters as a factor.  The closed form multiplies the differences of running sums that are
+    # -1e5 apart: e^-1e5 is zero too.
+    assert torch.equal(o3[:, n:], o2[:, n:]) and torch.equal(s3.states, s2.states)
 
 
 # one tiled copy per slab up to 32 levels, row by row beyond; more slabs than fit the GPU at once, and few
