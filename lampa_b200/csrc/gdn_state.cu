@@ -82,14 +82,16 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // Without a tail a ragged last chunk (cu_seqlens) is completed with null tokens (k = v = 0, beta = 0, g = 0).
 // Also writes counts.
 //
-// 64 tokens at a time in closed form instead of one after the other.  With G the running sum of g and
+// This kernel is for a longer tail: it and the chunk in front of it in closed form instead of one token after the other.  With G the running sum of g and
 // E_ij = e^{G_i - G_j} (j <= i), the states are independent linear recurrences with the same transitions:
 //     T = (I + tril(diag(beta) K K^T .* E, -1))^-1 diag(beta)          R = (tril(Q K^T) .* E) T
 //     a level that holds tokens j in J:   S = K^T diag(e^{Gl-G}) T[:, J] V[J]
 //     a slot that enters with X:          X <- e^{Gl} X - K^T diag(e^{Gl-G}) T diag(e^G) K X
 //     o_i = sum_j lambda[i, bit_length(i^j)] R_ij v_j + sum_slots lambda[i, slot] (e^{G_i} q_i X - (R diag(e^G) K X)_i)
 // all of it at fp32 accuracy: the products on the tensor cores with every operand in three bf16 pieces (split3.cuh), the 16 x 16
-// diagonal blocks of the inverse by substitution, and G summed in double so that E is exact to fp32.
+// diagonal blocks of the inverse by substitution, and G summed in double, so that an exponent G_i - G_j is rounded once however long
+// the sums are; E is __expf of it (two ulp and one more per unit of the exponent).  Error of the states against float64, 64
+// tokens of 64 x 64 heads: 0.9e-7 with g around -2, 1.3e-7 around -0.05, 3e-7 around -0.0025; token by token 0.4e-7, 1.9e-7, 4.2e-7.
 // A CTA takes eight state columns of a (sequence, head) after the other, as many as leave one CTA to an SM (one set of eight while
 // there are SMs for all); T and R do not depend on the column and are formed once by each CTA, two halves of it on the last
 // chunk and the tail side by side.  A column's arithmetic is the same whichever CTA has it.
@@ -100,7 +102,7 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
 // pass (launch_chained): the call 95 -> 67 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
-// cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (68 us the call).
+// cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (the call 68 us instead of 63).
 // -------------------------------------------------------------------------------------------------
 constexpr int TAIL_COLS = 8, TAIL_THREADS = 512, TAIL_GRP = 256, TAIL_BATCH = 4;      // states formed at a time
 constexpr int TAIL_AP = CHUNK + 4, TAIL_XP = TAIL_BATCH * TAIL_COLS + 4;              // pitches of 64- and 32-wide rows
@@ -113,7 +115,7 @@ struct TailSmem {                                            // offsets in float
     static constexpr int CH = CHUNK * KP + CHUNK * TAIL_AP + CHUNK * TAIL_COLS + SCAL;       // k, A -> T, v, scalars of one chunk
     static constexpr int K_ = 0, A_ = CHUNK * KP, V_ = A_ + CHUNK * TAIL_AP, S_ = V_ + CHUNK * TAIL_COLS;
     static constexpr int Z = CH;                             // [64][XP]
-    static constexpr int B = Z + CHUNK * TAIL_XP;            // (tail only) the tail's chunk
+    static constexpr int B = Z + CHUNK * TAIL_XP;            // the tail's chunk
     static constexpr int Q = B + CH;                         // [64][KP]
     static constexpr int P = Q + CHUNK * KP;                 // [64][AP], then R
     static constexpr int OUT = P + CHUNK * TAIL_AP;          // [64][8]
@@ -123,7 +125,7 @@ struct TailSmem {                                            // offsets in float
     static_assert(Y + CHUNK * TAIL_XP <= CH, "slots must fit");
     static_assert(CH % 4 == 0 && Q % 4 == 0 && LAM % 4 == 0, "16-byte rows");
     __host__ __device__ static constexpr int sum(int L) { return LAM + (CHUNK * L + 3) / 4 * 4 + KD * TAIL_COLS * L; }
-    __host__ __device__ static constexpr int floats(bool tail, int L, int slabs) { return tail ? sum(L) + slabs * KD * TAIL_COLS : B; }
+    __host__ __device__ static constexpr int floats(int L, int slabs) { return sum(L) + slabs * KD * TAIL_COLS; }
 };
 
 __device__ __forceinline__ void tail_meet(int grp) { asm volatile("bar.sync %0, %1;\n" :: "r"(grp + 1), "n"(TAIL_GRP) : "memory"); }
@@ -199,17 +201,11 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
     const int seq = blockIdx.x, h = blockIdx.y, H = a.H, L = a.L;
     const int tid = threadIdx.x, lane = tid & 31, gq = lane >> 2, tq = lane & 3, grp = tid / TAIL_GRP, t = tid % TAIL_GRP;
     int v0 = blockIdx.z * ta.slabs * TAIL_COLS;              // the first of the state columns that are being worked on
-    int nch = ta.n0;
-    int64_t tok0 = (int64_t)seq * a.fixed_stride, tok_end = 0;
-    if (ta.n0 < 0) {
-        const SeqLoc sq = locate_seq(a, seq);
-        nch = sq.nch; tok0 = sq.tok0; tok_end = sq.tok_end;
-    }
+    const int nch = ta.n0;
+    const int64_t tok0 = (int64_t)seq * a.fixed_stride;
     const int lvl0 = nch > 0 ? ELL0 + __ffs(nch) - 1 : -1;   // the slot that takes in the last chunk's tokens
-    const bool room = nch == 0 || lvl0 < L;                  // the first cascade must not leave the last level
-    const bool tailed = ta.tail > 0 && room;
     // tokens of the tail that are taken in: before token t > 0 levels 0..tz(t) move up one, which ends with the last level
-    const int done = tailed ? min(ta.tail, L < ELL0 ? 1 << (L - 1) : CHUNK) : 0;
+    const int done = min(ta.tail, L < ELL0 ? 1 << (L - 1) : CHUNK);
     const size_t bh = (size_t)seq * H + h;
     float* st = ta.states + (bh * KD * VD + v0) * L;         // row k: VD * L floats further each
     // the chunk a thread group works on: the last whole one, or the tail
@@ -247,11 +243,10 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             d[i] = raw_float(load_raw(a.v, ((size_t)(t0 + r) * H + h) * VD + c0 + i % TAIL_COLS, a.qkv_dt, r < len), a.qkv_dt);
         }
     };
-    const bool mine = grp == 0 ? nch > 0 : tailed;
-    if (mine) {
+    if (grp == 1 || nch > 0) {
         const bool tail = grp == 1;
         const int64_t t0 = tok0 + (int64_t)(tail ? nch : nch - 1) * CHUNK;
-        const int len = tail ? done : (ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - t0));
+        const int len = tail ? done : CHUNK;
         // rows as the kernel uses them, rows up to 64 null tokens: eight elements per thread and step, KD / 8 threads per row; every
         // load is in flight before the first is used
         constexpr int PPR = KD / 8, NIT = (CHUNK * PPR + TAIL_GRP - 1) / TAIL_GRP, NV = CHUNK * TAIL_COLS / TAIL_GRP, NL = 4;
@@ -394,7 +389,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         }
         tail_meet(grp);
         tail_inverse(sA, sBeta, t, grp);
-        for (int s = 0; s < ta.slabs && !tail && tailed; ++s) {      // all tokens of the last chunk as one state: they join a slot
+        for (int s = 0; s < ta.slabs && !tail; ++s) {      // all tokens of the last chunk as one state: they join a slot
             const int w = t >> 5;
             if (s > 0) {
                 tail_meet(grp);
@@ -423,12 +418,9 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         }
     }
     __syncthreads();
-    if (ta.early && !tailed) (void)chain_wait();             // the states are written from here on
-    // from here on everybody works on the tail's chunk, or on the last whole one when there is no tail
-    const float* cs = sm + (tailed ? M::B : 0);
+    // from here on everybody works on the tail's chunk
+    const float* cs = sm + M::B;
     const float *cK = cs + M::K_, *cT = cs + M::A_, *cV = cs + M::V_, *cEg = cs + M::S_ + 2 * CHUNK, *cEl = cEg + CHUNK;
-    const int r_all = tailed ? done : (nch > 0 ? CHUNK : 0);
-    const int len_all = tailed ? done : nch == 0 ? 0 : ta.n0 >= 0 ? CHUNK : (int)min((int64_t)CHUNK, tok_end - tok0 - (int64_t)(nch - 1) * CHUNK);
     const int row = tid >> 3, c8 = tid & 7;                  // row and column of what goes element by element
     const int warp = tid >> 5, mt = warp & 3, nt = warp >> 2;       // products: 16 rows, and eight columns: state nt of a batch
     // tokens of a chunk with a k or beta that is not finite, and with such a g, as masks; and what they take with them
@@ -440,19 +432,14 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
         m.g = (unsigned long long)__ballot_sync(0xffffffffu, f[CHUNK + 32]) << 32 | __ballot_sync(0xffffffffu, f[CHUNK]);
         return m;
     };
-    const Lost lost = r_all > 0 ? lost_tokens(cs) : Lost{0, 0}, before = tailed && nch > 0 ? lost_tokens(sm) : Lost{0, 0};
+    const Lost lost = lost_tokens(cs), before = nch > 0 ? lost_tokens(sm) : Lost{0, 0};
     const unsigned long long lost_out = lost.kb | (nch > 0 ? lost.g : lost.g & ~1ull), lost_in = lost.kb | lost.g >> 1;
     const int first_lost = lost_out ? __ffsll((long long)lost_out) - 1 : CHUNK;      // outputs from this token on
     const int last_lost = lost_in ? 63 - __clzll((long long)lost_in) : -1;           // states with a token up to this one
     const bool lost_slots = (lost.kb | lost.g) != 0, lost_before = (before.kb | before.g >> 1) != 0;
     const float nan = __int_as_float(0x7fffffff);
 
-    // where a state element of the result goes: the slab, which leaves at the end, or (no tail) the state itself
-    auto put = [&](int k, int v, int l, float x) {
-        if (tailed) slab[(k * TAIL_COLS + v) * L + l] = x;
-        else st[((size_t)k * VD + v) * L + l] = x;
-    };
-    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z, state nt to level l, or what is left of it (`gone`: nothing)
+    // states of the batch = e^{Gl} X (with X: the slots) -+ K^T Z, state nt to level l of the slab, or what is left of it (`gone`: nothing)
     auto kt_product = [&](const float* X, int l, bool gone) {
         if (mt >= KD / 16 || l < 0 || l >= L) return;        // (warp-uniform)
         float c[1][1][4] = {};
@@ -462,12 +449,11 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int k = 16 * mt + gq + 8 * (e >> 1), v = 2 * tq + (e & 1);
-            put(k, v, l, gone ? nan : X ? egl * X[k * XP + 8 * nt + v] - c[0][0][e] : c[0][0][e]);
+            slab[(k * TAIL_COLS + v) * L + l] = gone ? nan : X ? egl * X[k * XP + 8 * nt + v] - c[0][0][e] : c[0][0][e];
         }
     };
 
-    if (tailed) {
-        // R = P T, both lower triangular: warp = (16 rows, column tiles nt and nt + 4)
+    {   // R = P T, both lower triangular: warp = (16 rows, column tiles nt and nt + 4)
         float c[2][1][1][4] = {};
         const float* const P1[1] = {sP};
 #pragma unroll
@@ -487,52 +473,45 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             __syncthreads();                                 // the slab before is done with
             v0 += TAIL_COLS;
             st += TAIL_COLS * L;
-            stage_values(const_cast<float*>(cV), tid, TAIL_THREADS, tok0 + (int64_t)(tailed ? nch : nch - 1) * CHUNK, len_all, v0);
+            stage_values(const_cast<float*>(cV), tid, TAIL_THREADS, tok0 + (int64_t)nch * CHUNK, done, v0);
             __syncthreads();
         }
-        if (tailed) {
-            for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
-            // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
-            // row i reads are the 2^(l-1) below the highest set bit they differ in
-            {
-                const int hf = (tid >> 2) & 1, jg = tid & 3;
-                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (row < done) {
-                    for (int l = 0; l < ELL0 && l < L; ++l) {
-                        if (l > 0 && !((row >> (l - 1)) & 1)) continue;
-                        const int j0 = l == 0 ? row : (row >> l) << l, j1 = l == 0 ? row + 1 : j0 + (1 << (l - 1));
-                        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-                        for (int j = j0 + jg; j < j1; j += 4) {
-                            const float f = sP[row * AP + j];
-                            const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * hf);
-                            u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
-                        }
-                        const float w = sLam[row * L + l];
-                        o.x = fmaf(w, u.x, o.x); o.y = fmaf(w, u.y, o.y); o.z = fmaf(w, u.z, o.z); o.w = fmaf(w, u.w, o.w);
+        for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) slab[i] = 0.f;
+        // outputs from the tail's own tokens: thread = (row, half of the columns, every fourth token); the tokens of level l >= 1 that
+        // row i reads are the 2^(l-1) below the highest set bit they differ in
+        {
+            const int hf = (tid >> 2) & 1, jg = tid & 3;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < done) {
+                for (int l = 0; l < ELL0 && l < L; ++l) {
+                    if (l > 0 && !((row >> (l - 1)) & 1)) continue;
+                    const int j0 = l == 0 ? row : (row >> l) << l, j1 = l == 0 ? row + 1 : j0 + (1 << (l - 1));
+                    float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int j = j0 + jg; j < j1; j += 4) {
+                        const float f = sP[row * AP + j];
+                        const float4 v = *reinterpret_cast<const float4*>(cV + j * TAIL_COLS + 4 * hf);
+                        u.x = fmaf(f, v.x, u.x); u.y = fmaf(f, v.y, u.y); u.z = fmaf(f, v.z, u.z); u.w = fmaf(f, v.w, u.w);
                     }
+                    const float w = sLam[row * L + l];
+                    o.x = fmaf(w, u.x, o.x); o.y = fmaf(w, u.y, o.y); o.z = fmaf(w, u.z, o.z); o.w = fmaf(w, u.w, o.w);
                 }
-#pragma unroll
-                for (int d = 1; d < 4; d <<= 1) {
-                    o.x += __shfl_xor_sync(0xffffffffu, o.x, d); o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
-                    o.z += __shfl_xor_sync(0xffffffffu, o.z, d); o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
-                }
-                if (jg == 0) *reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * hf) = o;
             }
+#pragma unroll
+            for (int d = 1; d < 4; d <<= 1) {
+                o.x += __shfl_xor_sync(0xffffffffu, o.x, d); o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
+                o.z += __shfl_xor_sync(0xffffffffu, o.z, d); o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
+            }
+            if (jg == 0) *reinterpret_cast<float4*>(sOut + row * TAIL_COLS + 4 * hf) = o;
         }
         // token levels that hold tokens, four at a time: bit l of `held`
-        const uint32_t held = r_all > 0 ? (uint32_t)(r_all - 1) << 1 | 1u : 0u;
+        const uint32_t held = (uint32_t)(done - 1) << 1 | 1u;
         auto nth = [](uint32_t m, int n) {                       // its n-th level, or -1
             for (int i = 0; i < n; ++i) m &= m - 1;
             return m ? __ffs(m) - 1 : -1;
         };
-        if (!tailed)                                             // the slab is zero where no level is
-            for (int i = tid; i < KD * TAIL_COLS * 8; i += TAIL_THREADS) {
-                const int l = i & 7;
-                if (l < ELL0 && l < L && !((held >> l) & 1)) put(i >> 6, (i >> 3) & 7, l, 0.f);
-            }
         for (int n0 = 0; n0 < __popc(held); n0 += TAIL_BATCH) {
             const int l = nth(held, n0 + nt);
-            const int j0 = l < 0 ? 0 : l == 0 ? r_all - 1 : ((r_all - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? r_all : j0 + (1 << (l - 1));
+            const int j0 = l < 0 ? 0 : l == 0 ? done - 1 : ((done - 1) >> l) << l, j1 = l < 0 ? 0 : l == 0 ? done : j0 + (1 << (l - 1));
             float c[1][1][4] = {};
             const float* const T1[1] = {cT};
             tile_product3<1, 1, false, false>(c, T1, AP, 16 * mt, cV, TAIL_COLS, 0, 1, j0 & ~15, min(16 * mt + 16, (j1 + 15) & ~15), lane, j0, j1);
@@ -545,73 +524,71 @@ __global__ void __launch_bounds__(TAIL_THREADS) hgdn_tail_kernel(GdnArgs a, Tail
             kt_product(nullptr, l, j0 <= last_lost);
             __syncthreads();
         }
-        if (s == 0 && ta.early && tailed) (void)chain_wait();        // the chunk levels are there
-        if (tailed) {
-            float *sX = sm + M::X, *sD = sm + M::D, *sY = sm + M::Y;
-            const int nslot = __popc((uint32_t)nch);
-            for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
-                fetch_slots(s0);
+        if (s == 0 && ta.early) (void)chain_wait();        // the chunk levels are there
+        float *sX = sm + M::X, *sD = sm + M::D, *sY = sm + M::Y;
+        const int nslot = __popc((uint32_t)nch);
+        for (int s0 = 0; s0 < nslot; s0 += TAIL_BATCH) {
+            fetch_slots(s0);
 #pragma unroll
-                for (int i = 0; i < XR; ++i)
-                    sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs != 0 ? 0.f : lost_before ? nan : sSum[(s * KD + xk + 16 * i) * TAIL_COLS + xv]);
-                __syncthreads();
-                const int l = slot_level(s0 + nt);
-                float y[4];
-                {   // K X and Q X
-                    float c[2][1][4] = {};
-                    const float* const kq[2] = {cK, sQ};
-                    tile_product3<2, 1, false, false>(c, kq, KP, 16 * mt, sX, XP, 8 * nt, 1, 0, KD, lane);
+            for (int i = 0; i < XR; ++i)
+                sX[(xk + 16 * i) * XP + 8 * xs + xv] = xr[i] + (s0 + xs != 0 ? 0.f : lost_before ? nan : sSum[(s * KD + xk + 16 * i) * TAIL_COLS + xv]);
+            __syncthreads();
+            const int l = slot_level(s0 + nt);
+            float y[4];
+            {   // K X and Q X
+                float c[2][1][4] = {};
+                const float* const kq[2] = {cK, sQ};
+                tile_product3<2, 1, false, false>(c, kq, KP, 16 * mt, sX, XP, 8 * nt, 1, 0, KD, lane);
 #pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        const int i = 16 * mt + gq + 8 * hh;
-                        *reinterpret_cast<float2*>(sD + i * XP + 8 * nt + 2 * tq) = make_float2(cEg[i] * c[0][0][2 * hh], cEg[i] * c[0][0][2 * hh + 1]);
-                        y[2 * hh] = cEg[i] * c[1][0][2 * hh];
-                        y[2 * hh + 1] = cEg[i] * c[1][0][2 * hh + 1];
-                    }
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * mt + gq + 8 * hh;
+                    *reinterpret_cast<float2*>(sD + i * XP + 8 * nt + 2 * tq) = make_float2(cEg[i] * c[0][0][2 * hh], cEg[i] * c[0][0][2 * hh + 1]);
+                    y[2 * hh] = cEg[i] * c[1][0][2 * hh];
+                    y[2 * hh + 1] = cEg[i] * c[1][0][2 * hh + 1];
                 }
-                __syncthreads();
-                {   // T and R times that
-                    float c[2][1][4] = {};
-                    const float* const tr[2] = {cT, sP};
-                    tile_product3<2, 1, false, false>(c, tr, AP, 16 * mt, sD, XP, 8 * nt, 1, 0, 16 * mt + 16, lane);
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        const int i = 16 * mt + gq + 8 * hh;
-                        const float w = l >= 0 && i < done ? sLam[i * L + l] : 0.f;
-                        *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
-                        *reinterpret_cast<float2*>(sY + i * XP + 8 * nt + 2 * tq) = make_float2(w * (y[2 * hh] - c[1][0][2 * hh]), w * (y[2 * hh + 1] - c[1][0][2 * hh + 1]));
-                    }
-                }
-                __syncthreads();
-                {
-                    const float* p = sY + row * XP + c8;         // the slots of the batch
-                    sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
-                }
-                kt_product(sX, l, lost_slots);
-                __syncthreads();
             }
-            const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
-            for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
-                store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, i / TAIL_COLS < first_lost ? sOut[i] : nan, a.qkv_dt);
-            if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
-                fence_async_shared();
-                __syncthreads();
-                if (tid < KD) {
-                    bulk_s2g(st + (size_t)tid * VD * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
-                    bulk_commit();
-                    bulk_wait_read();
+            __syncthreads();
+            {   // T and R times that
+                float c[2][1][4] = {};
+                const float* const tr[2] = {cT, sP};
+                tile_product3<2, 1, false, false>(c, tr, AP, 16 * mt, sD, XP, 8 * nt, 1, 0, 16 * mt + 16, lane);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int i = 16 * mt + gq + 8 * hh;
+                    const float w = l >= 0 && i < done ? sLam[i * L + l] : 0.f;
+                    *reinterpret_cast<float2*>(sZ + i * XP + 8 * nt + 2 * tq) = make_float2(cEl[i] * c[0][0][2 * hh], cEl[i] * c[0][0][2 * hh + 1]);
+                    *reinterpret_cast<float2*>(sY + i * XP + 8 * nt + 2 * tq) = make_float2(w * (y[2 * hh] - c[1][0][2 * hh]), w * (y[2 * hh + 1] - c[1][0][2 * hh + 1]));
                 }
-            } else {
-                __syncthreads();
-                for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) {
-                    const int k = i / (TAIL_COLS * L);
-                    st[(size_t)k * VD * L + (i - k * TAIL_COLS * L)] = slab[i];
-                }
+            }
+            __syncthreads();
+            {
+                const float* p = sY + row * XP + c8;         // the slots of the batch
+                sOut[row * TAIL_COLS + c8] += (p[0] + p[8]) + (p[16] + p[24]);
+            }
+            kt_product(sX, l, lost_slots);
+            __syncthreads();
+        }
+        const int64_t t0 = tok0 + (int64_t)nch * CHUNK;
+        for (int i = tid; i < done * TAIL_COLS; i += TAIL_THREADS)
+            store_from_float(a.o, ((size_t)(t0 + i / TAIL_COLS) * H + h) * VD + v0 + i % TAIL_COLS, i / TAIL_COLS < first_lost ? sOut[i] : nan, a.qkv_dt);
+        if (((uintptr_t)ta.states & 15) == 0) {              // every level: the slab goes out as bulk copies of 8 columns x L
+            fence_async_shared();
+            __syncthreads();
+            if (tid < KD) {
+                bulk_s2g(st + (size_t)tid * VD * L, slab + tid * TAIL_COLS * L, TAIL_COLS * L * 4);
+                bulk_commit();
+                bulk_wait_read();
+            }
+        } else {
+            __syncthreads();
+            for (int i = tid; i < KD * TAIL_COLS * L; i += TAIL_THREADS) {
+                const int k = i / (TAIL_COLS * L);
+                st[(size_t)k * VD * L + (i - k * TAIL_COLS * L)] = slab[i];
             }
         }
     }
-    if (ta.tail > 0 && done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
-    if (h == 0 && blockIdx.z == 0 && tid == 0 && (ta.n0 < 0 || !ta.one_count || seq == 0)) {
+    if (done < ta.tail && tid == 0 && h == 0 && blockIdx.z == 0) set_status(a.status, LAMPA_ERR_LEVELS, 31, seq);
+    if (h == 0 && blockIdx.z == 0 && tid == 0 && (!ta.one_count || seq == 0)) {
         const int64_t n = (int64_t)nch * CHUNK + done;     // tokens held
         int32_t* cn = ta.counts + (size_t)seq * L;
         int64_t rem = n > 0 ? n - 1 : 0;
@@ -969,24 +946,25 @@ __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs 
     }
 }
 
-// Which form takes a tail follows from the tail alone, because the two do not round alike: a prompt's state and outputs are the
-// same alone and in a batch.  The closed form takes 30 us whatever the tail (8 heads, K = V = 64; 12 us without one), a CTA to an SM;
-// the steps 19 us and 0.4 us per token behind the last chunk (0.25 at head dims up to 32), any number of CTAs.  Both begin beside
-// the output pass.  Whole calls of 2,944 tokens and a tail, steps against closed form: 63 and 63 us at 2 and 18 tokens, 77 and 70 at
-// 22, 84 and 72 at 32; without a tail 66 and 58.  6 heads of 16 and 32: 320 tokens and 30 30 and 35 us, 256 and 44 39 and 39.
-// In batches a CTA of the closed form works through several slabs: 8 heads of 64, 704 tokens and 16, 32 and 60 behind
-// them, 71, 83 and 103 us by steps and 91, 93 and 93 at once for four prompts, 359, 409 and 503 against 497, 507 and 513 for 32; without
-// a tail 55 and 65 us, 279 and 317.
+// Which form takes a tail follows from the tail alone (and from L, where a level is missing), because the two do not round alike: a
+// prompt's state and outputs are the same bits alone and in a batch.  The steps' time grows with the tail, the closed form's does not,
+// and both begin beside the output pass.  Whole calls in us, steps against closed form, 8 heads of 64: 704 tokens and 8, 16, 24 and 63 behind
+// them 53 and 56, 56 and 58, 59 and 58, 74 and 59; 2,944 tokens 66 and 65, 71 and 67, 75 and 67, 97 and 68.  Heads of 32 and 16,
+// 2,944 tokens and 40, 48 and 63: 52 and 52, 54 and 52, 58 and 53 (32), 47 and 47, 48 and 47, 52 and 48 (16).  In batches of more than a CTA
+// to an SM a CTA of the closed form works through several slabs and gains later: 704 tokens and 16, 32, 48 and 63 in four prompts 71 and 91,
+// 82 and 92, 94 and 93, 106 and 94.  Without a tail the steps are faster in every batch: 44 and 49 (704 tokens, one prompt), 55 and 65 (four),
+// 155 and 169 (16).
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
     dim3 grid(a.nseq, a.H, VD / TAIL_COLS);
     ProfScope prof("hgdn_tail", st);
-    if (ta.tail == 0 || ta.tail >= (KD == 64 ? 16 : 48)) {
+    const bool room = ta.n0 <= 0 || ELL0 + __builtin_ctz((unsigned)ta.n0) < a.L;      // the first cascade must not leave the last level
+    if (ta.tail >= (KD == 64 ? 16 : 48) && room) {
         using M = TailSmem<KD>;
         TailArgs tc = ta;
         while ((int64_t)a.nseq * a.H * grid.z > sm_count() && grid.z > 1) { grid.z /= 2; tc.slabs *= 2; }
-        const int smem = M::floats(ta.tail > 0, a.L, tc.slabs) * 4;
-        constexpr int most = M::floats(true, 40, VD / TAIL_COLS) * 4;
+        const int smem = M::floats(a.L, tc.slabs) * 4;
+        constexpr int most = M::floats(40, VD / TAIL_COLS) * 4;
         static_assert(most <= 227 * 1024, "shared memory of an SM");
         static std::atomic<uint64_t> ready;
         if (!allow_smem(ready, hgdn_tail_kernel<KD, VD>, most)) return LAMPA_ERR_CUDA;

@@ -50,9 +50,9 @@ def test_short_prompts_are_fp32(K, V, T, L, shift, dt):
         for h in range(H):
             ro, rs = _fenwick64(*(x[i, :, h].double() for x in (qn, kn, v, g, b, lam)))
             d = st.states[i, h].cpu().double() - rs
-            # One decay factor is exp to two ulp, 2^-22.  At once (no tail, or one of 16 or 48 tokens and more) an element goes through one such
+            # One decay factor is exp to two ulp, 2^-22.  At once (a tail of 16 or 48 tokens and more) an element goes through one such
             # factor and a few dozen roundings of 2^-24: four times 2^-22.  Token by token it goes through one factor per token, and
-            # their errors may all point the same way.
+            # their errors may all point the same way.  (A whole chunk goes token by token too, at the tighter bound: it is within 0.65 of it.)
             bound = 2.0 ** -22 * (4 if T == n0 or T - n0 >= (16 if K == 64 else 48) else max(4, T))
             assert d.norm() <= bound * rs.norm(), (float(d.norm()), float(rs.norm()))
             if T > n0:
