@@ -269,7 +269,7 @@ def run_ours(args):
 
     # Device-resident leg.  Events are independent, so `--streams S` keeps S of them in flight, each on its own
     # stream with its own inputs and its own intermediates: kernels that cannot fill the GPU alone (the 120-CTA
-    # sort, the 40-CTA level scan, the second, partly empty round of the output pass) overlap with the other
+    # sort, the 160 single-warp CTAs of the level scan, the second, partly empty round of the output pass) overlap with the other
     # event's kernels.  S = 1 is the plain back-to-back sequence and is always reported beside it.
     n_streams = max(1, args.streams)
     streams = [torch.cuda.Stream(dev) for _ in range(n_streams)]
@@ -288,7 +288,7 @@ def run_ours(args):
             return step(inputs[k])
 
     def capture_graphs():
-        # one CUDA graph per stream: the nine launches and their scratch allocations of a step, replayed
+        # one CUDA graph per stream: the seven launches and their scratch allocations of a step, replayed
         for k in range(n_streams):
             g = torch.cuda.CUDAGraph()
             with torch.cuda.stream(streams[k]):

@@ -153,7 +153,9 @@ int lampa_hgdn_final_state(const lampa_gdn_desc* d, const void* k, const void* v
 /*
  * The forward and the Fenwick state of B equally long prompts in one call, T any length.
  * Replaces: hattention_prefill (models/hattention/kernel.py:470-560) with its split into whole chunks and the
- * remaining T mod 64 tokens, which here take one launch (fp32, the arithmetic of lampa_hgdn_step) instead of one per token.
+ * remaining T mod 64 tokens, which here take one launch instead of one per token.  Both forms of it have fp32 accuracy: shorter tails
+ * go token by token, as lampa_hgdn_step takes them, longer ones (and none) all at once in closed form.  Which one follows from
+ * T mod 64 and K alone, so that a prompt's state and outputs are the same bits alone and in a batch.
  *   Arguments as in lampa_hgdn_fwd (no cu_seqlens) and lampa_hgdn_final_state, except: counts int32 [L], one row;
  *   the state is the one after all T tokens, no null tokens; the workspace is the one of the whole chunks
  *   (lampa_gdn_workspace_bytes with T rounded down to a multiple of 64).  L has to hold the T tokens; when the tail

@@ -58,7 +58,6 @@ struct Rec {
     static constexpr int OL_OFF = BT_OFF + BT_BYTES;
     static constexpr int OL_BYTES = TV::bytes(CHUNK); // O_local, bf16 (added once, in fp32, by the output pass)
     static constexpr int LAM_OFF = OL_OFF + OL_BYTES; // lambda of chunk levels: [LC][64] fp32
-    static constexpr int PRE_BYTES = OL_OFF;          // M, Q~, B^T: what the compose pass streams
     static constexpr int ALIGN = T::SWZ ? 1024 : 128; // records and shared-memory stages
     __host__ __device__ static constexpr int bytes(int LC) { return LAM_OFF + LC * CHUNK * 4; }
     // block composite, in the order in which the lanes of the level pass take it (16 bytes per lane, whole lines per warp):

@@ -286,7 +286,7 @@ struct Compose {
     static constexpr int SPW = SPLIT == 1 && KD == 64 ? 2 : 1;
     static constexpr int SLABS = SPLIT == 1 ? SLABS_S + SLABS_P : (SLABS_S > SLABS_P ? SLABS_S : SLABS_P);
     static constexpr int NW = SLABS / SPW;
-    static constexpr int GRP = 1, NST = 3;       // 74 KB: three CTAs to an SM
+    static constexpr int GRP = 1, NST = 3;       // 49 KB of M and B^T at K = V = 64; registers leave room for three CTAs to an SM
     static_assert(SLABS % SPW == 0 && SLABS_S % SPW == 0, "a warp's slabs are of one kind");
 };
 

@@ -60,13 +60,7 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
         const float4 u = __ldcg(reinterpret_cast<const float4*>((const float*)p + i)), v = __ldcg(reinterpret_cast<const float4*>((const float*)p + i) + 1);
         x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
     } else {
-        const uint4 u = __ldcg(reinterpret_cast<const uint4*>((const uint16_t*)p + i));
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = dt == LAMPA_BF16 ? unpack_bf16x2(w[e]) : __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-            x[2 * e] = f.x; x[2 * e + 1] = f.y;
-        }
+        raw_floats(load8_raw(p, i, true), dt, x);
     }
 }
 
@@ -90,8 +84,9 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 //     o_i = sum_j lambda[i, bit_length(i^j)] R_ij v_j + sum_slots lambda[i, slot] (e^{G_i} q_i X - (R diag(e^G) K X)_i)
 // all of it at fp32 accuracy: the products on the tensor cores with every operand in three bf16 pieces (split3.cuh), the 16 x 16
 // diagonal blocks of the inverse by substitution, and G summed in double, so that an exponent G_i - G_j is rounded once however long
-// the sums are; E is __expf of it (two ulp and one more per unit of the exponent).  Error of the states against float64, 64
-// tokens of 64 x 64 heads: 0.9e-7 with g around -2, 1.3e-7 around -0.05, 3e-7 around -0.0025; token by token 0.4e-7, 1.9e-7, 4.2e-7.
+// the sums are; E is __expf of it (two ulp and one more per unit of the exponent).  Error of the states against float64, prompts of 57
+// to 121 tokens, 64 x 64 heads: 0.9e-7 with g around -2, 1.4e-7 around -0.08, 2.5e-7 around -0.004 (3.8e-7 in fp16); token by token
+// 0.4e-7, 2.1e-7, 4.2e-7 to 7.5e-7.
 // A CTA takes eight state columns of a (sequence, head) after the other, as many as leave one CTA to an SM (one set of eight while
 // there are SMs for all); T and R do not depend on the column and are formed once by each CTA, two halves of it on the last
 // chunk and the tail side by side.  A column's arithmetic is the same whichever CTA has it.
