@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(NG * VD * 2, KD == 64 ? 1 : 6 / NG) gdn_out_hi
 // memory in its own register order, and eight warps a chunk behind add the terms, in the order of gdn_out_hier_kernel and so with
 // its results to the bit, add O_local and store.
 // A block's chunk is then two levels deep instead of five, with no barrier but the one at its top.  17 warps and 200 KB, a CTA to an
-// SM: taken while the blocks of all heads are at most one to an SM (one event of 9,001 points, 72 CTAs: 25 -> 21 us; two events
+// SM: taken while the blocks of all heads are at most one to an SM (one event of 9,001 points, 72 CTAs: 25 -> 20 us; two events
 // 509 -> 480 us for the whole model; three events, two rounds: 620 against 622; 64 events: 960 against 1270 us a pass).
 // -------------------------------------------------------------------------------------------------
 constexpr int LV_SUM = 8, LV_MAX_PAIRS = 5, LV_MAX_THREADS = (2 * LV_MAX_PAIRS + 1 + LV_SUM) * 32;

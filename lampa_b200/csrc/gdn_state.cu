@@ -94,8 +94,8 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // tokens before it.  What the recurrence makes of it is filled in: with a k or beta the states that hold the token or
 // older ones are NaN from then on, with a g those that hold older ones, and so are the outputs, which read them all.  (q, v and
 // lambda reach only what they belong to.)
-// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 30 us, 20 of which run beside the output
-// pass (launch_chained): the call 95 -> 67 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
+// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 35 us, 20 of which run beside the output
+// pass (launch_chained): the call 95 -> 66 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
 // cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (the call 68 us instead of 63).
 // -------------------------------------------------------------------------------------------------
