@@ -79,7 +79,7 @@ int lampa_gdn_workspace_bytes(const lampa_gdn_desc* d, size_t* bytes);
  * out[6] chunk-level lambda (fp32 [LC][64], hierarchical only); out[7] = LC, out[8] = number of
  * chunk slots, out[9] = chunks per block (8 for sequences of up to 256 chunks, 16 up to 512, then 32; 0 for packed
  * sequences, which each have their own), out[10] / out[11] = byte offsets of the block composites
- * and of the block entry states.
+ * and of the block entry states (both in an order of the kernels' own: gdn.cuh, Rec).
  */
 int lampa_gdn_workspace_layout(const lampa_gdn_desc* d, size_t out[12]);
 
