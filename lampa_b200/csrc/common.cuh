@@ -211,7 +211,7 @@ __device__ __forceinline__ bool chain_wait() {
 }
 __device__ __forceinline__ void chain_signal() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 // All threads of the grid, behind chain_wait().  One thread signals for its CTA.  The word is on its way when the first one does, and
-// there before the next grid's CTAs are (a fence between the two only makes everybody wait: 0.4 us of a prefill's 66).
+// there before the next grid's CTAs are (a fence between the two only makes everybody wait: 0.4 us of a prefill's 65).
 __device__ __forceinline__ void chain_signal(unsigned long long* word, unsigned long long call) {
     if (threadIdx.x != 0) return;
     if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {

@@ -94,8 +94,8 @@ __device__ __forceinline__ void load8_float(const void* p, size_t i, int dt, boo
 // tokens before it.  What the recurrence makes of it is filled in: with a k or beta the states that hold the token or
 // older ones are NaN from then on, with a g those that hold older ones, and so are the outputs, which read them all.  (q, v and
 // lambda reach only what they belong to.)
-// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 35 us, 20 of which run beside the output
-// pass (launch_chained): the call 95 -> 66 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
+// 3,001 tokens, 8 heads, K = V = 64: 43 us token by token (0.3 - 0.4 us each) -> 33 us, 20 of which run beside the output
+// pass (launch_chained): the call 95 -> 65 us.  What bounds it now is the chain of dependent phases, each a few thousand cycles for
 // a few hundred products, and in them the fetching of code that a CTA passes through once (the first stall reason in ncu).  As fp32 multiply-adds it was bound by shared-memory loads (a 16-byte load of a warp returns 512 bytes, four
 // cycles, for 16 multiply-adds of four) and took 34 us; one copy of the product that all phases call is slower (the call 68 us instead of 63).
 // -------------------------------------------------------------------------------------------------
@@ -945,11 +945,12 @@ __global__ void __launch_bounds__(STEPS_THREADS) hgdn_tail_steps_kernel(GdnArgs 
 
 // Which form takes a tail follows from the tail alone (and from L, where a level is missing), because the two do not round alike: a
 // prompt's state and outputs are the same bits alone and in a batch.  The steps' time grows with the tail, the closed form's does not,
-// and both begin beside the output pass.  Whole calls in us, steps against closed form, 8 heads of 64: 704 tokens and 8, 16, 24 and 63 behind
-// them 53 and 56, 56 and 58, 59 and 58, 74 and 59; 2,944 tokens 66 and 65, 71 and 67, 75 and 67, 97 and 68.  Heads of 32 and 16,
-// 2,944 tokens and 40, 48 and 63: 52 and 52, 54 and 52, 58 and 53 (32), 47 and 47, 48 and 47, 52 and 48 (16).  In batches of more than a CTA
-// to an SM a CTA of the closed form works through several slabs and gains later: 704 tokens and 16, 32, 48 and 63 in four prompts 71 and 91,
-// 82 and 92, 94 and 93, 106 and 94.  Without a tail the steps are faster in every batch: 44 and 49 (704 tokens, one prompt), 55 and 65 (four),
+// and both begin beside the output pass.  Whole calls in us, steps against closed form, 8 heads of 64: 704 tokens and 16, 24 and 63 behind
+// them 56 and 56, 59 and 56, 74 and 57; 2,944 tokens 71 and 65, 75 and 65, 97 and 67; 8 behind them 53 and 56, 66 and 65 (in the form for
+// several slabs, 1 to 2 slower).  Heads of 32 and 16, 2,944 tokens and 48 and 63: 54 and 51, 58 and 51 (32), 48 and 46, 52 and 46 (16); 40
+// behind them 52 and 52, 47 and 47 (the same form).  In batches of more than a CTA
+// to an SM a CTA of the closed form works through several slabs and gains later: 704 tokens and 16, 32, 48 and 63 in four prompts 71 and 90,
+// 82 and 91, 94 and 92, 106 and 93.  Without a tail the steps are faster in every batch: 44 and 49 (704 tokens, one prompt), 55 and 65 (four),
 // 155 and 169 (16).
 template <int KD, int VD>
 int launch_hgdn_tail(const GdnArgs& a, const TailArgs& ta, cudaStream_t st) {
